@@ -53,6 +53,7 @@ bool row_op_emits_planes(const Operator &op);
 bool row_op_is_softmax(const Operator &op, long long *rows, long long *cols);
 std::shared_ptr<Operator> gemm_with_row_softmax(const Operator &op, long long rows, long long cols, const TensorDesc &out, bool tc_enabled);
 std::shared_ptr<Operator> gemm_with_attention(const Operator &outer_op, const Operator &score_op, long long rows, long long cols, bool tc_enabled);
+bool attention_small_products(const Operator &outer_op, const Operator &score_op, std::shared_ptr<Operator> *outer, std::shared_ptr<Operator> *score);
 bool is_attention_op(const Operator &op);
 bool is_grouped_gemm_op(const Operator &op);
 bool gemm_operand_static_direct(const Operator &op, int idx);
@@ -213,6 +214,32 @@ static bool attention_enabled() {
 
 static void lower(Node &n, bool tc, bool softmax_in_gemm, bool attention) {
     if (n.is_data) return;
+    if (attention && tc && is_gemm_op(*n.op) && n.args.size() == 2) {
+        // gemm(softmax(f(gemm)), V) of a short sequence: put both products on the tensor cores so that they fold below
+        auto below = [](Node *p) {
+            while (!p->is_data && is_reshape_op(*p->op)) p = &p->args[0];
+            return p;
+        };
+        Node *p = below(&n.args[0]);
+        long long rows = 0, cols = 0;
+        if (!p->is_data && row_op_is_softmax(*p->op, &rows, &cols) && p->args.size() == 1) {
+            Node *s = below(&p->args[0]);
+            if (!s->is_data && !is_gemm_op(*s->op) && map_expr_of(*s->op)) {  // the map between the scores and the softmax
+                for (Node &a : s->args) {
+                    Node *g = below(&a);
+                    if (!g->is_data && is_gemm_op(*g->op)) {
+                        s = g;
+                        break;
+                    }
+                }
+            }
+            std::shared_ptr<Operator> outer, score;
+            if (!s->is_data && is_gemm_op(*s->op) && attention_small_products(*n.op, *s->op, &outer, &score)) {
+                n.op = outer;
+                s->op = score;
+            }
+        }
+    }
     for (Node &a : n.args) lower(a, tc, softmax_in_gemm, attention);
     if (is_gemm_op(*n.op) && tc && n.args.size() == 2) {
         // the column matrix of a convolution: made by the GEMM itself, as planes (this may also bring a product onto the

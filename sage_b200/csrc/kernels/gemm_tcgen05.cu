@@ -336,17 +336,26 @@ std::string jit_source(const std::string &defines, int bn, int ctas) {
 
 }  // namespace
 
-bool gemm_tc_shape_ok(long long m, long long n, long long k, long long batch) {
-    // Tiny problems are latency-bound and would be mostly TMA padding: leave them to the SIMT kernel.  A short M
-    // with a long K (the weight gradient of a first convolution: 49 x 64 x 25088) is worth the padding: it is
-    // cut into K slices that fill the machine.
-    if ((m < 64 && !(m >= 16 && k >= 2048)) || n < 32 || k < 32 || batch < 1) return false;
+// The smallest products the tiled kernel takes from a caller that must know beforehand (sage_gemm_noalloc).
+static bool shape_fills_tiles(long long m, long long n, long long k) { return (m >= 64 || (m >= 16 && k >= 2048)) && n >= 32 && k >= 32; }
+
+static bool shape_within_limits(long long m, long long n, long long k, long long batch) {
+    if (m < 1 || n < 1 || k < 1 || batch < 1) return false;
     if (m > 0x7fffffffLL || n > 0x7fffffffLL || k > 0x7fffffffLL || batch > 0x7fffffffLL) return false;
     const long long tiles = ((m + BM - 1) / BM) * ((n + 63) / 64) * batch;
     return tiles < 0x7fffffffLL;
 }
 
-bool gemm_tc_supported(const GemmArgs &g) { return gemm_tc_shape_ok(g.m, g.n, g.k, g.batch); }
+bool gemm_tc_shape_ok(long long m, long long n, long long k, long long batch) {
+    // Tiny problems are latency-bound and would be mostly TMA padding: leave them to the SIMT kernel.  A short M is
+    // worth the padding once there is a weight matrix to stream: the SIMT kernel walks K with one CTA per 128 columns
+    // (24 x 768 x 768: 90 us against 12 us here), so the line lies where its K loop outlasts a launch of this kernel.  Up
+    // to 4096 outputs its warp-per-output kernel is the faster one (1 x 1000 x 512: 6 us, 16 x 33 x 2047: 8 us).
+    if (!shape_fills_tiles(m, n, k) && !(n >= 32 && k >= 128 && n * k >= 65536 && m * n > 4096)) return false;
+    return shape_within_limits(m, n, k, batch);
+}
+
+bool gemm_tc_supported(const GemmArgs &g) { return shape_fills_tiles(g.m, g.n, g.k) && shape_within_limits(g.m, g.n, g.k, g.batch); }
 
 bool tc_operand_ok(const TcOperand &o) {
     const long long lim = 1LL << 38;  // strides in floats; TMA strides are below 2^40 bytes
@@ -510,7 +519,7 @@ int gemm_tc_split_plan(Context &ctx, const TcGemm &g) {
 }
 
 sage_status gemm_tc_run(Context &ctx, const TcGemm &g0) {
-    if (!gemm_tc_shape_ok(g0.m, g0.n, g0.k, g0.batch)) return ctx.fail(SAGE_ERR_UNSUPPORTED, "gemm_tc: shape not supported");
+    if (!shape_within_limits(g0.m, g0.n, g0.k, g0.batch)) return ctx.fail(SAGE_ERR_UNSUPPORTED, "gemm_tc: shape not supported");
     int bn = 0;
     const int S = pick_split_k(ctx, g0, &bn);
     if (S < 2) return gemm_tc_launch(ctx, g0);
@@ -811,9 +820,7 @@ bool attention_tc_shape_ok(long long lq, long long lk, long long d, long long ba
     if (lq < 1 || lk < 1 || d < 4 || d > 64 || d % 4 || batch < 1) return false;
     if (lq > 0x7fffffffLL || lk > 0x7fffffffLL || batch > 0x7fffffffLL) return false;
     const long long tiles = ((lq + 127) / 128) * batch;
-    // below one query tile's worth of work per batch the decomposed kernels are as good, and tiny score matrices
-    // are mostly padding here
-    return tiles < 0x7fffffffLL && lq * lk >= 1024;
+    return tiles < 0x7fffffffLL;
 }
 
 sage_status attention_tc_run(Context &ctx, const TcAttn &a) {
@@ -939,7 +946,7 @@ sage_status gemm_tcgen05_planes(Context &ctx, const GemmArgs &g, const SplitPlan
 }
 
 sage_status gemm_tcgen05(Context &ctx, const GemmArgs &g) {
-    if (!gemm_tc_supported(g)) return SAGE_ERR_UNSUPPORTED;
+    if (!gemm_tc_shape_ok(g.m, g.n, g.k, g.batch)) return SAGE_ERR_UNSUPPORTED;
     // A as stored: [M,K] (K-major) or, transposed, [K,M] (MN-major); B: [K,N] (MN-major) or [N,K] (K-major).
     SplitPlanes a, b;
     sage_status st = split_tf32(ctx, g.a, g.lda, g.stride_a, g.ta ? (int)g.k : (int)g.m, g.ta ? (int)g.m : (int)g.k, (int)g.batch, &a);
