@@ -141,8 +141,8 @@ sage_status sage_var_info(const sage_var *v, int32_t *dtype, int32_t *ndim, int6
 }
 
 sage_status sage_eval(sage_session *s, sage_var *const *targets, int32_t n) {
-    std::vector<Var> t;
-    for (int i = 0; i < n; ++i) t.push_back(targets[i]->v);
+    std::vector<const Var *> t((size_t)(n > 0 ? n : 0));
+    for (int i = 0; i < n; ++i) t[i] = &targets[i]->v;
     s->impl->ctx().make_current();
     sage_status st = s->impl->eval(t);
     if (st) g_error = s->impl->ctx().last_error();
@@ -343,7 +343,7 @@ sage_status sage_conv2d_nhwc(sage_ctx *ctx, const sage_tensor *x, const sage_ten
             if (y->extents[i] != 1 && y->strides[i] != run) shape_fail("conv2d: y must be contiguous");
             run *= y->extents[i];
         }
-        sage_status e = session.eval({out});
+        sage_status e = session.eval({&out});
         if (e) return e;
         Tensor t;
         if (!session.get(out, &t)) return C.fail(SAGE_ERR_INVALID, "internal: conv2d result missing");

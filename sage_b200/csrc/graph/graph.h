@@ -7,6 +7,8 @@
 #include <cstdint>
 #include <algorithm>
 #include <functional>
+#include <initializer_list>
+#include <iterator>
 #include <memory>
 #include <string>
 #include <unordered_map>
@@ -18,12 +20,85 @@
 
 namespace sage {
 
-typedef std::vector<long long> Array;
-
 struct ShapeError {
     std::string msg;
 };
 [[noreturn]] void shape_fail(const std::string &msg);  // throws ShapeError; caught at the C ABI
+
+// Extents / strides of a tensor: a vector of at most SAGE_MAX_DIMS values held in place.  A Tensor is copied for every
+// operand of every launch, and two heap allocations per copy were a third of the host's time per launch.
+class Array {
+public:
+    typedef long long value_type;
+    typedef long long *iterator;
+    typedef const long long *const_iterator;
+    Array() {}
+    explicit Array(size_t n, long long v = 0) { resize(n, v); }
+    Array(std::initializer_list<long long> l) { assign(l.begin(), l.end()); }
+    template <typename It, typename = typename std::iterator_traits<It>::iterator_category>
+    Array(It first, It last) { assign(first, last); }
+    template <typename It>
+    void assign(It first, It last) {
+        n_ = 0;
+        for (; first != last; ++first) push_back(*first);
+    }
+    size_t size() const { return n_; }
+    bool empty() const { return n_ == 0; }
+    long long *begin() { return v_; }
+    long long *end() { return v_ + n_; }
+    const long long *begin() const { return v_; }
+    const long long *end() const { return v_ + n_; }
+    long long *data() { return v_; }
+    const long long *data() const { return v_; }
+    long long &operator[](size_t i) { return v_[i]; }
+    long long operator[](size_t i) const { return v_[i]; }
+    long long &back() { return v_[n_ - 1]; }
+    long long back() const { return v_[n_ - 1]; }
+    void clear() { n_ = 0; }
+    void pop_back() { --n_; }
+    void push_back(long long v) {
+        room(1);
+        v_[n_++] = v;
+    }
+    void resize(size_t n, long long v = 0) {
+        if (n > n_) room(n - n_);
+        for (size_t i = n_; i < n; ++i) v_[i] = v;
+        n_ = (unsigned)n;
+    }
+    void insert(const long long *at, long long v) {
+        room(1);
+        const size_t i = (size_t)(at - v_);
+        for (size_t j = n_; j > i; --j) v_[j] = v_[j - 1];
+        v_[i] = v;
+        ++n_;
+    }
+    template <typename It>
+    void insert(const long long *at, It first, It last) {
+        const Array tail(at, (const long long *)end());
+        n_ = (unsigned)(at - v_);
+        for (; first != last; ++first) push_back(*first);
+        for (long long v : tail) push_back(v);
+    }
+    void erase(const long long *at) {
+        for (size_t j = (size_t)(at - v_); j + 1 < n_; ++j) v_[j] = v_[j + 1];
+        --n_;
+    }
+    bool operator==(const Array &o) const {
+        if (n_ != o.n_) return false;
+        for (unsigned i = 0; i < n_; ++i)
+            if (v_[i] != o.v_[i]) return false;
+        return true;
+    }
+    bool operator!=(const Array &o) const { return !(*this == o); }
+
+private:
+    static constexpr unsigned kMax = 16;  // twice SAGE_MAX_DIMS: shapes are joined before they are checked
+    void room(size_t more) const {
+        if (n_ + more > kMax) shape_fail("too many dimensions");
+    }
+    unsigned n_ = 0;
+    long long v_[kMax];
+};
 
 // ---------------------------------------------------------------- Shape (src/shape.rs:37-279)
 struct Shape {
@@ -183,7 +258,7 @@ public:
     ~Session();
     Context &ctx() { return *ctx_; }
     // Context::eval, context.rs:96-117: evaluates the targets; results stay in `data`.
-    sage_status eval(const std::vector<Var> &targets);
+    sage_status eval(const std::vector<const Var *> &targets);
     void clear();  // Context::clear, context.rs:92-94
     bool get(const Var &v, Tensor *out) const;
     std::unordered_map<Origin *, std::pair<Var, Tensor>> data;  // Context::data

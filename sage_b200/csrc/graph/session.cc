@@ -23,6 +23,7 @@ namespace sage {
 struct Node {
     bool is_data = false;
     Var var;                       // data leaf: an input of the routine
+    int slot = -1;                 // ... computed by the program or evaluated before it: its place in a scheduled run
     std::shared_ptr<Operator> op;  // operation
     std::vector<Node> args;
     bool emit_planes = false;      // a tensor-core GEMM reads the result: ask the operator for its tf32 planes
@@ -112,6 +113,20 @@ struct Program {
     std::unordered_map<Origin *, int> consumers;  // how many routines read each state
     bool fusion = true, pattern = true;
     std::shared_ptr<RowProgram> row;  // set: the whole program is one generated row kernel (rowfuse.h)
+
+    // The order a completed run took, kept so that later runs need no search: every value the routines exchange has a
+    // slot, and a step says which slots it was the last to read.
+    struct Step {
+        Routine *routine;
+        std::vector<int> outputs;   // slots of what it computes (several for a row group)
+        std::vector<int> release;
+    };
+    std::vector<Step> schedule;
+    std::unordered_map<Origin *, int> slot_of;
+    std::vector<std::pair<Origin *, int>> given;  // values evaluated before the program
+    std::vector<char> is_output;                  // per slot
+    std::vector<Tensor> slots;                    // empty between runs
+    bool times_read = false;
 };
 
 Session::Session(Context *ctx) : ctx_(ctx) {}
@@ -125,12 +140,10 @@ void Session::drop_programs() {
 }
 
 static uint64_t program_key_hash(const std::vector<Origin *> &targets, const std::vector<Origin *> &inputs) {
-    uint64_t h = 0xcbf29ce484222325ull;  // FNV-1a over the two pointer lists and their lengths
+    uint64_t h = 0xcbf29ce484222325ull;  // over the two pointer lists and their lengths
     auto mix = [&](uint64_t v) {
-        for (int i = 0; i < 8; ++i) {
-            h ^= (v >> (8 * i)) & 0xff;
-            h *= 0x100000001b3ull;
-        }
+        h = (h ^ v) * 0x9e3779b97f4a7c15ull;
+        h ^= h >> 29;
     };
     mix(targets.size());
     for (Origin *o : targets) mix((uint64_t)(uintptr_t)o);
@@ -715,9 +728,18 @@ static std::unique_ptr<Program> compile(const std::vector<Var> &x, std::vector<V
 // Routine::exec, session.rs:612-673 (a recursive walk instead of the flattened stack).
 typedef std::unordered_map<const Node *, Tensor> SharedMemo;  // results of shared nodes during one routine run
 
-static sage_status run_node(const Node &n, Context &ctx, Session &s, const std::unordered_map<Origin *, Tensor> &temp,
-                            SharedMemo &memo, Tensor *out) {
+// Where a routine finds the values it reads: the slots of a scheduled run, or the values kept so far by origin.
+struct Values {
+    const std::unordered_map<Origin *, Tensor> *temp = nullptr;
+    const Tensor *slots = nullptr;
+};
+
+static sage_status run_node(const Node &n, Context &ctx, Session &s, const Values &values, SharedMemo &memo, Tensor *out) {
     if (n.is_data) {
+        if (values.slots && n.slot >= 0) {
+            *out = values.slots[n.slot];
+            return SAGE_OK;
+        }
         Origin *o = n.var.key();
         if (!n.var.is_op()) {
             if (!o->data.defined()) return ctx.fail(SAGE_ERR_INVALID, "uninitialized variable" + (o->name.empty() ? "" : " " + o->name));
@@ -731,21 +753,22 @@ static sage_status run_node(const Node &n, Context &ctx, Session &s, const std::
             *out = it->second.second;
             return SAGE_OK;
         }
-        auto jt = temp.find(o);
-        if (jt == temp.end()) return ctx.fail(SAGE_ERR_INVALID, "internal: routine input not available");
+        if (!values.temp) return ctx.fail(SAGE_ERR_INVALID, "internal: routine input not available");
+        auto jt = values.temp->find(o);
+        if (jt == values.temp->end()) return ctx.fail(SAGE_ERR_INVALID, "internal: routine input not available");
         *out = jt->second;
         return SAGE_OK;
     }
     std::vector<Tensor> args(n.args.size());
     for (size_t i = 0; i < n.args.size(); ++i) {
-        sage_status st = run_node(n.args[i], ctx, s, temp, memo, &args[i]);
+        sage_status st = run_node(n.args[i], ctx, s, values, memo, &args[i]);
         if (st) return st;
     }
     if (n.shared) {
         auto it = memo.find(n.shared.get());
         if (it == memo.end()) {
             Tensor t;
-            sage_status st = run_node(*n.shared, ctx, s, temp, memo, &t);
+            sage_status st = run_node(*n.shared, ctx, s, values, memo, &t);
             if (st) return st;
             it = memo.emplace(n.shared.get(), t).first;
         }
@@ -761,10 +784,123 @@ static sage_status run_node(const Node &n, Context &ctx, Session &s, const std::
     return st;
 }
 
-// Program::exec, session.rs:208-468.
-static sage_status exec(Program &p, Context &ctx, Session &s) {
-    for (auto &kv : p.routines) kv.second.resolve_time();  // timers of an earlier run whose events have completed
+static void assign_slots(Node &n, const std::unordered_map<Origin *, int> &slot_of) {
+    if (n.is_data) {
+        auto it = slot_of.find(n.var.key());
+        if (n.var.is_op() && it != slot_of.end()) n.slot = it->second;
+        return;
+    }
+    if (n.shared) assign_slots(*n.shared, slot_of);
+    for (Node &a : n.args) assign_slots(a, slot_of);
+}
+
+// Turns the order of a run that needed no eviction into the program's schedule.
+static void make_schedule(Program &p, const std::vector<Routine *> &order) {
+    auto slot = [&](Origin *o) {
+        auto it = p.slot_of.emplace(o, (int)p.slot_of.size());
+        return it.first->second;
+    };
+    for (Routine *r : order) {
+        Program::Step step{r, {}, {}};
+        if (r->row)
+            for (const Var &v : r->row_outputs) step.outputs.push_back(slot(v.key()));
+        else
+            step.outputs.push_back(slot(r->output.key()));
+        p.schedule.push_back(std::move(step));
+    }
+    const int computed = (int)p.slot_of.size();
+    for (Routine *r : order)
+        for (const Var &v : r->inputs)
+            if (v.is_op()) {
+                const int n = slot(v.key());
+                if (n >= computed && (size_t)(n - computed) == p.given.size()) p.given.push_back({v.key(), n});
+            }
+    p.is_output.assign(p.slot_of.size(), 0);
+    for (const Var &v : p.outputs) {
+        auto it = p.slot_of.find(v.key());
+        if (it != p.slot_of.end()) p.is_output[it->second] = 1;
+    }
+    std::vector<int> last(p.slot_of.size(), -1);
+    for (size_t i = 0; i < order.size(); ++i) {
+        for (int o : p.schedule[i].outputs) last[o] = (int)i;  // a value nothing reads goes at once
+        for (const Var &v : order[i]->inputs)
+            if (v.is_op()) last[p.slot_of[v.key()]] = (int)i;
+    }
+    for (int n = 0; n < computed; ++n)
+        if (last[n] >= 0) p.schedule[last[n]].release.push_back(n);
+    for (Routine *r : order)
+        if (!r->row) assign_slots(r->root, p.slot_of);
+    p.slots.resize(p.slot_of.size());
+}
+
+static sage_status exec(Program &p, Context &ctx, Session &s, std::unordered_map<Origin *, Tensor> temp = {});
+
+// A run along the schedule.  Out of memory, it hands what it has computed to the general run, which evicts and recomputes.
+static sage_status exec_scheduled(Program &p, Context &ctx, Session &s) {
+    if (!p.times_read) {  // timers of the first run
+        p.times_read = true;
+        for (auto &kv : p.routines)
+            if (!kv.second.resolve_time()) p.times_read = false;
+    }
+    for (auto &g : p.given) {
+        auto it = s.data.find(g.first);
+        if (it == s.data.end()) return ctx.fail(SAGE_ERR_INVALID, "internal: an evaluated input is gone");
+        p.slots[g.second] = it->second.second;
+    }
+    struct Empty {  // nothing stays in the slots after a run, whichever way it ends
+        std::vector<Tensor> &slots;
+        ~Empty() {
+            for (Tensor &t : slots) t = Tensor();
+        }
+    };
     std::unordered_map<Origin *, Tensor> temp;
+    {
+        Empty empty{p.slots};
+        Values values;
+        values.slots = p.slots.data();
+        sage_status st = SAGE_OK;
+        for (Program::Step &step : p.schedule) {
+            Routine &f = *step.routine;
+            if (f.row) {
+                std::vector<Tensor> outs;
+                st = row_program_run(*f.row, ctx, [&](const Var &k, Tensor *t) {
+                    auto it = p.slot_of.find(k.key());
+                    if (it == p.slot_of.end()) return s.get(k, t);
+                    *t = p.slots[it->second];
+                    return true;
+                }, &outs, f.row_emit_shared.get());
+                if (st) break;
+                for (size_t i = 0; i < outs.size(); ++i) p.slots[step.outputs[i]] = std::move(outs[i]);
+            } else {
+                SharedMemo memo;
+                st = run_node(f.root, ctx, s, values, memo, &p.slots[step.outputs[0]]);
+                if (st) break;
+            }
+            for (size_t i = 0; i < step.outputs.size(); ++i)
+                if (p.is_output[step.outputs[i]]) {
+                    const Var &v = f.row ? f.row_outputs[i] : f.output;
+                    s.data[v.key()] = std::make_pair(v, p.slots[step.outputs[i]]);
+                }
+            for (int n : step.release) p.slots[n] = Tensor();
+        }
+        if (st != SAGE_ERR_OOM) return st;
+        for (Program::Step &step : p.schedule)
+            for (size_t i = 0; i < step.outputs.size(); ++i) {
+                const int n = step.outputs[i];
+                if (p.slots[n].defined() && !p.is_output[n]) temp[(step.routine->row ? step.routine->row_outputs[i] : step.routine->output).key()] = p.slots[n];
+            }
+    }
+    return exec(p, ctx, s, std::move(temp));
+}
+
+// Program::exec, session.rs:208-468.
+static sage_status exec(Program &p, Context &ctx, Session &s, std::unordered_map<Origin *, Tensor> temp) {
+    for (auto &kv : p.routines) kv.second.resolve_time();  // timers of an earlier run whose events have completed
+    const bool first = temp.empty() && p.schedule.empty();
+    bool evictions = false;
+    std::vector<Routine *> order;
+    Values values;
+    values.temp = &temp;
     std::unordered_map<Origin *, int> remaining = p.consumers;
     std::unordered_map<Origin *, int> lock;        // how many pending routines need each state
     std::unordered_set<Origin *> pending, outputs;
@@ -814,7 +950,7 @@ static sage_status exec(Program &p, Context &ctx, Session &s) {
                     return s.get(k, t);
                 }, &row_outs, f.row_emit_shared.get());
             } else {
-                st = run_node(f.root, ctx, s, temp, memo, &out);
+                st = run_node(f.root, ctx, s, values, memo, &out);
             }
             if (timer && st == SAGE_OK && cudaEventRecord(timer->ev[1], ctx.stream()) == cudaSuccess) {
                 f.timer = timer;
@@ -824,6 +960,7 @@ static sage_status exec(Program &p, Context &ctx, Session &s) {
             }
             if (st == SAGE_OK) break;
             if (st != SAGE_ERR_OOM) return st;
+            evictions = true;
             // Out of memory: drop the intermediates that are cheapest to recompute per byte
             // (session.rs:259-331); they are rebuilt on demand when a later routine needs them.
             const uint64_t needed = ctx.allocator().oom_needed, start = ctx.allocator().mem_used();
@@ -868,34 +1005,33 @@ static sage_status exec(Program &p, Context &ctx, Session &s) {
             auto it = remaining.find(k.key());
             if (it != remaining.end() && --it->second == 0) temp.erase(k.key());
         }
+        order.push_back(&f);
         stack.pop_back();
     }
+    if (first && !evictions) make_schedule(p, order);
     return SAGE_OK;
 }
 
-sage_status Session::eval(const std::vector<Var> &targets) {
+sage_status Session::eval(const std::vector<const Var *> &targets) {
     // Context::eval, context.rs:96-117: everything already evaluated is an input of the program.
-    std::vector<Var> y;
-    for (const Var &t : targets)
-        if (t.is_op() && !data.count(t.key())) y.push_back(t);
-    if (y.empty()) return SAGE_OK;
-    std::vector<Var> x;
-    {
-        std::unordered_set<Origin *> seen;
-        std::vector<Var> stack = y;
-        while (!stack.empty()) {
-            Var e = stack.back();
-            stack.pop_back();
-            if (!seen.insert(e.key()).second) continue;
-            if (data.count(e.key())) x.push_back(e);
-            else if (e.is_op())
-                for (const Var &c : children(e, ctx_->opts().pattern_fusion != 0, nullptr)) stack.push_back(c);
-        }
-    }
     std::vector<Origin *> tk, xk;
-    for (const Var &v : y) tk.push_back(v.key());
-    for (const Var &v : x) xk.push_back(v.key());
-    std::sort(xk.begin(), xk.end());
+    for (const Var *t : targets)
+        if (t->is_op() && !data.count(t->key())) tk.push_back(t->key());
+    if (tk.empty()) return SAGE_OK;
+    const bool fusion = ctx_->opts().pattern_fusion != 0;
+    if (!data.empty()) {  // nothing evaluated, nothing to look for
+        std::unordered_set<Origin *> seen;
+        std::vector<Origin *> stack = tk;
+        while (!stack.empty()) {
+            Origin *e = stack.back();
+            stack.pop_back();
+            if (!seen.insert(e).second) continue;
+            if (data.count(e)) xk.push_back(e);
+            else if (e->op)
+                for (const Var &c : fusion && e->composite ? e->composite->inputs : e->inputs) stack.push_back(c.key());
+        }
+        std::sort(xk.begin(), xk.end());
+    }
     Program *prog = nullptr;
     const uint64_t key_hash = program_key_hash(tk, xk);
     for (size_t i = cache_.size(); i-- > 0;) {
@@ -907,6 +1043,10 @@ sage_status Session::eval(const std::vector<Var> &targets) {
     }
     if (!prog) {
         std::unique_ptr<Program> p;
+        std::vector<Var> x, y;
+        for (Origin *o : xk) x.push_back(data[o].first);
+        for (const Var *t : targets)
+            if (t->is_op() && !data.count(t->key())) y.push_back(*t);
         try {
             // pattern_fusion bit 0: composites and whole-row programs; bit 2 keeps the row programs off
             // A lone softmax / log_sum_exp / layer_norm of evaluated data keeps its hand-written row kernel
@@ -944,7 +1084,7 @@ sage_status Session::eval(const std::vector<Var> &targets) {
     last_ = prog;
     try {
         if (prog->row) return row_program_exec(*prog->row, *ctx_, *this);
-        return exec(*prog, *ctx_, *this);
+        return prog->schedule.empty() ? exec(*prog, *ctx_, *this) : exec_scheduled(*prog, *ctx_, *this);
     } catch (const ShapeError &e) {
         return ctx_->fail(SAGE_ERR_INVALID, e.msg);
     }

@@ -29,9 +29,9 @@ struct Prepared {
 sage_status prepare(const std::vector<Var> &params, const std::vector<Var> &grads, Session &s, Prepared *out) {
     Context &C = s.ctx();
     if (params.size() != grads.size()) return C.fail(SAGE_ERR_INVALID, "optimizer update: one gradient per parameter is needed");
-    std::vector<Var> missing;
+    std::vector<const Var *> missing;
     for (const Var &g : grads)
-        if (g.is_op() && !s.data.count(g.key())) missing.push_back(g);
+        if (g.is_op() && !s.data.count(g.key())) missing.push_back(&g);
     if (!missing.empty()) {  // "it is inefficient to evaluate gradients in the inside of an optimizer" (optim.rs:56-59)
         sage_status st = s.eval(missing);
         if (st) return st;
