@@ -1,0 +1,667 @@
+// Host side of the half-precision-pieces GEMM (gemm_h2_device.inc) and the kernels that bring fp32 data into its operand
+// form.  Reference: Gemm::compute_direct / GemmBatched::compute_direct (src/ops/gemm.rs:176-250, 338-421).
+#include <cuda.h>
+#include <cuda_runtime.h>
+
+#include <cstdlib>
+
+#include "kernels.h"
+#include "launch.h"
+// the kernels compiled here store the plain fp32 product
+#define SAGE_EPI_OUT 1
+#define SAGE_EPI_COLS 0
+#include "gemm_tc_device.inc"
+#include "gemm_h2_device.inc"
+#include "gemm_tc_device_src.h"
+#include "gemm_h2_device_src.h"
+
+namespace sage {
+void *driver_symbol(const char *name);  // runtime/context.cc
+const char *map_prelude_text();         // codegen/map_emit.cc
+namespace k {
+
+using namespace sage_tc;
+
+namespace {
+
+bool aligned16(const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
+
+// ---------------------------------------------------------------------------------- operand forms
+// Flat: 16 lanes hold the 64 floats of a group.  Bound by memory: 4 bytes read, 4.06 written per element.
+__global__ void __launch_bounds__(256) split_h2_flat_kernel(const float4 *__restrict__ src, long long n4, uint2 *__restrict__ hi, uint2 *__restrict__ lo,
+                                                            float *__restrict__ scale) {
+    grid_dependency_sync();
+    for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < n4; g += (long long)gridDim.x * blockDim.x) {
+        const float4 x = src[g];  // n4 is a multiple of 16: the lanes of a group are all here or all gone
+        unsigned b = max(max(h2_finite_bits(x.x), h2_finite_bits(x.y)), max(h2_finite_bits(x.z), h2_finite_bits(x.w)));
+        const unsigned lanes = 0xffffu << (threadIdx.x & 16);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) b = max(b, __shfl_xor_sync(lanes, b, o));
+        float s;
+        const float f = h2_factor(b, &s);
+        uint2 h, l;
+        h2_split2(x.x, x.y, f, &h.x, &l.x);
+        h2_split2(x.z, x.w, f, &h.y, &l.y);
+        hi[g] = h;
+        lo[g] = l;
+        if ((threadIdx.x & 15) == 0) scale[g >> 4] = s;
+    }
+}
+
+struct ViewP {
+    const float *src;
+    long long nb0, sb0, sb1, ld, cs;  // row and column strides of the source
+    long long rows, cols, pitch, plane;
+    int row_tiles, col_tiles;
+    int vec;  // whole 16-byte loads along the contiguous axis are aligned and inside
+};
+
+// A 64 x 64 tile of the view into shared memory, read along whichever axis is contiguous (256 threads).
+__device__ __forceinline__ void load_tile(const ViewP &v, const float *s, long long r0, long long c0, float (*tile)[65]) {
+    const int t = threadIdx.x, fast = t & 63, slow = t >> 6;  // 4 lines of 64 at a time
+    float x[16];
+    if (v.vec && v.cs != 1) {
+        const int r4 = (t & 15) * 4, line = t >> 4;
+        float4 q[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const long long r = r0 + r4, c = c0 + line + 16 * i;
+            q[i] = r < v.rows && c < v.cols ? *reinterpret_cast<const float4 *>(s + r + c * v.cs) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int c = line + 16 * i;
+            tile[r4][c] = q[i].x;
+            tile[r4 + 1][c] = q[i].y;
+            tile[r4 + 2][c] = q[i].z;
+            tile[r4 + 3][c] = q[i].w;
+        }
+    } else if (v.cs == 1 || v.ld != 1) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const long long r = r0 + slow + 4 * i, c = c0 + fast;
+            x[i] = r < v.rows && c < v.cols ? s[r * v.ld + c * v.cs] : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) tile[slow + 4 * i][fast] = x[i];
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const long long r = r0 + fast, c = c0 + slow + 4 * i;
+            x[i] = r < v.rows && c < v.cols ? s[r + c * v.cs] : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) tile[fast][slow + 4 * i] = x[i];
+    }
+}
+// A row of the tile per 4 lanes, columns 8 * part .. and 32 + 8 * part .. each: no bank conflicts, and the four lanes' 16-byte
+// stores lie side by side
+__device__ __forceinline__ void tile_row(const float (*tile)[65], float (&y)[16]) {
+    const float *t = tile[threadIdx.x >> 2] + (threadIdx.x & 3) * 8;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) y[i] = t[(i & 7) + (i & 8) * 4];
+}
+// This thread's 16 values of the tile at (r0, c0): straight from memory where the columns are contiguous and aligned,
+// else turned round in shared memory (a barrier inside: all threads call it).
+__device__ __forceinline__ void fetch_row(const ViewP &v, const float *s, long long r0, long long c0, float (*tile)[65], float (&y)[16]) {
+    if (v.vec && v.cs == 1) {
+        const long long r = r0 + (threadIdx.x >> 2), c = c0 + (threadIdx.x & 3) * 8;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const long long cc = c + (i & 1) * 4 + (i >> 1) * 32;
+            const float4 q = r < v.rows && cc < v.cols ? *reinterpret_cast<const float4 *>(s + r * v.ld + cc) : make_float4(0.f, 0.f, 0.f, 0.f);
+            y[4 * i] = q.x;
+            y[4 * i + 1] = q.y;
+            y[4 * i + 2] = q.z;
+            y[4 * i + 3] = q.w;
+        }
+        return;
+    }
+    load_tile(v, s, r0, c0, tile);
+    __syncthreads();
+    tile_row(tile, y);
+}
+__device__ __forceinline__ unsigned row_amax(const float (&y)[16]) {
+    unsigned m = 0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) m = max(m, h2_finite_bits(y[i]));
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+    return max(m, __shfl_xor_sync(0xffffffffu, m, 2));
+}
+__device__ __forceinline__ void store_row(const ViewP &v, long long b, long long r0, long long c0, const float (&y)[16], float factor, unsigned short *hi) {
+    const long long r = r0 + (threadIdx.x >> 2), c = c0 + (threadIdx.x & 3) * 8;
+    if (r >= v.rows) return;
+    unsigned h[8], l[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) h2_split2(y[2 * i], y[2 * i + 1], factor, &h[i], &l[i]);
+    unsigned short *d = hi + (b * v.rows + r) * v.pitch + c;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {  // pitch is a multiple of 8: whole 16-byte pieces, zeros behind the last column
+        if (c + 32 * i >= v.pitch) break;
+        *reinterpret_cast<uint4 *>(d + 32 * i) = make_uint4(h[4 * i], h[4 * i + 1], h[4 * i + 2], h[4 * i + 3]);
+        *reinterpret_cast<uint4 *>(d + v.plane + 32 * i) = make_uint4(l[4 * i], l[4 * i + 1], l[4 * i + 2], l[4 * i + 3]);
+    }
+}
+
+// Operand A: a scale per row and 64 columns.  One block per tile.
+__global__ void __launch_bounds__(256) split_h2_view_kernel(ViewP v, unsigned short *__restrict__ hi, float *__restrict__ scale) {
+    __shared__ float tile[64][65];
+    grid_dependency_sync();
+    const int per = v.row_tiles * v.col_tiles, rem = (int)(blockIdx.x % per);
+    const long long b = blockIdx.x / per, r0 = (long long)(rem / v.col_tiles) * 64, c0 = (long long)(rem % v.col_tiles) * 64;
+    float y[16], s;
+    fetch_row(v, v.src + (b / v.nb0) * v.sb1 + (b % v.nb0) * v.sb0, r0, c0, tile, y);
+    const float f = h2_factor(row_amax(y), &s);
+    const long long r = r0 + (threadIdx.x >> 2);
+    if ((threadIdx.x & 3) == 0 && r < v.rows) scale[(b * v.rows + r) * v.col_tiles + (c0 >> 6)] = s;
+    store_row(v, b, r0, c0, y, f, hi);
+}
+
+// Operand B: one scale per row.  A cluster of CTAs shares 64 rows, each with a run of their columns; the rows' largest
+// magnitudes are exchanged through distributed shared memory, then the columns are read again, from L2.  Keeping the tiles
+// in shared memory between the two looks (one read, 133 KB a CTA) left one block per SM and was slower: 4096 x 4096 80 us.
+__global__ void __launch_bounds__(256) split_h2_rows_kernel(ViewP v, unsigned short *__restrict__ hi, float *__restrict__ scale, int ctas, int tiles_per_cta) {
+    __shared__ float tiles[2][64][65];
+    __shared__ unsigned amax[64];
+    grid_dependency_sync();
+    const unsigned rank = blockIdx.x % ctas;
+    const long long group = blockIdx.x / ctas, b = group / v.row_tiles, r0 = (group % v.row_tiles) * 64;
+    const float *s = v.src + (b / v.nb0) * v.sb1 + (b % v.nb0) * v.sb0;
+    const int first = (int)rank * tiles_per_cta, last = min(v.col_tiles, first + tiles_per_cta);
+    unsigned m = 0;
+    float y[16];
+    for (int t = first; t < last; ++t) {
+        fetch_row(v, s, r0, (long long)t * 64, tiles[t & 1], y);
+        m = max(m, row_amax(y));
+    }
+    if ((threadIdx.x & 3) == 0) amax[threadIdx.x >> 2] = m;
+    __syncthreads();
+    if (ctas > 1) {
+        cluster_sync_all();
+        const unsigned at = smem_u32(&amax[threadIdx.x >> 2]);
+        for (int q = 0; q < ctas; ++q) {
+            unsigned o;
+            asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(o) : "r"(peer_addr(at, q)) : "memory");
+            m = max(m, o);
+        }
+        cluster_sync_all();  // nobody leaves while a peer may still read its shared memory
+    }
+    float sc;
+    const float f = h2_factor(m, &sc);
+    if (rank == 0 && (threadIdx.x & 3) == 0 && r0 + (threadIdx.x >> 2) < v.rows) scale[b * v.rows + r0 + (threadIdx.x >> 2)] = sc;
+    for (int t = last - 1; t >= first; --t) {  // backwards: the last tile is still in registers
+        if (t != last - 1) fetch_row(v, s, r0, (long long)t * 64, tiles[t & 1], y);
+        store_row(v, b, r0, (long long)t * 64, y, f, hi);
+    }
+}
+
+}  // namespace
+
+sage_status split_h2_flat(Context &ctx, const float *src, long long n, unsigned short *hi, long long plane, float *scale) {
+    ctx.note_launch("split_tf32");  // launch lists have one name for an operand's split
+    if (ctx.dry()) return SAGE_OK;
+    if (!aligned16(src) || !aligned16(hi) || plane % 8 || n % 64) return ctx.fail(SAGE_ERR_INVALID, "split_h2_flat: unaligned");
+    long long blocks = (n / 4 + 255) / 256;
+    const long long cap = (long long)ctx.sm_count * 16;
+    if (blocks > cap) blocks = cap;
+    return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), split_h2_flat_kernel, dim3((unsigned)(blocks < 1 ? 1 : blocks)), dim3(256), 0,
+                                           reinterpret_cast<const float4 *>(src), n / 4, reinterpret_cast<uint2 *>(hi), reinterpret_cast<uint2 *>(hi + plane), scale),
+                          "split_h2_flat launch");
+}
+
+static long long h2_pitch(long long cols) { return (cols + 7) / 8 * 8; }
+static size_t up256(size_t b) { return (b + 255) / 256 * 256; }
+
+// [hi][lo][scales]
+size_t split_h2_bytes(long long batches, long long rows, long long cols, bool whole_rows) {
+    const size_t planes = (size_t)(batches * rows * h2_pitch(cols)) * 2 * 2;
+    return up256(planes) + up256((size_t)(batches * rows * (whole_rows ? 1 : (cols + 63) / 64)) * 4);
+}
+
+sage_status split_h2_view_into(Context &ctx, const float *src, const SplitView &v, bool whole_rows, void *dst, H2Split *out) {
+    const long long batches = v.nb0 * v.nb1;
+    out->pitch = h2_pitch(v.cols);
+    out->plane = batches * v.rows * out->pitch;
+    out->hi = static_cast<unsigned short *>(dst);
+    out->scale = reinterpret_cast<float *>(static_cast<char *>(dst) + up256((size_t)out->plane * 4));
+    ViewP p{src, v.nb0, v.sb0, v.sb1, v.ld, v.col_stride, v.rows, v.cols, out->pitch, out->plane, (int)((v.rows + 63) / 64), (int)((v.cols + 63) / 64), 0};
+    p.vec = (v.col_stride == 1 || v.ld == 1) && aligned16(src) && v.sb0 % 4 == 0 && v.sb1 % 4 == 0 && (v.col_stride == 1 ? v.ld % 4 == 0 && v.cols % 4 == 0 : v.col_stride % 4 == 0 && v.rows % 4 == 0);
+    const long long groups = batches * p.row_tiles, blocks = groups * (whole_rows ? 8 : p.col_tiles);
+    if (blocks > 0x7fffffffLL) return ctx.fail(SAGE_ERR_UNSUPPORTED, "split_h2: extents beyond 2^31 tiles");
+    ctx.note_launch("split_tf32");  // launch lists have one name for an operand's split
+    if (ctx.dry()) return SAGE_OK;
+    if (!whole_rows)
+        return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), split_h2_view_kernel, dim3((unsigned)blocks), dim3(256), 0, p, out->hi, out->scale), "split_h2 launch");
+    int ctas = 1;
+    while (ctas < 8 && ctas * 2 <= p.col_tiles) ctas *= 2;
+    const int per = (p.col_tiles + ctas - 1) / ctas;
+    return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), ctas, split_h2_rows_kernel, dim3((unsigned)(groups * ctas)), dim3(256), 0, p, out->hi, out->scale, ctas, per),
+                          "split_h2 rows launch");
+}
+
+sage_status split_h2_view(Context &ctx, const float *src, const SplitView &v, bool whole_rows, H2Split *out) {
+    out->block = ctx.allocator().alloc(split_h2_bytes(v.nb0 * v.nb1, v.rows, v.cols, whole_rows));
+    if (!out->block) return ctx.fail(SAGE_ERR_OOM, "out of memory for an operand in half-precision pieces");
+    return split_h2_view_into(ctx, src, v, whole_rows, out->block->ptr, out);
+}
+
+H2Operand h2_operand(const H2Split &s, long long batches, long long rows, long long cols, bool whole_rows) {
+    H2Operand o;
+    o.hi = s.hi;
+    o.plane = s.plane;
+    o.ld = s.pitch;
+    o.rows = rows;
+    o.nb0 = batches;
+    o.sb0 = rows * s.pitch;
+    o.scale = s.scale;
+    o.s_row = whole_rows ? 1 : (cols + 63) / 64;
+    o.s_b0 = rows * o.s_row;
+    return o;
+}
+
+// ---------------------------------------------------------------------------------- launcher
+typedef CUresult (*PFN_encodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                    const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                    CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+typedef CUresult (*PFN_encodeIm2col)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                     const int *, const int *, cuuint32_t, cuuint32_t, const cuuint32_t *, CUtensorMapInterleave,
+                                     CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// dims {k, rows, batch low, batch high, piece}, box {64, box_rows, 1, 1, 1}
+static bool encode_operand(PFN_encodeTiled encode, const H2Operand &op, long long k, unsigned box_rows, CUtensorMap *map) {
+    const cuuint64_t row_b = (cuuint64_t)op.ld * 2;
+    const cuuint64_t dims[5] = {(cuuint64_t)k, (cuuint64_t)op.rows, (cuuint64_t)op.nb0, (cuuint64_t)op.nb1, 2};
+    const cuuint64_t strides[4] = {row_b, op.nb0 > 1 ? (cuuint64_t)op.sb0 * 2 : row_b, op.nb1 > 1 ? (cuuint64_t)op.sb1 * 2 : row_b, (cuuint64_t)op.plane * 2};
+    const cuuint32_t box[5] = {(cuuint32_t)HK, box_rows, 1, 1, 1}, estr[5] = {1, 1, 1, 1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, const_cast<unsigned short *>(op.hi), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// One piece of an NHWC image: im2col mode, 64 channels of 128 output pixels.
+static bool encode_im2col(PFN_encodeIm2col encode, const H2Gemm &g, const unsigned short *base, CUtensorMap *map) {
+    const cuuint64_t dims[4] = {(cuuint64_t)g.img_c, (cuuint64_t)g.img_w, (cuuint64_t)g.img_h, (cuuint64_t)g.img_n};
+    const cuuint64_t strides[3] = {(cuuint64_t)g.img_c * 2, (cuuint64_t)(g.img_w * g.img_c) * 2, (cuuint64_t)(g.img_h * g.img_w * g.img_c) * 2};
+    const Window &w = g.win;
+    const int lower[2] = {-w.pad_w, -w.pad_h};
+    const int upper[2] = {w.pad_w - (w.ker_w - 1) * w.dil_w, w.pad_h - (w.ker_h - 1) * w.dil_h};
+    const cuuint32_t estr[4] = {1, (cuuint32_t)w.stride_w, (cuuint32_t)w.stride_h, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<unsigned short *>(base), dims, strides, lower, upper, (cuuint32_t)HK, (cuuint32_t)BM, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// ... and tiled, a window of box_w x box_h pixels, for tap reuse
+static bool encode_halo(PFN_encodeTiled encode, const H2Gemm &g, const unsigned short *base, unsigned box_w, unsigned box_h, CUtensorMap *map) {
+    const cuuint64_t dims[4] = {(cuuint64_t)g.img_c, (cuuint64_t)g.img_w, (cuuint64_t)g.img_h, (cuuint64_t)g.img_n};
+    const cuuint64_t strides[3] = {(cuuint64_t)g.img_c * 2, (cuuint64_t)(g.img_w * g.img_c) * 2, (cuuint64_t)(g.img_h * g.img_w * g.img_c) * 2};
+    const cuuint32_t box[4] = {(cuuint32_t)HK, box_w, box_h, 1u}, estr[4] = {1, 1, 1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<unsigned short *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// The limits of im2col-mode tensor maps (as for the tf32 kernel), channels in whole groups.
+bool conv_h2_ok(const H2Gemm &g) {
+    const Window &w = g.win;
+    if (g.img_c < 64 || g.img_c % 64 || g.img_n < 1 || g.img_h < 1 || g.img_w < 1 || g.out_h < 1 || g.out_w < 1 || g.out_h * g.out_w > 0x7fffffffLL) return false;
+    if (w.stride_w < 1 || w.stride_w > 8 || w.stride_h < 1 || w.stride_h > 8) return false;
+    if (w.pad_w < 0 || w.pad_w > 127 || w.pad_h < 0 || w.pad_h > 127 || w.dil_w < 0 || w.dil_h < 0) return false;
+    if (w.pad_w - (w.ker_w - 1) * w.dil_w < -128 || w.pad_h - (w.ker_h - 1) * w.dil_h < -128) return false;
+    return (w.ker_w - 1) * w.dil_w <= 255 && (w.ker_h - 1) * w.dil_h <= 255 && g.img_n * g.img_h * g.img_w <= 0x7fffffffLL;
+}
+
+// Tap reuse: the rule of conv_halo_plan in gemm_tcgen05.cu (SAGE_CONV_HALO=0 turns it off, read per launch).
+static bool halo_plan(const H2Gemm &g, int *wb, int *rows) {
+    const char *env = getenv("SAGE_CONV_HALO");
+    const Window &w = g.win;
+    if ((env && atoi(env) == 0) || !g.conv || w.stride_w != 1 || w.stride_h != 1 || w.dil_w != 1 || w.dil_h != 1) return false;
+    if (w.ker_w * w.ker_h < 2 || g.n > 128 || g.n % 32) return false;
+    const long long b = g.out_w + w.ker_w - 1;
+    if (b > 128) return false;
+    long long r = 128 / b;
+    if (r > g.out_h) r = g.out_h;
+    if (r * g.out_w < 100 || b * (r + w.ker_h - 1) > 256 || 127 + (w.ker_h - 1) * b + (w.ker_w - 1) > 255) return false;
+    if (g.img_n * ((g.out_h + r - 1) / r) > 0x3fffffffLL) return false;
+    *wb = (int)b;
+    *rows = (int)r;
+    return true;
+}
+
+static bool pairs_on() {
+    static const bool on = !(getenv("SAGE_GEMM_PAIR") && atoi(getenv("SAGE_GEMM_PAIR")) == 0);
+    return on;
+}
+
+// How the columns are cut: tiles of `bn` columns, the last `narrow` of a row block 192 wide instead (only with bn = 256;
+// wide = 0: all of them).  The busiest CTA (pair) decides: a tile costs its width plus a fixed 24 columns' worth.
+struct ColumnPlan {
+    int bn, wide, narrow;
+};
+static ColumnPlan plan_columns(const Context &ctx, long long m, long long n, long long batch, int ctas) {
+    const long long slots = ctx.sm_count / ctas, row_tiles = (m + BM * ctas - 1) / (BM * ctas) * batch;
+    ColumnPlan best{128, 0, 0};
+    double best_cost = 1e300;
+    auto consider = [&](int bn, long long wide, long long narrow) {
+        const long long tw = row_tiles * wide, total = tw + row_tiles * narrow;
+        if (total > 0x7fffffffLL) return;
+        double worst = 0;
+        for (long long i = 0; i < slots && i < total; ++i) {  // pair i gets tiles i, i + slots, ..., the wide ones first
+            const long long mine = (total - i + slots - 1) / slots, mine_wide = i < tw ? (tw - i + slots - 1) / slots : 0;
+            const double load = (double)mine_wide * (bn + 24) + (double)(mine - mine_wide) * (192 + 24);
+            if (load > worst) worst = load;
+        }
+        if (worst < best_cost * (narrow ? 0.98 : 1.0)) {
+            best_cost = worst;
+            best = ColumnPlan{bn, (int)wide, (int)narrow};
+        }
+    };
+    for (int bn : {256, 128, 64})
+        if (bn == 64 || n > bn / 2) consider(bn, (n + bn - 1) / bn, 0);
+    for (long long nn = 1; nn * 192 <= n + 191 && n > 128; ++nn) {
+        const long long rest = n - nn * 192, nw = rest > 0 ? (rest + 255) / 256 : 0;
+        if (nw * 256 + nn * 192 - n < 192) consider(256, nw, nn);
+    }
+    return best;
+}
+
+static sage_status gemm_h2_launch(Context &ctx, const H2Gemm &g);
+
+// Split-K: as in gemm_tcgen05.cu, a product with few output tiles and a long K runs as a batch of K slices (multiples of
+// 64) followed by their sum in a fixed order.  Microseconds from measured launches: a K-block takes what its operand
+// bytes take from L2 (64 KB: 1.1 us with all SMs loading), a tile ~5 us beside its K loop, the sum 4 us and its bytes.
+static int pick_slices(const Context &ctx, const H2Gemm &g) {
+    static const bool enabled = !(getenv("SAGE_GEMM_SPLITK") && atoi(getenv("SAGE_GEMM_SPLITK")) == 0);
+    if (!enabled || g.conv || g.batch != 1 || g.naux || !g.epilogue.empty() || !g.c || g.c_hi || g.h_hi || g.ldc != g.n || g.k < 512) return 0;
+    const int ctas = (pairs_on() && g.m > BM) ? 2 : 1;
+    const long long units = ctx.sm_count / ctas;
+    double best = 1e300, unsplit = 1e300;
+    long long best_s = 0;
+    for (long long s = 1; s <= g.k / 256 && s <= 64; ++s) {
+        if (s > 1 && g.k % (64 * s)) continue;
+        const long long kb = (g.k / s + HK - 1) / HK;
+        for (int bn : {256, 128, 64}) {
+            if (bn > 64 && g.n <= bn / 2) continue;
+            const long long tiles = ((g.m + BM * ctas - 1) / (BM * ctas)) * ((g.n + bn - 1) / bn) * s, waves = (tiles + units - 1) / units;
+            double t = (double)waves * ((double)kb * 1.1 * (BM + bn / ctas) / 256.0 + 5.0);
+            if (s > 1) t += 4.0 + (double)(s + 1) * (double)g.m * (double)g.n * 4.0 / 5.0e6;
+            if (s == 1 && t < unsplit) unsplit = t;
+            if (t < best) {
+                best = t;
+                best_s = s;
+            }
+        }
+    }
+    return best_s >= 2 && best <= 0.9 * unsplit ? (int)best_s : 0;
+}
+
+int gemm_h2_slices(Context &ctx, const H2Gemm &g) { return pick_slices(ctx, g); }
+
+sage_status gemm_h2_run(Context &ctx, const H2Gemm &g0, bool no_slices) {
+    const int S = no_slices ? 0 : pick_slices(ctx, g0);
+    if (S < 2) return gemm_h2_launch(ctx, g0);
+    const long long ks = g0.k / S, mn = g0.m * g0.n;
+    Block *scratch = ctx.allocator().alloc((size_t)S * mn * sizeof(float));
+    if (!scratch) return gemm_h2_launch(ctx, g0);  // no room for the partial products: one pass over K
+    H2Gemm g = g0;
+    g.batch = S;
+    g.k = ks;
+    for (H2Operand *o : {&g.a, &g.b}) {
+        o->nb0 = S;
+        o->sb0 = ks;
+        o->nb1 = 1;
+        o->sb1 = 0;
+        o->bcast = false;
+    }
+    g.a.s_b0 = ks / HK;
+    g.b.s_b0 = 0;  // B's scales hold for all of K
+    g.c = reinterpret_cast<float *>(scratch->ptr);
+    g.sc0 = mn;
+    g.sc1 = 0;
+    g.nbc0 = S;
+    sage_status st = gemm_h2_launch(ctx, g);
+    if (!st) {
+        Dims outer, inner;
+        outer.ndim = 1;
+        outer.ext[0] = mn;
+        outer.str[0] = 1;
+        inner.ndim = 1;
+        inner.ext[0] = S;
+        inner.str[0] = mn;
+        st = reduce(ctx, SAGE_F32, 0 /* sum */, g.c, outer, inner, g0.c);
+    }
+    ctx.allocator().free(scratch);  // stream-ordered
+    return st;
+}
+
+// op(A) op(B) of plain fp32 operands: both brought into pieces, K contiguous.  `scratch`: where the pieces go (of
+// gemm_h2_scratch_bytes), or null to take them from the allocator.
+static SplitView operand_view(const float *, long long rows, long long cols, bool k_contiguous, long long ld, long long batch_stride, long long batch) {
+    SplitView v;
+    v.nb0 = batch;
+    v.sb0 = batch_stride;
+    v.rows = rows;
+    v.cols = cols;
+    v.ld = k_contiguous ? ld : 1;
+    v.col_stride = k_contiguous ? 1 : ld;
+    return v;
+}
+size_t gemm_h2_scratch_bytes(const GemmArgs &g) { return split_h2_bytes(g.batch, g.m, g.k, false) + split_h2_bytes(g.batch, g.n, g.k, true); }
+
+sage_status gemm_h2(Context &ctx, const GemmArgs &a, void *scratch) {
+    const SplitView va = operand_view(a.a, a.m, a.k, !a.ta, a.lda, a.stride_a, a.batch), vb = operand_view(a.b, a.n, a.k, a.tb, a.ldb, a.stride_b, a.batch);
+    Block *block = nullptr;
+    if (!scratch) {
+        block = ctx.allocator().alloc(gemm_h2_scratch_bytes(a));
+        if (!block) return ctx.fail(SAGE_ERR_OOM, "out of memory for the operands in half-precision pieces");
+        scratch = block->ptr;
+    }
+    H2Split pa, pb;
+    sage_status st = split_h2_view_into(ctx, a.a, va, false, scratch, &pa);
+    if (!st) st = split_h2_view_into(ctx, a.b, vb, true, static_cast<char *>(scratch) + split_h2_bytes(a.batch, a.m, a.k, false), &pb);
+    if (!st) {
+        H2Gemm g;
+        g.m = a.m;
+        g.n = a.n;
+        g.k = a.k;
+        g.batch = a.batch;
+        g.a = h2_operand(pa, a.batch, a.m, a.k, false);
+        g.b = h2_operand(pb, a.batch, a.n, a.k, true);
+        g.c = a.c;
+        g.ldc = a.ldc;
+        g.sc0 = a.stride_c;
+        g.nbc0 = a.batch;
+        st = gemm_h2_run(ctx, g, block == nullptr);
+    }
+    if (block) ctx.allocator().free(block);  // stream-ordered: later launches on this stream may reuse it
+    return st;
+}
+
+// The plain product (no epilogue, fp32 result): compiled with the library, so that an entry point which must not load a
+// module at run time can use it.
+template <int BN, int CTAS>
+__global__ void __launch_bounds__(kThreads, 1) gemm_h2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                                                              const __grid_constant__ CUtensorMap map_b2, const __grid_constant__ H2Params p) {
+    gemm_h2_body<BN, CTAS>(&map_a, &map_a, &map_b, &map_b2, p);
+}
+template <int BN, int CTAS>
+static sage_status launch_plain(Context &ctx, const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorMap &map_b2, const H2Params &p, int grid, size_t smem) {
+    static int attr_set[64] = {0};  // per instantiation and device
+    const int dev = ctx.device();
+    if (dev < 0 || dev >= 64 || attr_set[dev] != (int)smem) {
+        sage_status st = ctx.check_cuda(cudaFuncSetAttribute(gemm_h2_kernel<BN, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "gemm_h2 shared memory attribute");
+        if (st) return st;
+        if (dev >= 0 && dev < 64) attr_set[dev] = (int)smem;
+    }
+    return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), CTAS, gemm_h2_kernel<BN, CTAS>, dim3(grid), dim3(kThreads), smem, map_a, map_b, map_b2, p), "gemm_h2 launch");
+}
+
+static sage_status gemm_h2_launch(Context &ctx, const H2Gemm &g) {
+    static PFN_encodeTiled encode = nullptr;
+    static PFN_encodeIm2col encode_conv = nullptr;
+    if (!ctx.dry() && !encode) {
+        encode_conv = reinterpret_cast<PFN_encodeIm2col>(driver_symbol("cuTensorMapEncodeIm2col"));
+        encode = reinterpret_cast<PFN_encodeTiled>(driver_symbol("cuTensorMapEncodeTiled"));
+        if (!encode || !encode_conv) return ctx.fail(SAGE_ERR_DEVICE, "cuTensorMapEncode is not available");
+    }
+    if (g.m < 1 || g.n < 1 || g.k < 1 || g.batch < 1 || g.m > 0x7fffffffLL || g.n > 0x7fffffffLL || g.k > 0x7fffffffLL || g.batch > 0x7fffffffLL)
+        return ctx.fail(SAGE_ERR_UNSUPPORTED, "gemm_h2: shape not supported");
+    if (g.naux < 0 || g.naux > kMaxAux || (!g.c && !g.c_hi && !g.h_hi)) return ctx.fail(SAGE_ERR_INVALID, "gemm_h2: bad epilogue description");
+    if (g.conv && (g.batch != 1 || !conv_h2_ok(g) || g.m != g.img_n * g.out_h * g.out_w || g.k != (long long)g.win.ker_h * g.win.ker_w * g.img_c))
+        return ctx.fail(SAGE_ERR_INVALID, "gemm_h2: convolution description does not match the GEMM");
+    const int ctas = (pairs_on() && g.m > BM) ? 2 : 1;
+    int halo_wb = 0, halo_r = 0;
+    const bool halo = halo_plan(g, &halo_wb, &halo_r);
+    ColumnPlan cols = plan_columns(ctx, g.m, g.n, g.batch, ctas);
+    if (halo) cols = ColumnPlan{g.n <= 64 ? 64 : 128, 0, 0};  // all output channels in one tile: the window is loaded once
+    const int bn = cols.bn;
+    const int stage_bytes = halo ? 2 * (bn / ctas) * HK * 2 : 2 * BM * HK * 2 + 2 * (bn / ctas) * HK * 2;
+    const int staging = kEpiWarps * kStageBytesPerWarp, fixed = halo ? kHaloStages * kHaloStageBytes : 0;
+    int stages = (227 * 1024 - 2048 - staging - fixed) / stage_bytes;
+    if (stages > 8) stages = 8;
+    const size_t smem = (size_t)fixed + (size_t)stages * stage_bytes + staging + 1024;
+
+    H2Params p{};
+    p.c = g.c;
+    p.c_hi = g.c_hi;
+    p.c_plane = g.c_plane;
+    p.h_hi = g.h_hi;
+    p.h_plane = g.h_plane;
+    p.h_scale = g.h_scale;
+    p.ldc = g.ldc;
+    p.sc0 = g.sc0;
+    p.sc1 = g.sc1;
+    p.nbc0 = (int)(g.nbc0 < 1 ? 1 : g.nbc0);
+    p.na0 = (int)g.a.nb0;
+    p.nb0 = (int)g.b.nb0;
+    p.a_bcast = (g.a.bcast || g.conv) ? 1 : 0;
+    p.b_bcast = g.b.bcast ? 1 : 0;
+    p.m = (int)g.m;
+    p.n = (int)g.n;
+    p.k = (int)g.k;
+    p.stages = stages;
+    p.tiles_m = (int)((g.m + BM * ctas - 1) / (BM * ctas));
+    p.tiles_n = (cols.wide || cols.narrow) ? cols.wide + cols.narrow : (int)((g.n + bn - 1) / bn);
+    p.rag_wide = cols.wide;
+    p.rag_narrow = cols.narrow;
+    p.rag_bn = 192;
+    p.num_tiles = (int)((long long)p.tiles_m * p.tiles_n * g.batch);
+    p.sa = g.a.scale;
+    p.sa_row = g.a.s_row;
+    p.sa_b0 = g.a.s_b0;
+    p.sa_b1 = g.a.s_b1;
+    p.sb = g.b.scale;
+    p.sb_batch = g.b.bcast ? 0 : g.b.s_b0;
+    p.status = ctx.status_word_dev;
+    if (g.conv) {
+        p.conv_cb = (int)(g.img_c / HK);
+        p.conv_kw = g.win.ker_w;
+        p.conv_q = (int)g.out_w;
+        p.conv_pq = (int)(g.out_h * g.out_w);
+        p.conv_sw = g.win.stride_w;
+        p.conv_sh = g.win.stride_h;
+        p.conv_pw = g.win.pad_w;
+        p.conv_ph = g.win.pad_h;
+        p.conv_dw = g.win.dil_w;
+        p.conv_dh = g.win.dil_h;
+        p.conv_h = (int)g.img_h;
+        p.conv_w = (int)g.img_w;
+        p.conv_n = (int)g.img_n;
+        p.conv_p = (int)g.out_h;
+    }
+    if (halo) {
+        p.halo_wb = halo_wb;
+        p.halo_r = halo_r;
+        p.halo_rt = (int)((g.out_h + halo_r - 1) / halo_r);
+        p.halo_taps = g.win.ker_h * g.win.ker_w;
+        p.halo_box_bytes = 128 * halo_wb * (halo_r + g.win.ker_h - 1);
+        p.tiles_m = (int)((g.img_n * p.halo_rt + ctas - 1) / ctas);
+        p.num_tiles = p.tiles_m * p.tiles_n;
+    }
+    bool vec = g.n % 4 == 0 && g.ldc % 4 == 0 && g.sc0 % 4 == 0 && g.sc1 % 4 == 0 && (!g.c || aligned16(g.c)) && (!g.c_hi || (aligned16(g.c_hi) && g.c_plane % 4 == 0));
+    int rowinv = 0, per_col = 0;
+    for (int i = 0; i < g.naux; ++i) {
+        TcAux &a = p.aux[i];
+        a.ptr = g.aux[i].ptr;
+        a.s0 = g.aux[i].s0;
+        a.s1 = g.aux[i].s1;
+        a.sr = g.aux[i].sr;
+        a.sc = g.aux[i].sc;
+        if (a.sc != 0 && a.sc != 1) return ctx.fail(SAGE_ERR_INVALID, "gemm_h2: epilogue operand column stride must be 0 or 1");
+        if (a.sc == 1) vec = vec && aligned16(a.ptr) && a.s0 % 4 == 0 && a.s1 % 4 == 0 && a.sr % 4 == 0;
+        if (a.sr == 0) rowinv |= 1 << i;
+        if (a.sc != 0) per_col |= 1 << i;
+    }
+    p.vec_ok = vec ? 1 : 0;
+    if (g.h_hi && (!vec || g.n % 64 || g.ldc % 64 || g.sc0 % 64 || g.sc1 % 64 || !aligned16(g.h_hi) || g.h_plane % 8))
+        return ctx.fail(SAGE_ERR_INVALID, "gemm_h2: a result in half-precision pieces needs whole groups of 64 columns");
+    const int slots = ctx.sm_count / ctas, grid = ctas * (p.num_tiles < slots ? p.num_tiles : slots);
+
+    const int out_mask = (g.c ? 1 : 0) | (g.c_hi ? 2 : 0) | (g.h_hi ? 4 : 0);
+    char num[96];
+    snprintf(num, sizeof num, "gemm_h2 %d %d %d %d %d %d %d\n", bn, ctas, g.conv ? (halo ? 2 : 1) : 0, g.naux, rowinv, per_col, out_mask);
+    const bool plain = !g.conv && g.naux == 0 && g.epilogue.empty() && out_mask == 1;
+    const std::string key = num + g.epilogue;
+    Module *mod = plain ? nullptr : ctx.module_find(key);
+    if (!plain && !mod) {
+        std::string src = map_prelude_text();
+        src += "struct __align__(64) CUtensorMap { unsigned long long opaque[16]; };\n";
+        auto define = [&](const char *name, int v) { src += std::string("#define ") + name + " " + std::to_string(v) + "\n"; };
+        define("SAGE_EPI_ROWINV", rowinv);
+        define("SAGE_EPI_COLS", per_col);
+        define("SAGE_EPI_OUT", out_mask);
+        define("SAGE_EPI_NAUX", g.naux);
+        define("SAGE_H2_CONV", g.conv ? 1 : 0);
+        define("SAGE_H2_HALO", halo ? 1 : 0);
+        src += "#define SAGE_EPI_EXPR(x0, x1, x2, x3) (" + (g.epilogue.empty() ? std::string("x0") : g.epilogue) + ")\n";
+        src += kGemmTcDeviceSrc;
+        src += kGemmH2DeviceSrc;
+        src += "\nextern \"C\" __global__ void __launch_bounds__(sage_tc::kThreads, 1)\n"
+               "gemm_tc_h2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_a2,\n"
+               "           const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_b2, const sage_tc::H2Params p) {\n"
+               "    sage_tc::gemm_h2_body<" + std::to_string(bn) + ", " + std::to_string(ctas) + ">(&map_a, &map_a2, &map_b, &map_b2, p);\n}\n";
+        sage_status st = ctx.module_get(src, &mod);
+        if (st) return st;
+        ctx.module_remember(key, mod);
+    }
+    CUtensorMap map_a, map_a2, map_b, map_b2;
+    if (!ctx.dry()) {
+        auto ok = [](const H2Operand &o) {
+            return o.hi && aligned16(o.hi) && o.ld % 8 == 0 && o.ld > 0 && o.plane % 8 == 0 && o.plane > 0 && (o.nb0 == 1 || (o.sb0 % 8 == 0 && o.sb0 > 0)) &&
+                   (o.nb1 == 1 || (o.sb1 % 8 == 0 && o.sb1 > 0));
+        };
+        bool good = ok(g.b) && encode_operand(encode, g.b, g.k, (unsigned)(bn / ctas), &map_b);
+        map_b2 = map_b;
+        if (cols.narrow) good = good && encode_operand(encode, g.b, g.k, (unsigned)(p.rag_bn / ctas), &map_b2);
+        if (!g.conv) {
+            good = good && ok(g.a) && encode_operand(encode, g.a, g.k, BM, &map_a);
+            map_a2 = map_a;
+        } else {
+            good = good && aligned16(g.a.hi) && g.a.plane % 8 == 0;
+            if (halo)
+                good = good && encode_halo(encode, g, g.a.hi, (unsigned)halo_wb, (unsigned)(halo_r + g.win.ker_h - 1), &map_a) &&
+                       encode_halo(encode, g, g.a.hi + g.a.plane, (unsigned)halo_wb, (unsigned)(halo_r + g.win.ker_h - 1), &map_a2);
+            else
+                good = good && encode_im2col(encode_conv, g, g.a.hi, &map_a) && encode_im2col(encode_conv, g, g.a.hi + g.a.plane, &map_a2);
+        }
+        if (!good) return ctx.fail(SAGE_ERR_INVALID, "gemm_h2: an operand is not addressable by TMA");
+    }
+    std::string label;
+    if (ctx.verbose_names)
+        label = "gemm_tc_h2[" + std::to_string(g.m) + "x" + std::to_string(g.n) + "x" + std::to_string(g.k) + (g.batch > 1 ? "x" + std::to_string(g.batch) : "") +
+                (g.conv ? (halo ? ",conv,taps" : ",conv") : "") + ",bn" + std::to_string(bn) + (cols.narrow ? "/" + std::to_string(cols.wide) + "+" + std::to_string(cols.narrow) + "x192" : "") +
+                (ctas == 2 ? ",pair" : "") + "]o" + std::to_string(out_mask);
+    if (plain) {
+        ctx.note_launch(ctx.verbose_names ? label.c_str() : "gemm_tc_3xtf32");
+        if (ctx.dry()) return SAGE_OK;
+        if (ctas == 2)
+            return bn == 256 ? launch_plain<256, 2>(ctx, map_a, map_b, map_b2, p, grid, smem)
+                   : bn == 128 ? launch_plain<128, 2>(ctx, map_a, map_b, map_b2, p, grid, smem) : launch_plain<64, 2>(ctx, map_a, map_b, map_b2, p, grid, smem);
+        return bn == 256 ? launch_plain<256, 1>(ctx, map_a, map_b, map_b2, p, grid, smem)
+               : bn == 128 ? launch_plain<128, 1>(ctx, map_a, map_b, map_b2, p, grid, smem) : launch_plain<64, 1>(ctx, map_a, map_b, map_b2, p, grid, smem);
+    }
+    const uint32_t gr[3] = {(uint32_t)grid, 1, 1}, bl[3] = {(uint32_t)kThreads, 1, 1};
+    void *params[5] = {&map_a, &map_a2, &map_b, &map_b2, &p};
+    // launch lists have one name for a tensor-core product; verbose ones tell the kernels apart
+    return ctx.launch(mod, "gemm_tc_h2", gr, bl, (uint32_t)smem, params, ctx.verbose_names ? label.c_str() : "gemm_tc_3xtf32", true, ctas);
+}
+
+}  // namespace k
+}  // namespace sage

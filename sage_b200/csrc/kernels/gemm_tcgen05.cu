@@ -398,57 +398,21 @@ sage_status split_tf32_flat(Context &ctx, const float *src, long long n, float *
     return ctx.check_cuda(cudaGetLastError(), "split_tf32_flat launch");
 }
 
-static sage_status split_view_into(Context &ctx, const float *src, const SplitView &v, float *dst, SplitPlanes *out) {
-    out->planes = dst;
+sage_status split_tf32_view(Context &ctx, const float *src, const SplitView &v, SplitPlanes *out) {
+    if (v.rows > 0x7fffffffLL || v.cols > 0x7fffffffLL || v.nb0 * v.nb1 > 0x7fffffffLL)
+        return ctx.fail(SAGE_ERR_UNSUPPORTED, "split_tf32: extents beyond 2^31");
     out->rows = (int)v.rows;
     out->cols = (int)v.cols;
     out->batches = (int)(v.nb0 * v.nb1);
     out->pitch = (int)((v.cols + 3) / 4 * 4);
     const long long plane = (long long)out->batches * out->rows * out->pitch;
+    out->block = ctx.allocator().alloc((size_t)plane * 2 * sizeof(float));
+    if (!out->block) return ctx.fail(SAGE_ERR_OOM, "out of memory for the tf32 operand split");
+    out->planes = reinterpret_cast<float *>(out->block->ptr);
     ctx.note_launch("split_tf32");
     if (ctx.dry()) return SAGE_OK;
-    split_tf32_kernel<<<split_grid(ctx, plane / 4), 256, 0, ctx.stream()>>>(src, v, dst, out->pitch, plane);
+    split_tf32_kernel<<<split_grid(ctx, plane / 4), 256, 0, ctx.stream()>>>(src, v, out->planes, out->pitch, plane);
     return ctx.check_cuda(cudaGetLastError(), "split_tf32 launch");
-}
-
-size_t split_tf32_bytes(int rows, int cols, int batches) {
-    return (size_t)batches * rows * ((cols + 3) / 4 * 4) * 2 * sizeof(float);
-}
-
-sage_status split_tf32_view(Context &ctx, const float *src, const SplitView &v, SplitPlanes *out) {
-    if (v.rows > 0x7fffffffLL || v.cols > 0x7fffffffLL || v.nb0 * v.nb1 > 0x7fffffffLL)
-        return ctx.fail(SAGE_ERR_UNSUPPORTED, "split_tf32: extents beyond 2^31");
-    out->block = ctx.allocator().alloc(split_tf32_bytes((int)v.rows, (int)v.cols, (int)(v.nb0 * v.nb1)));
-    if (!out->block) return ctx.fail(SAGE_ERR_OOM, "out of memory for the tf32 operand split");
-    return split_view_into(ctx, src, v, reinterpret_cast<float *>(out->block->ptr), out);
-}
-
-static SplitView simple_view(long long ld, long long batch_stride, int rows, int cols, int batches) {
-    SplitView v;
-    v.nb0 = batches;
-    v.rows = rows;
-    v.cols = cols;
-    v.sb0 = batch_stride;
-    v.ld = ld;
-    return v;
-}
-
-sage_status split_tf32(Context &ctx, const float *src, long long ld, long long batch_stride, int rows, int cols, int batches,
-                       SplitPlanes *out) {
-    return split_tf32_view(ctx, src, simple_view(ld, batch_stride, rows, cols, batches), out);
-}
-
-// Same split, written into memory the caller provides (`dst` must hold split_tf32_bytes(...) bytes
-// and be 16-byte aligned).  Nothing is allocated; out->block stays null.
-sage_status split_tf32_into(Context &ctx, const float *src, long long ld, long long batch_stride, int rows, int cols, int batches,
-                            float *dst, SplitPlanes *out) {
-    out->block = nullptr;
-    return split_view_into(ctx, src, simple_view(ld, batch_stride, rows, cols, batches), dst, out);
-}
-
-void free_split(Context &ctx, SplitPlanes *s) {
-    if (s->block) ctx.allocator().free(s->block);
-    s->block = nullptr;
 }
 
 // ---------------------------------------------------------------------------------- GEMM launcher
@@ -915,48 +879,9 @@ sage_status attention_tc_run(Context &ctx, const TcAttn &a) {
     return ctx.launch(mod, "attention_tc_3xtf32", gr, bl, (uint32_t)smem, params, ctx.verbose_names ? label.c_str() : nullptr, true, 1);
 }
 
-static TcOperand operand_of(const SplitPlanes &s) {
-    TcOperand o;
-    o.hi = s.planes;
-    o.ld = s.pitch;
-    o.rows = s.rows;
-    o.cols = s.cols;
-    o.nb0 = s.batches;
-    o.sb0 = (long long)s.rows * s.pitch;
-    o.plane = (long long)s.batches * s.rows * s.pitch;
-    return o;
-}
-
-sage_status gemm_tcgen05_planes(Context &ctx, const GemmArgs &g, const SplitPlanes &a, const SplitPlanes &b, bool no_split_k) {
-    TcGemm t;
-    t.a_kmajor = !g.ta;
-    t.b_kmajor = g.tb;
-    t.m = g.m;
-    t.n = g.n;
-    t.k = g.k;
-    t.batch = g.batch;
-    t.a = operand_of(a);
-    t.b = operand_of(b);
-    t.c = g.c;
-    t.ldc = g.ldc;
-    t.sc0 = g.stride_c;
-    t.nbc0 = g.batch;
-    t.no_split_k = no_split_k;
-    return gemm_tc_run(ctx, t);
-}
-
 sage_status gemm_tcgen05(Context &ctx, const GemmArgs &g) {
     if (!gemm_tc_shape_ok(g.m, g.n, g.k, g.batch)) return SAGE_ERR_UNSUPPORTED;
-    // A as stored: [M,K] (K-major) or, transposed, [K,M] (MN-major); B: [K,N] (MN-major) or [N,K] (K-major).
-    SplitPlanes a, b;
-    sage_status st = split_tf32(ctx, g.a, g.lda, g.stride_a, g.ta ? (int)g.k : (int)g.m, g.ta ? (int)g.m : (int)g.k, (int)g.batch, &a);
-    if (st) return st;
-    st = split_tf32(ctx, g.b, g.ldb, g.stride_b, g.tb ? (int)g.n : (int)g.k, g.tb ? (int)g.k : (int)g.n, (int)g.batch, &b);
-    if (!st) st = gemm_tcgen05_planes(ctx, g, a, b);
-    // Stream-ordered: the split buffers may be reused by later launches on this stream.
-    free_split(ctx, &a);
-    free_split(ctx, &b);
-    return st;
+    return gemm_h2(ctx, g);
 }
 
 }  // namespace k

@@ -86,16 +86,6 @@ struct SplitPlanes {
     int rows = 0, cols = 0, pitch = 0, batches = 0;
 };
 bool gemm_tc_supported(const GemmArgs &g);
-sage_status split_tf32(Context &ctx, const float *src, long long ld, long long batch_stride, int rows, int cols, int batches,
-                       SplitPlanes *out);
-void free_split(Context &ctx, SplitPlanes *s);
-// The same split into caller-provided device memory of split_tf32_bytes(...) bytes; allocates nothing.
-size_t split_tf32_bytes(int rows, int cols, int batches);
-sage_status split_tf32_into(Context &ctx, const float *src, long long ld, long long batch_stride, int rows, int cols, int batches,
-                            float *dst, SplitPlanes *out);
-// `a` / `b` are the splits of g.a / g.b (as stored); g.a / g.b themselves are not read.  With `no_split_k` the
-// product runs as one pass over K whatever its shape, so neither the allocator nor a second kernel is reached.
-sage_status gemm_tcgen05_planes(Context &ctx, const GemmArgs &g, const SplitPlanes &a, const SplitPlanes &b, bool no_split_k = false);
 
 // ---- the general form of the tensor-core GEMM, used by the evaluator's fused GEMM operator.
 // A split operand as the tensor core reads it: `rows` x `cols` with cols contiguous, rows `ld` floats
@@ -178,6 +168,58 @@ struct SplitView {
     long long sb1 = 0, sb0 = 0, ld = 0, col_stride = 1;
 };
 sage_status split_tf32_view(Context &ctx, const float *src, const SplitView &v, SplitPlanes *out);
+// ---- gemm_h2.cu: the product over two half-precision pieces per operand (kernels/gemm_h2_device.inc states the
+// representation).  Both operands are read with K contiguous: `rows` x `k`, rows `ld` elements apart, batch index =
+// b1 * nb0 + b0 at b0 * sb0 + b1 * sb1.  `hi` points at the first hi piece, the lo pieces lie `plane` elements further.
+// Operand A has a scale per row and 64 k (`scale` + b0 * s_b0 + b1 * s_b1 + row * s_row + k / 64), operand B one per row
+// (`scale` + batch * s_b0 + row).  hi must be 16-byte aligned and ld, sb0, sb1, plane multiples of 8.
+struct H2Operand {
+    const unsigned short *hi = nullptr;
+    long long plane = 0, ld = 0, rows = 0;
+    long long nb0 = 1, nb1 = 1, sb0 = 0, sb1 = 0;
+    bool bcast = false;
+    const float *scale = nullptr;
+    long long s_row = 0, s_b0 = 0, s_b1 = 0;
+};
+struct H2Gemm {
+    bool conv = false;        // A is the im2col of a contiguous NHWC image (a.hi, a.plane, a.scale) with C % 64 == 0
+    long long img_n = 0, img_h = 0, img_w = 0, img_c = 0, out_h = 0, out_w = 0;
+    Window win{};
+    long long m = 0, n = 0, k = 0, batch = 1;
+    H2Operand a, b;
+    float *c = nullptr, *c_hi = nullptr;  // result as fp32 and / or as tf32 planes, as in TcGemm
+    long long c_plane = 0;
+    unsigned short *h_hi = nullptr;       // ... and / or in half-precision pieces: needs n, ldc, sc0, sc1 multiples of 64
+    long long h_plane = 0;
+    float *h_scale = nullptr;
+    long long ldc = 0, sc0 = 0, sc1 = 0, nbc0 = 1;
+    int naux = 0;
+    TcAuxArg aux[3];
+    std::string epilogue;
+};
+sage_status gemm_h2_run(Context &ctx, const H2Gemm &g, bool no_slices = false);
+// How many K slices gemm_h2_run would cut this product into (0 = none), as gemm_tc_split_plan.
+int gemm_h2_slices(Context &ctx, const H2Gemm &g);
+// The whole product of plain fp32 operands.  With `scratch` (gemm_h2_scratch_bytes of device memory, 256-byte aligned)
+// nothing is taken from the allocator and K is not cut.
+size_t gemm_h2_scratch_bytes(const GemmArgs &g);
+sage_status gemm_h2(Context &ctx, const GemmArgs &g, void *scratch = nullptr);
+bool conv_h2_ok(const H2Gemm &g);
+// Pieces of `n` consecutive floats (a multiple of 64), laid out like the source, a scale per 64.
+sage_status split_h2_flat(Context &ctx, const float *src, long long n, unsigned short *hi, long long plane, float *scale);
+// Pieces of a strided view (b1, b0, row, col) gathered with its columns contiguous: [batch][rows][pitch], pitch = cols
+// rounded up to 8.  `whole_rows`: one scale per row (operand B) instead of one per 64 columns.
+struct H2Split {
+    Block *block = nullptr;
+    unsigned short *hi = nullptr;
+    float *scale = nullptr;
+    long long plane = 0, pitch = 0;
+};
+size_t split_h2_bytes(long long batches, long long rows, long long cols, bool whole_rows);
+sage_status split_h2_view_into(Context &ctx, const float *src, const SplitView &v, bool whole_rows, void *dst, H2Split *out);
+sage_status split_h2_view(Context &ctx, const float *src, const SplitView &v, bool whole_rows, H2Split *out);
+H2Operand h2_operand(const H2Split &s, long long batches, long long rows, long long cols, bool whole_rows);
+
 // Launches a kernel whose bounded wait runs out (nothing arrives on its barrier): ~1 s, then status bit 0x140.
 sage_status bounded_wait_selftest(Context &ctx);
 sage_status gemm_simt(Context &ctx, const GemmArgs &g);

@@ -1,4 +1,4 @@
-// sage_gemm_noalloc: the 3xTF32 tensor-core GEMM for callers that must not allocate device memory.
+// sage_gemm_noalloc: the tensor-core GEMM for callers that must not allocate device memory.
 //
 // The regular entry points (sage_gemm, sage_gemm_strided_batched) take the scratch for the hi/lo
 // operand split from the context's allocator, which may reach cudaMalloc when its pool has to grow.
@@ -12,6 +12,7 @@
 // Limits and rules
 //   * 2 * 4 bytes * (rows_a * pitch(cols_a) + rows_b * pitch(cols_b)) must fit in kScratchBytes,
 //     where pitch rounds the contiguous extent up to 4 floats; larger problems get SAGE_ERR_INVALID.
+//     (The operands in half-precision pieces take half of that and their scales; the limit callers know stays.)
 //   * A long K is never cut into slices here (sage_gemm does that with allocator scratch), so for k >= 1024
 //     with few output tiles this entry point is slower than sage_gemm and its sum order differs from it.
 //   * The first call on a device looks up the device address of the array (cudaGetSymbolAddress,
@@ -66,23 +67,16 @@ extern "C" sage_status sage_gemm_noalloc(sage_ctx *ctx, int32_t trans_a, int32_t
     if (!k::gemm_tc_supported(g))
         return C.fail(SAGE_ERR_UNSUPPORTED,
                       "sage_gemm_noalloc: needs n >= 32, k >= 32 and m >= 64 (or m >= 16 with k >= 2048): the tensor-core path; use sage_gemm");
-    const int a_rows = g.ta ? (int)k : (int)m, a_cols = g.ta ? (int)m : (int)k;
-    const int b_rows = g.tb ? (int)n : (int)k, b_cols = g.tb ? (int)k : (int)n;
-    const size_t a_bytes = k::split_tf32_bytes(a_rows, a_cols, 1), b_bytes = k::split_tf32_bytes(b_rows, b_cols, 1);
-    const size_t a_span = (a_bytes + 255) / 256 * 256;  // keep the second operand 256-byte aligned
-    if (a_span + b_bytes > kScratchBytes)
+    auto limit_bytes = [](long long rows, long long cols) { return (size_t)rows * ((cols + 3) / 4 * 4) * 2 * sizeof(float); };
+    const size_t a_span = (limit_bytes(g.ta ? k : m, g.ta ? m : k) + 255) / 256 * 256, b_bytes = limit_bytes(g.tb ? n : k, g.tb ? k : n);
+    if (a_span + b_bytes > kScratchBytes || k::gemm_h2_scratch_bytes(g) > kScratchBytes)
         return C.fail(SAGE_ERR_INVALID, "sage_gemm_noalloc: the operand split needs " + std::to_string(a_span + b_bytes) +
                                             " bytes of scratch but the built-in scratch holds " + std::to_string(kScratchBytes) +
                                             "; use sage_gemm for this size");
     cudaError_t err;
     float *scratch = scratch_for_device(C.device(), &err);
     if (!scratch) return C.check_cuda(err, "cudaGetSymbolAddress(gemm scratch)");
-    k::SplitPlanes pa, pb;
-    sage_status st = k::split_tf32_into(C, g.a, g.lda, 0, a_rows, a_cols, 1, scratch, &pa);
-    if (st) return st;
-    st = k::split_tf32_into(C, g.b, g.ldb, 0, b_rows, b_cols, 1, scratch + a_span / sizeof(float), &pb);
-    if (st) return st;
     // One pass over K: sage_gemm may cut a long K into slices, which takes partial-product scratch from the
     // allocator and a second kernel.  Neither is reachable from here.
-    return k::gemm_tcgen05_planes(C, g, pa, pb, /*no_split_k=*/true);
+    return k::gemm_h2(C, g, scratch);
 }

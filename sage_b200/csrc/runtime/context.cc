@@ -257,7 +257,7 @@ int Context::blocks_per_sm(Module *m, const char *name, int block_threads, uint3
 
 sage_status Context::launch(Module *m, const char *name, const uint32_t grid[3], const uint32_t block[3],
                             uint32_t smem, void **params, const char *label, bool dependent, int cluster) {
-    note_launch(label && verbose_names ? label : name);
+    note_launch(label ? label : name);
     if (dry()) return SAGE_OK;
     Driver &d = driver();
     CUfunc_st *fn = nullptr;
