@@ -76,13 +76,43 @@ SG void sg_split_tf32(float x, float *hi, float *lo) {
 }
 )";
 
+// The half-precision pieces of four neighbouring results; 16 lanes hold a group of 64 (the rule of the GEMM's own split)
+static const char *kPreludeH2 = R"(
+SG uint sg_h2_bits(float x) { const uint b = __float_as_uint(x) & 0x7fffffffu; return b < 0x7f800000u ? b : 0u; }
+SG void sg_h2_two(float x0, float x1, float f, uint *hi, uint *lo) {
+  const float s0 = x0 * f, s1 = x1 * f;
+  uint h, l;
+  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(s1), "f"(s0));
+  float f0, f1;
+  asm("{.reg .f16 a, b; mov.b32 {a, b}, %2; cvt.f32.f16 %0, a; cvt.f32.f16 %1, b;}" : "=f"(f0), "=f"(f1) : "r"(h));
+  const float r0 = sg_h2_bits(x0) == 0u ? 0.f : (s0 - f0) * 2048.f, r1 = sg_h2_bits(x1) == 0u ? 0.f : (s1 - f1) * 2048.f;
+  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(l) : "f"(r1), "f"(r0));
+  *hi = h; *lo = l;
+}
+SG void sg_h2_store(float4 r, unsigned long long g, unsigned short *h2, long long plane, float *scale) {
+  uint b = sg_h2_bits(r.x);
+  uint t = sg_h2_bits(r.y); b = b > t ? b : t;
+  t = sg_h2_bits(r.z); b = b > t ? b : t;
+  t = sg_h2_bits(r.w); b = b > t ? b : t;
+  for (int o = 8; o > 0; o >>= 1) { t = __shfl_xor_sync(0xffffu << (threadIdx.x & 16), b, o); b = b > t ? b : t; }
+  int e = (int)(b >> 23); e = e < 27 ? 27 : e;
+  const float f = __uint_as_float((uint)(268 - e) << 23);
+  uint2 hi, lo;
+  sg_h2_two(r.x, r.y, f, &hi.x, &lo.x);
+  sg_h2_two(r.z, r.w, f, &hi.y, &lo.y);
+  *reinterpret_cast<uint2 *>(h2 + g) = hi;
+  *reinterpret_cast<uint2 *>(h2 + plane + g) = lo;
+  if ((threadIdx.x & 15) == 0) scale[g >> 6] = __uint_as_float((uint)(e - 14) << 23);
+}
+)";
+
 const char *map_prelude_text() { return kPrelude; }
 
 static const char *ctype(int dt) { return dt == SAGE_F32 ? "float" : dt == SAGE_I32 ? "int" : "uint"; }
 static const char *vtype(int dt) { return dt == SAGE_F32 ? "float4" : dt == SAGE_I32 ? "int4" : "uint4"; }
 
 sage_status map_plan(const std::string &expr, const std::vector<MapOperand> &in, int out_dtype, const void *y,
-                     int out_ndim, const long long *out_ext, MapPlan *plan, bool emit_source, bool planes) {
+                     int out_ndim, const long long *out_ext, MapPlan *plan, bool emit_source, int planes) {
     const int nin = (int)in.size();
     // ---- collapse axes
     long long ext[k::kMaxDims];
@@ -156,12 +186,15 @@ sage_status map_plan(const std::string &expr, const std::vector<MapOperand> &in,
     plan->vec = vec;
     const bool wide = n >= (1LL << 32);
     const char *it = wide ? "unsigned long long" : "unsigned int";
-    plan->signature = modes + ":" + std::to_string(vec) + ":" + std::to_string(nd) + (wide ? "w" : "n") + (planes ? "P" : "");
+    if (vec != 4 || n % 64 != 0) planes &= ~2;
+    plan->planes = planes;
+    plan->signature = modes + ":" + std::to_string(vec) + ":" + std::to_string(nd) + (wide ? "w" : "n") + ((planes & 1) ? "P" : "") + ((planes & 2) ? "H" : "");
     if (!emit_source) return SAGE_OK;  // the caller already holds the kernel for this signature
 
     // ---- emit
     std::ostringstream s;
     s << kPrelude;
+    if (planes & 2) s << kPreludeH2;
     s << "struct MapP { long long n; unsigned long long ext[" << k::kMaxDims << "]; long long str["
       << (nin > 0 ? nin : 1) << "][" << k::kMaxDims << "]; };\n";
     s << "SG " << ctype(out_dtype) << " sage_expr(";
@@ -169,7 +202,8 @@ sage_status map_plan(const std::string &expr, const std::vector<MapOperand> &in,
     s << ") { return (" << ctype(out_dtype) << ")(" << expr << "); }\n";
     s << "extern \"C\" __global__ void __launch_bounds__(256) sage_map(";
     for (int q = 0; q < nin; ++q) s << "const " << ctype(in[q].dtype) << " *__restrict__ x" << q << "_buf, ";
-    s << ctype(out_dtype) << " *__restrict__ y, const MapP p" << (planes ? ", float *__restrict__ hi, const long long plane" : "") << ") {\n";
+    s << ctype(out_dtype) << " *__restrict__ y, const MapP p" << ((planes & 1) ? ", float *__restrict__ hi, const long long plane" : "")
+      << ((planes & 2) ? ", unsigned short *__restrict__ h2, const long long h2_plane, float *__restrict__ h2_scale" : "") << ") {\n";
     // launched as a programmatic dependent: wait for the kernel before this one before touching memory
     s << "  asm volatile(\"griddepcontrol.launch_dependents;\" ::: \"memory\");\n";
     s << "  asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");\n";
@@ -204,7 +238,7 @@ sage_status map_plan(const std::string &expr, const std::vector<MapOperand> &in,
         s << "  const " << ctype(out_dtype) << " r = sage_expr(";
         for (int q = 0; q < nin; ++q) s << (q ? ", " : "") << "x" << q;
         s << ");\n  y[g] = r;\n";
-        if (planes) s << "  { float h, l; sg_split_tf32(r, &h, &l); hi[g] = h; hi[plane + g] = l; }\n";
+        if (planes & 1) s << "  { float h, l; sg_split_tf32(r, &h, &l); hi[g] = h; hi[plane + g] = l; }\n";
     } else {
         for (int q = 0; q < nin; ++q) {
             const char *ct = ctype(in[q].dtype);
@@ -226,7 +260,8 @@ sage_status map_plan(const std::string &expr, const std::vector<MapOperand> &in,
             s << ");\n";
         }
         s << "  *reinterpret_cast<" << vtype(out_dtype) << " *>(y + g) = r;\n";
-        if (planes)
+        if (planes & 2) s << "  sg_h2_store(r, g, h2, h2_plane, h2_scale);\n";
+        if (planes & 1)
             s << "  { float4 h, l; sg_split_tf32(r.x, &h.x, &l.x); sg_split_tf32(r.y, &h.y, &l.y); sg_split_tf32(r.z, &h.z, &l.z); "
                  "sg_split_tf32(r.w, &h.w, &l.w);\n    *reinterpret_cast<float4 *>(hi + g) = h; *reinterpret_cast<float4 *>(hi + plane + g) = l; }\n";
     }
@@ -241,8 +276,8 @@ struct MapPHost {
 };
 
 sage_status map_launch(Context &ctx, const std::string &expr, const std::vector<MapOperand> &in, int out_dtype,
-                       void *y, int out_ndim, const long long *out_ext, MapCache *cache, float *hi, long long plane) {
-    const bool planes = hi != nullptr && out_dtype == SAGE_F32;
+                       void *y, int out_ndim, const long long *out_ext, MapCache *cache, const k::PlaneOut &out) {
+    const int planes = out_dtype == SAGE_F32 ? (out.hi ? 1 : 0) | (out.h2 ? 2 : 0) : 0;
     MapPlan plan;
     sage_status st = map_plan(expr, in, out_dtype, y, out_ndim, out_ext, &plan, false, planes);
     if (st) return st;
@@ -280,9 +315,15 @@ sage_status map_launch(Context &ctx, const std::string &expr, const std::vector<
     }
     params.push_back(&y);
     params.push_back(pb.data());
-    if (planes) {
-        params.push_back(&hi);
-        params.push_back(&plane);
+    k::PlaneOut o = out;
+    if (plan.planes & 1) {
+        params.push_back(&o.hi);
+        params.push_back(&o.plane);
+    }
+    if (plan.planes & 2) {
+        params.push_back(&o.h2);
+        params.push_back(&o.h2_plane);
+        params.push_back(&o.h2_scale);
     }
     const long long chunks = (plan.n + plan.vec - 1) / plan.vec;
     const uint32_t grid[3] = {(uint32_t)((chunks + 255) / 256), 1, 1};
@@ -293,7 +334,9 @@ sage_status map_launch(Context &ctx, const std::string &expr, const std::vector<
         for (char &ch : label)
             if (ch == ' ') ch = '_';
     }
-    return ctx.launch(mod, "sage_map", grid, block, 0, params.data(), label.empty() ? nullptr : label.c_str(), true);
+    st = ctx.launch(mod, "sage_map", grid, block, 0, params.data(), label.empty() ? nullptr : label.c_str(), true);
+    if (!st && out.h2 && !(plan.planes & 2)) st = k::split_h2_flat(ctx, static_cast<const float *>(y), plan.n, out.h2, out.h2_plane, out.h2_scale);
+    return st;
 }
 
 }  // namespace sage

@@ -30,19 +30,21 @@ struct MapPlan {
     int vec = 1;
     int ndim = 1;
     long long n = 0;
+    int planes = 0;
     unsigned long long ext[k::kMaxDims] = {0};
     std::vector<std::vector<long long>> strides;  // per input, collapsed dims
 };
 
 // `expr` is a C expression over x0..x{n-1}; helper functions come from the prelude
 // (sg_exp, sg_max, ...).  The output is contiguous with `out_ext`.
-// `planes`: the kernel also writes the tf32 hi / lo split of every (f32) result, laid out like y.
+// `planes`: bit 0, the kernel also writes the tf32 hi / lo split of every (f32) result, laid out like y; bit 1, its
+// half-precision pieces (in the vector form only, and for whole groups of 64: else the plan drops the bit).
 sage_status map_plan(const std::string &expr, const std::vector<MapOperand> &in, int out_dtype, const void *y,
-                     int out_ndim, const long long *out_ext, MapPlan *plan, bool emit_source = true, bool planes = false);
+                     int out_ndim, const long long *out_ext, MapPlan *plan, bool emit_source = true, int planes = 0);
 
-// `hi` (optional, f32 results only): hi plane of y's tf32 split, the lo plane `plane` floats further; a
-// tensor-core GEMM that reads y next then needs no split pass.
+// `out` (f32 results only): operand forms of y to write as well; a tensor-core GEMM that reads y next then needs no
+// split pass.
 sage_status map_launch(Context &ctx, const std::string &expr, const std::vector<MapOperand> &in, int out_dtype,
-                       void *y, int out_ndim, const long long *out_ext, MapCache *cache, float *hi = nullptr, long long plane = 0);
+                       void *y, int out_ndim, const long long *out_ext, MapCache *cache, const k::PlaneOut &out = k::PlaneOut());
 
 }  // namespace sage

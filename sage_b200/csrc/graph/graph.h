@@ -153,14 +153,30 @@ struct SplitCache {
     }
 };
 
+// The half-precision pieces of (a view of) a storage, kept like the planes: `whole` mirrors the storage element for element
+// with a scale per 64, the compact forms hold one view gathered with its contraction axis contiguous.
+struct H2Cache {
+    k::H2Split pieces;
+    std::shared_ptr<Allocator> alloc;
+    Shape view;
+    bool swapped = false;  // compact: the view's last two axes were exchanged
+    ~H2Cache() {
+        if (alloc && pieces.block) alloc->free(pieces.block);
+    }
+};
+
 struct Storage {
     std::shared_ptr<SplitCache> split;       // whole-storage planes
     std::shared_ptr<SplitCache> split_view;  // last compact split of a view
+    std::shared_ptr<H2Cache> h2, h2_view, h2_rows;  // whole storage; last compact operand A; last compact operand B
     uint64_t version = 0;                    // bumped whenever the contents are rewritten
-    bool planes_only = false;                // the fp32 buffer was never written: only `split` holds the value
+    bool planes_only = false;                // the fp32 buffer was never written: only `split` / `h2` hold the value
     void drop_splits() {
         split.reset();
         split_view.reset();
+        h2.reset();
+        h2_view.reset();
+        h2_rows.reset();
         ++version;
     }
     Context *ctx = nullptr;  // identity only; never dereferenced by the destructor

@@ -47,6 +47,31 @@ static sage_status storage_planes(Context &ctx, Storage &st) {  // planes of exi
     return s;
 }
 
+// ------------------------------------------------------------------------------ half-precision pieces of a storage
+sage_status storage_h2_attach(Context &ctx, Storage &st) {  // allocate only; the caller's kernel fills them
+    if (st.h2) return SAGE_OK;
+    auto c = std::make_shared<H2Cache>();
+    c->alloc = ctx.allocator_ptr();
+    const long long n = ((long long)(st.bytes / 4) + 127) / 128 * 128;
+    c->pieces.plane = n;
+    c->pieces.block = ctx.allocator().alloc((size_t)n * 4 + (size_t)(n / 64) * 4);
+    if (!c->pieces.block) return ctx.fail(SAGE_ERR_OOM, "out of memory for half-precision pieces");
+    c->pieces.hi = reinterpret_cast<unsigned short *>(c->pieces.block->ptr);
+    c->pieces.scale = reinterpret_cast<float *>(c->pieces.block->ptr + n * 4);
+    st.h2 = c;
+    return SAGE_OK;
+}
+
+sage_status storage_h2(Context &ctx, Storage &st) {  // pieces of existing data: run the split pass
+    if (st.h2) return SAGE_OK;
+    if (st.planes_only) return ctx.fail(SAGE_ERR_INVALID, "internal: a tensor without fp32 values has no half-precision pieces");
+    sage_status s = storage_h2_attach(ctx, st);
+    if (s) return s;
+    s = k::split_h2_flat(ctx, (const float *)st.dev, (long long)(st.bytes / 4), st.h2->pieces.hi, st.h2->pieces.plane, st.h2->pieces.scale);
+    if (s) st.h2.reset();
+    return s;
+}
+
 // ------------------------------------------------------------------------------ operand views
 // A GEMM operand is a tensor view of rank >= 2: the last two axes are the matrix, the axes before
 // them the batch.  `levels` collapses the batch axes into at most two (extent, stride) pairs,
@@ -166,6 +191,94 @@ static sage_status make_operand(Context &ctx, const Tensor &t, k::TcOperand *op,
     return SAGE_OK;
 }
 
+// ------------------------------------------------------------------------------ operands in half-precision pieces
+// Can this view be read straight from the pieces of its whole storage?  Its contraction axis (the last one, or with `trans`
+// the one before) must be contiguous and every run of 64 along it a group of the storage.
+bool h2_view_direct(const Shape &sh, bool trans, BatchLevels *bl) {
+    const int r = sh.rank();
+    if (r < 2 || !collapse_batch(sh, r - 2, bl)) return false;
+    const int ka = trans ? r - 2 : r - 1, ma = trans ? r - 1 : r - 2;
+    if (sh.strides[ka] != 1 || sh.extents[ka] < 32 || sh.offset % 64) return false;
+    if (sh.extents[ma] > 1 && (sh.strides[ma] <= 0 || sh.strides[ma] % 64)) return false;
+    for (int l = 0; l < 2; ++l)
+        if (bl->n[l] > 1 && (bl->s[l] <= 0 || bl->s[l] % 64)) return false;
+    return true;
+}
+bool h2_view_ok(const Shape &sh, bool trans) {
+    BatchLevels bl;
+    return h2_view_direct(sh, trans, &bl);
+}
+
+// Operand A (`rows` = a scale per 64 k) or B (`whole_rows`: one per row, always a compact copy kept beside the storage).
+static sage_status make_h2_operand(Context &ctx, const Tensor &t, bool trans, bool whole_rows, k::H2Operand *op, std::shared_ptr<H2Cache> *hold) {
+    const Shape &sh = t.desc.shape;
+    const int r = sh.rank(), ka = trans ? r - 2 : r - 1, ma = trans ? r - 1 : r - 2;
+    const long long rows = sh.extents[ma], cols = sh.extents[ka];
+    BatchLevels bl;
+    Storage &st = *t.data;
+    const bool small_part = !st.h2 && (unsigned long long)sh.size() * 16 < st.bytes;
+    if (!whole_rows && h2_view_direct(sh, trans, &bl) && st.bytes % 256 == 0 && !small_part) {
+        sage_status s = storage_h2(ctx, st);
+        if (s) return s;
+        *hold = st.h2;
+        op->hi = st.h2->pieces.hi + sh.offset;
+        op->plane = st.h2->pieces.plane;
+        op->scale = st.h2->pieces.scale + sh.offset / 64;
+        op->rows = rows;
+        op->ld = rows == 1 ? (cols + 63) / 64 * 64 : sh.strides[ma];
+        op->s_row = op->ld / 64;
+        op->nb0 = bl.n[0];
+        op->nb1 = bl.n[1];
+        op->sb0 = bl.s[0];
+        op->sb1 = bl.s[1];
+        op->s_b0 = bl.s[0] / 64;
+        op->s_b1 = bl.s[1] / 64;
+        return SAGE_OK;
+    }
+    if (st.planes_only) return ctx.fail(SAGE_ERR_INVALID, "internal: a tensor without fp32 values reached an operand that has to be gathered");
+    if (!collapse_batch(sh, r - 2, &bl)) return ctx.fail(SAGE_ERR_UNSUPPORTED, "gemm: batch axes of an operand do not collapse to two levels");
+    std::shared_ptr<H2Cache> &c = whole_rows ? st.h2_rows : st.h2_view;
+    if (!(c && c->view == sh && c->swapped == trans)) {
+        auto fresh = std::make_shared<H2Cache>();
+        fresh->alloc = ctx.allocator_ptr();
+        fresh->view = sh;
+        fresh->swapped = trans;
+        k::SplitView v;
+        v.nb0 = bl.n[0];
+        v.nb1 = bl.n[1];
+        v.sb0 = bl.s[0];
+        v.sb1 = bl.s[1];
+        v.rows = rows;
+        v.cols = cols;
+        v.ld = sh.strides[ma];
+        v.col_stride = sh.strides[ka];
+        sage_status s = k::split_h2_view(ctx, (const float *)t.ptr(), v, whole_rows, &fresh->pieces);
+        if (s) return s;
+        c = fresh;
+    }
+    *hold = c;
+    *op = k::h2_operand(c->pieces, bl.n[0] * bl.n[1], rows, cols, whole_rows);
+    return SAGE_OK;
+}
+
+// Where a result's operand forms go, as its readers asked: attaches them to `y` and says whether the fp32 store may be left out.
+static sage_status attach_forms(Context &ctx, Tensor *y, bool emit, bool emit_h2, k::PlaneOut *o) {
+    if (emit) {
+        sage_status st = storage_planes_attach(ctx, *y->data);
+        if (st) return st;
+        o->hi = y->data->split->planes.planes + y->desc.shape.offset;
+        o->plane = y->data->split->plane;
+    }
+    if (emit_h2) {
+        sage_status st = storage_h2_attach(ctx, *y->data);
+        if (st) return st;
+        o->h2 = y->data->h2->pieces.hi;
+        o->h2_plane = y->data->h2->pieces.plane;
+        o->h2_scale = y->data->h2->pieces.scale;
+    }
+    return SAGE_OK;
+}
+
 // ------------------------------------------------------------------------------ the operator
 // Axis groups of the epilogue's index space.
 enum { GBatchHi = 0, GBatchLo = 1, GRow = 2, GCol = 3 };
@@ -190,6 +303,7 @@ struct GemmOp : Operator {
     bool conv = false;              // operand A is the im2col of input 0 ([N,H,W,C]), made on the fly as tf32 planes
     k::Window win{};
     long long img[6] = {0, 0, 0, 0, 0, 0};  // N, H, W, C, OH, OW
+    bool h2 = false;                // runs on half-precision pieces (gemm_h2); decided for a whole program (assign_h2)
     bool row_softmax = false;       // the stored value is softmax over the last axis of the (epilogue of the) product
     bool folded = false;            // result stored through (ldc, sc0, sc1, nbc0) instead of row-major [batch, M, N]
     long long ldc = 0, sc0 = 0, sc1 = 0, nbc0 = 1;
@@ -246,12 +360,16 @@ struct GemmOp : Operator {
     }
 
     sage_status compute(const std::vector<Tensor> &x, Context &ctx, Tensor *y) override {
-        const bool emit = ctx.hint_emit_planes, only = emit && ctx.hint_planes_only;
-        ctx.hint_emit_planes = ctx.hint_planes_only = false;
+        const bool emit = ctx.hint_emit_planes, emit_h2 = ctx.hint_emit_h2, only = (emit || emit_h2) && ctx.hint_planes_only;
+        ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = false;
         sage_status st = Tensor::uninit(ctx, out, y);
         if (st) return st;
         if (!lowered) dims_from_inputs();
-        if (attn) return compute_attention(x, ctx, y, emit, only);
+        if (h2) return compute_h2(x, ctx, y, emit, emit_h2, only);
+        if (!lowered && !attn && !batched && ctx.opts().pattern_fusion == 0 && ctx.opts().gemm_backend != 1 && k::gemm_tc_shape_ok(m, n, k, batch))
+            return compute_h2(x, ctx, y, false, false, false);  // the operator by itself
+        if (emit_h2 && !attn) return ctx.fail(SAGE_ERR_INVALID, "internal: the tf32 product does not write half-precision pieces");
+        if (attn) return compute_attention(x, ctx, y, emit, emit_h2, only);
         if (!lowered && (ctx.opts().gemm_backend == 1 || !k::gemm_tc_shape_ok(m, n, k, batch))) {
             const int o = batched ? 1 : 0;
             const Shape &a = x[0].desc.shape, &b = x[1].desc.shape;
@@ -423,19 +541,10 @@ struct GemmOp : Operator {
         g.naux = naux();
         g.epilogue = epilogue;
         g.row_softmax = row_softmax;
-        // the epilogue's batch decomposition: the axes of epi_ext tagged batch low / high
         long long e_nb0 = batch;
-        if (g.naux > 0) {
-            e_nb0 = 1;
-            bool any_hi = false;
-            for (size_t d = 0; d < epi_ext.size(); ++d) {
-                if (epi_group[d] == GBatchLo) e_nb0 *= epi_ext[d];
-                if (epi_group[d] == GBatchHi && epi_ext[d] > 1) any_hi = true;
-            }
-            if (!any_hi && e_nb0 != batch) return ctx.fail(SAGE_ERR_INVALID, "internal: gemm epilogue batch groups do not cover the batch");
-            if (folded && nbc0 != e_nb0 && batch > 1) return ctx.fail(SAGE_ERR_INVALID, "internal: gemm epilogue and store pattern split the batch differently");
-            if (!folded) g.nbc0 = e_nb0, g.sc0 = m * n, g.sc1 = m * n * e_nb0;
-        }
+        st = epilogue_batches(ctx, g.naux, &e_nb0);
+        if (st) return st;
+        if (g.naux > 0 && !folded) g.nbc0 = e_nb0, g.sc0 = m * n, g.sc1 = m * n * e_nb0;
         for (int i = 0; i < g.naux; ++i) {
             st = aux_strides(ctx, x[2 + i], &g.aux[i]);
             if (st) return st;
@@ -467,8 +576,10 @@ struct GemmOp : Operator {
                             operands[1 + i].ptr = x[2 + i].ptr();
                             operands[1 + i].view = x[2 + i].dims();
                         }
-                        st = map_launch(ctx, epilogue, operands, SAGE_F32, y->ptr(), out.shape.rank(), out.shape.extents.data(), &epi_cache, g.c_hi,
-                                        g.c_plane);
+                        k::PlaneOut planes;
+                        planes.hi = g.c_hi;
+                        planes.plane = g.c_plane;
+                        st = map_launch(ctx, epilogue, operands, SAGE_F32, y->ptr(), out.shape.rank(), out.shape.extents.data(), &epi_cache, planes);
                     }
                     ctx.allocator().free(sum);  // stream-ordered
                     return st;
@@ -476,6 +587,115 @@ struct GemmOp : Operator {
             }
         }
         return k::gemm_tc_run(ctx, g);
+    }
+    // The same product on half-precision pieces (see assign_h2).
+    sage_status compute_h2(const std::vector<Tensor> &x, Context &ctx, Tensor *y, bool emit, bool emit_h2, bool only) {
+        k::H2Gemm g;
+        g.m = m;
+        g.n = n;
+        g.k = k;
+        g.batch = batch;
+        std::shared_ptr<H2Cache> hold_a, hold_b;
+        sage_status st;
+        if (conv) {
+            const Shape &img_shape = x[0].desc.shape;
+            if (!img_shape.has_default_strides() || img_shape.offset % 64 || x[0].data->bytes % 256) return ctx.fail(SAGE_ERR_INVALID, "internal: conv gemm needs a contiguous image");
+            st = storage_h2(ctx, *x[0].data);
+            if (st) return st;
+            hold_a = x[0].data->h2;
+            g.conv = true;
+            g.a.hi = hold_a->pieces.hi + img_shape.offset;
+            g.a.plane = hold_a->pieces.plane;
+            g.a.scale = hold_a->pieces.scale + img_shape.offset / 64;
+            g.img_n = img[0];
+            g.img_h = img[1];
+            g.img_w = img[2];
+            g.img_c = img[3];
+            g.out_h = img[4];
+            g.out_w = img[5];
+            g.win = win;
+        } else {
+            st = make_h2_operand(ctx, x[0], ta, false, &g.a, &hold_a);
+            if (st) return st;
+            if (g.a.nb0 * g.a.nb1 != batch) return ctx.fail(SAGE_ERR_INVALID, "gemm: operand batch extents differ from the operator's");
+        }
+        st = make_h2_operand(ctx, x[1], !tb, true, &g.b, &hold_b);
+        if (st) return st;
+        if (g.b.nb0 * g.b.nb1 != batch) return ctx.fail(SAGE_ERR_INVALID, "gemm: operand batch extents differ from the operator's");
+        g.c = (float *)y->ptr();
+        g.ldc = folded ? ldc : n;
+        g.sc0 = folded ? sc0 : m * n;
+        g.sc1 = folded ? sc1 : 0;
+        g.nbc0 = folded ? nbc0 : batch;
+        k::PlaneOut o;
+        st = attach_forms(ctx, y, emit, emit_h2, &o);
+        if (st) return st;
+        g.c_hi = o.hi;
+        g.c_plane = o.plane;
+        g.h_hi = o.h2;
+        g.h_plane = o.h2_plane;
+        g.h_scale = o.h2_scale;
+        g.naux = naux();
+        g.epilogue = epilogue;
+        long long e_nb0 = batch;
+        st = epilogue_batches(ctx, g.naux, &e_nb0);
+        if (st) return st;
+        if (g.naux > 0 && !folded) g.nbc0 = e_nb0, g.sc1 = m * n * e_nb0;
+        for (int i = 0; i < g.naux; ++i) {
+            st = aux_strides(ctx, x[2 + i], &g.aux[i]);
+            if (st) return st;
+        }
+        // K slices have to be summed before an epilogue is applied: it then runs as a generated map kernel over the sum
+        if (!folded && batch == 1 && (epilogue.empty() || epi_ext == out.shape.extents)) {
+            k::H2Gemm raw = g;
+            raw.epilogue.clear();
+            raw.naux = 0;
+            raw.c_hi = nullptr;
+            raw.h_hi = nullptr;
+            raw.sc0 = m * n;
+            raw.sc1 = 0;
+            raw.nbc0 = 1;
+            const bool plain = epilogue.empty() && !emit && !emit_h2;
+            if (!plain && gemm_h2_slices(ctx, raw) >= 2) {
+                Block *sum = ctx.allocator().alloc((size_t)(m * n) * sizeof(float));
+                if (sum) {
+                    raw.c = reinterpret_cast<float *>(sum->ptr);
+                    st = k::gemm_h2_run(ctx, raw);
+                    if (!st) {
+                        std::vector<MapOperand> operands(1 + (size_t)g.naux);
+                        operands[0].dtype = SAGE_F32;
+                        operands[0].ptr = raw.c;
+                        operands[0].view = Tensor().with_shape(Shape(out.shape.extents)).dims();
+                        for (int i = 0; i < g.naux; ++i) {
+                            operands[1 + i].dtype = x[2 + i].desc.dtype;
+                            operands[1 + i].ptr = x[2 + i].ptr();
+                            operands[1 + i].view = x[2 + i].dims();
+                        }
+                        st = map_launch(ctx, epilogue.empty() ? "x0" : epilogue, operands, SAGE_F32, y->ptr(), out.shape.rank(), out.shape.extents.data(), &epi_cache, o);
+                    }
+                    ctx.allocator().free(sum);  // stream-ordered
+                    return st;
+                }
+            }
+        }
+        if (only) {
+            g.c = nullptr;
+            y->data->planes_only = true;
+        }
+        return k::gemm_h2_run(ctx, g);
+    }
+    // The epilogue's batch decomposition: the axes of epi_ext tagged batch low / high.
+    sage_status epilogue_batches(Context &ctx, int count, long long *e_nb0) const {
+        if (count == 0) return SAGE_OK;
+        *e_nb0 = 1;
+        bool any_hi = false;
+        for (size_t d = 0; d < epi_ext.size(); ++d) {
+            if (epi_group[d] == GBatchLo) *e_nb0 *= epi_ext[d];
+            if (epi_group[d] == GBatchHi && epi_ext[d] > 1) any_hi = true;
+        }
+        if (!any_hi && *e_nb0 != batch) return ctx.fail(SAGE_ERR_INVALID, "internal: gemm epilogue batch groups do not cover the batch");
+        if (folded && nbc0 != *e_nb0 && batch > 1) return ctx.fail(SAGE_ERR_INVALID, "internal: gemm epilogue and store pattern split the batch differently");
+        return SAGE_OK;
     }
     MapCache epi_cache;  // the epilogue as a map kernel, for products that are cut into K slices
 
@@ -503,44 +723,96 @@ struct GemmOp : Operator {
         return SAGE_OK;
     }
 
-    sage_status compute_attention(const std::vector<Tensor> &x, Context &ctx, Tensor *y, bool emit, bool only) {
+    // An operand of the fused attention: rows = tokens, head columns contiguous.  Straight from the pieces of its storage
+    // when each of its rows lies inside one group of 64, else gathered (a scale per row).  `trans`: stored with the tokens last.
+    static sage_status attention_operand(Context &ctx, const Tensor &t, bool trans, k::AttnOperand *op, std::shared_ptr<H2Cache> *hold) {
+        const Shape &sh = t.desc.shape;
+        const int r = sh.rank(), da = trans ? r - 2 : r - 1, ta_ = trans ? r - 1 : r - 2;
+        const long long d = sh.extents[da], rows = sh.extents[ta_];
+        BatchLevels bl;
+        if (!collapse_batch(sh, r - 2, &bl)) return ctx.fail(SAGE_ERR_UNSUPPORTED, "attention: batch axes of an operand do not collapse to two levels");
+        Storage &st = *t.data;
+        op->nb0 = bl.n[0];
+        op->nb1 = bl.n[1];
+        if (attention_view_direct(sh, trans) && st.bytes % 256 == 0) {
+            sage_status s = storage_h2(ctx, st);
+            if (s) return s;
+            *hold = st.h2;
+            op->hi = st.h2->pieces.hi + sh.offset;
+            op->plane = st.h2->pieces.plane;
+            op->ld = rows == 1 ? 64 : sh.strides[ta_];
+            op->sb0 = bl.s[0];
+            op->sb1 = bl.s[1];
+            op->scale = st.h2->pieces.scale;
+            op->s_off = sh.offset;
+            op->s_sb0 = bl.s[0];
+            op->s_sb1 = bl.s[1];
+            op->s_row = op->ld / 64;
+            op->s_shift = 6;
+            return SAGE_OK;
+        }
+        if (st.planes_only) return ctx.fail(SAGE_ERR_INVALID, "internal: a tensor without fp32 values reached an attention operand that has to be gathered");
+        auto fresh = std::make_shared<H2Cache>();
+        fresh->alloc = ctx.allocator_ptr();
+        k::SplitView v;
+        v.nb0 = bl.n[0];
+        v.nb1 = bl.n[1];
+        v.sb0 = bl.s[0];
+        v.sb1 = bl.s[1];
+        v.rows = rows;
+        v.cols = d;
+        v.ld = sh.strides[ta_];
+        v.col_stride = sh.strides[da];
+        sage_status s = k::split_h2_view(ctx, (const float *)t.ptr(), v, false, &fresh->pieces);
+        if (s) return s;
+        *hold = fresh;
+        op->hi = fresh->pieces.hi;
+        op->plane = fresh->pieces.plane;
+        op->ld = fresh->pieces.pitch;
+        op->sb0 = rows * op->ld;
+        op->sb1 = bl.n[0] * op->sb0;
+        op->scale = fresh->pieces.scale;
+        op->s_sb0 = rows;
+        op->s_sb1 = bl.n[0] * rows;
+        op->s_row = 1;
+        return SAGE_OK;
+    }
+    static bool attention_view_direct(const Shape &sh, bool trans) {
+        const int r = sh.rank(), da = trans ? r - 2 : r - 1, ta_ = trans ? r - 1 : r - 2;
+        const long long d = sh.extents[da];
+        BatchLevels bl;
+        if (sh.strides[da] != 1 || d % 8 || 64 % d || sh.offset % d || !collapse_batch(sh, r - 2, &bl)) return false;
+        if (sh.extents[ta_] > 1 && (sh.strides[ta_] <= 0 || sh.strides[ta_] % 64)) return false;
+        for (int l = 0; l < 2; ++l)
+            if (bl.n[l] > 1 && (bl.s[l] <= 0 || bl.s[l] % d)) return false;
+        return true;
+    }
+    // Operands in the order Q, V, K: are their tokens the last axis?
+    bool attention_trans(int idx) const { return idx == 0 ? score_ta : idx == 1 ? tb : !score_tb; }
+
+    sage_status compute_attention(const std::vector<Tensor> &x, Context &ctx, Tensor *y, bool emit, bool emit_h2, bool only) {
         k::TcAttn a;
         a.lq = m;
         a.lk = k;
         a.d = n;
         a.batch = batch;
-        std::shared_ptr<SplitCache> hold_q, hold_k, hold_v;
-        bool sw_q = false, sw_k = false, sw_v = false;
-        sage_status st = make_operand(ctx, x[0], &a.q, &sw_q, &hold_q);
-        if (!st) st = make_operand(ctx, x[2], &a.k, &sw_k, &hold_k);
-        if (!st) st = make_operand(ctx, x[1], &a.v, &sw_v, &hold_v);
+        std::shared_ptr<H2Cache> hold_q, hold_k, hold_v;
+        sage_status st = attention_operand(ctx, x[0], attention_trans(0), &a.q, &hold_q);
+        if (!st) st = attention_operand(ctx, x[2], attention_trans(2), &a.k, &hold_k);
+        if (!st) st = attention_operand(ctx, x[1], attention_trans(1), &a.v, &hold_v);
         if (st) return st;
-        a.q_kmajor = (!score_ta) != sw_q;  // Q lies as [queries, head columns] unless transposed
-        a.k_kmajor = score_tb != sw_k;     // K as operand B of Q K: [head columns, keys] unless transposed
-        a.v_kmajor = tb != sw_v;           // V as operand B of P V: [keys, head columns] unless transposed
         if (a.q.nb0 * a.q.nb1 != batch || a.k.nb0 * a.k.nb1 != batch || a.v.nb0 * a.v.nb1 != batch)
             return ctx.fail(SAGE_ERR_INVALID, "attention: operand batch extents differ from the operator's");
         a.o = (float *)y->ptr();
-        if (folded) {
-            a.ldo = ldc;
-            a.so0 = sc0;
-            a.so1 = sc1;
-            a.nbo0 = nbc0;
-        } else {
-            a.ldo = n;
-            a.so0 = m * n;
-            a.so1 = 0;
-            a.nbo0 = batch;
-        }
-        if (emit) {
-            st = storage_planes_attach(ctx, *y->data);
-            if (st) return st;
-            a.o_hi = y->data->split->planes.planes + y->desc.shape.offset;
-            a.o_plane = y->data->split->plane;
-            if (only) {
-                a.o = nullptr;
-                y->data->planes_only = true;
-            }
+        a.ldo = folded ? ldc : n;
+        a.so0 = folded ? sc0 : m * n;
+        a.so1 = folded ? sc1 : 0;
+        a.nbo0 = folded ? nbc0 : batch;
+        st = attach_forms(ctx, y, emit, emit_h2, &a.out);
+        if (st) return st;
+        if (only) {
+            a.o = nullptr;
+            y->data->planes_only = true;
         }
         a.naux = naux();
         a.epilogue = epilogue;
@@ -752,8 +1024,10 @@ std::shared_ptr<Operator> gemm_with_attention(const Operator &outer_op, const Op
     auto sc = lowered_clone(*s);
     if (c->batch != sc->batch || c->m != sc->m || c->k != sc->n || cols != sc->n || rows != sc->batch * sc->m) return nullptr;
     if (!k::attention_tc_shape_ok(c->m, c->k, c->n, c->batch) || sc->k != c->n) return nullptr;  // queries and values share the head width here
-    for (const TensorDesc &d : {sc->in[0], sc->in[1], c->in[1]})
-        if (d.dtype != SAGE_F32 || !gemm_operand_view_ok(d.shape)) return nullptr;
+    for (const TensorDesc &d : {sc->in[0], sc->in[1], c->in[1]}) {
+        BatchLevels bl;
+        if (d.dtype != SAGE_F32 || !collapse_batch(d.shape, d.shape.rank() - 2, &bl)) return nullptr;
+    }
     c->attn = true;
     c->score_ta = sc->ta;
     c->score_tb = sc->tb;
@@ -810,11 +1084,59 @@ std::shared_ptr<Operator> gemm_with_im2col(const Operator &op, const Operator &i
 
 // Will operand `idx` be read straight from whole-storage planes (never through the fp32 buffer)?
 bool is_grouped_gemm_op(const Operator &op);
+bool grouped_gemm_is_h2(const Operator &op);
+std::shared_ptr<Operator> grouped_gemm_on_h2(const Operator &op);
 bool gemm_operand_static_direct(const Operator &op, int idx) {
-    if (is_grouped_gemm_op(op)) return idx == 0 && gemm_operand_view_ok(op.in[0].shape);
+    if (is_grouped_gemm_op(op)) return idx == 0 && (grouped_gemm_is_h2(op) ? h2_view_ok(op.in[0].shape, false) : gemm_operand_view_ok(op.in[0].shape));
     const GemmOp *g = as_gemm(op);
+    if (g && g->attn) return idx >= 0 && idx < 3 && GemmOp::attention_view_direct(g->in[idx].shape, g->attention_trans(idx));
+    if (g && g->h2) return idx == 0 && (g->conv || h2_view_ok(g->in[0].shape, g->ta));
     if (g && g->conv && idx == 0) return g->conv_implicit() && !g->conv_raw();  // planes only when the kernel does not split the image itself
-    return g && idx >= 0 && idx < (g->attn ? 3 : 2) && gemm_operand_view_ok(g->in[idx].shape);
+    return g && idx >= 0 && idx < 2 && gemm_operand_view_ok(g->in[idx].shape);
+}
+
+// ---- which products run on half-precision pieces (session.cc: assign_h2)
+// A product the tensor cores run whose operand A has its contraction axis across its rows (a weight gradient) reads tf32
+// planes, and then so do its operands' other readers: a result in both forms would cost more than the faster product gains.
+bool gemm_needs_tf32(const Operator &op, bool tc_enabled) {
+    const GemmOp *g = as_gemm(op);
+    if (!g || g->attn || g->conv || !gemm_runs_on_tc(op, tc_enabled)) return false;
+    const Shape &a = g->in[0].shape;
+    const int r = a.rank(), ka = g->ta ? r - 2 : r - 1;
+    return a.strides[ka] != 1;
+}
+// This product on half-precision pieces, or null.  `a_given`: operand A is an input of the program (it may be gathered).
+std::shared_ptr<Operator> gemm_on_h2(const Operator &op, bool a_given, bool tc_enabled) {
+    if (is_grouped_gemm_op(op)) return grouped_gemm_on_h2(op);
+    const GemmOp *g = as_gemm(op);
+    if (!g || g->attn || g->row_softmax || g->h2 || !gemm_runs_on_tc(op, tc_enabled)) return nullptr;
+    auto c = lowered_clone(*g);
+    if (c->conv) {
+        k::H2Gemm probe;
+        probe.img_n = c->img[0];
+        probe.img_h = c->img[1];
+        probe.img_w = c->img[2];
+        probe.img_c = c->img[3];
+        probe.out_h = c->img[4];
+        probe.out_w = c->img[5];
+        probe.win = c->win;
+        if (!c->conv_implicit() || c->conv_raw() || !k::conv_h2_ok(probe)) return nullptr;
+    } else if (!h2_view_ok(c->in[0].shape, c->ta) && !a_given) {
+        return nullptr;
+    }
+    c->h2 = true;
+    return c;
+}
+bool gemm_is_h2(const Operator &op) {  // reads its operands in half-precision pieces
+    const GemmOp *g = as_gemm(op);
+    return (g && (g->h2 || g->attn)) || grouped_gemm_is_h2(op);
+}
+// Does an operator that runs on half-precision pieces write its result in them?  (Whole groups of 64 columns.)
+bool gemm_emits_h2(const Operator &op) {
+    const GemmOp *g = as_gemm(op);
+    if (!g) return grouped_gemm_is_h2(op) && op.out.shape.extents.back() % 64 == 0;
+    if (!(g->h2 || g->attn) || g->n % 64) return false;
+    return !g->folded || (g->ldc % 64 == 0 && g->sc0 % 64 == 0 && g->sc1 % 64 == 0);
 }
 
 std::string describe_gemm(const Operator &op) {
@@ -838,6 +1160,7 @@ std::string describe_gemm(const Operator &op) {
 struct GroupedGemmOp : Operator {
     int groups = 0;
     bool ta = false, tb = false, has_bias = false;
+    bool h2 = false;       // on half-precision pieces
     long long m = 0, n = 0, k = 0;
     std::string epilogue;  // over x0 (product) and, with has_bias, x1 (the bias row)
 
@@ -865,13 +1188,38 @@ struct GroupedGemmOp : Operator {
     }
 
     sage_status compute(const std::vector<Tensor> &x, Context &ctx, Tensor *y) override {
-        const bool emit = ctx.hint_emit_planes, only = emit && ctx.hint_planes_only;
-        ctx.hint_emit_planes = ctx.hint_planes_only = false;
+        const bool emit = ctx.hint_emit_planes, emit_h2 = ctx.hint_emit_h2, only = (emit || emit_h2) && ctx.hint_planes_only;
+        ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = false;
         sage_status st = Tensor::uninit(ctx, out, y);
         if (st) return st;
-        const long long wsize = k * n;
-        // ---- weights: [G] planes of K x N (or N x K), hi plane then lo plane
-        if (!same_key(weights.get(), x, 1, groups)) {
+        const long long wsize = k * n, pitch = (k + 7) / 8 * 8, hsize = n * pitch;
+        // ---- weights in half-precision pieces: [G][N][pitch] hi, the same lo, [G][N] scales
+        if (h2 && !same_key(weights.get(), x, 1, groups)) {
+            std::unique_ptr<Concat> c(new Concat());
+            c->alloc = ctx.allocator_ptr();
+            c->block = ctx.allocator().alloc((size_t)groups * hsize * 4 + (size_t)groups * n * 4);
+            if (!c->block) return ctx.fail(SAGE_ERR_OOM, "out of memory for the grouped gemm's weights");
+            for (int i = 0; i < groups; ++i) {
+                const Tensor &w = x[1 + i];
+                if (!w.desc.shape.has_default_strides()) return ctx.fail(SAGE_ERR_INVALID, "internal: grouped gemm weight is not contiguous");
+                k::SplitView v;
+                v.rows = n;
+                v.cols = k;
+                v.ld = tb ? k : 1;
+                v.col_stride = tb ? 1 : n;
+                k::H2Split to;
+                to.hi = reinterpret_cast<unsigned short *>(c->block->ptr) + i * hsize;
+                to.plane = groups * hsize;
+                to.pitch = pitch;
+                to.scale = reinterpret_cast<float *>(c->block->ptr + (size_t)groups * hsize * 4) + i * n;
+                st = k::split_h2_rows_at(ctx, (const float *)w.ptr(), v, to);
+                if (st) return st;
+                c->key.push_back({w.data.get(), w.data->version});
+            }
+            weights = std::move(c);
+        }
+        // ---- ... as tf32 planes: [G] planes of K x N (or N x K), hi plane then lo plane
+        if (!h2 && !same_key(weights.get(), x, 1, groups)) {
             std::unique_ptr<Concat> c(new Concat());
             c->alloc = ctx.allocator_ptr();
             c->block = ctx.allocator().alloc((size_t)groups * wsize * 2 * sizeof(float));
@@ -911,6 +1259,52 @@ struct GroupedGemmOp : Operator {
             }
             biases = std::move(c);
         }
+        if (h2) {
+            k::H2Gemm g;
+            g.m = m;
+            g.n = n;
+            g.k = k;
+            g.batch = groups;
+            std::shared_ptr<H2Cache> hold;
+            st = make_h2_operand(ctx, x[0], ta, false, &g.a, &hold);
+            if (st) return st;
+            if (g.a.nb0 * g.a.nb1 != 1) return ctx.fail(SAGE_ERR_INVALID, "internal: grouped gemm operand has a batch");
+            g.a.bcast = true;
+            g.b.hi = reinterpret_cast<const unsigned short *>(weights->block->ptr);
+            g.b.plane = groups * hsize;
+            g.b.ld = pitch;
+            g.b.rows = n;
+            g.b.nb0 = groups;
+            g.b.sb0 = hsize;
+            g.b.scale = reinterpret_cast<const float *>(weights->block->ptr + (size_t)groups * hsize * 4);
+            g.b.s_row = 1;
+            g.b.s_b0 = n;
+            g.c = (float *)y->ptr();
+            g.ldc = n;
+            g.sc0 = m * n;
+            g.nbc0 = groups;
+            k::PlaneOut o;
+            st = attach_forms(ctx, y, emit, emit_h2, &o);
+            if (st) return st;
+            g.c_hi = o.hi;
+            g.c_plane = o.plane;
+            g.h_hi = o.h2;
+            g.h_plane = o.h2_plane;
+            g.h_scale = o.h2_scale;
+            if (only) {
+                g.c = nullptr;
+                y->data->planes_only = true;
+            }
+            g.epilogue = epilogue;
+            if (has_bias) {
+                g.naux = 1;
+                g.aux[0].ptr = reinterpret_cast<const float *>(biases->block->ptr);
+                g.aux[0].s0 = n;
+                g.aux[0].sc = 1;
+            }
+            return k::gemm_h2_run(ctx, g);
+        }
+        if (emit_h2) return ctx.fail(SAGE_ERR_INVALID, "internal: the tf32 product does not write half-precision pieces");
         k::TcGemm g;
         g.m = m;
         g.n = n;
@@ -971,6 +1365,28 @@ struct SlabOp : Operator {
 
 bool is_slab_op(const Operator &op) { return dynamic_cast<const SlabOp *>(&op) != nullptr; }
 bool is_grouped_gemm_op(const Operator &op) { return dynamic_cast<const GroupedGemmOp *>(&op) != nullptr; }
+
+bool grouped_gemm_is_h2(const Operator &op) {
+    const GroupedGemmOp *g = dynamic_cast<const GroupedGemmOp *>(&op);
+    return g && g->h2;
+}
+std::shared_ptr<Operator> grouped_gemm_on_h2(const Operator &op) {
+    const GroupedGemmOp *g = dynamic_cast<const GroupedGemmOp *>(&op);
+    if (!g || g->h2 || g->ta || !h2_view_ok(g->in[0].shape, false)) return nullptr;
+    auto c = std::make_shared<GroupedGemmOp>();
+    c->groups = g->groups;
+    c->ta = g->ta;
+    c->tb = g->tb;
+    c->has_bias = g->has_bias;
+    c->m = g->m;
+    c->n = g->n;
+    c->k = g->k;
+    c->epilogue = g->epilogue;
+    c->in = g->in;
+    c->out = g->out;
+    c->h2 = true;
+    return c;
+}
 
 // Can this lowered GEMM join a group?  Fills a key that is equal for GEMMs that may share a launch
 // (same A view, same shape and transposes, same epilogue text); the caller adds A's identity.

@@ -49,7 +49,9 @@ std::string map_expr_text(const MapExpr &e) {
     return "";
 }
 
-sage_status storage_planes_attach(Context &ctx, Storage &st);  // ops_gemm.cc
+// ops_gemm.cc
+sage_status storage_planes_attach(Context &ctx, Storage &st);
+sage_status storage_h2_attach(Context &ctx, Storage &st);
 
 struct MapOp : Operator {
     MapExpr expr;
@@ -63,17 +65,23 @@ struct MapOp : Operator {
     std::vector<Var> grad(const std::vector<Var> &x, const Var &y, const Var &gy) override;
 
     sage_status compute(const std::vector<Tensor> &x, Context &ctx, Tensor *y) override {
-        const bool emit = ctx.hint_emit_planes && out.dtype == SAGE_F32;
-        ctx.hint_emit_planes = ctx.hint_planes_only = false;
+        const bool emit = ctx.hint_emit_planes && out.dtype == SAGE_F32, emit_h2 = ctx.hint_emit_h2 && out.dtype == SAGE_F32;
+        ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = false;
         sage_status st = Tensor::uninit(ctx, out, y);
         if (st) return st;
-        float *hi = nullptr;
-        long long plane = 0;
-        if (emit) {  // a tensor-core GEMM reads y next: the kernel writes its tf32 planes as well
+        k::PlaneOut planes;
+        if (emit) {  // a tensor-core GEMM reads y next: the kernel writes the form it reads as well
             st = storage_planes_attach(ctx, *y->data);
             if (st) return st;
-            hi = y->data->split->planes.planes + y->desc.shape.offset;
-            plane = y->data->split->plane;
+            planes.hi = y->data->split->planes.planes + y->desc.shape.offset;
+            planes.plane = y->data->split->plane;
+        }
+        if (emit_h2) {
+            st = storage_h2_attach(ctx, *y->data);
+            if (st) return st;
+            planes.h2 = y->data->h2->pieces.hi;
+            planes.h2_plane = y->data->h2->pieces.plane;
+            planes.h2_scale = y->data->h2->pieces.scale;
         }
         if (text.empty()) text = map_expr_text(expr);
         std::vector<MapOperand> operands(x.size());
@@ -82,7 +90,7 @@ struct MapOp : Operator {
             operands[i].ptr = x[i].ptr();
             operands[i].view = x[i].dims();
         }
-        return map_launch(ctx, text, operands, out.dtype, y->ptr(), out.shape.rank(), out.shape.extents.data(), &cache, hi, plane);
+        return map_launch(ctx, text, operands, out.dtype, y->ptr(), out.shape.rank(), out.shape.extents.data(), &cache, planes);
     }
 };
 
@@ -90,6 +98,8 @@ bool map_op_emits_planes(const Operator &op) {
     const MapOp *m = dynamic_cast<const MapOp *>(&op);
     return m && m->out.dtype == SAGE_F32 && !m->in.empty();
 }
+
+bool map_op_emits_h2(const Operator &op) { return map_op_emits_planes(op) && op.out.shape.size() % 64 == 0; }
 
 const MapExpr *map_expr_of(const Operator &op) {
     const MapOp *m = dynamic_cast<const MapOp *>(&op);

@@ -8,7 +8,10 @@
 namespace sage {
 using namespace ops;
 
-sage_status storage_planes_attach(Context &ctx, Storage &st);  // ops_gemm.cc
+// ops_gemm.cc
+sage_status storage_planes_attach(Context &ctx, Storage &st);
+sage_status storage_h2_attach(Context &ctx, Storage &st);
+sage_status storage_h2(Context &ctx, Storage &st);
 
 enum RowKind { RSoftmax, RLse, RLayerNorm };
 
@@ -26,30 +29,38 @@ struct RowOp : Operator {
     sage_status compute(const std::vector<Tensor> &x, Context &ctx, Tensor *y) override {
         if (!x[0].desc.shape.has_default_strides())
             return ctx.fail(SAGE_ERR_INVALID, std::string(name()) + ": input is not contiguous");
-        const bool emit = ctx.hint_emit_planes && kind != RLse, only = emit && ctx.hint_planes_only;
-        ctx.hint_emit_planes = ctx.hint_planes_only = false;
+        const float *xp = (const float *)x[0].ptr();
+        const bool emit = ctx.hint_emit_planes && kind != RLse, want_h2 = ctx.hint_emit_h2 && kind != RLse;
+        const bool emit_h2 = want_h2 && k::rows_write_pieces(xp, cols);
+        const bool only = (emit || want_h2) && ctx.hint_planes_only && emit_h2 == want_h2;
+        ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = false;
         sage_status st = Tensor::uninit(ctx, out, y);
         if (st) return st;
-        const float *xp = (const float *)x[0].ptr();
         float *yp = (float *)y->ptr();
-        float *hi = nullptr;
-        long long plane = 0;
-        if (emit) {  // a tensor-core GEMM reads y next: write its tf32 planes in the same pass
+        k::PlaneOut planes;
+        if (emit) {  // a tensor-core GEMM reads y next: write the form it reads in the same pass
             st = storage_planes_attach(ctx, *y->data);
             if (st) return st;
-            hi = y->data->split->planes.planes + y->desc.shape.offset;
-            plane = y->data->split->plane;
-            if (only) {
-                yp = nullptr;
-                y->data->planes_only = true;
-            }
+            planes.hi = y->data->split->planes.planes + y->desc.shape.offset;
+            planes.plane = y->data->split->plane;
+        }
+        if (emit_h2) {
+            st = storage_h2_attach(ctx, *y->data);
+            if (st) return st;
+            planes.h2 = y->data->h2->pieces.hi;
+            planes.h2_plane = y->data->h2->pieces.plane;
+            planes.h2_scale = y->data->h2->pieces.scale;
+        }
+        if (only) {
+            yp = nullptr;
+            y->data->planes_only = true;
         }
         switch (kind) {
-        case RSoftmax: return k::softmax_rows(ctx, xp, yp, rows, cols, hi, plane);
+        case RSoftmax: return k::softmax_rows(ctx, xp, yp, rows, cols, planes);
         case RLse: return k::lse_rows(ctx, xp, yp, rows, cols);
         case RLayerNorm:
             return k::layernorm_rows(ctx, xp, yp, rows, cols, (const float *)x[1].ptr(), x[1].desc.shape.size() == 1 ? 0 : 1,
-                                     (const float *)x[2].ptr(), x[2].desc.shape.size() == 1 ? 0 : 1, eps, hi, plane);
+                                     (const float *)x[2].ptr(), x[2].desc.shape.size() == 1 ? 0 : 1, eps, planes);
         }
         return SAGE_ERR_INVALID;
     }
@@ -66,6 +77,10 @@ bool row_op_is_softmax(const Operator &op, long long *rows, long long *cols) {
 bool row_op_emits_planes(const Operator &op) {
     const RowOp *r = dynamic_cast<const RowOp *>(&op);
     return r && r->kind != RLse;
+}
+bool row_op_emits_h2(const Operator &op) {
+    const RowOp *r = dynamic_cast<const RowOp *>(&op);
+    return r && r->kind != RLse && r->cols % 64 == 0;
 }
 
 // True when `axes` are exactly the last axes of x and x is float + contiguous; fills rows/cols.

@@ -26,7 +26,8 @@ struct Node {
     int slot = -1;                 // ... computed by the program or evaluated before it: its place in a scheduled run
     std::shared_ptr<Operator> op;  // operation
     std::vector<Node> args;
-    bool emit_planes = false;      // a tensor-core GEMM reads the result: ask the operator for its tf32 planes
+    bool emit_planes = false;      // a tensor-core GEMM reads the result: ask the operator for its tf32 planes ...
+    bool emit_h2 = false;          // ... or for its half-precision pieces
     std::shared_ptr<Node> shared;  // a node several parents read (a grouped GEMM): evaluated once per routine run,
                                    // and passed to `op` as its only operand
     bool visited = false;          // traversal mark for shared nodes
@@ -61,6 +62,12 @@ bool gemm_operand_static_direct(const Operator &op, int idx);
 bool gemm_group_key(const Operator &op, std::string *key);
 std::shared_ptr<Operator> make_grouped_gemm(const std::vector<const Operator *> &members);
 std::shared_ptr<Operator> make_slab(const Operator &grouped, int index, const TensorDesc &member_out);
+bool gemm_needs_tf32(const Operator &op, bool tc_enabled);
+std::shared_ptr<Operator> gemm_on_h2(const Operator &op, bool a_given, bool tc_enabled);
+bool gemm_is_h2(const Operator &op);
+bool gemm_emits_h2(const Operator &op);
+bool row_op_emits_h2(const Operator &op);
+bool map_op_emits_h2(const Operator &op);
 std::string describe_gemm(const Operator &op);  // "{epilogue}" / "[store]" of a lowered GEMM, else empty
 
 static bool row_programs_enabled() {
@@ -408,6 +415,42 @@ bool map_op_emits_planes(const Operator &op);
 static bool can_emit_planes(const Operator &op, bool tc) {
     return gemm_runs_on_tc(op, tc) || row_op_emits_planes(op) || is_grouped_gemm_op(op) || (tc && map_op_emits_planes(op));
 }
+static bool can_emit_h2(const Operator &op) { return gemm_emits_h2(op) || row_op_emits_h2(op) || map_op_emits_h2(op); }
+
+// Products with weights run on half-precision pieces, unless the program also multiplies by the transposes of its activations (training):
+// then everything keeps to tf32 planes.
+static bool any_needs_tf32(const Node &n, bool tc) {
+    if (n.is_data) return false;
+    if (gemm_needs_tf32(*n.op, tc) || (n.shared && any_needs_tf32(*n.shared, tc))) return true;
+    for (const Node &a : n.args)
+        if (any_needs_tf32(a, tc)) return true;
+    return false;
+}
+// The same choice whether operand A comes from the product's own routine or from another one: which values are kept must not
+// change what is computed.
+static void assign_h2(Node &n, bool tc, Program &p, std::unordered_set<Origin *> *done);
+static void assign_h2(Routine &r, bool tc, Program &p, std::unordered_set<Origin *> *done) {
+    if (!r.row && done->insert(r.output.key()).second) assign_h2(r.root, tc, p, done);
+}
+static void assign_h2(Node &n, bool tc, Program &p, std::unordered_set<Origin *> *done) {
+    if (n.is_data) return;
+    if (n.shared) assign_h2(*n.shared, tc, p, done);
+    for (Node &a : n.args) assign_h2(a, tc, p, done);
+    if (n.args.size() < 2 || !(is_gemm_op(*n.op) || is_grouped_gemm_op(*n.op))) return;
+    const Node *w = skip_views(&n.args[1]);
+    if (!w->is_data || w->var.is_op()) return;
+    const Node *a = skip_views(&n.args[0]);
+    const bool given = a->is_data && !a->var.is_op();
+    for (int hops = 0; a->is_data && a->var.is_op() && hops < 8; ++hops) {
+        auto it = p.routines.find(a->var.key());
+        if (it == p.routines.end() || it->second.row) break;
+        assign_h2(it->second, tc, p, done);
+        a = skip_views(&it->second.root);
+    }
+    // a producer that can only write tf32 planes (a product of two results) keeps its reader on them
+    if (!a->is_data && !can_emit_h2(*a->op) && can_emit_planes(*a->op, tc)) return;
+    if (std::shared_ptr<Operator> op = gemm_on_h2(*n.op, given, tc)) n.op = op;
+}
 
 // GEMMs of one routine that multiply the same A (same leaf, same view) by different weights, with
 // the same shape and epilogue, become one grouped launch; each member turns into a slab view of the
@@ -463,24 +506,25 @@ static void group_gemms(Node &root) {
     }
 }
 
-static void mark_plane_readers(Node &n, bool tc, std::unordered_set<Origin *> *states) {
+static void mark_plane_readers(Node &n, bool tc, std::unordered_set<Origin *> *states, std::unordered_set<Origin *> *h2_states) {
     if (n.is_data) return;
     if (n.shared && !n.shared->visited) {
         n.shared->visited = true;
-        mark_plane_readers(*n.shared, tc, states);
+        mark_plane_readers(*n.shared, tc, states, h2_states);
     }
-    for (Node &a : n.args) mark_plane_readers(a, tc, states);
+    for (Node &a : n.args) mark_plane_readers(a, tc, states, h2_states);
     const bool grouped = is_grouped_gemm_op(*n.op);
     if (!grouped && (!is_gemm_op(*n.op) || !gemm_runs_on_tc(*n.op, tc))) return;
-    for (int idx = 0; idx < (grouped ? 1 : is_attention_op(*n.op) ? 3 : 2); ++idx) {
+    const bool h2 = gemm_is_h2(*n.op);
+    for (int idx = 0; idx < (is_attention_op(*n.op) ? 3 : grouped || h2 ? 1 : 2); ++idx) {
         Node *p = skip_views(&n.args[idx]);
         if (p->is_data) {
-            if (p->var.is_op() && gemm_operand_static_direct(*n.op, idx)) states->insert(p->var.key());
-        } else if (can_emit_planes(*p->op, tc)) {
+            if (p->var.is_op() && gemm_operand_static_direct(*n.op, idx)) (h2 ? h2_states : states)->insert(p->var.key());
+        } else if (h2 ? can_emit_h2(*p->op) : can_emit_planes(*p->op, tc)) {
             // Inside a routine's tree a node has one reader, so this GEMM is the only one — unless the
             // node is shared (a grouped product): then every slab must end in a GEMM operand.
             const bool direct = gemm_operand_static_direct(*n.op, idx);
-            if (direct) p->emit_planes = true;
+            if (direct) (h2 ? p->emit_h2 : p->emit_planes) = true;
             if (p->readers > 0) {
                 if (direct) ++p->gemm_readers;
                 p->planes_only = p->gemm_readers == p->readers;
@@ -699,26 +743,36 @@ static std::unique_ptr<Program> compile(const std::vector<Var> &x, std::vector<V
         p->routines.emplace(node.key(), std::move(r));
     }
     if (pattern) {
-        std::unordered_set<Origin *> plane_states;
+        std::unordered_set<Origin *> plane_states, h2_states;
+        if (tc) {
+            bool tf32 = false;
+            for (auto &kv : p->routines) tf32 = tf32 || (!kv.second.row && any_needs_tf32(kv.second.root, tc));
+            std::unordered_set<Origin *> done;
+            if (!tf32)
+                for (auto &kv : p->routines) assign_h2(kv.second, tc, *p, &done);
+        }
         for (auto &kv : p->routines)
-            if (!kv.second.row) mark_plane_readers(kv.second.root, tc, &plane_states);
-        for (Origin *key : plane_states) {
-            // A state that is only a view of another state (reshape(state)) shares its storage, and planes
-            // belong to the storage: ask the state that really produces the values.
-            auto it = p->routines.find(key);
-            for (int hops = 0; it != p->routines.end() && !it->second.row && hops < 8; ++hops) {
+            if (!kv.second.row) mark_plane_readers(kv.second.root, tc, &plane_states, &h2_states);
+        for (int form = 0; form < 2; ++form) {
+            for (Origin *key : form ? h2_states : plane_states) {
+                // A state that is only a view of another state (reshape(state)) shares its storage, and planes
+                // belong to the storage: ask the state that really produces the values.
+                auto it = p->routines.find(key);
+                for (int hops = 0; it != p->routines.end() && !it->second.row && hops < 8; ++hops) {
+                    Node *root = skip_views(&it->second.root);
+                    if (!root->is_data || !root->var.is_op()) break;
+                    it = p->routines.find(root->var.key());
+                }
+                if (it == p->routines.end()) continue;  // an input of the program: split on first use
+                if (it->second.row) {                   // a row group: the generated kernel writes the planes of that output
+                    for (size_t i = 0; i < it->second.row_outputs.size(); ++i)
+                        if (!form && it->second.row_outputs[i].key() == it->first) (*it->second.row_emit_shared)[i] = 1;
+                    continue;
+                }
                 Node *root = skip_views(&it->second.root);
-                if (!root->is_data || !root->var.is_op()) break;
-                it = p->routines.find(root->var.key());
+                if (!root->is_data && form && can_emit_h2(*root->op)) root->emit_h2 = true;
+                if (!root->is_data && !form && can_emit_planes(*root->op, tc)) root->emit_planes = true;
             }
-            if (it == p->routines.end()) continue;  // an input of the program: split on first use
-            if (it->second.row) {                   // a row group: the generated kernel writes the planes of that output
-                for (size_t i = 0; i < it->second.row_outputs.size(); ++i)
-                    if (it->second.row_outputs[i].key() == it->first) (*it->second.row_emit_shared)[i] = 1;
-                continue;
-            }
-            Node *root = skip_views(&it->second.root);
-            if (!root->is_data && can_emit_planes(*root->op, tc)) root->emit_planes = true;
         }
     }
     p->outputs = y;
@@ -778,9 +832,10 @@ static sage_status run_node(const Node &n, Context &ctx, Session &s, const Value
         if (args[i].desc.shape.extents != n.op->in[i].shape.extents)
             return ctx.fail(SAGE_ERR_INVALID, std::string("operand extents differ from the operator's spec in ") + n.op->name());
     ctx.hint_emit_planes = n.emit_planes;
-    ctx.hint_planes_only = n.emit_planes && n.planes_only;
+    ctx.hint_emit_h2 = n.emit_h2;
+    ctx.hint_planes_only = (n.emit_planes || n.emit_h2) && n.planes_only;
     sage_status st = n.op->compute(args, ctx, out);
-    ctx.hint_emit_planes = ctx.hint_planes_only = false;
+    ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = false;
     return st;
 }
 
@@ -1098,7 +1153,7 @@ static void describe_node(const Node &n, std::string *out) {
     out->append(n.op->name());
     if (const MapExpr *e = map_expr_of(*n.op)) out->append("{" + map_expr_text(*e) + "}");
     out->append(describe_gemm(*n.op));
-    if (n.emit_planes) out->append(n.planes_only ? "=planes" : "+planes");
+    if (n.emit_planes || n.emit_h2) out->append(n.planes_only ? "=planes" : "+planes");
     out->push_back('(');
     if (n.shared) describe_node(*n.shared, out);
     for (size_t i = 0; i < n.args.size(); ++i) {

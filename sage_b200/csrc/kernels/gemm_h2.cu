@@ -12,8 +12,10 @@
 #define SAGE_EPI_COLS 0
 #include "gemm_tc_device.inc"
 #include "gemm_h2_device.inc"
+#include "attn_tc_device.inc"  // AttnParams and the tile constants; the kernel itself is only compiled by NVRTC
 #include "gemm_tc_device_src.h"
 #include "gemm_h2_device_src.h"
+#include "attn_tc_device_src.h"
 
 namespace sage {
 void *driver_symbol(const char *name);  // runtime/context.cc
@@ -218,25 +220,30 @@ size_t split_h2_bytes(long long batches, long long rows, long long cols, bool wh
     return up256(planes) + up256((size_t)(batches * rows * (whole_rows ? 1 : (cols + 63) / 64)) * 4);
 }
 
-sage_status split_h2_view_into(Context &ctx, const float *src, const SplitView &v, bool whole_rows, void *dst, H2Split *out) {
-    const long long batches = v.nb0 * v.nb1;
-    out->pitch = h2_pitch(v.cols);
-    out->plane = batches * v.rows * out->pitch;
-    out->hi = static_cast<unsigned short *>(dst);
-    out->scale = reinterpret_cast<float *>(static_cast<char *>(dst) + up256((size_t)out->plane * 4));
-    ViewP p{src, v.nb0, v.sb0, v.sb1, v.ld, v.col_stride, v.rows, v.cols, out->pitch, out->plane, (int)((v.rows + 63) / 64), (int)((v.cols + 63) / 64), 0};
+static sage_status split_view_to(Context &ctx, const float *src, const SplitView &v, bool whole_rows, const H2Split &out) {
+    ViewP p{src, v.nb0, v.sb0, v.sb1, v.ld, v.col_stride, v.rows, v.cols, out.pitch, out.plane, (int)((v.rows + 63) / 64), (int)((v.cols + 63) / 64), 0};
     p.vec = (v.col_stride == 1 || v.ld == 1) && aligned16(src) && v.sb0 % 4 == 0 && v.sb1 % 4 == 0 && (v.col_stride == 1 ? v.ld % 4 == 0 && v.cols % 4 == 0 : v.col_stride % 4 == 0 && v.rows % 4 == 0);
-    const long long groups = batches * p.row_tiles, blocks = groups * (whole_rows ? 8 : p.col_tiles);
+    const long long groups = v.nb0 * v.nb1 * p.row_tiles, blocks = groups * (whole_rows ? 8 : p.col_tiles);
     if (blocks > 0x7fffffffLL) return ctx.fail(SAGE_ERR_UNSUPPORTED, "split_h2: extents beyond 2^31 tiles");
     ctx.note_launch("split_tf32");  // launch lists have one name for an operand's split
     if (ctx.dry()) return SAGE_OK;
     if (!whole_rows)
-        return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), split_h2_view_kernel, dim3((unsigned)blocks), dim3(256), 0, p, out->hi, out->scale), "split_h2 launch");
+        return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), split_h2_view_kernel, dim3((unsigned)blocks), dim3(256), 0, p, out.hi, out.scale), "split_h2 launch");
     int ctas = 1;
     while (ctas < 8 && ctas * 2 <= p.col_tiles) ctas *= 2;
     const int per = (p.col_tiles + ctas - 1) / ctas;
-    return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), ctas, split_h2_rows_kernel, dim3((unsigned)(groups * ctas)), dim3(256), 0, p, out->hi, out->scale, ctas, per),
+    return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), ctas, split_h2_rows_kernel, dim3((unsigned)(groups * ctas)), dim3(256), 0, p, out.hi, out.scale, ctas, per),
                           "split_h2 rows launch");
+}
+
+sage_status split_h2_rows_at(Context &ctx, const float *src, const SplitView &v, const H2Split &out) { return split_view_to(ctx, src, v, true, out); }
+
+sage_status split_h2_view_into(Context &ctx, const float *src, const SplitView &v, bool whole_rows, void *dst, H2Split *out) {
+    out->pitch = h2_pitch(v.cols);
+    out->plane = v.nb0 * v.nb1 * v.rows * out->pitch;
+    out->hi = static_cast<unsigned short *>(dst);
+    out->scale = reinterpret_cast<float *>(static_cast<char *>(dst) + up256((size_t)out->plane * 4));
+    return split_view_to(ctx, src, v, whole_rows, *out);
 }
 
 sage_status split_h2_view(Context &ctx, const float *src, const SplitView &v, bool whole_rows, H2Split *out) {
@@ -364,24 +371,31 @@ static ColumnPlan plan_columns(const Context &ctx, long long m, long long n, lon
 
 static sage_status gemm_h2_launch(Context &ctx, const H2Gemm &g);
 
-// Split-K: as in gemm_tcgen05.cu, a product with few output tiles and a long K runs as a batch of K slices (multiples of
-// 64) followed by their sum in a fixed order.  Microseconds from measured launches: a K-block takes what its operand
-// bytes take from L2 (64 KB: 1.1 us with all SMs loading), a tile ~5 us beside its K loop, the sum 4 us and its bytes.
+// Split-K: as in gemm_tcgen05.cu, a product with few output tiles and a long K runs in slices of K (a whole number of
+// K-blocks each) followed by their sum in a fixed order.  Microseconds from measured launches: a K-block takes what its
+// operand bytes take from L2 (64 KB: 1.0 us with all SMs loading) but not less than 0.45, a tile ~5 us beside its K loop,
+// the sum 3.5 us and its bytes.  Slices must promise a fifth: they change the order of summation, and nearer to the line than
+// that the estimate says little.
 static int pick_slices(const Context &ctx, const H2Gemm &g) {
     static const bool enabled = !(getenv("SAGE_GEMM_SPLITK") && atoi(getenv("SAGE_GEMM_SPLITK")) == 0);
-    if (!enabled || g.conv || g.batch != 1 || g.naux || !g.epilogue.empty() || !g.c || g.c_hi || g.h_hi || g.ldc != g.n || g.k < 512) return 0;
+    if (!enabled || g.batch != 1 || g.naux || !g.epilogue.empty() || !g.c || g.c_hi || g.h_hi || g.ldc != g.n || g.k < 512) return 0;
+    int wb, rows;
+    if (halo_plan(g, &wb, &rows)) return 0;
     const int ctas = (pairs_on() && g.m > BM) ? 2 : 1;
-    const long long units = ctx.sm_count / ctas;
+    const long long units = ctx.sm_count / ctas, all_kb = (g.k + HK - 1) / HK;
     double best = 1e300, unsplit = 1e300;
     long long best_s = 0;
-    for (long long s = 1; s <= g.k / 256 && s <= 64; ++s) {
-        if (s > 1 && g.k % (64 * s)) continue;
-        const long long kb = (g.k / s + HK - 1) / HK;
+    for (long long s = 1; s <= all_kb / 2 && s <= 64; ++s) {
+        if (g.conv && all_kb % s) continue;  // a convolution has no K-blocks to fill a last slice with
+        const long long kb = (all_kb + s - 1) / s;
+        if (kb * (s - 1) >= all_kb) continue;
         for (int bn : {256, 128, 64}) {
             if (bn > 64 && g.n <= bn / 2) continue;
             const long long tiles = ((g.m + BM * ctas - 1) / (BM * ctas)) * ((g.n + bn - 1) / bn) * s, waves = (tiles + units - 1) / units;
-            double t = (double)waves * ((double)kb * 1.1 * (BM + bn / ctas) / 256.0 + 5.0);
-            if (s > 1) t += 4.0 + (double)(s + 1) * (double)g.m * (double)g.n * 4.0 / 5.0e6;
+            double per = 1.0 * (BM + bn / ctas) / 256.0;
+            if (per < 0.45) per = 0.45;
+            double t = (double)waves * ((double)kb * per + 5.0);
+            if (s > 1) t += 3.5 + (double)(s + 1) * (double)g.m * (double)g.n * 4.0 / 5.0e6;
             if (s == 1 && t < unsplit) unsplit = t;
             if (t < best) {
                 best = t;
@@ -389,7 +403,7 @@ static int pick_slices(const Context &ctx, const H2Gemm &g) {
             }
         }
     }
-    return best_s >= 2 && best <= 0.9 * unsplit ? (int)best_s : 0;
+    return best_s >= 2 && best <= 0.8 * unsplit ? (int)best_s : 0;
 }
 
 int gemm_h2_slices(Context &ctx, const H2Gemm &g) { return pick_slices(ctx, g); }
@@ -397,21 +411,11 @@ int gemm_h2_slices(Context &ctx, const H2Gemm &g) { return pick_slices(ctx, g); 
 sage_status gemm_h2_run(Context &ctx, const H2Gemm &g0, bool no_slices) {
     const int S = no_slices ? 0 : pick_slices(ctx, g0);
     if (S < 2) return gemm_h2_launch(ctx, g0);
-    const long long ks = g0.k / S, mn = g0.m * g0.n;
+    const long long mn = g0.m * g0.n;
     Block *scratch = ctx.allocator().alloc((size_t)S * mn * sizeof(float));
     if (!scratch) return gemm_h2_launch(ctx, g0);  // no room for the partial products: one pass over K
     H2Gemm g = g0;
-    g.batch = S;
-    g.k = ks;
-    for (H2Operand *o : {&g.a, &g.b}) {
-        o->nb0 = S;
-        o->sb0 = ks;
-        o->nb1 = 1;
-        o->sb1 = 0;
-        o->bcast = false;
-    }
-    g.a.s_b0 = ks / HK;
-    g.b.s_b0 = 0;  // B's scales hold for all of K
+    g.slices = S;
     g.c = reinterpret_cast<float *>(scratch->ptr);
     g.sc0 = mn;
     g.sc1 = 0;
@@ -510,6 +514,7 @@ static sage_status gemm_h2_launch(Context &ctx, const H2Gemm &g) {
     int halo_wb = 0, halo_r = 0;
     const bool halo = halo_plan(g, &halo_wb, &halo_r);
     ColumnPlan cols = plan_columns(ctx, g.m, g.n, g.batch, ctas);
+    if (g.slices > 1) cols = plan_columns(ctx, g.m, g.n, g.slices, ctas);
     if (halo) cols = ColumnPlan{g.n <= 64 ? 64 : 128, 0, 0};  // all output channels in one tile: the window is loaded once
     const int bn = cols.bn;
     const int stage_bytes = halo ? 2 * (bn / ctas) * HK * 2 : 2 * BM * HK * 2 + 2 * (bn / ctas) * HK * 2;
@@ -531,8 +536,12 @@ static sage_status gemm_h2_launch(Context &ctx, const H2Gemm &g) {
     p.nbc0 = (int)(g.nbc0 < 1 ? 1 : g.nbc0);
     p.na0 = (int)g.a.nb0;
     p.nb0 = (int)g.b.nb0;
-    p.a_bcast = (g.a.bcast || g.conv) ? 1 : 0;
-    p.b_bcast = g.b.bcast ? 1 : 0;
+    const bool sliced = g.slices > 1;
+    const long long batch = sliced ? g.slices : g.batch, all_kb = (g.k + HK - 1) / HK;
+    p.sliced = sliced ? 1 : 0;
+    p.kb_count = (int)(sliced ? (all_kb + g.slices - 1) / g.slices : all_kb);
+    p.a_bcast = (g.a.bcast || g.conv || sliced) ? 1 : 0;
+    p.b_bcast = (g.b.bcast || sliced) ? 1 : 0;
     p.m = (int)g.m;
     p.n = (int)g.n;
     p.k = (int)g.k;
@@ -542,13 +551,13 @@ static sage_status gemm_h2_launch(Context &ctx, const H2Gemm &g) {
     p.rag_wide = cols.wide;
     p.rag_narrow = cols.narrow;
     p.rag_bn = 192;
-    p.num_tiles = (int)((long long)p.tiles_m * p.tiles_n * g.batch);
+    p.num_tiles = (int)((long long)p.tiles_m * p.tiles_n * batch);
     p.sa = g.a.scale;
     p.sa_row = g.a.s_row;
     p.sa_b0 = g.a.s_b0;
     p.sa_b1 = g.a.s_b1;
     p.sb = g.b.scale;
-    p.sb_batch = g.b.bcast ? 0 : g.b.s_b0;
+    p.sb_batch = p.b_bcast ? 0 : g.b.s_b0;
     p.status = ctx.status_word_dev;
     if (g.conv) {
         p.conv_cb = (int)(g.img_c / HK);
@@ -575,7 +584,8 @@ static sage_status gemm_h2_launch(Context &ctx, const H2Gemm &g) {
         p.tiles_m = (int)((g.img_n * p.halo_rt + ctas - 1) / ctas);
         p.num_tiles = p.tiles_m * p.tiles_n;
     }
-    bool vec = g.n % 4 == 0 && g.ldc % 4 == 0 && g.sc0 % 4 == 0 && g.sc1 % 4 == 0 && (!g.c || aligned16(g.c)) && (!g.c_hi || (aligned16(g.c_hi) && g.c_plane % 4 == 0));
+    const bool vec = g.n % 4 == 0 && g.ldc % 4 == 0 && g.sc0 % 4 == 0 && g.sc1 % 4 == 0 && (!g.c || aligned16(g.c)) && (!g.c_hi || (aligned16(g.c_hi) && g.c_plane % 4 == 0));
+    bool aux_vec = true;
     int rowinv = 0, per_col = 0;
     for (int i = 0; i < g.naux; ++i) {
         TcAux &a = p.aux[i];
@@ -585,11 +595,12 @@ static sage_status gemm_h2_launch(Context &ctx, const H2Gemm &g) {
         a.sr = g.aux[i].sr;
         a.sc = g.aux[i].sc;
         if (a.sc != 0 && a.sc != 1) return ctx.fail(SAGE_ERR_INVALID, "gemm_h2: epilogue operand column stride must be 0 or 1");
-        if (a.sc == 1) vec = vec && aligned16(a.ptr) && a.s0 % 4 == 0 && a.s1 % 4 == 0 && a.sr % 4 == 0;
+        if (a.sc == 1) aux_vec = aux_vec && aligned16(a.ptr) && a.s0 % 4 == 0 && a.s1 % 4 == 0 && a.sr % 4 == 0;
         if (a.sr == 0) rowinv |= 1 << i;
         if (a.sc != 0) per_col |= 1 << i;
     }
     p.vec_ok = vec ? 1 : 0;
+    p.aux_vec = aux_vec ? 1 : 0;
     if (g.h_hi && (!vec || g.n % 64 || g.ldc % 64 || g.sc0 % 64 || g.sc1 % 64 || !aligned16(g.h_hi) || g.h_plane % 8))
         return ctx.fail(SAGE_ERR_INVALID, "gemm_h2: a result in half-precision pieces needs whole groups of 64 columns");
     const int slots = ctx.sm_count / ctas, grid = ctas * (p.num_tiles < slots ? p.num_tiles : slots);
@@ -615,7 +626,7 @@ static sage_status gemm_h2_launch(Context &ctx, const H2Gemm &g) {
         src += kGemmH2DeviceSrc;
         src += "\nextern \"C\" __global__ void __launch_bounds__(sage_tc::kThreads, 1)\n"
                "gemm_tc_h2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_a2,\n"
-               "           const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_b2, const sage_tc::H2Params p) {\n"
+               "           const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_b2, const __grid_constant__ sage_tc::H2Params p) {\n"
                "    sage_tc::gemm_h2_body<" + std::to_string(bn) + ", " + std::to_string(ctas) + ">(&map_a, &map_a2, &map_b, &map_b2, p);\n}\n";
         sage_status st = ctx.module_get(src, &mod);
         if (st) return st;
@@ -645,7 +656,7 @@ static sage_status gemm_h2_launch(Context &ctx, const H2Gemm &g) {
     }
     std::string label;
     if (ctx.verbose_names)
-        label = "gemm_tc_h2[" + std::to_string(g.m) + "x" + std::to_string(g.n) + "x" + std::to_string(g.k) + (g.batch > 1 ? "x" + std::to_string(g.batch) : "") +
+        label = "gemm_tc_h2[" + std::to_string(g.m) + "x" + std::to_string(g.n) + "x" + std::to_string(g.k) + (batch > 1 ? "x" + std::to_string(batch) : "") + (sliced ? "s" : "") +
                 (g.conv ? (halo ? ",conv,taps" : ",conv") : "") + ",bn" + std::to_string(bn) + (cols.narrow ? "/" + std::to_string(cols.wide) + "+" + std::to_string(cols.narrow) + "x192" : "") +
                 (ctas == 2 ? ",pair" : "") + "]o" + std::to_string(out_mask);
     if (plain) {
@@ -661,6 +672,113 @@ static sage_status gemm_h2_launch(Context &ctx, const H2Gemm &g) {
     void *params[5] = {&map_a, &map_a2, &map_b, &map_b2, &p};
     // launch lists have one name for a tensor-core product; verbose ones tell the kernels apart
     return ctx.launch(mod, "gemm_tc_h2", gr, bl, (uint32_t)smem, params, ctx.verbose_names ? label.c_str() : "gemm_tc_3xtf32", true, ctas);
+}
+
+// ---------------------------------------------------------------------------------- fused attention
+bool attention_tc_shape_ok(long long lq, long long lk, long long d, long long batch) {
+    if (lq < 1 || lk < 1 || d < 4 || d > 64 || d % 4 || batch < 1) return false;
+    if (lq > 0x7fffffffLL || lk > 0x7fffffffLL || batch > 0x7fffffffLL) return false;
+    return ((lq + 127) / 128) * batch < 0x7fffffffLL;
+}
+
+sage_status attention_tc_run(Context &ctx, const TcAttn &a) {
+    static PFN_encodeTiled encode = nullptr;
+    if (!ctx.dry() && !encode) {
+        encode = reinterpret_cast<PFN_encodeTiled>(driver_symbol("cuTensorMapEncodeTiled"));
+        if (!encode) return ctx.fail(SAGE_ERR_DEVICE, "cuTensorMapEncodeTiled is not available");
+    }
+    if (!attention_tc_shape_ok(a.lq, a.lk, a.d, a.batch)) return ctx.fail(SAGE_ERR_UNSUPPORTED, "attention_tc: shape not supported");
+    if (a.naux < 0 || a.naux > kMaxAux || (!a.o && !a.out.hi && !a.out.h2)) return ctx.fail(SAGE_ERR_INVALID, "attention_tc: bad description");
+    AttnParams p{};
+    p.o = a.o;
+    p.o_hi = a.out.hi;
+    p.o_plane = a.out.plane;
+    p.o_h2 = a.out.h2;
+    p.o_h2_plane = a.out.h2_plane;
+    p.o_h2_scale = a.out.h2_scale;
+    p.ldo = a.ldo;
+    p.so0 = a.so0;
+    p.so1 = a.so1;
+    p.nbo0 = (int)(a.nbo0 < 1 ? 1 : a.nbo0);
+    p.nq0 = (int)a.q.nb0;
+    p.nk0 = (int)a.k.nb0;
+    p.nv0 = (int)a.v.nb0;
+    p.nbe0 = (int)(a.nbe0 < 1 ? 1 : a.nbe0);
+    p.sq = AttnScale{a.q.scale, a.q.s_off, a.q.s_sb0, a.q.s_sb1, a.q.s_row, a.q.s_shift};
+    p.sk = AttnScale{a.k.scale, a.k.s_off, a.k.s_sb0, a.k.s_sb1, a.k.s_row, a.k.s_shift};
+    p.sv = AttnScale{a.v.scale, a.v.s_off, a.v.s_sb0, a.v.s_sb1, a.v.s_row, a.v.s_shift};
+    p.lq = (int)a.lq;
+    p.lk = (int)a.lk;
+    p.d = (int)a.d;
+    p.tiles_q = (int)((a.lq + kAttnQ - 1) / kAttnQ);
+    p.num_tiles = (int)((long long)p.tiles_q * a.batch);
+    p.from_zero = ctx.opts().ref_compat ? 1 : 0;
+    p.status = ctx.status_word_dev;
+    bool aux_vec = true;
+    const bool vec = a.d % 4 == 0 && a.ldo % 4 == 0 && a.so0 % 4 == 0 && a.so1 % 4 == 0 && (!a.o || aligned16(a.o)) && (!a.out.hi || (aligned16(a.out.hi) && a.out.plane % 4 == 0));
+    int rowinv_mask = 0;  // which operands of the score expression have no row stride: compiled in
+    for (int i = 0; i < a.naux; ++i) {
+        TcAux &x = p.aux[i];
+        x.ptr = a.aux[i].ptr;
+        x.s0 = a.aux[i].s0;
+        x.s1 = a.aux[i].s1;
+        x.sr = a.aux[i].sr;
+        x.sc = a.aux[i].sc;
+        if (x.sc != 0 && x.sc != 1) return ctx.fail(SAGE_ERR_INVALID, "attention_tc: expression operand column stride must be 0 or 1");
+        if (x.sc == 1) aux_vec = aux_vec && aligned16(x.ptr) && x.s0 % 4 == 0 && x.s1 % 4 == 0 && x.sr % 4 == 0;
+        if (x.sr == 0) rowinv_mask |= 1 << i;
+    }
+    p.vec_ok = vec ? 1 : 0;
+    p.aux_vec = aux_vec ? 1 : 0;
+    if (a.out.h2 && (!vec || a.d != 64 || a.ldo % 64 || a.so0 % 64 || a.so1 % 64 || !aligned16(a.out.h2) || a.out.h2_plane % 8))
+        return ctx.fail(SAGE_ERR_INVALID, "attention_tc: a result in half-precision pieces needs whole groups of 64 columns");
+    // Q, the K / V ring, 1 KiB per softmax warp for turning the output round, and the slack for 1024-byte alignment
+    const size_t smem = 2 * (size_t)kAttnQBytes + (size_t)kAttnStages * 4 * kAttnKVBytes + (size_t)kAttnSoftmaxWarps * 1024 + 1024;
+    const int grid = p.num_tiles < ctx.sm_count ? p.num_tiles : ctx.sm_count;
+    const int out_mask = (a.o ? 1 : 0) | (a.out.hi ? 2 : 0) | (a.out.h2 ? 4 : 0);
+    char num[64];
+    snprintf(num, sizeof num, "attention_tc %d %d %d\n", a.naux, rowinv_mask, out_mask);
+    const std::string key = num + a.epilogue;  // the rest of the translation unit is fixed text
+    Module *mod = ctx.module_find(key);
+    if (!mod) {
+        std::string src = map_prelude_text();
+        src += "struct __align__(64) CUtensorMap { unsigned long long opaque[16]; };\n";
+        src += "#define SAGE_EPI_NAUX " + std::to_string(a.naux) + "\n#define SAGE_EPI_ROWINV " + std::to_string(rowinv_mask) + "\n#define SAGE_EPI_OUT " + std::to_string(out_mask) + "\n";
+        src += "#define SAGE_EPI_EXPR(x0, x1, x2, x3) (" + (a.epilogue.empty() ? std::string("x0") : a.epilogue) + ")\n";
+        src += kGemmTcDeviceSrc;
+        src += kGemmH2DeviceSrc;
+        src += kAttnTcDeviceSrc;
+        src += "\nextern \"C\" __global__ void __launch_bounds__(sage_tc::kAttnThreads, 1)\n"
+               "attention_tc_h2(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,\n"
+               "                const __grid_constant__ CUtensorMap map_v, const __grid_constant__ sage_tc::AttnParams p) {\n"
+               "    sage_tc::attn_body(&map_q, &map_k, &map_v, p);\n}\n";
+        sage_status st = ctx.module_get(src, &mod);
+        if (st) return st;
+        ctx.module_remember(key, mod);
+    }
+    CUtensorMap map_q, map_k, map_v;
+    if (!ctx.dry()) {
+        auto map_of = [&](const AttnOperand &o, long long rows, unsigned box, CUtensorMap *map) {
+            H2Operand h;
+            h.hi = o.hi;
+            h.plane = o.plane;
+            h.ld = o.ld;
+            h.rows = rows;
+            h.nb0 = o.nb0;
+            h.nb1 = o.nb1;
+            h.sb0 = o.sb0;
+            h.sb1 = o.sb1;
+            return o.hi && aligned16(o.hi) && o.ld % 8 == 0 && o.plane % 8 == 0 && o.sb0 % 8 == 0 && o.sb1 % 8 == 0 && encode_operand(encode, h, a.d, box, map);
+        };
+        if (!map_of(a.q, a.lq, kAttnQ, &map_q) || !map_of(a.k, a.lk, kAttnKeys, &map_k) || !map_of(a.v, a.lk, kAttnKeys, &map_v))
+            return ctx.fail(SAGE_ERR_INVALID, "attention_tc: operand not addressable by TMA");
+    }
+    std::string label;
+    if (ctx.verbose_names)
+        label = "attention_tc_h2[" + std::to_string(a.lq) + "x" + std::to_string(a.lk) + "x" + std::to_string(a.d) + "x" + std::to_string(a.batch) + "]";
+    const uint32_t gr[3] = {(uint32_t)grid, 1, 1}, bl[3] = {(uint32_t)kAttnThreads, 1, 1};
+    void *params[4] = {&map_q, &map_k, &map_v, &p};
+    return ctx.launch(mod, "attention_tc_h2", gr, bl, (uint32_t)smem, params, ctx.verbose_names ? label.c_str() : "attention_tc_3xtf32", true, 1);
 }
 
 }  // namespace k

@@ -36,9 +36,7 @@
 #include "kernels.h"
 #include "launch.h"
 #include "gemm_tc_device.inc"
-#include "attn_tc_device.inc"  // AttnParams and the tile constants; the kernel itself is only compiled by NVRTC
 #include "gemm_tc_device_src.h"  // generated by the Makefile: the text of gemm_tc_device.inc as kGemmTcDeviceSrc
-#include "attn_tc_device_src.h"  // likewise attn_tc_device.inc as kAttnTcDeviceSrc (compiled by NVRTC only)
 
 namespace sage {
 void *driver_symbol(const char *name);  // runtime/context.cc
@@ -777,106 +775,6 @@ static sage_status gemm_tc_launch(Context &ctx, const TcGemm &g) {
     if (ctx.dry()) return SAGE_OK;
     return ctas == 2 ? launch_static_bn<2>(ctx, bn, map_a, map_a2, map_b, p, grid, smem)
                      : launch_static_bn<1>(ctx, bn, map_a, map_a2, map_b, p, grid, smem);
-}
-
-// ---------------------------------------------------------------------------------- fused attention launcher
-bool attention_tc_shape_ok(long long lq, long long lk, long long d, long long batch) {
-    if (lq < 1 || lk < 1 || d < 4 || d > 64 || d % 4 || batch < 1) return false;
-    if (lq > 0x7fffffffLL || lk > 0x7fffffffLL || batch > 0x7fffffffLL) return false;
-    const long long tiles = ((lq + 127) / 128) * batch;
-    return tiles < 0x7fffffffLL;
-}
-
-sage_status attention_tc_run(Context &ctx, const TcAttn &a) {
-    static PFN_encodeTiled encode = nullptr;
-    if (!ctx.dry() && !encode) {
-        encode = reinterpret_cast<PFN_encodeTiled>(driver_symbol("cuTensorMapEncodeTiled"));
-        if (!encode) return ctx.fail(SAGE_ERR_DEVICE, "cuTensorMapEncodeTiled is not available");
-    }
-    if (!attention_tc_shape_ok(a.lq, a.lk, a.d, a.batch)) return ctx.fail(SAGE_ERR_UNSUPPORTED, "attention_tc: shape not supported");
-    if (a.naux < 0 || a.naux > kMaxAux || (!a.o && !a.o_hi)) return ctx.fail(SAGE_ERR_INVALID, "attention_tc: bad description");
-    AttnParams p;
-    p.o = a.o;
-    p.o_hi = a.o_hi;
-    p.o_plane = a.o_plane;
-    p.ldo = a.ldo;
-    p.so0 = a.so0;
-    p.so1 = a.so1;
-    p.nbo0 = (int)(a.nbo0 < 1 ? 1 : a.nbo0);
-    p.nq0 = (int)a.q.nb0;
-    p.nk0 = (int)a.k.nb0;
-    p.nv0 = (int)a.v.nb0;
-    p.nbe0 = (int)(a.nbe0 < 1 ? 1 : a.nbe0);
-    p.q_kmajor = a.q_kmajor;
-    p.k_kmajor = a.k_kmajor;
-    p.v_kmajor = a.v_kmajor;
-    p.lq = (int)a.lq;
-    p.lk = (int)a.lk;
-    p.d = (int)a.d;
-    p.tiles_q = (int)((a.lq + kAttnQ - 1) / kAttnQ);
-    p.num_tiles = (int)((long long)p.tiles_q * a.batch);
-    p.stages = 2;
-    p.from_zero = ctx.opts().ref_compat ? 1 : 0;
-    p.status = ctx.status_word_dev;
-    bool vec = a.d % 4 == 0 && a.ldo % 4 == 0 && a.so0 % 4 == 0 && a.so1 % 4 == 0 && (!a.o || aligned16(a.o)) &&
-               (!a.o_hi || (aligned16(a.o_hi) && a.o_plane % 4 == 0));
-    for (int i = 0; i < kMaxAux; ++i) {
-        TcAux &x = p.aux[i];
-        x.ptr = nullptr;
-        x.s0 = x.s1 = x.sr = 0;
-        x.sc = 0;
-        if (i >= a.naux) continue;
-        x.ptr = a.aux[i].ptr;
-        x.s0 = a.aux[i].s0;
-        x.s1 = a.aux[i].s1;
-        x.sr = a.aux[i].sr;
-        x.sc = a.aux[i].sc;
-        if (x.sc != 0 && x.sc != 1) return ctx.fail(SAGE_ERR_INVALID, "attention_tc: expression operand column stride must be 0 or 1");
-        if (x.sc == 1) vec = vec && aligned16(x.ptr) && x.s0 % 4 == 0 && x.s1 % 4 == 0 && x.sr % 4 == 0;
-    }
-    p.vec_ok = vec ? 1 : 0;
-    // Q, the K / V ring, 1 KiB per softmax warp for turning the output round, and the slack for 1024-byte alignment
-    const size_t smem = 4 * (size_t)kAttnQBytes + (size_t)p.stages * 8 * kAttnKVBytes + (size_t)kAttnSoftmaxWarps * 1024 + 1024;
-    const int grid = p.num_tiles < ctx.sm_count ? p.num_tiles : ctx.sm_count;
-
-    std::string defines = "struct __align__(64) CUtensorMap { unsigned long long opaque[16]; };\n";
-    defines += "#define SAGE_EPI_NAUX " + std::to_string(a.naux) + "\n";
-    {
-        int rowinv_mask = 0;  // which operands of the score expression have no row stride; which results are stored: compiled in
-        for (int i = 0; i < a.naux; ++i)
-            if (a.aux[i].sr == 0) rowinv_mask |= 1 << i;
-        defines += "#define SAGE_EPI_ROWINV " + std::to_string(rowinv_mask) + "\n";
-        defines += "#define SAGE_EPI_OUT " + std::to_string((a.o ? 1 : 0) | (a.o_hi ? 2 : 0)) + "\n";
-    }
-    defines += "#define SAGE_EPI_EXPR(x0, x1, x2, x3) (" + (a.epilogue.empty() ? std::string("x0") : a.epilogue) + ")\n";
-    const std::string key = "attention_tc\n" + defines;  // the rest of the translation unit is fixed text
-    Module *mod = ctx.module_find(key);
-    if (!mod) {
-        std::string src = map_prelude_text();
-        src += defines;
-        src += kGemmTcDeviceSrc;
-        src += kAttnTcDeviceSrc;
-        src += "\nextern \"C\" __global__ void __launch_bounds__(sage_tc::kAttnThreads, 1)\n"
-               "attention_tc_3xtf32(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,\n"
-               "                    const __grid_constant__ CUtensorMap map_v, const sage_tc::AttnParams p) {\n"
-               "    sage_tc::attn_body(&map_q, &map_k, &map_v, p);\n}\n";
-        sage_status st = ctx.module_get(src, &mod);
-        if (st) return st;
-        ctx.module_remember(key, mod);
-    }
-    CUtensorMap map_q, map_k, map_v;
-    if (!ctx.dry()) {
-        if (!tc_operand_ok(a.q) || !tc_operand_ok(a.k) || !tc_operand_ok(a.v)) return ctx.fail(SAGE_ERR_INVALID, "attention_tc: operand not addressable by TMA");
-        if (!encode_map(encode, a.q, kAttnQ, a.q_kmajor, &map_q) || !encode_map(encode, a.k, kAttnKeys, a.k_kmajor, &map_k) ||
-            !encode_map(encode, a.v, kAttnD, a.v_kmajor, &map_v))
-            return ctx.fail(SAGE_ERR_DEVICE, "cuTensorMapEncodeTiled failed");
-    }
-    std::string label;
-    if (ctx.verbose_names)
-        label = "attention_tc_3xtf32[" + std::to_string(a.lq) + "x" + std::to_string(a.lk) + "x" + std::to_string(a.d) + "x" + std::to_string(a.batch) + "]";
-    const uint32_t gr[3] = {(uint32_t)grid, 1, 1}, bl[3] = {(uint32_t)kAttnThreads, 1, 1};
-    void *params[4] = {&map_q, &map_k, &map_v, &p};
-    return ctx.launch(mod, "attention_tc_3xtf32", gr, bl, (uint32_t)smem, params, ctx.verbose_names ? label.c_str() : nullptr, true, 1);
 }
 
 sage_status gemm_tcgen05(Context &ctx, const GemmArgs &g) {

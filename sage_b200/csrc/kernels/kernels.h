@@ -21,18 +21,29 @@ struct Dims {  // extents + strides of a (sub)space, row-major order of traversa
     }
 };
 
+// Operand forms of a result that its producer writes beside (or instead of) the fp32 values, for the tensor-core product
+// that reads it next: tf32 planes (`hi`, lo `plane` floats further) and half-precision pieces (`h2`, lo `h2_plane` elements
+// further, a scale per 64 elements).  Null = not wanted; all are laid out like the fp32 result.
+struct PlaneOut {
+    float *hi = nullptr;
+    long long plane = 0;
+    unsigned short *h2 = nullptr;
+    long long h2_plane = 0;
+    float *h2_scale = nullptr;
+};
+
 // reduce.cu — ReduceOperator / ReduceArgOperator (src/ops/reduce.rs:258-325, 372-431)
 sage_status reduce(Context &ctx, int dtype, int kind, const void *x, const Dims &outer, const Dims &inner, void *y);
 sage_status reduce_arg(Context &ctx, bool is_max, const float *x, const Dims &outer, long long inner_ext,
                        long long inner_str, uint32_t *y);
 
 // rowops.cu — softmax / log_sum_exp / layer_norm over contiguous rows (src/ops/nn.rs:42-100)
-// `hi` (optional): also write the tf32 hi / lo planes of y, laid out like y, lo `plane` floats after hi.
-sage_status softmax_rows(Context &ctx, const float *x, float *y, long long rows, long long cols, float *hi = nullptr,
-                         long long plane = 0);
+sage_status softmax_rows(Context &ctx, const float *x, float *y, long long rows, long long cols, const PlaneOut &planes = PlaneOut());
+// Do the kernels of these rows hold whole 64-element groups per half warp (and so write the half-precision pieces)?
+bool rows_write_pieces(const float *x, long long cols);
 sage_status lse_rows(Context &ctx, const float *x, float *y, long long rows, long long cols);
 sage_status layernorm_rows(Context &ctx, const float *x, float *y, long long rows, long long cols, const float *gamma,
-                           int gamma_stride, const float *beta, int beta_stride, float eps, float *hi = nullptr, long long plane = 0);
+                           int gamma_stride, const float *beta, int beta_stride, float eps, const PlaneOut &planes = PlaneOut());
 
 // index.cu — gather / scatter / strided copy (src/ops/core.rs:571-934)
 sage_status gather(Context &ctx, const uint32_t *x, const long long *x_str, const uint32_t *ind, const Dims &ind_dims,
@@ -136,25 +147,6 @@ struct TcGemm {
     int force_bn = 0;          // tile width chosen by the caller (64 / 128 / 192 / 256); 0 = the launcher's own choice
     bool no_split_k = false;   // never cut K into slices: the launch then needs no scratch from the allocator
 };
-// Fused attention: O[batch] = softmax_rows(f(Q[batch] K[batch]^T)) V[batch] in one launch (kernels/attn_tc_device.inc).
-// Q is lq x d, K is lk x d, V is lk x d per batch, each given as the tensor core reads it: `q` and `k` with rows =
-// tokens, cols = head columns when `*_kmajor` (the head columns are contiguous), else stored transposed (rows = head
-// columns, cols = tokens); `v` with rows = keys, cols = head columns when NOT `v_kmajor`, else stored transposed.
-// `epilogue` is f over x0 (the score) and x1.. (aux, addressed like a GEMM epilogue operand of the lq x lk score
-// matrix, batch cut by `nbe0`).  The result goes to o / o_hi exactly like TcGemm's c / c_hi.  d <= 64.
-struct TcAttn {
-    long long lq = 0, lk = 0, d = 0, batch = 1;
-    TcOperand q, k, v;
-    bool q_kmajor = true, k_kmajor = true, v_kmajor = false;
-    float *o = nullptr, *o_hi = nullptr;
-    long long o_plane = 0, ldo = 0, so0 = 0, so1 = 0, nbo0 = 1;
-    int naux = 0;
-    TcAuxArg aux[3];
-    long long nbe0 = 1;
-    std::string epilogue;  // empty = x0
-};
-bool attention_tc_shape_ok(long long lq, long long lk, long long d, long long batch);
-sage_status attention_tc_run(Context &ctx, const TcAttn &a);
 bool gemm_tc_shape_ok(long long m, long long n, long long k, long long batch);
 sage_status gemm_tc_run(Context &ctx, const TcGemm &g);
 // How many K slices gemm_tc_run would cut this product into (0 = none).  Only products without an epilogue are
@@ -186,6 +178,7 @@ struct H2Gemm {
     long long img_n = 0, img_h = 0, img_w = 0, img_c = 0, out_h = 0, out_w = 0;
     Window win{};
     long long m = 0, n = 0, k = 0, batch = 1;
+    int slices = 0;           // > 1 (set by gemm_h2_run): the batch of the result are partial products over slices of K
     H2Operand a, b;
     float *c = nullptr, *c_hi = nullptr;  // result as fp32 and / or as tf32 planes, as in TcGemm
     long long c_plane = 0;
@@ -218,8 +211,35 @@ struct H2Split {
 size_t split_h2_bytes(long long batches, long long rows, long long cols, bool whole_rows);
 sage_status split_h2_view_into(Context &ctx, const float *src, const SplitView &v, bool whole_rows, void *dst, H2Split *out);
 sage_status split_h2_view(Context &ctx, const float *src, const SplitView &v, bool whole_rows, H2Split *out);
+// Operand B straight into memory the caller laid out: rows of `out->pitch` at out->hi / out->hi + out->plane, out->scale.
+sage_status split_h2_rows_at(Context &ctx, const float *src, const SplitView &v, const H2Split &out);
 H2Operand h2_operand(const H2Split &s, long long batches, long long rows, long long cols, bool whole_rows);
 
+// Fused attention: O[batch] = softmax_rows(f(Q[batch] K[batch]^T)) V[batch] in one launch (kernels/attn_tc_device.inc), on
+// half-precision pieces.  Q is lq x d, K and V are lk x d per batch, head columns contiguous, every row inside one group:
+// its scale is scale[((s_off + b0 * s_sb0 + b1 * s_sb1) >> s_shift) + row * s_row].
+// `epilogue` is f over x0 (the score) and x1.. (aux, addressed like a GEMM epilogue operand of the lq x lk score
+// matrix, batch cut by `nbe0`).  The result goes to o and / or the forms in `out` like a GEMM's (pieces: d = 64).  d <= 64.
+struct AttnOperand {
+    const unsigned short *hi = nullptr;
+    long long plane = 0, ld = 0, nb0 = 1, nb1 = 1, sb0 = 0, sb1 = 0;
+    const float *scale = nullptr;
+    long long s_off = 0, s_sb0 = 0, s_sb1 = 0, s_row = 0;
+    int s_shift = 0;
+};
+struct TcAttn {
+    long long lq = 0, lk = 0, d = 0, batch = 1;
+    AttnOperand q, k, v;
+    float *o = nullptr;
+    PlaneOut out;
+    long long ldo = 0, so0 = 0, so1 = 0, nbo0 = 1;
+    int naux = 0;
+    TcAuxArg aux[3];
+    long long nbe0 = 1;
+    std::string epilogue;  // empty = x0
+};
+bool attention_tc_shape_ok(long long lq, long long lk, long long d, long long batch);
+sage_status attention_tc_run(Context &ctx, const TcAttn &a);
 // Launches a kernel whose bounded wait runs out (nothing arrives on its barrier): ~1 s, then status bit 0x140.
 sage_status bounded_wait_selftest(Context &ctx);
 sage_status gemm_simt(Context &ctx, const GemmArgs &g);

@@ -18,6 +18,7 @@
 #include "kernels.h"
 #include "launch.h"
 #include "gemm_tc_device.inc"  // split_tf32_value
+#include "gemm_h2_device.inc"  // h2_split2
 
 namespace sage {
 namespace k {
@@ -43,29 +44,44 @@ struct RowParams {
     int gamma_stride, beta_stride;
     float eps;
     int ref_compat;
-    float *hi;        // when set: also write the tf32 hi / lo planes of y (softmax, layer_norm), laid out like y
-    long long plane;  // floats from the hi to the lo plane
+    PlaneOut out;  // operand forms of y to write as well (softmax, layer_norm)
 };
 
+// With half-precision pieces the 16 lanes of a half warp hold the 64 elements of a group: all of them come here or none does.
 __device__ __forceinline__ void row_store4(const RowParams &p, long long at, float4 o) {
-    if (p.y) *reinterpret_cast<float4 *>(p.y + at) = o;  // y is null when only the planes are wanted
-    if (p.hi) {
+    if (p.y) *reinterpret_cast<float4 *>(p.y + at) = o;  // y is null when only the operand forms are wanted
+    if (p.out.hi) {
         float4 h, l;
         sage_tc::split_tf32_value(o.x, &h.x, &l.x);
         sage_tc::split_tf32_value(o.y, &h.y, &l.y);
         sage_tc::split_tf32_value(o.z, &h.z, &l.z);
         sage_tc::split_tf32_value(o.w, &h.w, &l.w);
-        *reinterpret_cast<float4 *>(p.hi + at) = h;
-        *reinterpret_cast<float4 *>(p.hi + p.plane + at) = l;
+        *reinterpret_cast<float4 *>(p.out.hi + at) = h;
+        *reinterpret_cast<float4 *>(p.out.hi + p.out.plane + at) = l;
+    }
+    if (p.out.h2) {
+        using namespace sage_tc;
+        unsigned b = max(max(h2_finite_bits(o.x), h2_finite_bits(o.y)), max(h2_finite_bits(o.z), h2_finite_bits(o.w)));
+        const unsigned lanes = 0xffffu << (threadIdx.x & 16);
+#pragma unroll
+        for (int off = 8; off > 0; off >>= 1) b = max(b, __shfl_xor_sync(lanes, b, off));
+        float scale;
+        const float f = h2_factor(b, &scale);
+        uint2 h, l;
+        h2_split2(o.x, o.y, f, &h.x, &l.x);
+        h2_split2(o.z, o.w, f, &h.y, &l.y);
+        *reinterpret_cast<uint2 *>(p.out.h2 + at) = h;
+        *reinterpret_cast<uint2 *>(p.out.h2 + p.out.h2_plane + at) = l;
+        if ((threadIdx.x & 15) == 0) p.out.h2_scale[at >> 6] = scale;
     }
 }
 __device__ __forceinline__ void row_store1(const RowParams &p, long long at, float o) {
     if (p.y) p.y[at] = o;
-    if (p.hi) {
+    if (p.out.hi) {
         float h, l;
         sage_tc::split_tf32_value(o, &h, &l);
-        p.hi[at] = h;
-        p.hi[p.plane + at] = l;
+        p.out.hi[at] = h;
+        p.out.hi[p.out.plane + at] = l;
     }
 }
 
@@ -290,7 +306,8 @@ static sage_status launch_rows(Context &ctx, RowParams p, const char *name) {
     cudaError_t err = cudaSuccess;
     const bool aligned = (reinterpret_cast<uintptr_t>(p.x) % 16 == 0) &&
                          (MODE == ROW_LSE || reinterpret_cast<uintptr_t>(p.y) % 16 == 0) &&
-                         (!p.hi || (reinterpret_cast<uintptr_t>(p.hi) % 16 == 0 && p.plane % 4 == 0));
+                         (!p.out.hi || (reinterpret_cast<uintptr_t>(p.out.hi) % 16 == 0 && p.out.plane % 4 == 0));
+    if (p.out.h2 && !(aligned && rows_write_pieces(p.x, p.cols))) return ctx.fail(SAGE_ERR_INVALID, "row kernel: half-precision pieces need whole groups");
     if (p.cols % 4 == 0 && p.cols <= 2048 && aligned) {
         const int chunks = (int)(p.cols / 4);
         const int v = (chunks + 31) / 32;
@@ -316,19 +333,21 @@ static sage_status launch_rows(Context &ctx, RowParams p, const char *name) {
     return ctx.check_cuda(err, name);
 }
 
-sage_status softmax_rows(Context &ctx, const float *x, float *y, long long rows, long long cols, float *hi, long long plane) {
-    RowParams p{x, y, rows, cols, nullptr, nullptr, 0, 0, 0.f, 1, hi, plane};
+bool rows_write_pieces(const float *x, long long cols) { return cols % 64 == 0 && cols <= 16384 && reinterpret_cast<uintptr_t>(x) % 16 == 0; }
+
+sage_status softmax_rows(Context &ctx, const float *x, float *y, long long rows, long long cols, const PlaneOut &planes) {
+    RowParams p{x, y, rows, cols, nullptr, nullptr, 0, 0, 0.f, 1, planes};
     return launch_rows<ROW_SOFTMAX>(ctx, p, "softmax_rows");
 }
 
 sage_status lse_rows(Context &ctx, const float *x, float *y, long long rows, long long cols) {
-    RowParams p{x, y, rows, cols, nullptr, nullptr, 0, 0, 0.f, 1, nullptr, 0};
+    RowParams p{x, y, rows, cols, nullptr, nullptr, 0, 0, 0.f, 1, PlaneOut()};
     return launch_rows<ROW_LSE>(ctx, p, "lse_rows");
 }
 
 sage_status layernorm_rows(Context &ctx, const float *x, float *y, long long rows, long long cols, const float *gamma,
-                           int gamma_stride, const float *beta, int beta_stride, float eps, float *hi, long long plane) {
-    RowParams p{x, y, rows, cols, gamma, beta, gamma_stride, beta_stride, eps, 1, hi, plane};
+                           int gamma_stride, const float *beta, int beta_stride, float eps, const PlaneOut &planes) {
+    RowParams p{x, y, rows, cols, gamma, beta, gamma_stride, beta_stride, eps, 1, planes};
     return launch_rows<ROW_LN>(ctx, p, "layernorm_rows");
 }
 

@@ -73,6 +73,9 @@ sage_status prepare(const std::vector<Var> &params, const std::vector<Var> &grad
         slot.n = p.size();
         Storage &ps = *pt.data;
         ps.split_view.reset();
+        ps.h2.reset();
+        ps.h2_view.reset();
+        ps.h2_rows.reset();
         ++ps.version;  // whoever cached something derived from the old values (concatenated weights) rebuilds it
         if (ps.split && ps.split->whole) {  // a GEMM reads this parameter: refresh its planes in the same pass
             slot.hi = ps.split->planes.planes;

@@ -177,10 +177,10 @@ public:
     Block *gemm_trace_block = nullptr;  // per-CTA cycle counters of a GEMM launch run with SAGE_GEMM_TRACE (sm_count x 16 words)
     size_t streamk_bytes = 0;
     uint32_t streamk_epoch = 0;
-    // Set by the evaluator around one operator's compute(): a tensor-core GEMM will read the result,
-    // so a producer that can should also write the tf32 hi/lo planes of what it computes.
-    bool hint_emit_planes = false;
-    // ... and nothing else reads it: the producer may skip the fp32 store and write only the planes.
+    // Set by the evaluator around one operator's compute(): a tensor-core GEMM will read the result as tf32 planes / in
+    // half-precision pieces, so a producer that can should also write that form of what it computes.
+    bool hint_emit_planes = false, hint_emit_h2 = false;
+    // ... and nothing else reads it: the producer may skip the fp32 store and write only those.
     bool hint_planes_only = false;
     int sm_count = 148;
 

@@ -102,3 +102,77 @@ def test_infinities_and_nan_stay_in_their_rows(ctx):
     rest = [i for i in range(140) if i not in (3, 5)]
     assert np.isfinite(got[rest]).all()
     assert ctx.status_word() == 0
+
+
+@pytest.mark.parametrize("m,k,n1,n2", [(129, 96, 64, 70), (300, 130, 192, 64), (2048, 64, 448, 96), (12544, 64, 512, 64), (70, 4096, 128, 33)])
+def test_a_product_hands_pieces_to_the_next(ctx, m, k, n1, n2):
+    """The first product's result exists only as pieces (with its epilogue applied, K slices summed where it has them); every
+    group of it lands in its place, also where the last column tile is cut off.  Tolerance: 1e-5 of max(|b|, rms), as for the
+    other products behind an epilogue."""
+    rng = np.random.default_rng(m + n1)
+    x, w1 = rng.uniform(-1, 1, (m, k)).astype(np.float32), rng.uniform(-1, 1, (k, n1)).astype(np.float32)
+    b, w2 = rng.uniform(-1, 1, (n1,)).astype(np.float32), rng.uniform(-1, 1, (n1, n2)).astype(np.float32)
+    y = S.matmul(S.relu(S.matmul(ctx.var(x) * 1.0, ctx.var(w1)) + ctx.var(b)), ctx.var(w2))
+    got = y.eval(ctx).astype(np.float64)
+    want = np.maximum(x.astype(np.float64) @ w1 + b, 0.0) @ w2.astype(np.float64)
+    assert (np.abs(got - want) / np.maximum(np.abs(want), np.sqrt((want ** 2).mean()))).max() <= 1e-5
+    assert ctx.status_word() == 0
+
+
+@pytest.mark.parametrize("n,h,c,oc,ker,stride", [(3, 9, 64, 64, 3, 1), (2, 17, 64, 192, 3, 2), (1, 7, 512, 128, 3, 1), (5, 8, 128, 64, 1, 2), (1, 56, 64, 64, 3, 1)])
+def test_convolutions_on_pieces(ctx, n, h, c, oc, ker, stride):
+    """Two convolutions in a row (windows kept in shared memory, gathered, cut into K slices), the second over the first's pieces."""
+    rng = np.random.default_rng(h * c)
+    x = rng.uniform(-1, 1, (n, h, h, c)).astype(np.float32)
+    f1, f2 = rng.uniform(-1, 1, (ker, ker, c, oc)).astype(np.float32), rng.uniform(-1, 1, (3, 3, oc, 64)).astype(np.float32)
+    b = rng.uniform(-1, 1, (oc,)).astype(np.float32)
+
+    def conv(a, f, s):
+        k, p = f.shape[0], f.shape[0] // 2
+        a = np.pad(a.astype(np.float64), ((0, 0), (p, p), (p, p), (0, 0)))
+        o = (a.shape[1] - k) // s + 1
+        return sum(a[:, i:i + s * o:s, j:j + s * o:s][:, :o, :o] @ f[i, j].astype(np.float64) for i in range(k) for j in range(k))
+    y = S.relu(S.conv_2d(ctx.var(x) * 1.0, ctx.var(f1), stride, ker // 2, 1) + ctx.var(b))
+    got = S.conv_2d(y, ctx.var(f2), 1, 1, 1).eval(ctx).astype(np.float64)
+    want = conv(np.maximum(conv(x, f1, stride) + b, 0.0), f2, 1)
+    assert got.shape == want.shape
+    assert (np.abs(got - want) / np.maximum(np.abs(want), np.sqrt((want ** 2).mean()))).max() <= 1e-5
+    assert ctx.status_word() == 0
+
+
+def test_epilogue_operands_off_the_16_byte_grid(ctx):
+    """A result in pieces behind operands that 16-byte loads cannot read (a slice that starts off the grid; an odd row pitch)."""
+    rng = np.random.default_rng(81)
+    x, w1 = rng.uniform(-1, 1, (150, 96)).astype(np.float32), rng.uniform(-1, 1, (96, 128)).astype(np.float32)
+    r, w2 = rng.uniform(-1, 1, (150, 131)).astype(np.float32), rng.uniform(-1, 1, (128, 64)).astype(np.float32)
+    y = S.matmul(S.relu(S.matmul(ctx.var(x) * 1.0, ctx.var(w1)) + ctx.var(r).slice(1, 1, 129)), ctx.var(w2))
+    got = y.eval(ctx).astype(np.float64)
+    want = np.maximum(x.astype(np.float64) @ w1 + r[:, 1:129], 0.0) @ w2.astype(np.float64)
+    assert (np.abs(got - want) / np.maximum(np.abs(want), np.sqrt((want ** 2).mean()))).max() <= 1e-5
+
+
+@pytest.mark.parametrize("n,length,heads,direct", [(3, 77, 4, True), (2, 130, 2, False), (1, 64, 1, True), (2, 257, 3, False)])
+def test_attention_hands_pieces_to_the_next(ctx, n, length, heads, direct):
+    """Masked attention over any number of keys, its context multiplied by a weight; queries, keys and values straight from
+    products or behind a sum.  Tolerance 1e-4, as for the other attention blocks."""
+    rng = np.random.default_rng(length)
+    e = heads * 64
+    x = rng.uniform(-1, 1, (n, length, e)).astype(np.float32)
+    w = [(rng.standard_normal((e, e)) / np.sqrt(e)).astype(np.float32) for _ in range(4)]
+    mask = (rng.random((n, length)) < 0.8).astype(np.float32)
+    mask[:, 0] = 1
+    X = ctx.var(x) * 1.0
+    q, k, v = [S.matmul(X, ctx.var(w[i])) + (0.0 if direct else X) for i in range(3)]
+
+    def split(t):
+        return S.transpose(S.view(t, [n, length, heads, 64]), 2, 1)
+    s = S.matmul_batched(split(q), S.transpose(split(k), -1, -2)) / 8.0 + (-(S.view(ctx.var(mask), [n, 1, 1, length])) + 1.0) * -1e5
+    y = S.view(S.transpose(S.matmul_batched(S.softmax(s, [3]), split(v)), 2, 1), [n, length, e])
+    got = S.matmul(y, ctx.var(w[3])).eval(ctx).astype(np.float64)
+    x64 = x.astype(np.float64)
+    q, k, v = [(x64 @ w[i] + (0.0 if direct else x64)).reshape(n, length, heads, 64).transpose(0, 2, 1, 3) for i in range(3)]
+    s = q @ k.transpose(0, 1, 3, 2) / 8.0 + (1.0 - mask.astype(np.float64))[:, None, None, :] * -1e5
+    p = np.exp(s - s.max(-1, keepdims=True))
+    want = ((p / p.sum(-1, keepdims=True)) @ v).transpose(0, 2, 1, 3).reshape(n, length, e) @ w[3].astype(np.float64)
+    assert (np.abs(got - want) / np.maximum(np.abs(want), np.sqrt((want ** 2).mean()))).max() <= 1e-4
+    assert ctx.status_word() == 0
