@@ -645,39 +645,6 @@ struct GemmOp : Operator {
             st = aux_strides(ctx, x[2 + i], &g.aux[i]);
             if (st) return st;
         }
-        // K slices have to be summed before an epilogue is applied: it then runs as a generated map kernel over the sum
-        if (!folded && batch == 1 && (epilogue.empty() || epi_ext == out.shape.extents)) {
-            k::H2Gemm raw = g;
-            raw.epilogue.clear();
-            raw.naux = 0;
-            raw.c_hi = nullptr;
-            raw.h_hi = nullptr;
-            raw.sc0 = m * n;
-            raw.sc1 = 0;
-            raw.nbc0 = 1;
-            const bool plain = epilogue.empty() && !emit && !emit_h2;
-            if (!plain && gemm_h2_slices(ctx, raw) >= 2) {
-                Block *sum = ctx.allocator().alloc((size_t)(m * n) * sizeof(float));
-                if (sum) {
-                    raw.c = reinterpret_cast<float *>(sum->ptr);
-                    st = k::gemm_h2_run(ctx, raw);
-                    if (!st) {
-                        std::vector<MapOperand> operands(1 + (size_t)g.naux);
-                        operands[0].dtype = SAGE_F32;
-                        operands[0].ptr = raw.c;
-                        operands[0].view = Tensor().with_shape(Shape(out.shape.extents)).dims();
-                        for (int i = 0; i < g.naux; ++i) {
-                            operands[1 + i].dtype = x[2 + i].desc.dtype;
-                            operands[1 + i].ptr = x[2 + i].ptr();
-                            operands[1 + i].view = x[2 + i].dims();
-                        }
-                        st = map_launch(ctx, epilogue.empty() ? "x0" : epilogue, operands, SAGE_F32, y->ptr(), out.shape.rank(), out.shape.extents.data(), &epi_cache, o);
-                    }
-                    ctx.allocator().free(sum);  // stream-ordered
-                    return st;
-                }
-            }
-        }
         if (only) {
             g.c = nullptr;
             y->data->planes_only = true;

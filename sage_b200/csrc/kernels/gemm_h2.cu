@@ -3,6 +3,8 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include <cstdlib>
 
 #include "kernels.h"
@@ -369,72 +371,6 @@ static ColumnPlan plan_columns(const Context &ctx, long long m, long long n, lon
     return best;
 }
 
-static sage_status gemm_h2_launch(Context &ctx, const H2Gemm &g);
-
-// Split-K: as in gemm_tcgen05.cu, a product with few output tiles and a long K runs in slices of K (a whole number of
-// K-blocks each) followed by their sum in a fixed order.  Microseconds from measured launches: a K-block takes what its
-// operand bytes take from L2 (64 KB: 1.0 us with all SMs loading) but not less than 0.45, a tile ~5 us beside its K loop,
-// the sum 3.5 us and its bytes.  Slices must promise a fifth: they change the order of summation, and nearer to the line than
-// that the estimate says little.
-static int pick_slices(const Context &ctx, const H2Gemm &g) {
-    static const bool enabled = !(getenv("SAGE_GEMM_SPLITK") && atoi(getenv("SAGE_GEMM_SPLITK")) == 0);
-    if (!enabled || g.batch != 1 || g.naux || !g.epilogue.empty() || !g.c || g.c_hi || g.h_hi || g.ldc != g.n || g.k < 512) return 0;
-    int wb, rows;
-    if (halo_plan(g, &wb, &rows)) return 0;
-    const int ctas = (pairs_on() && g.m > BM) ? 2 : 1;
-    const long long units = ctx.sm_count / ctas, all_kb = (g.k + HK - 1) / HK;
-    double best = 1e300, unsplit = 1e300;
-    long long best_s = 0;
-    for (long long s = 1; s <= all_kb / 2 && s <= 64; ++s) {
-        if (g.conv && all_kb % s) continue;  // a convolution has no K-blocks to fill a last slice with
-        const long long kb = (all_kb + s - 1) / s;
-        if (kb * (s - 1) >= all_kb) continue;
-        for (int bn : {256, 128, 64}) {
-            if (bn > 64 && g.n <= bn / 2) continue;
-            const long long tiles = ((g.m + BM * ctas - 1) / (BM * ctas)) * ((g.n + bn - 1) / bn) * s, waves = (tiles + units - 1) / units;
-            double per = 1.0 * (BM + bn / ctas) / 256.0;
-            if (per < 0.45) per = 0.45;
-            double t = (double)waves * ((double)kb * per + 5.0);
-            if (s > 1) t += 3.5 + (double)(s + 1) * (double)g.m * (double)g.n * 4.0 / 5.0e6;
-            if (s == 1 && t < unsplit) unsplit = t;
-            if (t < best) {
-                best = t;
-                best_s = s;
-            }
-        }
-    }
-    return best_s >= 2 && best <= 0.8 * unsplit ? (int)best_s : 0;
-}
-
-int gemm_h2_slices(Context &ctx, const H2Gemm &g) { return pick_slices(ctx, g); }
-
-sage_status gemm_h2_run(Context &ctx, const H2Gemm &g0, bool no_slices) {
-    const int S = no_slices ? 0 : pick_slices(ctx, g0);
-    if (S < 2) return gemm_h2_launch(ctx, g0);
-    const long long mn = g0.m * g0.n;
-    Block *scratch = ctx.allocator().alloc((size_t)S * mn * sizeof(float));
-    if (!scratch) return gemm_h2_launch(ctx, g0);  // no room for the partial products: one pass over K
-    H2Gemm g = g0;
-    g.slices = S;
-    g.c = reinterpret_cast<float *>(scratch->ptr);
-    g.sc0 = mn;
-    g.sc1 = 0;
-    g.nbc0 = S;
-    sage_status st = gemm_h2_launch(ctx, g);
-    if (!st) {
-        Dims outer, inner;
-        outer.ndim = 1;
-        outer.ext[0] = mn;
-        outer.str[0] = 1;
-        inner.ndim = 1;
-        inner.ext[0] = S;
-        inner.str[0] = mn;
-        st = reduce(ctx, SAGE_F32, 0 /* sum */, g.c, outer, inner, g0.c);
-    }
-    ctx.allocator().free(scratch);  // stream-ordered
-    return st;
-}
-
 // op(A) op(B) of plain fp32 operands: both brought into pieces, K contiguous.  `scratch`: where the pieces go (of
 // gemm_h2_scratch_bytes), or null to take them from the allocator.
 static SplitView operand_view(const float *, long long rows, long long cols, bool k_contiguous, long long ld, long long batch_stride, long long batch) {
@@ -472,7 +408,7 @@ sage_status gemm_h2(Context &ctx, const GemmArgs &a, void *scratch) {
         g.ldc = a.ldc;
         g.sc0 = a.stride_c;
         g.nbc0 = a.batch;
-        st = gemm_h2_run(ctx, g, block == nullptr);
+        st = gemm_h2_run(ctx, g);
     }
     if (block) ctx.allocator().free(block);  // stream-ordered: later launches on this stream may reuse it
     return st;
@@ -480,24 +416,104 @@ sage_status gemm_h2(Context &ctx, const GemmArgs &a, void *scratch) {
 
 // The plain product (no epilogue, fp32 result): compiled with the library, so that an entry point which must not load a
 // module at run time can use it.
-template <int BN, int CTAS>
-__global__ void __launch_bounds__(kThreads, 1) gemm_h2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+template <int BN, int CTAS, bool SLICED>
+__global__ void __launch_bounds__(SLICED ? 64 + 2 * BN : kThreads, SLICED && BN == 64 ? 2 : 1) gemm_h2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                                                               const __grid_constant__ CUtensorMap map_b2, const __grid_constant__ H2Params p) {
-    gemm_h2_body<BN, CTAS>(&map_a, &map_a, &map_b, &map_b2, p);
+    gemm_h2_body<BN, CTAS, SLICED>(&map_a, &map_a, &map_b, &map_b2, p);
 }
-template <int BN, int CTAS>
+template <int BN, int CTAS, bool SLICED>
 static sage_status launch_plain(Context &ctx, const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorMap &map_b2, const H2Params &p, int grid, size_t smem) {
-    static int attr_set[64] = {0};  // per instantiation and device
+    static int attr_set[64] = {0};  // per instantiation and device: the largest seen
     const int dev = ctx.device();
-    if (dev < 0 || dev >= 64 || attr_set[dev] != (int)smem) {
-        sage_status st = ctx.check_cuda(cudaFuncSetAttribute(gemm_h2_kernel<BN, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "gemm_h2 shared memory attribute");
+    if (dev < 0 || dev >= 64 || attr_set[dev] < (int)smem) {
+        sage_status st = ctx.check_cuda(cudaFuncSetAttribute(gemm_h2_kernel<BN, CTAS, SLICED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "gemm_h2 shared memory attribute");
         if (st) return st;
         if (dev >= 0 && dev < 64) attr_set[dev] = (int)smem;
     }
-    return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), CTAS, gemm_h2_kernel<BN, CTAS>, dim3(grid), dim3(kThreads), smem, map_a, map_b, map_b2, p), "gemm_h2 launch");
+    return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), SLICED ? p.slices : CTAS, gemm_h2_kernel<BN, CTAS, SLICED>, dim3(grid), dim3(SLICED ? 64 + 2 * BN : kThreads), smem, map_a, map_b, map_b2, p), "gemm_h2 launch");
 }
 
-static sage_status gemm_h2_launch(Context &ctx, const H2Gemm &g) {
+// How many clusters of `s` CTAs the chip holds at once: they do not cross a GPC, so fewer than SMs / s.
+static int clusters_at_once(const Context &ctx, int s) {
+    static std::atomic<int> known[64][9];
+    const int dev = ctx.device();
+    if (ctx.dry() || dev < 0 || dev >= 64) return ctx.sm_count / s * 9 / 10;
+    int n = known[dev][s].load(std::memory_order_relaxed);
+    if (n > 0) return n;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)s;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)(s * 256));
+    cfg.blockDim = dim3(64 + 2 * 128);
+    cfg.dynamicSmemBytes = 200 * 1024;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(gemm_h2_kernel<128, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, gemm_h2_kernel<128, 1, true>, &cfg) != cudaSuccess || n < 1) {
+        (void)cudaGetLastError();
+        n = ctx.sm_count / s * 9 / 10;
+    }
+    known[dev][s].store(n, std::memory_order_relaxed);
+    return n;
+}
+
+// Slices of K (gemm_h2_body's SLICED), or 0, and the width of their tiles.  Microseconds, from launches of one wave timed on
+// M 24 .. 3136, N 64 .. 3072, K 512 .. 4608: a K-block takes 0.52 / 0.67 / 0.92 with 64 / 128 / 256 columns (a pair of CTAs
+// 0.42 / 0.48 / 0.91, windows kept in shared memory 0.48), and not less than the bytes of all CTAs at 9 TB/s; a tile 3.5 beside
+// them, and 5 for operands that depend on the row, which slices fetch in time.  Meeting in shared memory: 1.5 and 1.1 per 128 x
+// 64 sums (256 columns: 9, never worth it).  Slices must promise a fifth: they change the order of summation, and nearer to the
+// line than that the estimate says little.
+struct SlicePlan {
+    int slices, bn;
+};
+static SlicePlan plan_slices(const Context &ctx, const H2Gemm &g) {
+    static const bool enabled = !(getenv("SAGE_GEMM_SPLITK") && atoi(getenv("SAGE_GEMM_SPLITK")) == 0);
+    const SlicePlan none{0, 0};
+    const long long all_kb = (g.k + HK - 1) / HK;
+    if (!enabled || all_kb < 4) return none;
+    const int ctas = (pairs_on() && g.m > BM) ? 2 : 1;
+    double best = 1e300, whole = 1e300, store = 3.5;
+    for (int i = 0; i < g.naux; ++i)
+        if (g.aux[i].sr != 0) store = 8.5;
+    SlicePlan plan = none;
+    int wb = 0, halo_rows = 0;
+    if (halo_plan(g, &wb, &halo_rows)) {
+        const long long tiles = (g.img_n * ((g.out_h + halo_rows - 1) / halo_rows) + ctas - 1) / ctas, slots = ctx.sm_count / ctas;
+        whole = (double)((tiles + slots - 1) / slots) * ((double)all_kb * 0.48 + store + 3.0);
+    }
+    for (int w = 0; w < 3; ++w) {
+        static const double alone[3] = {0.52, 0.67, 0.92}, paired[3] = {0.42, 0.48, 0.91};
+        const int bn = 64 << w;
+        if (w > 0 && g.n <= bn / 2) continue;
+        const long long cols = (g.n + bn - 1) / bn * g.batch;
+        auto block_us = [&](double us, long long busy, int pair) {
+            const double bytes = (double)busy * (BM + bn / pair) * HK * 4 / 9e6;
+            return us > bytes ? us : bytes;
+        };
+        if (!wb) {
+            const long long tiles = (g.m + BM * ctas - 1) / (BM * ctas) * cols, slots = ctx.sm_count / ctas, busy = tiles < slots ? tiles : slots;
+            const double t = (double)((tiles + slots - 1) / slots) * ((double)all_kb * block_us(ctas == 2 ? paired[w] : alone[w], busy * ctas, ctas) + store);
+            if (t < whole) whole = t;
+        }
+        const long long tiles = (g.m + BM - 1) / BM * cols;
+        for (int s = 2; s <= 8 && bn < 256; ++s) {
+            const long long kb = (all_kb + s - 1) / s;
+            if (kb < 2 || kb * (s - 1) >= all_kb || tiles > clusters_at_once(ctx, s)) continue;
+            const double filled = g.m < BM ? (double)g.m / BM : 1.0;
+            const double t = (double)kb * block_us(alone[w], tiles * s, 1) + 5.0 + filled * 1.1 * (1 << w);
+            if (t < best) {
+                best = t;
+                plan = SlicePlan{s, bn};
+            }
+        }
+    }
+    return best <= 0.8 * whole ? plan : none;
+}
+
+sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
     static PFN_encodeTiled encode = nullptr;
     static PFN_encodeIm2col encode_conv = nullptr;
     if (!ctx.dry() && !encode) {
@@ -510,17 +526,20 @@ static sage_status gemm_h2_launch(Context &ctx, const H2Gemm &g) {
     if (g.naux < 0 || g.naux > kMaxAux || (!g.c && !g.c_hi && !g.h_hi)) return ctx.fail(SAGE_ERR_INVALID, "gemm_h2: bad epilogue description");
     if (g.conv && (g.batch != 1 || !conv_h2_ok(g) || g.m != g.img_n * g.out_h * g.out_w || g.k != (long long)g.win.ker_h * g.win.ker_w * g.img_c))
         return ctx.fail(SAGE_ERR_INVALID, "gemm_h2: convolution description does not match the GEMM");
-    const int ctas = (pairs_on() && g.m > BM) ? 2 : 1;
+    const SlicePlan cut = plan_slices(ctx, g);
+    const bool sliced = cut.slices > 1;
+    const int ctas = (pairs_on() && g.m > BM && !sliced) ? 2 : 1;
     int halo_wb = 0, halo_r = 0;
-    const bool halo = halo_plan(g, &halo_wb, &halo_r);
-    ColumnPlan cols = plan_columns(ctx, g.m, g.n, g.batch, ctas);
-    if (g.slices > 1) cols = plan_columns(ctx, g.m, g.n, g.slices, ctas);
+    const bool halo = !sliced && halo_plan(g, &halo_wb, &halo_r);
+    ColumnPlan cols = sliced ? ColumnPlan{cut.bn, 0, 0} : plan_columns(ctx, g.m, g.n, g.batch, ctas);
     if (halo) cols = ColumnPlan{g.n <= 64 ? 64 : 128, 0, 0};  // all output channels in one tile: the window is loaded once
     const int bn = cols.bn;
     const int stage_bytes = halo ? 2 * (bn / ctas) * HK * 2 : 2 * BM * HK * 2 + 2 * (bn / ctas) * HK * 2;
     const int staging = kEpiWarps * kStageBytesPerWarp, fixed = halo ? kHaloStages * kHaloStageBytes : 0;
     int stages = (227 * 1024 - 2048 - staging - fixed) / stage_bytes;
     if (stages > 8) stages = 8;
+    const long long all_kb = (g.k + HK - 1) / HK, my_kb = sliced ? (all_kb + cut.slices - 1) / cut.slices : all_kb;
+    if (sliced && stages > my_kb) stages = (int)my_kb;  // two CTAs fit an SM then: the next kernel's start overlaps this one's end
     const size_t smem = (size_t)fixed + (size_t)stages * stage_bytes + staging + 1024;
 
     H2Params p{};
@@ -536,12 +555,10 @@ static sage_status gemm_h2_launch(Context &ctx, const H2Gemm &g) {
     p.nbc0 = (int)(g.nbc0 < 1 ? 1 : g.nbc0);
     p.na0 = (int)g.a.nb0;
     p.nb0 = (int)g.b.nb0;
-    const bool sliced = g.slices > 1;
-    const long long batch = sliced ? g.slices : g.batch, all_kb = (g.k + HK - 1) / HK;
-    p.sliced = sliced ? 1 : 0;
-    p.kb_count = (int)(sliced ? (all_kb + g.slices - 1) / g.slices : all_kb);
-    p.a_bcast = (g.a.bcast || g.conv || sliced) ? 1 : 0;
-    p.b_bcast = (g.b.bcast || sliced) ? 1 : 0;
+    p.slices = sliced ? cut.slices : 0;
+    p.kb_count = (int)my_kb;
+    p.a_bcast = (g.a.bcast || g.conv) ? 1 : 0;
+    p.b_bcast = g.b.bcast ? 1 : 0;
     p.m = (int)g.m;
     p.n = (int)g.n;
     p.k = (int)g.k;
@@ -551,7 +568,7 @@ static sage_status gemm_h2_launch(Context &ctx, const H2Gemm &g) {
     p.rag_wide = cols.wide;
     p.rag_narrow = cols.narrow;
     p.rag_bn = 192;
-    p.num_tiles = (int)((long long)p.tiles_m * p.tiles_n * batch);
+    p.num_tiles = (int)((long long)p.tiles_m * p.tiles_n * g.batch);
     p.sa = g.a.scale;
     p.sa_row = g.a.s_row;
     p.sa_b0 = g.a.s_b0;
@@ -600,14 +617,14 @@ static sage_status gemm_h2_launch(Context &ctx, const H2Gemm &g) {
         if (a.sc != 0) per_col |= 1 << i;
     }
     p.vec_ok = vec ? 1 : 0;
-    p.aux_vec = aux_vec ? 1 : 0;
     if (g.h_hi && (!vec || g.n % 64 || g.ldc % 64 || g.sc0 % 64 || g.sc1 % 64 || !aligned16(g.h_hi) || g.h_plane % 8))
         return ctx.fail(SAGE_ERR_INVALID, "gemm_h2: a result in half-precision pieces needs whole groups of 64 columns");
-    const int slots = ctx.sm_count / ctas, grid = ctas * (p.num_tiles < slots ? p.num_tiles : slots);
+    const int slots = ctx.sm_count / ctas, grid = sliced ? cut.slices * p.num_tiles : ctas * (p.num_tiles < slots ? p.num_tiles : slots);
+    const int threads = sliced ? 64 + 2 * bn : kThreads;
 
     const int out_mask = (g.c ? 1 : 0) | (g.c_hi ? 2 : 0) | (g.h_hi ? 4 : 0);
     char num[96];
-    snprintf(num, sizeof num, "gemm_h2 %d %d %d %d %d %d %d\n", bn, ctas, g.conv ? (halo ? 2 : 1) : 0, g.naux, rowinv, per_col, out_mask);
+    snprintf(num, sizeof num, "gemm_h2 %d %d %d %d %d %d %d %d %d\n", bn, ctas, sliced ? 1 : 0, aux_vec ? 1 : 0, g.conv ? (halo ? 2 : 1) : 0, g.naux, rowinv, per_col, out_mask);
     const bool plain = !g.conv && g.naux == 0 && g.epilogue.empty() && out_mask == 1;
     const std::string key = num + g.epilogue;
     Module *mod = plain ? nullptr : ctx.module_find(key);
@@ -620,14 +637,15 @@ static sage_status gemm_h2_launch(Context &ctx, const H2Gemm &g) {
         define("SAGE_EPI_OUT", out_mask);
         define("SAGE_EPI_NAUX", g.naux);
         define("SAGE_H2_CONV", g.conv ? 1 : 0);
+        define("SAGE_H2_AUX_VEC", aux_vec ? 1 : 0);
         define("SAGE_H2_HALO", halo ? 1 : 0);
         src += "#define SAGE_EPI_EXPR(x0, x1, x2, x3) (" + (g.epilogue.empty() ? std::string("x0") : g.epilogue) + ")\n";
         src += kGemmTcDeviceSrc;
         src += kGemmH2DeviceSrc;
-        src += "\nextern \"C\" __global__ void __launch_bounds__(sage_tc::kThreads, 1)\n"
+        src += "\nextern \"C\" __global__ void __launch_bounds__(" + std::to_string(threads) + (sliced && bn == 64 ? ", 2)\n" : ", 1)\n") +
                "gemm_tc_h2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_a2,\n"
                "           const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_b2, const __grid_constant__ sage_tc::H2Params p) {\n"
-               "    sage_tc::gemm_h2_body<" + std::to_string(bn) + ", " + std::to_string(ctas) + ">(&map_a, &map_a2, &map_b, &map_b2, p);\n}\n";
+               "    sage_tc::gemm_h2_body<" + std::to_string(bn) + ", " + std::to_string(ctas) + (sliced ? ", true" : ", false") + ">(&map_a, &map_a2, &map_b, &map_b2, p);\n}\n";
         sage_status st = ctx.module_get(src, &mod);
         if (st) return st;
         ctx.module_remember(key, mod);
@@ -656,22 +674,23 @@ static sage_status gemm_h2_launch(Context &ctx, const H2Gemm &g) {
     }
     std::string label;
     if (ctx.verbose_names)
-        label = "gemm_tc_h2[" + std::to_string(g.m) + "x" + std::to_string(g.n) + "x" + std::to_string(g.k) + (batch > 1 ? "x" + std::to_string(batch) : "") + (sliced ? "s" : "") +
+        label = "gemm_tc_h2[" + std::to_string(g.m) + "x" + std::to_string(g.n) + "x" + std::to_string(g.k) + (g.batch > 1 ? "x" + std::to_string(g.batch) : "") + (sliced ? ",slices" + std::to_string(cut.slices) : "") +
                 (g.conv ? (halo ? ",conv,taps" : ",conv") : "") + ",bn" + std::to_string(bn) + (cols.narrow ? "/" + std::to_string(cols.wide) + "+" + std::to_string(cols.narrow) + "x192" : "") +
                 (ctas == 2 ? ",pair" : "") + "]o" + std::to_string(out_mask);
     if (plain) {
         ctx.note_launch(ctx.verbose_names ? label.c_str() : "gemm_tc_3xtf32");
         if (ctx.dry()) return SAGE_OK;
+        if (sliced) return bn == 128 ? launch_plain<128, 1, true>(ctx, map_a, map_b, map_b2, p, grid, smem) : launch_plain<64, 1, true>(ctx, map_a, map_b, map_b2, p, grid, smem);
         if (ctas == 2)
-            return bn == 256 ? launch_plain<256, 2>(ctx, map_a, map_b, map_b2, p, grid, smem)
-                   : bn == 128 ? launch_plain<128, 2>(ctx, map_a, map_b, map_b2, p, grid, smem) : launch_plain<64, 2>(ctx, map_a, map_b, map_b2, p, grid, smem);
-        return bn == 256 ? launch_plain<256, 1>(ctx, map_a, map_b, map_b2, p, grid, smem)
-               : bn == 128 ? launch_plain<128, 1>(ctx, map_a, map_b, map_b2, p, grid, smem) : launch_plain<64, 1>(ctx, map_a, map_b, map_b2, p, grid, smem);
+            return bn == 256 ? launch_plain<256, 2, false>(ctx, map_a, map_b, map_b2, p, grid, smem)
+                   : bn == 128 ? launch_plain<128, 2, false>(ctx, map_a, map_b, map_b2, p, grid, smem) : launch_plain<64, 2, false>(ctx, map_a, map_b, map_b2, p, grid, smem);
+        return bn == 256 ? launch_plain<256, 1, false>(ctx, map_a, map_b, map_b2, p, grid, smem)
+               : bn == 128 ? launch_plain<128, 1, false>(ctx, map_a, map_b, map_b2, p, grid, smem) : launch_plain<64, 1, false>(ctx, map_a, map_b, map_b2, p, grid, smem);
     }
-    const uint32_t gr[3] = {(uint32_t)grid, 1, 1}, bl[3] = {(uint32_t)kThreads, 1, 1};
+    const uint32_t gr[3] = {(uint32_t)grid, 1, 1}, bl[3] = {(uint32_t)threads, 1, 1};
     void *params[5] = {&map_a, &map_a2, &map_b, &map_b2, &p};
     // launch lists have one name for a tensor-core product; verbose ones tell the kernels apart
-    return ctx.launch(mod, "gemm_tc_h2", gr, bl, (uint32_t)smem, params, ctx.verbose_names ? label.c_str() : "gemm_tc_3xtf32", true, ctas);
+    return ctx.launch(mod, "gemm_tc_h2", gr, bl, (uint32_t)smem, params, ctx.verbose_names ? label.c_str() : "gemm_tc_3xtf32", true, sliced ? cut.slices : ctas);
 }
 
 // ---------------------------------------------------------------------------------- fused attention

@@ -178,7 +178,6 @@ struct H2Gemm {
     long long img_n = 0, img_h = 0, img_w = 0, img_c = 0, out_h = 0, out_w = 0;
     Window win{};
     long long m = 0, n = 0, k = 0, batch = 1;
-    int slices = 0;           // > 1 (set by gemm_h2_run): the batch of the result are partial products over slices of K
     H2Operand a, b;
     float *c = nullptr, *c_hi = nullptr;  // result as fp32 and / or as tf32 planes, as in TcGemm
     long long c_plane = 0;
@@ -190,9 +189,7 @@ struct H2Gemm {
     TcAuxArg aux[3];
     std::string epilogue;
 };
-sage_status gemm_h2_run(Context &ctx, const H2Gemm &g, bool no_slices = false);
-// How many K slices gemm_h2_run would cut this product into (0 = none), as gemm_tc_split_plan.
-int gemm_h2_slices(Context &ctx, const H2Gemm &g);
+sage_status gemm_h2_run(Context &ctx, const H2Gemm &g);
 // The whole product of plain fp32 operands.  With `scratch` (gemm_h2_scratch_bytes of device memory, 256-byte aligned)
 // nothing is taken from the allocator and K is not cut.
 size_t gemm_h2_scratch_bytes(const GemmArgs &g);

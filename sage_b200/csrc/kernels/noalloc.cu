@@ -13,8 +13,7 @@
 //   * 2 * 4 bytes * (rows_a * pitch(cols_a) + rows_b * pitch(cols_b)) must fit in kScratchBytes,
 //     where pitch rounds the contiguous extent up to 4 floats; larger problems get SAGE_ERR_INVALID.
 //     (The operands in half-precision pieces take half of that and their scales; the limit callers know stays.)
-//   * A long K is never cut into slices here (sage_gemm does that with allocator scratch), so for k >= 1024
-//     with few output tiles this entry point is slower than sage_gemm and its sum order differs from it.
+//   * The product itself is the one sage_gemm launches for these sizes: its slices of a long K meet in shared memory.
 //   * The first call on a device looks up the device address of the array (cudaGetSymbolAddress,
 //     with that device current).  Make that first call before any stream capture begins.
 //   * All calls share the one array, and it keeps whatever the previous call left in it.  Nothing
@@ -76,7 +75,5 @@ extern "C" sage_status sage_gemm_noalloc(sage_ctx *ctx, int32_t trans_a, int32_t
     cudaError_t err;
     float *scratch = scratch_for_device(C.device(), &err);
     if (!scratch) return C.check_cuda(err, "cudaGetSymbolAddress(gemm scratch)");
-    // One pass over K: sage_gemm may cut a long K into slices, which takes partial-product scratch from the
-    // allocator and a second kernel.  Neither is reachable from here.
     return k::gemm_h2(C, g, scratch);
 }

@@ -242,14 +242,13 @@ int Context::blocks_per_sm(Module *m, const char *name, int block_threads, uint3
     typedef int (*PFN_occupancy)(int *, CUfunc_st *, int, size_t);
     static PFN_occupancy occupancy = (PFN_occupancy)dlsym(d.lib, "cuOccupancyMaxActiveBlocksPerMultiprocessor");
     CUfunc_st *fn = nullptr;
-    auto it = m->functions.find(name);
-    if (it == m->functions.end()) {
-        if (d.ModuleGetFunction(&fn, m->cu_module, name)) return 1;
-        if (smem > 48 * 1024 && d.FuncSetAttribute) d.FuncSetAttribute(fn, 8 /*MAX_DYNAMIC_SHARED_SIZE_BYTES*/, (int)smem);
-        m->functions[name] = fn;
-    } else {
-        fn = it->second;
+    Module::Function &f = m->functions[name];
+    if (!f.fn && d.ModuleGetFunction(&f.fn, m->cu_module, name)) return 1;
+    if (smem > f.smem && d.FuncSetAttribute) {
+        d.FuncSetAttribute(f.fn, 8 /*MAX_DYNAMIC_SHARED_SIZE_BYTES*/, (int)smem);
+        f.smem = smem;
     }
+    fn = f.fn;
     int n = 0;
     if (!occupancy || occupancy(&n, fn, block_threads, smem) || n < 1) return 1;
     return n;
@@ -261,15 +260,16 @@ sage_status Context::launch(Module *m, const char *name, const uint32_t grid[3],
     if (dry()) return SAGE_OK;
     Driver &d = driver();
     CUfunc_st *fn = nullptr;
-    auto it = m->functions.find(name);
-    if (it == m->functions.end()) {
-        int e = d.ModuleGetFunction(&fn, m->cu_module, name);
+    Module::Function &f = m->functions[name];
+    if (!f.fn) {
+        int e = d.ModuleGetFunction(&f.fn, m->cu_module, name);
         if (e) return fail(SAGE_ERR_DEVICE, std::string("cuModuleGetFunction(") + name + "): " + cu_err(e));
-        if (smem > 48 * 1024 && d.FuncSetAttribute) d.FuncSetAttribute(fn, 8 /*MAX_DYNAMIC_SHARED_SIZE_BYTES*/, (int)smem);
-        m->functions[name] = fn;
-    } else {
-        fn = it->second;
     }
+    if (smem > f.smem && d.FuncSetAttribute) {
+        d.FuncSetAttribute(f.fn, 8 /*MAX_DYNAMIC_SHARED_SIZE_BYTES*/, (int)smem);
+        f.smem = smem;
+    }
+    fn = f.fn;
     if (grid[0] == 0 || grid[1] == 0 || grid[2] == 0) return SAGE_OK;
     int e;
     if (cluster > 1 && !d.LaunchKernelEx) return fail(SAGE_ERR_DEVICE, "cuLaunchKernelEx is not available for a cluster launch");

@@ -96,7 +96,11 @@ struct Module {
     std::string source;
     std::vector<char> cubin;
     CUmod_st *cu_module = nullptr;  // null on a planning context
-    std::unordered_map<std::string, CUfunc_st *> functions;
+    struct Function {
+        CUfunc_st *fn = nullptr;
+        uint32_t smem = 48 * 1024;  // dynamic shared memory it may be launched with
+    };
+    std::unordered_map<std::string, Function> functions;
 };
 
 class Context {
