@@ -100,6 +100,9 @@ __global__ void __launch_bounds__(256) row_warp_kernel(RowParams p) {
         const int c = lane + 32 * i;
         if (c < chunks) v[i] = __ldg(xr + c);
     }
+    float g0 = 0.f, b0 = 0.f;  // one scale and one shift for all columns: asked for with the row
+    const bool one_gb = MODE == ROW_LN && p.gamma_stride == 0 && p.beta_stride == 0;
+    if (one_gb) g0 = __ldg(p.gamma), b0 = __ldg(p.beta);
     if (MODE == ROW_LN) {
         // scale and shift: 16 bytes at a time when they are plain vectors (the same for every row: L1 hits)
         const bool vec_gb = p.gamma_stride == 1 && p.beta_stride == 1 && ((reinterpret_cast<unsigned long long>(p.gamma) | reinterpret_cast<unsigned long long>(p.beta)) & 15ull) == 0;
@@ -122,7 +125,10 @@ __global__ void __launch_bounds__(256) row_warp_kernel(RowParams p) {
             if (c < chunks) {
                 const int e = c * 4;
                 float4 g, b;
-                if (vec_gb) {
+                if (one_gb) {
+                    g = make_float4(g0, g0, g0, g0);
+                    b = make_float4(b0, b0, b0, b0);
+                } else if (vec_gb) {
                     g = __ldg(reinterpret_cast<const float4 *>(p.gamma) + c);
                     b = __ldg(reinterpret_cast<const float4 *>(p.beta) + c);
                 } else {
@@ -188,12 +194,27 @@ __device__ __forceinline__ float block_reduce(float v, bool is_max, float *smem)
     return r;
 }
 
+// Two sums over the CTA in one exchange.
+__device__ __forceinline__ void block_sum2(float *a, float *b, float *smem) {
+    *a = warp_sum(*a);
+    *b = warp_sum(*b);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    __syncthreads();
+    if (lane == 0) smem[2 * warp] = *a, smem[2 * warp + 1] = *b;
+    __syncthreads();
+    *a = warp_sum(lane < nw ? smem[2 * lane] : 0.f);
+    *b = warp_sum(lane < nw ? smem[2 * lane + 1] : 0.f);
+}
+
 // Rows of 2049..16384 elements (multiple of 4): a CTA of 256 threads owns a row and keeps it in
 // registers (V float4 chunks per thread), so HBM still sees one read and one write per element.
+// Shorter rows come here too when there are at most eight per SM: a warp per row then takes as long as its chain of loads,
+// divisions and splits, most of it cold instructions (24 x 768 with pieces, between events: 9.6 -> 6.4 us, of
+// which 6 are the events').
 template <int MODE, int V>
 __global__ void __launch_bounds__(256) row_cta_kernel(RowParams p) {
     grid_dependency_sync();
-    __shared__ float smem[8];
+    __shared__ float smem[16];
     const long long row = blockIdx.x;
     const int chunks = (int)(p.cols >> 2);
     const float4 *xr = reinterpret_cast<const float4 *>(p.x + row * p.cols);
@@ -203,6 +224,9 @@ __global__ void __launch_bounds__(256) row_cta_kernel(RowParams p) {
         const int c = threadIdx.x + 256 * i;
         if (c < chunks) v[i] = __ldg(xr + c);
     }
+    float g0 = 0.f, b0 = 0.f;
+    const bool one_gb = MODE == ROW_LN && p.gamma_stride == 0 && p.beta_stride == 0;
+    if (one_gb) g0 = __ldg(p.gamma), b0 = __ldg(p.beta);
     if (MODE == ROW_LN) {
         float s1 = 0.f, s2 = 0.f;
 #pragma unroll
@@ -211,8 +235,7 @@ __global__ void __launch_bounds__(256) row_cta_kernel(RowParams p) {
                 s1 += (v[i].x + v[i].y) + (v[i].z + v[i].w);
                 s2 += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
             }
-        s1 = block_reduce(s1, false, smem);
-        s2 = block_reduce(s2, false, smem);
+        block_sum2(&s1, &s2, smem);
         const float n = (float)p.cols;
         const float mean = s1 / n;
         const float var = s2 / n - mean * mean;
@@ -222,11 +245,17 @@ __global__ void __launch_bounds__(256) row_cta_kernel(RowParams p) {
             const int c = threadIdx.x + 256 * i;
             if (c < chunks) {
                 const int e = c * 4;
+                const float4 g = one_gb ? make_float4(g0, g0, g0, g0)
+                                        : make_float4(p.gamma[(e + 0) * p.gamma_stride], p.gamma[(e + 1) * p.gamma_stride], p.gamma[(e + 2) * p.gamma_stride],
+                                                      p.gamma[(e + 3) * p.gamma_stride]);
+                const float4 b = one_gb ? make_float4(b0, b0, b0, b0)
+                                        : make_float4(p.beta[(e + 0) * p.beta_stride], p.beta[(e + 1) * p.beta_stride], p.beta[(e + 2) * p.beta_stride],
+                                                      p.beta[(e + 3) * p.beta_stride]);
                 float4 o;
-                o.x = (v[i].x - mean) / denom * p.gamma[(e + 0) * p.gamma_stride] + p.beta[(e + 0) * p.beta_stride];
-                o.y = (v[i].y - mean) / denom * p.gamma[(e + 1) * p.gamma_stride] + p.beta[(e + 1) * p.beta_stride];
-                o.z = (v[i].z - mean) / denom * p.gamma[(e + 2) * p.gamma_stride] + p.beta[(e + 2) * p.beta_stride];
-                o.w = (v[i].w - mean) / denom * p.gamma[(e + 3) * p.gamma_stride] + p.beta[(e + 3) * p.beta_stride];
+                o.x = (v[i].x - mean) / denom * g.x + b.x;
+                o.y = (v[i].y - mean) / denom * g.y + b.y;
+                o.z = (v[i].z - mean) / denom * g.z + b.z;
+                o.w = (v[i].w - mean) / denom * g.w + b.w;
                 row_store4(p, row * p.cols + 4LL * c, o);
             }
         }
@@ -308,7 +337,7 @@ static sage_status launch_rows(Context &ctx, RowParams p, const char *name) {
                          (MODE == ROW_LSE || reinterpret_cast<uintptr_t>(p.y) % 16 == 0) &&
                          (!p.out.hi || (reinterpret_cast<uintptr_t>(p.out.hi) % 16 == 0 && p.out.plane % 4 == 0));
     if (p.out.h2 && !(aligned && rows_write_pieces(p.x, p.cols))) return ctx.fail(SAGE_ERR_INVALID, "row kernel: half-precision pieces need whole groups");
-    if (p.cols % 4 == 0 && p.cols <= 2048 && aligned) {
+    if (p.cols % 4 == 0 && p.cols <= 2048 && aligned && (p.cols <= 256 || p.rows > 8LL * ctx.sm_count)) {
         const int chunks = (int)(p.cols / 4);
         const int v = (chunks + 31) / 32;
         // a warp per row; with few rows per SM smaller blocks spread them more evenly ([4096, 768]: 12.1 -> 11.0 us)
@@ -324,7 +353,9 @@ static sage_status launch_rows(Context &ctx, RowParams p, const char *name) {
         const int v = (int)((p.cols / 4 + 255) / 256);
         const unsigned blocks = (unsigned)p.rows;
         cudaStream_t s = ctx.stream();
-        if (v <= 4) err = launch_dependent(ctx.pdl, s, row_cta_kernel<MODE, 4>, dim3(blocks), dim3(256), 0, p);
+        if (v <= 1) err = launch_dependent(ctx.pdl, s, row_cta_kernel<MODE, 1>, dim3(blocks), dim3(256), 0, p);
+        else if (v <= 2) err = launch_dependent(ctx.pdl, s, row_cta_kernel<MODE, 2>, dim3(blocks), dim3(256), 0, p);
+        else if (v <= 4) err = launch_dependent(ctx.pdl, s, row_cta_kernel<MODE, 4>, dim3(blocks), dim3(256), 0, p);
         else if (v <= 8) err = launch_dependent(ctx.pdl, s, row_cta_kernel<MODE, 8>, dim3(blocks), dim3(256), 0, p);
         else err = launch_dependent(ctx.pdl, s, row_cta_kernel<MODE, 16>, dim3(blocks), dim3(256), 0, p);
     } else {
