@@ -136,6 +136,24 @@ std::string map_expr_text_remap(const MapExpr &e, const std::vector<int> &remap)
     return map_expr_text(walk(e));
 }
 
+// The map with operand i taken from operand remap[i] of the result's list (numbered in order of first use).
+std::shared_ptr<Operator> map_merge_inputs(const Operator &op, const std::vector<int> &remap) {
+    const MapOp &m = dynamic_cast<const MapOp &>(op);
+    auto f = std::make_shared<MapOp>();
+    f->primitive = false;
+    f->out = m.out;
+    std::function<MapExpr(const MapExpr &)> walk = [&](const MapExpr &x) {
+        MapExpr r = x;
+        if (r.kind == MapExpr::Input) r.input = remap[r.input];
+        for (auto &a : r.args) a = walk(a);
+        return r;
+    };
+    f->expr = walk(m.expr);
+    for (size_t i = 0; i < remap.size(); ++i)
+        if (remap[i] == (int)f->in.size()) f->in.push_back(m.in[i]);
+    return f;
+}
+
 static MapExpr input_expr(int i) {
     MapExpr e;
     e.kind = MapExpr::Input;

@@ -41,6 +41,7 @@ std::shared_ptr<Operator> map_over_expanded(const Operator &op, const Array &ext
 std::shared_ptr<Operator> make_expand_op(const TensorDesc &in, const Array &extents);
 bool is_expand_op(const Operator &op);
 std::string map_expr_text_remap(const MapExpr &e, const std::vector<int> &remap);
+std::shared_ptr<Operator> map_merge_inputs(const Operator &op, const std::vector<int> &remap);
 bool is_view_op(const Operator &op);
 bool is_reshape_op(const Operator &op);
 bool is_gemm_op(const Operator &op);
@@ -209,6 +210,68 @@ static Node build(const Var &v, const std::unordered_set<Origin *> &inputs, bool
     n.op = op;
     n.args = std::move(folded);
     return n;
+}
+
+// A state that one routine reads, and there only as several operands of one elementwise map (h of GELU: 0.5 h (1 + erf(h / 1.41)))
+// needs no tensor of its own: the map takes it once, so that its subtree can follow and, where it ends in a product, the map
+// become that product's epilogue.  Returns where the state's subtree belongs, or null.
+static void count_leaf(Node &n, Origin *key, int *total) {
+    if (n.is_data) {
+        *total += n.var.key() == key;
+        return;
+    }
+    for (Node &a : n.args) count_leaf(a, key, total);
+}
+static Node *sole_map_reader(Node &n, Origin *key, int total) {
+    if (n.is_data) return nullptr;
+    int here = 0;
+    for (Node &a : n.args) here += a.is_data && a.var.key() == key;
+    if (here == total && here >= 2 && map_expr_of(*n.op)) return &n;
+    for (Node &a : n.args)
+        if (Node *m = sole_map_reader(a, key, total)) return m;
+    return nullptr;
+}
+static bool inline_state(Node &root, const Var &state, const std::unordered_set<Origin *> &state_inputs, bool fusion, bool pattern) {
+    int total = 0;
+    count_leaf(root, state.key(), &total);
+    Node *m = total >= 2 ? sole_map_reader(root, state.key(), total) : nullptr;
+    if (!m) return false;
+    std::vector<int> remap(m->args.size());
+    int first = -1, next = 0;
+    for (size_t i = 0; i < m->args.size(); ++i) {
+        const bool same = m->args[i].is_data && m->args[i].var.key() == state.key();
+        if (same && first >= 0) {
+            if (!(m->op->in[i].shape == m->op->in[first].shape)) return false;
+            remap[i] = remap[first];
+            continue;
+        }
+        if (same) first = (int)i;
+        remap[i] = next++;
+    }
+    if (!m->op->in[first].shape.has_default_strides() || m->op->in[first].shape.offset || m->op->in[first].shape.extents != m->op->out.shape.extents) return false;
+    std::shared_ptr<Operator> op = map_merge_inputs(*m->op, remap);
+    std::vector<Node> args;
+    for (size_t i = 0; i < m->args.size(); ++i) {
+        if (remap[i] < (int)args.size()) continue;
+        args.push_back(std::move(m->args[i]));
+    }
+    const int at = remap[first];
+    Node sub = build(state, state_inputs, fusion, pattern, true);
+    if (std::shared_ptr<Operator> f = fuse_ops(*op, *sub.op, at)) {
+        std::vector<Node> all;
+        for (size_t i = 0; i < args.size(); ++i) {
+            if ((int)i != at) all.push_back(std::move(args[i]));
+            else
+                for (Node &g : sub.args) all.push_back(std::move(g));
+        }
+        m->op = f;
+        m->args = std::move(all);
+    } else {
+        args[at] = std::move(sub);
+        m->op = op;
+        m->args = std::move(args);
+    }
+    return true;
 }
 
 // ------------------------------------------------------------------------------ GEMM lowering
@@ -725,17 +788,39 @@ static std::unique_ptr<Program> compile(const std::vector<Var> &x, std::vector<V
             for (const Var &o : outs) p->routines.emplace(o.key(), r);
         }
     }
+    std::unordered_map<Origin *, int> readers_of;
+    for (auto &kv : states)
+        for (const Var &v : kv.second) ++readers_of[v.key()];
     for (const Var &node : state_order) {
         if (grouped.count(node.key())) continue;
         Routine r;
         r.inputs = states[node.key()];
         r.output = node;
         std::unordered_set<Origin *> in_keys;
-        for (const Var &v : r.inputs) {
-            in_keys.insert(v.key());
-            if (v.is_op()) ++p->consumers[v.key()];
-        }
+        for (const Var &v : r.inputs) in_keys.insert(v.key());
         r.root = build(node, in_keys, fusion, pattern, true);
+        if (pattern && tc) {
+            for (size_t i = 0; i < r.inputs.size(); ++i) {
+                const Var s = r.inputs[i];
+                auto it = p->routines.find(s.key());
+                if (it == p->routines.end() || it->second.row || yset.count(s.key()) || readers_of[s.key()] != 1) continue;
+                if (it->second.root.is_data || !is_gemm_op(*it->second.root.op)) continue;
+                std::unordered_set<Origin *> keys;
+                for (const Var &v : it->second.inputs) keys.insert(v.key());
+                if (!inline_state(r.root, s, keys, fusion, pattern)) continue;
+                r.inputs.erase(r.inputs.begin() + (long)i);
+                for (const Var &v : it->second.inputs) {
+                    if (in_keys.insert(v.key()).second) r.inputs.push_back(v);
+                    else --readers_of[v.key()];
+                }
+                for (const Var &v : it->second.inputs)
+                    if (v.is_op()) --p->consumers[v.key()];
+                p->routines.erase(it);
+                i = (size_t)-1;  // a product's own operands may follow
+            }
+        }
+        for (const Var &v : r.inputs)
+            if (v.is_op()) ++p->consumers[v.key()];
         if (pattern) {
             lower(r.root, tc, softmax_in_gemm, attention && tc && attention_enabled());
             if (tc) group_gemms(r.root);

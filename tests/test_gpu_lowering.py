@@ -605,3 +605,25 @@ def test_convolution_with_few_input_channels(shape, filt, stride, pad, dil):
     finally:
         lowered.close()
         plain.close()
+
+
+@pytest.mark.parametrize("m,n", [(70, 128), (300, 200), (2048, 256)])
+def test_a_product_read_twice_by_one_map(m, n):
+    """GELU reads its input twice: the map still becomes the product's epilogue, unless the product is a target itself."""
+    rng = np.random.default_rng(m)
+    x, w, b = (rng.uniform(-1, 1, s).astype(np.float32) for s in ((m, 128), (128, n), (n,)))
+    ctx = S.Context(0)
+    try:
+        h = S.matmul(ctx.var(x), ctx.var(w)) + ctx.var(b)
+        y = h * 0.5 * (S.erf(h / float(np.sqrt(2.0))) + 1.0)
+        got = y.eval(ctx)
+        assert "map{" not in ctx.describe()
+        h64 = x.astype(np.float64) @ w + b
+        from math import erf
+        want = 0.5 * h64 * (1.0 + np.vectorize(erf)(h64 / np.sqrt(2.0)))
+        assert gemm_err(got, want) <= 1e-5
+        ctx.clear()
+        ctx.eval(y, h)
+        assert gemm_err(ctx.read(h), h64) <= 1e-5 and gemm_err(ctx.read(y), want) <= 1e-5
+    finally:
+        ctx.close()
