@@ -378,6 +378,8 @@ struct GemmOp : Operator {
     bool conv_small_c() const {
         return conv && img[3] >= 1 && img[3] <= 4 && win.dil_w == 1 && win.ker_w >= 1 && win.ker_w <= 8 && n % 4 == 0 && img[0] * img[4] * img[5] >= 512;
     }
+    // ... and with columns two apart as a kernel of its own, on half-precision pieces (kernels/conv_first_device.inc)
+    bool conv_first() const { return conv_small_c() && !ta && !tb && !conv_raw_enabled() && img[0] <= 65535 && !folded && k::conv_first_ok(win.ker_h, win.stride_w, img[5]); }
     struct PackedFilter {  // the filter as the B operand of that GEMM, kept until the filter is rewritten
         const Storage *key = nullptr;
         uint64_t version = 0;
@@ -408,6 +410,7 @@ struct GemmOp : Operator {
         if (h2) return compute_h2(x, ctx, y, emit, emit_h2, only);
         if (!lowered && !attn && !batched && ctx.opts().pattern_fusion == 0 && ctx.opts().gemm_backend != 1 && k::gemm_tc_shape_ok(m, n, k, batch))
             return compute_h2(x, ctx, y, false, false, false);  // the operator by itself
+        if (conv_first() && x[0].desc.shape.has_default_strides() && x[1].desc.shape.has_default_strides() && !x[0].data->planes_only) return compute_first(x, ctx, y, emit, emit_h2, only);
         if (emit_h2 && !attn) return ctx.fail(SAGE_ERR_INVALID, "internal: the tf32 product does not write half-precision pieces");
         if (attn) return compute_attention(x, ctx, y, emit, emit_h2, only);
         if (!lowered && (ctx.opts().gemm_backend == 1 || !k::gemm_tc_shape_ok(m, n, k, batch))) {
@@ -627,6 +630,76 @@ struct GemmOp : Operator {
             }
         }
         return k::gemm_tc_run(ctx, g);
+    }
+    sage_status compute_first(const std::vector<Tensor> &x, Context &ctx, Tensor *y, bool emit, bool emit_h2, bool only) {
+        const long long N = img[0], H = img[1], W = img[2], OH = img[4], OW = img[5];
+        // a row holds the left padding, the image, and enough behind it for the last pixel's eight
+        const long long wp = (std::max(W + 2 * win.pad_w, (OW - 1) * win.stride_w + 8) + 1) / 2 * 2;
+        const long long hp = std::max(H + 2 * win.pad_h, (OH - 1) * win.stride_h + (long long)(win.ker_h - 1) * win.dil_h + 1);
+        const long long plane = (N * hp * wp * 4 + 127) / 128 * 128, piece_bytes = plane * 4 + 4096;  // a tile's last row is read 2112 bytes on
+        struct Held {
+            Context &c;
+            Block *b;
+            ~Held() {
+                if (b) c.allocator().free(b);  // stream-ordered: reused only by launches enqueued after the product
+            }
+        } image{ctx, ctx.allocator().alloc((size_t)(piece_bytes + N * 4 + N * 32 * 4))};
+        if (!image.b) return ctx.fail(SAGE_ERR_OOM, "out of memory for the channel-padded image");
+        k::FirstConv f;
+        unsigned short *hi = reinterpret_cast<unsigned short *>(image.b->ptr);
+        float *scale = reinterpret_cast<float *>(image.b->ptr + piece_bytes);
+        sage_status st = k::pack_first_image(ctx, (const float *)x[0].ptr(), N, H, W, img[3], hp, wp, win.pad_h, win.pad_w, hi, plane, scale, reinterpret_cast<unsigned *>(scale + N));
+        if (st) return st;
+        const Storage *key = x[1].data.get();
+        const long long chans = (n + 63) / 64 * 64, filter_bytes = chans * win.ker_h * 128;
+        if (!packed_filter || packed_filter->key != key || packed_filter->version != key->version) {
+            auto pf = std::make_shared<PackedFilter>();
+            pf->alloc = ctx.allocator_ptr();
+            pf->key = key;
+            pf->version = key->version;
+            pf->block = ctx.allocator().alloc((size_t)(filter_bytes + chans * 4));
+            if (!pf->block) return ctx.fail(SAGE_ERR_OOM, "out of memory for the re-laid filter");
+            st = k::pack_first_filter(ctx, (const float *)x[1].ptr(), win.ker_h, win.ker_w, (int)img[3], (int)n, reinterpret_cast<unsigned short *>(pf->block->ptr),
+                                      reinterpret_cast<float *>(pf->block->ptr + filter_bytes));
+            if (st) return st;
+            packed_filter = pf;
+        }
+        f.img = hi;
+        f.img_plane = plane;
+        f.filter = reinterpret_cast<const unsigned short *>(packed_filter->block->ptr);
+        f.hp = hp;
+        f.wp = wp;
+        f.kh = win.ker_h;
+        f.dil_h = win.dil_h;
+        f.stride_h = win.stride_h;
+        f.img_scale = scale;
+        f.filter_scale = reinterpret_cast<const float *>(packed_filter->block->ptr + filter_bytes);
+        k::H2Gemm g;
+        g.n = n;
+        g.img_n = N;
+        g.out_h = OH;
+        g.out_w = OW;
+        g.c = (float *)y->ptr();
+        g.ldc = n;
+        k::PlaneOut o;
+        st = attach_forms(ctx, y, emit, emit_h2, &o);
+        if (st) return st;
+        g.c_hi = o.hi;
+        g.c_plane = o.plane;
+        g.h_hi = o.h2;
+        g.h_plane = o.h2_plane;
+        g.h_scale = o.h2_scale;
+        g.naux = naux();
+        g.epilogue = epilogue;
+        for (int i = 0; i < g.naux; ++i) {
+            st = aux_strides(ctx, x[2 + i], &g.aux[i]);
+            if (st) return st;
+        }
+        if (only) {
+            g.c = nullptr;
+            y->data->planes_only = true;
+        }
+        return k::conv_first_run(ctx, g, f);
     }
     // The same product on half-precision pieces (see assign_h2).
     sage_status compute_h2(const std::vector<Tensor> &x, Context &ctx, Tensor *y, bool emit, bool emit_h2, bool only) {
@@ -1160,7 +1233,7 @@ bool gemm_is_h2(const Operator &op) {  // reads its operands in half-precision p
 bool gemm_emits_h2(const Operator &op) {
     const GemmOp *g = as_gemm(op);
     if (!g) return grouped_gemm_is_h2(op) && op.out.shape.extents.back() % 64 == 0;
-    if (!(g->h2 || g->attn) || g->n % 64) return false;
+    if (!(g->h2 || g->attn || g->conv_first()) || g->n % 64) return false;
     return !g->folded || (g->ldc % 64 == 0 && g->sc0 % 64 == 0 && g->sc1 % 64 == 0);
 }
 

@@ -14,6 +14,8 @@
 
 #include "kernels.h"
 #include "gemm_tc_device.inc"  // split_tf32_value
+#include "gemm_h2_device.inc"  // h2_split2
+#include "launch.h"
 
 namespace sage {
 namespace k {
@@ -352,6 +354,119 @@ sage_status pack_small_c_filter(Context &ctx, const float *filt, int kh, int kw,
     if (kw * 4 > 32 || c > 4) return ctx.fail(SAGE_ERR_INVALID, "pack_small_c_filter: window too wide");
     pack_small_c_filter_kernel<<<grid_for(ctx, (long long)kh * 32 * oc), 256, 0, ctx.stream()>>>(filt, hi, hi + plane, kh, kw, c, oc);
     return ctx.check_cuda(cudaGetLastError(), "pack_small_c_filter launch");
+}
+
+// ---- the first convolution on half-precision pieces
+constexpr int kAmaxParts = 32;  // blocks per image that look for its largest magnitude
+__global__ void __launch_bounds__(256) first_amax_kernel(const float *__restrict__ img, long long len, int vec, unsigned *__restrict__ parts) {
+    __shared__ unsigned warps[8];
+    grid_dependency_sync();
+    const float *s = img + blockIdx.y * len;
+    unsigned m = 0;
+    if (vec) {
+        const float4 *v = reinterpret_cast<const float4 *>(s);
+#pragma unroll 4
+        for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < len / 4; i += kAmaxParts * 256) {
+            const float4 x = __ldg(v + i);
+            m = max(m, max(max(sage_tc::h2_finite_bits(x.x), sage_tc::h2_finite_bits(x.y)), max(sage_tc::h2_finite_bits(x.z), sage_tc::h2_finite_bits(x.w))));
+        }
+    } else {
+        for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < len; i += kAmaxParts * 256) m = max(m, sage_tc::h2_finite_bits(s[i]));
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) warps[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        m = __reduce_max_sync(0xffffffffu, threadIdx.x < 8 ? warps[threadIdx.x] : 0u);
+        if (threadIdx.x == 0) parts[blockIdx.y * kAmaxParts + blockIdx.x] = m;
+    }
+}
+// A block takes four rows of the padded image, a thread two neighbouring pixels: 16 bytes of each piece.
+__global__ void __launch_bounds__(128) pack_first_kernel(const float *__restrict__ img, unsigned short *__restrict__ hi, long long plane, long long rows, int h, int w, int c, int hp,
+                                                         int wp, int pad_h, int pad_w, const unsigned *__restrict__ parts, float *__restrict__ scale) {
+    grid_dependency_sync();
+    for (int i = 0; i < 4; ++i) {
+        const long long r = (long long)blockIdx.x * 4 + i;
+        if (r >= rows) return;
+        const long long b = r / hp;
+        const int y = (int)(r - b * hp) - pad_h;
+        float s;
+        const float f = sage_tc::h2_factor(__reduce_max_sync(0xffffffffu, __ldg(parts + b * kAmaxParts + (threadIdx.x & 31))), &s);
+        if (y == -pad_h && threadIdx.x == 0) scale[b] = s;
+        for (int x2 = threadIdx.x; x2 < wp / 2; x2 += 128) {
+            float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            if (y >= 0 && y < h) {
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const int x = 2 * x2 + q - pad_w;
+                    if (x < 0 || x >= w) continue;
+                    const float *px = img + ((b * h + y) * (long long)w + x) * c;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (k < c) v[q * 4 + k] = __ldg(px + k);
+                }
+            }
+            uint4 a, l;
+            sage_tc::h2_split2(v[0], v[1], f, &a.x, &l.x);
+            sage_tc::h2_split2(v[2], v[3], f, &a.y, &l.y);
+            sage_tc::h2_split2(v[4], v[5], f, &a.z, &l.z);
+            sage_tc::h2_split2(v[6], v[7], f, &a.w, &l.w);
+            unsigned short *at = hi + (r * wp + 2 * x2) * 4;
+            *reinterpret_cast<uint4 *>(at) = a;
+            *reinterpret_cast<uint4 *>(at + plane) = l;
+        }
+    }
+}
+// One block per output channel, those that fill up the last 64 included (zeros).
+__global__ void __launch_bounds__(128) pack_first_filter_kernel(const float *__restrict__ f, unsigned short *__restrict__ out, float *__restrict__ scale, int kh, int kw, int c, int oc) {
+    __shared__ unsigned warps[4];
+    grid_dependency_sync();
+    const int o = blockIdx.x;
+    auto value = [&](int i) {  // k = ky * 32 + kx * 4 + channel
+        const int ky = i >> 5, kx = (i >> 2) & 7, cc = i & 3;
+        return (o < oc && kx < kw && cc < c) ? f[(((long long)ky * kw + kx) * c + cc) * oc + o] : 0.f;
+    };
+    unsigned m = 0;
+    for (int i = threadIdx.x; i < kh * 32; i += 128) m = max(m, sage_tc::h2_finite_bits(value(i)));
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) warps[threadIdx.x >> 5] = m;
+    __syncthreads();
+    m = max(max(warps[0], warps[1]), max(warps[2], warps[3]));
+    float s;
+    const float factor = sage_tc::h2_factor(m, &s);
+    if (threadIdx.x == 0) scale[o] = s;
+    unsigned short *tile = out + (long long)(o >> 6) * kh * 4096;
+    for (int i = threadIdx.x * 2; i < kh * 32; i += 256) {
+        unsigned a, l;
+        sage_tc::h2_split2(value(i), value(i + 1), factor, &a, &l);
+        const int at = ((i >> 3) * 128 + (o & 63)) * 8 + (i & 7);
+        *reinterpret_cast<unsigned *>(tile + at) = a;
+        *reinterpret_cast<unsigned *>(tile + at + 512) = l;
+    }
+}
+
+sage_status pack_first_image(Context &ctx, const float *img, long long n, long long h, long long w, long long c, long long hp, long long wp, int pad_h, int pad_w,
+                             unsigned short *hi, long long plane, float *scale, unsigned *parts) {
+    if (c < 1 || c > 4 || wp % 2 || plane % 8 || reinterpret_cast<uintptr_t>(hi) % 16 || h > 0x7fffffffLL || w > 0x7fffffffLL || hp > 0x7fffffffLL || wp > 0x7fffffffLL || n > 65535 ||
+        n * hp / 4 > 0x7ffffff0LL)
+        return ctx.fail(SAGE_ERR_INVALID, "pack_first_image: bad arguments");
+    ctx.note_launch("pack_small_c");
+    ctx.note_launch("pack_small_c");
+    if (ctx.dry()) return SAGE_OK;
+    const long long len = h * w * c;
+    const int vec = len % 4 == 0 && reinterpret_cast<uintptr_t>(img) % 16 == 0;
+    launch_dependent(ctx.pdl, ctx.stream(), first_amax_kernel, dim3(kAmaxParts, (unsigned)n), dim3(256), 0, img, len, vec, parts);
+    launch_dependent(ctx.pdl, ctx.stream(), pack_first_kernel, dim3((unsigned)((n * hp + 3) / 4)), dim3(128), 0, img, hi, plane, n * hp, (int)h, (int)w, (int)c, (int)hp, (int)wp, pad_h,
+                     pad_w, (const unsigned *)parts, scale);
+    return ctx.check_cuda(cudaGetLastError(), "pack_first_image launch");
+}
+
+sage_status pack_first_filter(Context &ctx, const float *filt, int kh, int kw, int c, int oc, unsigned short *out, float *scale) {
+    ctx.note_launch("pack_small_c_filter");
+    if (ctx.dry()) return SAGE_OK;
+    if (kw > 8 || c > 4) return ctx.fail(SAGE_ERR_INVALID, "pack_first_filter: window too wide");
+    return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), pack_first_filter_kernel, dim3((unsigned)((oc + 63) / 64 * 64)), dim3(128), 0, filt, out, scale, kh, kw, c, oc),
+                          "pack_first_filter launch");
 }
 
 sage_status im2col(Context &ctx, const float *img, float *col, long long n, long long img_h, long long img_w,

@@ -18,6 +18,8 @@
 #include "gemm_tc_device_src.h"
 #include "gemm_h2_device_src.h"
 #include "attn_tc_device_src.h"
+#include "conv_first_device.inc"
+#include "conv_first_device_src.h"
 
 namespace sage {
 void *driver_symbol(const char *name);  // runtime/context.cc
@@ -733,6 +735,96 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
     void *params[5] = {&map_a, &map_a2, &map_b, &map_b2, &p};
     // launch lists have one name for a tensor-core product; verbose ones tell the kernels apart
     return ctx.launch(mod, "gemm_tc_h2", gr, bl, (uint32_t)smem, params, ctx.verbose_names ? label.c_str() : "gemm_tc_3xtf32", true, sliced ? cut.slices : ctas);
+}
+
+// ---------------------------------------------------------------------------------- the first convolution
+// Columns two apart (the descriptor's row pitch), the filter and two stages of rows beside the store's staging, and at least six
+// tenths of the 128 pixels of a tile inside the row: below that the gathered operand's full tiles are the better ones.
+bool conv_first_ok(int kh, int stride_w, long long out_w) { return stride_w == 2 && kh >= 1 && kh <= 11 && out_w * 10 >= (out_w + 127) / 128 * 128 * 6; }
+
+sage_status conv_first_run(Context &ctx, const H2Gemm &g, const FirstConv &f) {
+    if (!conv_first_ok(f.kh, 2, g.out_w) || g.n < 1 || f.wp % 2 || f.img_plane % 8 || g.naux < 0 || g.naux > kMaxAux || (!g.c && !g.c_hi && !g.h_hi) ||
+        g.img_n * g.out_h * ((g.out_w + 127) / 128) > 0x3fffffffLL || g.img_n * g.out_h * g.out_w > 0x7fffffffLL)
+        return ctx.fail(SAGE_ERR_INVALID, "conv_first: bad description");
+    FirstParams p{};
+    p.h.c = g.c;
+    p.h.c_hi = g.c_hi;
+    p.h.c_plane = g.c_plane;
+    p.h.h_hi = g.h_hi;
+    p.h.h_plane = g.h_plane;
+    p.h.h_scale = g.h_scale;
+    p.h.ldc = g.ldc;
+    p.h.nbc0 = 1;
+    p.h.n = (int)g.n;
+    p.h.sa = f.img_scale;
+    p.h.sb = f.filter_scale;
+    p.h.status = ctx.status_word_dev;
+    p.img = f.img;
+    p.img_plane = f.img_plane;
+    p.filter = f.filter;
+    p.hp = (int)f.hp;
+    p.wp = (int)f.wp;
+    p.kh = f.kh;
+    p.dil_h = f.dil_h;
+    p.stride_h = f.stride_h;
+    p.out_h = (int)g.out_h;
+    p.out_w = (int)g.out_w;
+    p.segs = (int)((g.out_w + 127) / 128);
+    p.tiles_n = (int)((g.n + 63) / 64);
+    p.num_tiles = (int)(g.img_n * g.out_h * p.segs);
+    const bool vec = g.n % 4 == 0 && g.ldc % 4 == 0 && (!g.c || aligned16(g.c)) && (!g.c_hi || (aligned16(g.c_hi) && g.c_plane % 4 == 0));
+    bool aux_vec = true;
+    int rowinv = 0, per_col = 0;
+    for (int i = 0; i < g.naux; ++i) {
+        TcAux &a = p.h.aux[i];
+        a.ptr = g.aux[i].ptr;
+        a.s0 = a.s1 = 0;
+        a.sr = g.aux[i].sr;
+        a.sc = g.aux[i].sc;
+        if (a.sc != 0 && a.sc != 1) return ctx.fail(SAGE_ERR_INVALID, "conv_first: epilogue operand column stride must be 0 or 1");
+        if (a.sc == 1) aux_vec = aux_vec && aligned16(a.ptr) && a.sr % 4 == 0;
+        if (a.sr == 0) rowinv |= 1 << i;
+        if (a.sc != 0) per_col |= 1 << i;
+    }
+    p.h.vec_ok = vec ? 1 : 0;
+    if (g.h_hi && (!vec || g.n % 64 || g.ldc % 64 || !aligned16(g.h_hi) || g.h_plane % 8)) return ctx.fail(SAGE_ERR_INVALID, "conv_first: a result in half-precision pieces needs whole groups of 64 columns");
+    const int staging = kEpiWarps * kStageBytesPerWarp, stage_bytes = f.kh * 2 * kFirstRowBytes, filter_bytes = f.kh * 8192;
+    p.stages = (227 * 1024 - 2048 - staging - filter_bytes) / stage_bytes;
+    if (p.stages > 4) p.stages = 4;
+    const size_t smem = (size_t)filter_bytes + (size_t)p.stages * stage_bytes + staging + 1024;
+    long long ctas = ctx.sm_count / p.tiles_n;
+    if (ctas < 1) ctas = 1;
+    if (ctas > p.num_tiles) ctas = p.num_tiles;
+    const int out_mask = (g.c ? 1 : 0) | (g.c_hi ? 2 : 0) | (g.h_hi ? 4 : 0);
+    char num[96];
+    snprintf(num, sizeof num, "conv_first %d %d %d %d %d\n", aux_vec ? 1 : 0, g.naux, rowinv, per_col, out_mask);
+    const std::string key = num + g.epilogue;
+    Module *mod = ctx.module_find(key);
+    if (!mod) {
+        std::string src = map_prelude_text();
+        src += "struct __align__(64) CUtensorMap { unsigned long long opaque[16]; };\n";
+        auto define = [&](const char *name, int v) { src += std::string("#define ") + name + " " + std::to_string(v) + "\n"; };
+        define("SAGE_EPI_ROWINV", rowinv);
+        define("SAGE_EPI_COLS", per_col);
+        define("SAGE_EPI_OUT", out_mask);
+        define("SAGE_EPI_NAUX", g.naux);
+        define("SAGE_H2_AUX_VEC", aux_vec ? 1 : 0);
+        src += "#define SAGE_EPI_EXPR(x0, x1, x2, x3) (" + (g.epilogue.empty() ? std::string("x0") : g.epilogue) + ")\n";
+        src += kGemmTcDeviceSrc;
+        src += kGemmH2DeviceSrc;
+        src += kConvFirstDeviceSrc;
+        src += "\nextern \"C\" __global__ void __launch_bounds__(sage_tc::kThreads, 1)\n"
+               "conv_first_h2(const __grid_constant__ sage_tc::FirstParams p) {\n    sage_tc::conv_first_body(p);\n}\n";
+        sage_status st = ctx.module_get(src, &mod);
+        if (st) return st;
+        ctx.module_remember(key, mod);
+    }
+    std::string label;
+    if (ctx.verbose_names) label = "conv_first_h2[" + std::to_string(g.img_n * g.out_h * g.out_w) + "x" + std::to_string(g.n) + "x" + std::to_string(f.kh * 32) + "]o" + std::to_string(out_mask);
+    const uint32_t gr[3] = {(uint32_t)(ctas * p.tiles_n), 1, 1}, bl[3] = {(uint32_t)kThreads, 1, 1};
+    void *params[1] = {&p};
+    // launch lists have one name for a tensor-core product; verbose ones tell the kernels apart
+    return ctx.launch(mod, "conv_first_h2", gr, bl, (uint32_t)smem, params, ctx.verbose_names ? label.c_str() : "gemm_tc_3xtf32", true);
 }
 
 // ---------------------------------------------------------------------------------- fused attention

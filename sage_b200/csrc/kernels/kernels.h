@@ -74,6 +74,11 @@ sage_status col2im(Context &ctx, const float *col, float *img, long long n, long
 sage_status pack_small_c_image(Context &ctx, const float *img, long long n, long long h, long long w, long long c, long long hp, long long wp,
                                int pad_h, int pad_w, float *hi, long long plane);
 sage_status pack_small_c_filter(Context &ctx, const float *filt, int kh, int kw, int c, int oc, float *hi, long long plane);
+// The first convolution on half-precision pieces (conv_first_device.inc): the image as [n, hp, wp, 4] in pieces with a scale per image
+// (wp even; `parts`: 32 words per image of scratch), the filter as [oc / 64][kh][4][piece][64][8] with a scale per channel.
+sage_status pack_first_image(Context &ctx, const float *img, long long n, long long h, long long w, long long c, long long hp, long long wp, int pad_h, int pad_w,
+                             unsigned short *hi, long long plane, float *scale, unsigned *parts);
+sage_status pack_first_filter(Context &ctx, const float *filt, int kh, int kw, int c, int oc, unsigned short *out, float *scale);
 sage_status pool2d(Context &ctx, bool is_max, const float *img, float *out, long long n, long long img_h,
                    long long img_w, long long chan, long long out_h, long long out_w, const Window &w);
 
@@ -192,6 +197,15 @@ struct H2Gemm {
     std::string epilogue;
 };
 sage_status gemm_h2_run(Context &ctx, const H2Gemm &g);
+// The first convolution.  g: result and epilogue, img_n / out_h / out_w, n = output channels; the operands as pack_first_* lay them.
+struct FirstConv {
+    const unsigned short *img = nullptr, *filter = nullptr;
+    long long img_plane = 0, hp = 0, wp = 0;
+    int kh = 0, dil_h = 1, stride_h = 1;
+    const float *img_scale = nullptr, *filter_scale = nullptr;
+};
+bool conv_first_ok(int kh, int stride_w, long long out_w);
+sage_status conv_first_run(Context &ctx, const H2Gemm &g, const FirstConv &f);
 // The whole product of plain fp32 operands.  With `scratch` (gemm_h2_scratch_bytes of device memory, 256-byte aligned)
 // nothing is taken from the allocator and K is not cut.
 size_t gemm_h2_scratch_bytes(const GemmArgs &g);

@@ -627,3 +627,29 @@ def test_a_product_read_twice_by_one_map(m, n):
         assert gemm_err(ctx.read(h), h64) <= 1e-5 and gemm_err(ctx.read(y), want) <= 1e-5
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("shape,filt,stride_h,pad,dil_h,off", [
+    ((3, 30, 156, 3), (7, 7, 3, 64), 2, (3, 3), 1, 0),     # rows of 78 output pixels: one tile, cut
+    ((2, 9, 256, 4), (1, 8, 4, 192), 1, (0, 3), 1, 0),     # a whole tile, the widest window, three column tiles
+    ((1, 21, 516, 1), (11, 3, 1, 40), 3, (2, 0), 1, 1),    # tiles of one row, the tallest filter, half a column tile, an image off the 16-byte grid
+    ((2, 40, 200, 2), (3, 5, 2, 68), 2, (1, 2), 3, 0),     # dilated rows
+])
+def test_first_convolution_on_pieces(shape, filt, stride_h, pad, dil_h, off):
+    """Columns two apart and at most four channels: overlapping windows read from whole image rows.  Images of unequal size in
+    one batch (a scale each); tolerance as for the other convolutions."""
+    rng = np.random.default_rng(sum(shape))
+    x = rng.standard_normal(shape).astype(np.float32) * (10.0 ** np.arange(shape[0], dtype=np.float32))[:, None, None, None]
+    f = (rng.standard_normal(filt) / np.sqrt(filt[0] * filt[1] * filt[2])).astype(np.float32)
+    b = rng.standard_normal(filt[3]).astype(np.float32)
+    ctx = S.Context(0)
+    try:
+        big = ctx.var(np.concatenate([np.zeros((off,) + shape[1:], np.float32), x]))
+        X = big.slice(0, off, off + shape[0]) * 1.0 if off else ctx.var(x)
+        y = S.relu(S.conv_2d(X, ctx.var(f), [stride_h, 2], list(pad), [dil_h, 1]) + ctx.var(b)).eval(ctx)
+        ref = np.maximum(conv64(x, f, (stride_h, 2), pad, (dil_h, 1)) + b, 0)
+        for i in range(shape[0]):
+            assert gemm_err(y[i], ref[i]) <= 1e-5
+        assert ctx.status_word() == 0
+    finally:
+        ctx.close()
