@@ -428,7 +428,7 @@ sage_status sage_pool2d(sage_ctx *ctx, int32_t is_max, const sage_tensor *x, con
     CTX_OR_FAIL(ctx);
     if (x->ndim != 4 || y->ndim != 4 || !contiguous(x) || !contiguous(y)) return C.fail(SAGE_ERR_INVALID, "pool2d: bad layout");
     return k::pool2d(C, is_max != 0, (const float *)tensor_ptr(x), (float *)tensor_ptr(y), x->extents[0], x->extents[1],
-                     x->extents[2], x->extents[3], y->extents[1], y->extents[2], to_window(w));
+                     x->extents[2], x->extents[3], y->extents[1], y->extents[2], to_window(w), k::PlaneOut());
 }
 
 // ---------------------------------------------------------------- multi-GPU

@@ -101,6 +101,8 @@ Var ops::conv_2d(const Var &x, const Var &filter, Pair stride, Pair pad, Pair di
     return view(matmul(c2, f2), {n, ch, cw, cout});
 }
 
+sage_status storage_h2_attach(Context &ctx, Storage &st);  // ops_gemm.cc
+
 // Pooling as one kernel: the same value as im2col followed by mean / max over [KH,KW], without the
 // KH*KW-times larger intermediate.
 struct Pool2dOp : Operator {
@@ -111,14 +113,29 @@ struct Pool2dOp : Operator {
         shape_fail("pool2d composite is not differentiated; grad walks the decomposed graph");
     }
     sage_status compute(const std::vector<Tensor> &x, Context &ctx, Tensor *y) override {
+        const bool emit_h2 = ctx.hint_emit_h2, only = emit_h2 && !ctx.hint_emit_planes && ctx.hint_planes_only;
+        ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = false;
         sage_status st = Tensor::uninit(ctx, out, y);
         if (st) return st;
         const Array &e = x[0].desc.shape.extents;
         const Array &o = out.shape.extents;
-        return k::pool2d(ctx, is_max, (const float *)x[0].ptr(), (float *)y->ptr(), e[0], e[1], e[2], e[3], o[1], o[2],
-                         window(ker, stride, pad, dil));
+        k::PlaneOut forms;
+        if (emit_h2) {
+            st = storage_h2_attach(ctx, *y->data);
+            if (st) return st;
+            forms.h2 = y->data->h2->pieces.hi;
+            forms.h2_plane = y->data->h2->pieces.plane;
+            forms.h2_scale = y->data->h2->pieces.scale;
+            y->data->planes_only = only;
+        }
+        return k::pool2d(ctx, is_max, (const float *)x[0].ptr(), only ? nullptr : (float *)y->ptr(), e[0], e[1], e[2], e[3], o[1], o[2],
+                         window(ker, stride, pad, dil), forms);
     }
 };
+bool pool_op_emits_h2(const Operator &op) {
+    const Pool2dOp *p = dynamic_cast<const Pool2dOp *>(&op);
+    return p && k::pool2d_writes_pieces(p->out.shape.extents[3]);
+}
 
 static Var pool(const Var &x, Pair ker, Pair stride, Pair pad, Pair dil, bool is_max) {
     Var col = im2col(x, ker, stride, pad, dil);

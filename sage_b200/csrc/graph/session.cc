@@ -69,6 +69,7 @@ std::shared_ptr<Operator> gemm_on_h2(const Operator &op, bool a_given, bool tc_e
 bool gemm_is_h2(const Operator &op);
 bool gemm_emits_h2(const Operator &op);
 bool row_op_emits_h2(const Operator &op);
+bool pool_op_emits_h2(const Operator &op);  // ops_conv.cc
 bool map_op_emits_h2(const Operator &op);
 std::string describe_gemm(const Operator &op);  // "{epilogue}" / "[store]" of a lowered GEMM, else empty
 
@@ -479,7 +480,7 @@ bool map_op_emits_planes(const Operator &op);
 static bool can_emit_planes(const Operator &op, bool tc) {
     return gemm_runs_on_tc(op, tc) || row_op_emits_planes(op) || is_grouped_gemm_op(op) || (tc && map_op_emits_planes(op));
 }
-static bool can_emit_h2(const Operator &op) { return gemm_emits_h2(op) || row_op_emits_h2(op) || map_op_emits_h2(op); }
+static bool can_emit_h2(const Operator &op) { return gemm_emits_h2(op) || row_op_emits_h2(op) || map_op_emits_h2(op) || pool_op_emits_h2(op); }
 
 // Products with weights run on half-precision pieces.  A program that also multiplies by the transposes of its activations
 // (training) keeps tf32 planes for those, and its weights as pieces with block scales (`blocks` below), which its optimizer

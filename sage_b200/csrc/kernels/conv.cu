@@ -213,51 +213,88 @@ __global__ void __launch_bounds__(256) col2im_quads_kernel(const float *__restri
     }
 }
 
-// One thread per output pixel and group of 4 channels when C % 4 == 0 (16-byte loads, one 64-bit
-// division per thread), else one thread per element.
-template <int VEC>
+// One thread per output pixel and group of 4 channels when C % 4 == 0 (16-byte loads, one 64-bit division per thread), else
+// one thread per element.  Nine taps are asked for at a time, then taken in the window's order: tap after tap a thread waited
+// for the cache each time (3 x 3 over 256 x 112 x 112 x 64: 358 us and a split pass of 62 -> 264 with pieces; 7 x 7
+// over 7 x 7 x 512 of one image, between events: 20.5 -> 12.7).  With pieces
+// asked for, 16 threads hold the 64 channels of a group: no split pass reads the result again.
+template <int VEC, class I>
 __global__ void __launch_bounds__(256) pool2d_kernel(const float *__restrict__ img, float *__restrict__ out, ConvP p,
-                                                     long long total, int is_max, int ref_compat) {
+                                                     long long total, int is_max, int ref_compat, PlaneOut forms) {
+    grid_dependency_sync();
+    constexpr int U = 9;
     const unsigned cn = (unsigned)(p.chan / VEC);
+    const int taps = p.w.ker_w * p.w.ker_h;
     for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < total;
          g += (long long)gridDim.x * blockDim.x) {
-        const long long pix = g / cn;
-        const int c = (int)(g - pix * cn) * VEC;
+        const I pix = (I)g / (I)cn;
+        const int c = (int)((I)g - pix * (I)cn) * VEC;
         const unsigned per_img = (unsigned)(p.col_h * p.col_w);
-        const long long n = pix / per_img;
-        const unsigned r = (unsigned)(pix - n * per_img);
+        const I n = pix / (I)per_img;
+        const unsigned r = (unsigned)(pix - n * (I)per_img);
         const int oy = (int)(r / (unsigned)p.col_w), ox = (int)(r % (unsigned)p.col_w);
+        const int y0 = oy * p.w.stride_h - p.w.pad_h, x0 = ox * p.w.stride_w - p.w.pad_w;
+        const float *src = img + (long long)n * p.img_h * p.img_w * p.chan + c;
+        const I img_w = (I)p.img_w, chan = (I)p.chan;
         const float init = is_max ? (ref_compat ? 0.f : -INFINITY) : 0.f;
         float acc[VEC];
 #pragma unroll
         for (int j = 0; j < VEC; ++j) acc[j] = init;
         // reduce over axes [3,4] = [KH,KW]: the first listed axis (KH) is the inner loop
-        for (int kx = 0; kx < p.w.ker_w; ++kx)
-            for (int ky = 0; ky < p.w.ker_h; ++ky) {
-                const int iy = oy * p.w.stride_h - p.w.pad_h + ky * p.w.dil_h;
-                const int ix = ox * p.w.stride_w - p.w.pad_w + kx * p.w.dil_w;
-                float v[VEC];
+        int kx = 0, ky = 0;
+        for (int t = 0; t < taps; t += U) {
+            float v[U][VEC];
 #pragma unroll
-                for (int j = 0; j < VEC; ++j) v[j] = 0.f;
-                if (ix >= 0 && ix < p.img_w && iy >= 0 && iy < p.img_h) {
-                    const float *src = img + ((n * p.img_h + iy) * p.img_w + ix) * p.chan + c;
+            for (int u = 0; u < U; ++u) {
+                const int iy = y0 + ky * p.w.dil_h, ix = x0 + kx * p.w.dil_w;
+#pragma unroll
+                for (int j = 0; j < VEC; ++j) v[u][j] = 0.f;
+                if (t + u < taps && ix >= 0 && ix < (int)p.img_w && iy >= 0 && iy < (int)p.img_h) {
+                    const float *at = src + ((I)iy * img_w + (I)ix) * chan;
                     if (VEC == 4) {
-                        const float4 t = __ldg(reinterpret_cast<const float4 *>(src));
-                        v[0] = t.x; v[1 % VEC] = t.y; v[2 % VEC] = t.z; v[3 % VEC] = t.w;
+                        const float4 q = __ldg(reinterpret_cast<const float4 *>(at));
+                        v[u][0] = q.x; v[u][1 % VEC] = q.y; v[u][2 % VEC] = q.z; v[u][3 % VEC] = q.w;
                     } else {
-                        v[0] = __ldg(src);
+                        v[u][0] = __ldg(at);
                     }
                 }
-#pragma unroll
-                for (int j = 0; j < VEC; ++j) acc[j] = is_max ? fmaxf(acc[j], v[j]) : acc[j] + v[j];
+                if (++ky == p.w.ker_h) {
+                    ky = 0;
+                    ++kx;
+                }
             }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (t + u < taps)
+#pragma unroll
+                    for (int j = 0; j < VEC; ++j) acc[j] = is_max ? fmaxf(acc[j], v[u][j]) : acc[j] + v[u][j];
+        }
         if (!is_max) {
 #pragma unroll
             for (int j = 0; j < VEC; ++j) acc[j] = acc[j] / (float)(p.w.ker_w * p.w.ker_h);
         }
-        float *dst = out + pix * p.chan + c;
-        if (VEC == 4) *reinterpret_cast<float4 *>(dst) = make_float4(acc[0], acc[1 % VEC], acc[2 % VEC], acc[3 % VEC]);
-        else dst[0] = acc[0];
+        const long long at = (long long)pix * p.chan + c;
+        if (VEC == 1) {
+            out[at] = acc[0];
+            continue;
+        }
+        const float4 o = make_float4(acc[0], acc[1 % VEC], acc[2 % VEC], acc[3 % VEC]);
+        if (out) *reinterpret_cast<float4 *>(out + at) = o;
+        if (forms.h2) {
+            using namespace sage_tc;
+            unsigned b = max(max(h2_finite_bits(o.x), h2_finite_bits(o.y)), max(h2_finite_bits(o.z), h2_finite_bits(o.w)));
+            const unsigned lanes = 0xffffu << (threadIdx.x & 16);
+#pragma unroll
+            for (int off = 8; off > 0; off >>= 1) b = max(b, __shfl_xor_sync(lanes, b, off));
+            float scale;
+            const float f = h2_factor(b, &scale);
+            uint2 h, l;
+            h2_split2(o.x, o.y, f, &h.x, &l.x);
+            h2_split2(o.z, o.w, f, &h.y, &l.y);
+            *reinterpret_cast<uint2 *>(forms.h2 + at) = h;
+            *reinterpret_cast<uint2 *>(forms.h2 + forms.h2_plane + at) = l;
+            if ((threadIdx.x & 15) == 0) forms.h2_scale[at >> 6] = scale;
+        }
     }
 }
 
@@ -489,16 +526,22 @@ sage_status col2im(Context &ctx, const float *col, float *img, long long n, long
     return ctx.check_cuda(cudaGetLastError(), "col2im launch");
 }
 
+bool pool2d_writes_pieces(long long chan) { return chan % 64 == 0; }
+
 sage_status pool2d(Context &ctx, bool is_max, const float *img, float *out, long long n, long long img_h,
-                   long long img_w, long long chan, long long out_h, long long out_w, const Window &w) {
+                   long long img_w, long long chan, long long out_h, long long out_w, const Window &w, const PlaneOut &forms) {
     ConvP p{n, img_h, img_w, chan, out_h, out_w, w};
     long long total = n * out_h * out_w * chan;
     ctx.note_launch(is_max ? "max_pool2d" : "avg_pool2d");
     if (ctx.dry() || total == 0) return SAGE_OK;
     const bool vec = chan % 4 == 0 && reinterpret_cast<uintptr_t>(img) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0 &&
                      out_h * out_w <= 0x7fffffffLL;
-    if (vec) pool2d_kernel<4><<<grid_for(ctx, total / 4), 256, 0, ctx.stream()>>>(img, out, p, total / 4, is_max ? 1 : 0, ctx.opts().ref_compat);
-    else pool2d_kernel<1><<<grid_for(ctx, total), 256, 0, ctx.stream()>>>(img, out, p, total, is_max ? 1 : 0, ctx.opts().ref_compat);
+    if (forms.h2 && !(vec && pool2d_writes_pieces(chan))) return ctx.fail(SAGE_ERR_INVALID, "pool2d: half-precision pieces need whole groups of channels");
+    // 32-bit indices where they reach: two 64-bit divisions were a third of a thread's instructions
+    const bool narrow = total < (1LL << 31) && img_h * img_w * chan < (1LL << 31);
+    auto kernel = narrow ? pool2d_kernel<4, unsigned> : pool2d_kernel<4, long long>;
+    if (vec) launch_dependent(ctx.pdl, ctx.stream(), kernel, dim3(grid_for(ctx, total / 4)), dim3(256), 0, img, out, p, total / 4, is_max ? 1 : 0, (int)ctx.opts().ref_compat, forms);
+    else launch_dependent(ctx.pdl, ctx.stream(), pool2d_kernel<1, long long>, dim3(grid_for(ctx, total)), dim3(256), 0, img, out, p, total, is_max ? 1 : 0, (int)ctx.opts().ref_compat, forms);
     return ctx.check_cuda(cudaGetLastError(), "pool2d launch");
 }
 

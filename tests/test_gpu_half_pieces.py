@@ -176,3 +176,28 @@ def test_attention_hands_pieces_to_the_next(ctx, n, length, heads, direct):
     want = ((p / p.sum(-1, keepdims=True)) @ v).transpose(0, 2, 1, 3).reshape(n, length, e) @ w[3].astype(np.float64)
     assert (np.abs(got - want) / np.maximum(np.abs(want), np.sqrt((want ** 2).mean()))).max() <= 1e-4
     assert ctx.status_word() == 0
+
+
+@pytest.mark.parametrize("shape,ker,stride,pad,is_max", [((3, 11, 13, 64), 3, 2, 1, True), ((2, 9, 9, 128), 2, 2, 0, False), ((2, 20, 20, 64), 5, 3, 2, True), ((5, 12, 12, 192), 3, 1, 1, False)])
+def test_pooling_hands_pieces_to_a_convolution(ctx, shape, ker, stride, pad, is_max):
+    """Windows of more and fewer taps than are fetched at a time, cut at the image's edge; the convolution behind reads the
+    pool's pieces.  Tolerance as for the other convolutions."""
+    rng = np.random.default_rng(sum(shape))
+    x = rng.uniform(-1, 1, shape).astype(np.float32)
+    f = rng.uniform(-1, 1, (3, 3, shape[3], 64)).astype(np.float32)
+    pool = S.max_pool_2d if is_max else S.avg_pool_2d
+    p = pool(ctx.var(x) * 1.0, ker, stride, pad, 1)
+    alone = p.eval(ctx)
+    ctx.clear()
+    got = S.conv_2d(p, ctx.var(f), 1, 1, 1).eval(ctx).astype(np.float64)
+
+    def windows(a, k, s, q):
+        a = np.pad(a.astype(np.float64), ((0, 0), (q, q), (q, q), (0, 0)))
+        oh, ow = (a.shape[1] - k) // s + 1, (a.shape[2] - k) // s + 1
+        return [[a[:, i:i + s * oh:s, j:j + s * ow:s][:, :oh, :ow] for j in range(k)] for i in range(k)]
+    taps = np.stack([t for r in windows(x, ker, stride, pad) for t in r])
+    want = np.maximum(taps.max(0), 0) if is_max else taps.mean(0)
+    assert np.abs(alone - want).max() <= 1e-6 * ker * ker
+    w = windows(alone, 3, 1, 1)
+    want = sum(w[i][j] @ f[i, j].astype(np.float64) for i in range(3) for j in range(3))
+    assert (np.abs(got - want) / np.maximum(np.abs(want), np.sqrt((want ** 2).mean()))).max() <= 1e-5
