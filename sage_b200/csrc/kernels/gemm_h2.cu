@@ -17,6 +17,8 @@
 #include "attn_tc_device.inc"  // AttnParams and the tile constants; the kernel itself is only compiled by NVRTC
 #include "gemm_tc_device_src.h"
 #include "gemm_h2_device_src.h"
+#include "attn_quads_device_src.h"
+#include "attn_rows_device_src.h"
 #include "attn_tc_device_src.h"
 #include "conv_first_device.inc"
 #include "conv_first_device_src.h"
@@ -886,11 +888,14 @@ sage_status attention_tc_run(Context &ctx, const TcAttn &a) {
     if (a.out.h2 && (!vec || a.d != 64 || a.ldo % 64 || a.so0 % 64 || a.so1 % 64 || !aligned16(a.out.h2) || a.out.h2_plane % 8))
         return ctx.fail(SAGE_ERR_INVALID, "attention_tc: a result in half-precision pieces needs whole groups of 64 columns");
     // Q, the K / V ring, 1 KiB per softmax warp for turning the output round, and the slack for 1024-byte alignment
-    const size_t smem = 2 * (size_t)kAttnQBytes + (size_t)kAttnStages * 4 * kAttnKVBytes + (size_t)kAttnSoftmaxWarps * 1024 + 1024;
-    const int grid = p.num_tiles < ctx.sm_count ? p.num_tiles : ctx.sm_count;
+    // A thread per row where throughput counts: two tiles and more for every SM, more than three blocks of keys each.  With fewer
+    // blocks the way through a single tile is what the next kernel waits for (32 x 128 in a BERT-base pass: 2809 us, 2845 with it).
+    const bool by_rows = p.num_tiles >= 2 * ctx.sm_count && a.lk > 3 * kAttnKeys;
+    const int threads = by_rows ? kRowThreads : kQuadThreads, slots = by_rows ? 2 * ctx.sm_count : ctx.sm_count, grid = p.num_tiles < slots ? p.num_tiles : slots;
+    const size_t smem = 2 * (size_t)kAttnQBytes + (size_t)(by_rows ? kRowStages : kQuadStages) * 4 * kAttnKVBytes + (size_t)(threads - 64) * 32 + 1024;
     const int out_mask = (a.o ? 1 : 0) | (a.out.hi ? 2 : 0) | (a.out.h2 ? 4 : 0);
     char num[64];
-    snprintf(num, sizeof num, "attention_tc %d %d %d\n", a.naux, rowinv_mask, out_mask);
+    snprintf(num, sizeof num, "attention_tc %d %d %d %d\n", by_rows ? 1 : 0, a.naux, rowinv_mask, out_mask);
     const std::string key = num + a.epilogue;  // the rest of the translation unit is fixed text
     Module *mod = ctx.module_find(key);
     if (!mod) {
@@ -901,10 +906,11 @@ sage_status attention_tc_run(Context &ctx, const TcAttn &a) {
         src += kGemmTcDeviceSrc;
         src += kGemmH2DeviceSrc;
         src += kAttnTcDeviceSrc;
-        src += "\nextern \"C\" __global__ void __launch_bounds__(sage_tc::kAttnThreads, 1)\n"
+        src += by_rows ? kAttnRowsDeviceSrc : kAttnQuadsDeviceSrc;
+        src += std::string("\nextern \"C\" __global__ void __launch_bounds__(") + (by_rows ? "sage_tc::kRowThreads, 2)\n" : "sage_tc::kQuadThreads, 1)\n") +
                "attention_tc_h2(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,\n"
                "                const __grid_constant__ CUtensorMap map_v, const __grid_constant__ sage_tc::AttnParams p) {\n"
-               "    sage_tc::attn_body(&map_q, &map_k, &map_v, p);\n}\n";
+               "    sage_tc::" + (by_rows ? "attn_rows_body" : "attn_body") + "(&map_q, &map_k, &map_v, p);\n}\n";
         sage_status st = ctx.module_get(src, &mod);
         if (st) return st;
         ctx.module_remember(key, mod);
@@ -929,7 +935,7 @@ sage_status attention_tc_run(Context &ctx, const TcAttn &a) {
     std::string label;
     if (ctx.verbose_names)
         label = "attention_tc_h2[" + std::to_string(a.lq) + "x" + std::to_string(a.lk) + "x" + std::to_string(a.d) + "x" + std::to_string(a.batch) + "]";
-    const uint32_t gr[3] = {(uint32_t)grid, 1, 1}, bl[3] = {(uint32_t)kAttnThreads, 1, 1};
+    const uint32_t gr[3] = {(uint32_t)grid, 1, 1}, bl[3] = {(uint32_t)threads, 1, 1};
     void *params[4] = {&map_q, &map_k, &map_v, &p};
     return ctx.launch(mod, "attention_tc_h2", gr, bl, (uint32_t)smem, params, ctx.verbose_names ? label.c_str() : "attention_tc_3xtf32", true, 1);
 }

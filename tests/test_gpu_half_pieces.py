@@ -201,3 +201,24 @@ def test_pooling_hands_pieces_to_a_convolution(ctx, shape, ker, stride, pad, is_
     w = windows(alone, 3, 1, 1)
     want = sum(w[i][j] @ f[i, j].astype(np.float64) for i in range(3) for j in range(3))
     assert (np.abs(got - want) / np.maximum(np.abs(want), np.sqrt((want ** 2).mean()))).max() <= 1e-5
+
+
+@pytest.mark.parametrize("n,length,heads,keyed", [(10, 257, 12, True), (75, 200, 2, False), (37, 512, 2, True)])
+def test_attention_with_a_thread_per_row(ctx, n, length, heads, keyed):
+    """Enough tiles of more than three key blocks for the form with a thread per query row: a last tile of one row, a last block
+    of eight keys, tiles that follow one another in a CTA; with and without an operand of the scores.  Tolerance 1e-4, as for the
+    other attention blocks."""
+    rng = np.random.default_rng(length + n)
+    q, k, v = [rng.uniform(-2, 2, (n, heads, length, 64)).astype(np.float32) for _ in range(3)]
+    bias = rng.uniform(-3, 3, (n, length)).astype(np.float32)
+    s = S.matmul_batched(ctx.var(q), S.transpose(ctx.var(k), -1, -2)) / 8.0
+    if keyed:
+        s = s + S.view(ctx.var(bias), [n, 1, 1, length])
+    got = S.matmul_batched(S.softmax(s, [3]), ctx.var(v)).eval(ctx)
+    assert "attention" in ctx.describe()
+    for i in range(0, n, max(n // 4, 1)):
+        s = q[i].astype(np.float64) @ k[i].astype(np.float64).transpose(0, 2, 1) / 8.0 + (bias[i] if keyed else 0.0)
+        p = np.exp(s - s.max(-1, keepdims=True))
+        want = (p / p.sum(-1, keepdims=True)) @ v[i].astype(np.float64)
+        assert (np.abs(got[i] - want) / np.maximum(np.abs(want), np.sqrt((want ** 2).mean()))).max() <= 1e-4
+    assert ctx.status_word() == 0
