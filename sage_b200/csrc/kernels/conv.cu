@@ -40,6 +40,7 @@ struct ColOut {
 __device__ __forceinline__ void split_pair(float x, float *hi, float *lo) { sage_tc::split_tf32_value(x, hi, lo); }
 
 __global__ void __launch_bounds__(256) im2col_kernel(const float *__restrict__ img, ColOut o, ConvP p, long long pixels) {
+    grid_dependency_sync();
     const int lane = threadIdx.x & 31;
     const long long pix = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (pix >= pixels) return;
@@ -98,6 +99,7 @@ __global__ void __launch_bounds__(256) im2col_kernel(const float *__restrict__ i
 // table in shared memory, built once per block, instead of being divided out per element.
 constexpr int kTapTable = 1024;
 __global__ void __launch_bounds__(256) im2col_quads_kernel(const float *__restrict__ img, ColOut o, ConvP p, long long quads) {
+    grid_dependency_sync();
     __shared__ int tab_off[kTapTable];   // element offset of entry kk from the pixel's first tap, -1 beyond K
     __shared__ int tab_yx[kTapTable];    // (ky * dil_h) << 16 | (kx * dil_w)
     const int C = (int)p.chan, K = p.w.ker_h * p.w.ker_w * C;
@@ -150,6 +152,7 @@ __global__ void __launch_bounds__(256) im2col_quads_kernel(const float *__restri
 // dilation_w to the y tap (conv.rs:462-464); identical whenever both dilations are equal.
 __global__ void __launch_bounds__(256) col2im_kernel(const float *__restrict__ col, float *__restrict__ img, ConvP p,
                                                      long long total) {
+    grid_dependency_sync();
     for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < total;
          g += (long long)gridDim.x * blockDim.x) {
         long long r = g;
@@ -181,6 +184,7 @@ __global__ void __launch_bounds__(256) col2im_kernel(const float *__restrict__ c
 // The same gather with 32-bit index arithmetic and four channels per thread (C % 4 == 0): one 64-bit division per
 // thread instead of a dozen per element, 16-byte loads and stores.  Same tap test, same order of accumulation.
 __global__ void __launch_bounds__(256) col2im_quads_kernel(const float *__restrict__ col, float *__restrict__ img, ConvP p, long long total) {
+    grid_dependency_sync();
     const int cn = (int)(p.chan >> 2), W = (int)p.img_w, H = (int)p.img_h, CW = (int)p.col_w, CH = (int)p.col_h;
     const int sw = p.w.stride_w, sh = p.w.stride_h, dw = p.w.dil_w, dh = p.w.dil_h, kw = p.w.ker_w, kh = p.w.ker_h;
     const int ker_ew = (kw - 1) * dw + 1, ker_eh = (kh - 1) * dh + 1;
@@ -321,10 +325,10 @@ sage_status im2col_planes(Context &ctx, const float *img, long long n, long long
     if (!vec && hi && pitch % 4 == 0 && pitch <= kTapTable && reinterpret_cast<uintptr_t>(hi) % 16 == 0 && plane % 4 == 0 &&
         img_w * (long long)w.ker_h * w.dil_h * chan < (1LL << 30) && w.ker_w * w.dil_w < 65536) {
         const long long quads = pixels * (pitch / 4);
-        im2col_quads_kernel<<<grid_for(ctx, quads), 256, 0, ctx.stream()>>>(img, o, p, quads);
+        launch_dependent(ctx.pdl, ctx.stream(), im2col_quads_kernel, dim3(grid_for(ctx, quads)), dim3(256), 0, img, o, p, quads);
         return ctx.check_cuda(cudaGetLastError(), "im2col launch");
     }
-    im2col_kernel<<<(unsigned)((pixels + 7) / 8), 256, 0, ctx.stream()>>>(img, o, p, pixels);
+    launch_dependent(ctx.pdl, ctx.stream(), im2col_kernel, dim3((unsigned)((pixels + 7) / 8)), dim3(256), 0, img, o, p, pixels);
     return ctx.check_cuda(cudaGetLastError(), "im2col launch");
 }
 
@@ -336,6 +340,7 @@ sage_status im2col_planes(Context &ctx, const float *img, long long n, long long
 // implicit-GEMM kernel then runs a (1 x KH) convolution over it; the column matrix is never written.
 __global__ void __launch_bounds__(256) pack_small_c_kernel(const float *__restrict__ img, float4 *__restrict__ hi, float4 *__restrict__ lo, long long n,
                                                            int h, int w, int c, int hp, int wp, int pad_h, int pad_w) {
+    grid_dependency_sync();
     const long long total = n * hp * (long long)wp;
     for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < total; g += (long long)gridDim.x * blockDim.x) {
         const int x = (int)(g % wp) - pad_w;
@@ -365,6 +370,7 @@ __global__ void __launch_bounds__(256) pack_small_c_kernel(const float *__restri
 // channels and of the window's unused tail are zero, so whatever the overlapping operand rows hold there is ignored.
 __global__ void __launch_bounds__(256) pack_small_c_filter_kernel(const float *__restrict__ f, float *__restrict__ hi, float *__restrict__ lo,
                                                                   int kh, int kw, int c, int oc) {
+    grid_dependency_sync();
     const long long total = (long long)kh * 32 * oc;
     for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < total; g += (long long)gridDim.x * blockDim.x) {
         const int o = (int)(g % oc), row = (int)(g / oc), ky = row / 32, r = row % 32, kx = r / 4, cc = r % 4;
@@ -380,7 +386,7 @@ sage_status pack_small_c_image(Context &ctx, const float *img, long long n, long
     if (c < 1 || c > 4 || plane % 4 || reinterpret_cast<uintptr_t>(hi) % 16 || h > 0x7fffffffLL || w > 0x7fffffffLL || hp > 0x7fffffffLL || wp > 0x7fffffffLL)
         return ctx.fail(SAGE_ERR_INVALID, "pack_small_c: bad arguments");
     const long long total = n * hp * wp;
-    pack_small_c_kernel<<<grid_for(ctx, total), 256, 0, ctx.stream()>>>(img, reinterpret_cast<float4 *>(hi), plane ? reinterpret_cast<float4 *>(hi + plane) : nullptr, n, (int)h, (int)w,
+    launch_dependent(ctx.pdl, ctx.stream(), pack_small_c_kernel, dim3(grid_for(ctx, total)), dim3(256), 0, img, reinterpret_cast<float4 *>(hi), plane ? reinterpret_cast<float4 *>(hi + plane) : nullptr, n, (int)h, (int)w,
                                                                         (int)c, (int)hp, (int)wp, pad_h, pad_w);
     return ctx.check_cuda(cudaGetLastError(), "pack_small_c launch");
 }
@@ -389,7 +395,7 @@ sage_status pack_small_c_filter(Context &ctx, const float *filt, int kh, int kw,
     ctx.note_launch("pack_small_c_filter");
     if (ctx.dry()) return SAGE_OK;
     if (kw * 4 > 32 || c > 4) return ctx.fail(SAGE_ERR_INVALID, "pack_small_c_filter: window too wide");
-    pack_small_c_filter_kernel<<<grid_for(ctx, (long long)kh * 32 * oc), 256, 0, ctx.stream()>>>(filt, hi, hi + plane, kh, kw, c, oc);
+    launch_dependent(ctx.pdl, ctx.stream(), pack_small_c_filter_kernel, dim3(grid_for(ctx, (long long)kh * 32 * oc)), dim3(256), 0, filt, hi, hi + plane, kh, kw, c, oc);
     return ctx.check_cuda(cudaGetLastError(), "pack_small_c_filter launch");
 }
 
@@ -519,10 +525,10 @@ sage_status col2im(Context &ctx, const float *col, float *img, long long n, long
     if (ctx.dry() || total == 0) return SAGE_OK;
     if (chan % 4 == 0 && reinterpret_cast<uintptr_t>(col) % 16 == 0 && reinterpret_cast<uintptr_t>(img) % 16 == 0 && img_h * img_w <= 0x7fffffffLL &&
         col_h * col_w <= 0x7fffffffLL && w.dil_w >= 1 && w.dil_h >= 1) {
-        col2im_quads_kernel<<<grid_for(ctx, total / 4), 256, 0, ctx.stream()>>>(col, img, p, total / 4);
+        launch_dependent(ctx.pdl, ctx.stream(), col2im_quads_kernel, dim3(grid_for(ctx, total / 4)), dim3(256), 0, col, img, p, total / 4);
         return ctx.check_cuda(cudaGetLastError(), "col2im launch");
     }
-    col2im_kernel<<<grid_for(ctx, total), 256, 0, ctx.stream()>>>(col, img, p, total);
+    launch_dependent(ctx.pdl, ctx.stream(), col2im_kernel, dim3(grid_for(ctx, total)), dim3(256), 0, col, img, p, total);
     return ctx.check_cuda(cudaGetLastError(), "col2im launch");
 }
 

@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include "kernels.h"
+#include "launch.h"
 
 namespace sage {
 namespace k {
@@ -30,6 +31,7 @@ struct GemmP {
 
 template <bool TA, bool TB>
 __global__ void __launch_bounds__(256) gemm_simt_kernel(GemmP p) {
+    grid_dependency_sync();
     __shared__ __align__(16) float As[BK][BM];
     __shared__ __align__(16) float Bs[BK][BN];
     const int t = threadIdx.x;
@@ -115,6 +117,7 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(GemmP p) {
 // Few outputs, long K (a classifier head: 32 x 2 outputs, K = 768): one warp per output element,
 // the lanes share K, so the tile kernel's single CTA walking K alone is avoided.
 __global__ void __launch_bounds__(256) gemm_skinny_kernel(GemmP p, long long sai, long long sak, long long sbk, long long sbj) {
+    grid_dependency_sync();
     const int lane = threadIdx.x & 31;
     const long long out = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const long long per_batch = p.m * p.n;
@@ -138,16 +141,16 @@ sage_status gemm_simt(Context &ctx, const GemmArgs &g) {
     const long long grid_limit = 0x7fffffffLL;
     if (g.m * g.n <= 8192 && g.k >= 128 && (g.m * g.n * g.batch + 7) / 8 <= grid_limit) {
         const dim3 grid((unsigned)((g.m * g.n * g.batch + 7) / 8));
-        gemm_skinny_kernel<<<grid, 256, 0, ctx.stream()>>>(p, g.ta ? 1 : g.lda, g.ta ? g.lda : 1, g.tb ? 1 : g.ldb, g.tb ? g.ldb : 1);
+        launch_dependent(ctx.pdl, ctx.stream(), gemm_skinny_kernel, dim3(grid), dim3(256), 0, p, g.ta ? 1 : g.lda, g.ta ? g.lda : 1, g.tb ? 1 : g.ldb, g.tb ? g.ldb : 1);
         return ctx.check_cuda(cudaGetLastError(), "gemm_skinny launch");
     }
     if (p.tiles_n * p.tiles_m > grid_limit / g.batch) return ctx.fail(SAGE_ERR_UNSUPPORTED, "gemm_simt: more than 2^31 tiles");
     const dim3 grid((unsigned)(p.tiles_n * p.tiles_m * g.batch));
     cudaStream_t s = ctx.stream();
-    if (!g.ta && !g.tb) gemm_simt_kernel<false, false><<<grid, 256, 0, s>>>(p);
-    else if (!g.ta && g.tb) gemm_simt_kernel<false, true><<<grid, 256, 0, s>>>(p);
-    else if (g.ta && !g.tb) gemm_simt_kernel<true, false><<<grid, 256, 0, s>>>(p);
-    else gemm_simt_kernel<true, true><<<grid, 256, 0, s>>>(p);
+    if (!g.ta && !g.tb) launch_dependent(ctx.pdl, ctx.stream(), gemm_simt_kernel<false, false>, dim3(grid), dim3(256), 0, p);
+    else if (!g.ta && g.tb) launch_dependent(ctx.pdl, ctx.stream(), gemm_simt_kernel<false, true>, dim3(grid), dim3(256), 0, p);
+    else if (g.ta && !g.tb) launch_dependent(ctx.pdl, ctx.stream(), gemm_simt_kernel<true, false>, dim3(grid), dim3(256), 0, p);
+    else launch_dependent(ctx.pdl, ctx.stream(), gemm_simt_kernel<true, true>, dim3(grid), dim3(256), 0, p);
     return ctx.check_cuda(cudaGetLastError(), "gemm_simt launch");
 }
 

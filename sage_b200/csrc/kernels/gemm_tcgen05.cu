@@ -59,6 +59,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 // rounded up to 4; plane 0 = hi, plane 1 = lo.  Pad columns are written as zeros.
 __global__ void __launch_bounds__(256) split_tf32_kernel(const float *__restrict__ src, SplitView v, float *__restrict__ dst, int pitch,
                                                          long long plane_stride) {
+    grid_dependency_sync();
     const int groups = pitch >> 2;
     const long long batches = v.nb1 * v.nb0;
     const long long total = batches * v.rows * groups;
@@ -90,6 +91,7 @@ __global__ void __launch_bounds__(256) split_tf32_kernel(const float *__restrict
 // n4 groups of 4 consecutive floats; planes laid out like the source.
 __global__ void __launch_bounds__(256) split_tf32_flat_kernel(const float4 *__restrict__ src, long long n4, float4 *__restrict__ hi_out,
                                                               float4 *__restrict__ lo_out) {
+    grid_dependency_sync();
     for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < n4; g += (long long)gridDim.x * blockDim.x) {
         const float4 x = src[g];
         float4 hi, lo;
@@ -390,7 +392,7 @@ sage_status split_tf32_flat(Context &ctx, const float *src, long long n, float *
     if (ctx.dry()) return SAGE_OK;
     if (!aligned16(src) || !aligned16(dst_hi) || plane % 4) return ctx.fail(SAGE_ERR_INVALID, "split_tf32_flat: unaligned");
     const long long n4 = (n + 3) / 4;  // allocations are multiples of 512 bytes, so the last group is readable
-    split_tf32_flat_kernel<<<split_grid(ctx, n4), 256, 0, ctx.stream()>>>(reinterpret_cast<const float4 *>(src), n4,
+    launch_dependent(ctx.pdl, ctx.stream(), split_tf32_flat_kernel, dim3(split_grid(ctx, n4)), dim3(256), 0, reinterpret_cast<const float4 *>(src), n4,
                                                                           reinterpret_cast<float4 *>(dst_hi),
                                                                           reinterpret_cast<float4 *>(dst_hi + plane));
     return ctx.check_cuda(cudaGetLastError(), "split_tf32_flat launch");
@@ -409,7 +411,7 @@ sage_status split_tf32_view(Context &ctx, const float *src, const SplitView &v, 
     out->planes = reinterpret_cast<float *>(out->block->ptr);
     ctx.note_launch("split_tf32");
     if (ctx.dry()) return SAGE_OK;
-    split_tf32_kernel<<<split_grid(ctx, plane / 4), 256, 0, ctx.stream()>>>(src, v, out->planes, out->pitch, plane);
+    launch_dependent(ctx.pdl, ctx.stream(), split_tf32_kernel, dim3(split_grid(ctx, plane / 4)), dim3(256), 0, src, v, out->planes, out->pitch, plane);
     return ctx.check_cuda(cudaGetLastError(), "split_tf32 launch");
 }
 
