@@ -107,7 +107,6 @@ SG void sg_h2_store(float4 r, unsigned long long g, unsigned short *h2, long lon
 )";
 
 const char *map_prelude_text() { return kPrelude; }
-const char *map_prelude_h2_text() { return kPreludeH2; }
 
 static const char *ctype(int dt) { return dt == SAGE_F32 ? "float" : dt == SAGE_I32 ? "int" : "uint"; }
 static const char *vtype(int dt) { return dt == SAGE_F32 ? "float4" : dt == SAGE_I32 ? "int4" : "uint4"; }

@@ -169,7 +169,6 @@ struct Storage {
     std::shared_ptr<SplitCache> split;       // whole-storage planes
     std::shared_ptr<SplitCache> split_view;  // last compact split of a view
     std::shared_ptr<H2Cache> h2, h2_view, h2_rows;  // whole storage; last compact operand A; last compact operand B
-    std::shared_ptr<H2Cache> h2_blocks;             // a matrix as it lies, with a scale per 64 x 64 block
     uint64_t version = 0;                    // bumped whenever the contents are rewritten
     bool planes_only = false;                // the fp32 buffer was never written: only `split` / `h2` hold the value
     void drop_splits() {
@@ -178,7 +177,6 @@ struct Storage {
         h2.reset();
         h2_view.reset();
         h2_rows.reset();
-        h2_blocks.reset();
         ++version;
     }
     Context *ctx = nullptr;  // identity only; never dereferenced by the destructor

@@ -261,45 +261,6 @@ static sage_status make_h2_operand(Context &ctx, const Tensor &t, bool trans, bo
     return SAGE_OK;
 }
 
-// Operand B of a training step: a weight in natural order ([rows][cols], cols contiguous) with a scale per 64 x 64 block, one copy
-// for the product with the weight and for the one with its transpose.  `mode` as H2Gemm::b_blocks.
-static sage_status make_block_operand(Context &ctx, const Tensor &t, bool tb, int mode, k::H2Gemm *g, std::shared_ptr<H2Cache> *hold) {
-    const Shape &sh = t.desc.shape;
-    const int r = sh.rank(), ka = tb ? r - 1 : r - 2, na = tb ? r - 2 : r - 1, row_axis = mode == 2 ? ka : na, col_axis = mode == 2 ? na : ka;
-    const long long rows = sh.extents[row_axis], cols = sh.extents[col_axis], ld = rows > 1 ? sh.strides[row_axis] : cols;
-    if (sh.strides[col_axis] != 1 || cols % 64 || ld < cols) return ctx.fail(SAGE_ERR_INVALID, "internal: a weight with block scales arrived in another layout");
-    Storage &st = *t.data;
-    Shape view(Array{rows, cols});
-    view.strides[0] = ld;
-    view.offset = sh.offset;
-    if (!(st.h2_blocks && st.h2_blocks->view == view)) {
-        auto c = std::make_shared<H2Cache>();
-        c->alloc = ctx.allocator_ptr();
-        c->view = view;
-        c->pieces.pitch = cols;
-        c->pieces.plane = rows * cols;
-        const size_t planes = ((size_t)(rows * cols) * 4 + 255) / 256 * 256;
-        c->pieces.block = ctx.allocator().alloc(planes + (size_t)((rows + 63) / 64 * (cols / 64)) * 4);
-        if (!c->pieces.block) return ctx.fail(SAGE_ERR_OOM, "out of memory for half-precision pieces");
-        c->pieces.hi = reinterpret_cast<unsigned short *>(c->pieces.block->ptr);
-        c->pieces.scale = reinterpret_cast<float *>(c->pieces.block->ptr + planes);
-        sage_status s = k::split_h2_blocks(ctx, (const float *)t.ptr(), rows, cols, ld, c->pieces.hi, c->pieces.plane, c->pieces.scale);
-        if (s) return s;
-        st.h2_blocks = c;
-    }
-    *hold = st.h2_blocks;
-    const k::H2Split &p = st.h2_blocks->pieces;
-    g->b.hi = p.hi;
-    g->b.plane = p.plane;
-    g->b.scale = p.scale;
-    g->b.rows = rows;
-    g->b.ld = cols;
-    g->b_blocks = mode;
-    g->bs_n = mode == 2 ? 1 : cols / 64;
-    g->bs_k = mode == 2 ? cols / 64 : 1;
-    return SAGE_OK;
-}
-
 // Where a result's operand forms go, as its readers asked: attaches them to `y` and says whether the fp32 store may be left out.
 static sage_status attach_forms(Context &ctx, Tensor *y, bool emit, bool emit_h2, k::PlaneOut *o) {
     if (emit) {
@@ -343,7 +304,6 @@ struct GemmOp : Operator {
     k::Window win{};
     long long img[6] = {0, 0, 0, 0, 0, 0};  // N, H, W, C, OH, OW
     bool h2 = false;                // runs on half-precision pieces (gemm_h2); decided for a whole program (assign_h2)
-    int h2_blocks = 0;              // ... and operand B is a weight with block scales (H2Gemm::b_blocks): training steps
     bool row_softmax = false;       // the stored value is softmax over the last axis of the (epilogue of the) product
     bool folded = false;            // result stored through (ldc, sc0, sc1, nbc0) instead of row-major [batch, M, N]
     long long ldc = 0, sc0 = 0, sc1 = 0, nbc0 = 1;
@@ -732,7 +692,7 @@ struct GemmOp : Operator {
             if (st) return st;
             if (g.a.nb0 * g.a.nb1 != batch) return ctx.fail(SAGE_ERR_INVALID, "gemm: operand batch extents differ from the operator's");
         }
-        st = h2_blocks ? make_block_operand(ctx, x[1], tb, h2_blocks, &g, &hold_b) : make_h2_operand(ctx, x[1], !tb, true, &g.b, &hold_b);
+        st = make_h2_operand(ctx, x[1], !tb, true, &g.b, &hold_b);
         if (st) return st;
         if (g.b.nb0 * g.b.nb1 != batch) return ctx.fail(SAGE_ERR_INVALID, "gemm: operand batch extents differ from the operator's");
         g.c = (float *)y->ptr();
@@ -1204,24 +1164,6 @@ std::shared_ptr<Operator> gemm_on_h2(const Operator &op, bool a_given, bool tc_e
     } else if (!h2_view_ok(c->in[0].shape, c->ta) && !a_given) {
         return nullptr;
     }
-    c->h2 = true;
-    return c;
-}
-// The same in a program that also multiplies by the transposes of its activations: B (a weight, an input of the program) with
-// block scales.  Its optimizer rewrites those pieces with the weight.
-std::shared_ptr<Operator> gemm_on_h2_blocks(const Operator &op, bool tc_enabled) {
-    const GemmOp *g = as_gemm(op);
-    if (!g || g->attn || g->row_softmax || g->h2 || g->conv || !gemm_runs_on_tc(op, tc_enabled)) return nullptr;
-    auto c = lowered_clone(*g);
-    if (c->batch != 1 || !h2_view_ok(c->in[0].shape, c->ta)) return nullptr;
-    // below ~10 us of tensor time a product is launch and latency, and its operands' second form costs more than it gains
-    // (ResNet-18 on 28 x 28, batch 128, products of 0.5 GFLOP: 1500 -> 1530 us a step)
-    if ((double)c->m * (double)c->n * (double)c->k < 2e9) return nullptr;
-    const Shape &b = c->in[1].shape;
-    const int r = b.rank(), ka = c->tb ? r - 1 : r - 2, na = c->tb ? r - 2 : r - 1;
-    if (b.strides[na] == 1 && b.extents[na] % 64 == 0 && b.strides[ka] == b.extents[na]) c->h2_blocks = 2;
-    else if (b.strides[ka] == 1 && b.extents[ka] % 64 == 0 && b.strides[na] == b.extents[ka]) c->h2_blocks = 1;
-    else return nullptr;
     c->h2 = true;
     return c;
 }

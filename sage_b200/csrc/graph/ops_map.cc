@@ -99,14 +99,7 @@ bool map_op_emits_planes(const Operator &op) {
     return m && m->out.dtype == SAGE_F32 && !m->in.empty();
 }
 
-bool map_op_emits_h2(const Operator &op) {  // four neighbours at a time: operands read along their last axis
-    if (!map_op_emits_planes(op) || op.out.shape.size() % 64) return false;
-    for (const TensorDesc &d : op.in) {
-        const int r = d.shape.rank();
-        if (r > 0 && d.shape.extents[r - 1] > 1 && d.shape.strides[r - 1] > 1) return false;
-    }
-    return true;
-}
+bool map_op_emits_h2(const Operator &op) { return map_op_emits_planes(op) && op.out.shape.size() % 64 == 0; }
 
 const MapExpr *map_expr_of(const Operator &op) {
     const MapOp *m = dynamic_cast<const MapOp *>(&op);

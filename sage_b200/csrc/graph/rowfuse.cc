@@ -19,7 +19,6 @@
 namespace sage {
 
 const char *map_prelude_text();
-const char *map_prelude_h2_text();
 int view_op_kind(const Operator &op);
 int index_op_axis(const Operator &op, bool scatter);
 bool reduce_op_info(const Operator &op, int *kind, std::vector<int> *axes);
@@ -212,7 +211,7 @@ bool screen(const std::vector<Var> &targets, const std::unordered_set<Origin *> 
 void emit(RowProgram &p) {
     std::ostringstream s;
     const int E = p.nv * p.vec;
-    s << map_prelude_text() << map_prelude_h2_text();
+    s << map_prelude_text();
     s << "#define RP_C " << p.cols << "\n#define RP_T " << p.threads << "\n#define RP_NV " << p.nv << "\n#define RP_VEC " << p.vec << "\n";
     s << "#define RP_E " << E << "\n";
     int wp2 = 1;
@@ -223,8 +222,7 @@ void emit(RowProgram &p) {
     s << "#define RP_OK(e) (RP_WHOLE || RP_COL(e) < RP_C)\n";
     s << "struct RowP { long long rows; int compat; int pad; const void *in[" << std::max<size_t>(1, p.in_val.size()) << "]; void *out["
       << std::max<size_t>(1, p.out_val.size()) << "]; float *out_hi[" << std::max<size_t>(1, p.out_val.size()) << "]; long long out_plane["
-      << std::max<size_t>(1, p.out_val.size()) << "]; unsigned short *out_h2[" << std::max<size_t>(1, p.out_val.size()) << "]; long long out_h2_plane["
-      << std::max<size_t>(1, p.out_val.size()) << "]; float *out_h2_scale[" << std::max<size_t>(1, p.out_val.size()) << "]; };\n";
+      << std::max<size_t>(1, p.out_val.size()) << "]; };\n";
     s << R"(template <int K> SG float rp_apply(float a, float b) { return K == 0 ? a + b : K == 1 ? a * b : K == 2 ? fmaxf(a, b) : fminf(a, b); }
 template <int K> SG float rp_identity() { return K == 0 ? 0.f : K == 1 ? 1.f : K == 2 ? __int_as_float(0xff800000) : __int_as_float(0x7f800000); }
 // Every thread returns the same value: a butterfly combines the same pairs in every lane, and every
@@ -386,12 +384,6 @@ SG void rp_prefetch(const RowP &p, long long row, uint4 *stage);
                         s << "          float h, l;\n          sg_split_tf32(" << name << "[j], &h, &l);\n          hi[c0] = h;\n          lo[c0] = l;\n";
                     }
                     s << "        }\n      }\n    }\n";
-                    if (p.vec == 4 && p.cols % 64 == 0) {  // ... and its half-precision pieces: 16 lanes hold a group
-                        s << "    if (p.out_h2[" << v.output << "]) {\n#pragma unroll\n      for (int j = 0; j < RP_NV; ++j) {\n"
-                          << "        const int c0 = (j * RP_T + (int)threadIdx.x) * 4;\n        if (RP_WHOLE || c0 < RP_C)\n          sg_h2_store(make_float4("
-                          << name << "[4 * j], " << name << "[4 * j + 1], " << name << "[4 * j + 2], " << name << "[4 * j + 3]), (unsigned long long)(row * RP_C + c0), p.out_h2["
-                          << v.output << "], p.out_h2_plane[" << v.output << "], p.out_h2_scale[" << v.output << "]);\n      }\n    }\n";
-                    }
                 }
             } else {
                 s << "    if (threadIdx.x == 0) ((" << T << " *)p.out[" << v.output << "])[row] = " << name << ";\n";
@@ -499,15 +491,6 @@ sage_status row_program_exec(RowProgram &p, Context &ctx, Session &s) {
 }
 
 sage_status storage_planes_attach(Context &ctx, Storage &st);  // ops_gemm.cc
-sage_status storage_h2_attach(Context &ctx, Storage &st);
-
-bool row_program_emits_h2(const RowProgram &p, const Origin *target) {
-    for (int id : p.out_val) {
-        const Val &v = p.vals[id];
-        if (v.var.key() == target) return p.vec == 4 && p.cols % 64 == 0 && v.cls == Full && v.dtype == SAGE_F32;
-    }
-    return false;
-}
 
 sage_status row_program_run(RowProgram &p, Context &ctx, const std::function<bool(const Var &, Tensor *)> &fetch, std::vector<Tensor> *outs_,
                             const std::vector<char> *planes) {
@@ -520,7 +503,7 @@ sage_status row_program_run(RowProgram &p, Context &ctx, const std::function<boo
     }
     std::vector<Tensor> keep;
     const size_t nin = std::max<size_t>(1, p.in_val.size()), nout = std::max<size_t>(1, p.out_val.size());
-    std::vector<uint64_t> pb(2 + nin + 6 * nout, 0);  // rows, compat, in[], out[], out_hi[], out_plane[], out_h2[], out_h2_plane[], out_h2_scale[]
+    std::vector<uint64_t> pb(2 + nin + 3 * nout, 0);  // rows, compat, in[], out[], out_hi[], out_plane[]
     pb[0] = (uint64_t)p.rows;
     pb[1] = (uint64_t)(ctx.opts().ref_compat ? 1 : 0);
     for (size_t i = 0; i < p.in_val.size(); ++i) {
@@ -556,15 +539,7 @@ sage_status row_program_run(RowProgram &p, Context &ctx, const std::function<boo
         if (st) return st;
         pb[2 + nin + i] = (uint64_t)reinterpret_cast<uintptr_t>(outs[i].ptr());
         const Val &ov = p.vals[p.out_val[i]];
-        if (planes && i < planes->size() && ((*planes)[i] & 2) && ov.cls == Full && ov.dtype == SAGE_F32 && p.vec == 4 && p.cols % 64 == 0) {
-            st = storage_h2_attach(ctx, *outs[i].data);
-            if (st) return st;
-            const k::H2Split &h = outs[i].data->h2->pieces;
-            pb[2 + nin + 3 * nout + i] = (uint64_t)reinterpret_cast<uintptr_t>(h.hi);
-            pb[2 + nin + 4 * nout + i] = (uint64_t)h.plane;
-            pb[2 + nin + 5 * nout + i] = (uint64_t)reinterpret_cast<uintptr_t>(h.scale);
-        }
-        if (planes && i < planes->size() && ((*planes)[i] & 1) && ov.cls == Full && ov.dtype == SAGE_F32) {
+        if (planes && i < planes->size() && (*planes)[i] && ov.cls == Full && ov.dtype == SAGE_F32) {
             st = storage_planes_attach(ctx, *outs[i].data);
             if (st) return st;
             pb[2 + nin + nout + i] = (uint64_t)reinterpret_cast<uintptr_t>(outs[i].data->split->planes.planes + outs[i].desc.shape.offset);

@@ -29,11 +29,9 @@ std::shared_ptr<RowProgram> row_program_build(const std::vector<Var> &evaluated,
 // Allocates the targets, launches the kernel, stores the results in `s.data`.
 sage_status row_program_exec(RowProgram &p, Context &ctx, Session &s);
 // The same with the caller's own lookup of the (non-data) inputs; `outs` are the targets in order.
-// `planes` (optional, per target): also write operand forms of that (f32, full-size) target: 1 = tf32 hi / lo planes, 2 =
-// half-precision pieces (where row_program_emits_h2 says so).
+// `planes` (optional, one flag per target): also write the tf32 hi / lo planes of that (f32, full-size) target.
 sage_status row_program_run(RowProgram &p, Context &ctx, const std::function<bool(const Var &, Tensor *)> &fetch, std::vector<Tensor> *outs,
                             const std::vector<char> *planes = nullptr);
-bool row_program_emits_h2(const RowProgram &p, const Origin *target);
 void row_program_space(const RowProgram &p, long long *rows, long long *cols);
 std::vector<Var> row_program_inputs(const RowProgram &p);
 int row_program_exchanges(const RowProgram &p);  // reductions + gathers + scatters in the program

@@ -64,7 +64,6 @@ bool gemm_group_key(const Operator &op, std::string *key);
 std::shared_ptr<Operator> make_grouped_gemm(const std::vector<const Operator *> &members);
 std::shared_ptr<Operator> make_slab(const Operator &grouped, int index, const TensorDesc &member_out);
 bool gemm_needs_tf32(const Operator &op, bool tc_enabled);
-std::shared_ptr<Operator> gemm_on_h2_blocks(const Operator &op, bool tc_enabled);
 std::shared_ptr<Operator> gemm_on_h2(const Operator &op, bool a_given, bool tc_enabled);
 bool gemm_is_h2(const Operator &op);
 bool gemm_emits_h2(const Operator &op);
@@ -482,9 +481,8 @@ static bool can_emit_planes(const Operator &op, bool tc) {
 }
 static bool can_emit_h2(const Operator &op) { return gemm_emits_h2(op) || row_op_emits_h2(op) || map_op_emits_h2(op) || pool_op_emits_h2(op); }
 
-// Products with weights run on half-precision pieces.  A program that also multiplies by the transposes of its activations
-// (training) keeps tf32 planes for those, and its weights as pieces with block scales (`blocks` below), which its optimizer
-// refreshes: an activation is then written in both forms.
+// Products with weights run on half-precision pieces, unless the program also multiplies by the transposes of its activations (training):
+// then everything keeps to tf32 planes.
 static bool any_needs_tf32(const Node &n, bool tc) {
     if (n.is_data) return false;
     if (gemm_needs_tf32(*n.op, tc) || (n.shared && any_needs_tf32(*n.shared, tc))) return true;
@@ -494,62 +492,28 @@ static bool any_needs_tf32(const Node &n, bool tc) {
 }
 // The same choice whether operand A comes from the product's own routine or from another one: which values are kept must not
 // change what is computed.
-struct H2Choice {
-    bool tc = false, blocks = false;
-    std::unordered_set<Origin *> done, keep_tf32;  // routines gone through; weights that stay as planes
-    std::vector<std::pair<Node *, std::shared_ptr<Operator>>> changed;
-};
-// The input of the program that this operand is (a view of), through states that are only views; or null.
-static Origin *given_leaf(Node *n, Program &p) {
-    n = skip_views(n);
-    for (int hops = 0; n->is_data && n->var.is_op() && hops < 8; ++hops) {
-        auto it = p.routines.find(n->var.key());
-        if (it == p.routines.end() || it->second.row) return nullptr;
-        n = skip_views(&it->second.root);
-    }
-    return n->is_data && !n->var.is_op() ? n->var.key() : nullptr;
+static void assign_h2(Node &n, bool tc, Program &p, std::unordered_set<Origin *> *done);
+static void assign_h2(Routine &r, bool tc, Program &p, std::unordered_set<Origin *> *done) {
+    if (!r.row && done->insert(r.output.key()).second) assign_h2(r.root, tc, p, done);
 }
-static void assign_h2(Node &n, Program &p, H2Choice *c);
-static void assign_h2(Routine &r, Program &p, H2Choice *c) {
-    if (!r.row && c->done.insert(r.output.key()).second) assign_h2(r.root, p, c);
-}
-static void assign_h2(Node &n, Program &p, H2Choice *c) {
-    const bool tc = c->tc, blocks = c->blocks;
+static void assign_h2(Node &n, bool tc, Program &p, std::unordered_set<Origin *> *done) {
     if (n.is_data) return;
-    if (n.shared) assign_h2(*n.shared, p, c);
-    for (Node &a : n.args) assign_h2(a, p, c);
+    if (n.shared) assign_h2(*n.shared, tc, p, done);
+    for (Node &a : n.args) assign_h2(a, tc, p, done);
     if (n.args.size() < 2 || !(is_gemm_op(*n.op) || is_grouped_gemm_op(*n.op))) return;
-    Origin *w = given_leaf(&n.args[1], p);
-    if (!w || c->keep_tf32.count(w)) return;
+    const Node *w = skip_views(&n.args[1]);
+    if (!w->is_data || w->var.is_op()) return;
     const Node *a = skip_views(&n.args[0]);
     const bool given = a->is_data && !a->var.is_op();
     for (int hops = 0; a->is_data && a->var.is_op() && hops < 8; ++hops) {
         auto it = p.routines.find(a->var.key());
-        if (it == p.routines.end()) break;
-        if (it->second.row) {
-                    if (blocks && !row_program_emits_h2(*it->second.row, it->first)) return;
-            break;
-        }
-        assign_h2(it->second, p, c);
+        if (it == p.routines.end() || it->second.row) break;
+        assign_h2(it->second, tc, p, done);
         a = skip_views(&it->second.root);
     }
     // a producer that can only write tf32 planes (a product of two results) keeps its reader on them
     if (!a->is_data && !can_emit_h2(*a->op) && can_emit_planes(*a->op, tc)) return;
-    if (blocks && given) return;  // read as planes by the weight's gradient: a split pass for one form is enough
-    if (std::shared_ptr<Operator> op = blocks ? gemm_on_h2_blocks(*n.op, tc) : gemm_on_h2(*n.op, given, tc)) {
-        c->changed.emplace_back(&n, n.op);
-        n.op = op;
-    }
-}
-// Weights that some product still reads as planes
-static void weights_as_planes(Node &n, Program &p, const H2Choice &c, std::unordered_set<Origin *> *out) {
-    if (n.is_data) return;
-    if (n.shared) weights_as_planes(*n.shared, p, c, out);
-    for (Node &a : n.args) weights_as_planes(a, p, c, out);
-    if (n.args.size() < 2 || !is_gemm_op(*n.op) || gemm_is_h2(*n.op) || !gemm_runs_on_tc(*n.op, c.tc)) return;
-    for (int i = 0; i < 2; ++i) {
-        if (Origin *w = given_leaf(&n.args[i], p)) out->insert(w);
-    }
+    if (std::shared_ptr<Operator> op = gemm_on_h2(*n.op, given, tc)) n.op = op;
 }
 
 // GEMMs of one routine that multiply the same A (same leaf, same view) by different weights, with
@@ -869,25 +833,9 @@ static std::unique_ptr<Program> compile(const std::vector<Var> &x, std::vector<V
         if (tc) {
             bool tf32 = false;
             for (auto &kv : p->routines) tf32 = tf32 || (!kv.second.row && any_needs_tf32(kv.second.root, tc));
-            H2Choice c;
-            c.tc = tc;
-            c.blocks = tf32;
-            for (;;) {  // a weight takes one form for all its products: one split, one copy to refresh
-                for (auto &kv : p->routines) assign_h2(kv.second, *p, &c);
-                std::unordered_set<Origin *> planes;
-                if (c.blocks)
-                    for (auto &kv : p->routines)
-                        if (!kv.second.row) weights_as_planes(kv.second.root, *p, c, &planes);
-                bool clash = false;
-                for (auto &ch : c.changed) {
-                    Origin *w = given_leaf(&ch.first->args[1], *p);
-                    if (planes.count(w)) clash |= c.keep_tf32.insert(w).second;
-                }
-                            if (!clash) break;
-                for (auto it = c.changed.rbegin(); it != c.changed.rend(); ++it) it->first->op = it->second;
-                c.changed.clear();
-                c.done.clear();
-            }
+            std::unordered_set<Origin *> done;
+            if (!tf32)
+                for (auto &kv : p->routines) assign_h2(kv.second, tc, *p, &done);
         }
         for (auto &kv : p->routines)
             if (!kv.second.row) mark_plane_readers(kv.second.root, tc, &plane_states, &h2_states);
@@ -904,7 +852,7 @@ static std::unique_ptr<Program> compile(const std::vector<Var> &x, std::vector<V
                 if (it == p->routines.end()) continue;  // an input of the program: split on first use
                 if (it->second.row) {                   // a row group: the generated kernel writes the planes of that output
                     for (size_t i = 0; i < it->second.row_outputs.size(); ++i)
-                        if (it->second.row_outputs[i].key() == it->first) (*it->second.row_emit_shared)[i] |= form ? 2 : 1;
+                        if (!form && it->second.row_outputs[i].key() == it->first) (*it->second.row_emit_shared)[i] = 1;
                     continue;
                 }
                 Node *root = skip_views(&it->second.root);

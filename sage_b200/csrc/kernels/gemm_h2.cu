@@ -203,35 +203,7 @@ __global__ void __launch_bounds__(256) split_h2_rows_kernel(ViewP v, unsigned sh
     }
 }
 
-// A scale per 64 x 64 block: a weight that is read along its rows and along its columns.  One block per tile.
-__global__ void __launch_bounds__(256) split_h2_blocks_kernel(ViewP v, unsigned short *__restrict__ hi, float *__restrict__ scale) {
-    __shared__ float tile[64][65];
-    __shared__ unsigned amax[8];
-    grid_dependency_sync();
-    const long long r0 = (long long)(blockIdx.x / v.col_tiles) * 64, c0 = (long long)(blockIdx.x % v.col_tiles) * 64;
-    float y[16], s;
-    fetch_row(v, v.src, r0, c0, tile, y);
-    unsigned m = __reduce_max_sync(0xffffffffu, row_amax(y));
-    if ((threadIdx.x & 31) == 0) amax[threadIdx.x >> 5] = m;
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 8; ++i) m = max(m, amax[i]);
-    const float f = h2_factor(m, &s);
-    if (threadIdx.x == 0) scale[blockIdx.x] = s;
-    store_row(v, 0, r0, c0, y, f, hi);
-}
-
 }  // namespace
-
-sage_status split_h2_blocks(Context &ctx, const float *src, long long rows, long long cols, long long ld, unsigned short *hi, long long plane, float *scale) {
-    ctx.note_launch("split_tf32");  // launch lists have one name for an operand's split
-    if (ctx.dry()) return SAGE_OK;
-    ViewP p{src, 1, 0, 0, ld, 1, rows, cols, cols, plane, (int)((rows + 63) / 64), (int)(cols / 64), 0};
-    p.vec = aligned16(src) && ld % 4 == 0;
-    const long long blocks = (long long)p.row_tiles * p.col_tiles;
-    if (cols % 64 || !aligned16(hi) || plane % 8 || blocks > 0x7fffffffLL) return ctx.fail(SAGE_ERR_INVALID, "split_h2_blocks: unaligned");
-    return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), split_h2_blocks_kernel, dim3((unsigned)blocks), dim3(256), 0, p, hi, scale), "split_h2_blocks launch");
-}
 
 sage_status split_h2_flat(Context &ctx, const float *src, long long n, unsigned short *hi, long long plane, float *scale) {
     ctx.note_launch("split_tf32");  // launch lists have one name for an operand's split
@@ -314,15 +286,6 @@ static bool encode_operand(PFN_encodeTiled encode, const H2Operand &op, long lon
     const cuuint64_t dims[5] = {(cuuint64_t)k, (cuuint64_t)op.rows, (cuuint64_t)op.nb0, (cuuint64_t)op.nb1, 2};
     const cuuint64_t strides[4] = {row_b, op.nb0 > 1 ? (cuuint64_t)op.sb0 * 2 : row_b, op.nb1 > 1 ? (cuuint64_t)op.sb1 * 2 : row_b, (cuuint64_t)op.plane * 2};
     const cuuint32_t box[5] = {(cuuint32_t)HK, box_rows, 1, 1, 1}, estr[5] = {1, 1, 1, 1, 1};
-    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, const_cast<unsigned short *>(op.hi), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// ... and B as it lies with n contiguous: dims {n, k, batch low, batch high, piece}, box {64, 64, 1, 1, 1}
-static bool encode_operand_mn(PFN_encodeTiled encode, const H2Operand &op, long long n, CUtensorMap *map) {
-    const cuuint64_t row_b = (cuuint64_t)op.ld * 2;
-    const cuuint64_t dims[5] = {(cuuint64_t)n, (cuuint64_t)op.rows, 1, 1, 2}, strides[4] = {row_b, row_b, row_b, (cuuint64_t)op.plane * 2};
-    const cuuint32_t box[5] = {64, (cuuint32_t)HK, 1, 1, 1}, estr[5] = {1, 1, 1, 1, 1};
     return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, const_cast<unsigned short *>(op.hi), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -575,9 +538,7 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
     ColumnPlan cols = sliced ? ColumnPlan{cut.bn, 0, 0} : plan_columns(ctx, g.m, g.n, g.batch, ctas);
     if (halo) cols = ColumnPlan{g.n <= 64 ? 64 : 128, 0, 0};  // all output channels in one tile: the window is loaded once
     const int bn = cols.bn;
-    if (g.b_blocks && (g.conv || g.batch != 1)) return ctx.fail(SAGE_ERR_INVALID, "gemm_h2: a weight with block scales has no batch");
-    const int b_alloc = g.b_blocks == 2 ? (bn / ctas + 63) / 64 * 64 : bn / ctas;
-    const int stage_bytes = halo ? 2 * (bn / ctas) * HK * 2 : 2 * BM * HK * 2 + 2 * b_alloc * HK * 2;
+    const int stage_bytes = halo ? 2 * (bn / ctas) * HK * 2 : 2 * BM * HK * 2 + 2 * (bn / ctas) * HK * 2;
     const int staging = kEpiWarps * kStageBytesPerWarp, fixed = halo ? kHaloStages * kHaloStageBytes : 0;
     int stages = (227 * 1024 - 2048 - staging - fixed) / stage_bytes;
     if (stages > 8) stages = 8;
@@ -618,8 +579,6 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
     p.sa_b1 = g.a.s_b1;
     p.sb = g.b.scale;
     p.sb_batch = p.b_bcast ? 0 : g.b.s_b0;
-    p.sb_n = g.bs_n;
-    p.sb_k = g.bs_k;
     p.status = ctx.status_word_dev;
     if (g.conv) {
         p.conv_cb = (int)(g.img_c / HK);
@@ -669,8 +628,8 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
 
     const int out_mask = (g.c ? 1 : 0) | (g.c_hi ? 2 : 0) | (g.h_hi ? 4 : 0);
     char num[96];
-    snprintf(num, sizeof num, "gemm_h2 %d %d %d %d %d %d %d %d %d %d\n", bn, ctas, g.b_blocks, sliced ? 1 : 0, aux_vec ? 1 : 0, g.conv ? (halo ? 2 : 1) : 0, g.naux, rowinv, per_col, out_mask);
-    const bool plain = !g.conv && !g.b_blocks && g.naux == 0 && g.epilogue.empty() && out_mask == 1;
+    snprintf(num, sizeof num, "gemm_h2 %d %d %d %d %d %d %d %d %d\n", bn, ctas, sliced ? 1 : 0, aux_vec ? 1 : 0, g.conv ? (halo ? 2 : 1) : 0, g.naux, rowinv, per_col, out_mask);
+    const bool plain = !g.conv && g.naux == 0 && g.epilogue.empty() && out_mask == 1;
     const std::string key = num + g.epilogue;
     Module *mod = plain ? nullptr : ctx.module_find(key);
     if (!plain && !mod) {
@@ -683,7 +642,6 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
         define("SAGE_EPI_NAUX", g.naux);
         define("SAGE_H2_CONV", g.conv ? 1 : 0);
         define("SAGE_H2_AUX_VEC", aux_vec ? 1 : 0);
-        define("SAGE_H2_BLOCKS", g.b_blocks);
         define("SAGE_H2_HALO", halo ? 1 : 0);
         src += "#define SAGE_EPI_EXPR(x0, x1, x2, x3) (" + (g.epilogue.empty() ? std::string("x0") : g.epilogue) + ")\n";
         src += kGemmTcDeviceSrc;
@@ -702,9 +660,9 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
             return o.hi && aligned16(o.hi) && o.ld % 8 == 0 && o.ld > 0 && o.plane % 8 == 0 && o.plane > 0 && (o.nb0 == 1 || (o.sb0 % 8 == 0 && o.sb0 > 0)) &&
                    (o.nb1 == 1 || (o.sb1 % 8 == 0 && o.sb1 > 0));
         };
-        bool good = ok(g.b) && (g.b_blocks == 2 ? encode_operand_mn(encode, g.b, g.n, &map_b) : encode_operand(encode, g.b, g.k, (unsigned)(bn / ctas), &map_b));
+        bool good = ok(g.b) && encode_operand(encode, g.b, g.k, (unsigned)(bn / ctas), &map_b);
         map_b2 = map_b;
-        if (cols.narrow && g.b_blocks != 2) good = good && encode_operand(encode, g.b, g.k, (unsigned)(p.rag_bn / ctas), &map_b2);
+        if (cols.narrow) good = good && encode_operand(encode, g.b, g.k, (unsigned)(p.rag_bn / ctas), &map_b2);
         if (!g.conv) {
             good = good && ok(g.a) && encode_operand(encode, g.a, g.k, BM, &map_a);
             map_a2 = map_a;

@@ -185,8 +185,6 @@ struct H2Gemm {
     Window win{};
     long long m = 0, n = 0, k = 0, batch = 1;
     H2Operand a, b;
-    int b_blocks = 0;         // b.scale is one per 64 x 64 block: 1 = b's rows are n, 2 = they are k (and b.rows = k)
-    long long bs_n = 0, bs_k = 0;         // ... at column / 64 * bs_n + k / 64 * bs_k
     float *c = nullptr, *c_hi = nullptr;  // result as fp32 and / or as tf32 planes, as in TcGemm
     long long c_plane = 0;
     unsigned short *h_hi = nullptr;       // ... and / or in half-precision pieces: needs n, ldc, sc0, sc1 multiples of 64
@@ -225,8 +223,6 @@ struct H2Split {
 size_t split_h2_bytes(long long batches, long long rows, long long cols, bool whole_rows);
 sage_status split_h2_view_into(Context &ctx, const float *src, const SplitView &v, bool whole_rows, void *dst, H2Split *out);
 sage_status split_h2_view(Context &ctx, const float *src, const SplitView &v, bool whole_rows, H2Split *out);
-// [rows][cols] with a scale per 64 x 64 block, [(rows + 63) / 64][cols / 64]; cols a multiple of 64
-sage_status split_h2_blocks(Context &ctx, const float *src, long long rows, long long cols, long long ld, unsigned short *hi, long long plane, float *scale);
 // Operand B straight into memory the caller laid out: rows of `out->pitch` at out->hi / out->hi + out->plane, out->scale.
 sage_status split_h2_rows_at(Context &ctx, const float *src, const SplitView &v, const H2Split &out);
 H2Operand h2_operand(const H2Split &s, long long batches, long long rows, long long cols, bool whole_rows);
@@ -276,9 +272,6 @@ struct OptSlot {
     float *m = nullptr, *v = nullptr;
     float *hi = nullptr;
     long long plane = 0, n = 0;
-    unsigned short *h2 = nullptr;  // half-precision pieces with a scale per 64 x 64 block of [n / cols][cols]; needs 16-byte alignment throughout
-    long long h2_plane = 0, cols = 0;
-    float *h2_scale = nullptr;
     int first = 0, vec = 0;
 };
 struct OptSgd {

@@ -8,17 +8,13 @@
 // twenty million share a launch.  The arithmetic is the reference's, operation for operation and
 // rounded after every step (no contraction into fused multiply-adds), so the result does not depend
 // on how the expressions are cut into kernels.  A parameter that a GEMM reads keeps tf32 hi / lo
-// planes, or half-precision pieces with a scale per 64 x 64 block, beside it; the update writes those too, which saves the
-// separate split pass every step.
+// planes beside it; the update writes those too, which saves the separate split pass every step.
 #include <cuda.h>
 #include <cuda_runtime.h>
-
-#include <vector>
 
 #include "kernels.h"
 #include "launch.h"
 #include "gemm_tc_device.inc"  // split_tf32_value
-#include "gemm_h2_device.inc"  // h2_split2
 
 namespace sage {
 namespace k {
@@ -57,10 +53,8 @@ struct AdamRule {
     }
 };
 
-// BLOCKS: every slot keeps pieces with block scales (the others would pay for its registers: 105 -> 133 us per 32 slots)
-template <bool STATE, bool BLOCKS, class Rule>
+template <bool STATE, class Rule>
 __global__ void __launch_bounds__(256) optimizer_update_kernel(const __grid_constant__ OptBatch b, const Rule rule) {
-    __shared__ unsigned block_max[8];
     grid_dependency_sync();
     const unsigned total = b.first_chunk[b.count];
     for (unsigned chunk = blockIdx.x; chunk < total; chunk += gridDim.x) {
@@ -74,58 +68,6 @@ __global__ void __launch_bounds__(256) optimizer_update_kernel(const __grid_cons
         const long long begin = (long long)(chunk - b.first_chunk[lo]) * kChunk;
         const long long end = begin + kChunk < s.n ? begin + kChunk : s.n;
         const bool first = s.first != 0;
-        if constexpr (BLOCKS) {  // the chunk is a 64 x 64 block: its new values stay in registers until its largest magnitude is known
-            const long long tiles_c = s.cols >> 6, t = chunk - b.first_chunk[lo], rows = s.n / s.cols, r0 = t / tiles_c * 64;
-            const long long at0 = r0 * s.cols + t % tiles_c * 64 + (threadIdx.x & 15) * 4;
-            const int r_first = threadIdx.x >> 4;
-            float4 p[4], g[4], m[4], v[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const float4 zero = {0.f, 0.f, 0.f, 0.f};
-                const long long r = r_first + 16 * q, i = at0 + r * s.cols;
-                const bool in = r0 + r < rows;
-                p[q] = in ? *reinterpret_cast<const float4 *>(s.p + i) : zero;
-                g[q] = in ? *reinterpret_cast<const float4 *>(s.g + i) : zero;
-                m[q] = STATE && !first && in ? *reinterpret_cast<const float4 *>(s.m + i) : zero;
-                v[q] = STATE && !first && in ? *reinterpret_cast<const float4 *>(s.v + i) : zero;
-            }
-            unsigned big = 0;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const long long r = r_first + 16 * q, i = at0 + r * s.cols;
-                if (r0 + r >= rows) continue;
-                p[q].x = rule(p[q].x, g[q].x, &m[q].x, &v[q].x, first);
-                p[q].y = rule(p[q].y, g[q].y, &m[q].y, &v[q].y, first);
-                p[q].z = rule(p[q].z, g[q].z, &m[q].z, &v[q].z, first);
-                p[q].w = rule(p[q].w, g[q].w, &m[q].w, &v[q].w, first);
-                *reinterpret_cast<float4 *>(s.p + i) = p[q];
-                if (STATE) {
-                    *reinterpret_cast<float4 *>(s.m + i) = m[q];
-                    *reinterpret_cast<float4 *>(s.v + i) = v[q];
-                }
-                big = max(big, max(max(sage_tc::h2_finite_bits(p[q].x), sage_tc::h2_finite_bits(p[q].y)), max(sage_tc::h2_finite_bits(p[q].z), sage_tc::h2_finite_bits(p[q].w))));
-            }
-            big = __reduce_max_sync(0xffffffffu, big);
-            __syncthreads();  // the previous chunk's maxima have been read
-            if ((threadIdx.x & 31) == 0) block_max[threadIdx.x >> 5] = big;
-            __syncthreads();
-#pragma unroll
-            for (int w = 0; w < 8; ++w) big = max(big, block_max[w]);
-            float scale;
-            const float factor = sage_tc::h2_factor(big, &scale);
-            if (threadIdx.x == 0) s.h2_scale[t] = scale;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const long long r = r_first + 16 * q, i = at0 + r * s.cols;
-                if (r0 + r >= rows) continue;
-                uint2 h, l;
-                sage_tc::h2_split2(p[q].x, p[q].y, factor, &h.x, &l.x);
-                sage_tc::h2_split2(p[q].z, p[q].w, factor, &h.y, &l.y);
-                *reinterpret_cast<uint2 *>(s.h2 + i) = h;
-                *reinterpret_cast<uint2 *>(s.h2 + s.h2_plane + i) = l;
-            }
-            continue;
-        } else {
         if (s.vec) {
             for (long long i = begin + 4 * threadIdx.x; i + 3 < end; i += 4 * 256) {
                 const float4 p = *reinterpret_cast<const float4 *>(s.p + i);
@@ -176,15 +118,13 @@ __global__ void __launch_bounds__(256) optimizer_update_kernel(const __grid_cons
                 s.hi[s.plane + i] = l;
             }
         }
-        }
     }
 }
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-template <bool STATE, bool BLOCKS, class Rule>
-sage_status run_kind(Context &ctx, const std::vector<OptSlot> &slots, const Rule &rule, const char *label) {
-    const int count = (int)slots.size();
+template <bool STATE, class Rule>
+sage_status run(Context &ctx, const OptSlot *slots, int count, const Rule &rule, const char *label) {
     for (int at = 0; at < count; at += kOptSlots) {
         OptBatch b;
         b.count = count - at < kOptSlots ? count - at : kOptSlots;
@@ -196,8 +136,7 @@ sage_status run_kind(Context &ctx, const std::vector<OptSlot> &slots, const Rule
                     (!s.hi || (aligned16(s.hi) && s.plane % 4 == 0));
             b.slot[i] = s;
             b.first_chunk[i] = chunks;
-            if (s.h2 && (!s.vec || s.cols % 64 || s.n % s.cols || !aligned16(s.h2) || s.h2_plane % 8)) return ctx.fail(SAGE_ERR_INVALID, "optimizer update: pieces need whole columns of blocks");
-            const long long c = s.h2 ? (s.n / s.cols + 63) / 64 * (s.cols / 64) : (s.n + kChunk - 1) / kChunk;
+            const long long c = (s.n + kChunk - 1) / kChunk;
             if (c + chunks > 0x7fffffffll) return ctx.fail(SAGE_ERR_INVALID, "optimizer update: too many elements in one call");
             chunks += (unsigned)c;
         }
@@ -208,18 +147,10 @@ sage_status run_kind(Context &ctx, const std::vector<OptSlot> &slots, const Rule
         ctx.note_launch(label);
         if (ctx.dry()) continue;
         sage_status st = ctx.check_cuda(
-            launch_dependent(ctx.pdl, ctx.stream(), optimizer_update_kernel<STATE, BLOCKS, Rule>, dim3(grid), dim3(256), 0, b, rule), label);
+            launch_dependent(ctx.pdl, ctx.stream(), optimizer_update_kernel<STATE, Rule>, dim3(grid), dim3(256), 0, b, rule), label);
         if (st) return st;
     }
     return SAGE_OK;
-}
-
-template <bool STATE, class Rule>
-sage_status run(Context &ctx, const OptSlot *slots, int count, const Rule &rule, const char *label) {
-    std::vector<OptSlot> kind[2];
-    for (int i = 0; i < count; ++i) kind[slots[i].h2 ? 1 : 0].push_back(slots[i]);
-    sage_status st = run_kind<STATE, false>(ctx, kind[0], rule, label);
-    return st ? st : run_kind<STATE, true>(ctx, kind[1], rule, label);
 }
 
 }  // namespace

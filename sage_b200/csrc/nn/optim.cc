@@ -83,18 +83,6 @@ sage_status prepare(const std::vector<Var> &params, const std::vector<Var> &grad
         } else {
             ps.split.reset();
         }
-        if (ps.h2_blocks) {  // likewise
-            const Shape &bs = ps.h2_blocks->view;
-            const bool whole = bs.rank() == 2 && bs.offset == 0 && bs.has_default_strides() && bs.size() == slot.n;
-            if (whole && ((uintptr_t)slot.p | (uintptr_t)slot.g) % 16 == 0 && !slot.hi) {
-                slot.h2 = ps.h2_blocks->pieces.hi;
-                slot.h2_plane = ps.h2_blocks->pieces.plane;
-                slot.h2_scale = ps.h2_blocks->pieces.scale;
-                slot.cols = bs.extents[1];
-            } else {
-                ps.h2_blocks.reset();
-            }
-        }
         out->slots.push_back(slot);
         out->keep.push_back(gt);
     }

@@ -258,39 +258,3 @@ def test_bert_training_step_vs_oracle(ctx):
         if i not in noise:
             assert adam_close(ctx.read(p), r.data.numpy(), 1e-3, 3), i
     assert ctx.status_word() == 0
-
-
-@pytest.mark.parametrize("m,k,n", [(2100, 64, 1024), (8292, 128, 512), (1030, 64, 1472), (33000, 64, 256)])
-def test_weights_with_block_scales(m, k, n):
-    """A two-layer step whose weights are read as they lie and transposed: losses, gradients and the pieces the optimizer rewrites
-    (two steps), against float64.  Tolerance 1e-5 of max(|x|, rms) for a product, twice for the gradient behind two of them."""
-    rng = np.random.default_rng(m + n)
-    x, t = rng.uniform(-1, 1, (m, k)).astype(np.float32), rng.uniform(-1, 1, (m, 64)).astype(np.float32)
-    w = [rng.uniform(-1, 1, s).astype(np.float32) * np.float32(0.1) for s in ((k, n), (n, n), (n, 64))]
-    f = rng.uniform(0.5, 1.5, (m, n)).astype(np.float32)
-    ctx = S.Context(0)
-    try:
-        X, T, F, W = ctx.var(x), ctx.var(t), ctx.var(f), [ctx.var(a) for a in w]
-        h1 = S.matmul(X, W[0]) * F
-        h2 = S.matmul(h1, W[1]) * F
-        d = S.matmul(h2, W[2]) - T
-        loss = (d * d).sum([0, 1], False)
-        grads = S.grad(loss, W)
-        opt = S.Sgd(1e-3)
-        for _ in range(2):
-            ctx.clear()
-            ctx.eval(loss, *grads)
-            w64, x64 = [a.astype(np.float64) for a in w], x.astype(np.float64)
-            a1 = (x64 @ w64[0]) * f
-            a2 = (a1 @ w64[1]) * f
-            e = 2 * (a2 @ w64[2] - t)
-            g2 = (e @ w64[2].T) * f
-            g1 = (g2 @ w64[1].T) * f
-            for got, want in zip(grads, (x64.T @ g1, a1.T @ g2, a2.T @ e)):
-                got = ctx.read(got).astype(np.float64)
-                assert (np.abs(got - want) / np.maximum(np.abs(want), np.sqrt((want ** 2).mean()))).max() <= 2e-5
-            opt.update(dict(zip(W, grads)), ctx)
-            w = [ctx.read(a) for a in W]
-        assert ctx.status_word() == 0
-    finally:
-        ctx.close()
