@@ -222,3 +222,52 @@ def test_attention_with_a_thread_per_row(ctx, n, length, heads, keyed):
         want = (p / p.sum(-1, keepdims=True)) @ v[i].astype(np.float64)
         assert (np.abs(got[i] - want) / np.maximum(np.abs(want), np.sqrt((want ** 2).mean()))).max() <= 1e-4
     assert ctx.status_word() == 0
+
+
+@pytest.mark.parametrize("n,heads,length", [(5, 2, 77), (5, 1, 200), (5, 30, 257)])
+def test_attention_over_scores_far_below_zero(n, heads, length):
+    """Every score of a sequence shifted by the same amount, as a mask on the whole sequence does: the quotient is unchanged
+    whichever maximum is subtracted, also where the reference's reduce starts at 0 (ref_compat = 1) and exp(x - 0) lies far below
+    what half-precision pieces of a weight near 1 hold.  Both forms of the kernel.  Per row, relative to the row's rms: 1e-4, as
+    for the other attention blocks.  A row whose every exp(x) is 0 in fp32 is 0 / 0 under ref_compat, as in the reference."""
+    rng = np.random.default_rng(length)
+    q, k, v = [rng.uniform(-1, 1, (n, heads, length, 64)).astype(np.float32) for _ in range(3)]
+    shift = np.array([-20, -30, -40, -80, -150], np.float32)
+    q64, k64, v64 = [t.astype(np.float64) for t in (q, k, v)]
+    s = q64 @ k64.transpose(0, 1, 3, 2) / 8.0
+    p = np.exp(s - s.max(-1, keepdims=True))
+    want = (p / p.sum(-1, keepdims=True)) @ v64
+    for compat in (1, 0):
+        c = S.Context(0, ref_compat=compat)
+        try:
+            sc = S.matmul_batched(c.var(q), S.transpose(c.var(k), -1, -2)) / 8.0 + S.view(c.var(shift), [n, 1, 1, 1])
+            got = S.matmul_batched(S.softmax(sc, [3]), c.var(v)).eval(c).astype(np.float64)
+            assert "attention" in c.describe() and c.status_word() == 0
+        finally:
+            c.close()
+        if compat:
+            assert np.isnan(got[4]).all()
+        rows = slice(0, 4 if compat else 5)
+        err = np.abs(got - want) / np.sqrt((want ** 2).mean(-1, keepdims=True))
+        assert np.nanmax(err[rows]) <= 1e-4 and not np.isnan(err[rows]).any(), [float(e.max()) for e in err]
+
+
+@pytest.mark.parametrize("compat", [1, 0])
+def test_attention_whose_first_keys_are_masked_with_infinity(compat):
+    """More than one block of keys at -inf before the first finite score: their weights are 0, not exp(-inf + inf)."""
+    rng = np.random.default_rng(83)
+    n, heads, length = 2, 2, 300
+    q, k, v = [rng.uniform(-1, 1, (n, heads, length, 64)).astype(np.float32) for _ in range(3)]
+    bias = np.zeros((n, length), np.float32)
+    bias[:, :140] = -np.inf
+    c = S.Context(0, ref_compat=compat)
+    try:
+        sc = S.matmul_batched(c.var(q), S.transpose(c.var(k), -1, -2)) / 8.0 + S.view(c.var(bias), [n, 1, 1, length])
+        got = S.matmul_batched(S.softmax(sc, [3]), c.var(v)).eval(c).astype(np.float64)
+        assert "attention" in c.describe() and c.status_word() == 0
+    finally:
+        c.close()
+    s = q.astype(np.float64) @ k[:, :, 140:].astype(np.float64).transpose(0, 1, 3, 2) / 8.0
+    p = np.exp(s - s.max(-1, keepdims=True))
+    want = (p / p.sum(-1, keepdims=True)) @ v[:, :, 140:].astype(np.float64)
+    assert (np.abs(got - want) / np.maximum(np.abs(want), np.sqrt((want ** 2).mean()))).max() <= 1e-4
