@@ -113,12 +113,14 @@ struct Pool2dOp : Operator {
         shape_fail("pool2d composite is not differentiated; grad walks the decomposed graph");
     }
     sage_status compute(const std::vector<Tensor> &x, Context &ctx, Tensor *y) override {
-        const bool emit_h2 = ctx.hint_emit_h2, only = emit_h2 && !ctx.hint_emit_planes && ctx.hint_planes_only;
+        const Array &e = x[0].desc.shape.extents;
+        const Array &o = out.shape.extents;
+        // an image off the 16-byte grid takes the kernel without pieces; its reader splits the result
+        const bool emit_h2 = ctx.hint_emit_h2 && k::pool2d_writes_pieces((const float *)x[0].ptr(), e[3], o[1], o[2]);
+        const bool only = emit_h2 && !ctx.hint_emit_planes && ctx.hint_planes_only;
         ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = false;
         sage_status st = Tensor::uninit(ctx, out, y);
         if (st) return st;
-        const Array &e = x[0].desc.shape.extents;
-        const Array &o = out.shape.extents;
         k::PlaneOut forms;
         if (emit_h2) {
             st = storage_h2_attach(ctx, *y->data);
@@ -134,7 +136,7 @@ struct Pool2dOp : Operator {
 };
 bool pool_op_emits_h2(const Operator &op) {
     const Pool2dOp *p = dynamic_cast<const Pool2dOp *>(&op);
-    return p && k::pool2d_writes_pieces(p->out.shape.extents[3]);
+    return p && k::pool2d_writes_pieces(nullptr, p->out.shape.extents[3], p->out.shape.extents[1], p->out.shape.extents[2]);
 }
 
 static Var pool(const Var &x, Pair ker, Pair stride, Pair pad, Pair dil, bool is_max) {

@@ -532,7 +532,9 @@ sage_status col2im(Context &ctx, const float *col, float *img, long long n, long
     return ctx.check_cuda(cudaGetLastError(), "col2im launch");
 }
 
-bool pool2d_writes_pieces(long long chan) { return chan % 64 == 0; }
+bool pool2d_writes_pieces(const float *img, long long chan, long long out_h, long long out_w) {
+    return chan % 64 == 0 && reinterpret_cast<uintptr_t>(img) % 16 == 0 && out_h * out_w <= 0x7fffffffLL;
+}
 
 sage_status pool2d(Context &ctx, bool is_max, const float *img, float *out, long long n, long long img_h,
                    long long img_w, long long chan, long long out_h, long long out_w, const Window &w, const PlaneOut &forms) {
@@ -542,7 +544,7 @@ sage_status pool2d(Context &ctx, bool is_max, const float *img, float *out, long
     if (ctx.dry() || total == 0) return SAGE_OK;
     const bool vec = chan % 4 == 0 && reinterpret_cast<uintptr_t>(img) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0 &&
                      out_h * out_w <= 0x7fffffffLL;
-    if (forms.h2 && !(vec && pool2d_writes_pieces(chan))) return ctx.fail(SAGE_ERR_INVALID, "pool2d: half-precision pieces need whole groups of channels");
+    if (forms.h2 && !(vec && pool2d_writes_pieces(img, chan, out_h, out_w))) return ctx.fail(SAGE_ERR_INVALID, "pool2d: half-precision pieces need whole groups of channels");
     // 32-bit indices where they reach: two 64-bit divisions were a third of a thread's instructions
     const bool narrow = total < (1LL << 31) && img_h * img_w * chan < (1LL << 31);
     auto kernel = narrow ? pool2d_kernel<4, unsigned> : pool2d_kernel<4, long long>;

@@ -79,7 +79,7 @@ sage_status pack_small_c_filter(Context &ctx, const float *filt, int kh, int kw,
 sage_status pack_first_image(Context &ctx, const float *img, long long n, long long h, long long w, long long c, long long hp, long long wp, int pad_h, int pad_w,
                              unsigned short *hi, long long plane, float *scale, unsigned *parts);
 sage_status pack_first_filter(Context &ctx, const float *filt, int kh, int kw, int c, int oc, unsigned short *out, float *scale);
-bool pool2d_writes_pieces(long long chan);
+bool pool2d_writes_pieces(const float *img, long long chan, long long out_h, long long out_w);
 sage_status pool2d(Context &ctx, bool is_max, const float *img, float *out, long long n, long long img_h,
                    long long img_w, long long chan, long long out_h, long long out_w, const Window &w, const PlaneOut &forms);
 

@@ -271,3 +271,29 @@ def test_attention_whose_first_keys_are_masked_with_infinity(compat):
     p = np.exp(s - s.max(-1, keepdims=True))
     want = (p / p.sum(-1, keepdims=True)) @ v[:, :, 140:].astype(np.float64)
     assert (np.abs(got - want) / np.maximum(np.abs(want), np.sqrt((want ** 2).mean()))).max() <= 1e-4
+
+
+def _conv64(x, f, stride, pad):
+    x = np.pad(x.astype(np.float64), ((0, 0), (pad, pad), (pad, pad), (0, 0)))
+    k = f.shape[0]
+    oh, ow = (x.shape[1] - k) // stride + 1, (x.shape[2] - k) // stride + 1
+    return sum(x[:, i:i + stride * (oh - 1) + 1:stride, j:j + stride * (ow - 1) + 1:stride] @ f[i, j].astype(np.float64) for i in range(k) for j in range(k))
+
+
+def _close(got, want, tol=1e-5):
+    return (np.abs(got - want) / np.maximum(np.abs(want), np.sqrt((want ** 2).mean()))).max() <= tol
+
+
+@pytest.mark.parametrize("off", [0, 1, 3, 4])
+def test_pooling_of_an_image_off_the_16_byte_grid(ctx, off):
+    """The convolution behind reads the pool's pieces where the pool writes them, and splits its result where it does not."""
+    rng = np.random.default_rng(85)
+    shape = (4, 30, 30, 64)
+    n = int(np.prod(shape))
+    flat = rng.uniform(-1, 1, (off + n,)).astype(np.float32)
+    x, f = flat[off:].reshape(shape), rng.uniform(-1, 1, (3, 3, 64, 64)).astype(np.float32)
+    p = S.max_pool_2d(S.view(ctx.var(flat).slice(0, off, off + n), list(shape)), 2, 2, 0, 1)
+    got = S.conv_2d(p, ctx.var(f), 1, 1, 1).eval(ctx)
+    m = np.maximum(x.reshape(4, 15, 2, 15, 2, 64).max((2, 4)), 0)
+    assert _close(got, _conv64(m, f, 1, 1))
+    assert ctx.status_word() == 0
