@@ -83,6 +83,13 @@ std::shared_ptr<Operator> make_expand_op(const TensorDesc &in, const Array &exte
     return op;
 }
 
+// How much further into its operand's storage a view starts.  (A reshape keeps the start of what it reads, which its static
+// shape does not show.)
+long long view_op_offset(const Operator &op) {
+    const ViewOp *v = dynamic_cast<const ViewOp *>(&op);
+    return v && v->kind == VSlice ? v->start * v->in[0].shape.strides[v->axis] : 0;
+}
+
 // 0 reshape, 1 expand, 2 permute, 3 squeeze, 4 unsqueeze, 5 slice; -1 when `op` is no view
 int view_op_kind(const Operator &op) {
     const ViewOp *v = dynamic_cast<const ViewOp *>(&op);

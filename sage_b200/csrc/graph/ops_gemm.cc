@@ -204,9 +204,23 @@ bool h2_view_direct(const Shape &sh, bool trans, BatchLevels *bl) {
         if (bl->n[l] > 1 && (bl->s[l] <= 0 || bl->s[l] % 64)) return false;
     return true;
 }
+// The same for a convolution's image (contiguous, channels in whole groups).
+static bool conv_image_direct(const Shape &sh) { return sh.offset % 64 == 0; }
 bool h2_view_ok(const Shape &sh, bool trans) {
     BatchLevels bl;
     return h2_view_direct(sh, trans, &bl);
+}
+
+// Compact pieces of a view, kept beside the storage (`*c`) until another view is asked for there.
+static sage_status gather_h2(Context &ctx, const Tensor &t, bool swapped, const k::SplitView &v, bool whole_rows, std::shared_ptr<H2Cache> *c) {
+    if (*c && (*c)->view == t.desc.shape && (*c)->swapped == swapped) return SAGE_OK;
+    auto fresh = std::make_shared<H2Cache>();
+    fresh->alloc = ctx.allocator_ptr();
+    fresh->view = t.desc.shape;
+    fresh->swapped = swapped;
+    sage_status s = k::split_h2_view(ctx, (const float *)t.ptr(), v, whole_rows, &fresh->pieces);
+    if (!s) *c = fresh;
+    return s;
 }
 
 // Operand A (`rows` = a scale per 64 k) or B (`whole_rows`: one per row, always a compact copy kept beside the storage).
@@ -237,25 +251,18 @@ static sage_status make_h2_operand(Context &ctx, const Tensor &t, bool trans, bo
     }
     if (st.planes_only) return ctx.fail(SAGE_ERR_INVALID, "internal: a tensor without fp32 values reached an operand that has to be gathered");
     if (!collapse_batch(sh, r - 2, &bl)) return ctx.fail(SAGE_ERR_UNSUPPORTED, "gemm: batch axes of an operand do not collapse to two levels");
+    k::SplitView v;
+    v.nb0 = bl.n[0];
+    v.nb1 = bl.n[1];
+    v.sb0 = bl.s[0];
+    v.sb1 = bl.s[1];
+    v.rows = rows;
+    v.cols = cols;
+    v.ld = sh.strides[ma];
+    v.col_stride = sh.strides[ka];
     std::shared_ptr<H2Cache> &c = whole_rows ? st.h2_rows : st.h2_view;
-    if (!(c && c->view == sh && c->swapped == trans)) {
-        auto fresh = std::make_shared<H2Cache>();
-        fresh->alloc = ctx.allocator_ptr();
-        fresh->view = sh;
-        fresh->swapped = trans;
-        k::SplitView v;
-        v.nb0 = bl.n[0];
-        v.nb1 = bl.n[1];
-        v.sb0 = bl.s[0];
-        v.sb1 = bl.s[1];
-        v.rows = rows;
-        v.cols = cols;
-        v.ld = sh.strides[ma];
-        v.col_stride = sh.strides[ka];
-        sage_status s = k::split_h2_view(ctx, (const float *)t.ptr(), v, whole_rows, &fresh->pieces);
-        if (s) return s;
-        c = fresh;
-    }
+    sage_status s = gather_h2(ctx, t, trans, v, whole_rows, &c);
+    if (s) return s;
     *hold = c;
     *op = k::h2_operand(c->pieces, bl.n[0] * bl.n[1], rows, cols, whole_rows);
     return SAGE_OK;
@@ -672,14 +679,26 @@ struct GemmOp : Operator {
         sage_status st;
         if (conv) {
             const Shape &img_shape = x[0].desc.shape;
-            if (!img_shape.has_default_strides() || img_shape.offset % 64 || x[0].data->bytes % 256) return ctx.fail(SAGE_ERR_INVALID, "internal: conv gemm needs a contiguous image");
-            st = storage_h2(ctx, *x[0].data);
+            Storage &is = *x[0].data;
+            if (!img_shape.has_default_strides()) return ctx.fail(SAGE_ERR_INVALID, "internal: conv gemm needs a contiguous image");
+            long long at = 0;  // where the image starts in the pieces
+            if (conv_image_direct(img_shape) && is.bytes % 256 == 0) {
+                st = storage_h2(ctx, is);
+                hold_a = is.h2;
+                at = img_shape.offset;
+            } else {  // the storage's groups of 64 are not the image's: pieces of the image alone, laid out like it
+                if (is.planes_only) return ctx.fail(SAGE_ERR_INVALID, "internal: a tensor without fp32 values reached a convolution that has to gather it");
+                k::SplitView v;
+                v.rows = img[0] * img[1] * img[2];
+                v.cols = v.ld = img[3];
+                st = gather_h2(ctx, x[0], false, v, false, &is.h2_view);
+                hold_a = is.h2_view;
+            }
             if (st) return st;
-            hold_a = x[0].data->h2;
             g.conv = true;
-            g.a.hi = hold_a->pieces.hi + img_shape.offset;
+            g.a.hi = hold_a->pieces.hi + at;
             g.a.plane = hold_a->pieces.plane;
-            g.a.scale = hold_a->pieces.scale + img_shape.offset / 64;
+            g.a.scale = hold_a->pieces.scale + at / 64;
             g.img_n = img[0];
             g.img_h = img[1];
             g.img_w = img[2];
@@ -1122,17 +1141,21 @@ std::shared_ptr<Operator> gemm_with_im2col(const Operator &op, const Operator &i
     return c;
 }
 
-// Will operand `idx` be read straight from whole-storage planes (never through the fp32 buffer)?
+// Will operand `idx`, which starts `offset` elements into its producer's result, be read straight from whole-storage planes
+// (never through the fp32 buffer)?
 bool is_grouped_gemm_op(const Operator &op);
 bool grouped_gemm_is_h2(const Operator &op);
 std::shared_ptr<Operator> grouped_gemm_on_h2(const Operator &op);
-bool gemm_operand_static_direct(const Operator &op, int idx) {
-    if (is_grouped_gemm_op(op)) return idx == 0 && (grouped_gemm_is_h2(op) ? h2_view_ok(op.in[0].shape, false) : gemm_operand_view_ok(op.in[0].shape));
+bool gemm_operand_static_direct(const Operator &op, int idx, long long offset) {
+    if (idx < 0 || idx >= (int)op.in.size()) return false;
+    Shape sh = op.in[idx].shape;
+    sh.offset = offset;
+    if (is_grouped_gemm_op(op)) return idx == 0 && (grouped_gemm_is_h2(op) ? h2_view_ok(sh, false) : gemm_operand_view_ok(sh));
     const GemmOp *g = as_gemm(op);
-    if (g && g->attn) return idx >= 0 && idx < 3 && GemmOp::attention_view_direct(g->in[idx].shape, g->attention_trans(idx));
-    if (g && g->h2) return idx == 0 && (g->conv || h2_view_ok(g->in[0].shape, g->ta));
-    if (g && g->conv && idx == 0) return g->conv_implicit() && !g->conv_raw();  // planes only when the kernel does not split the image itself
-    return g && idx >= 0 && idx < 2 && gemm_operand_view_ok(g->in[idx].shape);
+    if (g && g->attn) return idx < 3 && GemmOp::attention_view_direct(sh, g->attention_trans(idx));
+    if (g && g->h2) return idx == 0 && (g->conv ? conv_image_direct(sh) : h2_view_ok(sh, g->ta));
+    if (g && g->conv && idx == 0) return g->conv_implicit() && !g->conv_raw() && offset % 4 == 0;  // planes only when the kernel does not split the image itself
+    return g && idx < 2 && gemm_operand_view_ok(sh);
 }
 
 // ---- which products run on half-precision pieces (session.cc: assign_h2)
@@ -1404,6 +1427,10 @@ struct SlabOp : Operator {
 };
 
 bool is_slab_op(const Operator &op) { return dynamic_cast<const SlabOp *>(&op) != nullptr; }
+long long slab_offset(const Operator &op) {
+    const SlabOp *s = dynamic_cast<const SlabOp *>(&op);
+    return s ? s->index * s->out.shape.size() : 0;
+}
 bool is_grouped_gemm_op(const Operator &op) { return dynamic_cast<const GroupedGemmOp *>(&op) != nullptr; }
 
 bool grouped_gemm_is_h2(const Operator &op) {

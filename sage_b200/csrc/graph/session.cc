@@ -59,7 +59,9 @@ std::shared_ptr<Operator> gemm_with_attention(const Operator &outer_op, const Op
 bool attention_small_products(const Operator &outer_op, const Operator &score_op, std::shared_ptr<Operator> *outer, std::shared_ptr<Operator> *score);
 bool is_attention_op(const Operator &op);
 bool is_grouped_gemm_op(const Operator &op);
-bool gemm_operand_static_direct(const Operator &op, int idx);
+bool gemm_operand_static_direct(const Operator &op, int idx, long long offset);
+long long view_op_offset(const Operator &op);
+long long slab_offset(const Operator &op);
 bool gemm_group_key(const Operator &op, std::string *key);
 std::shared_ptr<Operator> make_grouped_gemm(const std::vector<const Operator *> &members);
 std::shared_ptr<Operator> make_slab(const Operator &grouped, int index, const TensorDesc &member_out);
@@ -467,9 +469,11 @@ static void lower(Node &n, bool tc, bool softmax_in_gemm, bool attention) {
 
 // Which values a tensor-core GEMM reads (through views only): in-tree producers get emit_planes,
 // states are collected so that their routine's root gets it.
-static Node *skip_views(Node *p) {
+static Node *skip_views(Node *p, long long *offset = nullptr) {  // *offset: where in the producer's result the views start
+    if (offset) *offset = 0;
     for (;;) {
         if (p->is_data) return p;
+        if (offset) *offset += p->shared ? slab_offset(*p->op) : view_op_offset(*p->op);
         if (p->shared) p = p->shared.get();  // a slab of a grouped product
         else if (is_view_op(*p->op)) p = &p->args[0];
         else return p;
@@ -581,13 +585,14 @@ static void mark_plane_readers(Node &n, bool tc, std::unordered_set<Origin *> *s
     if (!grouped && (!is_gemm_op(*n.op) || !gemm_runs_on_tc(*n.op, tc))) return;
     const bool h2 = gemm_is_h2(*n.op);
     for (int idx = 0; idx < (is_attention_op(*n.op) ? 3 : grouped || h2 ? 1 : 2); ++idx) {
-        Node *p = skip_views(&n.args[idx]);
+        long long offset = 0;
+        Node *p = skip_views(&n.args[idx], &offset);
         if (p->is_data) {
-            if (p->var.is_op() && gemm_operand_static_direct(*n.op, idx)) (h2 ? h2_states : states)->insert(p->var.key());
+            if (p->var.is_op() && gemm_operand_static_direct(*n.op, idx, offset)) (h2 ? h2_states : states)->insert(p->var.key());
         } else if (h2 ? can_emit_h2(*p->op) : can_emit_planes(*p->op, tc)) {
             // Inside a routine's tree a node has one reader, so this GEMM is the only one — unless the
             // node is shared (a grouped product): then every slab must end in a GEMM operand.
-            const bool direct = gemm_operand_static_direct(*n.op, idx);
+            const bool direct = gemm_operand_static_direct(*n.op, idx, offset);
             if (direct) (h2 ? p->emit_h2 : p->emit_planes) = true;
             if (p->readers > 0) {
                 if (direct) ++p->gemm_readers;

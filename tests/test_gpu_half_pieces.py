@@ -284,6 +284,43 @@ def _close(got, want, tol=1e-5):
     return (np.abs(got - want) / np.maximum(np.abs(want), np.sqrt((want ** 2).mean()))).max() <= tol
 
 
+@pytest.mark.parametrize("off", [0, 1, 4, 32, 64])
+@pytest.mark.parametrize("tail", [0, 5])
+@pytest.mark.parametrize("ker,stride", [(3, 1), (1, 2)])
+def test_convolution_of_an_image_off_the_grid_of_groups(ctx, off, tail, ker, stride):
+    """A part of a flat array as the image: its start may lie anywhere and its storage be of any length.  Tolerance as for the
+    other convolutions."""
+    rng = np.random.default_rng(off + tail)
+    shape = (4, 16, 16, 64)
+    n = int(np.prod(shape))
+    flat = rng.uniform(-1, 1, (off + n + tail,)).astype(np.float32)
+    x = flat[off:off + n].reshape(shape)
+    f = rng.uniform(-1, 1, (ker, ker, 64, 64)).astype(np.float32)
+    v = ctx.var(flat)
+    y = S.conv_2d(S.view(v.slice(0, off, off + n), list(shape)), ctx.var(f), stride, ker // 2, 1)
+    assert _close(y.eval(ctx), _conv64(x, f, stride, ker // 2))
+    ctx.set(v, -flat)   # the gathered copy goes with the contents
+    ctx.clear()
+    assert _close(y.eval(ctx), _conv64(-x, f, stride, ker // 2))
+    assert ctx.status_word() == 0
+
+
+@pytest.mark.parametrize("off,tail", [(4, 0), (32, 0), (0, 3), (64, 0)])
+def test_convolution_entry_point_inside_a_larger_buffer(ctx, off, tail):
+    rng = np.random.default_rng(84)
+    x, f = rng.uniform(-1, 1, (2, 20, 20, 64)).astype(np.float32), rng.uniform(-1, 1, (3, 3, 64, 96)).astype(np.float32)
+    flat = np.concatenate([np.full(off, 7, np.float32), x.ravel(), np.full(tail, 7, np.float32)])
+    xt, ft, yt = ctx.tensor(flat), ctx.tensor(f), ctx.empty((2, 20, 20, 96))
+    cx, cf, cy = ctx.tensor(x), ft.c(), yt.c()
+    inner = cx.c()
+    inner.buf, inner.offset = xt.c().buf, off
+    win = S.window(1, 1, 1, 1)
+    ctx._ck(S.lib.sage_conv2d_nhwc(ctx.h, ctypes.byref(inner), ctypes.byref(cf), ctypes.byref(win), ctypes.byref(cy)))
+    assert _close(yt.numpy(), _conv64(x, f, 1, 1))
+    for t in (xt, ft, yt, cx):
+        t.release()
+
+
 @pytest.mark.parametrize("off", [0, 1, 3, 4])
 def test_pooling_of_an_image_off_the_16_byte_grid(ctx, off):
     """The convolution behind reads the pool's pieces where the pool writes them, and splits its result where it does not."""
@@ -296,4 +333,20 @@ def test_pooling_of_an_image_off_the_16_byte_grid(ctx, off):
     got = S.conv_2d(p, ctx.var(f), 1, 1, 1).eval(ctx)
     m = np.maximum(x.reshape(4, 15, 2, 15, 2, 64).max((2, 4)), 0)
     assert _close(got, _conv64(m, f, 1, 1))
+    assert ctx.status_word() == 0
+
+
+@pytest.mark.parametrize("off", [0, 1, 32])
+def test_part_of_a_result_behind_a_reshape(ctx, off):
+    """A convolution and a product over a part of another product's result that starts inside a group of 64."""
+    rng = np.random.default_rng(86)
+    n = 2 * 20 * 20 * 64
+    a, w = rng.uniform(-1, 1, (1600, 128)).astype(np.float32), rng.uniform(-1, 1, (128, 64)).astype(np.float32)
+    f, w2 = rng.uniform(-1, 1, (3, 3, 64, 64)).astype(np.float32), rng.uniform(-1, 1, (64, 128)).astype(np.float32)
+
+    def part():
+        return S.view(S.matmul(ctx.var(a) * 1.0, ctx.var(w)), [2 * n]).slice(0, off, off + n)
+    flat = (a.astype(np.float64) @ w).ravel()[off:off + n]
+    assert _close(S.conv_2d(S.view(part(), [2, 20, 20, 64]), ctx.var(f), 1, 1, 1).eval(ctx), _conv64(flat.reshape(2, 20, 20, 64), f, 1, 1))
+    assert _close(S.matmul(S.view(part(), [800, 64]), ctx.var(w2)).eval(ctx), flat.reshape(800, 64) @ w2.astype(np.float64))
     assert ctx.status_word() == 0
