@@ -286,6 +286,17 @@ static sage_status attach_forms(Context &ctx, Tensor *y, bool emit, bool emit_h2
     return SAGE_OK;
 }
 
+// The contents an operator has made a copy of, kept from pass to pass: a storage at a version, not its address, which may come
+// back as another storage's (a filter computed on every pass).  Held weakly, so that the storage is given back when its tensor is.
+struct StorageKey {
+    std::weak_ptr<Storage> storage;
+    uint64_t version = 0;
+    long long offset = 0;
+    StorageKey() {}
+    explicit StorageKey(const Tensor &t) : storage(t.data), version(t.data->version), offset(t.desc.shape.offset) {}
+    bool holds(const Tensor &t) const { return storage.lock() == t.data && version == t.data->version && offset == t.desc.shape.offset; }
+};
+
 // ------------------------------------------------------------------------------ the operator
 // Axis groups of the epilogue's index space.
 enum { GBatchHi = 0, GBatchLo = 1, GRow = 2, GCol = 3 };
@@ -348,8 +359,7 @@ struct GemmOp : Operator {
     // ... and with columns two apart as a kernel of its own, on half-precision pieces (kernels/conv_first_device.inc)
     bool conv_first() const { return conv_small_c() && !ta && !tb && !conv_raw_enabled() && img[0] <= 65535 && !folded && k::conv_first_ok(win.ker_h, win.stride_w, img[5]); }
     struct PackedFilter {  // the filter as the B operand of that GEMM, kept until the filter is rewritten
-        const Storage *key = nullptr;
-        uint64_t version = 0;
+        StorageKey key;
         std::shared_ptr<Allocator> alloc;
         Block *block = nullptr;
         ~PackedFilter() {
@@ -495,12 +505,10 @@ struct GemmOp : Operator {
             }
         } free_col{ctx, col_block};
         if (small_c) {
-            const Storage *key = x[1].data.get();
-            if (!packed_filter || packed_filter->key != key || packed_filter->version != key->version) {
+            if (!packed_filter || !packed_filter->key.holds(x[1])) {
                 auto pf = std::make_shared<PackedFilter>();
                 pf->alloc = ctx.allocator_ptr();
-                pf->key = key;
-                pf->version = key->version;
+                pf->key = StorageKey(x[1]);
                 const long long fplane = (long long)win.ker_h * 32 * n;
                 pf->block = ctx.allocator().alloc((size_t)fplane * 2 * sizeof(float));
                 if (!pf->block) return ctx.fail(SAGE_ERR_OOM, "out of memory for the re-laid filter");
@@ -617,13 +625,11 @@ struct GemmOp : Operator {
         float *scale = reinterpret_cast<float *>(image.b->ptr + piece_bytes);
         sage_status st = k::pack_first_image(ctx, (const float *)x[0].ptr(), N, H, W, img[3], hp, wp, win.pad_h, win.pad_w, hi, plane, scale, reinterpret_cast<unsigned *>(scale + N));
         if (st) return st;
-        const Storage *key = x[1].data.get();
         const long long chans = (n + 63) / 64 * 64, filter_bytes = chans * win.ker_h * 128;
-        if (!packed_filter || packed_filter->key != key || packed_filter->version != key->version) {
+        if (!packed_filter || !packed_filter->key.holds(x[1])) {
             auto pf = std::make_shared<PackedFilter>();
             pf->alloc = ctx.allocator_ptr();
-            pf->key = key;
-            pf->version = key->version;
+            pf->key = StorageKey(x[1]);
             pf->block = ctx.allocator().alloc((size_t)(filter_bytes + chans * 4));
             if (!pf->block) return ctx.fail(SAGE_ERR_OOM, "out of memory for the re-laid filter");
             st = k::pack_first_filter(ctx, (const float *)x[1].ptr(), win.ker_h, win.ker_w, (int)img[3], (int)n, reinterpret_cast<unsigned short *>(pf->block->ptr),
@@ -1228,7 +1234,7 @@ struct GroupedGemmOp : Operator {
     std::string epilogue;  // over x0 (product) and, with has_bias, x1 (the bias row)
 
     struct Concat {
-        std::vector<std::pair<const Storage *, uint64_t>> key;
+        std::vector<StorageKey> key;
         std::shared_ptr<Allocator> alloc;
         Block *block = nullptr;
         ~Concat() {
@@ -1246,7 +1252,7 @@ struct GroupedGemmOp : Operator {
     static bool same_key(const Concat *c, const std::vector<Tensor> &x, int first, int count) {
         if (!c || (int)c->key.size() != count) return false;
         for (int i = 0; i < count; ++i)
-            if (c->key[i].first != x[first + i].data.get() || c->key[i].second != x[first + i].data->version) return false;
+            if (!c->key[i].holds(x[first + i])) return false;
         return true;
     }
 
@@ -1277,7 +1283,7 @@ struct GroupedGemmOp : Operator {
                 to.scale = reinterpret_cast<float *>(c->block->ptr + (size_t)groups * hsize * 4) + i * n;
                 st = k::split_h2_rows_at(ctx, (const float *)w.ptr(), v, to);
                 if (st) return st;
-                c->key.push_back({w.data.get(), w.data->version});
+                c->key.push_back(StorageKey(w));
             }
             weights = std::move(c);
         }
@@ -1301,7 +1307,7 @@ struct GroupedGemmOp : Operator {
                     st = ctx.check_cuda(cudaMemcpyAsync(lo + i * wsize, src + sp.plane, wsize * 4, cudaMemcpyDeviceToDevice, ctx.stream()), "grouped gemm weights");
                     if (st) return st;
                 }
-                c->key.push_back({w.data.get(), w.data->version});
+                c->key.push_back(StorageKey(w));
             }
             weights = std::move(c);
         }
@@ -1318,7 +1324,7 @@ struct GroupedGemmOp : Operator {
                                         "grouped gemm biases");
                     if (st) return st;
                 }
-                c->key.push_back({b.data.get(), b.data->version});
+                c->key.push_back(StorageKey(b));
             }
             biases = std::move(c);
         }

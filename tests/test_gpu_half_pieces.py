@@ -350,3 +350,17 @@ def test_part_of_a_result_behind_a_reshape(ctx, off):
     assert _close(S.conv_2d(S.view(part(), [2, 20, 20, 64]), ctx.var(f), 1, 1, 1).eval(ctx), _conv64(flat.reshape(2, 20, 20, 64), f, 1, 1))
     assert _close(S.matmul(S.view(part(), [800, 64]), ctx.var(w2)).eval(ctx), flat.reshape(800, 64) @ w2.astype(np.float64))
     assert ctx.status_word() == 0
+
+
+@pytest.mark.parametrize("stride", [1, 2])
+def test_a_filter_that_is_computed_from_a_variable(ctx, stride):
+    """The packed filter of a first convolution follows the variable it is computed from, pass after pass."""
+    rng = np.random.default_rng(87)
+    x, m = rng.uniform(-1, 1, (2, 40, 40, 3)).astype(np.float32), rng.uniform(0.5, 1.5, (32,)).astype(np.float32)
+    f = ctx.var(np.zeros((3, 3, 3, 32), np.float32))
+    y = S.conv_2d(ctx.var(x), f * ctx.var(m), stride, 1, 1)
+    for _ in range(5):
+        values = rng.uniform(-1, 1, (3, 3, 3, 32)).astype(np.float32)
+        ctx.set(f, values)
+        ctx.clear()
+        assert _close(y.eval(ctx), _conv64(x, values * m, stride, 1))
