@@ -4,8 +4,8 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
-
 #include <cstdlib>
+#include <mutex>
 
 #include "kernels.h"
 #include "launch.h"
@@ -280,6 +280,16 @@ typedef CUresult (*PFN_encodeIm2col)(CUtensorMap *, CUtensorMapDataType, cuuint3
                                      const int *, const int *, cuuint32_t, cuuint32_t, const cuuint32_t *, CUtensorMapInterleave,
                                      CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
+// Looked up once, by whichever thread is first.
+static PFN_encodeTiled encode_tiled() {
+    static const PFN_encodeTiled f = reinterpret_cast<PFN_encodeTiled>(driver_symbol("cuTensorMapEncodeTiled"));
+    return f;
+}
+static PFN_encodeIm2col encode_im2col_mode() {
+    static const PFN_encodeIm2col f = reinterpret_cast<PFN_encodeIm2col>(driver_symbol("cuTensorMapEncodeIm2col"));
+    return f;
+}
+
 // dims {k, rows, batch low, batch high, piece}, box {64, box_rows, 1, 1, 1}
 static bool encode_operand(PFN_encodeTiled encode, const H2Operand &op, long long k, unsigned box_rows, CUtensorMap *map) {
     const cuuint64_t row_b = (cuuint64_t)op.ld * 2;
@@ -425,15 +435,25 @@ __global__ void __launch_bounds__(SLICED ? 64 + 2 * BN : kThreads, SLICED && BN 
                                                               const __grid_constant__ CUtensorMap map_b2, const __grid_constant__ H2Params p) {
     gemm_h2_body<BN, CTAS, SLICED>(&map_a, &map_a, &map_b, &map_b2, p);
 }
+// The dynamic shared memory a kernel may be launched with is a setting of the kernel on a device, shared by all threads: raised once,
+// to all there is, never to what one launch needs (a shorter ring asks for less, and could lower it under another thread's launch).
+template <int BN, int CTAS, bool SLICED>
+static cudaError_t allow_shared_memory(int dev) {
+    auto raise = [] {
+        cudaFuncAttributes a;
+        const cudaError_t e = cudaFuncGetAttributes(&a, gemm_h2_kernel<BN, CTAS, SLICED>);
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(gemm_h2_kernel<BN, CTAS, SLICED>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)a.sharedSizeBytes);
+    };
+    static std::once_flag once[64];
+    static cudaError_t result[64];
+    if (dev < 0 || dev >= 64) return raise();
+    std::call_once(once[dev], [&] { result[dev] = raise(); });
+    return result[dev];
+}
 template <int BN, int CTAS, bool SLICED>
 static sage_status launch_plain(Context &ctx, const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtensorMap &map_b2, const H2Params &p, int grid, size_t smem) {
-    static int attr_set[64] = {0};  // per instantiation and device: the largest seen
-    const int dev = ctx.device();
-    if (dev < 0 || dev >= 64 || attr_set[dev] < (int)smem) {
-        sage_status st = ctx.check_cuda(cudaFuncSetAttribute(gemm_h2_kernel<BN, CTAS, SLICED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "gemm_h2 shared memory attribute");
-        if (st) return st;
-        if (dev >= 0 && dev < 64) attr_set[dev] = (int)smem;
-    }
+    const sage_status st = ctx.check_cuda(allow_shared_memory<BN, CTAS, SLICED>(ctx.device()), "gemm_h2 shared memory attribute");
+    if (st) return st;
     return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), SLICED ? p.slices : CTAS, gemm_h2_kernel<BN, CTAS, SLICED>, dim3(grid), dim3(SLICED ? 64 + 2 * BN : kThreads), smem, map_a, map_b, map_b2, p), "gemm_h2 launch");
 }
 
@@ -455,7 +475,7 @@ static int clusters_at_once(const Context &ctx, int s) {
     cfg.dynamicSmemBytes = 200 * 1024;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaFuncSetAttribute(gemm_h2_kernel<128, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024) != cudaSuccess ||
+    if (allow_shared_memory<128, 1, true>(dev) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, gemm_h2_kernel<128, 1, true>, &cfg) != cudaSuccess || n < 1) {
         (void)cudaGetLastError();
         n = ctx.sm_count / s * 9 / 10;
@@ -518,13 +538,9 @@ static SlicePlan plan_slices(const Context &ctx, const H2Gemm &g) {
 }
 
 sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
-    static PFN_encodeTiled encode = nullptr;
-    static PFN_encodeIm2col encode_conv = nullptr;
-    if (!ctx.dry() && !encode) {
-        encode_conv = reinterpret_cast<PFN_encodeIm2col>(driver_symbol("cuTensorMapEncodeIm2col"));
-        encode = reinterpret_cast<PFN_encodeTiled>(driver_symbol("cuTensorMapEncodeTiled"));
-        if (!encode || !encode_conv) return ctx.fail(SAGE_ERR_DEVICE, "cuTensorMapEncode is not available");
-    }
+    const PFN_encodeTiled encode = ctx.dry() ? nullptr : encode_tiled();
+    const PFN_encodeIm2col encode_conv = ctx.dry() ? nullptr : encode_im2col_mode();
+    if (!ctx.dry() && (!encode || !encode_conv)) return ctx.fail(SAGE_ERR_DEVICE, "cuTensorMapEncode is not available");
     if (g.m < 1 || g.n < 1 || g.k < 1 || g.batch < 1 || g.m > 0x7fffffffLL || g.n > 0x7fffffffLL || g.k > 0x7fffffffLL || g.batch > 0x7fffffffLL)
         return ctx.fail(SAGE_ERR_UNSUPPORTED, "gemm_h2: shape not supported");
     if (g.naux < 0 || g.naux > kMaxAux || (!g.c && !g.c_hi && !g.h_hi)) return ctx.fail(SAGE_ERR_INVALID, "gemm_h2: bad epilogue description");
@@ -795,11 +811,8 @@ bool attention_tc_shape_ok(long long lq, long long lk, long long d, long long ba
 }
 
 sage_status attention_tc_run(Context &ctx, const TcAttn &a) {
-    static PFN_encodeTiled encode = nullptr;
-    if (!ctx.dry() && !encode) {
-        encode = reinterpret_cast<PFN_encodeTiled>(driver_symbol("cuTensorMapEncodeTiled"));
-        if (!encode) return ctx.fail(SAGE_ERR_DEVICE, "cuTensorMapEncodeTiled is not available");
-    }
+    const PFN_encodeTiled encode = ctx.dry() ? nullptr : encode_tiled();
+    if (!ctx.dry() && !encode) return ctx.fail(SAGE_ERR_DEVICE, "cuTensorMapEncodeTiled is not available");
     if (!attention_tc_shape_ok(a.lq, a.lk, a.d, a.batch)) return ctx.fail(SAGE_ERR_UNSUPPORTED, "attention_tc: shape not supported");
     if (a.naux < 0 || a.naux > kMaxAux || (!a.o && !a.out.hi && !a.out.h2)) return ctx.fail(SAGE_ERR_INVALID, "attention_tc: bad description");
     AttnParams p{};

@@ -364,3 +364,28 @@ def test_a_filter_that_is_computed_from_a_variable(ctx, stride):
         ctx.set(f, values)
         ctx.clear()
         assert _close(y.eval(ctx), _conv64(x, values * m, stride, 1))
+
+
+def test_products_from_two_threads():
+    """Two contexts on two host threads, each launching the same kernels with rings of its own length in shared memory."""
+    import threading
+    shapes = [[(24, 64, 256), (192, 512, 2048), (24, 128, 512)], [(24, 64, 4096), (192, 512, 320), (40, 96, 8192)]]
+    wrong = []
+
+    def work(mine):
+        c = S.Context(0)
+        try:
+            rng = np.random.default_rng(len(mine))
+            cases = [(rng.standard_normal((1, m, k), dtype=np.float32), rng.standard_normal((1, k, n), dtype=np.float32)) for m, n, k in mine]
+            for _ in range(60):
+                wrong.extend((a.shape, b.shape) for a, b in cases if not excess(product(c, a, b), a, b) <= 1.0)
+        except Exception as e:
+            wrong.append(repr(e))
+        finally:
+            c.close()
+    threads = [threading.Thread(target=work, args=(s,)) for s in shapes]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, wrong[:3]
