@@ -223,7 +223,7 @@ static sage_status gather_h2(Context &ctx, const Tensor &t, bool swapped, const 
     return s;
 }
 
-// Operand A (`rows` = a scale per 64 k) or B (`whole_rows`: one per row, always a compact copy kept beside the storage).
+// Operand A (a scale per row and 64 k) or B (`whole_rows`: one per row and factors, always a compact copy kept beside the storage).
 static sage_status make_h2_operand(Context &ctx, const Tensor &t, bool trans, bool whole_rows, k::H2Operand *op, std::shared_ptr<H2Cache> *hold) {
     const Shape &sh = t.desc.shape;
     const int r = sh.rank(), ka = trans ? r - 2 : r - 1, ma = trans ? r - 1 : r - 2;
@@ -1261,12 +1261,12 @@ struct GroupedGemmOp : Operator {
         ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = false;
         sage_status st = Tensor::uninit(ctx, out, y);
         if (st) return st;
-        const long long wsize = k * n, pitch = (k + 7) / 8 * 8, hsize = n * pitch;
-        // ---- weights in half-precision pieces: [G][N][pitch] hi, the same lo, [G][N] scales
+        const long long wsize = k * n, pitch = (k + 7) / 8 * 8, hsize = n * pitch, factors = (n + 63) / 64 * ((k + 63) / 64);
+        // ---- weights in half-precision pieces: [G][N][pitch] hi, the same lo, [G][N] scales, [G][N / 64][K / 64] factors
         if (h2 && !same_key(weights.get(), x, 1, groups)) {
             std::unique_ptr<Concat> c(new Concat());
             c->alloc = ctx.allocator_ptr();
-            c->block = ctx.allocator().alloc((size_t)groups * hsize * 4 + (size_t)groups * n * 4);
+            c->block = ctx.allocator().alloc((size_t)groups * (hsize + n + factors) * 4);
             if (!c->block) return ctx.fail(SAGE_ERR_OOM, "out of memory for the grouped gemm's weights");
             for (int i = 0; i < groups; ++i) {
                 const Tensor &w = x[1 + i];
@@ -1281,6 +1281,7 @@ struct GroupedGemmOp : Operator {
                 to.plane = groups * hsize;
                 to.pitch = pitch;
                 to.scale = reinterpret_cast<float *>(c->block->ptr + (size_t)groups * hsize * 4) + i * n;
+                to.ratio = reinterpret_cast<float *>(c->block->ptr + (size_t)groups * hsize * 4) + groups * n + i * factors;
                 st = k::split_h2_rows_at(ctx, (const float *)w.ptr(), v, to);
                 if (st) return st;
                 c->key.push_back(StorageKey(w));
@@ -1346,6 +1347,7 @@ struct GroupedGemmOp : Operator {
             g.b.nb0 = groups;
             g.b.sb0 = hsize;
             g.b.scale = reinterpret_cast<const float *>(weights->block->ptr + (size_t)groups * hsize * 4);
+            g.b.ratio = g.b.scale + groups * n;
             g.b.s_row = 1;
             g.b.s_b0 = n;
             g.c = (float *)y->ptr();

@@ -165,41 +165,78 @@ __global__ void __launch_bounds__(256) split_h2_view_kernel(ViewP v, unsigned sh
     store_row(v, b, r0, c0, y, f, hi);
 }
 
-// Operand B: one scale per row.  A cluster of CTAs shares 64 rows, each with a run of their columns; the rows' largest
-// magnitudes are exchanged through distributed shared memory, then the columns are read again, from L2.  Keeping the tiles
+// Operand B: a scale per row, and a factor per 64 rows and 64 columns (of K).  A cluster of CTAs shares 64 rows, each with a run of
+// their columns.  First look: the largest exponent of every tile, and of every row in it; each row's largest relative to the tiles'
+// is then exchanged through distributed shared memory, and the columns are read again, from L2.  Keeping the tiles
 // in shared memory between the two looks (one read, 133 KB a CTA) left one block per SM and was slower: 4096 x 4096 80 us.
-__global__ void __launch_bounds__(256) split_h2_rows_kernel(ViewP v, unsigned short *__restrict__ hi, float *__restrict__ scale, int ctas, int tiles_per_cta) {
+// (Every shuffle and vote below is outside of conditions that differ between a warp's rows.)
+constexpr int kFactors = 64;  // of a CTA: K up to 2^15 has one per 64, beyond it `span` tiles share one
+__global__ void __launch_bounds__(256) split_h2_rows_kernel(ViewP v, unsigned short *__restrict__ hi, float *__restrict__ scale, float *__restrict__ ratio, int ctas,
+                                                            int tiles_per_cta, int span) {
     __shared__ float tiles[2][64][65];
-    __shared__ unsigned amax[64];
+    __shared__ int row_rel[64], cta_top;
+    __shared__ unsigned char row_top[kFactors][64];               // biased exponents of the largest elements, 0 for none
+    __shared__ __align__(8) unsigned char warp_top[kFactors][8];
     grid_dependency_sync();
     const unsigned rank = blockIdx.x % ctas;
     const long long group = blockIdx.x / ctas, b = group / v.row_tiles, r0 = (group % v.row_tiles) * 64;
     const float *s = v.src + (b / v.nb0) * v.sb1 + (b % v.nb0) * v.sb0;
-    const int first = (int)rank * tiles_per_cta, last = min(v.col_tiles, first + tiles_per_cta);
-    unsigned m = 0;
+    const int first = (int)rank * tiles_per_cta, last = min(v.col_tiles, first + tiles_per_cta), row = threadIdx.x >> 2;
+    const bool row_lane = (threadIdx.x & 3) == 0;
+    auto tile_top = [&](int i) -> int {
+        const uint2 w = *reinterpret_cast<const uint2 *>(warp_top[i]);
+        const unsigned m = __vmaxu4(w.x, w.y), n = __vmaxu4(m, m >> 16);
+        return (int)max(n & 0xffu, (n >> 8) & 0xffu);
+    };
     float y[16];
-    for (int t = first; t < last; ++t) {
+    for (int t = first, top = 0; t < last; ++t) {
         fetch_row(v, s, r0, (long long)t * 64, tiles[t & 1], y);
-        m = max(m, row_amax(y));
+        const unsigned g = row_amax(y);
+        top = max(top, g == 0u ? 0 : max((int)(g >> 23), 27));  // (27: 2^-100, as in h2_factor)
+        if ((t - first) % span == span - 1 || t == last - 1) {
+            const int i = (t - first) / span;
+            const int w = __reduce_max_sync(0xffffffffu, top);
+            if ((threadIdx.x & 31) == 0) warp_top[i][threadIdx.x >> 5] = (unsigned char)w;
+            if (row_lane) row_top[i][row] = (unsigned char)top;
+            top = 0;
+        }
     }
-    if ((threadIdx.x & 3) == 0) amax[threadIdx.x >> 2] = m;
+    __syncthreads();
+    int rel = -1000, all = 0;  // this row's largest exponent relative to its tile's; the largest of all
+    for (int i = 0; i * span < last - first; ++i) {
+        const int c = tile_top(i), e = row_top[i][row];
+        rel = e == 0 ? rel : max(rel, e - c);
+        all = max(all, c);
+    }
+    if (row_lane) row_rel[row] = rel;
+    if (threadIdx.x == 0) cta_top = all;
     __syncthreads();
     if (ctas > 1) {
         cluster_sync_all();
-        const unsigned at = smem_u32(&amax[threadIdx.x >> 2]);
+        const unsigned at = smem_u32(&row_rel[row]), top_at = smem_u32(&cta_top);
         for (int q = 0; q < ctas; ++q) {
-            unsigned o;
-            asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(o) : "r"(peer_addr(at, q)) : "memory");
-            m = max(m, o);
+            int o, w;
+            asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(o) : "r"(peer_addr(at, q)) : "memory");
+            asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(w) : "r"(peer_addr(top_at, q)) : "memory");
+            rel = max(rel, o);
+            all = max(all, w);
         }
         cluster_sync_all();  // nobody leaves while a peer may still read its shared memory
     }
-    float sc;
-    const float f = h2_factor(m, &sc);
-    if (rank == 0 && (threadIdx.x & 3) == 0 && r0 + (threadIdx.x >> 2) < v.rows) scale[b * v.rows + r0 + (threadIdx.x >> 2)] = sc;
+    const int se = max(rel + all, 27);  // biased exponent of the row's scale times 2^14
+    if (rank == 0 && row_lane && r0 + row < v.rows) scale[b * v.rows + r0 + row] = __uint_as_float((unsigned)(se - 14) << 23);
     for (int t = last - 1; t >= first; --t) {  // backwards: the last tile is still in registers
         if (t != last - 1) fetch_row(v, s, r0, (long long)t * 64, tiles[t & 1], y);
-        store_row(v, b, r0, (long long)t * 64, y, f, hi);
+        const int c = tile_top((t - first) / span), f = c == 0 ? 0 : max(c - all, -kH2Far);  // 2^f: this tile's factor
+        if (threadIdx.x == 0) ratio[group * v.col_tiles + t] = __uint_as_float((unsigned)(127 + f) << 23);
+        int e = se + f;  // at least this row's largest in this tile
+        if (e < 27) {    // a factor of 2^(14 + 127 - e) would not be finite: two steps, both exact
+            const float up = __uint_as_float((unsigned)(127 + 27 - e) << 23);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) y[i] *= up;
+            e = 27;
+        }
+        store_row(v, b, r0, (long long)t * 64, y, __uint_as_float((unsigned)(268 - e) << 23), hi);
     }
 }
 
@@ -220,10 +257,11 @@ sage_status split_h2_flat(Context &ctx, const float *src, long long n, unsigned 
 static long long h2_pitch(long long cols) { return (cols + 7) / 8 * 8; }
 static size_t up256(size_t b) { return (b + 255) / 256 * 256; }
 
-// [hi][lo][scales]
+// [hi][lo][scales], operand B's [batch][rows] and behind them its factors [batch][row tiles][tiles]
 size_t split_h2_bytes(long long batches, long long rows, long long cols, bool whole_rows) {
     const size_t planes = (size_t)(batches * rows * h2_pitch(cols)) * 2 * 2;
-    return up256(planes) + up256((size_t)(batches * rows * (whole_rows ? 1 : (cols + 63) / 64)) * 4);
+    const long long tiles = (cols + 63) / 64;
+    return up256(planes) + up256((size_t)(batches * (whole_rows ? rows + (rows + 63) / 64 * tiles : rows * tiles)) * 4);
 }
 
 static sage_status split_view_to(Context &ctx, const float *src, const SplitView &v, bool whole_rows, const H2Split &out) {
@@ -238,7 +276,8 @@ static sage_status split_view_to(Context &ctx, const float *src, const SplitView
     int ctas = 1;
     while (ctas < 8 && ctas * 2 <= p.col_tiles) ctas *= 2;
     const int per = (p.col_tiles + ctas - 1) / ctas;
-    return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), ctas, split_h2_rows_kernel, dim3((unsigned)(groups * ctas)), dim3(256), 0, p, out.hi, out.scale, ctas, per),
+    return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), ctas, split_h2_rows_kernel, dim3((unsigned)(groups * ctas)), dim3(256), 0, p, out.hi, out.scale, out.ratio, ctas, per,
+                                           (per + kFactors - 1) / kFactors),
                           "split_h2 rows launch");
 }
 
@@ -249,6 +288,7 @@ sage_status split_h2_view_into(Context &ctx, const float *src, const SplitView &
     out->plane = v.nb0 * v.nb1 * v.rows * out->pitch;
     out->hi = static_cast<unsigned short *>(dst);
     out->scale = reinterpret_cast<float *>(static_cast<char *>(dst) + up256((size_t)out->plane * 4));
+    out->ratio = out->scale + v.nb0 * v.nb1 * v.rows;
     return split_view_to(ctx, src, v, whole_rows, *out);
 }
 
@@ -267,6 +307,7 @@ H2Operand h2_operand(const H2Split &s, long long batches, long long rows, long l
     o.nb0 = batches;
     o.sb0 = rows * s.pitch;
     o.scale = s.scale;
+    o.ratio = s.ratio;
     o.s_row = whole_rows ? 1 : (cols + 63) / 64;
     o.s_b0 = rows * o.s_row;
     return o;
@@ -544,6 +585,7 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
     if (g.m < 1 || g.n < 1 || g.k < 1 || g.batch < 1 || g.m > 0x7fffffffLL || g.n > 0x7fffffffLL || g.k > 0x7fffffffLL || g.batch > 0x7fffffffLL)
         return ctx.fail(SAGE_ERR_UNSUPPORTED, "gemm_h2: shape not supported");
     if (g.naux < 0 || g.naux > kMaxAux || (!g.c && !g.c_hi && !g.h_hi)) return ctx.fail(SAGE_ERR_INVALID, "gemm_h2: bad epilogue description");
+    if (!g.b.ratio || g.b.rows != g.n) return ctx.fail(SAGE_ERR_INVALID, "gemm_h2: operand B is incomplete");
     if (g.conv && (g.batch != 1 || !conv_h2_ok(g) || g.m != g.img_n * g.out_h * g.out_w || g.k != (long long)g.win.ker_h * g.win.ker_w * g.img_c))
         return ctx.fail(SAGE_ERR_INVALID, "gemm_h2: convolution description does not match the GEMM");
     const SlicePlan cut = plan_slices(ctx, g);
@@ -595,6 +637,7 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
     p.sa_b1 = g.a.s_b1;
     p.sb = g.b.scale;
     p.sb_batch = p.b_bcast ? 0 : g.b.s_b0;
+    p.sb_ratio = g.b.ratio;
     p.status = ctx.status_word_dev;
     if (g.conv) {
         p.conv_cb = (int)(g.img_c / HK);

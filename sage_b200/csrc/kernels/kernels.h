@@ -170,7 +170,7 @@ sage_status split_tf32_view(Context &ctx, const float *src, const SplitView &v, 
 // representation).  Both operands are read with K contiguous: `rows` x `k`, rows `ld` elements apart, batch index =
 // b1 * nb0 + b0 at b0 * sb0 + b1 * sb1.  `hi` points at the first hi piece, the lo pieces lie `plane` elements further.
 // Operand A has a scale per row and 64 k (`scale` + b0 * s_b0 + b1 * s_b1 + row * s_row + k / 64), operand B one per row
-// (`scale` + batch * s_b0 + row).  hi must be 16-byte aligned and ld, sb0, sb1, plane multiples of 8.
+// (`scale` + batch * s_b0 + row) and a factor to it per 64 rows and 64 k (`ratio`: [batch][row / 64][k / 64]).  hi must be 16-byte aligned and ld, sb0, sb1, plane multiples of 8.
 struct H2Operand {
     const unsigned short *hi = nullptr;
     long long plane = 0, ld = 0, rows = 0;
@@ -178,6 +178,7 @@ struct H2Operand {
     bool bcast = false;
     const float *scale = nullptr;
     long long s_row = 0, s_b0 = 0, s_b1 = 0;
+    const float *ratio = nullptr;
 };
 struct H2Gemm {
     bool conv = false;        // A is the im2col of a contiguous NHWC image (a.hi, a.plane, a.scale) with C % 64 == 0
@@ -213,11 +214,11 @@ bool conv_h2_ok(const H2Gemm &g);
 // Pieces of `n` consecutive floats (a multiple of 64), laid out like the source, a scale per 64.
 sage_status split_h2_flat(Context &ctx, const float *src, long long n, unsigned short *hi, long long plane, float *scale);
 // Pieces of a strided view (b1, b0, row, col) gathered with its columns contiguous: [batch][rows][pitch], pitch = cols
-// rounded up to 8.  `whole_rows`: one scale per row (operand B) instead of one per 64 columns.
+// rounded up to 8.  `whole_rows`: one scale per row and factors (operand B) instead of one per 64 columns.
 struct H2Split {
     Block *block = nullptr;
     unsigned short *hi = nullptr;
-    float *scale = nullptr;
+    float *scale = nullptr, *ratio = nullptr;
     long long plane = 0, pitch = 0;
 };
 size_t split_h2_bytes(long long batches, long long rows, long long cols, bool whole_rows);

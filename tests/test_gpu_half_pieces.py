@@ -389,3 +389,44 @@ def test_products_from_two_threads():
     for t in threads:
         t.join()
     assert not wrong, wrong[:3]
+
+
+@pytest.mark.parametrize("m,n,k,tb", [(200, 130, 512, False), (200, 130, 520, True), (24, 96, 4096, False), (70, 40, 40000, False)])
+@pytest.mark.parametrize("span,shift", [(30, 0), (50, 0), (80, 0), (90, -80)])
+def test_range_along_the_contraction(ctx, m, n, k, tb, span, shift):
+    """Rows of B scaled by 2^e and columns of A by 2^-e, e running over `span` along K: every term of a sum counts the same, and
+    both operands keep their bits because their scales follow K in steps of 64.  Inside a group e spans span * 64 / k <= 10."""
+    rng = np.random.default_rng(88)
+    e = np.round(np.linspace(-span / 2, span / 2, k)).astype(np.int32)
+    a = np.ldexp(rng.standard_normal((1, m, k)).astype(np.float32), -e[None, None, :] - shift)
+    b = np.ldexp(rng.standard_normal((1, k, n)).astype(np.float32), e[None, :, None] + shift)  # (shift: into the subnormal numbers)
+    got = product(ctx, a, np.ascontiguousarray(np.swapaxes(b, 1, 2)) if tb else b, tb=tb)
+    assert excess(got, a, b) <= 1.0
+    assert ctx.status_word() == 0
+
+
+def test_range_along_the_contraction_inside_a_program(ctx):
+    """The same for products of a program: separate and grouped weights, and a convolution's filter over its channels."""
+    rng = np.random.default_rng(89)
+    e = np.round(np.linspace(-20, 20, 512)).astype(np.int32)
+    a = np.ldexp(rng.standard_normal((150, 512)).astype(np.float32), -e[None, :])
+    w = np.ldexp(rng.standard_normal((512, 128)).astype(np.float32), e[:, None])
+    got = S.matmul(ctx.var(a) * 1.0, ctx.var(w)).eval(ctx)
+    assert excess(got[None], a[None], w[None]) <= 1.0
+    img = np.ldexp(rng.standard_normal((1, 12, 12, 512)).astype(np.float32), -e)
+    f = np.ldexp(rng.standard_normal((3, 3, 512, 64)).astype(np.float32), e[None, None, :, None])
+    got = S.conv_2d(ctx.var(img) * 1.0, ctx.var(f), 1, 1, 1).eval(ctx)
+    assert (np.abs(got - _conv64(img, f, 1, 1)) / _conv64(np.abs(img), np.abs(f), 1, 1)).max() <= 3e-6
+    scale = np.ldexp(np.ones(512, np.float32), -e)
+    x = (rng.standard_normal((1, 64, 512)) * scale).astype(np.float32)
+    ws = [np.ldexp(rng.standard_normal((512, 128)).astype(np.float32) / 16, e[:, None]) for _ in range(3)]
+    X = ctx.var(x)
+    q, k, v = [S.transpose(S.view(S.matmul(X, ctx.var(u)) + ctx.var(np.zeros(128, np.float32)), [1, 64, 2, 64]), 2, 1) for u in ws]
+    y = S.matmul_batched(S.softmax(S.matmul_batched(q, S.transpose(k, -1, -2)) / 64.0, [3]), v)
+    got = y.eval(ctx).astype(np.float64)
+    assert "gemm_grouped" in ctx.describe()
+    q, k, v = [(x.astype(np.float64) @ u).reshape(1, 64, 2, 64).transpose(0, 2, 1, 3) for u in ws]
+    s = q @ k.transpose(0, 1, 3, 2) / 64.0
+    p = np.exp(s - s.max(-1, keepdims=True))
+    want = (p / p.sum(-1, keepdims=True)) @ v
+    assert (np.abs(got - want) / np.maximum(np.abs(want), np.sqrt((want ** 2).mean()))).max() <= 1e-4
