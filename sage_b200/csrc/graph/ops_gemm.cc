@@ -618,12 +618,12 @@ struct GemmOp : Operator {
             ~Held() {
                 if (b) c.allocator().free(b);  // stream-ordered: reused only by launches enqueued after the product
             }
-        } image{ctx, ctx.allocator().alloc((size_t)(piece_bytes + N * 4 + N * 32 * 4))};
+        } image{ctx, ctx.allocator().alloc((size_t)(piece_bytes + (N + 1) / 2 * 8 + N * 64 * 4))};
         if (!image.b) return ctx.fail(SAGE_ERR_OOM, "out of memory for the channel-padded image");
         k::FirstConv f;
         unsigned short *hi = reinterpret_cast<unsigned short *>(image.b->ptr);
         float *scale = reinterpret_cast<float *>(image.b->ptr + piece_bytes);
-        sage_status st = k::pack_first_image(ctx, (const float *)x[0].ptr(), N, H, W, img[3], hp, wp, win.pad_h, win.pad_w, hi, plane, scale, reinterpret_cast<unsigned *>(scale + N));
+        sage_status st = k::pack_first_image(ctx, (const float *)x[0].ptr(), N, H, W, img[3], hp, wp, win.pad_h, win.pad_w, hi, plane, scale, reinterpret_cast<unsigned *>(scale + (N + 1) / 2 * 2));
         if (st) return st;
         const long long chans = (n + 63) / 64 * 64, filter_bytes = chans * win.ker_h * 128;
         if (!packed_filter || !packed_filter->key.holds(x[1])) {
@@ -645,6 +645,14 @@ struct GemmOp : Operator {
         f.kh = win.ker_h;
         f.dil_h = win.dil_h;
         f.stride_h = win.stride_h;
+        f.img_f32 = (const float *)x[0].ptr();
+        f.filter_f32 = (const float *)x[1].ptr();
+        f.img_h = H;
+        f.img_w = W;
+        f.chan = (int)img[3];
+        f.kw = win.ker_w;
+        f.pad_h = win.pad_h;
+        f.pad_w = win.pad_w;
         f.img_scale = scale;
         f.filter_scale = reinterpret_cast<const float *>(packed_filter->block->ptr + filter_bytes);
         k::H2Gemm g;

@@ -400,33 +400,44 @@ sage_status pack_small_c_filter(Context &ctx, const float *filt, int kh, int kw,
 }
 
 // ---- the first convolution on half-precision pieces
-constexpr int kAmaxParts = 32;  // blocks per image that look for its largest magnitude
-__global__ void __launch_bounds__(256) first_amax_kernel(const float *__restrict__ img, long long len, int vec, unsigned *__restrict__ parts) {
-    __shared__ unsigned warps[8];
+constexpr int kAmaxParts = 32;  // blocks per image that look for its largest magnitude, and for its smallest above 0
+// Magnitudes more than 2^29 apart: pieces under one scale would not hold 22 bits of each (`low1`: the smaller's bits less 1).
+__device__ __forceinline__ bool first_wide(unsigned high, unsigned low1) { return high != 0u && (int)(high >> 23) - (int)((low1 + 1u) >> 23) > 29; }
+__global__ void __launch_bounds__(256) first_amax_kernel(const float *__restrict__ img, long long len, int vec, uint2 *__restrict__ parts) {
+    __shared__ uint2 warps[8];
     grid_dependency_sync();
     const float *s = img + blockIdx.y * len;
-    unsigned m = 0;
+    unsigned m = 0, low1 = 0xffffffffu;  // (0 less 1 is the largest: zeros, infinities and nan do not count)
     if (vec) {
         const float4 *v = reinterpret_cast<const float4 *>(s);
 #pragma unroll 4
         for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < len / 4; i += kAmaxParts * 256) {
             const float4 x = __ldg(v + i);
-            m = max(m, max(max(sage_tc::h2_finite_bits(x.x), sage_tc::h2_finite_bits(x.y)), max(sage_tc::h2_finite_bits(x.z), sage_tc::h2_finite_bits(x.w))));
+            const unsigned b0 = sage_tc::h2_finite_bits(x.x), b1 = sage_tc::h2_finite_bits(x.y), b2 = sage_tc::h2_finite_bits(x.z), b3 = sage_tc::h2_finite_bits(x.w);
+            m = max(m, max(max(b0, b1), max(b2, b3)));
+            low1 = min(low1, min(min(b0 - 1u, b1 - 1u), min(b2 - 1u, b3 - 1u)));
         }
     } else {
-        for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < len; i += kAmaxParts * 256) m = max(m, sage_tc::h2_finite_bits(s[i]));
+        for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < len; i += kAmaxParts * 256) {
+            const unsigned b = sage_tc::h2_finite_bits(s[i]);
+            m = max(m, b);
+            low1 = min(low1, b - 1u);
+        }
     }
     m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0) warps[threadIdx.x >> 5] = m;
+    low1 = __reduce_min_sync(0xffffffffu, low1);
+    if ((threadIdx.x & 31) == 0) warps[threadIdx.x >> 5] = make_uint2(m, low1);
     __syncthreads();
     if (threadIdx.x < 32) {
-        m = __reduce_max_sync(0xffffffffu, threadIdx.x < 8 ? warps[threadIdx.x] : 0u);
-        if (threadIdx.x == 0) parts[blockIdx.y * kAmaxParts + blockIdx.x] = m;
+        const uint2 p = threadIdx.x < 8 ? warps[threadIdx.x] : make_uint2(0u, 0xffffffffu);
+        m = __reduce_max_sync(0xffffffffu, p.x);
+        low1 = __reduce_min_sync(0xffffffffu, p.y);
+        if (threadIdx.x == 0) parts[blockIdx.y * kAmaxParts + blockIdx.x] = make_uint2(m, low1);
     }
 }
 // A block takes four rows of the padded image, a thread two neighbouring pixels: 16 bytes of each piece.
 __global__ void __launch_bounds__(128) pack_first_kernel(const float *__restrict__ img, unsigned short *__restrict__ hi, long long plane, long long rows, int h, int w, int c, int hp,
-                                                         int wp, int pad_h, int pad_w, const unsigned *__restrict__ parts, float *__restrict__ scale) {
+                                                         int wp, int pad_h, int pad_w, const uint2 *__restrict__ parts, float *__restrict__ scale) {
     grid_dependency_sync();
     for (int i = 0; i < 4; ++i) {
         const long long r = (long long)blockIdx.x * 4 + i;
@@ -434,8 +445,10 @@ __global__ void __launch_bounds__(128) pack_first_kernel(const float *__restrict
         const long long b = r / hp;
         const int y = (int)(r - b * hp) - pad_h;
         float s;
-        const float f = sage_tc::h2_factor(__reduce_max_sync(0xffffffffu, __ldg(parts + b * kAmaxParts + (threadIdx.x & 31))), &s);
-        if (y == -pad_h && threadIdx.x == 0) scale[b] = s;
+        const uint2 part = __ldg(parts + b * kAmaxParts + (threadIdx.x & 31));
+        const unsigned high = __reduce_max_sync(0xffffffffu, part.x), low1 = __reduce_min_sync(0xffffffffu, part.y);
+        const float f = sage_tc::h2_factor(high, &s);
+        if (y == -pad_h && threadIdx.x == 0) scale[b] = first_wide(high, low1) ? -s : s;
         for (int x2 = threadIdx.x; x2 < wp / 2; x2 += 128) {
             float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             if (y >= 0 && y < h) {
@@ -462,22 +475,28 @@ __global__ void __launch_bounds__(128) pack_first_kernel(const float *__restrict
 }
 // One block per output channel, those that fill up the last 64 included (zeros).
 __global__ void __launch_bounds__(128) pack_first_filter_kernel(const float *__restrict__ f, unsigned short *__restrict__ out, float *__restrict__ scale, int kh, int kw, int c, int oc) {
-    __shared__ unsigned warps[4];
+    __shared__ uint2 warps[4];
     grid_dependency_sync();
     const int o = blockIdx.x;
     auto value = [&](int i) {  // k = ky * 32 + kx * 4 + channel
         const int ky = i >> 5, kx = (i >> 2) & 7, cc = i & 3;
         return (o < oc && kx < kw && cc < c) ? f[(((long long)ky * kw + kx) * c + cc) * oc + o] : 0.f;
     };
-    unsigned m = 0;
-    for (int i = threadIdx.x; i < kh * 32; i += 128) m = max(m, sage_tc::h2_finite_bits(value(i)));
+    unsigned m = 0, low1 = 0xffffffffu;
+    for (int i = threadIdx.x; i < kh * 32; i += 128) {
+        const unsigned b = sage_tc::h2_finite_bits(value(i));
+        m = max(m, b);
+        low1 = min(low1, b - 1u);
+    }
     m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0) warps[threadIdx.x >> 5] = m;
+    low1 = __reduce_min_sync(0xffffffffu, low1);
+    if ((threadIdx.x & 31) == 0) warps[threadIdx.x >> 5] = make_uint2(m, low1);
     __syncthreads();
-    m = max(max(warps[0], warps[1]), max(warps[2], warps[3]));
+    m = max(max(warps[0].x, warps[1].x), max(warps[2].x, warps[3].x));
+    low1 = min(min(warps[0].y, warps[1].y), min(warps[2].y, warps[3].y));
     float s;
     const float factor = sage_tc::h2_factor(m, &s);
-    if (threadIdx.x == 0) scale[o] = s;
+    if (threadIdx.x == 0) scale[o] = first_wide(m, low1) ? -s : s;
     unsigned short *tile = out + (long long)(o >> 6) * kh * 4096;
     for (int i = threadIdx.x * 2; i < kh * 32; i += 256) {
         unsigned a, l;
@@ -489,18 +508,20 @@ __global__ void __launch_bounds__(128) pack_first_filter_kernel(const float *__r
 }
 
 sage_status pack_first_image(Context &ctx, const float *img, long long n, long long h, long long w, long long c, long long hp, long long wp, int pad_h, int pad_w,
-                             unsigned short *hi, long long plane, float *scale, unsigned *parts) {
-    if (c < 1 || c > 4 || wp % 2 || plane % 8 || reinterpret_cast<uintptr_t>(hi) % 16 || h > 0x7fffffffLL || w > 0x7fffffffLL || hp > 0x7fffffffLL || wp > 0x7fffffffLL || n > 65535 ||
+                             unsigned short *hi, long long plane, float *scale, unsigned *scratch) {
+    if (c < 1 || c > 4 || wp % 2 || plane % 8 || reinterpret_cast<uintptr_t>(hi) % 16 || reinterpret_cast<uintptr_t>(scratch) % 8 || h > 0x7fffffffLL || w > 0x7fffffffLL || hp > 0x7fffffffLL ||
+        wp > 0x7fffffffLL || n > 65535 ||
         n * hp / 4 > 0x7ffffff0LL)
         return ctx.fail(SAGE_ERR_INVALID, "pack_first_image: bad arguments");
     ctx.note_launch("pack_small_c");
     ctx.note_launch("pack_small_c");
     if (ctx.dry()) return SAGE_OK;
     const long long len = h * w * c;
+    uint2 *parts = reinterpret_cast<uint2 *>(scratch);
     const int vec = len % 4 == 0 && reinterpret_cast<uintptr_t>(img) % 16 == 0;
     launch_dependent(ctx.pdl, ctx.stream(), first_amax_kernel, dim3(kAmaxParts, (unsigned)n), dim3(256), 0, img, len, vec, parts);
     launch_dependent(ctx.pdl, ctx.stream(), pack_first_kernel, dim3((unsigned)((n * hp + 3) / 4)), dim3(128), 0, img, hi, plane, n * hp, (int)h, (int)w, (int)c, (int)hp, (int)wp, pad_h,
-                     pad_w, (const unsigned *)parts, scale);
+                     pad_w, (const uint2 *)parts, scale);
     return ctx.check_cuda(cudaGetLastError(), "pack_first_image launch");
 }
 

@@ -762,7 +762,7 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
 bool conv_first_ok(int kh, int stride_w, long long out_w) { return stride_w == 2 && kh >= 1 && kh <= 11 && out_w * 10 >= (out_w + 127) / 128 * 128 * 6; }
 
 sage_status conv_first_run(Context &ctx, const H2Gemm &g, const FirstConv &f) {
-    if (!conv_first_ok(f.kh, 2, g.out_w) || g.n < 1 || f.wp % 2 || f.img_plane % 8 || g.naux < 0 || g.naux > kMaxAux || (!g.c && !g.c_hi && !g.h_hi) ||
+    if (!conv_first_ok(f.kh, 2, g.out_w) || g.n < 1 || f.wp % 2 || f.img_plane % 8 || !f.img_f32 || !f.filter_f32 || g.naux < 0 || g.naux > kMaxAux || (!g.c && !g.c_hi && !g.h_hi) ||
         g.img_n * g.out_h * ((g.out_w + 127) / 128) > 0x3fffffffLL || g.img_n * g.out_h * g.out_w > 0x7fffffffLL)
         return ctx.fail(SAGE_ERR_INVALID, "conv_first: bad description");
     FirstParams p{};
@@ -786,6 +786,14 @@ sage_status conv_first_run(Context &ctx, const H2Gemm &g, const FirstConv &f) {
     p.kh = f.kh;
     p.dil_h = f.dil_h;
     p.stride_h = f.stride_h;
+    p.img_f32 = f.img_f32;
+    p.filter_f32 = f.filter_f32;
+    p.img_h = (int)f.img_h;
+    p.img_w = (int)f.img_w;
+    p.chan = f.chan;
+    p.kw = f.kw;
+    p.pad_h = f.pad_h;
+    p.pad_w = f.pad_w;
     p.out_h = (int)g.out_h;
     p.out_w = (int)g.out_w;
     p.segs = (int)((g.out_w + 127) / 128);

@@ -75,7 +75,8 @@ sage_status pack_small_c_image(Context &ctx, const float *img, long long n, long
                                int pad_h, int pad_w, float *hi, long long plane);
 sage_status pack_small_c_filter(Context &ctx, const float *filt, int kh, int kw, int c, int oc, float *hi, long long plane);
 // The first convolution on half-precision pieces (conv_first_device.inc): the image as [n, hp, wp, 4] in pieces with a scale per image
-// (wp even; `parts`: 32 words per image of scratch), the filter as [oc / 64][kh][4][piece][64][8] with a scale per channel.
+// (wp even; `parts`: 64 words per image of scratch, 8-byte aligned), the filter as [oc / 64][kh][4][piece][64][8] with a scale per
+// channel.  A negative scale: its image or channel spans more than one scale holds.
 sage_status pack_first_image(Context &ctx, const float *img, long long n, long long h, long long w, long long c, long long hp, long long wp, int pad_h, int pad_w,
                              unsigned short *hi, long long plane, float *scale, unsigned *parts);
 sage_status pack_first_filter(Context &ctx, const float *filt, int kh, int kw, int c, int oc, unsigned short *out, float *scale);
@@ -202,6 +203,9 @@ struct FirstConv {
     const unsigned short *img = nullptr, *filter = nullptr;
     long long img_plane = 0, hp = 0, wp = 0;
     int kh = 0, dil_h = 1, stride_h = 1;
+    const float *img_f32 = nullptr, *filter_f32 = nullptr;  // what they were made from, contiguous
+    long long img_h = 0, img_w = 0;
+    int chan = 0, kw = 0, pad_h = 0, pad_w = 0;
     const float *img_scale = nullptr, *filter_scale = nullptr;
 };
 bool conv_first_ok(int kh, int stride_w, long long out_w);

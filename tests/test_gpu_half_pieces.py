@@ -430,3 +430,51 @@ def test_range_along_the_contraction_inside_a_program(ctx):
     p = np.exp(s - s.max(-1, keepdims=True))
     want = (p / p.sum(-1, keepdims=True)) @ v
     assert (np.abs(got - want) / np.maximum(np.abs(want), np.sqrt((want ** 2).mean()))).max() <= 1e-4
+
+
+def _excess_conv(got, x, f, stride, pad):
+    """Largest error over the bound: pieces and one chain of 4 KH additions on the tensor cores, or a sum in fp32 over the whole
+    window, with S = the convolution of the magnitudes."""
+    k = f.shape[0] * f.shape[1] * f.shape[2]
+    s = _conv64(np.abs(x), np.abs(f), stride, pad)
+    return float((np.abs(got - _conv64(x, f, stride, pad)) / np.maximum(s * max((k + 2) * 2.0 ** -24, 2.0 ** -22 + 2.0 ** -24 + (4 * f.shape[0] + 2) * 2.0 ** -23), 1e-300)).max())
+
+
+@pytest.mark.parametrize("chan,oc,ker,width", [(3, 64, 7, 224), (3, 72, 7, 224), (4, 64, 3, 180), (1, 32, 8, 160), (2, 128, 5, 315)])
+@pytest.mark.parametrize("what", ["plain", "channels", "filter", "dark", "stray", "special"])
+def test_range_inside_a_first_convolution(monkeypatch, chan, oc, ker, width, what):
+    """Images and filters whose elements are further apart than pieces under one scale hold: channels in different units that the
+    filter makes up for, one output channel's filter over a wide range, an image dark but for a spot, one stray tiny pixel; and
+    infinities, which stay near where they are.  An image without them beside one with them takes the ordinary way."""
+    monkeypatch.setenv("SAGE_VERBOSE_NAMES", "1")
+    rng = np.random.default_rng(90 + chan)
+    pad = ker // 2
+    x = rng.uniform(0.5, 1.0, (3, 30, width, chan)).astype(np.float32) * rng.choice(np.array([-1, 1], np.float32), (3, 30, width, chan))
+    f = rng.standard_normal((ker, ker, chan, oc)).astype(np.float32)
+    if what == "channels":
+        e = np.linspace(-30, 30, chan).astype(np.int32) if chan > 1 else np.zeros(1, np.int32)
+        x[1], f = np.ldexp(x[1], -e), np.ldexp(f, e[:, None])
+    elif what == "filter":
+        f[..., oc // 2] = np.ldexp(f[..., oc // 2], rng.integers(-60, 1, f.shape[:3]))
+        x[:, :, :width // 2] = 0.0
+    elif what == "dark":
+        x[2] = np.ldexp(x[2], -40)
+        x[2, 3:5, 7:9] = 1.0
+    elif what == "stray":
+        x[0, 11, 13, 0] = 1e-30
+    elif what == "special":
+        x[0, 20, 50, 0], x[1, 5, 60, 0] = np.inf, np.nan
+    c = S.Context(0)
+    try:
+        c.trace_begin()
+        got = S.conv_2d(c.var(x), c.var(f), 2, pad, 1).eval(c).astype(np.float64)
+        assert any(n.startswith("conv_first_h2") for n in c.trace()) and c.status_word() == 0
+    finally:
+        c.close()
+    if what == "special":
+        touched = ~np.isfinite(_conv64(np.where(np.isfinite(x), x, np.nan), f, 2, pad))
+        near = np.zeros(got.shape[:3], bool)
+        near[0, 10 - ker:10 + ker, 25 - ker:25 + ker] = near[1, :3 + ker, 30 - ker:30 + ker] = True
+        assert not np.isfinite(got[touched]).any() and np.isfinite(got[~near]).all()
+        return
+    assert _excess_conv(got, x, f, 2, pad) <= 1.0
