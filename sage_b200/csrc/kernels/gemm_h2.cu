@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(256) split_h2_rows_kernel(ViewP v, unsigned sh
 }  // namespace
 
 sage_status split_h2_flat(Context &ctx, const float *src, long long n, unsigned short *hi, long long plane, float *scale) {
-    ctx.note_launch("split_tf32");  // launch lists have one name for an operand's split
+    ctx.note_launch(ctx.verbose_names ? "split_h2" : "split_tf32");  // launch lists have one name for an operand's split
     if (ctx.dry()) return SAGE_OK;
     if (!aligned16(src) || !aligned16(hi) || plane % 8 || n % 64) return ctx.fail(SAGE_ERR_INVALID, "split_h2_flat: unaligned");
     long long blocks = (n / 4 + 255) / 256;
@@ -269,7 +269,7 @@ static sage_status split_view_to(Context &ctx, const float *src, const SplitView
     p.vec = (v.col_stride == 1 || v.ld == 1) && aligned16(src) && v.sb0 % 4 == 0 && v.sb1 % 4 == 0 && (v.col_stride == 1 ? v.ld % 4 == 0 && v.cols % 4 == 0 : v.col_stride % 4 == 0 && v.rows % 4 == 0);
     const long long groups = v.nb0 * v.nb1 * p.row_tiles, blocks = groups * (whole_rows ? 8 : p.col_tiles);
     if (blocks > 0x7fffffffLL) return ctx.fail(SAGE_ERR_UNSUPPORTED, "split_h2: extents beyond 2^31 tiles");
-    ctx.note_launch("split_tf32");  // launch lists have one name for an operand's split
+    ctx.note_launch(ctx.verbose_names ? "split_h2" : "split_tf32");  // launch lists have one name for an operand's split
     if (ctx.dry()) return SAGE_OK;
     if (!whole_rows)
         return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), split_h2_view_kernel, dim3((unsigned)blocks), dim3(256), 0, p, out.hi, out.scale), "split_h2 launch");
@@ -956,7 +956,7 @@ sage_status attention_tc_run(Context &ctx, const TcAttn &a) {
     }
     std::string label;
     if (ctx.verbose_names)
-        label = "attention_tc_h2[" + std::to_string(a.lq) + "x" + std::to_string(a.lk) + "x" + std::to_string(a.d) + "x" + std::to_string(a.batch) + "]";
+        label = "attention_tc_h2[" + std::to_string(a.lq) + "x" + std::to_string(a.lk) + "x" + std::to_string(a.d) + "x" + std::to_string(a.batch) + (by_rows ? ",rows]" : "]");
     const uint32_t gr[3] = {(uint32_t)grid, 1, 1}, bl[3] = {(uint32_t)threads, 1, 1};
     void *params[4] = {&map_q, &map_k, &map_v, &p};
     return ctx.launch(mod, "attention_tc_h2", gr, bl, (uint32_t)smem, params, ctx.verbose_names ? label.c_str() : "attention_tc_3xtf32", true, 1);

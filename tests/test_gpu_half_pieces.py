@@ -6,6 +6,7 @@ within 2^-29 of its group's largest (2 x 2^-23 S), the dropped lo x lo term adds
 at most 12 x 2^-23 S, and the sum of the K / 64 chains in fp32 (K / 64 + 2) x 2^-24 S.
 """
 import ctypes
+import re
 
 import numpy as np
 import pytest
@@ -18,9 +19,23 @@ L = ctypes.c_int64
 
 @pytest.fixture(scope="module")
 def ctx():
-    c = S.Context(0)
+    """A context whose launch list tells the kernels apart (the plain list has one name for every tensor-core product)."""
+    with pytest.MonkeyPatch.context() as m:
+        m.setenv("SAGE_VERBOSE_NAMES", "1")
+        c = S.Context(0)
     yield c
     c.close()
+
+
+def evaluated(ctx, y, pattern, count=1, splits=None):
+    """The value of y, whose evaluation launched at least `count` kernels of names that `pattern` finds, and `splits` passes that
+    only split an operand."""
+    ctx.trace_begin()
+    ctx.eval(y)
+    names = ctx.trace()
+    assert sum(bool(re.search(pattern, n)) for n in names) >= count, (pattern, names)
+    assert splits is None or names.count("split_h2") == splits, names
+    return ctx.read(y)
 
 
 def product(ctx, a, b, ta=False, tb=False):
@@ -28,8 +43,11 @@ def product(ctx, a, b, ta=False, tb=False):
     n_b, m, k = a.shape[0], a.shape[2 if ta else 1], a.shape[1 if ta else 2]
     n = b.shape[1 if tb else 2]
     A, B, C = ctx.tensor(a), ctx.tensor(b), ctx.empty((n_b, m, n))
+    ctx.trace_begin()
     ctx._ck(S.lib.sage_gemm_strided_batched(ctx.h, int(ta), int(tb), L(m), L(n), L(k), A.buf, L(0), L(a.shape[2]), L(m * k), B.buf, L(0), L(b.shape[2]), L(k * n),
                                             C.buf, L(0), L(n), L(m * n), L(n_b)))
+    names = ctx.trace()
+    assert names[:-1] == ["split_h2"] * 2 and names[-1].startswith("gemm_tc_h2["), names
     out = C.numpy()
     for t in (A, B, C):
         t.release()
@@ -104,7 +122,7 @@ def test_infinities_and_nan_stay_in_their_rows(ctx):
     assert ctx.status_word() == 0
 
 
-@pytest.mark.parametrize("m,k,n1,n2", [(129, 96, 64, 70), (300, 130, 192, 64), (2048, 64, 448, 96), (12544, 64, 512, 64), (70, 4096, 128, 33)])
+@pytest.mark.parametrize("m,k,n1,n2", [(129, 128, 64, 70), (300, 192, 192, 64), (2048, 64, 448, 96), (12544, 64, 512, 64), (70, 4096, 128, 33)])
 def test_a_product_hands_pieces_to_the_next(ctx, m, k, n1, n2):
     """The first product's result exists only as pieces (with its epilogue applied, K slices summed where it has them); every
     group of it lands in its place, also where the last column tile is cut off.  Tolerance: 1e-5 of max(|b|, rms), as for the
@@ -113,13 +131,13 @@ def test_a_product_hands_pieces_to_the_next(ctx, m, k, n1, n2):
     x, w1 = rng.uniform(-1, 1, (m, k)).astype(np.float32), rng.uniform(-1, 1, (k, n1)).astype(np.float32)
     b, w2 = rng.uniform(-1, 1, (n1,)).astype(np.float32), rng.uniform(-1, 1, (n1, n2)).astype(np.float32)
     y = S.matmul(S.relu(S.matmul(ctx.var(x) * 1.0, ctx.var(w1)) + ctx.var(b)), ctx.var(w2))
-    got = y.eval(ctx).astype(np.float64)
+    got = evaluated(ctx, y, r"^gemm_tc_h2\[", 2, splits=2).astype(np.float64)  # (the weights)
     want = np.maximum(x.astype(np.float64) @ w1 + b, 0.0) @ w2.astype(np.float64)
     assert (np.abs(got - want) / np.maximum(np.abs(want), np.sqrt((want ** 2).mean()))).max() <= 1e-5
     assert ctx.status_word() == 0
 
 
-@pytest.mark.parametrize("n,h,c,oc,ker,stride", [(3, 9, 64, 64, 3, 1), (2, 17, 64, 192, 3, 2), (1, 7, 512, 128, 3, 1), (5, 8, 128, 64, 1, 2), (1, 56, 64, 64, 3, 1)])
+@pytest.mark.parametrize("n,h,c,oc,ker,stride", [(7, 9, 64, 64, 3, 1), (3, 17, 64, 192, 3, 2), (6, 7, 512, 128, 3, 1), (33, 8, 128, 64, 1, 2), (1, 56, 64, 64, 3, 1)])
 def test_convolutions_on_pieces(ctx, n, h, c, oc, ker, stride):
     """Two convolutions in a row (windows kept in shared memory, gathered, cut into K slices), the second over the first's pieces."""
     rng = np.random.default_rng(h * c)
@@ -133,7 +151,7 @@ def test_convolutions_on_pieces(ctx, n, h, c, oc, ker, stride):
         o = (a.shape[1] - k) // s + 1
         return sum(a[:, i:i + s * o:s, j:j + s * o:s][:, :o, :o] @ f[i, j].astype(np.float64) for i in range(k) for j in range(k))
     y = S.relu(S.conv_2d(ctx.var(x) * 1.0, ctx.var(f1), stride, ker // 2, 1) + ctx.var(b))
-    got = S.conv_2d(y, ctx.var(f2), 1, 1, 1).eval(ctx).astype(np.float64)
+    got = evaluated(ctx, S.conv_2d(y, ctx.var(f2), 1, 1, 1), r"^gemm_tc_h2\[.*,conv", 2, splits=2).astype(np.float64)  # (the filters)
     want = conv(np.maximum(conv(x, f1, stride) + b, 0.0), f2, 1)
     assert got.shape == want.shape
     assert (np.abs(got - want) / np.maximum(np.abs(want), np.sqrt((want ** 2).mean()))).max() <= 1e-5
@@ -143,10 +161,10 @@ def test_convolutions_on_pieces(ctx, n, h, c, oc, ker, stride):
 def test_epilogue_operands_off_the_16_byte_grid(ctx):
     """A result in pieces behind operands that 16-byte loads cannot read (a slice that starts off the grid; an odd row pitch)."""
     rng = np.random.default_rng(81)
-    x, w1 = rng.uniform(-1, 1, (150, 96)).astype(np.float32), rng.uniform(-1, 1, (96, 128)).astype(np.float32)
+    x, w1 = rng.uniform(-1, 1, (150, 64)).astype(np.float32), rng.uniform(-1, 1, (64, 128)).astype(np.float32)
     r, w2 = rng.uniform(-1, 1, (150, 131)).astype(np.float32), rng.uniform(-1, 1, (128, 64)).astype(np.float32)
     y = S.matmul(S.relu(S.matmul(ctx.var(x) * 1.0, ctx.var(w1)) + ctx.var(r).slice(1, 1, 129)), ctx.var(w2))
-    got = y.eval(ctx).astype(np.float64)
+    got = evaluated(ctx, y, r"^gemm_tc_h2\[", 2, splits=2).astype(np.float64)
     want = np.maximum(x.astype(np.float64) @ w1 + r[:, 1:129], 0.0) @ w2.astype(np.float64)
     assert (np.abs(got - want) / np.maximum(np.abs(want), np.sqrt((want ** 2).mean()))).max() <= 1e-5
 
@@ -168,7 +186,7 @@ def test_attention_hands_pieces_to_the_next(ctx, n, length, heads, direct):
         return S.transpose(S.view(t, [n, length, heads, 64]), 2, 1)
     s = S.matmul_batched(split(q), S.transpose(split(k), -1, -2)) / 8.0 + (-(S.view(ctx.var(mask), [n, 1, 1, length])) + 1.0) * -1e5
     y = S.view(S.transpose(S.matmul_batched(S.softmax(s, [3]), split(v)), 2, 1), [n, length, e])
-    got = S.matmul(y, ctx.var(w[3])).eval(ctx).astype(np.float64)
+    got = evaluated(ctx, S.matmul(y, ctx.var(w[3])), r"^(attention|gemm)_tc_h2\[", 3, splits=4 if direct else None).astype(np.float64)
     x64 = x.astype(np.float64)
     q, k, v = [(x64 @ w[i] + (0.0 if direct else x64)).reshape(n, length, heads, 64).transpose(0, 2, 1, 3) for i in range(3)]
     s = q @ k.transpose(0, 1, 3, 2) / 8.0 + (1.0 - mask.astype(np.float64))[:, None, None, :] * -1e5
@@ -178,7 +196,7 @@ def test_attention_hands_pieces_to_the_next(ctx, n, length, heads, direct):
     assert ctx.status_word() == 0
 
 
-@pytest.mark.parametrize("shape,ker,stride,pad,is_max", [((3, 11, 13, 64), 3, 2, 1, True), ((2, 9, 9, 128), 2, 2, 0, False), ((2, 20, 20, 64), 5, 3, 2, True), ((5, 12, 12, 192), 3, 1, 1, False)])
+@pytest.mark.parametrize("shape,ker,stride,pad,is_max", [((13, 11, 13, 64), 3, 2, 1, True), ((17, 9, 9, 128), 2, 2, 0, False), ((11, 20, 20, 64), 5, 3, 2, True), ((5, 12, 12, 192), 3, 1, 1, False)])
 def test_pooling_hands_pieces_to_a_convolution(ctx, shape, ker, stride, pad, is_max):
     """Windows of more and fewer taps than are fetched at a time, cut at the image's edge; the convolution behind reads the
     pool's pieces.  Tolerance as for the other convolutions."""
@@ -189,7 +207,7 @@ def test_pooling_hands_pieces_to_a_convolution(ctx, shape, ker, stride, pad, is_
     p = pool(ctx.var(x) * 1.0, ker, stride, pad, 1)
     alone = p.eval(ctx)
     ctx.clear()
-    got = S.conv_2d(p, ctx.var(f), 1, 1, 1).eval(ctx).astype(np.float64)
+    got = evaluated(ctx, S.conv_2d(p, ctx.var(f), 1, 1, 1), r"^gemm_tc_h2\[.*,conv", splits=1).astype(np.float64)  # (the filter)
 
     def windows(a, k, s, q):
         a = np.pad(a.astype(np.float64), ((0, 0), (q, q), (q, q), (0, 0)))
@@ -214,8 +232,7 @@ def test_attention_with_a_thread_per_row(ctx, n, length, heads, keyed):
     s = S.matmul_batched(ctx.var(q), S.transpose(ctx.var(k), -1, -2)) / 8.0
     if keyed:
         s = s + S.view(ctx.var(bias), [n, 1, 1, length])
-    got = S.matmul_batched(S.softmax(s, [3]), ctx.var(v)).eval(ctx)
-    assert "attention" in ctx.describe()
+    got = evaluated(ctx, S.matmul_batched(S.softmax(s, [3]), ctx.var(v)), r"^attention_tc_h2\[.*,rows")
     for i in range(0, n, max(n // 4, 1)):
         s = q[i].astype(np.float64) @ k[i].astype(np.float64).transpose(0, 2, 1) / 8.0 + (bias[i] if keyed else 0.0)
         p = np.exp(s - s.max(-1, keepdims=True))
@@ -225,11 +242,12 @@ def test_attention_with_a_thread_per_row(ctx, n, length, heads, keyed):
 
 
 @pytest.mark.parametrize("n,heads,length", [(5, 2, 77), (5, 1, 200), (5, 30, 257)])
-def test_attention_over_scores_far_below_zero(n, heads, length):
+def test_attention_over_scores_far_below_zero(monkeypatch, n, heads, length):
     """Every score of a sequence shifted by the same amount, as a mask on the whole sequence does: the quotient is unchanged
     whichever maximum is subtracted, also where the reference's reduce starts at 0 (ref_compat = 1) and exp(x - 0) lies far below
     what half-precision pieces of a weight near 1 hold.  Both forms of the kernel.  Per row, relative to the row's rms: 1e-4, as
     for the other attention blocks.  A row whose every exp(x) is 0 in fp32 is 0 / 0 under ref_compat, as in the reference."""
+    monkeypatch.setenv("SAGE_VERBOSE_NAMES", "1")
     rng = np.random.default_rng(length)
     q, k, v = [rng.uniform(-1, 1, (n, heads, length, 64)).astype(np.float32) for _ in range(3)]
     shift = np.array([-20, -30, -40, -80, -150], np.float32)
@@ -241,8 +259,8 @@ def test_attention_over_scores_far_below_zero(n, heads, length):
         c = S.Context(0, ref_compat=compat)
         try:
             sc = S.matmul_batched(c.var(q), S.transpose(c.var(k), -1, -2)) / 8.0 + S.view(c.var(shift), [n, 1, 1, 1])
-            got = S.matmul_batched(S.softmax(sc, [3]), c.var(v)).eval(c).astype(np.float64)
-            assert "attention" in c.describe() and c.status_word() == 0
+            got = evaluated(c, S.matmul_batched(S.softmax(sc, [3]), c.var(v)), r"^attention_tc_h2\[.*,rows" if heads == 30 else r"^attention_tc_h2\[[0-9x]*\]").astype(np.float64)
+            assert c.status_word() == 0
         finally:
             c.close()
         if compat:
@@ -298,7 +316,7 @@ def test_convolution_of_an_image_off_the_grid_of_groups(ctx, off, tail, ker, str
     f = rng.uniform(-1, 1, (ker, ker, 64, 64)).astype(np.float32)
     v = ctx.var(flat)
     y = S.conv_2d(S.view(v.slice(0, off, off + n), list(shape)), ctx.var(f), stride, ker // 2, 1)
-    assert _close(y.eval(ctx), _conv64(x, f, stride, ker // 2))
+    assert _close(evaluated(ctx, y, r"^gemm_tc_h2\[.*,conv"), _conv64(x, f, stride, ker // 2))
     ctx.set(v, -flat)   # the gathered copy goes with the contents
     ctx.clear()
     assert _close(y.eval(ctx), _conv64(-x, f, stride, ker // 2))
@@ -330,7 +348,7 @@ def test_pooling_of_an_image_off_the_16_byte_grid(ctx, off):
     flat = rng.uniform(-1, 1, (off + n,)).astype(np.float32)
     x, f = flat[off:].reshape(shape), rng.uniform(-1, 1, (3, 3, 64, 64)).astype(np.float32)
     p = S.max_pool_2d(S.view(ctx.var(flat).slice(0, off, off + n), list(shape)), 2, 2, 0, 1)
-    got = S.conv_2d(p, ctx.var(f), 1, 1, 1).eval(ctx)
+    got = evaluated(ctx, S.conv_2d(p, ctx.var(f), 1, 1, 1), r"^gemm_tc_h2\[.*,conv", splits=2 if off % 4 else 1)
     m = np.maximum(x.reshape(4, 15, 2, 15, 2, 64).max((2, 4)), 0)
     assert _close(got, _conv64(m, f, 1, 1))
     assert ctx.status_word() == 0
@@ -347,8 +365,8 @@ def test_part_of_a_result_behind_a_reshape(ctx, off):
     def part():
         return S.view(S.matmul(ctx.var(a) * 1.0, ctx.var(w)), [2 * n]).slice(0, off, off + n)
     flat = (a.astype(np.float64) @ w).ravel()[off:off + n]
-    assert _close(S.conv_2d(S.view(part(), [2, 20, 20, 64]), ctx.var(f), 1, 1, 1).eval(ctx), _conv64(flat.reshape(2, 20, 20, 64), f, 1, 1))
-    assert _close(S.matmul(S.view(part(), [800, 64]), ctx.var(w2)).eval(ctx), flat.reshape(800, 64) @ w2.astype(np.float64))
+    assert _close(evaluated(ctx, S.conv_2d(S.view(part(), [2, 20, 20, 64]), ctx.var(f), 1, 1, 1), r"^gemm_tc_h2\[", 2), _conv64(flat.reshape(2, 20, 20, 64), f, 1, 1))
+    assert _close(evaluated(ctx, S.matmul(S.view(part(), [800, 64]), ctx.var(w2)), r"^gemm_tc_h2\[", 2), flat.reshape(800, 64) @ w2.astype(np.float64))
     assert ctx.status_word() == 0
 
 
@@ -356,20 +374,21 @@ def test_part_of_a_result_behind_a_reshape(ctx, off):
 def test_a_filter_that_is_computed_from_a_variable(ctx, stride):
     """The packed filter of a first convolution follows the variable it is computed from, pass after pass."""
     rng = np.random.default_rng(87)
-    x, m = rng.uniform(-1, 1, (2, 40, 40, 3)).astype(np.float32), rng.uniform(0.5, 1.5, (32,)).astype(np.float32)
+    x, m = rng.uniform(-1, 1, (2, 20, 200, 3)).astype(np.float32), rng.uniform(0.5, 1.5, (32,)).astype(np.float32)
     f = ctx.var(np.zeros((3, 3, 3, 32), np.float32))
     y = S.conv_2d(ctx.var(x), f * ctx.var(m), stride, 1, 1)
     for _ in range(5):
         values = rng.uniform(-1, 1, (3, 3, 3, 32)).astype(np.float32)
         ctx.set(f, values)
         ctx.clear()
-        assert _close(y.eval(ctx), _conv64(x, values * m, stride, 1))
+        assert _close(evaluated(ctx, y, r"^conv_first_h2\[" if stride == 2 else r"^gemm_tc_3xtf32\[.*,conv"), _conv64(x, values * m, stride, 1))
 
 
-def test_products_from_two_threads():
+def test_products_from_two_threads(monkeypatch):
     """Two contexts on two host threads, each launching the same kernels with rings of its own length in shared memory."""
     import threading
-    shapes = [[(24, 64, 256), (192, 512, 2048), (24, 128, 512)], [(24, 64, 4096), (192, 512, 320), (40, 96, 8192)]]
+    monkeypatch.setenv("SAGE_VERBOSE_NAMES", "1")
+    shapes = [[(64, 64, 256), (192, 512, 2048), (70, 128, 512)], [(24, 64, 4096), (192, 512, 320), (40, 96, 8192)]]
     wrong = []
 
     def work(mine):
@@ -411,11 +430,11 @@ def test_range_along_the_contraction_inside_a_program(ctx):
     e = np.round(np.linspace(-20, 20, 512)).astype(np.int32)
     a = np.ldexp(rng.standard_normal((150, 512)).astype(np.float32), -e[None, :])
     w = np.ldexp(rng.standard_normal((512, 128)).astype(np.float32), e[:, None])
-    got = S.matmul(ctx.var(a) * 1.0, ctx.var(w)).eval(ctx)
+    got = evaluated(ctx, S.matmul(ctx.var(a) * 1.0, ctx.var(w)), r"^gemm_tc_h2\[")
     assert excess(got[None], a[None], w[None]) <= 1.0
     img = np.ldexp(rng.standard_normal((1, 12, 12, 512)).astype(np.float32), -e)
     f = np.ldexp(rng.standard_normal((3, 3, 512, 64)).astype(np.float32), e[None, None, :, None])
-    got = S.conv_2d(ctx.var(img) * 1.0, ctx.var(f), 1, 1, 1).eval(ctx)
+    got = evaluated(ctx, S.conv_2d(ctx.var(img) * 1.0, ctx.var(f), 1, 1, 1), r"^gemm_tc_h2\[.*,conv")
     assert (np.abs(got - _conv64(img, f, 1, 1)) / _conv64(np.abs(img), np.abs(f), 1, 1)).max() <= 3e-6
     scale = np.ldexp(np.ones(512, np.float32), -e)
     x = (rng.standard_normal((1, 64, 512)) * scale).astype(np.float32)
@@ -423,8 +442,7 @@ def test_range_along_the_contraction_inside_a_program(ctx):
     X = ctx.var(x)
     q, k, v = [S.transpose(S.view(S.matmul(X, ctx.var(u)) + ctx.var(np.zeros(128, np.float32)), [1, 64, 2, 64]), 2, 1) for u in ws]
     y = S.matmul_batched(S.softmax(S.matmul_batched(q, S.transpose(k, -1, -2)) / 64.0, [3]), v)
-    got = y.eval(ctx).astype(np.float64)
-    assert "gemm_grouped" in ctx.describe()
+    got = evaluated(ctx, y, r"^gemm_tc_h2\[64x128x512x3").astype(np.float64)
     q, k, v = [(x.astype(np.float64) @ u).reshape(1, 64, 2, 64).transpose(0, 2, 1, 3) for u in ws]
     s = q @ k.transpose(0, 1, 3, 2) / 64.0
     p = np.exp(s - s.max(-1, keepdims=True))

@@ -635,19 +635,21 @@ def test_a_product_read_twice_by_one_map(m, n):
     ((1, 21, 516, 1), (11, 3, 1, 40), 3, (2, 0), 1, 1),    # tiles of one row, the tallest filter, half a column tile, an image off the 16-byte grid
     ((2, 40, 200, 2), (3, 5, 2, 68), 2, (1, 2), 3, 0),     # dilated rows
 ])
-def test_first_convolution_on_pieces(shape, filt, stride_h, pad, dil_h, off):
+def test_first_convolution_on_pieces(monkeypatch, shape, filt, stride_h, pad, dil_h, off):
     """Columns two apart and at most four channels: overlapping windows read from whole image rows.  Images of unequal size in
     one batch (a scale each); tolerance as for the other convolutions."""
     rng = np.random.default_rng(sum(shape))
     x = rng.standard_normal(shape).astype(np.float32) * (10.0 ** np.arange(shape[0], dtype=np.float32))[:, None, None, None]
     f = (rng.standard_normal(filt) / np.sqrt(filt[0] * filt[1] * filt[2])).astype(np.float32)
     b = rng.standard_normal(filt[3]).astype(np.float32)
+    monkeypatch.setenv("SAGE_VERBOSE_NAMES", "1")
     ctx = S.Context(0)
     try:
-        big = ctx.var(np.concatenate([np.zeros((off,) + shape[1:], np.float32), x]))
-        X = big.slice(0, off, off + shape[0]) * 1.0 if off else ctx.var(x)
-        y = S.relu(S.conv_2d(X, ctx.var(f), [stride_h, 2], list(pad), [dil_h, 1]) + ctx.var(b)).eval(ctx)
-        ref = np.maximum(conv64(x, f, (stride_h, 2), pad, (dil_h, 1)) + b, 0)
+        X = S.view(ctx.var(np.concatenate([np.zeros(off, np.float32), x.ravel()])).slice(0, off, off + x.size), list(shape)) if off else ctx.var(x)
+        ctx.trace_begin()
+        y = S.relu(S.conv_2d(X, ctx.var(f), [2, stride_h], [pad[1], pad[0]], [1, dil_h]) + ctx.var(b)).eval(ctx)  # pairs run [w, h]
+        assert any(t.startswith("conv_first_h2[") for t in ctx.trace())
+        ref = np.maximum(conv64(x, f, (2, stride_h), (pad[1], pad[0]), (1, dil_h)) + b, 0)
         for i in range(shape[0]):
             assert gemm_err(y[i], ref[i]) <= 1e-5
         assert ctx.status_word() == 0

@@ -14,7 +14,9 @@ pytestmark = pytest.mark.gpu
 
 @pytest.fixture(scope="module")
 def ctx():
-    c = S.Context(0)
+    with pytest.MonkeyPatch.context() as m:
+        m.setenv("SAGE_VERBOSE_NAMES", "1")  # the launch list tells the kernels apart
+        c = S.Context(0)
     yield c
     c.close()
 
@@ -56,7 +58,7 @@ def test_attention_over_short_sequences(ctx, n, heads, l, d):
     ctx.clear()
     ctx.trace_begin()
     got = y.eval(ctx)
-    assert "attention_tc_3xtf32" in ctx.trace()
+    assert any(t.startswith("attention_tc_h2[") for t in ctx.trace())
     q64, k64, v64 = (t.astype(np.float64).reshape(n, l, heads, d).transpose(0, 2, 1, 3) for t in (q, k, v))
     s = q64 @ k64.transpose(0, 1, 3, 2) / np.sqrt(d) + (1.0 - mask)[:, None, None, :] * -1e5
     e = np.exp(s - np.maximum(s.max(-1, keepdims=True), 0.0))
