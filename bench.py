@@ -61,30 +61,7 @@ RESNET18_FLOPS_PER_IMAGE = 2 * 1814073344  # sage's d18 graph at 224 x 224 x 3, 
 # DRAM traffic of the dominant kernel (the tensor-core GEMM) per launch: dram__bytes_read.sum + dram__bytes_write.sum
 # summed by ncu over the GEMM launches of one step of this workload, divided by their number.  A profiler figure
 # cannot be taken inside a timed run; it is re-captured whenever the GEMM path changes.
-GEMM_DRAM_BYTES_PER_LAUNCH = 94.35e6
-
-
-def tf32_library_peak(device):
-    """TF32 GEMM rate of the vendor library on this GPU (torch.matmul, 8192^3, best of 3 bursts of 10):
-    the same method as the bf16 figure of MEASURED_PEAKS.json.  Only a denominator; nothing on the
-    benchmarked path uses it."""
-    import torch
-    torch.backends.cuda.matmul.allow_tf32 = True
-    n = 8192
-    x, y = torch.randn(n, n, device=device), torch.randn(n, n, device=device)
-    for _ in range(3):
-        x @ y
-    torch.cuda.synchronize(device)
-    best = 0.0
-    for _ in range(3):
-        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        e0.record()
-        for _ in range(10):
-            x @ y
-        e1.record()
-        torch.cuda.synchronize(device)
-        best = max(best, 2.0 * n ** 3 * 10 / (e0.elapsed_time(e1) * 1e-3) / 1e12)
-    return best
+GEMM_DRAM_BYTES_PER_LAUNCH = 36.81e6
 
 
 def peaks():
@@ -278,7 +255,6 @@ def sharded_extras(S, ctx, dist, rank, world, local_rank, pk):
     """The batch-sharded workloads with the global batch fixed (strong scaling): BERT-large-shaped, ResNet-18, and,
     on more than one GPU, BERT-base at a global batch of 32."""
     out = {}
-    tf32_burst = pk["bf16"] / 2
     # BERT-large-shaped encoder, b256 x 512 tokens, ragged padding 0..128 per sequence
     rng = np.random.default_rng(4001)
     model = init_bert(S, ctx, LARGE, 4001)
@@ -292,7 +268,7 @@ def sharded_extras(S, ctx, dist, rank, world, local_rank, pk):
         "metric": "seq/s", "value": SHARDED_BATCH / (ms * 1e-3), "ms_per_step": ms, "steps": 3, "global_batch": SHARDED_BATCH,
         "batch_per_gpu": SHARDED_BATCH // world, "scaling": "strong", "gathered_ok": ok, "status_word": st,
         "f32_equivalent_tflops": (dense + attn) / (ms * 1e-3) / 1e12, "tensor_pipe_tflops": 3 * (dense + attn) / (ms * 1e-3) / 1e12,
-        "frac_of_tf32_burst_peak_all_gpus": 3 * (dense + attn) / (ms * 1e-3) / 1e12 / (tf32_burst * world),
+        "frac_of_burst_peak_all_gpus": 3 * (dense + attn) / (ms * 1e-3) / 1e12 / (pk["bf16"] * world),
         "workload": "24 layers, hidden 1024, 16 heads, FFN 4096, seq 512, per-sequence padding 0-128, N(0,0.02) weights"}
     del model
     # ResNet-18, b256 x 224 x 224 x 3
@@ -304,7 +280,7 @@ def sharded_extras(S, ctx, dist, rank, world, local_rank, pk):
         "metric": "img/s", "value": SHARDED_BATCH / (ms * 1e-3), "ms_per_step": ms, "steps": 5, "global_batch": SHARDED_BATCH,
         "batch_per_gpu": SHARDED_BATCH // world, "scaling": "strong", "gathered_ok": ok, "status_word": st,
         "f32_equivalent_tflops": fl / (ms * 1e-3) / 1e12, "tensor_pipe_tflops": 3 * fl / (ms * 1e-3) / 1e12,
-        "frac_of_tf32_burst_peak_all_gpus": 3 * fl / (ms * 1e-3) / 1e12 / (tf32_burst * world),
+        "frac_of_burst_peak_all_gpus": 3 * fl / (ms * 1e-3) / 1e12 / (pk["bf16"] * world),
         "workload": "sage ResNet d18(3, 1000), He-normal filters, input N(0,1) [256,224,224,3] NHWC"}
     del model, x
     if world > 1:  # BERT-base with the global batch held at 32 (32 / N sequences per GPU)
@@ -333,14 +309,13 @@ def single_gpu_extras(S, ctx, pk):
                                "kernels": {k: v[0] for k, v in r["kernels"].items()}, "note": label})
         ctx.clear()
         ctx.drop_programs()
-    tf32_burst, tf32_sust = pk["bf16"] / 2, pk["bf16_sustained"] / 2
     for m, n, k, b in ((1024, 1024, 1024, 1), (4096, 4096, 4096, 1), (8192, 8192, 8192, 1), (512, 512, 64, 16), (512, 64, 512, 16)):
         r = M.case_gemm(ctx, A(m=m, n=n, k=k, batch=b, reps=10 if m < 8192 else 5))
         pipe = r["tensor_pipe_tflops"]
         out["config2"].append({"m": m, "n": n, "k": k, "batch": b, "us": r["us"], "operand_split_us": r["split_us"],
                                "f32_equivalent_tflops": r["tflops_f32_equivalent"], "tensor_pipe_tflops": pipe,
-                               "roofline": {"bound": "tensor", "achieved": pipe, "peak": tf32_burst, "unit": "TFLOP/s", "frac": pipe / tf32_burst,
-                                            "frac_of_sustained": pipe / tf32_sust, "traffic": None},
+                               "roofline": {"bound": "tensor", "achieved": pipe, "peak": pk["bf16"], "unit": "TFLOP/s", "frac": pipe / pk["bf16"],
+                                            "frac_of_sustained": pipe / pk["bf16_sustained"], "traffic": None},
                                "l2": "operands above the 126 MB L2" if (m * k + k * n + m * n) * b * 4 > 126e6 else "operands fit the L2 (no flush between repetitions)"})
     return out
 
@@ -450,13 +425,7 @@ def run_ours(args, rank, local_rank, world, dist):
         extras = sharded_extras(S, ctx, dist, rank, world, local_rank, pk)
         if world == 1:
             extras.update(single_gpu_extras(S, ctx, pk))
-    tf32_live = None
-    if rank == 0:
-        try:
-            tf32_live = tf32_library_peak("cuda:%d" % local_rank)
-        except Exception as e:  # the denominator is optional; the benchmark is not
-            tf32_live = "unavailable: %s" % e
-    return dict(tf32_live=tf32_live, reps=reps, e2e_s=e2e_s, clocks=clocks, launches=launches, prof=prof, gathered_ok=gathered_ok, status=status,
+    return dict(reps=reps, e2e_s=e2e_s, clocks=clocks, launches=launches, prof=prof, gathered_ok=gathered_ok, status=status,
                 mem=mem, extras=extras, pk=pk)
 
 
@@ -505,28 +474,28 @@ def main():
     attn_n = sum(n for name, (n, t) in prof.items() if name.startswith("attention"))
     total_ms = sum(t for n, t in prof.values()) or 1.0
     tc = any(name.startswith("gemm_tc") for name in prof)
-    # The GEMMs run 3xTF32: every logical product is three tensor-core MMAs on the TF32 pipe, whose dense rate is
-    # half the bf16 rate.  achieved = tensor-pipe work (6*M*N*K per GEMM) / summed GEMM launch time; the peak is the
-    # measured bf16 figure / 2 — the burst one when the sampled clocks stayed at the maximum with no power cap (a
+    # A product runs on two half-precision pieces per operand: three f16 MMAs per logical product, at the bf16 rate.
+    # achieved = tensor-pipe work (6*M*N*K per GEMM) / summed GEMM launch time; the peak is the
+    # measured bf16 figure — the burst one when the sampled clocks stayed at the maximum with no power cap (a
     # short timed region), the sustained one otherwise; both fractions are printed.  When the attention block runs as
     # its own fused kernel its products are accounted under "attention", not here.
     gemm_flops = dense_flops + (0 if attn_n else attn_flops)
     f32_eq = (gemm_flops * args.steps / (gemm_ms / 1e3) / 1e12) if gemm_ms else None
-    burst, sustained = pk["bf16"] / 2, pk["bf16_sustained"] / 2
+    burst, sustained = pk["bf16"], pk["bf16_sustained"]
     ck = r["clocks"]
     capped = "sw_power_cap" in (ck.get("reasons") or [])
     at_max = bool(ck.get("sm_mhz") and ck.get("sm_max_mhz") and ck["sm_mhz"] >= 0.95 * ck["sm_max_mhz"])
     regime = "burst" if (at_max and not capped) else "sustained"
     peak = burst if regime == "burst" else sustained
     roofline = {
-        "bound": "tensor", "kernel": "gemm_tcgen05_3xtf32" if tc else "gemm_simt",
+        "bound": "tensor", "kernel": "gemm_tc_h2" if tc else "gemm_simt",
         "achieved": 3 * f32_eq if f32_eq else None, "peak": peak, "unit": "TFLOP/s",
         "frac": (3 * f32_eq / peak) if f32_eq else None, "traffic": GEMM_DRAM_BYTES_PER_LAUNCH,
         "regime": regime, "peak_burst": burst, "peak_sustained": sustained,
         "frac_of_burst": (3 * f32_eq / burst) if f32_eq else None, "frac_of_sustained": (3 * f32_eq / sustained) if f32_eq else None,
-        "peak_source": "%s bf16 dense (MEASURED_PEAKS.json) / 2: the TF32 pipe runs at half the bf16 rate; regime from the sampled clocks "
+        "peak_source": "%s bf16 dense (MEASURED_PEAKS.json): f16 MMAs run at the bf16 rate; regime from the sampled clocks "
                        "(at the maximum SM clock and no power cap = burst)" % pk["source"],
-        "f32_equivalent_tflops": f32_eq, "tf32_library_peak_live": r.get("tf32_live"),
+        "f32_equivalent_tflops": f32_eq,
         "algorithmic_flops_per_step": gemm_flops, "tensor_pipe_flops_per_step": 3 * gemm_flops,
         "launches_per_step": gemm_n / args.steps if args.steps else None,
         "avg_launch_us": 1e3 * gemm_ms / gemm_n if gemm_n else None, "share_of_device_time": gemm_ms / total_ms,
@@ -534,7 +503,7 @@ def main():
         "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum over the tensor-core GEMM launches of one step / their number",
     }
     if attn_n:
-        roofline["attention"] = {"kernel": "attention_tc_3xtf32", "launches_per_step": attn_n / args.steps, "avg_launch_us": 1e3 * attn_ms / attn_n,
+        roofline["attention"] = {"kernel": "attention_tc_h2", "launches_per_step": attn_n / args.steps, "avg_launch_us": 1e3 * attn_ms / attn_n,
                                  "tensor_pipe_tflops": 3 * attn_flops * args.steps / (attn_ms / 1e3) / 1e12, "share_of_device_time": attn_ms / total_ms}
     whole = 3 * (dense_flops + attn_flops) / (ms / args.steps / 1e3) / 1e12
     out = {

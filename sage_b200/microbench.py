@@ -63,24 +63,25 @@ def case_gemm(ctx, a):
     tf = 2.0 * m * n * k * b / (ms * 1e-3) / 1e12
     return {"case": "gemm", "m": m, "n": n, "k": k, "batch": b, "ta": ta, "tb": tb, "us": 1e3 * ms, "split_us": 1e3 * split_ms, "tflops_f32_equivalent": tf,
             "tensor_pipe_tflops": 3 * tf, "peak_bf16_tflops": bf16, "frac_of_bf16_peak": 3 * tf / bf16,
-            "note": "3xTF32: 3 tensor-core MMAs per logical product; TF32 runs at half the bf16 rate, so 1.0 here would be frac 0.5",
+            "note": "three f16 MMAs per logical product, at the bf16 rate",
             "peak_source": src, "kernel": [k_ for k_ in prof if k_.startswith("gemm")][0]}
 
 
 def case_gemm_trace(ctx, a):
-    """Where the cycles of one tensor-core GEMM launch go, counted inside the kernel (SAGE_GEMM_TRACE: the launch runs
+    """Where the cycles of one launch of the tf32-plane GEMM go (the products of training programs; here A^T B, whose
+    contraction axis runs across A's rows), counted inside the kernel (SAGE_GEMM_TRACE: the launch runs
     the instrumented build and the host reads 16 words per CTA; see TcParams::trace).  Cycles become microseconds with
     the launch's own clock: cycles of the longest CTA / its global-timer duration."""
     import struct
     import tempfile
     m, n, k, b = a.m, a.n, a.k, a.batch
-    A = ctx.tensor(np.random.default_rng(0).uniform(-1, 1, (b, m, k)).astype(np.float32))
-    B = ctx.tensor(np.random.default_rng(1).uniform(-1, 1, (b, k, n)).astype(np.float32))
-    C = ctx.empty((b, m, n))
+    A = ctx.var(np.random.default_rng(0).uniform(-1, 1, (b, k, m)).astype(np.float32))
+    B = ctx.var(np.random.default_rng(1).uniform(-1, 1, (b, k, n)).astype(np.float32))
+    y = S.matmul_batched(S.transpose(A, -1, -2), B)
 
     def go():
-        ctx._ck(S.lib.sage_gemm_strided_batched(ctx.h, 0, 0, L(m), L(n), L(k), A.buf, L(0), L(k), L(m * k), B.buf, L(0), L(n), L(k * n),
-                                                C.buf, L(0), L(n), L(m * n), L(b)))
+        ctx.clear()
+        ctx.eval(y)
     for _ in range(3):
         go()
     ctx.sync()
