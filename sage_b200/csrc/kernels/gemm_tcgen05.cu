@@ -438,7 +438,7 @@ static bool pairs_on() {
 // including the sum).
 static int pick_split_k(Context &ctx, const TcGemm &g, int *bn_out) {
     static const bool enabled = !(getenv("SAGE_GEMM_SPLITK") && atoi(getenv("SAGE_GEMM_SPLITK")) == 0);
-    if (!enabled || g.no_split_k || g.conv.on || g.batch != 1 || g.naux != 0 || !g.epilogue.empty() || g.row_softmax || !g.c || g.c_hi || g.ldc != g.n ||
+    if (!enabled || g.conv.on || g.batch != 1 || g.naux != 0 || !g.epilogue.empty() || g.row_softmax || !g.c || g.c_hi || g.ldc != g.n ||
         g.k < 1024)
         return 0;
     const int ctas = (pairs_on() && g.m > BM) ? 2 : 1;
@@ -666,7 +666,7 @@ static sage_status gemm_tc_launch(Context &ctx, const TcGemm &g) {
         const long long num_kb = (g.k + BK - 1) / BK, total = (long long)p.num_tiles * num_kb;
         const double waves = (double)p.num_tiles / (double)slots;
         const bool badly_filled = waves / std::ceil(waves) < 0.92 && p.num_tiles <= 8LL * slots;
-        if (enabled && !ctx.dry() && !g.conv.on && !g.row_softmax && !g.no_split_k && p.rag_narrow == 0 && num_kb >= 8 && total >= 6LL * slots && badly_filled) {
+        if (enabled && !ctx.dry() && !g.conv.on && !g.row_softmax && p.rag_narrow == 0 && num_kb >= 8 && total >= 6LL * slots && badly_filled) {
             const size_t partial_bytes = (size_t)ctx.sm_count * BM * 256 * sizeof(float);  // one 128 x 256 fp32 tile per CTA at most
             const size_t flag_bytes = (size_t)ctx.sm_count * kEpiWarps * sizeof(unsigned);
             if (!ctx.streamk_block) {
