@@ -78,7 +78,14 @@ typedef struct {
                                     (src/ops/reduce.rs:276-285); 0 = true identities */
     int32_t pattern_fusion;      /* 1 (default) = softmax / log_sum_exp / layer_norm / pooling run as
                                     single kernels; 0 = op-by-op like the reference */
-    int32_t gemm_backend;        /* 0 = auto (tcgen05 3xTF32 where shapes allow), 1 = SIMT fp32 only */
+    int32_t gemm_backend;        /* 0 = auto: the tensor cores (tcgen05) where shapes allow, 1 = SIMT fp32 only.
+                                    On the tensor cores an fp32 operand is taken apart into two f16 pieces under
+                                    power-of-two scales (products with k contiguous or gathered: sage_gemm*, conv2d and
+                                    forward graphs) or two tf32 planes (training graphs).  The pieces hold at least 22
+                                    bits of every element within 2^-29 of the largest of its scale's group; smaller ones
+                                    have an absolute error of 2^-51 of that largest.  Groups: 64 consecutive k of a row
+                                    of A; for B, 64 consecutive k of a column where its 64 neighbouring columns agree on
+                                    how the 64-groups compare (a column's scale times a factor per 64 x 64 block). */
 } sage_ctx_opts;
 
 void sage_ctx_opts_default(sage_ctx_opts *opts);

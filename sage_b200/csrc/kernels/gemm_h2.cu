@@ -910,8 +910,11 @@ sage_status attention_tc_run(Context &ctx, const TcAttn &a) {
     if (a.out.h2 && (!vec || a.d != 64 || a.ldo % 64 || a.so0 % 64 || a.so1 % 64 || !aligned16(a.out.h2) || a.out.h2_plane % 8))
         return ctx.fail(SAGE_ERR_INVALID, "attention_tc: a result in half-precision pieces needs whole groups of 64 columns");
     // Q, the K / V ring, 1 KiB per softmax warp for turning the output round, and the slack for 1024-byte alignment
-    // A thread per row where throughput counts: two tiles and more for every SM, more than three blocks of keys each.  With fewer
-    // blocks the way through a single tile is what the next kernel waits for (32 x 128 in a BERT-base pass: 2809 us, 2845 with it).
+    // A thread per row where throughput counts: two tiles and more for every SM, more than three blocks of keys each.  With few
+    // tiles and blocks the way through a single tile is what the next kernel waits for (32 x 128 in a BERT-base pass: 2809 us, 2845
+    // with it).  Both forms, 12 heads, us a launch (a thread a row | four): 4 blocks 32 x 256: 78 | 93; 6 blocks 32 x 384: 141 | 171;
+    // 8 blocks 32 x 512: 230 | 285; 3 blocks 32 x 192: 62 | 74; 2 blocks 32 x 128: 35 | 33, 64 x 128: 58 | 65, 128 x 128: 113 | 126.
+    // The line is on the safe side: with 700 tiles and more the form with a thread a row is ahead at two blocks already.
     const bool by_rows = p.num_tiles >= 2 * ctx.sm_count && a.lk > 3 * kAttnKeys;
     const int threads = by_rows ? kRowThreads : kQuadThreads, slots = by_rows ? 2 * ctx.sm_count : ctx.sm_count, grid = p.num_tiles < slots ? p.num_tiles : slots;
     const size_t smem = 2 * (size_t)kAttnQBytes + (size_t)(by_rows ? kRowStages : kQuadStages) * 4 * kAttnKVBytes + (size_t)(threads - 64) * 32 + 1024;

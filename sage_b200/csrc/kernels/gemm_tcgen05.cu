@@ -433,9 +433,10 @@ static bool pairs_on() {
 // of a (BM x bn) tile costs 1.31 us x (BM + bn / ctas) / (BM + 256 / ctas); a tile has ~7 us of fixed cost;
 // the sum over the slices reads S x m x n floats at ~3 TB/s plus ~10 us of launch and scratch handling.  A split
 // must promise 12 % over the best unsplit choice (the model is only that good).  One case is taken from
-// measurement directly: a large product whose waves of tiles are poorly filled (4096^3: 256 pair tiles on 74
+// measurement directly: a large product whose waves of tiles are poorly filled (4096^3, such as the weight gradient
+// of a 4096 x 4096 layer over 4096 rows: 256 pair tiles on 74
 // SM pairs = 3.46 waves, 86 % of 4) runs in two K slices when that fills them (6.92 of 7: 772 -> 622 us
-// including the sum).
+// including the sum, measured while products through sage_gemm ran on these planes too).
 static int pick_split_k(Context &ctx, const TcGemm &g, int *bn_out) {
     static const bool enabled = !(getenv("SAGE_GEMM_SPLITK") && atoi(getenv("SAGE_GEMM_SPLITK")) == 0);
     if (!enabled || g.conv.on || g.batch != 1 || g.naux != 0 || !g.epilogue.empty() || g.row_softmax || !g.c || g.c_hi || g.ldc != g.n ||
