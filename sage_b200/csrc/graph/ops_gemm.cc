@@ -344,8 +344,8 @@ struct GemmOp : Operator {
         return {g(x[1], gy, true, true), g(gy, x[0], true, true)};
     }
 
-    // Implicit GEMM needs 32-channel K-blocks; images below 128 KiB take the explicit path (im2col-mode
-    // tensor maps over very small tensors are avoided).
+    // On tf32 planes an implicit GEMM needs 32-channel K-blocks; images below 128 KiB take the explicit path (im2col-mode
+    // tensor maps over very small tensors are avoided; on half-precision pieces they are read through boxes, gemm_h2_device.inc).
     // Opt-in: narrow products (at most 128 output channels) read the image as plain fp32 and split it per tile in
     // shared memory.  Wider ones always keep whole-image planes (their kernels have no registers to spare for four more warps).
     bool conv_raw() const { return conv_raw_enabled() && n <= 128; }
@@ -1197,7 +1197,8 @@ std::shared_ptr<Operator> gemm_on_h2(const Operator &op, bool a_given, bool tc_e
         probe.out_h = c->img[4];
         probe.out_w = c->img[5];
         probe.win = c->win;
-        if (!c->conv_implicit() || c->conv_raw() || !k::conv_h2_ok(probe)) return nullptr;
+        probe.conv = true;
+        if ((c->conv_implicit() && c->conv_raw()) || !k::conv_h2_ok(probe)) return nullptr;
     } else if (!h2_view_ok(c->in[0].shape, c->ta) && !a_given) {
         return nullptr;
     }
@@ -1221,7 +1222,7 @@ std::string describe_gemm(const Operator &op) {
     if (!g) return "";
     std::string s;
     if (g->attn) return "{" + (g->epilogue.empty() ? std::string("x0") : g->epilogue) + "}" + (g->folded ? "[store]" : "");
-    if (g->conv) s += g->conv_implicit() ? "<implicit conv>" : g->conv_small_c() ? "<implicit conv, channels padded to 4>" : "<im2col>";
+    if (g->conv) s += g->conv_implicit() || g->h2 ? "<implicit conv>" : g->conv_small_c() ? "<implicit conv, channels padded to 4>" : "<im2col>";
     if (!g->epilogue.empty()) s += "{" + g->epilogue + "}";
     if (g->row_softmax) s += "|softmax";
     if (g->folded) s += "[store]";

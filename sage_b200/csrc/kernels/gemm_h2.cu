@@ -362,6 +362,37 @@ static bool encode_halo(PFN_encodeTiled encode, const H2Gemm &g, const unsigned 
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Images below 128 KiB (of fp32) are read through tiled boxes instead of im2col-mode maps: `rows` whole output rows of one image to
+// a tile, or `imgs` whole images where several fit its 128 pixels.
+struct BoxPlan {
+    int imgs, rows, row_tiles;  // row_tiles: of an image
+    long long tiles(const H2Gemm &g) const { return (g.img_n + imgs - 1) / imgs * row_tiles; }
+};
+static bool box_wanted(const H2Gemm &g) { return g.conv && g.img_n * g.img_h * g.img_w * g.img_c * 4 < 131072; }
+static bool box_plan(const H2Gemm &g, BoxPlan *plan) {
+    if (g.out_w > BM || (g.out_w - 1) * g.win.stride_w + 1 > 256) return false;
+    long long r = BM / g.out_w;
+    if (r > g.out_h) r = g.out_h;
+    const long long in_reach = 255 / g.win.stride_h + 1;  // the box spans (r - 1) * stride + 1 <= 256 image rows
+    if (r > in_reach) r = in_reach;
+    long long imgs = r == g.out_h ? BM / (g.out_w * g.out_h) : 1;
+    if (imgs > g.img_n) imgs = g.img_n;
+    plan->imgs = (int)imgs;
+    plan->rows = (int)r;
+    plan->row_tiles = (int)((g.out_h + r - 1) / r);
+    return true;
+}
+// ... one piece of the image, the pixels of a tile a stride apart
+static bool encode_box(PFN_encodeTiled encode, const H2Gemm &g, const BoxPlan &plan, const unsigned short *base, CUtensorMap *map) {
+    const cuuint64_t dims[4] = {(cuuint64_t)g.img_c, (cuuint64_t)g.img_w, (cuuint64_t)g.img_h, (cuuint64_t)g.img_n};
+    const cuuint64_t strides[3] = {(cuuint64_t)g.img_c * 2, (cuuint64_t)(g.img_w * g.img_c) * 2, (cuuint64_t)(g.img_h * g.img_w * g.img_c) * 2};
+    const Window &w = g.win;
+    const cuuint32_t box[4] = {(cuuint32_t)HK, (cuuint32_t)((g.out_w - 1) * w.stride_w + 1), (cuuint32_t)((plan.rows - 1) * w.stride_h + 1), (cuuint32_t)plan.imgs};
+    const cuuint32_t estr[4] = {1, (cuuint32_t)w.stride_w, (cuuint32_t)w.stride_h, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<unsigned short *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // The limits of im2col-mode tensor maps (as for the tf32 kernel), channels in whole groups.
 bool conv_h2_ok(const H2Gemm &g) {
     const Window &w = g.win;
@@ -369,6 +400,8 @@ bool conv_h2_ok(const H2Gemm &g) {
     if (w.stride_w < 1 || w.stride_w > 8 || w.stride_h < 1 || w.stride_h > 8) return false;
     if (w.pad_w < 0 || w.pad_w > 127 || w.pad_h < 0 || w.pad_h > 127 || w.dil_w < 0 || w.dil_h < 0) return false;
     if (w.pad_w - (w.ker_w - 1) * w.dil_w < -128 || w.pad_h - (w.ker_h - 1) * w.dil_h < -128) return false;
+    BoxPlan plan;
+    if (box_wanted(g) && !box_plan(g, &plan)) return false;
     return (w.ker_w - 1) * w.dil_w <= 255 && (w.ker_h - 1) * w.dil_h <= 255 && g.img_n * g.img_h * g.img_w <= 0x7fffffffLL;
 }
 
@@ -539,13 +572,15 @@ static SlicePlan plan_slices(const Context &ctx, const H2Gemm &g) {
     const SlicePlan none{0, 0};
     const long long all_kb = (g.k + HK - 1) / HK;
     if (!enabled || all_kb < 4) return none;
-    const int ctas = (pairs_on() && g.m > BM) ? 2 : 1;
+    BoxPlan box{};
+    int wb = 0, halo_rows = 0;
+    const bool halo = halo_plan(g, &wb, &halo_rows), boxed = box_wanted(g) && box_plan(g, &box);
+    const int ctas = (pairs_on() && g.m > BM && (halo || !boxed)) ? 2 : 1;
     double best = 1e300, whole = 1e300, store = 3.5;
     for (int i = 0; i < g.naux; ++i)
         if (g.aux[i].sr != 0) store = 8.5;
     SlicePlan plan = none;
-    int wb = 0, halo_rows = 0;
-    if (halo_plan(g, &wb, &halo_rows)) {
+    if (halo) {
         const long long tiles = (g.img_n * ((g.out_h + halo_rows - 1) / halo_rows) + ctas - 1) / ctas, slots = ctx.sm_count / ctas;
         whole = (double)((tiles + slots - 1) / slots) * ((double)all_kb * 0.48 + store + 3.0);
     }
@@ -558,12 +593,12 @@ static SlicePlan plan_slices(const Context &ctx, const H2Gemm &g) {
             const double bytes = (double)busy * (BM + bn / pair) * HK * 4 / 9e6;
             return us > bytes ? us : bytes;
         };
-        if (!wb) {
-            const long long tiles = (g.m + BM * ctas - 1) / (BM * ctas) * cols, slots = ctx.sm_count / ctas, busy = tiles < slots ? tiles : slots;
+        if (!halo) {
+            const long long tiles = (boxed ? box.tiles(g) : (g.m + BM * ctas - 1) / (BM * ctas)) * cols, slots = ctx.sm_count / ctas, busy = tiles < slots ? tiles : slots;
             const double t = (double)((tiles + slots - 1) / slots) * ((double)all_kb * block_us(ctas == 2 ? paired[w] : alone[w], busy * ctas, ctas) + store);
             if (t < whole) whole = t;
         }
-        const long long tiles = (g.m + BM - 1) / BM * cols;
+        const long long tiles = (boxed ? box.tiles(g) : (g.m + BM - 1) / BM) * cols;
         for (int s = 2; s <= 8 && bn < 256; ++s) {
             const long long kb = (all_kb + s - 1) / s;
             if (kb < 2 || kb * (s - 1) >= all_kb || tiles > clusters_at_once(ctx, s)) continue;
@@ -590,10 +625,12 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
         return ctx.fail(SAGE_ERR_INVALID, "gemm_h2: convolution description does not match the GEMM");
     const SlicePlan cut = plan_slices(ctx, g);
     const bool sliced = cut.slices > 1;
-    const int ctas = (pairs_on() && g.m > BM && !sliced) ? 2 : 1;
     int halo_wb = 0, halo_r = 0;
     const bool halo = !sliced && halo_plan(g, &halo_wb, &halo_r);
-    ColumnPlan cols = sliced ? ColumnPlan{cut.bn, 0, 0} : plan_columns(ctx, g.m, g.n, g.batch, ctas);
+    BoxPlan box{};
+    const bool boxed = !halo && box_wanted(g) && box_plan(g, &box);
+    const int ctas = (pairs_on() && g.m > BM && !sliced && !boxed) ? 2 : 1;
+    ColumnPlan cols = sliced ? ColumnPlan{cut.bn, 0, 0} : plan_columns(ctx, boxed ? box.tiles(g) * BM : g.m, g.n, g.batch, ctas);
     if (halo) cols = ColumnPlan{g.n <= 64 ? 64 : 128, 0, 0};  // all output channels in one tile: the window is loaded once
     const int bn = cols.bn;
     const int stage_bytes = halo ? 2 * (bn / ctas) * HK * 2 : 2 * BM * HK * 2 + 2 * (bn / ctas) * HK * 2;
@@ -664,6 +701,14 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
         p.tiles_m = (int)((g.img_n * p.halo_rt + ctas - 1) / ctas);
         p.num_tiles = p.tiles_m * p.tiles_n;
     }
+    if (boxed) {
+        p.box_imgs = box.imgs;
+        p.box_r = box.rows;
+        p.box_rt = box.row_tiles;
+        p.box_bytes = (int)(box.imgs * box.rows * g.out_w) * HK * 2;
+        p.tiles_m = (int)box.tiles(g);
+        p.num_tiles = p.tiles_m * p.tiles_n;
+    }
     const bool vec = g.n % 4 == 0 && g.ldc % 4 == 0 && g.sc0 % 4 == 0 && g.sc1 % 4 == 0 && (!g.c || aligned16(g.c)) && (!g.c_hi || (aligned16(g.c_hi) && g.c_plane % 4 == 0));
     bool aux_vec = true;
     int rowinv = 0, per_col = 0;
@@ -687,7 +732,7 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
 
     const int out_mask = (g.c ? 1 : 0) | (g.c_hi ? 2 : 0) | (g.h_hi ? 4 : 0);
     char num[96];
-    snprintf(num, sizeof num, "gemm_h2 %d %d %d %d %d %d %d %d %d\n", bn, ctas, sliced ? 1 : 0, aux_vec ? 1 : 0, g.conv ? (halo ? 2 : 1) : 0, g.naux, rowinv, per_col, out_mask);
+    snprintf(num, sizeof num, "gemm_h2 %d %d %d %d %d %d %d %d %d\n", bn, ctas, sliced ? 1 : 0, aux_vec ? 1 : 0, g.conv ? (halo ? 2 : boxed ? 3 : 1) : 0, g.naux, rowinv, per_col, out_mask);
     const bool plain = !g.conv && g.naux == 0 && g.epilogue.empty() && out_mask == 1;
     const std::string key = num + g.epilogue;
     Module *mod = plain ? nullptr : ctx.module_find(key);
@@ -699,7 +744,7 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
         define("SAGE_EPI_COLS", per_col);
         define("SAGE_EPI_OUT", out_mask);
         define("SAGE_EPI_NAUX", g.naux);
-        define("SAGE_H2_CONV", g.conv ? 1 : 0);
+        define("SAGE_H2_CONV", g.conv ? (boxed ? 2 : 1) : 0);
         define("SAGE_H2_AUX_VEC", aux_vec ? 1 : 0);
         define("SAGE_H2_HALO", halo ? 1 : 0);
         src += "#define SAGE_EPI_EXPR(x0, x1, x2, x3) (" + (g.epilogue.empty() ? std::string("x0") : g.epilogue) + ")\n";
@@ -730,6 +775,8 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
             if (halo)
                 good = good && encode_halo(encode, g, g.a.hi, (unsigned)halo_wb, (unsigned)(halo_r + g.win.ker_h - 1), &map_a) &&
                        encode_halo(encode, g, g.a.hi + g.a.plane, (unsigned)halo_wb, (unsigned)(halo_r + g.win.ker_h - 1), &map_a2);
+            else if (boxed)
+                good = good && encode_box(encode, g, box, g.a.hi, &map_a) && encode_box(encode, g, box, g.a.hi + g.a.plane, &map_a2);
             else
                 good = good && encode_im2col(encode_conv, g, g.a.hi, &map_a) && encode_im2col(encode_conv, g, g.a.hi + g.a.plane, &map_a2);
         }
@@ -738,7 +785,7 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
     std::string label;
     if (ctx.verbose_names)
         label = "gemm_tc_h2[" + std::to_string(g.m) + "x" + std::to_string(g.n) + "x" + std::to_string(g.k) + (g.batch > 1 ? "x" + std::to_string(g.batch) : "") + (sliced ? ",slices" + std::to_string(cut.slices) : "") +
-                (g.conv ? (halo ? ",conv,taps" : ",conv") : "") + ",bn" + std::to_string(bn) + (cols.narrow ? "/" + std::to_string(cols.wide) + "+" + std::to_string(cols.narrow) + "x192" : "") +
+                (g.conv ? (halo ? ",conv,taps" : boxed ? ",conv,boxes" : ",conv") : "") + ",bn" + std::to_string(bn) + (cols.narrow ? "/" + std::to_string(cols.wide) + "+" + std::to_string(cols.narrow) + "x192" : "") +
                 (ctas == 2 ? ",pair" : "") + "]o" + std::to_string(out_mask);
     if (plain) {
         ctx.note_launch(ctx.verbose_names ? label.c_str() : "gemm_tc_3xtf32");

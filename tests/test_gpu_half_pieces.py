@@ -302,6 +302,31 @@ def _close(got, want, tol=1e-5):
     return (np.abs(got - want) / np.maximum(np.abs(want), np.sqrt((want ** 2).mean()))).max() <= tol
 
 
+# One picture in one tile (cut into K slices); several pictures a tile, the last tile not full; rows of a picture in tiles, the last
+# with fewer; pixels two apart, with and without a window; dilated taps; rows of the longest a tile takes.
+@pytest.mark.parametrize("n,h,w,c,oc,ker,stride,dil", [(1, 7, 7, 512, 512, 3, 1, 1), (17, 2, 2, 512, 128, 3, 1, 1), (20, 5, 5, 64, 64, 3, 2, 1), (30, 4, 4, 64, 200, 1, 1, 1),
+                                                       (1, 16, 16, 64, 320, 3, 1, 1), (1, 20, 23, 64, 192, 3, 1, 1), (2, 15, 11, 64, 256, 1, 2, 1), (1, 12, 12, 192, 160, 3, 1, 2),
+                                                       (1, 3, 128, 64, 136, 3, 1, 1), (70, 2, 2, 64, 64, 1, 2, 1)])
+def test_convolutions_of_images_below_128_kib(ctx, n, h, w, c, oc, ker, stride, dil):
+    """Small images are read through tiled boxes: bias and relu behind, the result handed to a second convolution.  Tolerance as for
+    the other convolutions."""
+    rng = np.random.default_rng(h * w + c)
+    x, f = rng.uniform(-1, 1, (n, h, w, c)).astype(np.float32), rng.uniform(-1, 1, (ker, ker, c, oc)).astype(np.float32)
+    b = rng.uniform(-1, 1, (oc,)).astype(np.float32)
+    wide = np.zeros((dil * (ker - 1) + 1,) * 2 + f.shape[2:], np.float32)
+    wide[::dil, ::dil] = f
+    pad = dil * (ker // 2)
+    y = S.relu(S.conv_2d(ctx.var(x) * 1.0, ctx.var(f), stride, pad, dil) + ctx.var(b))
+    want = np.maximum(_conv64(x, wide, stride, pad) + b, 0.0)
+    assert _close(evaluated(ctx, y, r"^gemm_tc_h2\[.*,conv"), want)
+    assert "im2col" not in " ".join(ctx.trace())
+    if oc % 64 == 0:
+        ctx.clear()
+        f2 = rng.uniform(-1, 1, (3, 3, oc, 64)).astype(np.float32)
+        assert _close(evaluated(ctx, S.conv_2d(y, ctx.var(f2), 1, 1, 1), r"^gemm_tc_h2\[.*,conv", 2, splits=1), _conv64(want, f2, 1, 1))
+    assert ctx.status_word() == 0
+
+
 @pytest.mark.parametrize("off", [0, 1, 4, 32, 64])
 @pytest.mark.parametrize("tail", [0, 5])
 @pytest.mark.parametrize("ker,stride", [(3, 1), (1, 2)])
