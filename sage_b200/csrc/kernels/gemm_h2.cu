@@ -64,10 +64,28 @@ struct ViewP {
     int vec;  // whole 16-byte loads along the contiguous axis are aligned and inside
 };
 
+// Single elements of a 64 x 64 tile, four lines of 64 at a time along whichever axis is contiguous.
+__device__ __forceinline__ bool along_columns(const ViewP &v) { return v.cs == 1 || v.ld != 1; }
+__device__ __forceinline__ void load_singles(const ViewP &v, const float *s, long long r0, long long c0, float (&x)[16]) {
+    const int fast = threadIdx.x & 63, slow = threadIdx.x >> 6;
+    const bool columns = along_columns(v);
+    const long long r = r0 + (columns ? slow : fast), c = c0 + (columns ? fast : slow), step = columns ? 4 * v.ld : 4 * v.cs;
+    const int left = (int)min(columns ? v.rows - r : v.cols - c, 64LL);
+    const float *at = s + r * v.ld + c * v.cs;
+    const bool in = columns ? c < v.cols : r < v.rows;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) x[i] = in && 4 * i < left ? at[i * step] : 0.f;
+}
+__device__ __forceinline__ void store_singles(const ViewP &v, const float (&x)[16], float (*tile)[65]) {
+    const int fast = threadIdx.x & 63, slow = threadIdx.x >> 6;
+    float *at = along_columns(v) ? &tile[slow][fast] : &tile[fast][slow];
+    const int step = along_columns(v) ? 4 * 65 : 4;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) at[i * step] = x[i];
+}
 // A 64 x 64 tile of the view into shared memory, read along whichever axis is contiguous (256 threads).
 __device__ __forceinline__ void load_tile(const ViewP &v, const float *s, long long r0, long long c0, float (*tile)[65]) {
-    const int t = threadIdx.x, fast = t & 63, slow = t >> 6;  // 4 lines of 64 at a time
-    float x[16];
+    const int t = threadIdx.x;
     if (v.vec && v.cs != 1) {
         const int r4 = (t & 15) * 4, line = t >> 4;
         float4 q[4];
@@ -84,22 +102,10 @@ __device__ __forceinline__ void load_tile(const ViewP &v, const float *s, long l
             tile[r4 + 2][c] = q[i].z;
             tile[r4 + 3][c] = q[i].w;
         }
-    } else if (v.cs == 1 || v.ld != 1) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const long long r = r0 + slow + 4 * i, c = c0 + fast;
-            x[i] = r < v.rows && c < v.cols ? s[r * v.ld + c * v.cs] : 0.f;
-        }
-#pragma unroll
-        for (int i = 0; i < 16; ++i) tile[slow + 4 * i][fast] = x[i];
     } else {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const long long r = r0 + fast, c = c0 + slow + 4 * i;
-            x[i] = r < v.rows && c < v.cols ? s[r + c * v.cs] : 0.f;
-        }
-#pragma unroll
-        for (int i = 0; i < 16; ++i) tile[fast][slow + 4 * i] = x[i];
+        float x[16];
+        load_singles(v, s, r0, c0, x);
+        store_singles(v, x, tile);
     }
 }
 // A row of the tile per 4 lanes, columns 8 * part .. and 32 + 8 * part .. each: no bank conflicts, and the four lanes' 16-byte
@@ -109,134 +115,358 @@ __device__ __forceinline__ void tile_row(const float (*tile)[65], float (&y)[16]
 #pragma unroll
     for (int i = 0; i < 16; ++i) y[i] = t[(i & 7) + (i & 8) * 4];
 }
-// This thread's 16 values of the tile at (r0, c0): straight from memory where the columns are contiguous and aligned,
-// else turned round in shared memory (a barrier inside: all threads call it).
-__device__ __forceinline__ void fetch_row(const ViewP &v, const float *s, long long r0, long long c0, float (*tile)[65], float (&y)[16]) {
-    if (v.vec && v.cs == 1) {
-        const long long r = r0 + (threadIdx.x >> 2), c = c0 + (threadIdx.x & 3) * 8;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const long long cc = c + (i & 1) * 4 + (i >> 1) * 32;
-            const float4 q = r < v.rows && cc < v.cols ? *reinterpret_cast<const float4 *>(s + r * v.ld + cc) : make_float4(0.f, 0.f, 0.f, 0.f);
-            y[4 * i] = q.x;
-            y[4 * i + 1] = q.y;
-            y[4 * i + 2] = q.z;
-            y[4 * i + 3] = q.w;
-        }
-        return;
-    }
-    load_tile(v, s, r0, c0, tile);
-    __syncthreads();
-    tile_row(tile, y);
-}
 __device__ __forceinline__ unsigned row_amax(const float (&y)[16]) {
-    unsigned m = 0;
+    float m = 0.f;  // (fmaxf passes over nan)
 #pragma unroll
-    for (int i = 0; i < 16; ++i) m = max(m, h2_finite_bits(y[i]));
-    m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
-    return max(m, __shfl_xor_sync(0xffffffffu, m, 2));
+    for (int i = 0; i < 16; ++i) m = fmaxf(m, fabsf(y[i]));
+    unsigned b = __float_as_uint(m);
+    if (b >= 0x7f800000u) {
+        b = 0u;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) b = max(b, h2_finite_bits(y[i]));
+    }
+    b = max(b, __shfl_xor_sync(0xffffffffu, b, 1));
+    return max(b, __shfl_xor_sync(0xffffffffu, b, 2));
 }
-__device__ __forceinline__ void store_row(const ViewP &v, long long b, long long r0, long long c0, const float (&y)[16], float factor, unsigned short *hi) {
-    const long long r = r0 + (threadIdx.x >> 2), c = c0 + (threadIdx.x & 3) * 8;
-    if (r >= v.rows) return;
+// ... split and stored at `d`, `left` before the row's end in memory (whole 16-byte pieces, zeros behind the last column).
+__device__ __forceinline__ void store_row(const float (&y)[16], float factor, unsigned short *d, long long plane, int left) {
     unsigned h[8], l[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) h2_split2(y[2 * i], y[2 * i + 1], factor, &h[i], &l[i]);
-    unsigned short *d = hi + (b * v.rows + r) * v.pitch + c;
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {  // pitch is a multiple of 8: whole 16-byte pieces, zeros behind the last column
-        if (c + 32 * i >= v.pitch) break;
+    for (int i = 0; i < 2; ++i) {
+        if (32 * i >= left) break;
         *reinterpret_cast<uint4 *>(d + 32 * i) = make_uint4(h[4 * i], h[4 * i + 1], h[4 * i + 2], h[4 * i + 3]);
-        *reinterpret_cast<uint4 *>(d + v.plane + 32 * i) = make_uint4(l[4 * i], l[4 * i + 1], l[4 * i + 2], l[4 * i + 3]);
+        *reinterpret_cast<uint4 *>(d + plane + 32 * i) = make_uint4(l[4 * i], l[4 * i + 1], l[4 * i + 2], l[4 * i + 3]);
     }
 }
 
-// Operand A: a scale per row and 64 columns.  One block per tile.
-__global__ void __launch_bounds__(256) split_h2_view_kernel(ViewP v, unsigned short *__restrict__ hi, float *__restrict__ scale) {
-    __shared__ float tile[64][65];
-    grid_dependency_sync();
-    const int per = v.row_tiles * v.col_tiles, rem = (int)(blockIdx.x % per);
-    const long long b = blockIdx.x / per, r0 = (long long)(rem / v.col_tiles) * 64, c0 = (long long)(rem % v.col_tiles) * 64;
-    float y[16], s;
-    fetch_row(v, v.src + (b / v.nb0) * v.sb1 + (b % v.nb0) * v.sb0, r0, c0, tile, y);
-    const float f = h2_factor(row_amax(y), &s);
-    const long long r = r0 + (threadIdx.x >> 2);
-    if ((threadIdx.x & 3) == 0 && r < v.rows) scale[(b * v.rows + r) * v.col_tiles + (c0 >> 6)] = s;
-    store_row(v, b, r0, c0, y, f, hi);
+// Where an operand's pieces go.
+struct SplitOut {
+    unsigned short *hi;
+    float *scale, *ratio;
+};
+
+// A thread's four 16-byte loads of a tile: of one row (its columns contiguous; as tile_row has them), or of four rows and two pairs
+// of columns.  `at`: its first one, null for rows outside; `left`: columns from there to the view's end.
+template <bool FOUR_ROWS>
+__device__ __forceinline__ void load_quads(const float *at, long long cs, int left, float4 (&q)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int step = (FOUR_ROWS ? (i & 1) : (i & 1) * 4) + (i >> 1) * 32;
+        q[i] = at && step < left ? *reinterpret_cast<const float4 *>(at + (FOUR_ROWS ? step * cs : step)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+__device__ __forceinline__ void quads_row(const float4 (&q)[4], float (&y)[16]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        y[4 * i] = q[i].x;
+        y[4 * i + 1] = q[i].y;
+        y[4 * i + 2] = q[i].z;
+        y[4 * i + 3] = q[i].w;
+    }
+}
+__device__ __forceinline__ const float *batch_of(const ViewP &v, unsigned b) {
+    return b == 0 ? v.src : v.src + (b / (unsigned)v.nb0) * v.sb1 + (b % (unsigned)v.nb0) * v.sb0;
+}
+
+// Operand A: a scale per row and 64 columns.  A block takes `run` tiles side by side, the next one's rows on their way.
+__device__ __forceinline__ void split_tiles(const ViewP &v, const SplitOut &o, unsigned block, int run, float (*tile)[65]) {
+    const unsigned runs = (unsigned)(v.col_tiles + run - 1) / run, line = block / runs, b = line / (unsigned)v.row_tiles;
+    const int first = (int)(block - line * runs) * run, last = min(v.col_tiles, first + run);
+    const long long r0 = (long long)(line - b * v.row_tiles) * 64, r = r0 + (threadIdx.x >> 2), at_row = b * v.rows + r;
+    const float *s = batch_of(v, b);
+    const bool straight = v.vec && v.cs == 1, in = r < v.rows;
+    const int c = (threadIdx.x & 3) * 8;
+    const float *at = straight && in ? s + r * v.ld + c : nullptr;
+    float4 q[4];
+    if (straight) load_quads<false>(at ? at + first * 64 : nullptr, 1, (int)v.cols - c - first * 64, q);
+    for (int t = first; t < last; ++t) {
+        float y[16], scale;
+        if (straight) {
+            quads_row(q, y);
+            if (t + 1 < last) load_quads<false>(at ? at + (t + 1) * 64 : nullptr, 1, (int)v.cols - c - (t + 1) * 64, q);
+        } else {
+            if (t != first) __syncthreads();
+            load_tile(v, s, r0, (long long)t * 64, tile);
+            __syncthreads();
+            tile_row(tile, y);
+        }
+        const float f = h2_factor(row_amax(y), &scale);
+        if (!in) continue;
+        if ((threadIdx.x & 3) == 0) o.scale[at_row * v.col_tiles + t] = scale;
+        store_row(y, f, o.hi + at_row * v.pitch + t * 64 + c, v.plane, (int)v.pitch - t * 64 - c);
+    }
 }
 
 // Operand B: a scale per row, and a factor per 64 rows and 64 columns (of K).  A cluster of CTAs shares 64 rows, each with a run of
 // their columns.  First look: the largest exponent of every tile, and of every row in it; each row's largest relative to the tiles'
-// is then exchanged through distributed shared memory, and the columns are read again, from L2.  Keeping the tiles
-// in shared memory between the two looks (one read, 133 KB a CTA) left one block per SM and was slower: 4096 x 4096 80 us.
+// is then exchanged through distributed shared memory, and the columns are read again, from L2.
+// The tile after the present one is on its way in both looks.  With whole 16-byte loads the first look needs neither a transposition
+// nor a barrier a tile, and rows that lie across are split before they are turned round, as pairs.
+// Keeping the tiles in shared memory between the two looks (one read, 133 KB a CTA) left one block per SM: 4096 x 4096 80 us.
 // (Every shuffle and vote below is outside of conditions that differ between a warp's rows.)
 constexpr int kFactors = 64;  // of a CTA: K up to 2^15 has one per 64, beyond it `span` tiles share one
-__global__ void __launch_bounds__(256) split_h2_rows_kernel(ViewP v, unsigned short *__restrict__ hi, float *__restrict__ scale, float *__restrict__ ratio, int ctas,
-                                                            int tiles_per_cta, int span) {
-    __shared__ float tiles[2][64][65];
-    __shared__ int row_rel[64], cta_top;
-    __shared__ unsigned char row_top[kFactors][64];               // biased exponents of the largest elements, 0 for none
-    __shared__ __align__(8) unsigned char warp_top[kFactors][8];
-    grid_dependency_sync();
-    const unsigned rank = blockIdx.x % ctas;
-    const long long group = blockIdx.x / ctas, b = group / v.row_tiles, r0 = (group % v.row_tiles) * 64;
-    const float *s = v.src + (b / v.nb0) * v.sb1 + (b % v.nb0) * v.sb0;
-    const int first = (int)rank * tiles_per_cta, last = min(v.col_tiles, first + tiles_per_cta), row = threadIdx.x >> 2;
-    const bool row_lane = (threadIdx.x & 3) == 0;
-    auto tile_top = [&](int i) -> int {
-        const uint2 w = *reinterpret_cast<const uint2 *>(warp_top[i]);
-        const unsigned m = __vmaxu4(w.x, w.y), n = __vmaxu4(m, m >> 16);
-        return (int)max(n & 0xffu, (n >> 8) & 0xffu);
+struct RowsShared {
+    union {
+        float tiles[2][64][65];
+        uint4 pieces[2][2][64][8];             // [buffer][hi, lo][row]: 16-byte chunks, a row's swizzled by piece_swizzle
+        unsigned warp_words[kFactors][8][16];  // first look, four rows to a thread: their exponents, a warp's
     };
-    float y[16];
-    for (int t = first, top = 0; t < last; ++t) {
-        fetch_row(v, s, r0, (long long)t * 64, tiles[t & 1], y);
-        const unsigned g = row_amax(y);
-        top = max(top, g == 0u ? 0 : max((int)(g >> 23), 27));  // (27: 2^-100, as in h2_factor)
-        if ((t - first) % span == span - 1 || t == last - 1) {
-            const int i = (t - first) / span;
-            const int w = __reduce_max_sync(0xffffffffu, top);
-            if ((threadIdx.x & 31) == 0) warp_top[i][threadIdx.x >> 5] = (unsigned char)w;
-            if (row_lane) row_top[i][row] = (unsigned char)top;
-            top = 0;
+    int row_rel[64], cta_top;
+    __align__(16) int row_scale[64];                    // biased exponent of a row's scale times 2^14
+    __align__(16) unsigned char row_top[kFactors][64];  // biased exponents of the largest elements, 0 for none
+    unsigned char tile_top[kFactors];
+};
+// Writers: sixteen rows four apart, the same chunk; readers: two neighbouring rows, four chunks each.
+__device__ __forceinline__ int piece_swizzle(int row) { return ((row >> 2) ^ (row << 2)) & 7; }
+// Biased exponent of a magnitude that fmaxf found (it passes over nan), 0 for none (27: 2^-100, as in h2_factor), 255 for inf.
+__device__ __forceinline__ unsigned h2_exponent(float m) {
+    const unsigned b = __float_as_uint(m);
+    return b == 0u ? 0u : max(b >> 23, 27u);
+}
+__device__ __forceinline__ float largest4(float a, float b, float c, float d) { return fmaxf(fmaxf(fabsf(a), fabsf(b)), fmaxf(fabsf(c), fabsf(d))); }
+__device__ __forceinline__ float largest_finite4(float a, float b, float c, float d) {
+    return __uint_as_float(max(max(h2_finite_bits(a), h2_finite_bits(b)), max(h2_finite_bits(c), h2_finite_bits(d))));
+}
+__device__ __forceinline__ bool is_finite(float m) { return m < __uint_as_float(0x7f800000u); }
+
+enum { kRowsAny, kRowsOne, kRowsFour };  // a thread's loads: single elements; 16 bytes of one row; 16 bytes of four rows
+template <int LOADS>
+__device__ __forceinline__ void split_rows(const ViewP &v, const SplitOut &o, unsigned block, int ctas, int tiles_per_cta, int span, RowsShared &sh) {
+    const unsigned group = block / (unsigned)ctas, rank = block - group * ctas, b = group / (unsigned)v.row_tiles;
+    const long long r0 = (long long)(group - b * v.row_tiles) * 64;
+    const float *s = batch_of(v, b);
+    const int first = (int)rank * tiles_per_cta, last = min(v.col_tiles, first + tiles_per_cta), row = threadIdx.x >> 2;
+    const int factors = first < last ? (last - first + span - 1) / span : 0;
+    const bool row_lane = (threadIdx.x & 3) == 0, row_in = r0 + row < v.rows;
+    constexpr bool four = LOADS == kRowsFour, any = LOADS == kRowsAny;
+    const int r4 = (threadIdx.x & 15) * 4, line = threadIdx.x >> 4;  // four: this thread's rows, and half its first column
+    const int c = four ? line * 2 : (threadIdx.x & 3) * 8, cols = (int)v.cols;
+    const float *at = nullptr;
+    if (!any) {
+        const long long r = r0 + (four ? r4 : row);
+        if (r < v.rows) at = s + (four ? r + c * v.cs : r * v.ld + c);
+    }
+    float4 q[4], next[4];
+    float x[16];  // single elements, as they are loaded
+    auto load = [&](int t, float4 (&to)[4]) {
+        if constexpr (any) load_singles(v, s, r0, (long long)t * 64, x);
+        else load_quads<four>(at ? at + (four ? t * 64 * v.cs : (long long)t * 64) : nullptr, v.cs, cols - c - t * 64, to);
+    };
+    // ---- first look
+    load(first, q);
+    float m[4] = {0.f, 0.f, 0.f, 0.f};  // four rows' largest, or one's
+    for (int t = first, left = span, i = 0; t < last; ++t) {
+        float y[16];
+        if constexpr (any) {
+            store_singles(v, x, sh.tiles[t & 1]);
+            if (t + 1 < last) load(t + 1, next);
+            __syncthreads();
+            tile_row(sh.tiles[t & 1], y);
+        } else if (t + 1 < last) {
+            load(t + 1, next);
+        }
+        if constexpr (four) {
+            float n[4] = {largest4(q[0].x, q[1].x, q[2].x, q[3].x), largest4(q[0].y, q[1].y, q[2].y, q[3].y), largest4(q[0].z, q[1].z, q[2].z, q[3].z),
+                          largest4(q[0].w, q[1].w, q[2].w, q[3].w)};
+            if (!is_finite(largest4(n[0], n[1], n[2], n[3]))) {
+                n[0] = largest_finite4(q[0].x, q[1].x, q[2].x, q[3].x);
+                n[1] = largest_finite4(q[0].y, q[1].y, q[2].y, q[3].y);
+                n[2] = largest_finite4(q[0].z, q[1].z, q[2].z, q[3].z);
+                n[3] = largest_finite4(q[0].w, q[1].w, q[2].w, q[3].w);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) m[j] = fmaxf(m[j], n[j]);
+        } else {
+            if constexpr (!any) quads_row(q, y);
+            float n = 0.f;
+#pragma unroll
+            for (int k = 0; k < 16; k += 4) n = fmaxf(n, largest4(y[k], y[k + 1], y[k + 2], y[k + 3]));
+            if (!is_finite(n)) {
+                n = 0.f;
+#pragma unroll
+                for (int k = 0; k < 16; k += 4) n = fmaxf(n, largest_finite4(y[k], y[k + 1], y[k + 2], y[k + 3]));
+            }
+            m[0] = fmaxf(m[0], n);
+        }
+        if (--left == 0 || t == last - 1) {
+            if constexpr (four) {
+                unsigned lo = h2_exponent(m[0]) | h2_exponent(m[1]) << 16, hi = h2_exponent(m[2]) | h2_exponent(m[3]) << 16;
+                lo = __vmaxu2(lo, __shfl_xor_sync(0xffffffffu, lo, 16));
+                hi = __vmaxu2(hi, __shfl_xor_sync(0xffffffffu, hi, 16));
+                if ((threadIdx.x & 16) == 0) sh.warp_words[i][threadIdx.x >> 5][threadIdx.x & 15] = __byte_perm(lo, hi, 0x6420);
+            } else {
+                m[0] = fmaxf(m[0], __shfl_xor_sync(0xffffffffu, m[0], 1));
+                m[0] = fmaxf(m[0], __shfl_xor_sync(0xffffffffu, m[0], 2));
+                if (row_lane) sh.row_top[i][row] = (unsigned char)h2_exponent(m[0]);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) m[j] = 0.f;
+            left = span;
+            ++i;
+        }
+        if (!any && t + 1 < last) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) q[k] = next[k];
         }
     }
     __syncthreads();
-    int rel = -1000, all = 0;  // this row's largest exponent relative to its tile's; the largest of all
-    for (int i = 0; i * span < last - first; ++i) {
-        const int c = tile_top(i), e = row_top[i][row];
-        rel = e == 0 ? rel : max(rel, e - c);
-        all = max(all, c);
+    for (int k = threadIdx.x; k < factors * 16; k += 256) {  // a factor to 16 lanes, a word of four rows each
+        const int i = k >> 4, word = k & 15;
+        unsigned *tops = reinterpret_cast<unsigned *>(sh.row_top[i]) + word, w = 0;
+        if constexpr (four) {
+#pragma unroll
+            for (int p = 0; p < 8; ++p) w = __vmaxu4(w, sh.warp_words[i][p][word]);
+            *tops = w;
+        } else {
+            w = *tops;
+        }
+        w = __vmaxu4(w, w >> 16);
+        w = max(w & 0xffu, (w >> 8) & 0xffu);
+        const unsigned lanes = 0xffffu << (threadIdx.x & 16);
+#pragma unroll
+        for (int d = 8; d > 0; d >>= 1) w = max(w, __shfl_xor_sync(lanes, w, d));
+        if (word == 0) sh.tile_top[i] = (unsigned char)w;
     }
-    if (row_lane) row_rel[row] = rel;
-    if (threadIdx.x == 0) cta_top = all;
     __syncthreads();
+    int rel = -1000, all = 0;  // this row's largest exponent relative to its tile's; the largest of all
+    for (int i = 0; i < factors; ++i) {
+        const int top = sh.tile_top[i], e = sh.row_top[i][row];
+        rel = e == 0 ? rel : max(rel, e - top);
+        all = max(all, top);
+    }
     if (ctas > 1) {
+        if (row_lane) sh.row_rel[row] = rel;
+        if (threadIdx.x == 0) sh.cta_top = all;
         cluster_sync_all();
-        const unsigned at = smem_u32(&row_rel[row]), top_at = smem_u32(&cta_top);
-        for (int q = 0; q < ctas; ++q) {
-            int o, w;
-            asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(o) : "r"(peer_addr(at, q)) : "memory");
-            asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(w) : "r"(peer_addr(top_at, q)) : "memory");
-            rel = max(rel, o);
+        const unsigned rel_at = smem_u32(&sh.row_rel[row]), top_at = smem_u32(&sh.cta_top);
+        for (int p = 0; p < ctas; ++p) {
+            int d, w;
+            asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(d) : "r"(peer_addr(rel_at, p)) : "memory");
+            asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(w) : "r"(peer_addr(top_at, p)) : "memory");
+            rel = max(rel, d);
             all = max(all, w);
         }
         cluster_sync_all();  // nobody leaves while a peer may still read its shared memory
     }
-    const int se = max(rel + all, 27);  // biased exponent of the row's scale times 2^14
-    if (rank == 0 && row_lane && r0 + row < v.rows) scale[b * v.rows + r0 + row] = __uint_as_float((unsigned)(se - 14) << 23);
-    for (int t = last - 1; t >= first; --t) {  // backwards: the last tile is still in registers
-        if (t != last - 1) fetch_row(v, s, r0, (long long)t * 64, tiles[t & 1], y);
-        const int c = tile_top((t - first) / span), f = c == 0 ? 0 : max(c - all, -kH2Far);  // 2^f: this tile's factor
-        if (threadIdx.x == 0) ratio[group * v.col_tiles + t] = __uint_as_float((unsigned)(127 + f) << 23);
-        int e = se + f;  // at least this row's largest in this tile
-        if (e < 27) {    // a factor of 2^(14 + 127 - e) would not be finite: two steps, both exact
-            const float up = __uint_as_float((unsigned)(127 + 27 - e) << 23);
+    int se[4];  // biased exponent of the scale of this thread's row(s), times 2^14
+    se[0] = max(rel + all, 27);
+    const long long at_row = b * v.rows + r0 + row;
+    if (rank == 0 && row_lane && row_in) o.scale[at_row] = __uint_as_float((unsigned)(se[0] - 14) << 23);
+    if constexpr (four) {
+        if (row_lane) sh.row_scale[row] = se[0];
+        __syncthreads();
+        const int4 w = *reinterpret_cast<const int4 *>(&sh.row_scale[r4]);
+        se[0] = w.x;
+        se[1] = w.y;
+        se[2] = w.z;
+        se[3] = w.w;
+    }
+    // ---- second look, backwards: the last tile is still in registers (single elements: in its buffer, and the one before it too)
+    if (any && last - 3 >= first) load(last - 3, next);
+    const int lowest = four ? min(min(se[0], se[1]), min(se[2], se[3])) : se[0];
+    const int part = (threadIdx.x & 3) * 8;
+    unsigned short *d = o.hi + at_row * v.pitch + part;
+    float *ratio = o.ratio + (long long)group * v.col_tiles;
+    for (int t = last - 1; t >= first; --t) {
+        const int top = sh.tile_top[span == 1 ? t - first : (t - first) / span], f = top == 0 ? 0 : max(top - all, -kH2Far);  // 2^f: this tile's factor
+        if (threadIdx.x == 0) ratio[t] = __uint_as_float((unsigned)(127 + f) << 23);
+        float factor[4];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) y[i] *= up;
-            e = 27;
+        for (int j = 0; j < (four ? 4 : 1); ++j) factor[j] = __uint_as_float((unsigned)(268 - se[j] - f) << 23);  // (se + f: at least the row's largest in this tile)
+        const bool far = lowest + f < 27;  // a factor would not be finite: two steps, both exact
+        if constexpr (four) {
+            if (t > first) load(t - 1, next);
+            if (far) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (se[j] + f >= 27) continue;
+                    const float up = __uint_as_float((unsigned)(127 + 27 - se[j] - f) << 23);
+                    factor[j] = __uint_as_float((unsigned)(268 - 27) << 23);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        if (j == 0) q[i].x *= up;
+                        if (j == 1) q[i].y *= up;
+                        if (j == 2) q[i].z *= up;
+                        if (j == 3) q[i].w *= up;
+                    }
+                }
+            }
+            unsigned *hi = reinterpret_cast<unsigned *>(sh.pieces[t & 1][0][r4]), *lo = reinterpret_cast<unsigned *>(sh.pieces[t & 1][1][r4]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const float4 &qa = q[2 * half], &qb = q[2 * half + 1];
+                    unsigned h, l;
+                    h2_split2(j == 0 ? qa.x : j == 1 ? qa.y : j == 2 ? qa.z : qa.w, j == 0 ? qb.x : j == 1 ? qb.y : j == 2 ? qb.z : qb.w, factor[j], &h, &l);
+                    const int word = j * 32 + (((line >> 2) + 4 * half) ^ piece_swizzle(r4 + j)) * 4 + (line & 3);
+                    hi[word] = h;
+                    lo[word] = l;
+                }
+            }
+            __syncthreads();  // (one a tile: the buffer's next writers have passed the barrier behind these reads)
+            if (row_in) {
+                const int left = (int)v.pitch - t * 64 - part;  // pitch is a multiple of 8: whole 16-byte pieces, zeros behind the last column
+                unsigned short *to = d + t * 64;
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    if (32 * half >= left) break;
+                    const int chunk = ((threadIdx.x & 3) + 4 * half) ^ piece_swizzle(row);
+                    *reinterpret_cast<uint4 *>(to + 32 * half) = sh.pieces[t & 1][0][row][chunk];
+                    *reinterpret_cast<uint4 *>(to + v.plane + 32 * half) = sh.pieces[t & 1][1][row][chunk];
+                }
+            }
+            if (t > first) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) q[i] = next[i];
+            }
+        } else {
+            float y[16];
+            if constexpr (any) {
+                if (t < last - 2) {
+                    if (t == last - 3) __syncthreads();  // the two tiles that lay in the buffers have been read
+                    store_singles(v, x, sh.tiles[t & 1]);
+                    if (t > first) load(t - 1, next);
+                    __syncthreads();
+                }
+                tile_row(sh.tiles[t & 1], y);
+            } else {
+                quads_row(q, y);
+                if (t > first) load(t - 1, q);
+            }
+            if (far) {
+                const float up = __uint_as_float((unsigned)(127 + 27 - se[0] - f) << 23);
+                factor[0] = __uint_as_float((unsigned)(268 - 27) << 23);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) y[i] *= up;
+            }
+            if (row_in) store_row(y, factor[0], d + t * 64, v.plane, (int)v.pitch - t * 64 - part);
         }
-        store_row(v, b, r0, (long long)t * 64, y, __uint_as_float((unsigned)(268 - e) << 23), hi);
+    }
+}
+
+// Operand B's blocks (in clusters of `ctas`), then operand A's; a launch may have either kind alone.  A plain product brings both in
+// with one launch: the second kernel's start and its first loads no longer follow the first one's end.  Whole calls, us, two kernels
+// | one: 997 x 1234 x 777 28.4 | 26.2, 512^3 17 | 14, 12 x (300 x 400 x 500) 39.5 | 31, 1000 x 100 x 5000 52.6 | 39, 8192 x 64 x 1024
+// 29.4 | 24.4, 4096^3 (320 MB of traffic in the chain, with the last result on its way out of L2) 388 | 380.
+struct SplitPair {
+    ViewP a, b;
+    SplitOut out_a, out_b;
+    unsigned b_blocks, a_blocks;
+    int ctas, tiles_per_cta, span, run;
+};
+__global__ void __launch_bounds__(256, 4) split_h2_kernel(const __grid_constant__ SplitPair p) {
+    __shared__ RowsShared sh;
+    grid_dependency_sync();
+    const unsigned block = blockIdx.x;
+    if (block < p.b_blocks) {
+        if (!p.b.vec) split_rows<kRowsAny>(p.b, p.out_b, block, p.ctas, p.tiles_per_cta, p.span, sh);
+        else if (p.b.cs == 1) split_rows<kRowsOne>(p.b, p.out_b, block, p.ctas, p.tiles_per_cta, p.span, sh);
+        else split_rows<kRowsFour>(p.b, p.out_b, block, p.ctas, p.tiles_per_cta, p.span, sh);
+    } else if (block - p.b_blocks < p.a_blocks) {
+        split_tiles(p.a, p.out_a, block - p.b_blocks, p.run, sh.tiles[0]);
     }
 }
 
@@ -264,38 +494,60 @@ size_t split_h2_bytes(long long batches, long long rows, long long cols, bool wh
     return up256(planes) + up256((size_t)(batches * (whole_rows ? rows + (rows + 63) / 64 * tiles : rows * tiles)) * 4);
 }
 
-static sage_status split_view_to(Context &ctx, const float *src, const SplitView &v, bool whole_rows, const H2Split &out) {
+static ViewP view_params(const float *src, const SplitView &v, const H2Split &out) {
     ViewP p{src, v.nb0, v.sb0, v.sb1, v.ld, v.col_stride, v.rows, v.cols, out.pitch, out.plane, (int)((v.rows + 63) / 64), (int)((v.cols + 63) / 64), 0};
     p.vec = (v.col_stride == 1 || v.ld == 1) && aligned16(src) && v.sb0 % 4 == 0 && v.sb1 % 4 == 0 && (v.col_stride == 1 ? v.ld % 4 == 0 && v.cols % 4 == 0 : v.col_stride % 4 == 0 && v.rows % 4 == 0);
-    const long long groups = v.nb0 * v.nb1 * p.row_tiles, blocks = groups * (whole_rows ? 8 : p.col_tiles);
+    return p;
+}
+static sage_status split_views(Context &ctx, const float *src_a, const SplitView *va, const H2Split &out_a, const float *src_b, const SplitView *vb, const H2Split &out_b) {
+    SplitPair p{};
+    long long a_blocks = 0, b_blocks = 0;
+    p.ctas = p.tiles_per_cta = p.span = p.run = 1;
+    if (va) {
+        p.a = view_params(src_a, *va, out_a);
+        p.out_a = SplitOut{out_a.hi, out_a.scale, nullptr};
+        const long long lines = va->nb0 * va->nb1 * p.a.row_tiles, fill = (long long)ctx.sm_count * 16;
+        while (p.run < 8 && lines * p.a.col_tiles >= fill * p.run * 2) p.run *= 2;  // as long as the chip is filled several times over
+        a_blocks = lines * ((p.a.col_tiles + p.run - 1) / p.run);
+    }
+    if (vb) {
+        p.b = view_params(src_b, *vb, out_b);
+        p.out_b = SplitOut{out_b.hi, out_b.scale, out_b.ratio};
+        while (p.ctas < 8 && p.ctas * 2 <= p.b.col_tiles) p.ctas *= 2;
+        p.tiles_per_cta = (p.b.col_tiles + p.ctas - 1) / p.ctas;
+        p.span = (p.tiles_per_cta + kFactors - 1) / kFactors;
+        b_blocks = vb->nb0 * vb->nb1 * p.b.row_tiles * p.ctas;
+    }
+    const long long blocks = b_blocks + (a_blocks + p.ctas - 1) / p.ctas * p.ctas;
     if (blocks > 0x7fffffffLL) return ctx.fail(SAGE_ERR_UNSUPPORTED, "split_h2: extents beyond 2^31 tiles");
-    ctx.note_launch(ctx.verbose_names ? "split_h2" : "split_tf32");  // launch lists have one name for an operand's split
+    p.a_blocks = (unsigned)a_blocks;
+    p.b_blocks = (unsigned)b_blocks;
+    const char *name = ctx.verbose_names ? "split_h2" : "split_tf32";  // launch lists have one name for an operand's split
+    if (va && vb) ctx.note_part(name);
+    ctx.note_launch(name);
     if (ctx.dry()) return SAGE_OK;
-    if (!whole_rows)
-        return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), split_h2_view_kernel, dim3((unsigned)blocks), dim3(256), 0, p, out.hi, out.scale), "split_h2 launch");
-    int ctas = 1;
-    while (ctas < 8 && ctas * 2 <= p.col_tiles) ctas *= 2;
-    const int per = (p.col_tiles + ctas - 1) / ctas;
-    return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), ctas, split_h2_rows_kernel, dim3((unsigned)(groups * ctas)), dim3(256), 0, p, out.hi, out.scale, out.ratio, ctas, per,
-                                           (per + kFactors - 1) / kFactors),
-                          "split_h2 rows launch");
+    return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), p.ctas, split_h2_kernel, dim3((unsigned)blocks), dim3(256), 0, p), "split_h2 launch");
 }
 
-sage_status split_h2_rows_at(Context &ctx, const float *src, const SplitView &v, const H2Split &out) { return split_view_to(ctx, src, v, true, out); }
+sage_status split_h2_rows_at(Context &ctx, const float *src, const SplitView &v, const H2Split &out) { return split_views(ctx, nullptr, nullptr, H2Split(), src, &v, out); }
 
-sage_status split_h2_view_into(Context &ctx, const float *src, const SplitView &v, bool whole_rows, void *dst, H2Split *out) {
-    out->pitch = h2_pitch(v.cols);
-    out->plane = v.nb0 * v.nb1 * v.rows * out->pitch;
-    out->hi = static_cast<unsigned short *>(dst);
-    out->scale = reinterpret_cast<float *>(static_cast<char *>(dst) + up256((size_t)out->plane * 4));
-    out->ratio = out->scale + v.nb0 * v.nb1 * v.rows;
-    return split_view_to(ctx, src, v, whole_rows, *out);
+// The layout of an operand's pieces in `dst` (of split_h2_bytes).
+static H2Split split_layout(const SplitView &v, void *dst) {
+    H2Split out;
+    out.pitch = h2_pitch(v.cols);
+    out.plane = v.nb0 * v.nb1 * v.rows * out.pitch;
+    out.hi = static_cast<unsigned short *>(dst);
+    out.scale = reinterpret_cast<float *>(static_cast<char *>(dst) + up256((size_t)out.plane * 4));
+    out.ratio = out.scale + v.nb0 * v.nb1 * v.rows;
+    return out;
 }
 
 sage_status split_h2_view(Context &ctx, const float *src, const SplitView &v, bool whole_rows, H2Split *out) {
-    out->block = ctx.allocator().alloc(split_h2_bytes(v.nb0 * v.nb1, v.rows, v.cols, whole_rows));
-    if (!out->block) return ctx.fail(SAGE_ERR_OOM, "out of memory for an operand in half-precision pieces");
-    return split_h2_view_into(ctx, src, v, whole_rows, out->block->ptr, out);
+    Block *block = ctx.allocator().alloc(split_h2_bytes(v.nb0 * v.nb1, v.rows, v.cols, whole_rows));
+    if (!block) return ctx.fail(SAGE_ERR_OOM, "out of memory for an operand in half-precision pieces");
+    *out = split_layout(v, block->ptr);
+    out->block = block;
+    return whole_rows ? split_views(ctx, nullptr, nullptr, H2Split(), src, &v, *out) : split_views(ctx, src, &v, *out, nullptr, nullptr, H2Split());
 }
 
 H2Operand h2_operand(const H2Split &s, long long batches, long long rows, long long cols, bool whole_rows) {
@@ -481,9 +733,8 @@ sage_status gemm_h2(Context &ctx, const GemmArgs &a, void *scratch) {
         if (!block) return ctx.fail(SAGE_ERR_OOM, "out of memory for the operands in half-precision pieces");
         scratch = block->ptr;
     }
-    H2Split pa, pb;
-    sage_status st = split_h2_view_into(ctx, a.a, va, false, scratch, &pa);
-    if (!st) st = split_h2_view_into(ctx, a.b, vb, true, static_cast<char *>(scratch) + split_h2_bytes(a.batch, a.m, a.k, false), &pb);
+    const H2Split pa = split_layout(va, scratch), pb = split_layout(vb, static_cast<char *>(scratch) + split_h2_bytes(a.batch, a.m, a.k, false));
+    sage_status st = split_views(ctx, a.a, &va, pa, a.b, &vb, pb);
     if (!st) {
         H2Gemm g;
         g.m = a.m;

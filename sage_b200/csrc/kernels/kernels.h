@@ -225,7 +225,6 @@ struct H2Split {
     long long plane = 0, pitch = 0;
 };
 size_t split_h2_bytes(long long batches, long long rows, long long cols, bool whole_rows);
-sage_status split_h2_view_into(Context &ctx, const float *src, const SplitView &v, bool whole_rows, void *dst, H2Split *out);
 sage_status split_h2_view(Context &ctx, const float *src, const SplitView &v, bool whole_rows, H2Split *out);
 // Operand B straight into memory the caller laid out: rows of `out->pitch` at out->hi / out->hi + out->plane, out->scale.
 sage_status split_h2_rows_at(Context &ctx, const float *src, const SplitView &v, const H2Split &out);

@@ -155,6 +155,10 @@ public:
         if (tracing) trace.append(name).push_back('\n');
         if (profiling) profile_mark(name);
     }
+    // A pass that shares the next launch with another one: launch lists name both, the count is of launches.
+    void note_part(const char *name) {
+        if (tracing) trace.append(name).push_back('\n');
+    }
     void note_memset() { ++memset_launches; }
     uint64_t kernel_launches = 0, memset_launches = 0;
     bool tracing = false;

@@ -82,6 +82,22 @@ def test_transposed_and_batched_operands(ctx, ta, tb, batch, m, n, k):
     assert excess(got, np.swapaxes(a, 1, 2) if ta else a, np.swapaxes(b, 1, 2) if tb else b) <= 1.0
 
 
+# How operand B is read: single elements along K and across it, 16 bytes of one row, of four; one to five tiles of 64 k a CTA, the last
+# one cut; K beyond 2^15, where tiles share a factor.  Operand A's blocks of one tile and of several.
+@pytest.mark.parametrize("tb,n,k", [(True, 67, 1985), (True, 68, 1984), (False, 67, 1985), (False, 68, 1985), (True, 96, 1028), (False, 132, 520), (True, 33, 2561), (False, 64, 33000),
+                                    (True, 64, 33000), (True, 40, 33001)])
+@pytest.mark.parametrize("m", [70, 2500])
+def test_splits_of_operands(ctx, tb, n, k, m):
+    rng = np.random.default_rng(n + k)
+    if k > 30000 and m > 70:
+        pytest.skip("one size of A is enough for the longest K")
+    a, b = rng.standard_normal((1, m, k), dtype=np.float32), rng.standard_normal((1, n, k) if tb else (1, k, n), dtype=np.float32)
+    b[0, :: 7 if tb else 1, 1::3] *= 2.0 ** -20   # rows, and tiles of them, of different ranges
+    a[0, 1::5] *= 2.0 ** 18
+    assert excess(product(ctx, a, b, False, tb), a, np.swapaxes(b, 1, 2) if tb else b) <= 1.0
+    assert ctx.status_word() == 0
+
+
 @pytest.mark.parametrize("ea,eb", [(100, -100), (-90, 90), (120, 0), (0, 120), (-90, 20)])
 def test_operands_far_from_one(ctx, ea, eb):
     """Whole operands scaled by powers of two give the scaled product, bit for bit, for rows of A above 2^-96."""
