@@ -3,6 +3,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 #include <mutex>
@@ -885,11 +886,13 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
     if (halo) cols = ColumnPlan{g.n <= 64 ? 64 : 128, 0, 0};  // all output channels in one tile: the window is loaded once
     const int bn = cols.bn;
     const int stage_bytes = halo ? 2 * (bn / ctas) * HK * 2 : 2 * BM * HK * 2 + 2 * (bn / ctas) * HK * 2;
-    const int staging = kEpiWarps * kStageBytesPerWarp, fixed = halo ? kHaloStages * kHaloStageBytes : 0;
+    const long long octets = std::min<long long>(BM / 8, (g.m + 7) / 8);  // of a tile: H2Tasks
+    const int staging = sliced ? (int)((octets * (bn / 64) + cut.slices - 1) / cut.slices) * cut.slices * 2048 : kEpiWarps * kStageBytesPerWarp;
+    const int fixed = halo ? kHaloStages * kHaloStageBytes : 0;
     int stages = (227 * 1024 - 2048 - staging - fixed) / stage_bytes;
     if (stages > 8) stages = 8;
     const long long all_kb = (g.k + HK - 1) / HK, my_kb = sliced ? (all_kb + cut.slices - 1) / cut.slices : all_kb;
-    if (sliced && stages > my_kb) stages = (int)my_kb;  // two CTAs fit an SM then: the next kernel's start overlaps this one's end
+    if (sliced && stages > my_kb) stages = (int)my_kb;
     const size_t smem = (size_t)fixed + (size_t)stages * stage_bytes + staging + 1024;
 
     H2Params p{};
