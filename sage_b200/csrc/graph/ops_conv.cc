@@ -15,6 +15,8 @@ static long long conv_size(long long size, long long ker, long long stride, long
     return (size + 2 * pad - dil * (ker - 1) - 1) / stride + 1;
 }
 
+sage_status storage_planes_attach(Context &ctx, Storage &st);  // ops_gemm.cc
+
 struct Im2colOp : Operator {
     Pair ker, stride, pad, dil, col;
     const char *name() const override { return "im2col"; }
@@ -22,13 +24,28 @@ struct Im2colOp : Operator {
         return {col2im(gy, Pair{x[0].extent(2), x[0].extent(1)}, ker, stride, pad, dil)};
     }
     sage_status compute(const std::vector<Tensor> &x, Context &ctx, Tensor *y) override {
+        const bool emit = ctx.hint_emit_planes && emits_planes();
+        ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = false;
         sage_status st = Tensor::uninit(ctx, out, y);
         if (st) return st;
         const Array &e = x[0].desc.shape.extents;
-        return k::im2col(ctx, (const float *)x[0].ptr(), (float *)y->ptr(), e[0], e[1], e[2], e[3], col.h, col.w,
-                         window(ker, stride, pad, dil));
+        if (!emit)
+            return k::im2col(ctx, (const float *)x[0].ptr(), (float *)y->ptr(), e[0], e[1], e[2], e[3], col.h, col.w, window(ker, stride, pad, dil));
+        st = storage_planes_attach(ctx, *y->data);
+        if (st) return st;
+        const SplitCache &c = *y->data->split;
+        return k::im2col_planes(ctx, (const float *)x[0].ptr(), e[0], e[1], e[2], e[3], col.h, col.w, window(ker, stride, pad, dil), (float *)y->ptr(), c.planes.planes, c.plane,
+                                (int)(ker.h * ker.w * e[3]));
     }
+    // the planes lie like the result, whole 16-byte pieces at a time
+    bool emits_planes() const { return in[0].shape.extents[3] % 4 == 0 && ker.h * ker.w * in[0].shape.extents[3] <= 0x7fffffffLL; }
 };
+// Does the column matrix come with its tf32 planes when a product reads it (the forward and the weight gradient of a convolution in a
+// training program)?  Split by a pass of their own they were 19 launches of a ResNet-18 step.
+bool im2col_op_emits_planes(const Operator &op) {
+    const Im2colOp *o = dynamic_cast<const Im2colOp *>(&op);
+    return o && o->emits_planes();
+}
 
 bool im2col_params(const Operator &op, k::Window *w, long long dims[6]) {
     const Im2colOp *o = dynamic_cast<const Im2colOp *>(&op);

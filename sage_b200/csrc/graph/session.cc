@@ -71,6 +71,7 @@ bool gemm_is_h2(const Operator &op);
 bool gemm_emits_h2(const Operator &op);
 bool row_op_emits_h2(const Operator &op);
 bool pool_op_emits_h2(const Operator &op);  // ops_conv.cc
+bool im2col_op_emits_planes(const Operator &op);
 bool map_op_emits_h2(const Operator &op);
 std::string describe_gemm(const Operator &op);  // "{epilogue}" / "[store]" of a lowered GEMM, else empty
 
@@ -481,7 +482,7 @@ static Node *skip_views(Node *p, long long *offset = nullptr) {  // *offset: whe
 }
 bool map_op_emits_planes(const Operator &op);
 static bool can_emit_planes(const Operator &op, bool tc) {
-    return gemm_runs_on_tc(op, tc) || row_op_emits_planes(op) || is_grouped_gemm_op(op) || (tc && map_op_emits_planes(op));
+    return gemm_runs_on_tc(op, tc) || row_op_emits_planes(op) || is_grouped_gemm_op(op) || (tc && (map_op_emits_planes(op) || im2col_op_emits_planes(op)));
 }
 static bool can_emit_h2(const Operator &op) { return gemm_emits_h2(op) || row_op_emits_h2(op) || map_op_emits_h2(op) || pool_op_emits_h2(op); }
 
@@ -516,7 +517,7 @@ static void assign_h2(Node &n, bool tc, Program &p, std::unordered_set<Origin *>
         a = skip_views(&it->second.root);
     }
     // a producer that can only write tf32 planes (a product of two results) keeps its reader on them
-    if (!a->is_data && !can_emit_h2(*a->op) && can_emit_planes(*a->op, tc)) return;
+    if (!a->is_data && !can_emit_h2(*a->op) && can_emit_planes(*a->op, tc) && !im2col_op_emits_planes(*a->op)) return;
     if (std::shared_ptr<Operator> op = gemm_on_h2(*n.op, given, tc)) n.op = op;
 }
 

@@ -39,10 +39,11 @@ struct ColOut {
 
 __device__ __forceinline__ void split_pair(float x, float *hi, float *lo) { sage_tc::split_tf32_value(x, hi, lo); }
 
-__global__ void __launch_bounds__(256) im2col_kernel(const float *__restrict__ img, ColOut o, ConvP p, long long pixels) {
+// `share` warps to a pixel where there are few of them (128 pixels of 9 x 512 values, one warp each: 16 blocks, 8 us).
+__global__ void __launch_bounds__(256) im2col_kernel(const float *__restrict__ img, ColOut o, ConvP p, long long pixels, int share) {
     grid_dependency_sync();
-    const int lane = threadIdx.x & 31;
-    const long long pix = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const long long warp = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), pix = warp / share;
+    const int lane = (threadIdx.x & 31) + 32 * (int)(warp - pix * share), step = 32 * share;
     if (pix >= pixels) return;
     const unsigned per_img = (unsigned)(p.col_h * p.col_w);
     const long long n = pix / per_img;
@@ -53,7 +54,7 @@ __global__ void __launch_bounds__(256) im2col_kernel(const float *__restrict__ i
     const float *im = img + n * p.img_h * p.img_w * C;
     if ((C & 3) == 0) {
         const int c4n = C >> 2, chunks = K >> 2;
-        for (int ch = lane; ch < chunks; ch += 32) {
+        for (int ch = lane; ch < chunks; ch += step) {
             const int tap = ch / c4n, c = (ch - tap * c4n) << 2;
             const int ky = tap / p.w.ker_w, kx = tap - ky * p.w.ker_w;
             const int iy = iy0 + ky * p.w.dil_h, ix = ix0 + kx * p.w.dil_w;
@@ -74,7 +75,7 @@ __global__ void __launch_bounds__(256) im2col_kernel(const float *__restrict__ i
         }
     } else {
         const int width = o.hi ? o.pitch : K;
-        for (int kk = lane; kk < width; kk += 32) {
+        for (int kk = lane; kk < width; kk += step) {
             float v = 0.f;
             if (kk < K) {
                 const int tap = kk / C, c = kk - tap * C;
@@ -200,19 +201,30 @@ __global__ void __launch_bounds__(256) col2im_quads_kernel(const float *__restri
         const int xe = min(xp / sw + 1, CW), ye = min(yp / sh + 1, CH);
         const float *cb = col + n * (long long)CH * CW * kh * kw * p.chan + c;
         float4 val = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int cx = xs; cx < xe; ++cx)
-            for (int cy = ys; cy < ye; ++cy) {
+        for (int cx = xs, cy = ys; cx < xe && ys < ye;) {  // nine taps asked for at a time, taken in the window's order
+            float4 v[9];
+#pragma unroll
+            for (int u = 0; u < 9; ++u) {
+                v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
                 int kx = xp - cx * sw, ky = yp - cy * sh;
-                if (kx % dh == 0 && ky % dw == 0) {  // the reference's test (conv.rs:462-464), dilations crossed as there
+                if (cx < xe && (dh == 1 || kx % dh == 0) && (dw == 1 || ky % dw == 0)) {  // the reference's test (conv.rs:462-464), dilations crossed as there
                     kx /= dh;
                     ky /= dw;
-                    const float4 v = __ldg(reinterpret_cast<const float4 *>(cb + ((((long long)cy * CW + cx) * kh + ky) * kw + kx) * p.chan));
-                    val.x += v.x;
-                    val.y += v.y;
-                    val.z += v.z;
-                    val.w += v.w;
+                    v[u] = __ldg(reinterpret_cast<const float4 *>(cb + ((((long long)cy * CW + cx) * kh + ky) * kw + kx) * p.chan));
+                }
+                if (++cy == ye) {
+                    cy = ys;
+                    ++cx;
                 }
             }
+#pragma unroll
+            for (int u = 0; u < 9; ++u) {
+                val.x += v[u].x;
+                val.y += v[u].y;
+                val.z += v[u].z;
+                val.w += v[u].w;
+            }
+        }
         *reinterpret_cast<float4 *>(img + (pix * p.chan + c)) = val;
     }
 }
@@ -328,7 +340,10 @@ sage_status im2col_planes(Context &ctx, const float *img, long long n, long long
         launch_dependent(ctx.pdl, ctx.stream(), im2col_quads_kernel, dim3(grid_for(ctx, quads)), dim3(256), 0, img, o, p, quads);
         return ctx.check_cuda(cudaGetLastError(), "im2col launch");
     }
-    launch_dependent(ctx.pdl, ctx.stream(), im2col_kernel, dim3((unsigned)((pixels + 7) / 8)), dim3(256), 0, img, o, p, pixels);
+    int share = 1;
+    const long long length = w.ker_h * w.ker_w * chan / (vec ? 4 : 1);  // loads of a pixel
+    while (share < 16 && pixels * share < 32LL * ctx.sm_count && length >= 128LL * share) share *= 2;
+    launch_dependent(ctx.pdl, ctx.stream(), im2col_kernel, dim3((unsigned)((pixels * share + 7) / 8)), dim3(256), 0, img, o, p, pixels, share);
     return ctx.check_cuda(cudaGetLastError(), "im2col launch");
 }
 
