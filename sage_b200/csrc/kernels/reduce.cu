@@ -321,6 +321,92 @@ __global__ void __launch_bounds__(256) reduce_cols_kernel(const T *__restrict__ 
     reduce_cols_store<T, VEC>(part, y, cols, kind, ref_compat);
 }
 
+// Column reduction of up to 1024 rows a CTA: the CTAs of a cluster take a run of rows of one column tile each (64 columns, 16 lanes
+// with 16-byte loads; or 32 columns, one to a lane), eight loads in flight to a thread, and meet through distributed shared memory,
+// each finishing a part of the tile's columns.  Bound by latency: the start, two or three rounds of loads, one cluster barrier.  The
+// form above leaves partial rows in memory, and its last block's fence, ticket and second pass were a third of it.  Rows and ranks are
+// combined in a fixed order.
+template <typename T, int VEC>
+__global__ void __launch_bounds__(512) reduce_cols_cluster_kernel(const T *__restrict__ x, T *__restrict__ y, long long rows, long long cols, long long pitch, int rows_per_cta, int ctas,
+                                                                  int kind, int ref_compat) {
+    constexpr int LANES = VEC == 4 ? 16 : 32, TILE = LANES * VEC, GROUPS = 512 / LANES, U = 8;
+    struct alignas(sizeof(T) * VEC) Vec {
+        T v[VEC];
+    };
+    __shared__ T part[GROUPS][TILE + 1];
+    __shared__ T mine[TILE];
+    const int rank = (int)(blockIdx.x % (unsigned)ctas), lane = threadIdx.x % LANES, group = threadIdx.x / LANES;
+    const long long tile = blockIdx.x / (unsigned)ctas, col = tile * TILE + lane * VEC, r0 = (long long)rank * rows_per_cta;
+    const int left = (int)(min(rows, r0 + rows_per_cta) - r0);
+    T acc[VEC];
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) acc[e] = Ops<T>::identity(kind);
+    grid_dependency_sync();
+    if (col < cols) {
+        const T *base = x + r0 * pitch + col;
+        for (int r = group; r < left; r += GROUPS * U) {
+            Vec v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int at = r + GROUPS * u;
+                if (at < left) {
+                    v[u] = *reinterpret_cast<const Vec *>(base + at * pitch);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < VEC; ++e) v[u].v[e] = Ops<T>::identity(kind);
+                }
+            }
+#pragma unroll
+            for (int w = 1; w < U; w *= 2)  // pairwise: (0 1) (2 3) ..., then (01 23) ...
+#pragma unroll
+                for (int u = 0; u + w < U; u += 2 * w)
+#pragma unroll
+                    for (int e = 0; e < VEC; ++e) v[u].v[e] = Ops<T>::apply(kind, v[u].v[e], v[u + w].v[e]);
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) acc[e] = Ops<T>::apply(kind, acc[e], v[0].v[e]);
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) part[group][lane * VEC + e] = acc[e];
+    __syncthreads();
+    // 512 threads: 512 / TILE of them to a column, neighbours in a warp
+    constexpr int SHARE = 512 / TILE;
+    {
+        const int c = threadIdx.x / SHARE, k = threadIdx.x % SHARE;
+        T a = part[k][c];
+#pragma unroll
+        for (int g = k + SHARE; g < GROUPS; g += SHARE) a = Ops<T>::apply(kind, a, part[g][c]);
+#pragma unroll
+        for (int d = 1; d < SHARE; d *= 2) a = Ops<T>::apply(kind, a, __shfl_xor_sync(0xffffffffu, a, d));
+        if (k == 0) mine[c] = a;
+    }
+    const unsigned at = (unsigned)__cvta_generic_to_shared(mine);
+    if (ctas > 1) {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    } else {
+        __syncthreads();
+    }
+    const int share = TILE / ctas, c = rank * share + (int)threadIdx.x;
+    if ((int)threadIdx.x < share && tile * TILE + c < cols) {
+        T a = Ops<T>::identity(kind);
+        for (int q = 0; q < ctas; ++q) {
+            unsigned peer, raw;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(at + (unsigned)c * 4u), "r"(q));
+            asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(raw) : "r"(peer) : "memory");
+            T v;
+            memcpy(&v, &raw, sizeof(v));
+            a = q == 0 ? v : Ops<T>::apply(kind, a, v);
+        }
+        if (ref_compat) a = Ops<T>::apply(kind, (T)0, a);
+        y[tile * TILE + c] = a;
+    }
+    if (ctas > 1) {  // nobody leaves while a peer may still read its shared memory
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+}
+
 // Few slices of a long run: y[i] = x[i] (+) x[i + pitch] (+) ... over `slices` < 64 rows (the partial products of a
 // GEMM split over K, [S, m * n] -> [m * n]).  A thread owns four consecutive outputs and keeps up to eight 16-byte
 // loads in flight; the slices are combined in index order, so the result repeats bit for bit.
@@ -360,6 +446,20 @@ __global__ void __launch_bounds__(256) reduce_slices_kernel(const T *__restrict_
 template <typename T>
 static sage_status launch_reduce_cols(Context &ctx, int kind, const T *x, long long rows, long long cols, long long pitch, T *y, int compat_in) {
     const int compat = compat_in < 0 ? ctx.opts().ref_compat : compat_in;
+    {  // clusters of up to eight CTAs of up to 1024 rows (64 columns) each: beyond that too few loads are in flight on the chip
+        const bool quads = cols % 4 == 0 && pitch % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && cols >= 64;
+        const long long tiles = quads ? (cols + 63) / 64 : (cols + 31) / 32;
+        int ctas = 8;
+        while (ctas > 1 && (tiles * ctas > 4LL * ctx.sm_count || rows < 64LL * ctas)) ctas /= 2;
+        const long long per = (rows + ctas - 1) / ctas;
+        if (per <= (quads ? 1024 : 2048) && tiles * ctas <= 0x7fffffffLL) {
+            ctx.note_launch("reduce_cols");
+            if (ctx.dry()) return SAGE_OK;
+            launch_dependent(ctx.pdl, ctx.stream(), ctas, quads ? reduce_cols_cluster_kernel<T, 4> : reduce_cols_cluster_kernel<T, 1>, dim3((unsigned)(tiles * ctas)), dim3(512), 0, x, y,
+                             rows, cols, pitch, (int)per, ctas, kind, compat);
+            return ctx.check_cuda(cudaGetLastError(), "reduce_cols launch");
+        }
+    }
     // 16-byte loads (4 columns per lane) when the rows allow; the partial rows are read with pitch = cols
     const bool vec = cols % 4 == 0 && pitch % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && cols >= 256;
     const long long tiles = vec ? (cols + 127) / 128 : (cols + 31) / 32;
@@ -464,7 +564,9 @@ static sage_status launch_reduce(Context &ctx, int kind, const T *x, const Dims 
         }
     }
     int G = 1;
-    if (inner_contig && n_in >= 64) G = (n_in >= 8192 || n_out < 2LL * ctx.sm_count) ? 256 : 32;
+    // A block to an output for long runs, for few outputs, and where one wave of blocks holds all of them: a warp to each of the 512
+    // chunks of a [4096, 768] -> [1] sum has twelve rounds of loads, 64 blocks in all.
+    if (inner_contig && n_in >= 64) G = (n_in >= 8192 || n_out < 2LL * ctx.sm_count || (n_in >= 2048 && n_out <= 8LL * ctx.sm_count)) ? 256 : 32;
     // A column reduction with very few outputs would leave the GPU idle; a CTA per output is
     // uncoalesced but at least parallel.
     if (!inner_contig && n_out < 1024 && n_in >= 4096) G = 256;
