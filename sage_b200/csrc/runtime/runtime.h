@@ -98,7 +98,7 @@ struct Module {
     CUmod_st *cu_module = nullptr;  // null on a planning context
     struct Function {
         CUfunc_st *fn = nullptr;
-        uint32_t smem = 48 * 1024;  // dynamic shared memory it may be launched with
+        uint32_t smem = 40 * 1024;  // dynamic shared memory it may be launched with: 48 KiB less what a kernel may hold statically
     };
     std::unordered_map<std::string, Function> functions;
 };

@@ -1,0 +1,34 @@
+"""Whole-row programs (graph/rowfuse.cc) over column counts where the block's shape changes."""
+import numpy as np
+import pytest
+
+import sage_b200 as S
+
+pytestmark = pytest.mark.gpu
+
+
+# 3000: the two prefetch stages take 48 KiB exactly, and the kernel's own shared memory lies beside them
+@pytest.mark.parametrize("rows,cols", [(37, 3000)])
+def test_cross_entropy_and_gradient(rows, cols):
+    """Loss and gradient of the cross entropy of x y + 3.14 x against float64.  Tolerance: sums of `cols` fp32 terms and a few
+    roundings of the exponentials, 1e-5 of the value or of the rms."""
+    rng = np.random.default_rng(cols)
+    x, y = (rng.standard_normal((rows, cols), dtype=np.float32) for _ in range(2))
+    labels = rng.integers(0, cols, (rows, 1)).astype(np.uint32)
+    ctx = S.Context(0)
+    try:
+        xv = ctx.var(x)
+        loss = S.softmax_cross_entropy(xv * ctx.var(y) + xv * 3.14, ctx.var(labels))
+        gx = xv.grad(loss)
+        ctx.eval(loss, gx)
+        assert ctx.describe().startswith("row_program[%dx%d" % (rows, cols))
+        z = x.astype(np.float64) * y + x * np.float64(np.float32(3.14))
+        m = z.max(1, keepdims=True)
+        lse = np.log(np.exp(z - m).sum(1, keepdims=True)) + m
+        p = np.exp(z - lse)
+        p[np.arange(rows), labels[:, 0]] -= 1
+        for got, want in ((ctx.read(loss).reshape(-1), (lse - np.take_along_axis(z, labels.astype(np.int64), 1))[:, 0]), (ctx.read(gx), p * (y.astype(np.float64) + np.float32(3.14)))):
+            assert (np.abs(got - want) / np.maximum(np.abs(want), np.sqrt((want ** 2).mean()))).max() <= 1e-5
+        assert ctx.status_word() == 0
+    finally:
+        ctx.close()
