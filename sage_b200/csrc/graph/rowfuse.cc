@@ -60,6 +60,7 @@ constexpr size_t kMaxValues = 256;
 struct RowProgram {
     long long rows = 0, cols = 0;
     int threads = 0, nv = 0, vec = 0;
+    int regs = 80;  // registers per thread the kernel is compiled to fit
     std::vector<Val> vals;  // topological order
     std::vector<int> in_val, out_val;
     int n_map = 0, n_reduce = 0, n_index = 0;
@@ -273,9 +274,9 @@ SG void rp_prefetch(const RowP &p, long long row, uint4 *stage);
         if (bytes <= 96 * 1024) p.stage_bytes = (uint32_t)bytes;
     }
     s << "#define RP_STAGE " << (size_t)n_stage * p.nv * p.threads << "\n";
-    // at least as many blocks per SM as ~80 registers per thread allow: more warps to hide the latency of
+    // at least as many blocks per SM as p.regs registers per thread allow: more warps to hide the latency of
     // exp, shared memory and shuffles (the kernels run at low occupancy by construction)
-    s << "extern \"C\" __global__ void __launch_bounds__(RP_T, " << std::max(1, 65536 / (p.threads * 80)) << ") sage_row_program(const RowP p) {\n"
+    s << "extern \"C\" __global__ void __launch_bounds__(RP_T, " << std::max(1, 65536 / (p.threads * p.regs)) << ") sage_row_program(const RowP p) {\n"
       << "  asm volatile(\"griddepcontrol.launch_dependents;\" ::: \"memory\");\n"
       << "  asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");\n"
       << "  __shared__ float sh[2][" << std::max(1, n_red) << "][32];\n  __shared__ uint sh_pick[2][" << std::max(1, n_pick) << "];\n";
@@ -440,6 +441,20 @@ std::shared_ptr<RowProgram> row_program_build(const std::vector<Var> &evaluated,
     }
     if (p->nv * p->vec > 32) return nullptr;
     p->threads = (int)((t + 31) / 32 * 32);
+    // Rows of 4096 columns and more, with at most two whole-row inputs and one whole-row result: 32 elements per thread halve what the
+    // reductions cost per element.  Only where the threads have whole shares and twelve warps stay on an SM.  Loss and gradient of
+    // a cross entropy over 2^25 elements, us, 16 | 32 a thread: 4096 columns 80.0 | 75.8, 6144 86.6 | 80.7, 7000 124.7 | 93.7, 12000 105.2 | 100.6,
+    // 16384 111.6 | 102.2; outside the rule 4500 (an eighth of the threads idle) 98.2 | 108.0, 5120 (ten warps) 84.9 | 87.7, 2048 70.9 | 85.5.
+    int full_in = 0, full_out = 0;
+    for (int id : p->in_val) full_in += p->vals[id].cls == Full;
+    for (int id : p->out_val) full_out += p->vals[id].cls == Full;
+    const int wide = (int)((C + 1023) / 1024 * 32), wide_regs = 140;  // threads with 32 elements each
+    if (elems == 16 && p->vec == 4 && C >= 4096 && full_in <= 2 && full_out <= 1 && wide <= 1024 && wide * 32LL * 100 <= C * 103LL &&
+        std::max(1, 65536 / (wide * wide_regs)) * (wide / 32) >= 12) {
+        p->nv = 8;
+        p->threads = wide;
+        p->regs = wide_regs;
+    }
     if (!emit_source) return p;  // analysis only: is the graph a row program, and over which space
     emit(*p);
     if (const char *path = getenv("SAGE_ROW_PROGRAM_DUMP")) {  // diagnostics: the generated source

@@ -7,8 +7,9 @@ import sage_b200 as S
 pytestmark = pytest.mark.gpu
 
 
-# 3000: the two prefetch stages take 48 KiB exactly, and the kernel's own shared memory lies beside them
-@pytest.mark.parametrize("rows,cols", [(37, 3000)])
+# 3000: the two prefetch stages take 48 KiB exactly, and the kernel's own shared memory lies beside them.  From 4096: 32 elements a
+# thread where the threads have whole shares (4096, 4100 not, 6140 with an idle vector, 7000, 16384 and one vector less), 16 elsewhere.
+@pytest.mark.parametrize("rows,cols", [(37, 3000), (600, 4096), (5, 4092), (37, 4100), (300, 6140), (33, 7000), (5, 8192), (200, 16384), (2, 16380)])
 def test_cross_entropy_and_gradient(rows, cols):
     """Loss and gradient of the cross entropy of x y + 3.14 x against float64.  Tolerance: sums of `cols` fp32 terms and a few
     roundings of the exponentials, 1e-5 of the value or of the rms."""
