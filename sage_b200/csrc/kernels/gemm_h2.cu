@@ -814,7 +814,8 @@ static int clusters_at_once(const Context &ctx, int s) {
 // M 24 .. 3136, N 64 .. 3072, K 512 .. 4608: a K-block takes 0.52 / 0.67 / 0.92 with 64 / 128 / 256 columns (a pair of CTAs
 // 0.42 / 0.48 / 0.91, windows kept in shared memory 0.48), and not less than the bytes of all CTAs at 9 TB/s; a tile 3.5 beside
 // them, and 5 for operands that depend on the row, which slices fetch in time.  Meeting in shared memory: 1.5 and 1.1 per 128 x
-// 64 sums (256 columns: 9, never worth it).  Slices must promise a fifth: they change the order of summation, and nearer to the
+// 64 sums (256 columns: 9, never worth it), timed when the sums were fetched after a barrier; sent, they take less, and the line
+// is left on the safe side.  Slices must promise a fifth: they change the order of summation, and nearer to the
 // line than that the estimate says little.
 struct SlicePlan {
     int slices, bn;
