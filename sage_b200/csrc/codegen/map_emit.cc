@@ -89,7 +89,7 @@ SG void sg_h2_two(float x0, float x1, float f, uint *hi, uint *lo) {
   asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(l) : "f"(r1), "f"(r0));
   *hi = h; *lo = l;
 }
-SG void sg_h2_store(float4 r, unsigned long long g, unsigned short *h2, long long plane, float *scale) {
+SG void sg_h2_store(float4 r, unsigned long long g, unsigned short *h2, long long plane, float *scale, float *marked) {
   uint b = sg_h2_bits(r.x);
   uint t = sg_h2_bits(r.y); b = b > t ? b : t;
   t = sg_h2_bits(r.z); b = b > t ? b : t;
@@ -103,6 +103,14 @@ SG void sg_h2_store(float4 r, unsigned long long g, unsigned short *h2, long lon
   *reinterpret_cast<uint2 *>(h2 + g) = hi;
   *reinterpret_cast<uint2 *>(h2 + plane + g) = lo;
   if ((threadIdx.x & 15) == 0) scale[g >> 6] = __uint_as_float((uint)(e - 14) << 23);
+  if (marked) {  // an element other than 0 below 2^-14 once scaled (0, inf and nan less 1 are the largest)
+    b = sg_h2_bits(r.x) - 1u;
+    t = sg_h2_bits(r.y) - 1u; b = b < t ? b : t;
+    t = sg_h2_bits(r.z) - 1u; b = b < t ? b : t;
+    t = sg_h2_bits(r.w) - 1u; b = b < t ? b : t;
+    for (int o = 8; o > 0; o >>= 1) { t = __shfl_xor_sync(0xffffu << (threadIdx.x & 16), b, o); b = b < t ? b : t; }
+    if ((threadIdx.x & 15) == 0) marked[g >> 6] = (b != 0xffffffffu && __uint_as_float(b + 1u) * f < 1.f / 16384.f ? -1.f : 1.f) * __uint_as_float((uint)(e - 14) << 23);
+  }
 }
 )";
 
@@ -203,7 +211,7 @@ sage_status map_plan(const std::string &expr, const std::vector<MapOperand> &in,
     s << "extern \"C\" __global__ void __launch_bounds__(256) sage_map(";
     for (int q = 0; q < nin; ++q) s << "const " << ctype(in[q].dtype) << " *__restrict__ x" << q << "_buf, ";
     s << ctype(out_dtype) << " *__restrict__ y, const MapP p" << ((planes & 1) ? ", float *__restrict__ hi, const long long plane" : "")
-      << ((planes & 2) ? ", unsigned short *__restrict__ h2, const long long h2_plane, float *__restrict__ h2_scale" : "") << ") {\n";
+      << ((planes & 2) ? ", unsigned short *__restrict__ h2, const long long h2_plane, float *__restrict__ h2_scale, float *__restrict__ h2_marked" : "") << ") {\n";
     // launched as a programmatic dependent: wait for the kernel before this one before touching memory
     s << "  asm volatile(\"griddepcontrol.launch_dependents;\" ::: \"memory\");\n";
     s << "  asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");\n";
@@ -260,7 +268,7 @@ sage_status map_plan(const std::string &expr, const std::vector<MapOperand> &in,
             s << ");\n";
         }
         s << "  *reinterpret_cast<" << vtype(out_dtype) << " *>(y + g) = r;\n";
-        if (planes & 2) s << "  sg_h2_store(r, g, h2, h2_plane, h2_scale);\n";
+        if (planes & 2) s << "  sg_h2_store(r, g, h2, h2_plane, h2_scale, h2_marked);\n";
         if (planes & 1)
             s << "  { float4 h, l; sg_split_tf32(r.x, &h.x, &l.x); sg_split_tf32(r.y, &h.y, &l.y); sg_split_tf32(r.z, &h.z, &l.z); "
                  "sg_split_tf32(r.w, &h.w, &l.w);\n    *reinterpret_cast<float4 *>(hi + g) = h; *reinterpret_cast<float4 *>(hi + plane + g) = l; }\n";
@@ -324,6 +332,7 @@ sage_status map_launch(Context &ctx, const std::string &expr, const std::vector<
         params.push_back(&o.h2);
         params.push_back(&o.h2_plane);
         params.push_back(&o.h2_scale);
+        params.push_back(&o.h2_marked);
     }
     const long long chunks = (plan.n + plan.vec - 1) / plan.vec;
     const uint32_t grid[3] = {(uint32_t)((chunks + 255) / 256), 1, 1};
@@ -335,7 +344,7 @@ sage_status map_launch(Context &ctx, const std::string &expr, const std::vector<
             if (ch == ' ') ch = '_';
     }
     st = ctx.launch(mod, "sage_map", grid, block, 0, params.data(), label.empty() ? nullptr : label.c_str(), true);
-    if (!st && out.h2 && !(plan.planes & 2)) st = k::split_h2_flat(ctx, static_cast<const float *>(y), plan.n, out.h2, out.h2_plane, out.h2_scale);
+    if (!st && out.h2 && !(plan.planes & 2)) st = k::split_h2_flat(ctx, static_cast<const float *>(y), plan.n, out.h2, out.h2_plane, out.h2_scale, out.h2_marked);
     return st;
 }
 

@@ -118,7 +118,7 @@ Var ops::conv_2d(const Var &x, const Var &filter, Pair stride, Pair pad, Pair di
     return view(matmul(c2, f2), {n, ch, cw, cout});
 }
 
-sage_status storage_h2_attach(Context &ctx, Storage &st);  // ops_gemm.cc
+sage_status storage_h2_attach(Context &ctx, Storage &st, bool wide);  // ops_gemm.cc
 
 // Pooling as one kernel: the same value as im2col followed by mean / max over [KH,KW], without the
 // KH*KW-times larger intermediate.
@@ -134,17 +134,18 @@ struct Pool2dOp : Operator {
         const Array &o = out.shape.extents;
         // an image off the 16-byte grid takes the kernel without pieces; its reader splits the result
         const bool emit_h2 = ctx.hint_emit_h2 && k::pool2d_writes_pieces((const float *)x[0].ptr(), e[3], o[1], o[2]);
-        const bool only = emit_h2 && !ctx.hint_emit_planes && ctx.hint_planes_only;
-        ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = false;
+        const bool only = emit_h2 && !ctx.hint_emit_planes && ctx.hint_planes_only, wide = ctx.hint_mark_wide;
+        ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = ctx.hint_mark_wide = false;
         sage_status st = Tensor::uninit(ctx, out, y);
         if (st) return st;
         k::PlaneOut forms;
         if (emit_h2) {
-            st = storage_h2_attach(ctx, *y->data);
+            st = storage_h2_attach(ctx, *y->data, wide);
             if (st) return st;
             forms.h2 = y->data->h2->pieces.hi;
             forms.h2_plane = y->data->h2->pieces.plane;
             forms.h2_scale = y->data->h2->pieces.scale;
+            forms.h2_marked = y->data->h2->pieces.marked;
             y->data->planes_only = only;
         }
         return k::pool2d(ctx, is_max, (const float *)x[0].ptr(), only ? nullptr : (float *)y->ptr(), e[0], e[1], e[2], e[3], o[1], o[2],

@@ -48,26 +48,27 @@ static sage_status storage_planes(Context &ctx, Storage &st) {  // planes of exi
 }
 
 // ------------------------------------------------------------------------------ half-precision pieces of a storage
-sage_status storage_h2_attach(Context &ctx, Storage &st) {  // allocate only; the caller's kernel fills them
+sage_status storage_h2_attach(Context &ctx, Storage &st, bool wide) {  // allocate only; the caller's kernel fills them
     if (st.h2) return SAGE_OK;
     auto c = std::make_shared<H2Cache>();
     c->alloc = ctx.allocator_ptr();
     const long long n = ((long long)(st.bytes / 4) + 127) / 128 * 128;
     c->pieces.plane = n;
-    c->pieces.block = ctx.allocator().alloc((size_t)n * 4 + (size_t)(n / 64) * 4);
+    c->pieces.block = ctx.allocator().alloc((size_t)n * 4 + (size_t)(n / 64) * (wide ? 8 : 4));
     if (!c->pieces.block) return ctx.fail(SAGE_ERR_OOM, "out of memory for half-precision pieces");
     c->pieces.hi = reinterpret_cast<unsigned short *>(c->pieces.block->ptr);
     c->pieces.scale = reinterpret_cast<float *>(c->pieces.block->ptr + n * 4);
+    if (wide) c->pieces.marked = c->pieces.scale + n / 64;
     st.h2 = c;
     return SAGE_OK;
 }
 
-sage_status storage_h2(Context &ctx, Storage &st) {  // pieces of existing data: run the split pass
+sage_status storage_h2(Context &ctx, Storage &st, bool wide = false) {  // pieces of existing data: run the split pass
     if (st.h2) return SAGE_OK;
     if (st.planes_only) return ctx.fail(SAGE_ERR_INVALID, "internal: a tensor without fp32 values has no half-precision pieces");
-    sage_status s = storage_h2_attach(ctx, st);
+    sage_status s = storage_h2_attach(ctx, st, wide);
     if (s) return s;
-    s = k::split_h2_flat(ctx, (const float *)st.dev, (long long)(st.bytes / 4), st.h2->pieces.hi, st.h2->pieces.plane, st.h2->pieces.scale);
+    s = k::split_h2_flat(ctx, (const float *)st.dev, (long long)(st.bytes / 4), st.h2->pieces.hi, st.h2->pieces.plane, st.h2->pieces.scale, st.h2->pieces.marked);
     if (s) st.h2.reset();
     return s;
 }
@@ -212,19 +213,19 @@ bool h2_view_ok(const Shape &sh, bool trans) {
 }
 
 // Compact pieces of a view, kept beside the storage (`*c`) until another view is asked for there.
-static sage_status gather_h2(Context &ctx, const Tensor &t, bool swapped, const k::SplitView &v, bool whole_rows, std::shared_ptr<H2Cache> *c) {
-    if (*c && (*c)->view == t.desc.shape && (*c)->swapped == swapped) return SAGE_OK;
+static sage_status gather_h2(Context &ctx, const Tensor &t, bool swapped, const k::SplitView &v, bool whole_rows, std::shared_ptr<H2Cache> *c, bool mark = false) {
+    if (*c && (*c)->view == t.desc.shape && (*c)->swapped == swapped && (!mark || (*c)->pieces.marked)) return SAGE_OK;
     auto fresh = std::make_shared<H2Cache>();
     fresh->alloc = ctx.allocator_ptr();
     fresh->view = t.desc.shape;
     fresh->swapped = swapped;
-    sage_status s = k::split_h2_view(ctx, (const float *)t.ptr(), v, whole_rows, &fresh->pieces);
+    sage_status s = k::split_h2_view(ctx, (const float *)t.ptr(), v, whole_rows, &fresh->pieces, mark);
     if (!s) *c = fresh;
     return s;
 }
 
 // Operand A (a scale per row and 64 k) or B (`whole_rows`: one per row and factors, always a compact copy kept beside the storage).
-static sage_status make_h2_operand(Context &ctx, const Tensor &t, bool trans, bool whole_rows, k::H2Operand *op, std::shared_ptr<H2Cache> *hold) {
+static sage_status make_h2_operand(Context &ctx, const Tensor &t, bool trans, bool whole_rows, k::H2Operand *op, std::shared_ptr<H2Cache> *hold, bool mark = false) {
     const Shape &sh = t.desc.shape;
     const int r = sh.rank(), ka = trans ? r - 2 : r - 1, ma = trans ? r - 1 : r - 2;
     const long long rows = sh.extents[ma], cols = sh.extents[ka];
@@ -261,15 +262,17 @@ static sage_status make_h2_operand(Context &ctx, const Tensor &t, bool trans, bo
     v.ld = sh.strides[ma];
     v.col_stride = sh.strides[ka];
     std::shared_ptr<H2Cache> &c = whole_rows ? st.h2_rows : st.h2_view;
-    sage_status s = gather_h2(ctx, t, trans, v, whole_rows, &c);
+    sage_status s = gather_h2(ctx, t, trans, v, whole_rows, &c, mark);
     if (s) return s;
     *hold = c;
     *op = k::h2_operand(c->pieces, bl.n[0] * bl.n[1], rows, cols, whole_rows);
+    op->marked = c->pieces.marked;
+    op->columns = c->pieces.columns;
     return SAGE_OK;
 }
 
 // Where a result's operand forms go, as its readers asked: attaches them to `y` and says whether the fp32 store may be left out.
-static sage_status attach_forms(Context &ctx, Tensor *y, bool emit, bool emit_h2, k::PlaneOut *o) {
+static sage_status attach_forms(Context &ctx, Tensor *y, bool emit, bool emit_h2, k::PlaneOut *o, bool wide = false) {
     if (emit) {
         sage_status st = storage_planes_attach(ctx, *y->data);
         if (st) return st;
@@ -277,11 +280,12 @@ static sage_status attach_forms(Context &ctx, Tensor *y, bool emit, bool emit_h2
         o->plane = y->data->split->plane;
     }
     if (emit_h2) {
-        sage_status st = storage_h2_attach(ctx, *y->data);
+        sage_status st = storage_h2_attach(ctx, *y->data, wide);
         if (st) return st;
         o->h2 = y->data->h2->pieces.hi;
         o->h2_plane = y->data->h2->pieces.plane;
         o->h2_scale = y->data->h2->pieces.scale;
+        o->h2_marked = y->data->h2->pieces.marked;
     }
     return SAGE_OK;
 }
@@ -349,6 +353,7 @@ struct GemmOp : Operator {
     // Opt-in: narrow products (at most 128 output channels) read the image as plain fp32 and split it per tile in
     // shared memory.  Wider ones always keep whole-image planes (their kernels have no registers to spare for four more warps).
     bool conv_raw() const { return conv_raw_enabled() && n <= 128; }
+    bool conv_small() const { return k::conv_h2_small(img[0], img[1], img[2], img[3]); }  // (h2 only)
     bool conv_implicit() const { return conv && img[3] % 32 == 0 && img[0] * img[1] * img[2] * img[3] * 4 >= 131072; }
     // At most 4 input channels (the first convolution of an image model): the image is re-laid with 4-float pixels so
     // that the taps of a filter row are contiguous, and runs as an implicit GEMM over overlapping 32-float windows
@@ -379,14 +384,14 @@ struct GemmOp : Operator {
     }
 
     sage_status compute(const std::vector<Tensor> &x, Context &ctx, Tensor *y) override {
-        const bool emit = ctx.hint_emit_planes, emit_h2 = ctx.hint_emit_h2, only = (emit || emit_h2) && ctx.hint_planes_only;
-        ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = false;
+        const bool emit = ctx.hint_emit_planes, emit_h2 = ctx.hint_emit_h2, only = (emit || emit_h2) && ctx.hint_planes_only, mark = ctx.hint_mark_wide;
+        ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = ctx.hint_mark_wide = false;
         sage_status st = Tensor::uninit(ctx, out, y);
         if (st) return st;
         if (!lowered) dims_from_inputs();
-        if (h2) return compute_h2(x, ctx, y, emit, emit_h2, only);
+        if (h2) return compute_h2(x, ctx, y, emit, emit_h2, only, mark);
         if (!lowered && !attn && !batched && ctx.opts().pattern_fusion == 0 && ctx.opts().gemm_backend != 1 && k::gemm_tc_shape_ok(m, n, k, batch))
-            return compute_h2(x, ctx, y, false, false, false);  // the operator by itself
+            return compute_h2(x, ctx, y, false, false, false, false);  // the operator by itself
         if (conv_first() && x[0].desc.shape.has_default_strides() && x[1].desc.shape.has_default_strides() && !x[0].data->planes_only) return compute_first(x, ctx, y, emit, emit_h2, only);
         if (emit_h2 && !attn) return ctx.fail(SAGE_ERR_INVALID, "internal: the tf32 product does not write half-precision pieces");
         if (attn) return compute_attention(x, ctx, y, emit, emit_h2, only);
@@ -683,7 +688,7 @@ struct GemmOp : Operator {
         return k::conv_first_run(ctx, g, f);
     }
     // The same product on half-precision pieces (see assign_h2).
-    sage_status compute_h2(const std::vector<Tensor> &x, Context &ctx, Tensor *y, bool emit, bool emit_h2, bool only) {
+    sage_status compute_h2(const std::vector<Tensor> &x, Context &ctx, Tensor *y, bool emit, bool emit_h2, bool only, bool mark) {
         k::H2Gemm g;
         g.m = m;
         g.n = n;
@@ -696,16 +701,16 @@ struct GemmOp : Operator {
             Storage &is = *x[0].data;
             if (!img_shape.has_default_strides()) return ctx.fail(SAGE_ERR_INVALID, "internal: conv gemm needs a contiguous image");
             long long at = 0;  // where the image starts in the pieces
-            if (conv_image_direct(img_shape) && is.bytes % 256 == 0) {
-                st = storage_h2(ctx, is);
+            if (conv_image_direct(img_shape) && is.bytes % 256 == 0 && (!conv_small() || !is.h2 || is.h2->pieces.marked)) {
+                st = storage_h2(ctx, is, conv_small());
                 hold_a = is.h2;
                 at = img_shape.offset;
-            } else {  // the storage's groups of 64 are not the image's: pieces of the image alone, laid out like it
+            } else {  // the storage's groups of 64 are not the image's (or were made for other readers): pieces of the image alone, laid out like it
                 if (is.planes_only) return ctx.fail(SAGE_ERR_INVALID, "internal: a tensor without fp32 values reached a convolution that has to gather it");
                 k::SplitView v;
                 v.rows = img[0] * img[1] * img[2];
                 v.cols = v.ld = img[3];
-                st = gather_h2(ctx, x[0], false, v, false, &is.h2_view);
+                st = gather_h2(ctx, x[0], false, v, false, &is.h2_view, conv_small());
                 hold_a = is.h2_view;
             }
             if (st) return st;
@@ -713,6 +718,15 @@ struct GemmOp : Operator {
             g.a.hi = hold_a->pieces.hi + at;
             g.a.plane = hold_a->pieces.plane;
             g.a.scale = hold_a->pieces.scale + at / 64;
+            if (conv_small()) {
+                if (is.planes_only) return ctx.fail(SAGE_ERR_INVALID, "internal: a tensor without fp32 values reached a small convolution");
+                g.a.marked = hold_a->pieces.marked + at / 64;
+                g.a_f32 = (const float *)x[0].ptr();
+                g.b_f32 = (const float *)x[1].ptr();
+                const Array &fs = x[1].desc.shape.strides;
+                g.b_k = fs[fs.size() - (tb ? 1 : 2)];
+                g.b_n = fs[fs.size() - (tb ? 2 : 1)];
+            }
             g.img_n = img[0];
             g.img_h = img[1];
             g.img_w = img[2];
@@ -725,7 +739,7 @@ struct GemmOp : Operator {
             if (st) return st;
             if (g.a.nb0 * g.a.nb1 != batch) return ctx.fail(SAGE_ERR_INVALID, "gemm: operand batch extents differ from the operator's");
         }
-        st = make_h2_operand(ctx, x[1], !tb, true, &g.b, &hold_b);
+        st = make_h2_operand(ctx, x[1], !tb, true, &g.b, &hold_b, conv && conv_small());
         if (st) return st;
         if (g.b.nb0 * g.b.nb1 != batch) return ctx.fail(SAGE_ERR_INVALID, "gemm: operand batch extents differ from the operator's");
         g.c = (float *)y->ptr();
@@ -734,13 +748,14 @@ struct GemmOp : Operator {
         g.sc1 = folded ? sc1 : 0;
         g.nbc0 = folded ? nbc0 : batch;
         k::PlaneOut o;
-        st = attach_forms(ctx, y, emit, emit_h2, &o);
+        st = attach_forms(ctx, y, emit, emit_h2, &o, mark);
         if (st) return st;
         g.c_hi = o.hi;
         g.c_plane = o.plane;
         g.h_hi = o.h2;
         g.h_plane = o.h2_plane;
         g.h_scale = o.h2_scale;
+        g.h_marked = o.h2_marked;
         g.naux = naux();
         g.epilogue = epilogue;
         long long e_nb0 = batch;
@@ -1208,6 +1223,15 @@ std::shared_ptr<Operator> gemm_on_h2(const Operator &op, bool a_given, bool tc_e
 bool gemm_is_h2(const Operator &op) {  // reads its operands in half-precision pieces
     const GemmOp *g = as_gemm(op);
     return (g && (g->h2 || g->attn)) || grouped_gemm_is_h2(op);
+}
+// Does it want to know of its image's groups what the pieces have not room for, and have the fp32 values for those?
+bool gemm_reads_wide(const Operator &op) {
+    const GemmOp *g = as_gemm(op);
+    return g && g->h2 && g->conv && g->conv_small();
+}
+bool gemm_emits_wide(const Operator &op) {
+    const GemmOp *g = as_gemm(op);
+    return g && g->h2 && !g->attn;
 }
 // Does an operator that runs on half-precision pieces write its result in them?  (Whole groups of 64 columns.)
 bool gemm_emits_h2(const Operator &op) {

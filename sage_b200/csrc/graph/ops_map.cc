@@ -51,7 +51,7 @@ std::string map_expr_text(const MapExpr &e) {
 
 // ops_gemm.cc
 sage_status storage_planes_attach(Context &ctx, Storage &st);
-sage_status storage_h2_attach(Context &ctx, Storage &st);
+sage_status storage_h2_attach(Context &ctx, Storage &st, bool wide);
 
 struct MapOp : Operator {
     MapExpr expr;
@@ -66,7 +66,8 @@ struct MapOp : Operator {
 
     sage_status compute(const std::vector<Tensor> &x, Context &ctx, Tensor *y) override {
         const bool emit = ctx.hint_emit_planes && out.dtype == SAGE_F32, emit_h2 = ctx.hint_emit_h2 && out.dtype == SAGE_F32;
-        ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = false;
+        const bool wide = ctx.hint_mark_wide;
+        ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = ctx.hint_mark_wide = false;
         sage_status st = Tensor::uninit(ctx, out, y);
         if (st) return st;
         k::PlaneOut planes;
@@ -77,11 +78,12 @@ struct MapOp : Operator {
             planes.plane = y->data->split->plane;
         }
         if (emit_h2) {
-            st = storage_h2_attach(ctx, *y->data);
+            st = storage_h2_attach(ctx, *y->data, wide);
             if (st) return st;
             planes.h2 = y->data->h2->pieces.hi;
             planes.h2_plane = y->data->h2->pieces.plane;
             planes.h2_scale = y->data->h2->pieces.scale;
+            planes.h2_marked = y->data->h2->pieces.marked;
         }
         if (text.empty()) text = map_expr_text(expr);
         std::vector<MapOperand> operands(x.size());

@@ -10,7 +10,7 @@ using namespace ops;
 
 // ops_gemm.cc
 sage_status storage_planes_attach(Context &ctx, Storage &st);
-sage_status storage_h2_attach(Context &ctx, Storage &st);
+sage_status storage_h2_attach(Context &ctx, Storage &st, bool wide);
 sage_status storage_h2(Context &ctx, Storage &st);
 
 enum RowKind { RSoftmax, RLse, RLayerNorm };
@@ -45,7 +45,7 @@ struct RowOp : Operator {
             planes.plane = y->data->split->plane;
         }
         if (emit_h2) {
-            st = storage_h2_attach(ctx, *y->data);
+            st = storage_h2_attach(ctx, *y->data, false);
             if (st) return st;
             planes.h2 = y->data->h2->pieces.hi;
             planes.h2_plane = y->data->h2->pieces.plane;

@@ -28,6 +28,7 @@ struct Node {
     std::vector<Node> args;
     bool emit_planes = false;      // a tensor-core GEMM reads the result: ask the operator for its tf32 planes ...
     bool emit_h2 = false;          // ... or for its half-precision pieces
+    bool mark_wide = false;        // ... and for which of their groups are wide
     std::shared_ptr<Node> shared;  // a node several parents read (a grouped GEMM): evaluated once per routine run,
                                    // and passed to `op` as its only operand
     bool visited = false;          // traversal mark for shared nodes
@@ -484,6 +485,9 @@ bool map_op_emits_planes(const Operator &op);
 static bool can_emit_planes(const Operator &op, bool tc) {
     return gemm_runs_on_tc(op, tc) || row_op_emits_planes(op) || is_grouped_gemm_op(op) || (tc && (map_op_emits_planes(op) || im2col_op_emits_planes(op)));
 }
+bool gemm_reads_wide(const Operator &op);
+bool gemm_emits_wide(const Operator &op);
+static bool can_mark_wide(const Operator &op) { return gemm_emits_wide(op) || map_op_emits_h2(op) || pool_op_emits_h2(op); }
 static bool can_emit_h2(const Operator &op) { return gemm_emits_h2(op) || row_op_emits_h2(op) || map_op_emits_h2(op) || pool_op_emits_h2(op); }
 
 // Products with weights run on half-precision pieces, unless the program also multiplies by the transposes of its activations (training):
@@ -575,21 +579,23 @@ static void group_gemms(Node &root) {
     }
 }
 
-static void mark_plane_readers(Node &n, bool tc, std::unordered_set<Origin *> *states, std::unordered_set<Origin *> *h2_states) {
+static void mark_plane_readers(Node &n, bool tc, std::unordered_set<Origin *> *states, std::unordered_set<Origin *> *h2_states, std::unordered_set<Origin *> *wide_states) {
     if (n.is_data) return;
     if (n.shared && !n.shared->visited) {
         n.shared->visited = true;
-        mark_plane_readers(*n.shared, tc, states, h2_states);
+        mark_plane_readers(*n.shared, tc, states, h2_states, wide_states);
     }
-    for (Node &a : n.args) mark_plane_readers(a, tc, states, h2_states);
+    for (Node &a : n.args) mark_plane_readers(a, tc, states, h2_states, wide_states);
     const bool grouped = is_grouped_gemm_op(*n.op);
     if (!grouped && (!is_gemm_op(*n.op) || !gemm_runs_on_tc(*n.op, tc))) return;
-    const bool h2 = gemm_is_h2(*n.op);
+    const bool h2 = gemm_is_h2(*n.op), wide = gemm_reads_wide(*n.op);
     for (int idx = 0; idx < (is_attention_op(*n.op) ? 3 : grouped || h2 ? 1 : 2); ++idx) {
         long long offset = 0;
         Node *p = skip_views(&n.args[idx], &offset);
         if (p->is_data) {
-            if (p->var.is_op() && gemm_operand_static_direct(*n.op, idx, offset)) (h2 ? h2_states : states)->insert(p->var.key());
+            if (p->var.is_op() && gemm_operand_static_direct(*n.op, idx, offset)) (wide ? wide_states : h2 ? h2_states : states)->insert(p->var.key());
+        } else if (wide) {  // (it reads the fp32 values of wide groups: they stay)
+            if (can_mark_wide(*p->op) && gemm_operand_static_direct(*n.op, idx, offset)) p->emit_h2 = p->mark_wide = true;
         } else if (h2 ? can_emit_h2(*p->op) : can_emit_planes(*p->op, tc)) {
             // Inside a routine's tree a node has one reader, so this GEMM is the only one — unless the
             // node is shared (a grouped product): then every slab must end in a GEMM operand.
@@ -835,7 +841,7 @@ static std::unique_ptr<Program> compile(const std::vector<Var> &x, std::vector<V
         p->routines.emplace(node.key(), std::move(r));
     }
     if (pattern) {
-        std::unordered_set<Origin *> plane_states, h2_states;
+        std::unordered_set<Origin *> plane_states, h2_states, wide_states;  // (a state that both kinds of pieces are asked of is marked)
         if (tc) {
             bool tf32 = false;
             for (auto &kv : p->routines) tf32 = tf32 || (!kv.second.row && any_needs_tf32(kv.second.root, tc));
@@ -844,9 +850,9 @@ static std::unique_ptr<Program> compile(const std::vector<Var> &x, std::vector<V
                 for (auto &kv : p->routines) assign_h2(kv.second, tc, *p, &done);
         }
         for (auto &kv : p->routines)
-            if (!kv.second.row) mark_plane_readers(kv.second.root, tc, &plane_states, &h2_states);
-        for (int form = 0; form < 2; ++form) {
-            for (Origin *key : form ? h2_states : plane_states) {
+            if (!kv.second.row) mark_plane_readers(kv.second.root, tc, &plane_states, &h2_states, &wide_states);
+        for (int form = 0; form < 3; ++form) {
+            for (Origin *key : form == 2 ? wide_states : form ? h2_states : plane_states) {
                 // A state that is only a view of another state (reshape(state)) shares its storage, and planes
                 // belong to the storage: ask the state that really produces the values.
                 auto it = p->routines.find(key);
@@ -862,7 +868,8 @@ static std::unique_ptr<Program> compile(const std::vector<Var> &x, std::vector<V
                     continue;
                 }
                 Node *root = skip_views(&it->second.root);
-                if (!root->is_data && form && can_emit_h2(*root->op)) root->emit_h2 = true;
+                if (!root->is_data && form == 1 && can_emit_h2(*root->op)) root->emit_h2 = true;
+                if (!root->is_data && form == 2 && can_mark_wide(*root->op)) root->emit_h2 = root->mark_wide = true;
                 if (!root->is_data && !form && can_emit_planes(*root->op, tc)) root->emit_planes = true;
             }
         }
@@ -926,8 +933,9 @@ static sage_status run_node(const Node &n, Context &ctx, Session &s, const Value
     ctx.hint_emit_planes = n.emit_planes;
     ctx.hint_emit_h2 = n.emit_h2;
     ctx.hint_planes_only = (n.emit_planes || n.emit_h2) && n.planes_only;
+    ctx.hint_mark_wide = n.mark_wide;
     sage_status st = n.op->compute(args, ctx, out);
-    ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = false;
+    ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = ctx.hint_mark_wide = false;
     return st;
 }
 

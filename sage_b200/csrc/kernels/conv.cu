@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(256) col2im_quads_kernel(const float *__restri
 // for the cache each time (3 x 3 over 256 x 112 x 112 x 64: 358 us and a split pass of 62 -> 264 with pieces; 7 x 7
 // over 7 x 7 x 512 of one image, between events: 20.5 -> 12.7).  With pieces
 // asked for, 16 threads hold the 64 channels of a group: no split pass reads the result again.
-template <int VEC, class I>
+template <int VEC, class I, bool MARK>
 __global__ void __launch_bounds__(256) pool2d_kernel(const float *__restrict__ img, float *__restrict__ out, ConvP p,
                                                      long long total, int is_max, int ref_compat, PlaneOut forms) {
     grid_dependency_sync();
@@ -310,6 +310,12 @@ __global__ void __launch_bounds__(256) pool2d_kernel(const float *__restrict__ i
             *reinterpret_cast<uint2 *>(forms.h2 + at) = h;
             *reinterpret_cast<uint2 *>(forms.h2 + forms.h2_plane + at) = l;
             if ((threadIdx.x & 15) == 0) forms.h2_scale[at >> 6] = scale;
+            if (MARK) {
+                unsigned low1 = min(min(h2_low1(o.x), h2_low1(o.y)), min(h2_low1(o.z), h2_low1(o.w)));
+#pragma unroll
+                for (int off = 8; off > 0; off >>= 1) low1 = min(low1, __shfl_xor_sync(lanes, low1, off));
+                if ((threadIdx.x & 15) == 0) forms.h2_marked[at >> 6] = h2_wide(low1, f) ? -scale : scale;
+            }
         }
     }
 }
@@ -583,9 +589,10 @@ sage_status pool2d(Context &ctx, bool is_max, const float *img, float *out, long
     if (forms.h2 && !(vec && pool2d_writes_pieces(img, chan, out_h, out_w))) return ctx.fail(SAGE_ERR_INVALID, "pool2d: half-precision pieces need whole groups of channels");
     // 32-bit indices where they reach: two 64-bit divisions were a third of a thread's instructions
     const bool narrow = total < (1LL << 31) && img_h * img_w * chan < (1LL << 31);
-    auto kernel = narrow ? pool2d_kernel<4, unsigned> : pool2d_kernel<4, long long>;
+    const bool mark = forms.h2 && forms.h2_marked;
+    auto kernel = narrow ? (mark ? pool2d_kernel<4, unsigned, true> : pool2d_kernel<4, unsigned, false>) : (mark ? pool2d_kernel<4, long long, true> : pool2d_kernel<4, long long, false>);
     if (vec) launch_dependent(ctx.pdl, ctx.stream(), kernel, dim3(grid_for(ctx, total / 4)), dim3(256), 0, img, out, p, total / 4, is_max ? 1 : 0, (int)ctx.opts().ref_compat, forms);
-    else launch_dependent(ctx.pdl, ctx.stream(), pool2d_kernel<1, long long>, dim3(grid_for(ctx, total)), dim3(256), 0, img, out, p, total, is_max ? 1 : 0, (int)ctx.opts().ref_compat, forms);
+    else launch_dependent(ctx.pdl, ctx.stream(), pool2d_kernel<1, long long, false>, dim3(grid_for(ctx, total)), dim3(256), 0, img, out, p, total, is_max ? 1 : 0, (int)ctx.opts().ref_compat, forms);
     return ctx.check_cuda(cudaGetLastError(), "pool2d launch");
 }
 

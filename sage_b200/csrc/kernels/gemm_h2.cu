@@ -37,8 +37,9 @@ bool aligned16(const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0;
 
 // ---------------------------------------------------------------------------------- operand forms
 // Flat: 16 lanes hold the 64 floats of a group.  Bound by memory: 4 bytes read, 4.06 written per element.
+template <bool MARK>
 __global__ void __launch_bounds__(256) split_h2_flat_kernel(const float4 *__restrict__ src, long long n4, uint2 *__restrict__ hi, uint2 *__restrict__ lo,
-                                                            float *__restrict__ scale) {
+                                                            float *__restrict__ scale, float *__restrict__ marked) {
     grid_dependency_sync();
     for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < n4; g += (long long)gridDim.x * blockDim.x) {
         const float4 x = src[g];  // n4 is a multiple of 16: the lanes of a group are all here or all gone
@@ -54,6 +55,12 @@ __global__ void __launch_bounds__(256) split_h2_flat_kernel(const float4 *__rest
         hi[g] = h;
         lo[g] = l;
         if ((threadIdx.x & 15) == 0) scale[g >> 4] = s;
+        if (MARK) {
+            unsigned low1 = min(min(h2_low1(x.x), h2_low1(x.y)), min(h2_low1(x.z), h2_low1(x.w)));
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) low1 = min(low1, __shfl_xor_sync(lanes, low1, o));
+            if ((threadIdx.x & 15) == 0) marked[g >> 4] = h2_wide(low1, f) ? -s : s;
+        }
     }
 }
 
@@ -146,7 +153,15 @@ __device__ __forceinline__ void store_row(const float (&y)[16], float factor, un
 struct SplitOut {
     unsigned short *hi;
     float *scale, *ratio;
+    float *marked;  // MARK
+    unsigned long long *columns;
 };
+__device__ __forceinline__ unsigned row_low1(const float (&y)[16]) {
+    unsigned low1 = 0xffffffffu;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) low1 = min(low1, h2_low1(y[i]));
+    return low1;
+}
 
 // A thread's four 16-byte loads of a tile: of one row (its columns contiguous; as tile_row has them), or of four rows and two pairs
 // of columns.  `at`: its first one, null for rows outside; `left`: columns from there to the view's end.
@@ -172,6 +187,7 @@ __device__ __forceinline__ const float *batch_of(const ViewP &v, unsigned b) {
 }
 
 // Operand A: a scale per row and 64 columns.  A block takes `run` tiles side by side, the next one's rows on their way.
+template <bool MARK>
 __device__ __forceinline__ void split_tiles(const ViewP &v, const SplitOut &o, unsigned block, int run, float (*tile)[65]) {
     const unsigned runs = (unsigned)(v.col_tiles + run - 1) / run, line = block / runs, b = line / (unsigned)v.row_tiles;
     const int first = (int)(block - line * runs) * run, last = min(v.col_tiles, first + run);
@@ -194,8 +210,17 @@ __device__ __forceinline__ void split_tiles(const ViewP &v, const SplitOut &o, u
             tile_row(tile, y);
         }
         const float f = h2_factor(row_amax(y), &scale);
+        [[maybe_unused]] bool wide = false;
+        if (MARK) {
+            unsigned low1 = row_low1(y);
+            low1 = min(low1, __shfl_xor_sync(0xffffffffu, low1, 1));
+            wide = h2_wide(min(low1, __shfl_xor_sync(0xffffffffu, low1, 2)), f);
+        }
         if (!in) continue;
-        if ((threadIdx.x & 3) == 0) o.scale[at_row * v.col_tiles + t] = scale;
+        if ((threadIdx.x & 3) == 0) {
+            o.scale[at_row * v.col_tiles + t] = scale;
+            if (MARK) o.marked[at_row * v.col_tiles + t] = wide ? -scale : scale;
+        }
         store_row(y, f, o.hi + at_row * v.pitch + t * 64 + c, v.plane, (int)v.pitch - t * 64 - c);
     }
 }
@@ -233,7 +258,7 @@ __device__ __forceinline__ float largest_finite4(float a, float b, float c, floa
 __device__ __forceinline__ bool is_finite(float m) { return m < __uint_as_float(0x7f800000u); }
 
 enum { kRowsAny, kRowsOne, kRowsFour };  // a thread's loads: single elements; 16 bytes of one row; 16 bytes of four rows
-template <int LOADS>
+template <int LOADS, bool MARK>
 __device__ __forceinline__ void split_rows(const ViewP &v, const SplitOut &o, unsigned block, int ctas, int tiles_per_cta, int span, RowsShared &sh) {
     const unsigned group = block / (unsigned)ctas, rank = block - group * ctas, b = group / (unsigned)v.row_tiles;
     const long long r0 = (long long)(group - b * v.row_tiles) * 64;
@@ -370,8 +395,26 @@ __device__ __forceinline__ void split_rows(const ViewP &v, const SplitOut &o, un
     const int part = (threadIdx.x & 3) * 8;
     unsigned short *d = o.hi + at_row * v.pitch + part;
     float *ratio = o.ratio + (long long)group * v.col_tiles;
+    // 2^f: a tile's factor
+    const auto factor_of = [&](int t) {
+        const int top = sh.tile_top[span == 1 ? t - first : (t - first) / span];
+        return top == 0 ? 0 : max(top - all, -kH2Far);
+    };
+    [[maybe_unused]] float *marked = MARK ? o.marked + (long long)group * v.col_tiles : nullptr;
+    [[maybe_unused]] unsigned long long *columns = MARK ? o.columns + (long long)group * v.col_tiles : nullptr;
+    if (MARK) {  // none, before the first thread that finds one
+        for (int t = first + threadIdx.x; t < last; t += 256) {
+            marked[t] = __uint_as_float((unsigned)(127 + factor_of(t)) << 23);
+            columns[t] = 0;
+        }
+        __syncthreads();
+    }
+    [[maybe_unused]] const auto mark = [&](int t, unsigned long long rows) {
+        atomicOr(reinterpret_cast<unsigned *>(marked + t), 0x80000000u);
+        atomicOr(columns + t, rows);
+    };
     for (int t = last - 1; t >= first; --t) {
-        const int top = sh.tile_top[span == 1 ? t - first : (t - first) / span], f = top == 0 ? 0 : max(top - all, -kH2Far);  // 2^f: this tile's factor
+        const int f = factor_of(t);
         if (threadIdx.x == 0) ratio[t] = __uint_as_float((unsigned)(127 + f) << 23);
         float factor[4];
 #pragma unroll
@@ -393,6 +436,13 @@ __device__ __forceinline__ void split_rows(const ViewP &v, const SplitOut &o, un
                         if (j == 3) q[i].w *= up;
                     }
                 }
+            }
+            if (MARK) {
+                unsigned rows = h2_wide(min(min(h2_low1(q[0].x), h2_low1(q[1].x)), min(h2_low1(q[2].x), h2_low1(q[3].x))), factor[0]) ? 1u : 0u;
+                rows |= h2_wide(min(min(h2_low1(q[0].y), h2_low1(q[1].y)), min(h2_low1(q[2].y), h2_low1(q[3].y))), factor[1]) ? 2u : 0u;
+                rows |= h2_wide(min(min(h2_low1(q[0].z), h2_low1(q[1].z)), min(h2_low1(q[2].z), h2_low1(q[3].z))), factor[2]) ? 4u : 0u;
+                rows |= h2_wide(min(min(h2_low1(q[0].w), h2_low1(q[1].w)), min(h2_low1(q[2].w), h2_low1(q[3].w))), factor[3]) ? 8u : 0u;
+                if (rows) mark(t, (unsigned long long)rows << r4);
             }
             unsigned *hi = reinterpret_cast<unsigned *>(sh.pieces[t & 1][0][r4]), *lo = reinterpret_cast<unsigned *>(sh.pieces[t & 1][1][r4]);
 #pragma unroll
@@ -443,6 +493,7 @@ __device__ __forceinline__ void split_rows(const ViewP &v, const SplitOut &o, un
 #pragma unroll
                 for (int i = 0; i < 16; ++i) y[i] *= up;
             }
+            if (MARK && h2_wide(row_low1(y), factor[0])) mark(t, 1ull << row);
             if (row_in) store_row(y, factor[0], d + t * 64, v.plane, (int)v.pitch - t * 64 - part);
         }
     }
@@ -458,30 +509,31 @@ struct SplitPair {
     unsigned b_blocks, a_blocks;
     int ctas, tiles_per_cta, span, run;
 };
+template <bool MARK>
 __global__ void __launch_bounds__(256, 4) split_h2_kernel(const __grid_constant__ SplitPair p) {
     __shared__ RowsShared sh;
     grid_dependency_sync();
     const unsigned block = blockIdx.x;
     if (block < p.b_blocks) {
-        if (!p.b.vec) split_rows<kRowsAny>(p.b, p.out_b, block, p.ctas, p.tiles_per_cta, p.span, sh);
-        else if (p.b.cs == 1) split_rows<kRowsOne>(p.b, p.out_b, block, p.ctas, p.tiles_per_cta, p.span, sh);
-        else split_rows<kRowsFour>(p.b, p.out_b, block, p.ctas, p.tiles_per_cta, p.span, sh);
+        if (!p.b.vec) split_rows<kRowsAny, MARK>(p.b, p.out_b, block, p.ctas, p.tiles_per_cta, p.span, sh);
+        else if (p.b.cs == 1) split_rows<kRowsOne, MARK>(p.b, p.out_b, block, p.ctas, p.tiles_per_cta, p.span, sh);
+        else split_rows<kRowsFour, MARK>(p.b, p.out_b, block, p.ctas, p.tiles_per_cta, p.span, sh);
     } else if (block - p.b_blocks < p.a_blocks) {
-        split_tiles(p.a, p.out_a, block - p.b_blocks, p.run, sh.tiles[0]);
+        split_tiles<MARK>(p.a, p.out_a, block - p.b_blocks, p.run, sh.tiles[0]);
     }
 }
 
 }  // namespace
 
-sage_status split_h2_flat(Context &ctx, const float *src, long long n, unsigned short *hi, long long plane, float *scale) {
+sage_status split_h2_flat(Context &ctx, const float *src, long long n, unsigned short *hi, long long plane, float *scale, float *marked) {
     ctx.note_launch(ctx.verbose_names ? "split_h2" : "split_tf32");  // launch lists have one name for an operand's split
     if (ctx.dry()) return SAGE_OK;
     if (!aligned16(src) || !aligned16(hi) || plane % 8 || n % 64) return ctx.fail(SAGE_ERR_INVALID, "split_h2_flat: unaligned");
     long long blocks = (n / 4 + 255) / 256;
     const long long cap = (long long)ctx.sm_count * 16;
     if (blocks > cap) blocks = cap;
-    return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), split_h2_flat_kernel, dim3((unsigned)(blocks < 1 ? 1 : blocks)), dim3(256), 0,
-                                           reinterpret_cast<const float4 *>(src), n / 4, reinterpret_cast<uint2 *>(hi), reinterpret_cast<uint2 *>(hi + plane), scale),
+    return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), marked ? split_h2_flat_kernel<true> : split_h2_flat_kernel<false>, dim3((unsigned)(blocks < 1 ? 1 : blocks)), dim3(256), 0,
+                                           reinterpret_cast<const float4 *>(src), n / 4, reinterpret_cast<uint2 *>(hi), reinterpret_cast<uint2 *>(hi + plane), scale, marked),
                           "split_h2_flat launch");
 }
 
@@ -506,14 +558,14 @@ static sage_status split_views(Context &ctx, const float *src_a, const SplitView
     p.ctas = p.tiles_per_cta = p.span = p.run = 1;
     if (va) {
         p.a = view_params(src_a, *va, out_a);
-        p.out_a = SplitOut{out_a.hi, out_a.scale, nullptr};
+        p.out_a = SplitOut{out_a.hi, out_a.scale, nullptr, out_a.marked, nullptr};
         const long long lines = va->nb0 * va->nb1 * p.a.row_tiles, fill = (long long)ctx.sm_count * 16;
         while (p.run < 8 && lines * p.a.col_tiles >= fill * p.run * 2) p.run *= 2;  // as long as the chip is filled several times over
         a_blocks = lines * ((p.a.col_tiles + p.run - 1) / p.run);
     }
     if (vb) {
         p.b = view_params(src_b, *vb, out_b);
-        p.out_b = SplitOut{out_b.hi, out_b.scale, out_b.ratio};
+        p.out_b = SplitOut{out_b.hi, out_b.scale, out_b.ratio, out_b.marked, out_b.columns};
         while (p.ctas < 8 && p.ctas * 2 <= p.b.col_tiles) p.ctas *= 2;
         p.tiles_per_cta = (p.b.col_tiles + p.ctas - 1) / p.ctas;
         p.span = (p.tiles_per_cta + kFactors - 1) / kFactors;
@@ -527,7 +579,7 @@ static sage_status split_views(Context &ctx, const float *src_a, const SplitView
     if (va && vb) ctx.note_part(name);
     ctx.note_launch(name);
     if (ctx.dry()) return SAGE_OK;
-    return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), p.ctas, split_h2_kernel, dim3((unsigned)blocks), dim3(256), 0, p), "split_h2 launch");
+    return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), p.ctas, out_a.marked || out_b.marked ? split_h2_kernel<true> : split_h2_kernel<false>, dim3((unsigned)blocks), dim3(256), 0, p), "split_h2 launch");
 }
 
 sage_status split_h2_rows_at(Context &ctx, const float *src, const SplitView &v, const H2Split &out) { return split_views(ctx, nullptr, nullptr, H2Split(), src, &v, out); }
@@ -543,11 +595,18 @@ static H2Split split_layout(const SplitView &v, void *dst) {
     return out;
 }
 
-sage_status split_h2_view(Context &ctx, const float *src, const SplitView &v, bool whole_rows, H2Split *out) {
-    Block *block = ctx.allocator().alloc(split_h2_bytes(v.nb0 * v.nb1, v.rows, v.cols, whole_rows));
+sage_status split_h2_view(Context &ctx, const float *src, const SplitView &v, bool whole_rows, H2Split *out, bool mark) {
+    const size_t bytes = split_h2_bytes(v.nb0 * v.nb1, v.rows, v.cols, whole_rows);
+    const long long marks = mark ? v.nb0 * v.nb1 * (whole_rows ? (v.rows + 63) / 64 : v.rows) * ((v.cols + 63) / 64) : 0;
+    Block *block = ctx.allocator().alloc(bytes + (size_t)marks * (whole_rows ? 12 : 4));
     if (!block) return ctx.fail(SAGE_ERR_OOM, "out of memory for an operand in half-precision pieces");
     *out = split_layout(v, block->ptr);
     out->block = block;
+    if (mark) {
+        char *at = block->ptr + bytes;  // (a multiple of 256)
+        if (whole_rows) out->columns = reinterpret_cast<unsigned long long *>(at);
+        out->marked = reinterpret_cast<float *>(at + (whole_rows ? marks * 8 : 0));
+    }
     return whole_rows ? split_views(ctx, nullptr, nullptr, H2Split(), src, &v, *out) : split_views(ctx, src, &v, *out, nullptr, nullptr, H2Split());
 }
 
@@ -615,13 +674,13 @@ static bool encode_halo(PFN_encodeTiled encode, const H2Gemm &g, const unsigned 
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Images below 128 KiB (of fp32) are read through tiled boxes instead of im2col-mode maps: `rows` whole output rows of one image to
-// a tile, or `imgs` whole images where several fit its 128 pixels.
+// Images below 128 KiB (of fp32) are read through tiled boxes instead of im2col-mode maps or windows kept in shared memory: `rows` whole
+// output rows of one image to a tile, or `imgs` whole images where several fit its 128 pixels.
 struct BoxPlan {
     int imgs, rows, row_tiles;  // row_tiles: of an image
     long long tiles(const H2Gemm &g) const { return (g.img_n + imgs - 1) / imgs * row_tiles; }
 };
-static bool box_wanted(const H2Gemm &g) { return g.conv && g.img_n * g.img_h * g.img_w * g.img_c * 4 < 131072; }
+static bool box_wanted(const H2Gemm &g) { return g.conv && conv_h2_small(g.img_n, g.img_h, g.img_w, g.img_c); }
 static bool box_plan(const H2Gemm &g, BoxPlan *plan) {
     if (g.out_w > BM || (g.out_w - 1) * g.win.stride_w + 1 > 256) return false;
     long long r = BM / g.out_w;
@@ -662,7 +721,7 @@ bool conv_h2_ok(const H2Gemm &g) {
 static bool halo_plan(const H2Gemm &g, int *wb, int *rows) {
     const char *env = getenv("SAGE_CONV_HALO");
     const Window &w = g.win;
-    if ((env && atoi(env) == 0) || !g.conv || w.stride_w != 1 || w.stride_h != 1 || w.dil_w != 1 || w.dil_h != 1) return false;
+    if ((env && atoi(env) == 0) || !g.conv || box_wanted(g) || w.stride_w != 1 || w.stride_h != 1 || w.dil_w != 1 || w.dil_h != 1) return false;
     if (w.ker_w * w.ker_h < 2 || g.n > 128 || g.n % 32) return false;
     const long long b = g.out_w + w.ker_w - 1;
     if (b > 128) return false;
@@ -828,7 +887,7 @@ static SlicePlan plan_slices(const Context &ctx, const H2Gemm &g) {
     BoxPlan box{};
     int wb = 0, halo_rows = 0;
     const bool halo = halo_plan(g, &wb, &halo_rows), boxed = box_wanted(g) && box_plan(g, &box);
-    const int ctas = (pairs_on() && g.m > BM && (halo || !boxed)) ? 2 : 1;
+    const int ctas = (pairs_on() && g.m > BM && !boxed) ? 2 : 1;
     double best = 1e300, whole = 1e300, store = 3.5;
     for (int i = 0; i < g.naux; ++i)
         if (g.aux[i].sr != 0) store = 8.5;
@@ -881,7 +940,7 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
     int halo_wb = 0, halo_r = 0;
     const bool halo = !sliced && halo_plan(g, &halo_wb, &halo_r);
     BoxPlan box{};
-    const bool boxed = !halo && box_wanted(g) && box_plan(g, &box);
+    const bool boxed = box_wanted(g) && box_plan(g, &box);
     const int ctas = (pairs_on() && g.m > BM && !sliced && !boxed) ? 2 : 1;
     ColumnPlan cols = sliced ? ColumnPlan{cut.bn, 0, 0} : plan_columns(ctx, boxed ? box.tiles(g) * BM : g.m, g.n, g.batch, ctas);
     if (halo) cols = ColumnPlan{g.n <= 64 ? 64 : 128, 0, 0};  // all output channels in one tile: the window is loaded once
@@ -903,6 +962,7 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
     p.h_hi = g.h_hi;
     p.h_plane = g.h_plane;
     p.h_scale = g.h_scale;
+    p.h_marked = g.h_marked;
     p.ldc = g.ldc;
     p.sc0 = g.sc0;
     p.sc1 = g.sc1;
@@ -957,11 +1017,19 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
         p.num_tiles = p.tiles_m * p.tiles_n;
     }
     if (boxed) {
+        if (!g.a.marked || !g.b.marked || !g.b.columns || !g.a_f32 || !g.b_f32) return ctx.fail(SAGE_ERR_INVALID, "gemm_h2: a small convolution without its wide groups");
         p.box_imgs = box.imgs;
         p.box_r = box.rows;
         p.box_rt = box.row_tiles;
         p.box_bytes = (int)(box.imgs * box.rows * g.out_w) * HK * 2;
         p.tiles_m = (int)box.tiles(g);
+        p.sa = g.a.marked;
+        p.sb_ratio = g.b.marked;
+        p.b_columns = g.b.columns;
+        p.a_f32 = g.a_f32;
+        p.b_f32 = g.b_f32;
+        p.b_k = g.b_k;
+        p.b_n = g.b_n;
         p.num_tiles = p.tiles_m * p.tiles_n;
     }
     const bool vec = g.n % 4 == 0 && g.ldc % 4 == 0 && g.sc0 % 4 == 0 && g.sc1 % 4 == 0 && (!g.c || aligned16(g.c)) && (!g.c_hi || (aligned16(g.c_hi) && g.c_plane % 4 == 0));
@@ -985,7 +1053,7 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
     const int slots = ctx.sm_count / ctas, grid = sliced ? cut.slices * p.num_tiles : ctas * (p.num_tiles < slots ? p.num_tiles : slots);
     const int threads = sliced ? 64 + 2 * bn : kThreads;
 
-    const int out_mask = (g.c ? 1 : 0) | (g.c_hi ? 2 : 0) | (g.h_hi ? 4 : 0);
+    const int out_mask = (g.c ? 1 : 0) | (g.c_hi ? 2 : 0) | (g.h_hi ? 4 : 0) | (g.h_hi && g.h_marked ? 8 : 0);
     char num[96];
     snprintf(num, sizeof num, "gemm_h2 %d %d %d %d %d %d %d %d %d\n", bn, ctas, sliced ? 1 : 0, aux_vec ? 1 : 0, g.conv ? (halo ? 2 : boxed ? 3 : 1) : 0, g.naux, rowinv, per_col, out_mask);
     const bool plain = !g.conv && g.naux == 0 && g.epilogue.empty() && out_mask == 1;

@@ -30,6 +30,7 @@ struct PlaneOut {
     unsigned short *h2 = nullptr;
     long long h2_plane = 0;
     float *h2_scale = nullptr;
+    float *h2_marked = nullptr;  // the scales again, negative where a group is wide (gemm_h2_device.inc), for a reader that asks
 };
 
 // reduce.cu — ReduceOperator / ReduceArgOperator (src/ops/reduce.rs:258-325, 372-431)
@@ -179,6 +180,8 @@ struct H2Operand {
     const float *scale = nullptr;
     long long s_row = 0, s_b0 = 0, s_b1 = 0;
     const float *ratio = nullptr;
+    const float *marked = nullptr;               // of a small convolution's operands: A's scales or B's factors with the wide ones negative
+    const unsigned long long *columns = nullptr;
 };
 struct H2Gemm {
     bool conv = false;        // A is the im2col of a contiguous NHWC image (a.hi, a.plane, a.scale) with C % 64 == 0
@@ -191,6 +194,9 @@ struct H2Gemm {
     unsigned short *h_hi = nullptr;       // ... and / or in half-precision pieces: needs n, ldc, sc0, sc1 multiples of 64
     long long h_plane = 0;
     float *h_scale = nullptr;
+    float *h_marked = nullptr;
+    const float *a_f32 = nullptr, *b_f32 = nullptr;  // a small convolution (conv_h2_small): what the pieces were made from, the filter at
+    long long b_k = 0, b_n = 0;                      // [k * b_k + column * b_n]
     long long ldc = 0, sc0 = 0, sc1 = 0, nbc0 = 1;
     int naux = 0;
     TcAuxArg aux[3];
@@ -214,18 +220,24 @@ sage_status conv_first_run(Context &ctx, const H2Gemm &g, const FirstConv &f);
 size_t gemm_h2_scratch_bytes(const GemmArgs &g);
 sage_status gemm_h2(Context &ctx, const GemmArgs &g, void *scratch = nullptr);
 bool conv_h2_ok(const H2Gemm &g);
+// Images below 128 KiB (of fp32) are read through tiled boxes, and their wide groups worked out in fp32: both operands' pieces come
+// `marked`.
+inline bool conv_h2_small(long long n, long long h, long long w, long long c) { return n * h * w * c * 4 < 131072; }
 // Pieces of `n` consecutive floats (a multiple of 64), laid out like the source, a scale per 64.
-sage_status split_h2_flat(Context &ctx, const float *src, long long n, unsigned short *hi, long long plane, float *scale);
+sage_status split_h2_flat(Context &ctx, const float *src, long long n, unsigned short *hi, long long plane, float *scale, float *marked = nullptr);
 // Pieces of a strided view (b1, b0, row, col) gathered with its columns contiguous: [batch][rows][pitch], pitch = cols
-// rounded up to 8.  `whole_rows`: one scale per row and factors (operand B) instead of one per 64 columns.
+// rounded up to 8.  `whole_rows`: one scale per row and factors (operand B) instead of one per 64 columns.  `mark`: with
+// `marked`, A's scales or B's factors again with the wide ones negative, and of B `columns`, which of a block's 64 are wide.
 struct H2Split {
     Block *block = nullptr;
     unsigned short *hi = nullptr;
     float *scale = nullptr, *ratio = nullptr;
+    float *marked = nullptr;
+    unsigned long long *columns = nullptr;
     long long plane = 0, pitch = 0;
 };
 size_t split_h2_bytes(long long batches, long long rows, long long cols, bool whole_rows);
-sage_status split_h2_view(Context &ctx, const float *src, const SplitView &v, bool whole_rows, H2Split *out);
+sage_status split_h2_view(Context &ctx, const float *src, const SplitView &v, bool whole_rows, H2Split *out, bool mark = false);
 // Operand B straight into memory the caller laid out: rows of `out->pitch` at out->hi / out->hi + out->plane, out->scale.
 sage_status split_h2_rows_at(Context &ctx, const float *src, const SplitView &v, const H2Split &out);
 H2Operand h2_operand(const H2Split &s, long long batches, long long rows, long long cols, bool whole_rows);

@@ -190,6 +190,8 @@ public:
     bool hint_emit_planes = false, hint_emit_h2 = false;
     // ... and nothing else reads it: the producer may skip the fp32 store and write only those.
     bool hint_planes_only = false;
+    // ... and the reader of the pieces wants to know which groups they have not room for (a small convolution).
+    bool hint_mark_wide = false;
     int sm_count = 148;
 
 private:

@@ -343,6 +343,92 @@ def test_convolutions_of_images_below_128_kib(ctx, n, h, w, c, oc, ker, stride, 
     assert ctx.status_word() == 0
 
 
+def _conv_excess(got, x, f, stride, pad):
+    """Largest error over the bound at the top of the file, the chains of 16 and 4 fp32 terms of a wide group's 64 k (20 x 2^-24) with it."""
+    want, s = _conv64(x, f, stride, pad), _conv64(np.abs(x), np.abs(f), stride, pad)
+    bound = s * (2.0 ** -22 + 2.0 ** -24 + 12 * 2.0 ** -23 + (f[..., 0].size / 64 + 22) * 2.0 ** -24)
+    return float((np.abs(got - want) / np.maximum(bound, 1e-300)).max())
+
+
+def _spread(rng, n, span):
+    """Powers of two over `span` binades, the ends among them."""
+    e = rng.integers(0, span + 1, n)
+    e[:2] = 0, span
+    return (2.0 ** (span // 2 - rng.permutation(e))).astype(np.float32)
+
+
+# Slices of K and none; several images a tile; a window, columns two apart, a single tap; channels that end inside a tile of columns;
+# a filter whose columns are not loaded four at a time.
+@pytest.mark.parametrize("span", [20, 30, 60])
+@pytest.mark.parametrize("n,h,w,c,oc,ker,stride", [(1, 7, 7, 512, 512, 3, 1), (9, 5, 5, 64, 130, 3, 2), (1, 20, 23, 64, 192, 3, 1), (3, 6, 6, 192, 33, 1, 1), (1, 16, 16, 64, 64, 2, 1)])
+def test_small_images_whose_channels_lie_far_apart(ctx, n, h, w, c, oc, ker, stride, span):
+    """Channels of one group of 64 over up to 2^60, and a filter that makes up for it: every product counts, and keeps the bits it has in
+    single precision.  As an input, as a map's result, and as views that have to be gathered."""
+    rng = np.random.default_rng(span + oc)
+    d = _spread(rng, c, span)
+    x = (rng.uniform(0.5, 1, (n, h, w, c)) * rng.choice([-1, 0, 1], (n, h, w, c)) * d).astype(np.float32)
+    f = (rng.uniform(0.5, 1, (ker, ker, c, oc)) * rng.choice([-1, 1], (ker, ker, c, oc)) / d[:, None]).astype(np.float32)
+    pad = ker // 2 if ker % 2 else 0
+    xv, fv = ctx.var(x), ctx.var(f)
+    label = r"^gemm_tc_h2\[.*,conv,boxes"
+    for y in (S.conv_2d(xv, fv, stride, pad, 1), S.conv_2d(xv * 1.0, fv, stride, pad, 1)):
+        assert _conv_excess(evaluated(ctx, y, label), x, f, stride, pad) <= 1.0
+        ctx.clear()
+    flat = np.concatenate([np.ones(7, np.float32), x.ravel()])
+    y = S.conv_2d(S.view(ctx.var(flat).slice(0, 7, 7 + x.size), list(x.shape)), fv, stride, pad, 1)
+    assert _conv_excess(evaluated(ctx, y, label), x, f, stride, pad) <= 1.0
+    assert ctx.status_word() == 0
+
+
+def test_small_images_with_one_far_operand(ctx):
+    """A channel far above the others that no filter uses, and filters that lie far apart between such channels: the small ones count."""
+    rng = np.random.default_rng(7)
+    x, f = rng.uniform(-1, 1, (2, 9, 9, 128)).astype(np.float32), rng.uniform(-1, 1, (3, 3, 128, 96)).astype(np.float32)
+    x[..., 5] *= 2.0 ** 50
+    f[:, :, 5] = 0
+    assert _conv_excess(evaluated(ctx, S.conv_2d(ctx.var(x), ctx.var(f), 1, 1, 1), r"conv,boxes"), x, f, 1, 1) <= 1.0
+    x[..., 5], f[:, :, 5] = 0, 2.0 ** 50
+    f[..., 7] *= np.float32(2.0 ** -60)
+    assert _conv_excess(evaluated(ctx, S.conv_2d(ctx.var(x), ctx.var(f), 1, 1, 1), r"conv,boxes"), x, f, 1, 1) <= 1.0
+    x[0, 0, 0, 0], x[1, 3, 4, 6] = np.inf, np.nan  # ... and what is not finite stays where it belongs
+    got = evaluated(ctx, S.conv_2d(ctx.var(x), ctx.var(f), 1, 1, 1), r"conv,boxes")
+    want = _conv64(x, f, 1, 1)
+    assert np.array_equal(np.isfinite(got), np.isfinite(want)) and not np.isfinite(got[0, 0, 0]).any()
+    fin = np.isfinite(want)
+    x[0, 0, 0, 0] = x[1, 3, 4, 6] = 0
+    assert (np.abs(got - _conv64(x, f, 1, 1)) / np.maximum(2e-6 * _conv64(np.abs(x), np.abs(f), 1, 1), 1e-300))[fin].max() <= 1.0
+    assert ctx.status_word() == 0
+
+
+# The image as another convolution's result, out of slices (512 channels) and not; out of a pool; beside another reader; kept.
+@pytest.mark.parametrize("c,hw,oc", [(512, 7, 64), (64, 14, 64), (64, 8, 128)])
+def test_small_images_that_a_program_makes(ctx, c, hw, oc):
+    """The producers of an image note its wide groups.  The second convolution against float64 of the first one's own result."""
+    rng = np.random.default_rng(c + hw)
+    d = _spread(rng, c, 44)
+    x = rng.uniform(0, 1, (1, 2 * hw, 2 * hw, c)).astype(np.float32)
+    f1 = (rng.uniform(-1, 1, (1, 1, c, c)) * d).astype(np.float32)
+    f2 = (rng.uniform(-1, 1, (3, 3, c, oc)) / d[:, None]).astype(np.float32)
+    xv, b = ctx.var(x), ctx.var((rng.uniform(-1, 1, (c,)) * d).astype(np.float32))
+    img = S.max_pool_2d(xv * ctx.var(d), 2, 2, 0, 1)
+    first = S.relu(S.conv_2d(S.max_pool_2d(xv, 2, 2, 0, 1), ctx.var(f1), 1, 0, 1) + b)
+    for made in (first, img):
+        z = S.conv_2d(made, ctx.var(f2), 1, 1, 1)
+        alone = evaluated(ctx, z, r"conv,boxes")
+        ctx.clear()
+        ctx.eval(z, made)
+        kept, both = ctx.read(made), ctx.read(z)
+        assert _conv_excess(both, kept, f2, 1, 1) <= 1.0
+        assert np.array_equal(alone, both)
+        ctx.clear()
+        other = S.gemm(S.view(made, [hw * hw, c]), ctx.var(f2[0, 0]))  # a reader that takes the same pieces
+        ctx.eval(z, other)
+        assert np.array_equal(ctx.read(z), alone)
+        assert np.isfinite(ctx.read(other)).all()
+        ctx.clear()
+    assert ctx.status_word() == 0
+
+
 @pytest.mark.parametrize("off", [0, 1, 4, 32, 64])
 @pytest.mark.parametrize("tail", [0, 5])
 @pytest.mark.parametrize("ker,stride", [(3, 1), (1, 2)])
