@@ -873,8 +873,8 @@ static int clusters_at_once(const Context &ctx, int s) {
 // M 24 .. 3136, N 64 .. 3072, K 512 .. 4608: a K-block takes 0.52 / 0.67 / 0.92 with 64 / 128 / 256 columns (a pair of CTAs
 // 0.42 / 0.48 / 0.91, windows kept in shared memory 0.48), and not less than the bytes of all CTAs at 9 TB/s; a tile 3.5 beside
 // them, and 5 for operands that depend on the row, which slices fetch in time.  Meeting in shared memory: 1.5 and 1.1 per 128 x
-// 64 sums (256 columns: 9, never worth it), timed when the sums were fetched after a barrier; sent, they take less, and the line
-// is left on the safe side.  Slices must promise a fifth: they change the order of summation, and nearer to the
+// 64 sums (256 columns: 9, never worth it), timed when the sums were fetched after a barrier; sent, they take up to 2 us less
+// (eight slices) or as much (two to four), and the line is left on the safe side.  Slices must promise a fifth: they change the order of summation, and nearer to the
 // line than that the estimate says little.
 struct SlicePlan {
     int slices, bn;
@@ -947,15 +947,27 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
     const int bn = cols.bn;
     const int stage_bytes = halo ? 2 * (bn / ctas) * HK * 2 : 2 * BM * HK * 2 + 2 * (bn / ctas) * HK * 2;
     const long long octets = std::min<long long>(BM / 8, (g.m + 7) / 8);  // of a tile: H2Tasks
-    const int staging = sliced ? (int)((octets * (bn / 64) + cut.slices - 1) / cut.slices) * cut.slices * 2048 : kEpiWarps * kStageBytesPerWarp;
+    const int region = sliced ? (int)((octets * (bn / 64) + cut.slices - 1) / cut.slices) * cut.slices * 2048 : kEpiWarps * kStageBytesPerWarp;
     const int fixed = halo ? kHaloStages * kHaloStageBytes : 0;
-    int stages = (227 * 1024 - 2048 - staging - fixed) / stage_bytes;
-    if (stages > 8) stages = 8;
     const long long all_kb = (g.k + HK - 1) / HK, my_kb = sliced ? (all_kb + cut.slices - 1) / cut.slices : all_kb;
-    if (sliced && stages > my_kb) stages = (int)my_kb;
+    const auto fitting = [&](int beside) { return (int)std::min<long long>((227 * 1024 - 2048 - beside - fixed) / stage_bytes, sliced && my_kb < 8 ? my_kb : 8); };
+    // Where a sliced tile's sums meet (H2Tasks).  Beside the operands: sent as each CTA is done with its own.  Over them, once the cluster's
+    // products are done, where that keeps a stage of the ring (3 of 128 columns, else 2) and a CTA has K-blocks enough to need
+    // it.  Left where they are and fetched, with two slices, or with four and nothing else to load in the store.  us a product
+    // in chains of equal 3 x 3 convolutions (channels, pixels, slices; + residual), fetched | beside | over; what is chosen in
+    // brackets:  512, 16 x 7 x 7, 4: [21.55] | 22.27 | 21.67, + 22.71 | 22.77 | [22.25];  512, 24 x 7 x 7, 3 +: 27.49 | 27.41 | [26.60];
+    // 256, 16 x 14 x 14, 2 +: [22.61] | 23.50 | 22.94;  256, 8 x 14 x 14, 4: [15.47] | 15.77 | 15.71, + 16.63 | 16.30 | [16.28];
+    // 128, 8 x 28 x 28, 2 +: [16.62] | 17.01 | 16.97;  128, 6 x 28 x 28, 3: 14.32 | [13.88];  128, 28 x 28, 6: 9.60 | [8.42].
+    // Plain products of the same sizes, whose operands come faster, and 64 columns lose by the wait: beside.
+    bool row_operands = false;
+    for (int i = 0; i < g.naux; ++i) row_operands = row_operands || g.aux[i].sr != 0;
+    const bool fetch = sliced && g.conv && bn == 128 && (cut.slices == 2 || (cut.slices == 4 && !row_operands));
+    const bool over = fetch || (sliced && g.conv && bn == 128 && my_kb >= 9 && fitting(0) > fitting(region));
+    const int staging = over ? 0 : region, stages = fitting(staging);
     const size_t smem = (size_t)fixed + (size_t)stages * stage_bytes + staging + 1024;
 
     H2Params p{};
+    p.sums_at = over ? 0 : stages * stage_bytes;
     p.c = g.c;
     p.c_hi = g.c_hi;
     p.c_plane = g.c_plane;
@@ -1055,7 +1067,7 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
 
     const int out_mask = (g.c ? 1 : 0) | (g.c_hi ? 2 : 0) | (g.h_hi ? 4 : 0) | (g.h_hi && g.h_marked ? 8 : 0);
     char num[96];
-    snprintf(num, sizeof num, "gemm_h2 %d %d %d %d %d %d %d %d %d\n", bn, ctas, sliced ? 1 : 0, aux_vec ? 1 : 0, g.conv ? (halo ? 2 : boxed ? 3 : 1) : 0, g.naux, rowinv, per_col, out_mask);
+    snprintf(num, sizeof num, "gemm_h2 %d %d %d %d %d %d %d %d %d\n", bn, ctas, sliced ? 1 : 0, aux_vec ? 1 : 0, (g.conv ? (halo ? 2 : boxed ? 3 : 1) : 0) + (fetch ? 4 : 0), g.naux, rowinv, per_col, out_mask);
     const bool plain = !g.conv && g.naux == 0 && g.epilogue.empty() && out_mask == 1;
     const std::string key = num + g.epilogue;
     Module *mod = plain ? nullptr : ctx.module_find(key);
@@ -1070,6 +1082,7 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
         define("SAGE_H2_CONV", g.conv ? (boxed ? 2 : 1) : 0);
         define("SAGE_H2_AUX_VEC", aux_vec ? 1 : 0);
         define("SAGE_H2_HALO", halo ? 1 : 0);
+        define("SAGE_H2_FETCH", fetch ? 1 : 0);
         src += "#define SAGE_EPI_EXPR(x0, x1, x2, x3) (" + (g.epilogue.empty() ? std::string("x0") : g.epilogue) + ")\n";
         src += kGemmTcDeviceSrc;
         src += kGemmH2DeviceSrc;
@@ -1107,7 +1120,7 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
     }
     std::string label;
     if (ctx.verbose_names)
-        label = "gemm_tc_h2[" + std::to_string(g.m) + "x" + std::to_string(g.n) + "x" + std::to_string(g.k) + (g.batch > 1 ? "x" + std::to_string(g.batch) : "") + (sliced ? ",slices" + std::to_string(cut.slices) : "") +
+        label = "gemm_tc_h2[" + std::to_string(g.m) + "x" + std::to_string(g.n) + "x" + std::to_string(g.k) + (g.batch > 1 ? "x" + std::to_string(g.batch) : "") + (sliced ? (fetch ? ",fetched" : over ? ",over" : "") + std::string(",slices") + std::to_string(cut.slices) : "") +
                 (g.conv ? (halo ? ",conv,taps" : boxed ? ",conv,boxes" : ",conv") : "") + ",bn" + std::to_string(bn) + (cols.narrow ? "/" + std::to_string(cols.wide) + "+" + std::to_string(cols.narrow) + "x192" : "") +
                 (ctas == 2 ? ",pair" : "") + "]o" + std::to_string(out_mask);
     if (plain) {

@@ -27,8 +27,8 @@ def test_aligned_cluster_barriers_follow_a_reconvergence():
     for m in re.finditer(r"barrier\.cluster\.(arrive|wait)\.\w+\.aligned", body):
         found += 1
         before = body[: m.start()].rstrip()
-        before = re.sub(r"(if \(SLICED\)( \{)?\s*)?asm volatile\(\"$", "", before).rstrip()
-        # the statement in front; conditions of the whole block (SLICED, PAIR, the role of a warp) do not separate lanes
-        before = re.sub(r"if (constexpr )?\((SLICED|PAIR)\)( \{|[^;\n]*;)$", "", before).rstrip()
+        before = re.sub(r"(if \(!?S\w+\)( \{)?\s*)?asm volatile\(\"$", "", before).rstrip()
+        # the statement in front; conditions of the whole block (SLICED, SEND, PAIR, the role of a warp) do not separate lanes
+        before = re.sub(r"if (constexpr )?\(!?(SLICED|SEND|PAIR)\)( \{|[^;\n]*;)$", "", before).rstrip()
         assert before.endswith(("__syncwarp();", "__syncthreads();")), before[-200:]
     assert found >= 5

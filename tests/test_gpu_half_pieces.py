@@ -98,6 +98,42 @@ def test_splits_of_operands(ctx, tb, n, k, m):
     assert ctx.status_word() == 0
 
 
+# Slices of K that meet in a cluster: one task of 8 x 64 sums for eight CTAs, fewer tasks than slices, tasks that the slices do not divide,
+# a last task with one row, the last column tile cut; several tiles, a batch.
+@pytest.mark.parametrize("m,n,k,batch", [(5, 1000, 4096, 1), (7, 640, 4608, 1), (9, 513, 4096, 1), (24, 192, 2304, 1), (127, 64, 1536, 1), (127, 130, 1536, 1), (128, 512, 2304, 1), (250, 300, 2304, 1),
+                                         (65, 64, 1152, 3), (384, 768, 3072, 1), (768, 512, 2304, 1), (400, 512, 2048, 1)])
+def test_slices_that_meet_in_a_cluster(ctx, m, n, k, batch):
+    rng = np.random.default_rng(m + n + k)
+    a, b = rng.standard_normal((batch, m, k), dtype=np.float32), rng.standard_normal((batch, n, k), dtype=np.float32)
+    got = product(ctx, a, b, False, True)
+    assert ",slices" in ctx.trace()[-1], ctx.trace()
+    assert excess(got, a, np.swapaxes(b, 1, 2)) <= 1.0
+    assert np.array_equal(got, product(ctx, a, b, False, True))
+    assert ctx.status_word() == 0
+
+
+# Sums sent beside the operands, sent over them (three slices of many K-blocks), and fetched (two slices; four without a residual).
+@pytest.mark.parametrize("n,hw,c,residual,how", [(8, 28, 128, True, ",fetched,slices2"), (8, 14, 256, False, ",fetched,slices4"), (8, 14, 256, True, ",over,slices4"), (24, 7, 512, True, ",over,slices3"),
+                                                 (6, 28, 128, True, ",slices3"), (3, 28, 128, False, ",slices6"), (8, 7, 512, False, ",over,slices6"), (9, 14, 320, True, ",slices")])
+def test_slices_of_convolutions(ctx, n, hw, c, residual, how):
+    """3 x 3, bias, residual and relu behind, the result read by a second convolution.  Tolerance as for the other convolutions."""
+    rng = np.random.default_rng(n + c)
+    x, f = rng.uniform(-1, 1, (n, hw, hw, c)).astype(np.float32), rng.uniform(-1, 1, (3, 3, c, c)).astype(np.float32)
+    b = rng.uniform(-1, 1, (c,)).astype(np.float32)
+    xv, fv = ctx.var(x), ctx.var(f)
+    y = S.conv_2d(xv, fv, 1, 1, 1) + ctx.var(b)
+    y = S.relu(y + xv) if residual else S.relu(y)
+    want = np.maximum(_conv64(x, f, 1, 1) + b + (x if residual else 0), 0.0)
+    got = evaluated(ctx, y, re.escape(how))
+    assert _close(got, want)
+    ctx.clear()
+    assert np.array_equal(got, y.eval(ctx))
+    ctx.clear()
+    z = S.conv_2d(y, ctx.var(f[:, :, :, :64].copy()), 1, 1, 1)
+    assert _close(z.eval(ctx), _conv64(want, f[:, :, :, :64], 1, 1))
+    assert ctx.status_word() == 0
+
+
 @pytest.mark.parametrize("ea,eb", [(100, -100), (-90, 90), (120, 0), (0, 120), (-90, 20)])
 def test_operands_far_from_one(ctx, ea, eb):
     """Whole operands scaled by powers of two give the scaled product, bit for bit, for rows of A above 2^-96."""
