@@ -579,7 +579,14 @@ static sage_status split_views(Context &ctx, const float *src_a, const SplitView
     if (va && vb) ctx.note_part(name);
     ctx.note_launch(name);
     if (ctx.dry()) return SAGE_OK;
-    return ctx.check_cuda(launch_dependent(ctx.pdl, ctx.stream(), p.ctas, out_a.marked || out_b.marked ? split_h2_kernel<true> : split_h2_kernel<false>, dim3((unsigned)blocks), dim3(256), 0, p), "split_h2 launch");
+    // Long runs of operand B (six tiles of 64 k a CTA and more) are not launched while the kernel before still holds most of the chip:
+    // the clusters that come early pile up on the SMs it leaves free, four CTAs to each, and finish last.  us a call in a row of calls,
+    // two kernels as they once were | one, launched early | as now: 64 x 768 x 3072 26.6 | 27.4 | 20.7, 64 x 1024 x 4096 34.0 | 35.5 | 26.8,
+    // 64 x 2048 x 8192 76.3 | 82.8 | 69.5, 512 x 1024 x 4096 44.4 | 45.6 | 37.2, 128 x 1023 x 4099 51.9 | 63.6 | 41.2, 300 x 770 x 3073
+    // 47.9 | 55.5 | 35.0, 4096^3 373 | 372 | 362.  Shorter runs, and a few blocks, are better off early: 64 x 768 x 768 13.0 | 13.7,
+    // 1000 x 1001 x 1002 23.5 | 23.8 late, 64 x 64 x 4096 19.0 | 20.7.
+    const bool early = ctx.pdl && !(p.tiles_per_cta >= 6 && b_blocks >= 32);
+    return ctx.check_cuda(launch_dependent(early, ctx.stream(), p.ctas, out_a.marked || out_b.marked ? split_h2_kernel<true> : split_h2_kernel<false>, dim3((unsigned)blocks), dim3(256), 0, p), "split_h2 launch");
 }
 
 sage_status split_h2_rows_at(Context &ctx, const float *src, const SplitView &v, const H2Split &out) { return split_views(ctx, nullptr, nullptr, H2Split(), src, &v, out); }
