@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(256) reduce_cols_kernel(const T *__restrict__ 
     reduce_cols_store<T, VEC>(part, y, cols, kind, ref_compat);
 }
 
-// Column reduction of up to 1024 rows a CTA: the CTAs of a cluster take a run of rows of one column tile each (64 columns, 16 lanes
+// Column reduction of short runs of rows: the CTAs of a cluster take a run of rows of one column tile each (64 columns, 16 lanes
 // with 16-byte loads; or 32 columns, one to a lane), eight loads in flight to a thread, and meet through distributed shared memory,
 // each finishing a part of the tile's columns.  Bound by latency: the start, two or three rounds of loads, one cluster barrier.  The
 // form above leaves partial rows in memory, and its last block's fence, ticket and second pass were a third of it.  Rows and ranks are
@@ -446,19 +446,29 @@ __global__ void __launch_bounds__(256) reduce_slices_kernel(const T *__restrict_
 template <typename T>
 static sage_status launch_reduce_cols(Context &ctx, int kind, const T *x, long long rows, long long cols, long long pitch, T *y, int compat_in) {
     const int compat = compat_in < 0 ? ctx.opts().ref_compat : compat_in;
-    {  // clusters of up to eight CTAs of up to 1024 rows (64 columns) each: beyond that too few loads are in flight on the chip
-        const bool quads = cols % 4 == 0 && pitch % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && cols >= 64;
-        const long long tiles = quads ? (cols + 63) / 64 : (cols + 31) / 32;
-        int ctas = 8;
-        while (ctas > 1 && (tiles * ctas > 4LL * ctx.sm_count || rows < 64LL * ctas)) ctas /= 2;
-        const long long per = (rows + ctas - 1) / ctas;
-        if (per <= (quads ? 1024 : 2048) && tiles * ctas <= 0x7fffffffLL) {
-            ctx.note_launch("reduce_cols");
-            if (ctx.dry()) return SAGE_OK;
-            launch_dependent(ctx.pdl, ctx.stream(), ctas, quads ? reduce_cols_cluster_kernel<T, 4> : reduce_cols_cluster_kernel<T, 1>, dim3((unsigned)(tiles * ctas)), dim3(512), 0, x, y,
-                             rows, cols, pitch, (int)per, ctas, kind, compat);
-            return ctx.check_cuda(cudaGetLastError(), "reduce_cols launch");
-        }
+    // Clusters of up to eight CTAs, 64 rows each at least, where all of them run at once and none has a long run: there the form below
+    // spends its time on meeting.  Of singles two thirds of the loads are in flight, so the runs are shorter.  Beyond the caches (128 MiB,
+    // 512 rows) a CTA to a column tile of all rows: for single columns, and for rows a multiple of 4 KiB apart, which meet in the same
+    // memory channels.  us, the form below | clusters; what is chosen in brackets:
+    //   rows x 768: 384 6.33 | [4.66], 1000 5.66 | [4.65], 4096 7.65 | [6.33], 8192 [8.24] | 8.53;  x 2048: 512 6.27 | [5.22], 2048 6.87 | [6.21];
+    //   x 4096: 384 5.40 | [4.68], 512 [5.47] | 9.37, 1024 [6.46] | 9.75;  x 9472: 256 [5.62] | 11.10, 1000 [8.31] | 12.20;
+    //   x 64: 1024 4.68 | [4.71], 4096 [4.52] | 6.27;  x 31: 512 6.18 | [4.68], 1024 6.33 | [4.63], 8192 [5.03] | 8.65;
+    //   x 1001: 1000 6.29 | [5.74], 2048 [6.47] | 7.57;  x 9473: 1000 [9.07] | 16.85;
+    //   64 x 65536 [6.2] | 9.1, 64 x 524288 [29] | 70, 128 x 262144 [26.9] | 39.2, 1000 x 50000 [33.6] | 36.1;
+    //   1024 x 32768 33.0 | [25.3], 1000 x 65536 55.1 | [46.0], 1000 x 30011 42.0 | [30.3], 2048 x 30001 81.1 | [56.2].
+    const bool quads = cols % 4 == 0 && pitch % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && cols >= 64;
+    const long long tiles_64 = quads ? (cols + 63) / 64 : (cols + 31) / 32;
+    int ctas = 8;
+    while (ctas > 1 && rows < 64LL * ctas) ctas /= 2;
+    const bool at_once = tiles_64 * ctas <= 2LL * ctx.sm_count && (rows + ctas - 1) / ctas <= (!quads ? 128 : tiles_64 < 4 ? 256 : 512);
+    const bool streams = rows >= 512 && rows <= (quads ? 1024 : 2048) && rows * cols * (long long)sizeof(T) >= (128LL << 20) && (!quads || pitch % 1024 == 0);
+    if ((at_once || streams) && tiles_64 * ctas <= 0x7fffffffLL) {
+        if (!at_once) ctas = 1;
+        ctx.note_launch(ctx.verbose_names ? "reduce_cols_cluster" : "reduce_cols");
+        if (ctx.dry()) return SAGE_OK;
+        launch_dependent(ctx.pdl, ctx.stream(), ctas, quads ? reduce_cols_cluster_kernel<T, 4> : reduce_cols_cluster_kernel<T, 1>, dim3((unsigned)(tiles_64 * ctas)), dim3(512), 0, x, y, rows,
+                         cols, pitch, (int)((rows + ctas - 1) / ctas), ctas, kind, compat);
+        return ctx.check_cuda(cudaGetLastError(), "reduce_cols launch");
     }
     // 16-byte loads (4 columns per lane) when the rows allow; the partial rows are read with pitch = cols
     const bool vec = cols % 4 == 0 && pitch % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && cols >= 256;
