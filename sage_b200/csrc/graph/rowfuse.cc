@@ -209,6 +209,23 @@ bool screen(const std::vector<Var> &targets, const std::unordered_set<Origin *> 
     return largest > 0 && *R > 1 && *C > 1 && (reduces || maps_suffice);
 }
 
+// Whole-row values that a thread holds across an exchange at once: each is a register per element.
+int rows_alive(const RowProgram &p) {
+    std::vector<int> last(p.vals.size(), -1);  // where a value is read last (outputs are stored where they are computed)
+    for (size_t id = 0; id < p.vals.size(); ++id)
+        if (p.vals[id].kind != KAlias)
+            for (int a : p.vals[id].args) last[p.resolve(a)] = (int)id;
+    int most = 0;
+    for (size_t at = 0; at < p.vals.size(); ++at) {
+        const Val &v = p.vals[at];
+        if (!(v.kind == KGather || (v.kind == KReduce && p.vals[p.resolve(v.args[0])].cls == Full))) continue;
+        int alive = 0;
+        for (size_t id = 0; id < at; ++id) alive += p.vals[id].kind != KAlias && p.vals[id].cls == Full && last[id] > (int)at;
+        most = std::max(most, alive);
+    }
+    return most;
+}
+
 void emit(RowProgram &p) {
     std::ostringstream s;
     const int E = p.nv * p.vec;
@@ -441,15 +458,22 @@ std::shared_ptr<RowProgram> row_program_build(const std::vector<Var> &evaluated,
     }
     if (p->nv * p->vec > 32) return nullptr;
     p->threads = (int)((t + 31) / 32 * 32);
-    // Rows of 4096 columns and more, with at most two whole-row inputs and one whole-row result: 32 elements per thread halve what the
-    // reductions cost per element.  Only where the threads have whole shares and twelve warps stay on an SM.  Loss and gradient of
-    // a cross entropy over 2^25 elements, us, 16 | 32 a thread: 4096 columns 80.0 | 75.8, 6144 86.6 | 80.7, 7000 124.7 | 93.7, 12000 105.2 | 100.6,
-    // 16384 111.6 | 102.2; outside the rule 4500 (an eighth of the threads idle) 98.2 | 108.0, 5120 (ten warps) 84.9 | 87.7, 2048 70.9 | 85.5.
+    // Rows of 4096 columns and more, in programs that pick an element of the row (losses over labels), with at most two whole-row inputs,
+    // one whole-row result and four whole rows alive across an exchange (with more they spill: 168 registers, 128 of them rows): 32
+    // elements per thread halve what the exchanges cost per element.  Only where the threads have whole shares and twelve warps stay on
+    // an SM.  us, 16 | 32 a thread, 2^25 elements; loss and gradient of a cross entropy of x y + 3.14 x (four alive): 4096 columns
+    // 80.7 | 76.0, 6144 87.7 | 81.2, 7000 126.6 | 94.2, 12000 106.7 | 101.8, 16384 111.4 | 102.7; of x: 64.6 | 59.2, 69.4 | 64.3, 88.1 |
+    // 79.0, 82.2 | 82.5, 87.6 | 82.0; the loss alone: 48.7 | 47.3, 51.1 | 50.0, 78.7 | 49.4, 64.3 | 60.5, 59.9 | 55.4; the gradient for
+    // tanh x: 105.0 | 105.2, 109.0 | 107.0, 127.5 | 137.8, 115.1 | 120.0, 139.1 | 137.2.
+    // Outside the rule: 4500 columns (an eighth of the threads idle) 98.2 | 108.0, 5120 (ten warps) 84.9 | 87.7, 2048 70.9 | 85.5;
+    // nothing picked (softmax 68.7 | 64.1, 68.3 | 66.4, 69.8 | 77.6, 91.0 | 93.4, 87.5 | 86.8; a softmax of a layer norm 75.8 | 73.3, 77.3 | 90.1,
+    // 107.7 | 88.9, 89.1 | 95.3, 101.4 | 101.5; a sum and a map of one row 48.5 | 50.5, 45.7 | 49.1, 46.8 | 48.2, 45.9 | 48.5, 63.4 | 64.4);
+    // more alive (five: 245.8 | 418.2 and 250.6 | 435.3; six, nothing picked: 404 | 970, 365 | 800, 338 | 738, 382 | 638, 491 | 633).
     int full_in = 0, full_out = 0;
     for (int id : p->in_val) full_in += p->vals[id].cls == Full;
     for (int id : p->out_val) full_out += p->vals[id].cls == Full;
     const int wide = (int)((C + 1023) / 1024 * 32), wide_regs = 140;  // threads with 32 elements each
-    if (elems == 16 && p->vec == 4 && C >= 4096 && full_in <= 2 && full_out <= 1 && wide <= 1024 && wide * 32LL * 100 <= C * 103LL &&
+    if (elems == 16 && p->vec == 4 && C >= 4096 && p->n_index > 0 && rows_alive(*p) <= 4 && full_in <= 2 && full_out <= 1 && wide <= 1024 && wide * 32LL * 100 <= C * 103LL &&
         std::max(1, 65536 / (wide * wide_regs)) * (wide / 32) >= 12) {
         p->nv = 8;
         p->threads = wide;
