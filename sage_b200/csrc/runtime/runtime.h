@@ -98,7 +98,7 @@ struct Module {
     CUmod_st *cu_module = nullptr;  // null on a planning context
     struct Function {
         CUfunc_st *fn = nullptr;
-        uint32_t smem = 40 * 1024;  // dynamic shared memory it may be launched with: 48 KiB less what a kernel may hold statically
+        uint32_t smem = 0;  // dynamic shared memory it has been allowed; how much it may have unasked depends on what it holds statically
     };
     std::unordered_map<std::string, Function> functions;
 };
