@@ -24,7 +24,7 @@ struct Im2colOp : Operator {
         return {col2im(gy, Pair{x[0].extent(2), x[0].extent(1)}, ker, stride, pad, dil)};
     }
     sage_status compute(const std::vector<Tensor> &x, Context &ctx, Tensor *y) override {
-        const bool emit = ctx.hint_emit_planes && emits_planes();
+        const bool emit = ctx.hint_emit_planes && emits_planes(), only = emit && ctx.hint_planes_only;
         ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = false;
         sage_status st = Tensor::uninit(ctx, out, y);
         if (st) return st;
@@ -34,7 +34,8 @@ struct Im2colOp : Operator {
         st = storage_planes_attach(ctx, *y->data);
         if (st) return st;
         const SplitCache &c = *y->data->split;
-        return k::im2col_planes(ctx, (const float *)x[0].ptr(), e[0], e[1], e[2], e[3], col.h, col.w, window(ker, stride, pad, dil), (float *)y->ptr(), c.planes.planes, c.plane,
+        y->data->planes_only = only;
+        return k::im2col_planes(ctx, (const float *)x[0].ptr(), e[0], e[1], e[2], e[3], col.h, col.w, window(ker, stride, pad, dil), only ? nullptr : (float *)y->ptr(), c.planes.planes, c.plane,
                                 (int)(ker.h * ker.w * e[3]));
     }
     // the planes lie like the result, whole 16-byte pieces at a time

@@ -330,7 +330,7 @@ sage_status im2col_planes(Context &ctx, const float *img, long long n, long long
                           long long col_h, long long col_w, const Window &w, float *col, float *hi, long long plane, int pitch) {
     ConvP p{n, img_h, img_w, chan, col_h, col_w, w};
     const long long pixels = n * col_h * col_w;
-    ctx.note_launch("im2col");
+    ctx.note_launch(ctx.verbose_names && hi ? (col ? "im2col+planes" : "im2col=planes") : "im2col");
     if (ctx.dry() || pixels == 0) return SAGE_OK;
     if (col_h * col_w > 0x7fffffffLL || img_h > 0x7fffffffLL || img_w > 0x7fffffffLL || (long long)w.ker_h * w.ker_w * chan > 0x7fffffffLL ||
         (pixels + 7) / 8 > 0x7fffffffLL)
