@@ -155,7 +155,7 @@ public:
         if (tracing) trace.append(name).push_back('\n');
         if (profiling) profile_mark(name);
     }
-    // A pass that shares the next launch with another one: launch lists name both, the count is of launches.
+    // A pass that shares the next launch with another one: launch lists name both (sage_trace_get says so), the count is of launches.
     void note_part(const char *name) {
         if (tracing) trace.append(name).push_back('\n');
     }

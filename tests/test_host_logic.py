@@ -493,3 +493,23 @@ def test_program_cache_is_bounded_and_least_recently_used():
         assert ctx.programs_compiled() == before + 1
     finally:
         ctx.close()
+
+
+def test_launch_list_and_count_of_a_plain_product():
+    """Both operands are brought into pieces by one launch that the list names once for each: include/sage_cuda.h says so, and this is
+    the only launch with two lines."""
+    header = open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "include", "sage_cuda.h")).read()
+    assert "longer than" in header.split("sage_status sage_trace_begin")[0].rsplit("/*", 1)[1]
+    ctx = S.Context(-1)
+    L = ctypes.c_int64
+    a, b, c = ctx.empty((256, 256)), ctx.empty((256, 256)), ctx.empty((256, 256))
+    before = ctx.launch_count()[0]
+    ctx.trace_begin()
+    ctx._ck(S.lib.sage_gemm_strided_batched(ctx.h, 0, 0, L(256), L(256), L(256), a.buf, L(0), L(256), L(0), b.buf, L(0), L(256), L(0), c.buf, L(0), L(256), L(0), L(1)))
+    assert ctx.trace() == ["split_tf32", "split_tf32", "gemm_tc_3xtf32"] and ctx.launch_count()[0] - before == 2
+    x, w = ctx.var(np.zeros((256, 256), np.float32)), ctx.var(np.zeros((256, 256), np.float32))
+    before = ctx.launch_count()[0]
+    ctx.trace_begin()
+    ctx.eval(S.relu(x.matmul(w) + 1.0).sum([0], False))
+    assert len(ctx.trace()) == ctx.launch_count()[0] - before
+    ctx.close()
