@@ -57,7 +57,8 @@ Block *Allocator::find_free(FreeSet &pool, size_t size) {
     auto it = pool.lower_bound(&key);
     for (; it != pool.end(); ++it) {
         Block *b = *it;
-        if (size < kSplitLim && b->size >= kSplitLim) return nullptr;  // sorted: all later ones too
+        // (but a request above 38 MiB gets the 40 MiB that grow() made for it)
+        if (size < kSplitLim && b->size >= kSplitLim && b->size - size >= kRoundLarge) return nullptr;  // sorted: all later ones too
         if (size >= kSplitLim && b->size > size + kLargeBuffer) return nullptr;
         pool.erase(it);
         size_t rem = b->size - size;

@@ -513,3 +513,19 @@ def test_launch_list_and_count_of_a_plain_product():
     ctx.eval(S.relu(x.matmul(w) + 1.0).sum([0], False))
     assert len(ctx.trace()) == ctx.launch_count()[0] - before
     ctx.close()
+
+
+@pytest.mark.parametrize("elements", [38 * 262144, 38 * 262144 + 1, 10 ** 7, 40 * 262144 - 128, 40 * 262144 - 1, 40 * 262144, 40 * 262144 + 1])
+def test_tensors_of_38_to_40_mib(elements):
+    """Their segment is as large as those that small requests may not be carved from; it is theirs all the same, also when it comes back."""
+    ctx = S.Context(-1)
+    first = ctx.empty((elements,))
+    allocs = ctx.mem_stats()["num_device_allocs"]
+    first.release()
+    again = ctx.empty((elements,))
+    assert ctx.mem_stats()["num_device_allocs"] == allocs
+    small = ctx.empty((1 << 20,))  # not carved from it
+    assert ctx.mem_stats()["num_device_allocs"] == allocs + 1
+    for t in (again, small):
+        t.release()
+    ctx.close()
