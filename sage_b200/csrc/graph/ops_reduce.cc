@@ -52,15 +52,25 @@ struct ReduceOp : Operator {
     }
 
     sage_status compute(const std::vector<Tensor> &x, Context &ctx, Tensor *y) override {
+        k::LeafBatch *batch = ctx.hint_batch;
+        ctx.hint_batch = nullptr;
         sage_status st = Tensor::uninit(ctx, out, y);
         if (st) return st;
         Shape inner, outer;
         x[0].desc.shape.extract(axes, &inner, &outer);
+        k::ColumnSum sum;
+        if (batch && k::column_sum_of(x[0].desc.dtype, (int)kind, (const char *)x[0].data->dev + outer.offset * 4, to_dims(outer), to_dims(inner), y->ptr(), &sum)) {
+            batch->column_sums.push_back(sum);
+            batch->held.push_back(x[0].data);
+            batch->held.push_back(y->data);
+            return SAGE_OK;
+        }
         return k::reduce(ctx, x[0].desc.dtype, (int)kind, (const char *)x[0].data->dev + outer.offset * 4, to_dims(outer),
                          to_dims(inner), y->ptr());
     }
 };
 
+bool is_reduce_op(const Operator &op) { return dynamic_cast<const ReduceOp *>(&op) != nullptr; }
 bool reduce_op_info(const Operator &op, int *kind, std::vector<int> *axes) {
     const ReduceOp *r = dynamic_cast<const ReduceOp *>(&op);
     if (!r) return false;

@@ -34,6 +34,7 @@ struct Node {
     bool visited = false;          // traversal mark for shared nodes
     bool planes_only = false;      // ... and that GEMM is the only reader: the fp32 result need not be stored
     int readers = 0, gemm_readers = 0;  // shared nodes: how many parents, how many of them GEMM operands
+    bool leaf = false;             // nothing of the program reads the result: its launch may wait for others of its kind
 };
 
 // ops_map.cc / ops_core.cc / ops_gemm.cc / ops_nn.cc
@@ -46,6 +47,7 @@ std::shared_ptr<Operator> map_merge_inputs(const Operator &op, const std::vector
 bool is_view_op(const Operator &op);
 bool is_reshape_op(const Operator &op);
 bool is_gemm_op(const Operator &op);
+bool is_reduce_op(const Operator &op);  // ops_reduce.cc
 bool gemm_runs_on_tc(const Operator &op, bool tc_enabled);
 bool gemm_can_fuse(const Operator &op, bool tc_enabled);
 std::shared_ptr<Operator> gemm_with_operand_view(const Operator &op, int idx, const TensorDesc &view, bool tc_enabled);
@@ -127,12 +129,13 @@ struct Program {
     bool fusion = true, pattern = true;
     std::shared_ptr<RowProgram> row;  // set: the whole program is one generated row kernel (rowfuse.h)
 
-    // The order a completed run took, kept so that later runs need no search: every value the routines exchange has a
-    // slot, and a step says which slots it was the last to read.
+    // The order of a run that needs no eviction, worked out once; every run follows it while there is memory.  Every value the
+    // routines exchange has a slot, and a step says which slots it was the last to read.
     struct Step {
         Routine *routine;
         std::vector<int> outputs;   // slots of what it computes (several for a row group)
         std::vector<int> release;
+        bool leaf;                  // no step reads what it computes
     };
     std::vector<Step> schedule;
     std::unordered_map<Origin *, int> slot_of;
@@ -887,7 +890,8 @@ struct Values {
     const Tensor *slots = nullptr;
 };
 
-static sage_status run_node(const Node &n, Context &ctx, Session &s, const Values &values, SharedMemo &memo, Tensor *out) {
+// `batch`: where the launches of leaf nodes are collected, or null.
+static sage_status run_node(const Node &n, Context &ctx, Session &s, const Values &values, SharedMemo &memo, Tensor *out, k::LeafBatch *batch = nullptr) {
     if (n.is_data) {
         if (values.slots && n.slot >= 0) {
             *out = values.slots[n.slot];
@@ -914,7 +918,7 @@ static sage_status run_node(const Node &n, Context &ctx, Session &s, const Value
     }
     std::vector<Tensor> args(n.args.size());
     for (size_t i = 0; i < n.args.size(); ++i) {
-        sage_status st = run_node(n.args[i], ctx, s, values, memo, &args[i]);
+        sage_status st = run_node(n.args[i], ctx, s, values, memo, &args[i], batch);
         if (st) return st;
     }
     if (n.shared) {
@@ -934,8 +938,10 @@ static sage_status run_node(const Node &n, Context &ctx, Session &s, const Value
     ctx.hint_emit_h2 = n.emit_h2;
     ctx.hint_planes_only = (n.emit_planes || n.emit_h2) && n.planes_only;
     ctx.hint_mark_wide = n.mark_wide;
+    ctx.hint_batch = n.leaf ? batch : nullptr;
     sage_status st = n.op->compute(args, ctx, out);
     ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = ctx.hint_mark_wide = false;
+    ctx.hint_batch = nullptr;
     return st;
 }
 
@@ -949,14 +955,53 @@ static void assign_slots(Node &n, const std::unordered_map<Origin *, int> &slot_
     for (Node &a : n.args) assign_slots(a, slot_of);
 }
 
-// Turns the order of a run that needed no eviction into the program's schedule.
+// The order in which exec() runs the routines while nothing is evicted.
+static bool plan_order(Program &p, const Session &s, std::vector<Routine *> *order) {
+    std::unordered_set<Origin *> computed;
+    std::vector<Var> stack(p.outputs.begin(), p.outputs.end());
+    auto available = [&](const Var &v) { return v.is_data() || s.data.count(v.key()) || computed.count(v.key()); };
+    while (!stack.empty()) {
+        const Var v = stack.back();
+        if (available(v)) {
+            stack.pop_back();
+            continue;
+        }
+        auto it = p.routines.find(v.key());
+        if (it == p.routines.end()) return false;
+        Routine &f = it->second;
+        bool ready = true;
+        for (const Var &k : f.inputs)
+            if (!available(k)) {
+                stack.push_back(k);
+                ready = false;
+            }
+        if (!ready) continue;
+        if (f.row)
+            for (const Var &o : f.row_outputs) computed.insert(o.key());
+        else
+            computed.insert(v.key());
+        order->push_back(&f);
+        stack.pop_back();
+    }
+    return true;
+}
+
+// Turns that order into the program's schedule.
 static void make_schedule(Program &p, const std::vector<Routine *> &order) {
     auto slot = [&](Origin *o) {
         auto it = p.slot_of.emplace(o, (int)p.slot_of.size());
         return it.first->second;
     };
+    std::unordered_set<Origin *> read;
+    for (Routine *r : order)
+        for (const Var &v : r->inputs) read.insert(v.key());
     for (Routine *r : order) {
-        Program::Step step{r, {}, {}};
+        Program::Step step{r, {}, {}, !r->row && !read.count(r->output.key())};
+        if (step.leaf) {
+            Node *n = &r->root;
+            while (!n->is_data && !n->shared && is_view_op(*n->op) && n->args.size() == 1) n = &n->args[0];
+            n->leaf = !n->is_data && !n->shared && is_reduce_op(*n->op);
+        }
         if (r->row)
             for (const Var &v : r->row_outputs) step.outputs.push_back(slot(v.key()));
         else
@@ -990,7 +1035,32 @@ static void make_schedule(Program &p, const std::vector<Routine *> &order) {
 
 static sage_status exec(Program &p, Context &ctx, Session &s, std::unordered_map<Origin *, Tensor> temp = {});
 
+// Device time of a routine's first run, for the choice of what to evict.
+struct FirstRun {
+    Routine &f;
+    Context &ctx;
+    std::shared_ptr<RoutineTimer> timer;
+    std::chrono::steady_clock::time_point t0 = std::chrono::steady_clock::now();
+    FirstRun(Routine &f_, Context &c) : f(f_), ctx(c) {
+        if (f.timed || ctx.dry()) return;
+        timer = std::make_shared<RoutineTimer>();
+        if (cudaEventCreate(&timer->ev[0]) != cudaSuccess || cudaEventCreate(&timer->ev[1]) != cudaSuccess || cudaEventRecord(timer->ev[0], ctx.stream()) != cudaSuccess) timer.reset();
+    }
+    void done(sage_status st) {
+        if (timer && st == SAGE_OK && cudaEventRecord(timer->ev[1], ctx.stream()) == cudaSuccess) {
+            f.timer = timer;
+            f.timed = true;
+        } else if (!f.timed) {
+            f.exec_time = 1e6 * std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+        }
+    }
+};
+
 // A run along the schedule.  Out of memory, it hands what it has computed to the general run, which evicts and recomputes.
+//
+// Steps that follow one another and whose results no step reads (a training step ends with the gradients of all parameters) leave
+// column sums to a batch: one pass for all of them.  What they read lives until the batch has run, as it
+// did at the first of them.
 static sage_status exec_scheduled(Program &p, Context &ctx, Session &s) {
     if (!p.times_read) {  // timers of the first run
         p.times_read = true;
@@ -1014,8 +1084,20 @@ static sage_status exec_scheduled(Program &p, Context &ctx, Session &s) {
         Values values;
         values.slots = p.slots.data();
         sage_status st = SAGE_OK;
+        k::LeafBatch batch;
+        std::vector<std::pair<Var, Tensor>> batched;  // results that the batch computes
+        auto flush = [&]() {
+            const sage_status ran = batch.empty() ? SAGE_OK : batch.run(ctx);
+            if (ran == SAGE_OK)
+                for (auto &v : batched) s.data[v.first.key()] = v;
+            batched.clear();
+            return ran;
+        };
         for (Program::Step &step : p.schedule) {
             Routine &f = *step.routine;
+            if (!step.leaf && (st = flush())) break;
+            FirstRun first(f, ctx);
+            const size_t before = batch.held.size();
             if (f.row) {
                 std::vector<Tensor> outs;
                 st = row_program_run(*f.row, ctx, [&](const Var &k, Tensor *t) {
@@ -1024,20 +1106,24 @@ static sage_status exec_scheduled(Program &p, Context &ctx, Session &s) {
                     *t = p.slots[it->second];
                     return true;
                 }, &outs, f.row_emit_shared.get());
-                if (st) break;
-                for (size_t i = 0; i < outs.size(); ++i) p.slots[step.outputs[i]] = std::move(outs[i]);
+                if (!st)
+                    for (size_t i = 0; i < outs.size(); ++i) p.slots[step.outputs[i]] = std::move(outs[i]);
             } else {
                 SharedMemo memo;
-                st = run_node(f.root, ctx, s, values, memo, &p.slots[step.outputs[0]]);
-                if (st) break;
+                st = run_node(f.root, ctx, s, values, memo, &p.slots[step.outputs[0]], step.leaf ? &batch : nullptr);
             }
+            first.done(st);
+            if (st) break;
             for (size_t i = 0; i < step.outputs.size(); ++i)
                 if (p.is_output[step.outputs[i]]) {
                     const Var &v = f.row ? f.row_outputs[i] : f.output;
-                    s.data[v.key()] = std::make_pair(v, p.slots[step.outputs[i]]);
+                    if (batch.held.size() > before) batched.push_back({v, p.slots[step.outputs[i]]});
+                    else s.data[v.key()] = std::make_pair(v, p.slots[step.outputs[i]]);
                 }
             for (int n : step.release) p.slots[n] = Tensor();
         }
+        const sage_status ran = flush();  // (out of memory or not: what is collected needs no more of it)
+        if (!st) st = ran;
         if (st != SAGE_ERR_OOM) return st;
         for (Program::Step &step : p.schedule)
             for (size_t i = 0; i < step.outputs.size(); ++i) {
@@ -1051,9 +1137,6 @@ static sage_status exec_scheduled(Program &p, Context &ctx, Session &s) {
 // Program::exec, session.rs:208-468.
 static sage_status exec(Program &p, Context &ctx, Session &s, std::unordered_map<Origin *, Tensor> temp) {
     for (auto &kv : p.routines) kv.second.resolve_time();  // timers of an earlier run whose events have completed
-    const bool first = temp.empty() && p.schedule.empty();
-    bool evictions = false;
-    std::vector<Routine *> order;
     Values values;
     values.temp = &temp;
     std::unordered_map<Origin *, int> remaining = p.consumers;
@@ -1085,14 +1168,7 @@ static sage_status exec(Program &p, Context &ctx, Session &s, std::unordered_map
         Tensor out;
         std::vector<Tensor> row_outs;
         for (;;) {
-            auto t0 = std::chrono::steady_clock::now();
-            std::shared_ptr<RoutineTimer> timer;
-            if (!f.timed && !ctx.dry()) {
-                timer = std::make_shared<RoutineTimer>();
-                if (cudaEventCreate(&timer->ev[0]) != cudaSuccess || cudaEventCreate(&timer->ev[1]) != cudaSuccess ||
-                    cudaEventRecord(timer->ev[0], ctx.stream()) != cudaSuccess)
-                    timer.reset();
-            }
+            FirstRun timed(f, ctx);
             SharedMemo memo;
             sage_status st;
             if (f.row) {
@@ -1107,15 +1183,9 @@ static sage_status exec(Program &p, Context &ctx, Session &s, std::unordered_map
             } else {
                 st = run_node(f.root, ctx, s, values, memo, &out);
             }
-            if (timer && st == SAGE_OK && cudaEventRecord(timer->ev[1], ctx.stream()) == cudaSuccess) {
-                f.timer = timer;
-                f.timed = true;
-            } else if (!f.timed) {
-                f.exec_time = 1e6 * std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-            }
+            timed.done(st);
             if (st == SAGE_OK) break;
             if (st != SAGE_ERR_OOM) return st;
-            evictions = true;
             // Out of memory: drop the intermediates that are cheapest to recompute per byte
             // (session.rs:259-331); they are rebuilt on demand when a later routine needs them.
             const uint64_t needed = ctx.allocator().oom_needed, start = ctx.allocator().mem_used();
@@ -1160,10 +1230,8 @@ static sage_status exec(Program &p, Context &ctx, Session &s, std::unordered_map
             auto it = remaining.find(k.key());
             if (it != remaining.end() && --it->second == 0) temp.erase(k.key());
         }
-        order.push_back(&f);
         stack.pop_back();
     }
-    if (first && !evictions) make_schedule(p, order);
     return SAGE_OK;
 }
 
@@ -1239,6 +1307,8 @@ sage_status Session::eval(const std::vector<const Var *> &targets) {
     last_ = prog;
     try {
         if (prog->row) return row_program_exec(*prog->row, *ctx_, *this);
+        std::vector<Routine *> order;
+        if (prog->schedule.empty() && plan_order(*prog, *this, &order)) make_schedule(*prog, order);
         return prog->schedule.empty() ? exec(*prog, *ctx_, *this) : exec_scheduled(*prog, *ctx_, *this);
     } catch (const ShapeError &e) {
         return ctx_->fail(SAGE_ERR_INVALID, e.msg);

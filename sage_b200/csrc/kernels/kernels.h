@@ -2,6 +2,9 @@
 // addresses with the tensor's element offset already applied; strides are in elements.
 #pragma once
 #include <cstdint>
+#include <memory>
+#include <string>
+#include <vector>
 
 #include "../runtime/runtime.h"
 
@@ -32,6 +35,16 @@ struct PlaneOut {
     float *h2_scale = nullptr;
     float *h2_marked = nullptr;  // the scales again, negative where a group is wide (gemm_h2_device.inc), for a reader that asks
 };
+
+// column_sums.cu — several [rows, cols] -> [cols] sums in one pass over all of them (src/ops/reduce.rs:258-325, kind Sum)
+struct ColumnSum {
+    const float *x = nullptr;
+    float *y = nullptr;
+    long long rows = 0, cols = 0, pitch = 0;
+};
+// Is this reduction of floats such a sum?
+bool column_sum_of(int dtype, int kind, const void *x, const Dims &outer, const Dims &inner, void *y, ColumnSum *out);
+sage_status column_sums_run(Context &ctx, const std::vector<ColumnSum> &all);
 
 // reduce.cu — ReduceOperator / ReduceArgOperator (src/ops/reduce.rs:258-325, 372-431)
 sage_status reduce(Context &ctx, int dtype, int kind, const void *x, const Dims &outer, const Dims &inner, void *y);
@@ -159,6 +172,14 @@ sage_status gemm_tc_run(Context &ctx, const TcGemm &g);
 // How many K slices gemm_tc_run would cut this product into (0 = none).  Only products without an epilogue are
 // cut; a caller with an epilogue may ask for the plain product and apply the epilogue to the sum itself.
 int gemm_tc_split_plan(Context &ctx, const TcGemm &g);
+// Work that nothing of a program reads, put off until launches of one kind can be made together.  `held` keeps alive what it reads
+// and writes.
+struct LeafBatch {
+    std::vector<ColumnSum> column_sums;
+    std::vector<std::shared_ptr<void>> held;
+    bool empty() const { return column_sums.empty(); }
+    sage_status run(Context &ctx);  // ... and empties it
+};
 // hi/lo split of `n` consecutive floats into planes laid out like the source (dst_hi[i], dst_hi[plane + i]).
 sage_status split_tf32_flat(Context &ctx, const float *src, long long n, float *dst_hi, long long plane);
 // hi/lo split of a strided 4-level view (b1, b0, row, col) into compact planes owned by `out`.

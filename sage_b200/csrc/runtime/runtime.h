@@ -19,6 +19,9 @@ struct CUfunc_st;
 typedef struct CUstream_st *cudaStream_t;
 
 namespace sage {
+namespace k {
+struct LeafBatch;  // kernels/kernels.h
+}
 
 // ------------------------------------------------------------------------------------------
 // Allocator: restates the pool policy of src/session/memory.rs (size classes :23-43, best fit
@@ -192,6 +195,8 @@ public:
     bool hint_planes_only = false;
     // ... and the reader of the pieces wants to know which groups they have not room for (a small convolution).
     bool hint_mark_wide = false;
+    // Set likewise: nothing of the running program reads the result, so the operator may leave its launch to this batch.
+    k::LeafBatch *hint_batch = nullptr;
     int sm_count = 148;
 
 private:
