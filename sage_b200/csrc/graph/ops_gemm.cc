@@ -386,6 +386,8 @@ struct GemmOp : Operator {
     sage_status compute(const std::vector<Tensor> &x, Context &ctx, Tensor *y) override {
         const bool emit = ctx.hint_emit_planes, emit_h2 = ctx.hint_emit_h2, only = (emit || emit_h2) && ctx.hint_planes_only, mark = ctx.hint_mark_wide;
         ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = ctx.hint_mark_wide = false;
+        k::LeafBatch *batch_to = ctx.hint_batch;
+        ctx.hint_batch = nullptr;
         sage_status st = Tensor::uninit(ctx, out, y);
         if (st) return st;
         if (!lowered) dims_from_inputs();
@@ -571,6 +573,12 @@ struct GemmOp : Operator {
         for (int i = 0; i < g.naux; ++i) {
             st = aux_strides(ctx, x[2 + i], &g.aux[i]);
             if (st) return st;
+        }
+        if (batch_to && !col_block && k::gemm_tc_groupable(g)) {
+            batch_to->products.push_back(g);
+            for (std::shared_ptr<void> held : {std::shared_ptr<void>(x[0].data), std::shared_ptr<void>(x[1].data), std::shared_ptr<void>(hold_a), std::shared_ptr<void>(hold_b), std::shared_ptr<void>(y->data)})
+                batch_to->held.push_back(held);
+            return SAGE_OK;
         }
         // An epilogue cannot be applied before the K slices of a split product are summed.  Where the cost model
         // wants slices (few output tiles, long K: a convolution of a small feature map at a small batch), the

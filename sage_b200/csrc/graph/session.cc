@@ -1000,7 +1000,7 @@ static void make_schedule(Program &p, const std::vector<Routine *> &order) {
         if (step.leaf) {
             Node *n = &r->root;
             while (!n->is_data && !n->shared && is_view_op(*n->op) && n->args.size() == 1) n = &n->args[0];
-            n->leaf = !n->is_data && !n->shared && is_reduce_op(*n->op);
+            n->leaf = !n->is_data && !n->shared && (is_gemm_op(*n->op) || is_reduce_op(*n->op));
         }
         if (r->row)
             for (const Var &v : r->row_outputs) step.outputs.push_back(slot(v.key()));
@@ -1059,7 +1059,7 @@ struct FirstRun {
 // A run along the schedule.  Out of memory, it hands what it has computed to the general run, which evicts and recomputes.
 //
 // Steps that follow one another and whose results no step reads (a training step ends with the gradients of all parameters) leave
-// column sums to a batch: one pass for all of them.  What they read lives until the batch has run, as it
+// products and column sums to a batch: one launch for all of a kind.  What they read lives until the batch has run, as it
 // did at the first of them.
 static sage_status exec_scheduled(Program &p, Context &ctx, Session &s) {
     if (!p.times_read) {  // timers of the first run

@@ -227,7 +227,9 @@ sage_status column_sums_run(Context &ctx, const std::vector<ColumnSum> &all) {
 
 sage_status LeafBatch::run(Context &ctx) {
     sage_status st = SAGE_OK;
-    if (!column_sums.empty()) st = column_sums_run(ctx, column_sums);
+    if (!products.empty()) st = gemm_tc_group_run(ctx, products);
+    if (!st && !column_sums.empty()) st = column_sums_run(ctx, column_sums);
+    products.clear();
     column_sums.clear();
     held.clear();
     return st;

@@ -386,6 +386,15 @@ sage_status bounded_wait_selftest(Context &ctx) {
     return ctx.check_cuda(cudaGetLastError(), "bounded_wait_probe launch");
 }
 
+// The tensor map of an operand without a batch for gemm_group.cu: whole K-blocks of an MN-major operand in one load where that
+// can be (*blocked).
+bool encode_tc_operand(const TcOperand &op, unsigned box_rows, bool kmajor, bool *blocked, CUtensorMap *map) {
+    static const PFN_encodeTiled encode = reinterpret_cast<PFN_encodeTiled>(driver_symbol("cuTensorMapEncodeTiled"));
+    if (!encode || !tc_operand_ok(op)) return false;
+    *blocked = mn_blocked_ok(op, kmajor) && encode_map(encode, op, 32, false, map, box_rows / 32);
+    return *blocked || encode_map(encode, op, kmajor ? box_rows : 32, kmajor, map);
+}
+
 // ---------------------------------------------------------------------------------- split launchers
 sage_status split_tf32_flat(Context &ctx, const float *src, long long n, float *dst_hi, long long plane) {
     ctx.note_launch("split_tf32");
@@ -427,6 +436,7 @@ static bool pairs_on() {
     static const bool on = !(getenv("SAGE_GEMM_PAIR") && atoi(getenv("SAGE_GEMM_PAIR")) == 0);
     return on;
 }
+bool gemm_tc_pairs() { return pairs_on(); }
 
 // Chooses the number of K slices and the tile width together.  Cost model (microseconds, from the
 // measured launches): the main loop is bound by operand delivery from L2, ~50 GB/s per SM, i.e. a K block

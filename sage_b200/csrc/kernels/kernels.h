@@ -172,12 +172,16 @@ sage_status gemm_tc_run(Context &ctx, const TcGemm &g);
 // How many K slices gemm_tc_run would cut this product into (0 = none).  Only products without an epilogue are
 // cut; a caller with an epilogue may ask for the plain product and apply the epilogue to the sum itself.
 int gemm_tc_split_plan(Context &ctx, const TcGemm &g);
+// gemm_group.cu: may this product run beside others in one launch; and that launch (several, where there are very many).
+bool gemm_tc_groupable(const TcGemm &g);
+sage_status gemm_tc_group_run(Context &ctx, const std::vector<TcGemm> &all);
 // Work that nothing of a program reads, put off until launches of one kind can be made together.  `held` keeps alive what it reads
 // and writes.
 struct LeafBatch {
     std::vector<ColumnSum> column_sums;
+    std::vector<TcGemm> products;
     std::vector<std::shared_ptr<void>> held;
-    bool empty() const { return column_sums.empty(); }
+    bool empty() const { return column_sums.empty() && products.empty(); }
     sage_status run(Context &ctx);  // ... and empties it
 };
 // hi/lo split of `n` consecutive floats into planes laid out like the source (dst_hi[i], dst_hi[plane + i]).

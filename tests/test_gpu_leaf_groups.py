@@ -1,11 +1,62 @@
-"""Column sums that nothing of a program reads, in one pass over all of them (kernels/column_sums.cu): rows of one chunk and of many,
-columns past one block, both widths of load."""
+"""Results that nothing of a program reads, computed together: products in one launch (kernels/gemm_group.cu), column sums in one pass
+(kernels/column_sums.cu).  Gradients of s = sum(((X W) + b) * C) over W (X^T C) and b (the column sums of C) for matrices of many
+sizes in one program."""
 import numpy as np
 import pytest
 
 import sage_b200 as S
 
 pytestmark = pytest.mark.gpu
+
+# (rows, inputs, outputs): K of one chain and of many slices, ragged M, N and K, tiles of every width, single columns (130 + 1), a
+# pair's second CTA without rows, rows of one chunk, columns past one block
+SIZES = {
+    "two": [(64, 64, 32), (4096, 768, 768)],
+    "narrow": [(6272, 576, 64), (25088, 49, 64), (6271, 65, 33), (100, 2304, 96), (4100, 300, 160)],
+    "wide": [(130, 257, 1001), (2049, 256, 2052), (512, 1152, 260), (96, 4608, 512), (1000, 129, 131)],
+    "many": [(64 + 37 * i, 64 + 29 * (i % 7), 32 + 13 * (i % 11)) for i in range(15)],
+}
+
+
+@pytest.mark.parametrize("which", sorted(SIZES))
+def test_gradients_of_many_products(which):
+    rng = np.random.default_rng(len(which))
+    ctx = S.Context(0)
+    try:
+        ctx_vars, xs, cs, loss = [], [], [], None
+        for rows, k, n in SIZES[which]:
+            x = (rng.standard_normal((rows, k)) * np.exp2(rng.integers(-12, 12, (1, k)))).astype(np.float32)
+            c = (rng.standard_normal((rows, n)) + 0.25).astype(np.float32)
+            w, b = ctx.var(np.zeros((k, n), np.float32)), ctx.var(np.zeros((n,), np.float32))
+            s = ((ctx.var(x).matmul(w) + b) * ctx.var(c)).sum([0, 1], False)
+            loss = s if loss is None else loss + s
+            xs.append(x)
+            cs.append(c)
+            ctx_vars.append((w, b))
+        targets = [v.grad(loss) for pair in ctx_vars for v in pair]
+        runs = []
+        for _ in range(2):
+            ctx.clear()
+            ctx.eval(*targets)
+            runs.append([ctx.read(t).copy() for t in targets])
+        assert ctx.status_word() == 0
+        for first, second in zip(*runs):  # the first pass and the later ones take the same way
+            assert np.array_equal(first, second)
+        before = ctx.launch_count()[0]
+        ctx.clear()
+        ctx.trace_begin()
+        ctx.eval(*targets)
+        assert len(ctx.trace()) - (ctx.launch_count()[0] - before) >= 2 * (len(xs) - 1)  # launches that did several results' work
+        for i, (x, c) in enumerate(zip(xs, cs)):
+            dw, db = runs[0][2 * i].reshape(x.shape[1], c.shape[1]), runs[0][2 * i + 1].reshape(-1)
+            x64, c64 = x.astype(np.float64), c.astype(np.float64)
+            size = np.abs(x64).T @ np.abs(c64)
+            # the dropped low x low products, 48 truncating additions of a chain, a rounding for every chain
+            bound = (2.0 ** -22 + 48 * 2.0 ** -23 + (x.shape[0] / 128 + 1) * 2.0 ** -24) * size
+            assert (np.abs(dw - x64.T @ c64) <= bound).all(), (which, i)
+            assert (np.abs(db - c64.sum(0)) <= x.shape[0] * 2.0 ** -24 * np.abs(c64).sum(0)).all(), (which, i)
+    finally:
+        ctx.close()
 
 
 def test_column_sums_pass_on_what_is_not_finite():
