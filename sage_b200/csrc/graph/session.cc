@@ -1088,7 +1088,7 @@ static sage_status exec_scheduled(Program &p, Context &ctx, Session &s) {
         std::vector<std::pair<Var, Tensor>> batched;  // results that the batch computes
         auto flush = [&]() {
             const sage_status ran = batch.empty() ? SAGE_OK : batch.run(ctx);
-            if (ran == SAGE_OK)
+            if (ran == SAGE_OK && st == SAGE_OK)
                 for (auto &v : batched) s.data[v.first.key()] = v;
             batched.clear();
             return ran;
@@ -1097,7 +1097,7 @@ static sage_status exec_scheduled(Program &p, Context &ctx, Session &s) {
             Routine &f = *step.routine;
             if (!step.leaf && (st = flush())) break;
             FirstRun first(f, ctx);
-            const size_t before = batch.held.size();
+            const size_t before = batch.held.size() + batch.held_by_sums.size();
             if (f.row) {
                 std::vector<Tensor> outs;
                 st = row_program_run(*f.row, ctx, [&](const Var &k, Tensor *t) {
@@ -1117,7 +1117,7 @@ static sage_status exec_scheduled(Program &p, Context &ctx, Session &s) {
             for (size_t i = 0; i < step.outputs.size(); ++i)
                 if (p.is_output[step.outputs[i]]) {
                     const Var &v = f.row ? f.row_outputs[i] : f.output;
-                    if (batch.held.size() > before) batched.push_back({v, p.slots[step.outputs[i]]});
+                    if (batch.held.size() + batch.held_by_sums.size() > before) batched.push_back({v, p.slots[step.outputs[i]]});
                     else s.data[v.key()] = std::make_pair(v, p.slots[step.outputs[i]]);
                 }
             for (int n : step.release) p.slots[n] = Tensor();

@@ -36,7 +36,8 @@ struct PlaneOut {
     float *h2_marked = nullptr;  // the scales again, negative where a group is wide (gemm_h2_device.inc), for a reader that asks
 };
 
-// column_sums.cu — several [rows, cols] -> [cols] sums in one pass over all of them (src/ops/reduce.rs:258-325, kind Sum)
+// column_sums.cu — several [rows, cols] -> [cols] sums in one pass over all of them (src/ops/reduce.rs:258-325, kind Sum); with one
+// column and a pitch of 1 the sum over a whole tensor
 struct ColumnSum {
     const float *x = nullptr;
     float *y = nullptr;
@@ -175,14 +176,17 @@ int gemm_tc_split_plan(Context &ctx, const TcGemm &g);
 // gemm_group.cu: may this product run beside others in one launch; and that launch (several, where there are very many).
 bool gemm_tc_groupable(const TcGemm &g);
 sage_status gemm_tc_group_run(Context &ctx, const std::vector<TcGemm> &all);
-// Work that nothing of a program reads, put off until launches of one kind can be made together.  `held` keeps alive what it reads
-// and writes.
+// Work that nothing of a program reads, put off until launches of one kind can be made together.  `held` keeps alive what it
+// reads and writes.
 struct LeafBatch {
     std::vector<ColumnSum> column_sums;
     std::vector<TcGemm> products;
-    std::vector<std::shared_ptr<void>> held;
+    std::vector<std::shared_ptr<void>> held, held_by_sums;
+    size_t own_bytes = 0;  // of the sums' operands that nothing but the batch keeps alive
+    static constexpr size_t kMaxOwnBytes = (size_t)128 << 20;
     bool empty() const { return column_sums.empty() && products.empty(); }
     sage_status run(Context &ctx);  // ... and empties it
+    sage_status run_sums(Context &ctx);  // the sums alone
 };
 // hi/lo split of `n` consecutive floats into planes laid out like the source (dst_hi[i], dst_hi[plane + i]).
 sage_status split_tf32_flat(Context &ctx, const float *src, long long n, float *dst_hi, long long plane);

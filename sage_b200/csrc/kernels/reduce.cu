@@ -612,10 +612,11 @@ static sage_status launch_reduce(Context &ctx, int kind, const T *x, const Dims 
 }
 
 bool column_sum_of(int dtype, int kind, const void *x, const Dims &outer, const Dims &inner_in, void *y, ColumnSum *out) {
-    if (dtype != SAGE_F32 || kind != 0 || outer.ndim != 1 || outer.str[0] != 1 || inner_in.ndim < 1) return false;
+    if (dtype != SAGE_F32 || kind != 0 || inner_in.ndim < 1) return false;
     const RDims inner = canonical_inner(inner_in);
-    const long long cols = outer.ext[0], rows = inner.ext[0];
-    if (inner.ndim != 1 || inner.str[0] < cols || cols < 2 || rows < 64 || cols > (1LL << 30) || rows > (1LL << 40)) return false;
+    const long long cols = outer.size(), rows = inner.ext[0];
+    if (inner.ndim != 1 || rows < 64 || rows > (1LL << 40)) return false;
+    if (cols == 1 ? inner.str[0] != 1 : (outer.ndim != 1 || outer.str[0] != 1 || inner.str[0] < cols || cols < 2 || cols > (1LL << 30))) return false;
     out->x = static_cast<const float *>(x);
     out->y = static_cast<float *>(y);
     out->rows = rows;

@@ -80,3 +80,25 @@ def test_column_sums_pass_on_what_is_not_finite():
         assert ctx.status_word() == 0
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+def test_sums_over_whole_tensors(shift):
+    """Runs of one block and of many, an end inside a thread's loads, an operand off the 16-byte grid, and operands that exist only for
+    their sum, more of them than are kept at once."""
+    rng = np.random.default_rng(6)
+    ctx = S.Context(0)
+    try:
+        xs = [rng.standard_normal(n).astype(np.float32) for n in (64, 67, 16384, 16388, 3145728, 5000001)]
+        variables = [ctx.var(x) for x in xs]
+        if shift:
+            variables, xs = [v.slice(0, 1, v.extents[0]) for v in variables], [x[1:] for x in xs]
+        big = ctx.var(rng.standard_normal(1 << 23).astype(np.float32))
+        sums = [v.sum([0], False) for v in variables] + [(big * (i + 0.5)).sum([0], False) for i in range(10)]
+        ctx.eval(*sums)
+        big64 = ctx.read(big).astype(np.float64)
+        for got, x in zip((ctx.read(s).reshape(-1)[0] for s in sums), [x.astype(np.float64) for x in xs] + [big64 * (i + 0.5) for i in range(10)]):
+            assert abs(got - x.sum()) <= 64 * 2.0 ** -24 * np.abs(x).sum()  # fewer than 64 roundings on the way of any element
+        assert ctx.status_word() == 0
+    finally:
+        ctx.close()
