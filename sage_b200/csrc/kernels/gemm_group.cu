@@ -9,7 +9,7 @@
 // as far as the pairs' shares need evening out.  Weight gradients of a BERT-base step (72, 32 x 128 tokens) and of a ResNet-18
 // step (20, 128 images of 28 x 28): the figures are at gemm_tc_group_run.
 //
-// The arithmetic is gemm_tc_body's (gemm_tc_device.inc): 3xTF32, chains of 128 k, chains added in fp32 registers.
+// The arithmetic is gemm_tc_body's (gemm_tc_device.inc): 3xTF32, chains of at most 128 k, chains added in fp32 registers.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -45,6 +45,7 @@ struct alignas(64) GroupItem {
     int unit0;        // units of the items before this one
     int tiles_m, tiles_n;
     short bn, flags;
+    int chain;        // K-blocks of an accumulation chain
 };
 template <int MAX>
 struct GroupParams {
@@ -193,7 +194,7 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, 1) gemm_tc_group_kernel(c
             const unsigned long long a_desc0 = smem_desc(0u, a_kmajor ? 16u : (unsigned)(BK * 128), a_kmajor ? 8u * BK * 4u : 512u, a_kmajor ? 2u : 1u);
             const unsigned long long b_desc0 = smem_desc(0u, b_kmajor ? 16u : (unsigned)(BK * 128), b_kmajor ? 8u * BK * 4u : 512u, b_kmajor ? 2u : 1u);
             const unsigned a_step16 = (a_kmajor ? 32u : 1024u) >> 4, b_step16 = (b_kmajor ? 32u : 1024u) >> 4;
-            for (int kb_begin = g.kb0; kb_begin < g.kb1 && ok; kb_begin += kChunkKB, ++cg) {
+            for (int kb_begin = g.kb0; kb_begin < g.kb1 && ok; kb_begin += it.chain, ++cg) {
                 const int buf = cg & 1;
                 if (!mbar_wait_warp(&tmem_empty[buf], ((cg >> 1) & 1) ^ 1)) {
                     if (lane == 0) timeout(16);
@@ -202,7 +203,7 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, 1) gemm_tc_group_kernel(c
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned tmem_d = tmem_base + (unsigned)(buf * kGroupBN);
-                const int kb_end = min(g.kb1, kb_begin + kChunkKB);
+                const int kb_end = min(g.kb1, kb_begin + it.chain);
                 for (int kb = kb_begin; kb < kb_end; ++kb) {
                     if (!mbar_wait_warp(&full_bar[s], s_parity)) {
                         if (lane == 0 && !abort_flag) timeout(4);
@@ -249,7 +250,7 @@ __global__ void __launch_bounds__(64 + 32 * kEpiWarps, 1) gemm_tc_group_kernel(c
             const int part = it.bn / 4, runs = it.bn / 64;  // columns of this warp, in runs of 16
 #pragma unroll
             for (int i = 0; i < 64; ++i) acc[i] = 0.f;
-            for (int kb = g.kb0; kb < g.kb1; kb += kChunkKB, ++cg) {
+            for (int kb = g.kb0; kb < g.kb1; kb += it.chain, ++cg) {
                 const int buf = cg & 1;
                 ok = mbar_wait_warp(&tmem_full[buf], (cg >> 1) & 1);
                 if (!ok) {
@@ -379,6 +380,11 @@ bool aligned16(const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0;
 // cycle and pair (72 products of a BERT-base step: 8.1 TB/s).
 int kb_cycles(int bn) { return (65536 + bn * 256) / 57; }
 
+// The tensor core truncates when it adds, so the length of a chain is most of the error.  Narrow tiles have time for more drains than
+// gemm_tc_body's one in 128 k, and long sums are theirs (error of X^T Y against float64, 25088 x 64 x 64: 9.0e-7 ... 9.4e-7 with
+// chains of 128; one launch a product, in slices of 392 k, 8.9e-7 ... 9.1e-7).
+int chain_kb(int bn) { return bn <= 128 ? 3 : kChunkKB; }
+
 struct Planned {
     const TcGemm *g;
     int bn, kb, slices, per_slice, tiles_m, tiles_n;
@@ -416,6 +422,7 @@ sage_status run_items(Context &ctx, std::vector<Planned> &plan, const std::vecto
         it.tiles_m = x.tiles_m;
         it.tiles_n = x.tiles_n;
         it.bn = (short)x.bn;
+        it.chain = chain_kb(x.bn);
         bool a_blocked = true, b_blocked = true;
         if (!encode_tc_operand(g.a, BM, g.a_kmajor, &a_blocked, &it.a) || !encode_tc_operand(g.b, (unsigned)(x.bn / 2), g.b_kmajor, &b_blocked, &it.b))
             return ctx.fail(SAGE_ERR_INVALID, "gemm_tc_group: operand not addressable by TMA");
@@ -481,7 +488,7 @@ sage_status gemm_tc_group_run(Context &ctx, const std::vector<TcGemm> &all) {
         for (Planned &x : plan) {
             long long s = (long long)((double)x.cost / most) + 1;
             s = std::max(1LL, std::min(s, (long long)x.kb / kMinKB));
-            x.per_slice = (int)(((x.kb + s - 1) / s + kChunkKB - 1) / kChunkKB * kChunkKB);  // whole chains
+            x.per_slice = (int)(((x.kb + s - 1) / s + chain_kb(x.bn) - 1) / chain_kb(x.bn) * chain_kb(x.bn));  // whole chains
             x.slices = (x.kb + x.per_slice - 1) / x.per_slice;
             x.cost = (long long)std::min(x.per_slice, x.kb) * kb_cycles(x.bn);
             if (x.slices > 1) floats += x.slices * ((x.g->m * x.g->n + 3) / 4 * 4);
