@@ -63,6 +63,7 @@ struct RowProgram {
     int regs = 80;  // registers per thread the kernel is compiled to fit
     std::vector<Val> vals;  // topological order
     std::vector<int> in_val, out_val;
+    std::vector<Var> out_var;  // the value under the shape it was asked for
     int n_map = 0, n_reduce = 0, n_index = 0;
     std::string source;
     uint32_t stage_bytes = 0;  // dynamic shared memory of the prefetch stages (0: inputs are loaded directly)
@@ -431,14 +432,25 @@ std::shared_ptr<RowProgram> row_program_build(const std::vector<Var> &evaluated,
     p->rows = R;
     p->cols = C;
     Builder b{*p, ev, {}, true};
+    bool reshaped = false;
     for (const Var &t : targets) {
-        const int id = b.add(t);
+        int id = b.add(t);
         if (!b.ok) return nullptr;
+        if (p->vals[id].kind == KAlias) {
+            // The value under another shape, contiguous: stored under that one.  (Not of a composite, which has a kernel of its own;
+            // and as part of a larger program, where it is worth a generated kernel for its reductions.)
+            id = p->resolve(id);
+            const Shape &sh = t.desc.shape;
+            if (whole_program || !sh.has_default_strides() || sh.offset || t.size() != p->vals[id].var.size() || p->vals[id].var.origin->composite) return nullptr;
+            reshaped = true;
+        }
         Val &v = p->vals[id];
-        if (v.kind == KLeaf || v.kind == KAlias || v.cls == Scalar || v.output >= 0) return nullptr;
+        if (v.kind == KLeaf || v.cls == Scalar || v.output >= 0) return nullptr;
         v.output = (int)p->out_val.size();
         p->out_val.push_back(id);
+        p->out_var.push_back(t);
     }
+    if (reshaped && p->n_reduce + p->n_index == 0) return nullptr;
     bool full_leaf = false;
     for (int id : p->in_val) full_leaf = full_leaf || p->vals[id].cls == Full;
     if (whole_program && (!full_leaf || p->n_reduce + p->n_index == 0)) return nullptr;
@@ -523,7 +535,7 @@ sage_status row_program_exec(RowProgram &p, Context &ctx, Session &s) {
     sage_status st = row_program_run(p, ctx, [&](const Var &v, Tensor *t) { return s.get(v, t); }, &outs);
     if (st) return st;
     for (size_t i = 0; i < p.out_val.size(); ++i) {
-        const Var &v = p.vals[p.out_val[i]].var;
+        const Var &v = p.out_var[i];
         s.data[v.key()] = std::make_pair(v, outs[i]);
     }
     return SAGE_OK;
@@ -574,7 +586,7 @@ sage_status row_program_run(RowProgram &p, Context &ctx, const std::function<boo
     std::vector<Tensor> &outs = *outs_;
     outs.assign(p.out_val.size(), Tensor());
     for (size_t i = 0; i < p.out_val.size(); ++i) {
-        sage_status st = Tensor::uninit(ctx, p.vals[p.out_val[i]].var.desc, &outs[i]);
+        sage_status st = Tensor::uninit(ctx, p.out_var[i].desc, &outs[i]);
         if (st) return st;
         pb[2 + nin + i] = (uint64_t)reinterpret_cast<uintptr_t>(outs[i].ptr());
         const Val &ov = p.vals[p.out_val[i]];

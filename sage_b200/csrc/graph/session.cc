@@ -689,7 +689,7 @@ static std::vector<RowGroupPlan> plan_row_groups(const std::vector<Var> &order, 
     // several kernels); a lone map chain already is one kernel, and a lone softmax / log_sum_exp /
     // layer_norm has its hand-written kernel (which also writes the tf32 planes a GEMM reads next)
     for (int g = 0; g < n; ++g)
-        if (members[g].size() >= 2 || (members[g].size() == 1 && ok[g] && exchanges[g] && !order[g].origin->composite)) {
+        if (members[g].size() >= 2 || (members[g].size() == 1 && ok[g] && exchanges[g] && !order[g].origin->composite && !is_view_op(*order[g].origin->op))) {
             RowGroupPlan plan;
             plan.members = members[g];
             std::sort(plan.members.begin(), plan.members.end());
