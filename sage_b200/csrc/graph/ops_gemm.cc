@@ -1093,6 +1093,28 @@ std::shared_ptr<Operator> gemm_with_store(const Operator &op, const Shape &view,
     return c;
 }
 
+// The same for a view in which the product's columns do not lie contiguous but its rows would: the product of the transposes, with
+// its operands exchanged.
+std::shared_ptr<Operator> gemm_with_transposed_store(const Operator &op, const Shape &view, const TensorDesc &out, bool tc_enabled) {
+    const GemmOp *g = as_gemm(op);
+    if (!g || g->folded || g->conv || g->attn || g->h2 || g->row_softmax || !g->epilogue.empty() || g->naux() || view.offset != 0 || !gemm_runs_on_tc(op, tc_enabled)) return nullptr;
+    auto c = lowered_clone(*g);
+    if (!k::gemm_tc_shape_ok(c->n, c->m, c->k, c->batch)) return nullptr;
+    Shape turned = view;  // into the transposes' [batch, N, M]
+    for (size_t d = 0; d < turned.strides.size(); ++d) {
+        const long long s = view.strides[d];
+        if (view.extents[d] == 1 || s >= c->m * c->n) continue;
+        if (s >= c->n ? s % c->n != 0 || s * view.extents[d] > c->m * c->n : s < 1 || s * view.extents[d] > c->n) return nullptr;
+        turned.strides[d] = s >= c->n ? s / c->n : s * c->m;
+    }
+    std::swap(c->in[0], c->in[1]);
+    std::swap(c->m, c->n);
+    const bool ta = c->ta;
+    c->ta = !c->tb;
+    c->tb = !ta;
+    return gemm_with_store(*c, turned, out, tc_enabled);
+}
+
 // softmax over the last axis of a product whose rows fit one tile (n <= 256): computed by the GEMM's
 // epilogue warps before the store, so neither the scores nor a softmax kernel touch memory.
 // Opt-in (pattern_fusion bit 1): on the BERT-base step it measured slower than the separate row

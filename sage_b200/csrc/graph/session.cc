@@ -55,6 +55,7 @@ std::shared_ptr<Operator> gemm_with_epilogue(const Operator &op, const std::stri
                                              const TensorDesc &out);
 std::shared_ptr<Operator> gemm_with_im2col(const Operator &op, const Operator &im2col_op, bool tc_enabled);
 std::shared_ptr<Operator> gemm_with_store(const Operator &op, const Shape &view, const TensorDesc &out, bool tc_enabled);
+std::shared_ptr<Operator> gemm_with_transposed_store(const Operator &op, const Shape &view, const TensorDesc &out, bool tc_enabled);
 bool row_op_emits_planes(const Operator &op);
 bool row_op_is_softmax(const Operator &op, long long *rows, long long *cols);
 std::shared_ptr<Operator> gemm_with_row_softmax(const Operator &op, long long rows, long long cols, const TensorDesc &out, bool tc_enabled);
@@ -303,6 +304,8 @@ static bool attention_enabled() {
     return on;
 }
 
+static Node *skip_views(Node *p, long long *offset = nullptr);
+
 static void lower(Node &n, bool tc, bool softmax_in_gemm, bool attention) {
     if (n.is_data) return;
     if (attention && tc && is_gemm_op(*n.op) && n.args.size() == 2) {
@@ -439,8 +442,16 @@ static void lower(Node &n, bool tc, bool softmax_in_gemm, bool attention) {
         while (!p->is_data && is_view_op(*p->op)) p = &p->args[0];
         if (p != &n.args[0] && !p->is_data && is_gemm_op(*p->op)) {
             std::shared_ptr<Operator> f = gemm_with_store(*p->op, n.op->in[0].shape, n.op->out, tc);
+            bool swapped = false;
+            if (!f && p->args.size() == 2 && !p->shared) {
+                // rows and columns exchanged: the product of the transposes, of two results (weights stay operand B)
+                const Node *a = skip_views(&p->args[0]), *b = skip_views(&p->args[1]);
+                if ((!a->is_data || a->var.is_op()) && (!b->is_data || b->var.is_op())) f = gemm_with_transposed_store(*p->op, n.op->in[0].shape, n.op->out, tc);
+                swapped = f != nullptr;
+            }
             if (f) {
                 std::vector<Node> args = std::move(p->args);
+                if (swapped) std::swap(args[0], args[1]);
                 n.op = f;
                 n.args = std::move(args);
             }
@@ -474,7 +485,7 @@ static void lower(Node &n, bool tc, bool softmax_in_gemm, bool attention) {
 
 // Which values a tensor-core GEMM reads (through views only): in-tree producers get emit_planes,
 // states are collected so that their routine's root gets it.
-static Node *skip_views(Node *p, long long *offset = nullptr) {  // *offset: where in the producer's result the views start
+static Node *skip_views(Node *p, long long *offset) {  // *offset: where in the producer's result the views start
     if (offset) *offset = 0;
     for (;;) {
         if (p->is_data) return p;
@@ -732,6 +743,39 @@ static std::unique_ptr<Program> compile(const std::vector<Var> &x, std::vector<V
         if (kv.second >= 2 && v.is_op() && !xset.count(kv.first) && !yset.count(kv.first)) candidates.push_back(v);
     }
     for (const Var &v : y) candidates.push_back(v);
+    // A value that is a permuted copy of another one and that only products read (the heads of an attention block in a training
+    // step) is not kept: the products read the other one through the view, as they do where the copy has one reader.
+    std::unordered_set<Origin *> kept_instead;
+    if (pattern && tc) {
+        std::unordered_map<Origin *, std::vector<std::pair<Var, int>>> readers;
+        for (auto &kv : nodes)
+            if (kv.second.is_op() && !xset.count(kv.first)) {
+                const std::vector<Var> &kids = children(kv.second, pattern, nullptr);
+                for (size_t i = 0; i < kids.size(); ++i) readers[kids[i].key()].push_back({kv.second, (int)i});
+            }
+        const size_t before = candidates.size();
+        for (size_t i = 0; i < before; ++i) {
+            const Var v = candidates[i];
+            if (yset.count(v.key())) continue;
+            Var at = v;
+            auto below = [&](const Var &w) { return w.is_op() && !xset.count(w.key()) && !yset.count(w.key()) && !w.origin->composite && w.origin->inputs.size() == 1 && (w.key() == v.key() || edges[w.key()] == 1); };
+            while (below(at) && is_reshape_op(*at.origin->op) && reshape_keeps_matrix(*at.origin->op)) at = at.origin->inputs[0];
+            if (!below(at) || !is_copy_map(*at.origin->op) || at.origin->op->in[0].shape.has_default_strides()) continue;
+            const TensorDesc view = at.origin->op->in[0];
+            at = at.origin->inputs[0];
+            while (below(at) && is_view_op(*at.origin->op)) at = at.origin->inputs[0];
+            if (!at.is_op() || is_view_op(*at.origin->op) || !at.desc.shape.has_default_strides()) continue;
+            bool products = true;
+            for (auto &r : readers[v.key()]) {
+                std::shared_ptr<Operator> op;
+                children(r.first, pattern, &op);
+                if (!is_gemm_op(*op) || !gemm_with_operand_view(*op, r.second, view, tc)) products = false;
+            }
+            if (!products) continue;
+            candidates[i] = at;  // (perhaps one of them already)
+            kept_instead.insert(at.key());
+        }
+    }
     std::stable_sort(candidates.begin(), candidates.end(), [](const Var &a, const Var &b) {
         return a.t_order() != b.t_order() ? a.t_order() < b.t_order() : a.key() < b.key();
     });
@@ -739,7 +783,7 @@ static std::unique_ptr<Program> compile(const std::vector<Var> &x, std::vector<V
     std::unordered_map<Origin *, std::vector<Var>> states;
     std::vector<Var> state_order;
     for (const Var &node : candidates) {
-        if (states.count(node.key())) continue;
+        if (states.count(node.key()) || xset.count(node.key())) continue;
         std::unordered_map<Origin *, Var> inputs;
         size_t num_ops = 0;
         bool complex_op = false;
@@ -762,7 +806,7 @@ static std::unique_ptr<Program> compile(const std::vector<Var> &x, std::vector<V
                 shape_fail("uninitialized variable");
             }
         }
-        if (yset.count(node.key()) || complex_op || num_ops * inputs.size() > THRES) {
+        if (yset.count(node.key()) || kept_instead.count(node.key()) || complex_op || num_ops * inputs.size() > THRES) {
             std::vector<Var> in;
             for (auto &kv : inputs) in.push_back(kv.second);
             states[node.key()] = in;

@@ -1,0 +1,57 @@
+"""What a training step's plan leaves out: copies of the attention heads that only products read (they read them through the view),
+the copy behind a product whose transpose has the wanted layout, and passes of a softmax's gradient beside its row program."""
+import numpy as np
+import pytest
+
+import sage_b200 as S
+
+
+def gradients(ctx, heads, d, length, batch, layers=1, seed=0):
+    w = heads * d
+    rng = np.random.default_rng(seed)
+    model = S.Bert(embed_dim=w, num_vocabs=50, max_num_tokens=max(length, 4), hidden_dim=2 * w, num_layers=layers, num_heads=heads, num_classes=2)
+    for i, p in enumerate(model.params()):
+        ctx.set(p, (rng.standard_normal(p.extents) * 0.2 + (1.0 if p.extents == (1,) and i % 2 == 0 else 0.0)).astype(np.float32))
+    ids = ctx.var(rng.integers(0, 50, (batch, length)).astype(np.uint32))
+    mask = np.ones((batch, length), np.float32)
+    mask[0, length - length // 4:] = 0
+    loss = S.softmax_cross_entropy(model.pass_(ids, ctx.var(mask)), ctx.var(rng.integers(0, 2, (batch, 1)).astype(np.uint32))).mean([0], False)
+    return [loss] + list(S.grad_param(loss, model).values())
+
+
+@pytest.mark.parametrize("heads,d,length", [(12, 64, 128), (3, 64, 72)])
+def test_no_copies_of_heads_are_left(heads, d, length):
+    c = S.Context(-1)
+    targets = gradients(c, heads, d, length, 4)
+    c.eval(*targets)
+    plan = c.describe()
+    copies = [line for line in plan.splitlines() if "map{(x0)}" in line and "permute" in line]
+    assert not copies, copies
+    assert plan.count("permute(reshape(state))") >= 4 and "[store]" in plan
+    assert "14 maps, 2 reductions" in plan  # the softmax's gradient, scale included, is one row program
+    c.close()
+
+
+# (34 elements a head: rows off the 16-byte grid, which TMA cannot read: the copies stay)
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,d,length,batch", [(2, 64, 64, 2), (3, 36, 72, 3), (3, 20, 72, 2), (2, 34, 65, 2), (1, 32, 128, 2), (4, 64, 33, 5)])
+def test_gradients_are_those_of_the_plain_evaluation(heads, d, length, batch):
+    """Against the same graph evaluated operator by operator.  Gradients are sums of a few thousand products through two row
+    normalisations: the largest difference stays below 2^-14 of the gradient's largest element (rounding 2^-24 x sqrt(terms) ~ 2^-18,
+    times the amplification of two LayerNorms); of LayerNorm's scalars, sums over all n ~ 10^4 elements that cancel, sqrt(n) ~ 2^7 less."""
+    got = []
+    for fusion in (1, 0):
+        c = S.Context(0, pattern_fusion=fusion)
+        try:
+            targets = gradients(c, heads, d, length, batch, layers=2)
+            for _ in range(2):
+                c.clear()
+                c.eval(*targets)
+            got.append([c.read(t).copy() for t in targets])
+            assert c.status_word() == 0
+        finally:
+            c.close()
+    assert np.abs(got[0][0] - got[1][0]).max() <= 1e-5 * max(1.0, np.abs(got[1][0]).max())
+    scale = max(np.abs(g).max() for g in got[1][1:])
+    for a, b in zip(got[0][1:], got[1][1:]):
+        assert np.abs(a - b).max() <= 2.0 ** (-14 if a.size > 1 else -14 + 7) * max(np.abs(b).max(), 2.0 ** -10 * scale)
