@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdlib>
+#include <cstring>
 #include <mutex>
 
 #include "kernels.h"
@@ -932,6 +933,17 @@ static SlicePlan plan_slices(const Context &ctx, const H2Gemm &g) {
     return best <= 0.8 * whole ? plan : none;
 }
 
+// Does the expression call a function of more than a few instructions?
+static bool long_expression(const std::string &e) {
+    static const char *const kShort[] = {"lit", "abs", "square", "sign", "min", "max", "ceil", "floor", "round", "recip"};
+    for (size_t at = e.find("sg_"); at != std::string::npos; at = e.find("sg_", at + 3)) {
+        bool is_short = false;
+        for (const char *name : kShort) is_short = is_short || e.compare(at + 3, strlen(name), name) == 0;
+        if (!is_short) return true;
+    }
+    return false;
+}
+
 sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
     const PFN_encodeTiled encode = ctx.dry() ? nullptr : encode_tiled();
     const PFN_encodeIm2col encode_conv = ctx.dry() ? nullptr : encode_im2col_mode();
@@ -1073,8 +1085,14 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
     const int threads = sliced ? 64 + 2 * bn : kThreads;
 
     const int out_mask = (g.c ? 1 : 0) | (g.c_hi ? 2 : 0) | (g.h_hi ? 4 : 0) | (g.h_hi && g.h_marked ? 8 : 0);
+    // A store that is worked through once is bound by the fetching of its instructions: its four sub-tiles in a loop, where no operand's
+    // rows have to be on their way meanwhile (a residual: 32 x 128 tokens of BERT-base 2850 -> 3117 us).  The same for an expression so
+    // long that a tile's four copies of it are slower to fetch than to repeat.  us, unrolled | as chosen: GELU on 6 x 77 tokens 986 | 948,
+    // 2 x 64 816 | 768, 12 x 128 1617 | 1502, 32 x 128 3018 | 2968 (only single tiles: 3022); without it 6 x 77 894 | 884, 2 x 64 705 |
+    // 700, 12 x 128 1411 | 1406, 16 x 128 of width 512 595 | 599.  Several tiles and a short expression: 32 x 128 2762 | 2786 if rolled.
+    const bool roll = !sliced && rowinv == (1 << g.naux) - 1 && (p.num_tiles <= slots || long_expression(g.epilogue));
     char num[96];
-    snprintf(num, sizeof num, "gemm_h2 %d %d %d %d %d %d %d %d %d\n", bn, ctas, sliced ? 1 : 0, aux_vec ? 1 : 0, (g.conv ? (halo ? 2 : boxed ? 3 : 1) : 0) + (fetch ? 4 : 0), g.naux, rowinv, per_col, out_mask);
+    snprintf(num, sizeof num, "gemm_h2 %d %d %d %d %d %d %d %d %d %d\n", roll ? 1 : 0, bn, ctas, sliced ? 1 : 0, aux_vec ? 1 : 0, (g.conv ? (halo ? 2 : boxed ? 3 : 1) : 0) + (fetch ? 4 : 0), g.naux, rowinv, per_col, out_mask);
     const bool plain = !g.conv && g.naux == 0 && g.epilogue.empty() && out_mask == 1;
     const std::string key = num + g.epilogue;
     Module *mod = plain ? nullptr : ctx.module_find(key);
@@ -1090,6 +1108,7 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
         define("SAGE_H2_AUX_VEC", aux_vec ? 1 : 0);
         define("SAGE_H2_HALO", halo ? 1 : 0);
         define("SAGE_H2_FETCH", fetch ? 1 : 0);
+        define("SAGE_H2_ROLL", roll ? 1 : 0);
         src += "#define SAGE_EPI_EXPR(x0, x1, x2, x3) (" + (g.epilogue.empty() ? std::string("x0") : g.epilogue) + ")\n";
         src += kGemmTcDeviceSrc;
         src += kGemmH2DeviceSrc;

@@ -1,0 +1,45 @@
+"""Products whose store loops over its sub-tiles (kernels/gemm_h2_device.inc, SAGE_H2_ROLL): one tile a CTA, and expressions that call long
+functions, at the edges of tiles and sub-tiles, stored as fp32, as pieces for a following product, and both."""
+import numpy as np
+import pytest
+import torch
+
+import sage_b200 as S
+
+pytestmark = pytest.mark.gpu
+
+
+# rows, k, columns: one tile cut in both directions; no whole 16 bytes in a row; whole groups of 64 (pieces); several tiles a CTA
+@pytest.mark.parametrize("m,k,n", [(129, 256, 192), (200, 320, 97), (462, 768, 3072), (4096, 512, 2048), (130, 64, 130), (5000, 256, 1000)])
+@pytest.mark.parametrize("long", [False, True])
+def test_epilogues(m, k, n, long):
+    """Against float64: the product within 2^-19 of |x| |w| (its bound, tests of the half-precision products), through a function whose
+    slope is at most 1.13, and the second product, of 64 columns, likewise."""
+    rng = np.random.default_rng(m + n)
+    x, w, b = rng.standard_normal((m, k)).astype(np.float32), (rng.standard_normal((k, n)) / np.sqrt(k)).astype(np.float32), rng.standard_normal(n).astype(np.float32)
+    w2 = (rng.standard_normal((n, 64)) / np.sqrt(n)).astype(np.float32)
+    ctx = S.Context(0)
+    try:
+        h = ctx.var(x).matmul(ctx.var(w)) + ctx.var(b)
+        y = h * 0.5 * ((h * 0.70710678).erf() + 1.0) if long else S.relu(h)
+        z = y.matmul(ctx.var(w2))
+        got_y = y.eval(ctx).copy()
+        ctx.clear()
+        got_z = z.eval(ctx).copy()
+        ctx.clear()
+        ctx.eval(y, z)
+        both = ctx.read(y).copy(), ctx.read(z).copy()
+        assert ctx.status_word() == 0
+    finally:
+        ctx.close()
+    x64, w64 = torch.from_numpy(x).double(), torch.from_numpy(w).double()
+    h64 = x64 @ w64 + torch.from_numpy(b).double()
+    size = x64.abs() @ w64.abs() + torch.from_numpy(b).double().abs()
+    y64 = h64 * 0.5 * (torch.erf(h64 * np.float64(np.float32(0.70710678))) + 1) if long else h64.clamp(min=0)
+    y_bound = 2.0 ** -19 * size
+    w2_64 = torch.from_numpy(w2).double()
+    z_bound = y_bound @ w2_64.abs() + 2.0 ** -19 * (y64.abs() @ w2_64.abs())
+    for a in (got_y, both[0]):
+        assert ((torch.from_numpy(a).double() - y64).abs() <= y_bound).all()
+    for a in (got_z, both[1]):
+        assert ((torch.from_numpy(a).double() - y64 @ w2_64).abs() <= z_bound).all()
