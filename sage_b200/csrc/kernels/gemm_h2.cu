@@ -17,10 +17,12 @@
 #include "gemm_tc_device.inc"
 #include "gemm_h2_device.inc"
 #include "attn_tc_device.inc"  // AttnParams and the tile constants; the kernel itself is only compiled by NVRTC
+#include "attn_small_device.inc"
 #include "gemm_tc_device_src.h"
 #include "gemm_h2_device_src.h"
 #include "attn_quads_device_src.h"
 #include "attn_rows_device_src.h"
+#include "attn_small_device_src.h"
 #include "attn_tc_device_src.h"
 #include "conv_first_device.inc"
 #include "conv_first_device_src.h"
@@ -1318,6 +1320,52 @@ sage_status attention_tc_run(Context &ctx, const TcAttn &a) {
     p.aux_vec = aux_vec ? 1 : 0;
     if (a.out.h2 && (!vec || a.d != 64 || a.ldo % 64 || a.so0 % 64 || a.so1 % 64 || !aligned16(a.out.h2) || a.out.h2_plane % 8))
         return ctx.fail(SAGE_ERR_INVALID, "attention_tc: a result in half-precision pieces needs whole groups of 64 columns");
+    // Few short sequences: attn_small_device.inc.  Up to 16 keys always; up to 32 where its blocks are few, or so many that the other
+    // form's tiles, a quarter or less filled, come in rounds; up to 48 where there is hardly anything to do.  In between its many small blocks
+    // leave the next product's less room to start early.  us a layer of BERT (other form | this one; 12 heads unless said otherwise):
+    // 8 tokens x 1 51.98 | 45.76, x 16 55.92 | 51.61, x 64 79.33 | 62.33; 16 x 1 60.64 | 53.92, x 4 44.38 | 43.05, x 64 92.44 | 78.04;
+    // 24 x 1 44.38 | 40.79, x 4 50.22 | 49.04, x 8 (96 blocks) [55.67] | 58.69, x 32 74.76 | 70.80; 32 x 1 44.15 | 41.70, x 2 46.12 | 43.79,
+    // x 4 [53.22] | 54.74, x 16 [63.72] | 66.46, x 32 (384) 82.15 | 80.91, x 64 113.76 | 102.89, 4 heads x 64 (256) [59.71] | 61.59;
+    // 40 x 1 44.82 | 42.77, x 2 (48) [49.46] | 51.95; 48 x 1 45.94 | 42.75, 4 heads x 4 (32) [45.64] | 46.36; 64 x 1 [45.42] | 45.93.
+    const long long small_blocks = (a.lq + kSmallQ - 1) / kSmallQ * a.batch;
+    const bool few = a.lq <= kSmallQ && a.lk <= 32 ? a.lk <= 16 || small_blocks <= 36 || 2 * small_blocks >= 5 * ctx.sm_count : a.lq <= 2 * kSmallQ && a.lk <= 48 && small_blocks <= 24;
+    auto operand_ok = [](const AttnOperand &o) { return o.hi && aligned16(o.hi) && o.ld % 8 == 0 && o.plane % 8 == 0 && o.sb0 % 8 == 0 && o.sb1 % 8 == 0; };
+    if (few && (ctx.dry() || (operand_ok(a.q) && operand_ok(a.k) && operand_ok(a.v)))) {
+        const int nk = (int)((a.lk + 31) / 32), out_mask = (a.o ? 1 : 0) | (a.out.hi ? 2 : 0) | (a.out.h2 ? 4 : 0);
+        AttnSmallParams sp{};
+        p.tiles_q = (int)((a.lq + kSmallQ - 1) / kSmallQ);
+        sp.h = p;
+        auto source = [](const AttnOperand &o) { return AttnSource{o.hi, o.plane, o.ld, o.sb0, o.sb1, (int)o.nb0}; };
+        sp.q = source(a.q);
+        sp.k = source(a.k);
+        sp.v = source(a.v);
+        char num[64];
+        snprintf(num, sizeof num, "attention_small %d %d %d %d\n", nk, a.naux, rowinv_mask, out_mask);
+        const std::string key = num + a.epilogue;
+        Module *mod = ctx.module_find(key);
+        if (!mod) {
+            std::string src = map_prelude_text();
+            src += "struct __align__(64) CUtensorMap { unsigned long long opaque[16]; };\n#define SAGE_ATTN_NK " + std::to_string(nk) + "\n";
+            src += "#define SAGE_EPI_NAUX " + std::to_string(a.naux) + "\n#define SAGE_EPI_ROWINV " + std::to_string(rowinv_mask) + "\n#define SAGE_EPI_OUT " + std::to_string(out_mask) + "\n";
+            src += "#define SAGE_EPI_EXPR(x0, x1, x2, x3) (" + (a.epilogue.empty() ? std::string("x0") : a.epilogue) + ")\n";
+            src += kGemmTcDeviceSrc;
+            src += kGemmH2DeviceSrc;
+            src += kAttnTcDeviceSrc;
+            src += kAttnSmallDeviceSrc;
+            src += "\nextern \"C\" __global__ void __launch_bounds__(sage_tc::kSmallThreads)\n"
+                   "attention_small(const __grid_constant__ sage_tc::AttnSmallParams p) {\n    sage_tc::attn_small_body(p);\n}\n";
+            sage_status st = ctx.module_get(src, &mod);
+            if (st) return st;
+            ctx.module_remember(key, mod);
+        }
+        std::string label;
+        if (ctx.verbose_names) label = "attention_tc_h2[" + std::to_string(a.lq) + "x" + std::to_string(a.lk) + "x" + std::to_string(a.d) + "x" + std::to_string(a.batch) + ",small]";
+        const size_t smem = sizeof(float) * ((size_t)kSmallQ * kSmallPitch + (size_t)nk * 32 * (kSmallPitch + 64 + kSmallThreads / 32 * 4));
+        const uint32_t gr[3] = {(uint32_t)small_blocks, 1, 1}, bl[3] = {(uint32_t)kSmallThreads, 1, 1};
+        void *params[1] = {&sp};
+        // launch lists have one name for the fused attention; verbose ones tell the kernels apart
+        return ctx.launch(mod, "attention_small", gr, bl, (uint32_t)smem, params, ctx.verbose_names ? label.c_str() : "attention_tc_3xtf32", true);
+    }
     // Q, the K / V ring, 1 KiB per softmax warp for turning the output round, and the slack for 1024-byte alignment
     // A thread per row where throughput counts: two tiles and more for every SM, more than three blocks of keys each.  With few
     // tiles and blocks the way through a single tile is what the next kernel waits for (32 x 128 in a BERT-base pass: 2809 us, 2845
