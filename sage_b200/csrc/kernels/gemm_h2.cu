@@ -663,6 +663,14 @@ static bool encode_operand(PFN_encodeTiled encode, const H2Operand &op, long lon
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// A row-dependent operand of the expression, in boxes of 128 rows x 32 columns.
+static bool encode_residual(PFN_encodeTiled encode, const TcAuxArg &x, long long m, long long n, CUtensorMap *map) {
+    const cuuint64_t dims[2] = {(cuuint64_t)n, (cuuint64_t)m}, strides[1] = {(cuuint64_t)x.sr * 4};
+    const cuuint32_t box[2] = {32, BM}, estr[2] = {1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(x.ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // One piece of an NHWC image: im2col mode, 64 channels of 128 output pixels.
 static bool encode_im2col(PFN_encodeIm2col encode, const H2Gemm &g, const unsigned short *base, CUtensorMap *map) {
     const cuuint64_t dims[4] = {(cuuint64_t)g.img_c, (cuuint64_t)g.img_w, (cuuint64_t)g.img_h, (cuuint64_t)g.img_n};
@@ -1087,6 +1095,13 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
     const int threads = sliced ? 64 + 2 * bn : kThreads;
 
     const int out_mask = (g.c ? 1 : 0) | (g.c_hi ? 2 : 0) | (g.h_hi ? 4 : 0) | (g.h_hi && g.h_marked ? 8 : 0);
+    // A residual through shared memory, where the ring behind a CTA's only tile takes it.  us, fetched by the store | this: BERT-base 32 x 128
+    // 2790 | 2741, 12 x 128 1414 | 1342, 8 x 200 1783 | 1700, of width 512 16 x 128 (6 layers) 610 | 578, 256 40 x 100 1016 | 930, 1024
+    // 20 x 128 (8) 2013 | 1965.  (With the store in a loop, as below, 32 x 128 2849.)
+    int res = 0;
+    if (!sliced && !g.conv && g.batch == 1 && p.num_tiles <= slots && vec && aux_vec)
+        for (int i = g.naux; i-- > 0;)
+            if (g.aux[i].sr > 0 && g.aux[i].sc == 1 && g.aux[i].sr < (1LL << 36)) res = i + 1;
     // A store that is worked through once is bound by the fetching of its instructions: its four sub-tiles in a loop, where no operand's
     // rows have to be on their way meanwhile (a residual: 32 x 128 tokens of BERT-base 2850 -> 3117 us).  The same for an expression so
     // long that a tile's four copies of it are slower to fetch than to repeat.  us, unrolled | as chosen: GELU on 6 x 77 tokens 986 | 948,
@@ -1094,7 +1109,7 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
     // 700, 12 x 128 1411 | 1406, 16 x 128 of width 512 595 | 599.  Several tiles and a short expression: 32 x 128 2762 | 2786 if rolled.
     const bool roll = !sliced && rowinv == (1 << g.naux) - 1 && (p.num_tiles <= slots || long_expression(g.epilogue));
     char num[96];
-    snprintf(num, sizeof num, "gemm_h2 %d %d %d %d %d %d %d %d %d %d\n", roll ? 1 : 0, bn, ctas, sliced ? 1 : 0, aux_vec ? 1 : 0, (g.conv ? (halo ? 2 : boxed ? 3 : 1) : 0) + (fetch ? 4 : 0), g.naux, rowinv, per_col, out_mask);
+    snprintf(num, sizeof num, "gemm_h2 %d %d %d %d %d %d %d %d %d %d %d\n", res, roll ? 1 : 0, bn, ctas, sliced ? 1 : 0, aux_vec ? 1 : 0, (g.conv ? (halo ? 2 : boxed ? 3 : 1) : 0) + (fetch ? 4 : 0), g.naux, rowinv, per_col, out_mask);
     const bool plain = !g.conv && g.naux == 0 && g.epilogue.empty() && out_mask == 1;
     const std::string key = num + g.epilogue;
     Module *mod = plain ? nullptr : ctx.module_find(key);
@@ -1111,6 +1126,7 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
         define("SAGE_H2_HALO", halo ? 1 : 0);
         define("SAGE_H2_FETCH", fetch ? 1 : 0);
         define("SAGE_H2_ROLL", roll ? 1 : 0);
+        define("SAGE_H2_RES", res);
         src += "#define SAGE_EPI_EXPR(x0, x1, x2, x3) (" + (g.epilogue.empty() ? std::string("x0") : g.epilogue) + ")\n";
         src += kGemmTcDeviceSrc;
         src += kGemmH2DeviceSrc;
@@ -1134,6 +1150,7 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
         if (!g.conv) {
             good = good && ok(g.a) && encode_operand(encode, g.a, g.k, BM, &map_a);
             map_a2 = map_a;
+            if (res) good = good && encode_residual(encode, g.aux[res - 1], g.m, g.n, &map_a2);
         } else {
             good = good && aligned16(g.a.hi) && g.a.plane % 8 == 0;
             if (halo)

@@ -43,3 +43,29 @@ def test_epilogues(m, k, n, long):
         assert ((torch.from_numpy(a).double() - y64).abs() <= y_bound).all()
     for a in (got_z, both[1]):
         assert ((torch.from_numpy(a).double() - y64 @ w2_64).abs() <= z_bound).all()
+
+
+# a residual through the operand ring: tiles of every width, one cut in both directions, rows longer than the result's, one tile and
+# several to a CTA, a single K-block, an operand off the 16-byte grid (which the store fetches itself)
+@pytest.mark.parametrize("m,k,n", [(129, 64, 64), (200, 320, 100), (300, 256, 128), (4096, 768, 768), (1536, 128, 192), (2000, 200, 516), (6000, 128, 1024), (130, 96, 260)])
+@pytest.mark.parametrize("wider,shift", [(0, 0), (8, 4), (8, 1)])
+def test_residuals(m, k, n, wider, shift):
+    """Against float64, within 2^-19 of |x| |w| + |r|."""
+    rng = np.random.default_rng(m + n + wider)
+    x, w, b = rng.standard_normal((m, k)).astype(np.float32), (rng.standard_normal((k, n)) / np.sqrt(k)).astype(np.float32), rng.standard_normal(n).astype(np.float32)
+    r = rng.standard_normal((m, n + wider)).astype(np.float32)
+    ctx = S.Context(0)
+    try:
+        rv = ctx.var(r)
+        if wider:
+            rv = rv.slice(1, shift, shift + n)
+        y = ctx.var(x).matmul(ctx.var(w)) + ctx.var(b) + rv
+        for _ in range(2):
+            ctx.clear()
+            got = y.eval(ctx).copy()
+        assert ctx.status_word() == 0
+    finally:
+        ctx.close()
+    x64, w64 = x.astype(np.float64), w.astype(np.float64)
+    r64 = r[:, shift:shift + n].astype(np.float64)
+    assert (np.abs(got - (x64 @ w64 + b + r64)) <= 2.0 ** -19 * (np.abs(x64) @ np.abs(w64) + np.abs(b) + np.abs(r64))).all()
