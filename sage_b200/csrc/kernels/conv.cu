@@ -320,6 +320,53 @@ __global__ void __launch_bounds__(256) pool2d_kernel(const float *__restrict__ i
     }
 }
 
+// Large windows, few results (the mean over 7 x 7 x 512 at an image model's end): a block has 64 channels of a result, four to a thread,
+// its 16 groups of threads share the window's taps, all of a thread's (of 64 at a time) in flight, and meet in shared memory in order.
+// A thread to four channels took 7.5 us, six rounds of nine taps each.
+__global__ void __launch_bounds__(256) pool2d_window_kernel(const float *__restrict__ img, float *__restrict__ out, ConvP p, int chan_blocks, int is_max, int ref_compat) {
+    constexpr int U = 4;
+    __shared__ float4 part[16][16];
+    grid_dependency_sync();
+    const int lane = threadIdx.x & 15, group = threadIdx.x >> 4, taps = p.w.ker_w * p.w.ker_h;
+    const long long pix = blockIdx.x / chan_blocks;
+    const int c = ((int)(blockIdx.x - pix * chan_blocks) * 16 + lane) * 4;
+    const long long per_img = p.col_h * p.col_w, n = pix / per_img;
+    const int r = (int)(pix - n * per_img), oy = r / (int)p.col_w, ox = r - oy * (int)p.col_w;
+    const int y0 = oy * p.w.stride_h - p.w.pad_h, x0 = ox * p.w.stride_w - p.w.pad_w;
+    const float *src = img + n * p.img_h * p.img_w * p.chan + c;
+    const float init = is_max ? (ref_compat ? 0.f : -INFINITY) : 0.f;
+    float4 acc = make_float4(init, init, init, init);
+    auto take = [&](float4 &a, const float4 &v) {
+        a.x = is_max ? fmaxf(a.x, v.x) : a.x + v.x;
+        a.y = is_max ? fmaxf(a.y, v.y) : a.y + v.y;
+        a.z = is_max ? fmaxf(a.z, v.z) : a.z + v.z;
+        a.w = is_max ? fmaxf(a.w, v.w) : a.w + v.w;
+    };
+    if (c < (int)p.chan) {
+        for (int t = group; t < taps; t += 16 * U) {
+            float4 v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int tap = t + 16 * u, kx = tap / p.w.ker_h, ky = tap - kx * p.w.ker_h, iy = y0 + ky * p.w.dil_h, ix = x0 + kx * p.w.dil_w;
+                const bool in = tap < taps && ix >= 0 && ix < (int)p.img_w && iy >= 0 && iy < (int)p.img_h;
+                v[u] = in ? __ldg(reinterpret_cast<const float4 *>(src + ((long long)iy * p.img_w + ix) * p.chan)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (t + 16 * u < taps) take(acc, v[u]);
+        }
+    }
+    part[group][lane] = acc;
+    __syncthreads();
+    if (group || c >= (int)p.chan) return;
+    for (int g = 1; g < 16; ++g) take(acc, part[g][lane]);
+    if (!is_max) {
+        const float taps_f = (float)taps;
+        acc = make_float4(acc.x / taps_f, acc.y / taps_f, acc.z / taps_f, acc.w / taps_f);
+    }
+    *reinterpret_cast<float4 *>(out + pix * p.chan + c) = acc;
+}
+
 static unsigned grid_for(Context &ctx, long long n) {
     long long blocks = (n + 255) / 256;
     long long cap = (long long)ctx.sm_count * 32;
@@ -590,6 +637,12 @@ sage_status pool2d(Context &ctx, bool is_max, const float *img, float *out, long
     // 32-bit indices where they reach: two 64-bit divisions were a third of a thread's instructions
     const bool narrow = total < (1LL << 31) && img_h * img_w * chan < (1LL << 31);
     const bool mark = forms.h2 && forms.h2_marked;
+    const long long chan_blocks = (chan + 63) / 64;
+    // (from two rounds of taps on, while its blocks are few enough to run at once)
+    if (vec && out && !forms.h2 && w.ker_w * w.ker_h >= 16 && n * out_h * out_w * chan_blocks <= 4LL * ctx.sm_count && img_h <= 0x7fffffffLL && img_w <= 0x7fffffffLL) {
+        launch_dependent(ctx.pdl, ctx.stream(), pool2d_window_kernel, dim3((unsigned)(n * out_h * out_w * chan_blocks)), dim3(256), 0, img, out, p, (int)chan_blocks, is_max ? 1 : 0, (int)ctx.opts().ref_compat);
+        return ctx.check_cuda(cudaGetLastError(), "pool2d launch");
+    }
     auto kernel = narrow ? (mark ? pool2d_kernel<4, unsigned, true> : pool2d_kernel<4, unsigned, false>) : (mark ? pool2d_kernel<4, long long, true> : pool2d_kernel<4, long long, false>);
     if (vec) launch_dependent(ctx.pdl, ctx.stream(), kernel, dim3(grid_for(ctx, total / 4)), dim3(256), 0, img, out, p, total / 4, is_max ? 1 : 0, (int)ctx.opts().ref_compat, forms);
     else launch_dependent(ctx.pdl, ctx.stream(), pool2d_kernel<1, long long, false>, dim3(grid_for(ctx, total)), dim3(256), 0, img, out, p, total, is_max ? 1 : 0, (int)ctx.opts().ref_compat, forms);

@@ -114,23 +114,77 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(GemmP p) {
         }
     }
 }
-// Few outputs, long K (a classifier head: 32 x 2 outputs, K = 768): one warp per output element,
-// the lanes share K, so the tile kernel's single CTA walking K alone is avoided.
+// Few outputs, long K (a classifier head: 32 x 2 outputs, K = 768): one warp per output element, the lanes share K, so the tile
+// kernel's single CTA walking K alone is avoided.  Bound by latency: eight loads of each operand in flight to a lane, eight sums that
+// meet in pairs.  (One load at a time, 32 x 2 x 768: 12.4 us, of which a launch is 2.5.)
 __global__ void __launch_bounds__(256) gemm_skinny_kernel(GemmP p, long long sai, long long sak, long long sbk, long long sbj) {
-    grid_dependency_sync();
+    constexpr int U = 8;
     const int lane = threadIdx.x & 31;
     const long long out = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const long long per_batch = p.m * p.n;
-    if (out >= per_batch * p.batch) return;
     const long long bz = out / per_batch, rem = out % per_batch;
     const long long i = rem / p.n, j = rem % p.n;
-    const float *A = p.a + bz * p.sa + i * sai;
-    const float *B = p.b + bz * p.sb + j * sbj;
-    float acc = 0.f;
-    for (long long kk = lane; kk < p.k; kk += 32) acc = fmaf(A[kk * sak], B[kk * sbk], acc);
+    const float *A = p.a + bz * p.sa + i * sai + lane * sak;
+    const float *B = p.b + bz * p.sb + j * sbj + lane * sbk;
+    grid_dependency_sync();
+    if (out >= per_batch * p.batch) return;
+    float acc[U] = {};
+    const long long left = p.k - lane;  // this lane's first k inside
+    for (long long kk = 0; kk < left; kk += 32 * U) {
+        float a[U], b[U];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-    if (lane == 0) p.c[bz * p.sc + i * p.ldc + j] = acc;
+        for (int u = 0; u < U; ++u) {
+            const bool in = kk + 32 * u < left;
+            a[u] = in ? A[(kk + 32 * u) * sak] : 0.f;
+            b[u] = in ? B[(kk + 32 * u) * sbk] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (kk + 32 * u < left) acc[u] = fmaf(a[u], b[u], acc[u]);
+    }
+#pragma unroll
+    for (int w = 1; w < U; w *= 2)
+#pragma unroll
+        for (int u = 0; u + w < U; u += 2 * w) acc[u] += acc[u + w];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], off);
+    if (lane == 0) p.c[bz * p.sc + i * p.ldc + j] = acc[0];
+}
+// The same where operand B's columns lie beside one another: a block takes 32 of them, a column to a lane, its 16 warps share K and
+// meet in shared memory.  Rows of 128 bytes instead of an element out of each 32 (1 x 1000 x 512, weights from memory: 11.8 us with a
+// warp per output).
+__global__ void __launch_bounds__(512) gemm_skinny_columns_kernel(GemmP p, long long sai, long long sak) {
+    constexpr int U = 8, WARPS = 16;
+    __shared__ float part[WARPS][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long tile_n = blockIdx.x % p.tiles_n, row = blockIdx.x / p.tiles_n, bz = row / p.m, i = row % p.m, j = tile_n * 32 + lane;
+    const float *A = p.a + bz * p.sa + i * sai + warp * sak, *B = p.b + bz * p.sb + warp * p.ldb + (j < p.n ? j : p.n - 1);
+    grid_dependency_sync();
+    float acc[U] = {};
+    const long long left = p.k - warp;
+    for (long long kk = 0; kk < left; kk += WARPS * U) {
+        float a[U], b[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool in = kk + WARPS * u < left;
+            a[u] = in ? A[(kk + WARPS * u) * sak] : 0.f;
+            b[u] = in ? B[(kk + WARPS * u) * p.ldb] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (kk + WARPS * u < left) acc[u] = fmaf(a[u], b[u], acc[u]);
+    }
+#pragma unroll
+    for (int w = 1; w < U; w *= 2)
+#pragma unroll
+        for (int u = 0; u + w < U; u += 2 * w) acc[u] += acc[u + w];
+    part[warp][lane] = acc[0];
+    __syncthreads();
+    if (warp || j >= p.n) return;
+    float sum = part[0][lane];
+#pragma unroll
+    for (int w = 1; w < WARPS; ++w) sum += part[w][lane];
+    p.c[bz * p.sc + i * p.ldc + j] = sum;
 }
 }  // namespace
 
@@ -140,6 +194,11 @@ sage_status gemm_simt(Context &ctx, const GemmArgs &g) {
     GemmP p{g.m, g.n, g.k, g.a, g.lda, g.stride_a, g.b, g.ldb, g.stride_b, g.c, g.ldc, g.stride_c, (g.n + BN - 1) / BN, (g.m + BM - 1) / BM, g.batch};
     const long long grid_limit = 0x7fffffffLL;
     if (g.m * g.n <= 8192 && g.k >= 128 && (g.m * g.n * g.batch + 7) / 8 <= grid_limit) {
+        if (!g.tb && g.n >= 32) {
+            p.tiles_n = (g.n + 31) / 32;
+            launch_dependent(ctx.pdl, ctx.stream(), gemm_skinny_columns_kernel, dim3((unsigned)(p.tiles_n * g.m * g.batch)), dim3(512), 0, p, g.ta ? 1 : g.lda, g.ta ? g.lda : 1);
+            return ctx.check_cuda(cudaGetLastError(), "gemm_skinny launch");
+        }
         const dim3 grid((unsigned)((g.m * g.n * g.batch + 7) / 8));
         launch_dependent(ctx.pdl, ctx.stream(), gemm_skinny_kernel, dim3(grid), dim3(256), 0, p, g.ta ? 1 : g.lda, g.ta ? g.lda : 1, g.tb ? 1 : g.ldb, g.tb ? g.ldb : 1);
         return ctx.check_cuda(cudaGetLastError(), "gemm_skinny launch");
