@@ -174,6 +174,11 @@ sage_status map_plan(const std::string &expr, const std::vector<MapOperand> &in,
         char m = direct ? 'D' : scalar ? 'S' : 'G';
         const bool aligned = reinterpret_cast<uintptr_t>(in[q].ptr) % 16 == 0;
         if (m == 'D' && !aligned) vec_ok = false;
+        if (in[q].slices > 1) {
+            if (!direct || in[q].dtype != SAGE_F32) return SAGE_ERR_INVALID;
+            m = 'Z';
+            if (!aligned || in[q].slice_stride % 4) vec_ok = false;
+        }
         if (m == 'G') {
             const long long inner = str[q][nd - 1];
             if (inner == 1) {
@@ -211,7 +216,10 @@ sage_status map_plan(const std::string &expr, const std::vector<MapOperand> &in,
     s << "extern \"C\" __global__ void __launch_bounds__(256) sage_map(";
     for (int q = 0; q < nin; ++q) s << "const " << ctype(in[q].dtype) << " *__restrict__ x" << q << "_buf, ";
     s << ctype(out_dtype) << " *__restrict__ y, const MapP p" << ((planes & 1) ? ", float *__restrict__ hi, const long long plane" : "")
-      << ((planes & 2) ? ", unsigned short *__restrict__ h2, const long long h2_plane, float *__restrict__ h2_scale, float *__restrict__ h2_marked" : "") << ") {\n";
+      << ((planes & 2) ? ", unsigned short *__restrict__ h2, const long long h2_plane, float *__restrict__ h2_scale, float *__restrict__ h2_marked" : "");
+    for (int q = 0; q < nin; ++q)
+        if (modes[q] == 'Z') s << ", const int slices" << q << ", const long long apart" << q;
+    s << ") {\n";
     // launched as a programmatic dependent: wait for the kernel before this one before touching memory
     s << "  asm volatile(\"griddepcontrol.launch_dependents;\" ::: \"memory\");\n";
     s << "  asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");\n";
@@ -223,7 +231,7 @@ sage_status map_plan(const std::string &expr, const std::vector<MapOperand> &in,
         if (m == 'G' || m == 'B' || m == 'X') need_coords = true;
     if (need_coords) {
         for (int q = 0; q < nin; ++q)
-            if (modes[q] != 'D' && modes[q] != 'S') s << "  long long i" << q << " = 0;\n";
+            if (modes[q] != 'D' && modes[q] != 'S' && modes[q] != 'Z') s << "  long long i" << q << " = 0;\n";
         s << "  { " << it << " rem = g, c;\n";
         for (int d = nd - 1; d >= 0; --d) {
             if (d == 0)
@@ -231,12 +239,16 @@ sage_status map_plan(const std::string &expr, const std::vector<MapOperand> &in,
             else
                 s << "    c = rem % (" << it << ")p.ext[" << d << "]; rem /= (" << it << ")p.ext[" << d << "];\n";
             for (int q = 0; q < nin; ++q)
-                if (modes[q] != 'D' && modes[q] != 'S') s << "    i" << q << " += (long long)c * p.str[" << q << "][" << d << "];\n";
+                if (modes[q] != 'D' && modes[q] != 'S' && modes[q] != 'Z') s << "    i" << q << " += (long long)c * p.str[" << q << "][" << d << "];\n";
         }
         s << "  }\n";
     }
     if (vec == 1) {
         for (int q = 0; q < nin; ++q) {
+            if (modes[q] == 'Z') {
+                s << "  float x" << q << " = x" << q << "_buf[g];\n#pragma unroll 8\n  for (int s = 1; s < slices" << q << "; ++s) x" << q << " += x" << q << "_buf[s * apart" << q << " + g];\n";
+                continue;
+            }
             s << "  const " << ctype(in[q].dtype) << " x" << q << " = x" << q << "_buf[";
             if (modes[q] == 'D') s << "g";
             else if (modes[q] == 'S') s << "0";
@@ -250,6 +262,13 @@ sage_status map_plan(const std::string &expr, const std::vector<MapOperand> &in,
     } else {
         for (int q = 0; q < nin; ++q) {
             const char *ct = ctype(in[q].dtype);
+            if (modes[q] == 'Z') {  // eight slices in flight, added in order
+                s << "  float4 v" << q << " = *reinterpret_cast<const float4 *>(x" << q << "_buf + g);\n  for (int s = 1; s < slices" << q << "; s += 8) {\n    float4 t[8];\n"
+                  << "#pragma unroll\n    for (int u = 0; u < 8; ++u) if (s + u < slices" << q << ") t[u] = *reinterpret_cast<const float4 *>(x" << q << "_buf + (s + u) * apart" << q << " + g);\n"
+                  << "#pragma unroll\n    for (int u = 0; u < 8; ++u) if (s + u < slices" << q << ") { v" << q << ".x += t[u].x; v" << q << ".y += t[u].y; v" << q << ".z += t[u].z; v" << q << ".w += t[u].w; }\n  }\n"
+                  << "  const float a" << q << "[4] = {v" << q << ".x, v" << q << ".y, v" << q << ".z, v" << q << ".w};\n";
+                continue;
+            }
             if (modes[q] == 'D' || modes[q] == 'G') {
                 s << "  const " << vtype(in[q].dtype) << " v" << q << " = *reinterpret_cast<const " << vtype(in[q].dtype)
                   << " *>(x" << q << "_buf + " << (modes[q] == 'D' ? std::string("g") : "i" + std::to_string(q)) << ");\n";
@@ -334,6 +353,15 @@ sage_status map_launch(Context &ctx, const std::string &expr, const std::vector<
         params.push_back(&o.h2_scale);
         params.push_back(&o.h2_marked);
     }
+    std::vector<int> slices(nin);
+    std::vector<long long> apart(nin);
+    for (int q = 0; q < nin; ++q)
+        if (in[q].slices > 1) {
+            slices[q] = in[q].slices;
+            apart[q] = in[q].slice_stride;
+            params.push_back(&slices[q]);
+            params.push_back(&apart[q]);
+        }
     const long long chunks = (plan.n + plan.vec - 1) / plan.vec;
     const uint32_t grid[3] = {(uint32_t)((chunks + 255) / 256), 1, 1};
     const uint32_t block[3] = {256, 1, 1};

@@ -14,6 +14,9 @@ struct MapOperand {
     int dtype;        // sage_dtype
     const void *ptr;  // device address with the element offset applied
     k::Dims view;     // extents (equal to the output's) + element strides (0 = broadcast)
+    // > 1: a contiguous f32 operand that is the sum, in order, of so many tensors `slice_stride` elements apart (a product's K slices)
+    int slices = 0;
+    long long slice_stride = 0;
 };
 
 // Per-operator memo of compiled kernels, the counterpart of CachedAccess

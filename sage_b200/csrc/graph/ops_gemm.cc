@@ -582,7 +582,7 @@ struct GemmOp : Operator {
         }
         // An epilogue cannot be applied before the K slices of a split product are summed.  Where the cost model
         // wants slices (few output tiles, long K: a convolution of a small feature map at a small batch), the
-        // plain product goes to scratch and the epilogue runs as a generated map kernel over the sum.
+        // slices' products go to scratch and the epilogue runs as a generated map kernel that adds them up as it reads them.
         if (!g.epilogue.empty() && !g.row_softmax && !g.conv.on && !folded && batch == 1 && g.c && epi_ext == out.shape.extents) {
             k::TcGemm raw = g;
             raw.epilogue.clear();
@@ -593,26 +593,28 @@ struct GemmOp : Operator {
             raw.sc1 = 0;
             raw.nbc0 = 1;
             if (k::gemm_tc_split_plan(ctx, raw) >= 2) {
-                Block *sum = ctx.allocator().alloc((size_t)(m * n) * sizeof(float));
-                if (sum) {
-                    raw.c = reinterpret_cast<float *>(sum->ptr);
-                    st = k::gemm_tc_run(ctx, raw);
-                    if (!st) {
-                        std::vector<MapOperand> operands(1 + (size_t)g.naux);
-                        operands[0].dtype = SAGE_F32;
-                        operands[0].ptr = raw.c;
-                        operands[0].view = Tensor().with_shape(Shape(out.shape.extents)).dims();
-                        for (int i = 0; i < g.naux; ++i) {
-                            operands[1 + i].dtype = x[2 + i].desc.dtype;
-                            operands[1 + i].ptr = x[2 + i].ptr();
-                            operands[1 + i].view = x[2 + i].dims();
-                        }
-                        k::PlaneOut planes;
-                        planes.hi = g.c_hi;
-                        planes.plane = g.c_plane;
-                        st = map_launch(ctx, epilogue, operands, SAGE_F32, y->ptr(), out.shape.rank(), out.shape.extents.data(), &epi_cache, planes);
+                raw.c = g.c;  // (its slices' products go to scratch)
+                Block *partial = nullptr;
+                int slices = 0;
+                st = k::gemm_tc_partials(ctx, raw, &partial, &slices);
+                if (st) return st;
+                if (partial) {
+                    std::vector<MapOperand> operands(1 + (size_t)g.naux);
+                    operands[0].dtype = SAGE_F32;
+                    operands[0].ptr = partial->ptr;
+                    operands[0].view = Tensor().with_shape(Shape(out.shape.extents)).dims();
+                    operands[0].slices = slices;
+                    operands[0].slice_stride = m * n;
+                    for (int i = 0; i < g.naux; ++i) {
+                        operands[1 + i].dtype = x[2 + i].desc.dtype;
+                        operands[1 + i].ptr = x[2 + i].ptr();
+                        operands[1 + i].view = x[2 + i].dims();
                     }
-                    ctx.allocator().free(sum);  // stream-ordered
+                    k::PlaneOut planes;
+                    planes.hi = g.c_hi;
+                    planes.plane = g.c_plane;
+                    st = map_launch(ctx, epilogue, operands, SAGE_F32, y->ptr(), out.shape.rank(), out.shape.extents.data(), &epi_cache, planes);
+                    ctx.allocator().free(partial);  // stream-ordered
                     return st;
                 }
             }

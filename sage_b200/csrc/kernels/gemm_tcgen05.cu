@@ -493,14 +493,15 @@ int gemm_tc_split_plan(Context &ctx, const TcGemm &g) {
     return pick_split_k(ctx, g, &bn);
 }
 
-sage_status gemm_tc_run(Context &ctx, const TcGemm &g0) {
-    if (!shape_within_limits(g0.m, g0.n, g0.k, g0.batch)) return ctx.fail(SAGE_ERR_UNSUPPORTED, "gemm_tc: shape not supported");
+sage_status gemm_tc_partials(Context &ctx, const TcGemm &g0, Block **partial, int *slices) {
     int bn = 0;
     const int S = pick_split_k(ctx, g0, &bn);
-    if (S < 2) return gemm_tc_launch(ctx, g0);
+    *partial = nullptr;
+    *slices = S;
+    if (S < 2) return SAGE_OK;
     const long long ks = g0.k / S, mn = g0.m * g0.n;
     Block *scratch = ctx.allocator().alloc((size_t)S * mn * sizeof(float));
-    if (!scratch) return gemm_tc_launch(ctx, g0);  // no room for the partial products: one pass over K
+    if (!scratch) return SAGE_OK;
     TcGemm g = g0;
     g.batch = S;
     g.k = ks;
@@ -526,16 +527,26 @@ sage_status gemm_tc_run(Context &ctx, const TcGemm &g0) {
     g.sc1 = 0;
     g.nbc0 = S;
     sage_status st = gemm_tc_launch(ctx, g);
-    if (!st) {
-        Dims outer, inner;
-        outer.ndim = 1;
-        outer.ext[0] = mn;
-        outer.str[0] = 1;
-        inner.ndim = 1;
-        inner.ext[0] = S;
-        inner.str[0] = mn;
-        st = reduce(ctx, SAGE_F32, 0 /* sum */, g.c, outer, inner, g0.c);
-    }
+    if (st) ctx.allocator().free(scratch);  // stream-ordered
+    else *partial = scratch;
+    return st;
+}
+
+sage_status gemm_tc_run(Context &ctx, const TcGemm &g0) {
+    if (!shape_within_limits(g0.m, g0.n, g0.k, g0.batch)) return ctx.fail(SAGE_ERR_UNSUPPORTED, "gemm_tc: shape not supported");
+    Block *scratch = nullptr;
+    int S = 0;
+    sage_status st = gemm_tc_partials(ctx, g0, &scratch, &S);
+    if (st) return st;
+    if (!scratch) return gemm_tc_launch(ctx, g0);  // no slices, or no room for the partial products: one pass over K
+    Dims outer, inner;
+    outer.ndim = 1;
+    outer.ext[0] = g0.m * g0.n;
+    outer.str[0] = 1;
+    inner.ndim = 1;
+    inner.ext[0] = S;
+    inner.str[0] = g0.m * g0.n;
+    st = reduce(ctx, SAGE_F32, 0 /* sum */, reinterpret_cast<float *>(scratch->ptr), outer, inner, g0.c);
     ctx.allocator().free(scratch);  // stream-ordered
     return st;
 }

@@ -173,6 +173,9 @@ sage_status gemm_tc_run(Context &ctx, const TcGemm &g);
 // How many K slices gemm_tc_run would cut this product into (0 = none).  Only products without an epilogue are
 // cut; a caller with an epilogue may ask for the plain product and apply the epilogue to the sum itself.
 int gemm_tc_split_plan(Context &ctx, const TcGemm &g);
+// The K slices' partial products alone, m * n floats apart, in memory of `*partial` (whoever asked frees it), and how many there are.
+// Without room for them: SAGE_OK and no memory.
+sage_status gemm_tc_partials(Context &ctx, const TcGemm &g, Block **partial, int *slices);
 // gemm_group.cu: may this product run beside others in one launch; and that launch (several, where there are very many).
 bool gemm_tc_groupable(const TcGemm &g);
 sage_status gemm_tc_group_run(Context &ctx, const std::vector<TcGemm> &all);
