@@ -19,6 +19,8 @@ sage_status storage_planes_attach(Context &ctx, Storage &st);  // ops_gemm.cc
 
 struct Im2colOp : Operator {
     Pair ker, stride, pad, dil, col;
+    std::string pre;  // C expression over x0 that every value of the image goes through first (a map before the column matrix)
+    MapCache maps;
     const char *name() const override { return "im2col"; }
     std::vector<Var> grad(const std::vector<Var> &x, const Var &, const Var &gy) override {
         return {col2im(gy, Pair{x[0].extent(2), x[0].extent(1)}, ker, stride, pad, dil)};
@@ -29,13 +31,26 @@ struct Im2colOp : Operator {
         sage_status st = Tensor::uninit(ctx, out, y);
         if (st) return st;
         const Array &e = x[0].desc.shape.extents;
+        Tensor image = x[0];
+        const bool spliced = !pre.empty() && k::cols_mappable(image.ptr(), y->ptr(), e[1], e[2], e[3], col.h, col.w, window(ker, stride, pad, dil));
+        if (!pre.empty() && !spliced) {  // an image off the 16-byte grid: the map by itself
+            st = Tensor::uninit(ctx, x[0].desc.pristine(), &image);
+            if (st) return st;
+            st = map_launch(ctx, pre, {MapOperand{SAGE_F32, x[0].ptr(), x[0].dims()}}, SAGE_F32, image.ptr(), (int)e.size(), e.data(), &maps);
+            if (st) return st;
+        }
+        if (!emit && spliced)
+            return k::im2col_mapped(ctx, pre, (const float *)x[0].ptr(), e[0], e[1], e[2], e[3], col.h, col.w, window(ker, stride, pad, dil), (float *)y->ptr(), nullptr, 0, 0);
         if (!emit)
-            return k::im2col(ctx, (const float *)x[0].ptr(), (float *)y->ptr(), e[0], e[1], e[2], e[3], col.h, col.w, window(ker, stride, pad, dil));
+            return k::im2col(ctx, (const float *)image.ptr(), (float *)y->ptr(), e[0], e[1], e[2], e[3], col.h, col.w, window(ker, stride, pad, dil));
         st = storage_planes_attach(ctx, *y->data);
         if (st) return st;
         const SplitCache &c = *y->data->split;
         y->data->planes_only = only;
-        return k::im2col_planes(ctx, (const float *)x[0].ptr(), e[0], e[1], e[2], e[3], col.h, col.w, window(ker, stride, pad, dil), only ? nullptr : (float *)y->ptr(), c.planes.planes, c.plane,
+        if (spliced)
+            return k::im2col_mapped(ctx, pre, (const float *)x[0].ptr(), e[0], e[1], e[2], e[3], col.h, col.w, window(ker, stride, pad, dil), only ? nullptr : (float *)y->ptr(),
+                                    c.planes.planes, c.plane, (int)(ker.h * ker.w * e[3]));
+        return k::im2col_planes(ctx, (const float *)image.ptr(), e[0], e[1], e[2], e[3], col.h, col.w, window(ker, stride, pad, dil), only ? nullptr : (float *)y->ptr(), c.planes.planes, c.plane,
                                 (int)(ker.h * ker.w * e[3]));
     }
     // the planes lie like the result, whole 16-byte pieces at a time
@@ -50,7 +65,7 @@ bool im2col_op_emits_planes(const Operator &op) {
 
 bool im2col_params(const Operator &op, k::Window *w, long long dims[6]) {
     const Im2colOp *o = dynamic_cast<const Im2colOp *>(&op);
-    if (!o || o->in[0].dtype != SAGE_F32 || !o->in[0].shape.has_default_strides()) return false;
+    if (!o || !o->pre.empty() || o->in[0].dtype != SAGE_F32 || !o->in[0].shape.has_default_strides()) return false;
     *w = window(o->ker, o->stride, o->pad, o->dil);
     const Array &e = o->in[0].shape.extents;
     dims[0] = e[0];
@@ -64,18 +79,92 @@ bool im2col_params(const Operator &op, k::Window *w, long long dims[6]) {
 
 struct Col2imOp : Operator {
     Pair img, ker, stride, pad, dil;
+    std::string post;  // C expression over x0, a value of the image, and x1 ... (inputs 1 ..., laid out like it): the map that follows
+    MapCache maps;
     const char *name() const override { return "col2im"; }
     std::vector<Var> grad(const std::vector<Var> &, const Var &, const Var &gy) override {
         return {im2col(gy, ker, stride, pad, dil)};
     }
     sage_status compute(const std::vector<Tensor> &x, Context &ctx, Tensor *y) override {
+        const bool emit = ctx.hint_emit_planes && !post.empty(), only = emit && ctx.hint_planes_only;
+        ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = false;
         sage_status st = Tensor::uninit(ctx, out, y);
         if (st) return st;
         const Array &e = x[0].desc.shape.extents;  // [N, col_h, col_w, KH, KW, C]
+        if (!post.empty()) {
+            float *hi = nullptr;
+            long long plane = 0;
+            if (emit) {
+                st = storage_planes_attach(ctx, *y->data);
+                if (st) return st;
+                hi = y->data->split->planes.planes + y->desc.shape.offset;
+                plane = y->data->split->plane;
+                y->data->planes_only = only;
+            }
+            const float *aux[3] = {nullptr, nullptr, nullptr};
+            bool aligned = k::cols_mappable(x[0].ptr(), y->ptr(), img.h, img.w, e[5], e[1], e[2], window(ker, stride, pad, dil));
+            for (size_t i = 1; i < x.size(); ++i) {
+                aux[i - 1] = (const float *)x[i].ptr();
+                aligned = aligned && k::cols_mappable(aux[i - 1], nullptr, img.h, img.w, e[5], e[1], e[2], window(ker, stride, pad, dil));
+            }
+            if (!aligned) {  // an operand off the 16-byte grid: the map by itself
+                Tensor sum;
+                st = Tensor::uninit(ctx, out, &sum);
+                if (!st) st = k::col2im(ctx, (const float *)x[0].ptr(), (float *)sum.ptr(), e[0], img.h, img.w, e[5], e[1], e[2], window(ker, stride, pad, dil));
+                if (st) return st;
+                std::vector<MapOperand> operands = {MapOperand{SAGE_F32, sum.ptr(), sum.dims()}};
+                for (size_t i = 1; i < x.size(); ++i) operands.push_back(MapOperand{SAGE_F32, x[i].ptr(), x[i].dims()});
+                y->data->planes_only = false;
+                k::PlaneOut forms;
+                forms.hi = hi;
+                forms.plane = plane;
+                return map_launch(ctx, post, operands, SAGE_F32, y->ptr(), out.shape.rank(), out.shape.extents.data(), &maps, forms);
+            }
+            return k::col2im_mapped(ctx, post, (int)x.size() - 1, aux, (const float *)x[0].ptr(), only ? nullptr : (float *)y->ptr(), hi, plane, e[0], img.h, img.w, e[5], e[1], e[2],
+                                    window(ker, stride, pad, dil));
+        }
         return k::col2im(ctx, (const float *)x[0].ptr(), (float *)y->ptr(), e[0], img.h, img.w, e[5], e[1], e[2],
                          window(ker, stride, pad, dil));
     }
 };
+
+// A map of one operand before a column matrix, as part of it: null where the operand is not laid out like the image or the kernel does not
+// take four channels at a time.  (Storages start on 512 bytes: the offset says where a tensor lies.)
+std::shared_ptr<Operator> im2col_with_map(const Operator &op, const Operator &map, const std::string &expr) {
+    const Im2colOp *o = dynamic_cast<const Im2colOp *>(&op);
+    if (!o || !o->pre.empty() || map.in.size() != 1 || k::long_expression(expr)) return nullptr;  // (it is worked out for every tap)
+    const TensorDesc &src = map.in[0];
+    const Array &e = o->in[0].shape.extents;
+    if (src.dtype != SAGE_F32 || src.shape.extents != e || !src.shape.has_default_strides() || src.shape.offset % 4) return nullptr;
+    if (!k::cols_mappable(nullptr, nullptr, e[1], e[2], e[3], o->col.h, o->col.w, window(o->ker, o->stride, o->pad, o->dil)) || e[0] * o->col.h * o->col.w > (1LL << 29)) return nullptr;
+    auto c = std::make_shared<Im2colOp>(*o);
+    c->pre = expr;
+    c->in = {src};
+    return c;
+}
+// The map `expr` over (the gathered image, aux ...), as part of the gather.
+std::shared_ptr<Operator> col2im_with_map(const Operator &op, const std::string &expr, const std::vector<TensorDesc> &aux, const TensorDesc &out) {
+    const Col2imOp *o = dynamic_cast<const Col2imOp *>(&op);
+    if (!o || !o->post.empty() || aux.size() > 3 || out.dtype != SAGE_F32 || out.shape.size() != o->out.shape.size()) return nullptr;
+    const Array &e = o->in[0].shape.extents;
+    if (!o->in[0].shape.has_default_strides() || o->in[0].shape.offset % 4 || !k::cols_mappable(nullptr, nullptr, o->img.h, o->img.w, e[5], e[1], e[2], window(o->ker, o->stride, o->pad, o->dil))) return nullptr;
+    for (const TensorDesc &a : aux)
+        if (a.dtype != SAGE_F32 || a.shape.extents != out.shape.extents || !a.shape.has_default_strides() || a.shape.offset % 4) return nullptr;
+    auto c = std::make_shared<Col2imOp>(*o);
+    c->post = expr;
+    c->in.resize(1);
+    for (const TensorDesc &a : aux) c->in.push_back(a);
+    c->out = out.pristine();
+    return c;
+}
+bool col2im_op_emits_planes(const Operator &op) {
+    const Col2imOp *o = dynamic_cast<const Col2imOp *>(&op);
+    return o && !o->post.empty();
+}
+bool is_col2im_op(const Operator &op) {
+    const Col2imOp *o = dynamic_cast<const Col2imOp *>(&op);
+    return o && o->post.empty();
+}
 
 Var ops::im2col(const Var &x0, Pair ker, Pair stride, Pair pad, Pair dil) {
     Var x = x0.organize();

@@ -76,6 +76,10 @@ bool gemm_emits_h2(const Operator &op);
 bool row_op_emits_h2(const Operator &op);
 bool pool_op_emits_h2(const Operator &op);  // ops_conv.cc
 bool im2col_op_emits_planes(const Operator &op);
+bool col2im_op_emits_planes(const Operator &op);
+bool is_col2im_op(const Operator &op);
+std::shared_ptr<Operator> im2col_with_map(const Operator &op, const Operator &map, const std::string &expr);
+std::shared_ptr<Operator> col2im_with_map(const Operator &op, const std::string &expr, const std::vector<TensorDesc> &aux, const TensorDesc &out);
 bool map_op_emits_h2(const Operator &op);
 std::string describe_gemm(const Operator &op);  // "{epilogue}" / "[store]" of a lowered GEMM, else empty
 
@@ -459,6 +463,27 @@ static void lower(Node &n, bool tc, bool softmax_in_gemm, bool attention) {
         return;
     }
     if (n.op->out.dtype != SAGE_F32) return;
+    for (size_t j = 0; j < n.args.size(); ++j) {  // a map over the gradient of a convolution's image
+        Node *p = &n.args[j];
+        while (!p->is_data && is_reshape_op(*p->op)) p = &p->args[0];
+        if (p->is_data || !is_col2im_op(*p->op)) continue;
+        std::vector<int> remap(n.args.size());
+        std::vector<TensorDesc> aux;
+        int next = 1;
+        for (size_t i = 0; i < n.args.size(); ++i) {
+            remap[i] = i == j ? 0 : next++;
+            if (i != j) aux.push_back(n.op->in[i]);
+        }
+        std::shared_ptr<Operator> f = col2im_with_map(*p->op, map_expr_text_remap(*expr, remap), aux, n.op->out);
+        if (!f) continue;
+        std::vector<Node> args;
+        args.push_back(std::move(p->args[0]));
+        for (size_t i = 0; i < n.args.size(); ++i)
+            if (i != j) args.push_back(std::move(n.args[i]));
+        n.op = f;
+        n.args = std::move(args);
+        return;
+    }
     for (size_t j = 0; j < n.args.size(); ++j) {  // a map over a product
         Node *p = &n.args[j];
         while (!p->is_data && is_reshape_op(*p->op)) p = &p->args[0];
@@ -497,7 +522,7 @@ static Node *skip_views(Node *p, long long *offset) {  // *offset: where in the 
 }
 bool map_op_emits_planes(const Operator &op);
 static bool can_emit_planes(const Operator &op, bool tc) {
-    return gemm_runs_on_tc(op, tc) || row_op_emits_planes(op) || is_grouped_gemm_op(op) || (tc && (map_op_emits_planes(op) || im2col_op_emits_planes(op)));
+    return gemm_runs_on_tc(op, tc) || row_op_emits_planes(op) || is_grouped_gemm_op(op) || (tc && (map_op_emits_planes(op) || im2col_op_emits_planes(op) || col2im_op_emits_planes(op)));
 }
 bool gemm_reads_wide(const Operator &op);
 bool gemm_emits_wide(const Operator &op);
@@ -884,6 +909,16 @@ static std::unique_ptr<Program> compile(const std::vector<Var> &x, std::vector<V
         if (pattern) {
             lower(r.root, tc, softmax_in_gemm, attention && tc && attention_enabled());
             if (tc) group_gemms(r.root);
+            // A column matrix that is kept (a training step's, for both of its products) takes the map before it along.
+            Node *top = &r.root;
+            while (!top->is_data && !top->shared && is_view_op(*top->op) && top->args.size() == 1) top = &top->args[0];
+            if (!top->is_data && !top->shared && im2col_op_emits_planes(*top->op) && top->args.size() == 1 && !top->args[0].is_data && !top->args[0].shared)
+                if (const MapExpr *e = map_expr_of(*top->args[0].op))
+                    if (std::shared_ptr<Operator> f = im2col_with_map(*top->op, *top->args[0].op, map_expr_text(*e))) {
+                        std::vector<Node> args = std::move(top->args[0].args);
+                        top->op = f;
+                        top->args = std::move(args);
+                    }
         }
         p->routines.emplace(node.key(), std::move(r));
     }

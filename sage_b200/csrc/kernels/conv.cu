@@ -18,6 +18,7 @@
 #include "launch.h"
 
 namespace sage {
+const char *map_prelude_text();  // codegen/map_emit.cc
 namespace k {
 
 struct ConvP {
@@ -38,6 +39,11 @@ struct ColOut {
 };
 
 __device__ __forceinline__ void split_pair(float x, float *hi, float *lo) { sage_tc::split_tf32_value(x, hi, lo); }
+#define SAGE_COLS_SPLIT split_pair
+#define SAGE_COLS_PRE(x0) (x0)
+#define SAGE_COLS_POST(x0, x1, x2, x3) (x0)
+#include "conv_cols_device.inc"
+#include "conv_cols_device_src.h"  // generated by the Makefile: the text of conv_cols_device.inc as kConvColsDeviceSrc
 
 // `share` warps to a pixel where there are few of them (128 pixels of 9 x 512 values, one warp each: 16 blocks, 8 us).
 __global__ void __launch_bounds__(256) im2col_kernel(const float *__restrict__ img, ColOut o, ConvP p, long long pixels, int share) {
@@ -53,26 +59,7 @@ __global__ void __launch_bounds__(256) im2col_kernel(const float *__restrict__ i
     const int C = (int)p.chan, K = p.w.ker_h * p.w.ker_w * C;
     const float *im = img + n * p.img_h * p.img_w * C;
     if ((C & 3) == 0) {
-        const int c4n = C >> 2, chunks = K >> 2;
-        for (int ch = lane; ch < chunks; ch += step) {
-            const int tap = ch / c4n, c = (ch - tap * c4n) << 2;
-            const int ky = tap / p.w.ker_w, kx = tap - ky * p.w.ker_w;
-            const int iy = iy0 + ky * p.w.dil_h, ix = ix0 + kx * p.w.dil_w;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (ix >= 0 && ix < p.img_w && iy >= 0 && iy < p.img_h)
-                v = __ldg(reinterpret_cast<const float4 *>(im + ((long long)iy * p.img_w + ix) * C + c));
-            if (o.col) *reinterpret_cast<float4 *>(o.col + pix * K + (ch << 2)) = v;
-            if (o.hi) {
-                float4 h, l;
-                split_pair(v.x, &h.x, &l.x);
-                split_pair(v.y, &h.y, &l.y);
-                split_pair(v.z, &h.z, &l.z);
-                split_pair(v.w, &h.w, &l.w);
-                float *d = o.hi + pix * o.pitch + (ch << 2);
-                *reinterpret_cast<float4 *>(d) = h;
-                *reinterpret_cast<float4 *>(d + o.plane) = l;
-            }
-        }
+        im2col_quads_of_pixel(im, o.col, o.hi, o.plane, o.pitch, p, pix, iy0, ix0, lane, step);
     } else {
         const int width = o.hi ? o.pitch : K;
         for (int kk = lane; kk < width; kk += step) {
@@ -182,51 +169,10 @@ __global__ void __launch_bounds__(256) col2im_kernel(const float *__restrict__ c
     }
 }
 
-// The same gather with 32-bit index arithmetic and four channels per thread (C % 4 == 0): one 64-bit division per
-// thread instead of a dozen per element, 16-byte loads and stores.  Same tap test, same order of accumulation.
+// The same gather with 32-bit index arithmetic and four channels per thread (C % 4 == 0).
 __global__ void __launch_bounds__(256) col2im_quads_kernel(const float *__restrict__ col, float *__restrict__ img, ConvP p, long long total) {
     grid_dependency_sync();
-    const int cn = (int)(p.chan >> 2), W = (int)p.img_w, H = (int)p.img_h, CW = (int)p.col_w, CH = (int)p.col_h;
-    const int sw = p.w.stride_w, sh = p.w.stride_h, dw = p.w.dil_w, dh = p.w.dil_h, kw = p.w.ker_w, kh = p.w.ker_h;
-    const int ker_ew = (kw - 1) * dw + 1, ker_eh = (kh - 1) * dh + 1;
-    const unsigned per_img = (unsigned)(H * W);
-    for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < total; g += (long long)gridDim.x * blockDim.x) {
-        const long long pix = g / cn;
-        const int c = (int)(g - pix * cn) << 2;
-        const long long n = pix / per_img;
-        const unsigned r = (unsigned)(pix - n * per_img);
-        const int img_y = (int)(r / (unsigned)W), img_x = (int)(r - (unsigned)img_y * (unsigned)W);
-        const int xp = img_x + p.w.pad_w, yp = img_y + p.w.pad_h;
-        const int xs = xp < ker_ew ? 0 : (xp - ker_ew) / sw + 1, ys = yp < ker_eh ? 0 : (yp - ker_eh) / sh + 1;
-        const int xe = min(xp / sw + 1, CW), ye = min(yp / sh + 1, CH);
-        const float *cb = col + n * (long long)CH * CW * kh * kw * p.chan + c;
-        float4 val = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int cx = xs, cy = ys; cx < xe && ys < ye;) {  // nine taps asked for at a time, taken in the window's order
-            float4 v[9];
-#pragma unroll
-            for (int u = 0; u < 9; ++u) {
-                v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                int kx = xp - cx * sw, ky = yp - cy * sh;
-                if (cx < xe && (dh == 1 || kx % dh == 0) && (dw == 1 || ky % dw == 0)) {  // the reference's test (conv.rs:462-464), dilations crossed as there
-                    kx /= dh;
-                    ky /= dw;
-                    v[u] = __ldg(reinterpret_cast<const float4 *>(cb + ((((long long)cy * CW + cx) * kh + ky) * kw + kx) * p.chan));
-                }
-                if (++cy == ye) {
-                    cy = ys;
-                    ++cx;
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 9; ++u) {
-                val.x += v[u].x;
-                val.y += v[u].y;
-                val.z += v[u].z;
-                val.w += v[u].w;
-            }
-        }
-        *reinterpret_cast<float4 *>(img + (pix * p.chan + c)) = val;
-    }
+    col2im_quads(col, img, nullptr, 0, p, total, nullptr, nullptr, nullptr);
 }
 
 // One thread per output pixel and group of 4 channels when C % 4 == 0 (16-byte loads, one 64-bit division per thread), else
@@ -619,6 +565,73 @@ sage_status col2im(Context &ctx, const float *col, float *img, long long n, long
     }
     launch_dependent(ctx.pdl, ctx.stream(), col2im_kernel, dim3(grid_for(ctx, total)), dim3(256), 0, col, img, p, total);
     return ctx.check_cuda(cudaGetLastError(), "col2im launch");
+}
+
+// ---- with a map spliced in
+bool cols_mappable(const void *a, const void *b, long long img_h, long long img_w, long long chan, long long col_h, long long col_w, const Window &w) {
+    return chan % 4 == 0 && reinterpret_cast<uintptr_t>(a) % 16 == 0 && reinterpret_cast<uintptr_t>(b) % 16 == 0 && img_h * img_w <= 0x7fffffffLL && col_h * col_w <= 0x7fffffffLL &&
+           w.dil_w >= 1 && w.dil_h >= 1 && (long long)w.ker_h * w.ker_w * chan <= 0x7fffffffLL;
+}
+static sage_status cols_module(Context &ctx, const char *what, const std::string &expr, int naux, Module **mod) {
+    const std::string key = std::string(what) + " " + std::to_string(naux) + "\n" + expr;
+    *mod = ctx.module_find(key);
+    if (*mod) return SAGE_OK;
+    const bool pre = what[0] == 'i';
+    std::string src = map_prelude_text();
+    src += "struct Window { int ker_w, ker_h, stride_w, stride_h, pad_w, pad_h, dil_w, dil_h; };\n"
+           "struct ConvP { long long n, img_h, img_w, chan, col_h, col_w; Window w; };\n"
+           "#define SAGE_COLS_SPLIT sg_split_tf32\n#define SAGE_COLS_NAUX " + std::to_string(naux) + "\n";
+    src += "#define SAGE_COLS_PRE(x0) (" + (pre ? expr : std::string("x0")) + ")\n#define SAGE_COLS_POST(x0, x1, x2, x3) (" + (pre ? std::string("x0") : expr) + ")\n";
+    src += kConvColsDeviceSrc;
+    const char *wait = "    asm volatile(\"griddepcontrol.launch_dependents;\" ::: \"memory\");\n    asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");\n";
+    if (pre)
+        src += std::string("extern \"C\" __global__ void __launch_bounds__(256) sage_im2col(const float *img, float *col, float *hi, const long long plane, const int pitch, const ConvP p, const long long pixels, const int share) {\n") + wait +
+               "    const long long warp = (long long)blockIdx.x * 8 + (threadIdx.x >> 5), pix = warp / share;\n"
+               "    if (pix >= pixels) return;\n"
+               "    const long long per_img = p.col_h * p.col_w, n = pix / per_img;\n"
+               "    const int r = (int)(pix - n * per_img), oy = r / (int)p.col_w, ox = r % (int)p.col_w;\n"
+               "    im2col_quads_of_pixel(img + n * p.img_h * p.img_w * p.chan, col, hi, plane, pitch, p, pix, oy * p.w.stride_h - p.w.pad_h, ox * p.w.stride_w - p.w.pad_w,\n"
+               "                          (int)(threadIdx.x & 31) + 32 * (int)(warp - pix * share), 32 * share);\n}\n";
+    else
+        src += std::string("extern \"C\" __global__ void __launch_bounds__(256) sage_col2im(const float *col, float *img, float *hi, const long long plane, const ConvP p, const long long total, const float *x1, const float *x2, const float *x3) {\n") + wait +
+               "    col2im_quads(col, img, hi, plane, p, total, x1, x2, x3);\n}\n";
+    sage_status st = ctx.module_get(src, mod);
+    if (!st) ctx.module_remember(key, *mod);
+    return st;
+}
+
+sage_status im2col_mapped(Context &ctx, const std::string &expr, const float *img, long long n, long long img_h, long long img_w, long long chan, long long col_h, long long col_w, const Window &w,
+                          float *col, float *hi, long long plane, int pitch) {
+    ConvP p{n, img_h, img_w, chan, col_h, col_w, w};
+    const long long pixels = n * col_h * col_w;
+    if (!cols_mappable(img, col, img_h, img_w, chan, col_h, col_w, w) || reinterpret_cast<uintptr_t>(hi) % 16 || plane % 4 || pitch % 4 || (pixels * 16 + 7) / 8 > 0x7fffffffLL)
+        return ctx.fail(SAGE_ERR_UNSUPPORTED, "im2col: not addressable four channels at a time");
+    Module *mod = nullptr;
+    sage_status st = cols_module(ctx, "im2col", expr, 0, &mod);
+    if (st || pixels == 0) return st;
+    int share = 1;
+    const long long length = w.ker_h * w.ker_w * chan / 4;  // loads of a pixel
+    while (share < 16 && pixels * share < 32LL * ctx.sm_count && length >= 128LL * share) share *= 2;
+    long long pix = pixels;
+    void *params[8] = {&img, &col, &hi, &plane, &pitch, &p, &pix, &share};
+    const uint32_t grid[3] = {(uint32_t)((pixels * share + 7) / 8), 1, 1}, block[3] = {256, 1, 1};
+    return ctx.launch(mod, "sage_im2col", grid, block, 0, params, ctx.verbose_names ? (col ? "im2col{map}" : "im2col{map}=planes") : "im2col", true);
+}
+
+sage_status col2im_mapped(Context &ctx, const std::string &expr, int naux, const float *const aux[3], const float *col, float *img, float *hi, long long plane, long long n, long long img_h,
+                          long long img_w, long long chan, long long col_h, long long col_w, const Window &w) {
+    ConvP p{n, img_h, img_w, chan, col_h, col_w, w};
+    long long total = n * img_h * img_w * chan / 4;
+    if (!cols_mappable(col, img, img_h, img_w, chan, col_h, col_w, w) || reinterpret_cast<uintptr_t>(hi) % 16 || plane % 4) return ctx.fail(SAGE_ERR_UNSUPPORTED, "col2im: not addressable four channels at a time");
+    for (int i = 0; i < naux; ++i)
+        if (reinterpret_cast<uintptr_t>(aux[i]) % 16) return ctx.fail(SAGE_ERR_UNSUPPORTED, "col2im: not addressable four channels at a time");
+    Module *mod = nullptr;
+    sage_status st = cols_module(ctx, "col2im", expr, naux, &mod);
+    if (st || total == 0) return st;
+    const float *x[3] = {aux[0], aux[1], aux[2]};
+    void *params[9] = {&col, &img, &hi, &plane, &p, &total, &x[0], &x[1], &x[2]};
+    const uint32_t grid[3] = {grid_for(ctx, total), 1, 1}, block[3] = {256, 1, 1};
+    return ctx.launch(mod, "sage_col2im", grid, block, 0, params, ctx.verbose_names ? "col2im{map}" : "col2im", true);
 }
 
 bool pool2d_writes_pieces(const float *img, long long chan, long long out_h, long long out_w) {

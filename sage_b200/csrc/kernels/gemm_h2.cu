@@ -944,7 +944,7 @@ static SlicePlan plan_slices(const Context &ctx, const H2Gemm &g) {
 }
 
 // Does the expression call a function of more than a few instructions?
-static bool long_expression(const std::string &e) {
+bool long_expression(const std::string &e) {
     static const char *const kShort[] = {"lit", "abs", "square", "sign", "min", "max", "ceil", "floor", "round", "recip"};
     for (size_t at = e.find("sg_"); at != std::string::npos; at = e.find("sg_", at + 3)) {
         bool is_short = false;

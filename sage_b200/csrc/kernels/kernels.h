@@ -95,6 +95,14 @@ sage_status pack_small_c_filter(Context &ctx, const float *filt, int kh, int kw,
 sage_status pack_first_image(Context &ctx, const float *img, long long n, long long h, long long w, long long c, long long hp, long long wp, int pad_h, int pad_w,
                              unsigned short *hi, long long plane, float *scale, unsigned *parts);
 sage_status pack_first_filter(Context &ctx, const float *filt, int kh, int kw, int c, int oc, unsigned short *out, float *scale);
+// The same with a map before the column matrix (`expr` over x0, an image's value) or behind the image's gradient (over x0, the gathered
+// sum, and x1 ... x3, dense like the image), spliced in: C % 4 == 0 and 16-byte alignment throughout.  Results that are null are not stored.
+bool long_expression(const std::string &e);  // calls a function of more than a few instructions (gemm_h2.cu)
+bool cols_mappable(const void *a, const void *b, long long img_h, long long img_w, long long chan, long long col_h, long long col_w, const Window &w);
+sage_status im2col_mapped(Context &ctx, const std::string &expr, const float *img, long long n, long long img_h, long long img_w, long long chan, long long col_h, long long col_w, const Window &w,
+                          float *col, float *hi, long long plane, int pitch);
+sage_status col2im_mapped(Context &ctx, const std::string &expr, int naux, const float *const aux[3], const float *col, float *img, float *hi, long long plane, long long n, long long img_h,
+                          long long img_w, long long chan, long long col_h, long long col_w, const Window &w);
 bool pool2d_writes_pieces(const float *img, long long chan, long long out_h, long long out_w);
 sage_status pool2d(Context &ctx, bool is_max, const float *img, float *out, long long n, long long img_h,
                    long long img_w, long long chan, long long out_h, long long out_w, const Window &w, const PlaneOut &forms);
