@@ -201,7 +201,7 @@ sage_status map_plan(const std::string &expr, const std::vector<MapOperand> &in,
     const char *it = wide ? "unsigned long long" : "unsigned int";
     if (vec != 4 || n % 64 != 0) planes &= ~2;
     plan->planes = planes;
-    plan->signature = modes + ":" + std::to_string(vec) + ":" + std::to_string(nd) + (wide ? "w" : "n") + ((planes & 1) ? "P" : "") + ((planes & 2) ? "H" : "");
+    plan->signature = modes + ":" + std::to_string(vec) + ":" + std::to_string(nd) + (wide ? "w" : "n") + ((planes & 1) ? "P" : "") + ((planes & 2) ? "H" : "") + ((planes & 4) ? "O" : "");
     if (!emit_source) return SAGE_OK;  // the caller already holds the kernel for this signature
 
     // ---- emit
@@ -257,7 +257,8 @@ sage_status map_plan(const std::string &expr, const std::vector<MapOperand> &in,
         }
         s << "  const " << ctype(out_dtype) << " r = sage_expr(";
         for (int q = 0; q < nin; ++q) s << (q ? ", " : "") << "x" << q;
-        s << ");\n  y[g] = r;\n";
+        s << ");\n";
+        if (!(planes & 4)) s << "  y[g] = r;\n";
         if (planes & 1) s << "  { float h, l; sg_split_tf32(r, &h, &l); hi[g] = h; hi[plane + g] = l; }\n";
     } else {
         for (int q = 0; q < nin; ++q) {
@@ -286,7 +287,7 @@ sage_status map_plan(const std::string &expr, const std::vector<MapOperand> &in,
             for (int q = 0; q < nin; ++q) s << (q ? ", " : "") << "a" << q << "[" << e << "]";
             s << ");\n";
         }
-        s << "  *reinterpret_cast<" << vtype(out_dtype) << " *>(y + g) = r;\n";
+        if (!(planes & 4)) s << "  *reinterpret_cast<" << vtype(out_dtype) << " *>(y + g) = r;\n";
         if (planes & 2) s << "  sg_h2_store(r, g, h2, h2_plane, h2_scale, h2_marked);\n";
         if (planes & 1)
             s << "  { float4 h, l; sg_split_tf32(r.x, &h.x, &l.x); sg_split_tf32(r.y, &h.y, &l.y); sg_split_tf32(r.z, &h.z, &l.z); "
@@ -304,7 +305,7 @@ struct MapPHost {
 
 sage_status map_launch(Context &ctx, const std::string &expr, const std::vector<MapOperand> &in, int out_dtype,
                        void *y, int out_ndim, const long long *out_ext, MapCache *cache, const k::PlaneOut &out) {
-    const int planes = out_dtype == SAGE_F32 ? (out.hi ? 1 : 0) | (out.h2 ? 2 : 0) : 0;
+    const int planes = out_dtype == SAGE_F32 ? (out.hi ? 1 : 0) | (out.h2 ? 2 : 0) | (out.only && out.hi && !out.h2 ? 4 : 0) : 0;
     MapPlan plan;
     sage_status st = map_plan(expr, in, out_dtype, y, out_ndim, out_ext, &plan, false, planes);
     if (st) return st;

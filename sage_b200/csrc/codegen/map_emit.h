@@ -41,7 +41,7 @@ struct MapPlan {
 // `expr` is a C expression over x0..x{n-1}; helper functions come from the prelude
 // (sg_exp, sg_max, ...).  The output is contiguous with `out_ext`.
 // `planes`: bit 0, the kernel also writes the tf32 hi / lo split of every (f32) result, laid out like y; bit 1, its
-// half-precision pieces (in the vector form only, and for whole groups of 64: else the plan drops the bit).
+// half-precision pieces (in the vector form only, and for whole groups of 64: else the plan drops the bit); bit 2, and not y.
 sage_status map_plan(const std::string &expr, const std::vector<MapOperand> &in, int out_dtype, const void *y,
                      int out_ndim, const long long *out_ext, MapPlan *plan, bool emit_source = true, int planes = 0);
 

@@ -558,10 +558,6 @@ struct GemmOp : Operator {
             if (st) return st;
             g.c_hi = y->data->split->planes.planes + y->desc.shape.offset;
             g.c_plane = y->data->split->plane;
-            if (only) {
-                g.c = nullptr;
-                y->data->planes_only = true;
-            }
         }
         g.naux = naux();
         g.epilogue = epilogue;
@@ -579,6 +575,16 @@ struct GemmOp : Operator {
             for (std::shared_ptr<void> held : {std::shared_ptr<void>(x[0].data), std::shared_ptr<void>(x[1].data), std::shared_ptr<void>(hold_a), std::shared_ptr<void>(hold_b), std::shared_ptr<void>(y->data)})
                 batch_to->held.push_back(held);
             return SAGE_OK;
+        }
+        // (A product that is cut into K slices stores its values too: the map that adds them up takes the place of the epilogue.)
+        k::TcGemm whole = g;
+        whole.epilogue.clear();
+        whole.naux = 0;
+        whole.c_hi = nullptr;
+        whole.ldc = n;
+        if (emit && only && (folded || k::gemm_tc_split_plan(ctx, whole) < 2)) {
+            g.c = nullptr;
+            y->data->planes_only = true;
         }
         // An epilogue cannot be applied before the K slices of a split product are summed.  Where the cost model
         // wants slices (few output tiles, long K: a convolution of a small feature map at a small batch), the

@@ -66,7 +66,7 @@ struct MapOp : Operator {
 
     sage_status compute(const std::vector<Tensor> &x, Context &ctx, Tensor *y) override {
         const bool emit = ctx.hint_emit_planes && out.dtype == SAGE_F32, emit_h2 = ctx.hint_emit_h2 && out.dtype == SAGE_F32;
-        const bool wide = ctx.hint_mark_wide;
+        const bool wide = ctx.hint_mark_wide, only = emit && !emit_h2 && ctx.hint_planes_only;
         ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = ctx.hint_mark_wide = false;
         sage_status st = Tensor::uninit(ctx, out, y);
         if (st) return st;
@@ -76,6 +76,7 @@ struct MapOp : Operator {
             if (st) return st;
             planes.hi = y->data->split->planes.planes + y->desc.shape.offset;
             planes.plane = y->data->split->plane;
+            planes.only = y->data->planes_only = only;
         }
         if (emit_h2) {
             st = storage_h2_attach(ctx, *y->data, wide);

@@ -64,6 +64,7 @@ struct RowProgram {
     std::vector<Val> vals;  // topological order
     std::vector<int> in_val, out_val;
     std::vector<Var> out_var;  // the value under the shape it was asked for
+    bool part = false;         // of a larger program, where a result may be wanted as planes alone
     int n_map = 0, n_reduce = 0, n_index = 0;
     std::string source;
     uint32_t stage_bytes = 0;  // dynamic shared memory of the prefetch stages (0: inputs are loaded directly)
@@ -379,7 +380,7 @@ SG void rp_prefetch(const RowP &p, long long row, uint4 *stage);
         }
         if (v.output >= 0) {
             if (v.cls == Full) {
-                s << "    {\n      " << T << " *dst = (" << T << " *)p.out[" << v.output << "] + row * RP_C;\n#pragma unroll\n"
+                s << "    " << (p.part ? "if (p.out[" + std::to_string(v.output) + "]) " : "") << "{\n      " << T << " *dst = (" << T << " *)p.out[" << v.output << "] + row * RP_C;\n#pragma unroll\n"
                   << "      for (int j = 0; j < RP_NV; ++j) {\n        const int c0 = (j * RP_T + (int)threadIdx.x) * RP_VEC;\n"
                   << "        if (RP_WHOLE || c0 < RP_C) ";
                 if (p.vec == 4) {
@@ -431,6 +432,7 @@ std::shared_ptr<RowProgram> row_program_build(const std::vector<Var> &evaluated,
     auto p = std::make_shared<RowProgram>();
     p->rows = R;
     p->cols = C;
+    p->part = !whole_program;
     Builder b{*p, ev, {}, true};
     bool reshaped = false;
     for (const Var &t : targets) {
@@ -590,6 +592,11 @@ sage_status row_program_run(RowProgram &p, Context &ctx, const std::function<boo
         if (st) return st;
         pb[2 + nin + i] = (uint64_t)reinterpret_cast<uintptr_t>(outs[i].ptr());
         const Val &ov = p.vals[p.out_val[i]];
+        // 2: nothing reads the values themselves
+        if (planes && i < planes->size() && (*planes)[i] == 2 && ov.cls == Full && ov.dtype == SAGE_F32) {
+            pb[2 + nin + i] = 0;
+            outs[i].data->planes_only = true;
+        }
         if (planes && i < planes->size() && (*planes)[i] && ov.cls == Full && ov.dtype == SAGE_F32) {
             st = storage_planes_attach(ctx, *outs[i].data);
             if (st) return st;

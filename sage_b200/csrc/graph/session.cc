@@ -618,13 +618,15 @@ static void group_gemms(Node &root) {
     }
 }
 
-static void mark_plane_readers(Node &n, bool tc, std::unordered_set<Origin *> *states, std::unordered_set<Origin *> *h2_states, std::unordered_set<Origin *> *wide_states) {
+// `direct`: how many operands read a state's planes.
+static void mark_plane_readers(Node &n, bool tc, std::unordered_set<Origin *> *states, std::unordered_set<Origin *> *h2_states, std::unordered_set<Origin *> *wide_states,
+                               std::unordered_map<Origin *, int> *direct_reads) {
     if (n.is_data) return;
     if (n.shared && !n.shared->visited) {
         n.shared->visited = true;
-        mark_plane_readers(*n.shared, tc, states, h2_states, wide_states);
+        mark_plane_readers(*n.shared, tc, states, h2_states, wide_states, direct_reads);
     }
-    for (Node &a : n.args) mark_plane_readers(a, tc, states, h2_states, wide_states);
+    for (Node &a : n.args) mark_plane_readers(a, tc, states, h2_states, wide_states, direct_reads);
     const bool grouped = is_grouped_gemm_op(*n.op);
     if (!grouped && (!is_gemm_op(*n.op) || !gemm_runs_on_tc(*n.op, tc))) return;
     const bool h2 = gemm_is_h2(*n.op), wide = gemm_reads_wide(*n.op);
@@ -632,7 +634,10 @@ static void mark_plane_readers(Node &n, bool tc, std::unordered_set<Origin *> *s
         long long offset = 0;
         Node *p = skip_views(&n.args[idx], &offset);
         if (p->is_data) {
-            if (p->var.is_op() && gemm_operand_static_direct(*n.op, idx, offset)) (wide ? wide_states : h2 ? h2_states : states)->insert(p->var.key());
+            if (p->var.is_op() && gemm_operand_static_direct(*n.op, idx, offset)) {
+                (wide ? wide_states : h2 ? h2_states : states)->insert(p->var.key());
+                if (!wide && !h2) ++(*direct_reads)[p->var.key()];
+            }
         } else if (wide) {  // (it reads the fp32 values of wide groups: they stay)
             if (can_mark_wide(*p->op) && gemm_operand_static_direct(*n.op, idx, offset)) p->emit_h2 = p->mark_wide = true;
         } else if (h2 ? can_emit_h2(*p->op) : can_emit_planes(*p->op, tc)) {
@@ -648,6 +653,15 @@ static void mark_plane_readers(Node &n, bool tc, std::unordered_set<Origin *> *s
             }
         }
     }
+}
+
+static void count_reads(const Node &n, std::unordered_map<Origin *, int> *reads, std::unordered_set<const Node *> *shared) {
+    if (n.is_data) {
+        ++(*reads)[n.var.key()];
+        return;
+    }
+    if (n.shared && shared->insert(n.shared.get()).second) count_reads(*n.shared, reads, shared);
+    for (const Node &a : n.args) count_reads(a, reads, shared);
 }
 
 // ------------------------------------------------------------------------------ row groups
@@ -931,8 +945,9 @@ static std::unique_ptr<Program> compile(const std::vector<Var> &x, std::vector<V
             if (!tf32)
                 for (auto &kv : p->routines) assign_h2(kv.second, tc, *p, &done);
         }
+        std::unordered_map<Origin *, int> direct_reads;
         for (auto &kv : p->routines)
-            if (!kv.second.row) mark_plane_readers(kv.second.root, tc, &plane_states, &h2_states, &wide_states);
+            if (!kv.second.row) mark_plane_readers(kv.second.root, tc, &plane_states, &h2_states, &wide_states, &direct_reads);
         for (int form = 0; form < 3; ++form) {
             for (Origin *key : form == 2 ? wide_states : form ? h2_states : plane_states) {
                 // A state that is only a view of another state (reshape(state)) shares its storage, and planes
@@ -954,6 +969,38 @@ static std::unique_ptr<Program> compile(const std::vector<Var> &x, std::vector<V
                 if (!root->is_data && form == 2 && can_mark_wide(*root->op)) root->emit_h2 = root->mark_wide = true;
                 if (!root->is_data && !form && can_emit_planes(*root->op, tc)) root->emit_planes = true;
             }
+        }
+        // States that nothing but products read, all of them the planes, need no values.
+        std::unordered_map<Origin *, int> reads;                   // of a state, by whatever reads it
+        std::unordered_map<Origin *, std::vector<Origin *>> views;  // states that are a view of a state
+        std::unordered_set<const RowProgram *> counted;
+        std::unordered_set<const Node *> shared;
+        for (auto &kv : p->routines) {
+            if (kv.second.row) {
+                if (counted.insert(kv.second.row.get()).second)
+                    for (const Var &v : kv.second.inputs) ++reads[v.key()];
+                continue;
+            }
+            count_reads(kv.second.root, &reads, &shared);
+            const Node *root = skip_views(&kv.second.root);
+            if (root->is_data) views[root->var.key()].push_back(kv.first);
+        }
+        const std::function<bool(Origin *)> products_alone = [&](Origin *key) {
+            if (yset.count(key) || h2_states.count(key) || wide_states.count(key)) return false;
+            const std::vector<Origin *> &v = views[key];
+            if (reads[key] != direct_reads[key] + (int)v.size()) return false;
+            for (Origin *o : v)
+                if (!products_alone(o)) return false;
+            return true;
+        };
+        for (auto &kv : p->routines) {
+            if (kv.second.row) {
+                for (size_t i = 0; i < kv.second.row_outputs.size(); ++i)
+                    if ((*kv.second.row_emit_shared)[i] && products_alone(kv.second.row_outputs[i].key())) (*kv.second.row_emit_shared)[i] = 2;
+                continue;
+            }
+            Node *root = skip_views(&kv.second.root);
+            if (!root->is_data && root->emit_planes && !root->emit_h2 && products_alone(kv.first)) root->planes_only = true;
         }
     }
     p->outputs = y;

@@ -34,6 +34,7 @@ struct PlaneOut {
     long long h2_plane = 0;
     float *h2_scale = nullptr;
     float *h2_marked = nullptr;  // the scales again, negative where a group is wide (gemm_h2_device.inc), for a reader that asks
+    bool only = false;           // (maps) the planes are all that is read: no fp32 values
 };
 
 // column_sums.cu — several [rows, cols] -> [cols] sums in one pass over all of them (src/ops/reduce.rs:258-325, kind Sum); with one
