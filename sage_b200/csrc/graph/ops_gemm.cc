@@ -1222,6 +1222,7 @@ bool gemm_operand_static_direct(const Operator &op, int idx, long long offset) {
     if (g && g->attn) return idx < 3 && GemmOp::attention_view_direct(sh, g->attention_trans(idx));
     if (g && g->h2) return idx == 0 && (g->conv ? conv_image_direct(sh) : h2_view_ok(sh, g->ta));
     if (g && g->conv && idx == 0) return g->conv_implicit() && !g->conv_raw() && offset % 4 == 0;  // planes only when the kernel does not split the image itself
+    if (g && g->conv && idx == 1 && g->conv_small_c()) return false;  // the filter is packed from its values
     return g && idx < 2 && gemm_operand_view_ok(sh);
 }
 
