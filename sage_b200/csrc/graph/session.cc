@@ -786,33 +786,34 @@ static std::unique_ptr<Program> compile(const std::vector<Var> &x, std::vector<V
     // step) is not kept: the products read the other one through the view, as they do where the copy has one reader.
     std::unordered_set<Origin *> kept_instead;
     if (pattern && tc) {
-        std::unordered_map<Origin *, std::vector<std::pair<Var, int>>> readers;
-        for (auto &kv : nodes)
-            if (kv.second.is_op() && !xset.count(kv.first)) {
-                const std::vector<Var> &kids = children(kv.second, pattern, nullptr);
-                for (size_t i = 0; i < kids.size(); ++i) readers[kids[i].key()].push_back({kv.second, (int)i});
-            }
+        std::unordered_map<Origin *, std::vector<std::pair<const Var *, int>>> readers;  // made when first asked for
         const size_t before = candidates.size();
         for (size_t i = 0; i < before; ++i) {
-            const Var v = candidates[i];
-            if (yset.count(v.key())) continue;
-            Var at = v;
-            auto below = [&](const Var &w) { return w.is_op() && !xset.count(w.key()) && !yset.count(w.key()) && !w.origin->composite && w.origin->inputs.size() == 1 && (w.key() == v.key() || edges[w.key()] == 1); };
-            while (below(at) && is_reshape_op(*at.origin->op) && reshape_keeps_matrix(*at.origin->op)) at = at.origin->inputs[0];
-            if (!below(at) || !is_copy_map(*at.origin->op) || at.origin->op->in[0].shape.has_default_strides()) continue;
-            const TensorDesc view = at.origin->op->in[0];
-            at = at.origin->inputs[0];
-            while (below(at) && is_view_op(*at.origin->op)) at = at.origin->inputs[0];
-            if (!at.is_op() || is_view_op(*at.origin->op) || !at.desc.shape.has_default_strides()) continue;
+            Origin *const v = candidates[i].key();
+            const Var *at = &candidates[i];
+            auto below = [&](const Var &w) { return w.is_op() && !xset.count(w.key()) && !yset.count(w.key()) && !w.origin->composite && w.origin->inputs.size() == 1 && (w.key() == v || edges[w.key()] == 1); };
+            while (below(*at) && is_reshape_op(*at->origin->op) && reshape_keeps_matrix(*at->origin->op)) at = &at->origin->inputs[0];
+            if (!below(*at) || !is_copy_map(*at->origin->op) || at->origin->op->in[0].shape.has_default_strides()) continue;
+            const TensorDesc &view = at->origin->op->in[0];
+            at = &at->origin->inputs[0];
+            while (below(*at) && is_view_op(*at->origin->op)) at = &at->origin->inputs[0];
+            if (!at->is_op() || is_view_op(*at->origin->op) || !at->desc.shape.has_default_strides()) continue;
+            if (readers.empty())
+                for (auto &kv : nodes)
+                    if (kv.second.is_op() && !xset.count(kv.first)) {
+                        const std::vector<Var> &kids = children(kv.second, pattern, nullptr);
+                        for (size_t j = 0; j < kids.size(); ++j) readers[kids[j].key()].push_back({&kv.second, (int)j});
+                    }
             bool products = true;
-            for (auto &r : readers[v.key()]) {
+            for (auto &r : readers[v]) {
                 std::shared_ptr<Operator> op;
-                children(r.first, pattern, &op);
+                children(*r.first, pattern, &op);
                 if (!is_gemm_op(*op) || !gemm_with_operand_view(*op, r.second, view, tc)) products = false;
             }
             if (!products) continue;
-            candidates[i] = at;  // (perhaps one of them already)
-            kept_instead.insert(at.key());
+            kept_instead.insert(at->key());
+            const Var base = *at;  // (it lies in what the candidate keeps alive)
+            candidates[i] = base;  // (perhaps one of them already)
         }
     }
     std::stable_sort(candidates.begin(), candidates.end(), [](const Var &a, const Var &b) {
@@ -1084,28 +1085,29 @@ static void assign_slots(Node &n, const std::unordered_map<Origin *, int> &slot_
 // The order in which exec() runs the routines while nothing is evicted.
 static bool plan_order(Program &p, const Session &s, std::vector<Routine *> *order) {
     std::unordered_set<Origin *> computed;
-    std::vector<Var> stack(p.outputs.begin(), p.outputs.end());
+    std::vector<const Var *> stack;
+    for (const Var &v : p.outputs) stack.push_back(&v);
     auto available = [&](const Var &v) { return v.is_data() || s.data.count(v.key()) || computed.count(v.key()); };
     while (!stack.empty()) {
-        const Var v = stack.back();
-        if (available(v)) {
+        const Var *const v = stack.back();
+        if (available(*v)) {
             stack.pop_back();
             continue;
         }
-        auto it = p.routines.find(v.key());
+        auto it = p.routines.find(v->key());
         if (it == p.routines.end()) return false;
         Routine &f = it->second;
         bool ready = true;
         for (const Var &k : f.inputs)
             if (!available(k)) {
-                stack.push_back(k);
+                stack.push_back(&k);
                 ready = false;
             }
         if (!ready) continue;
         if (f.row)
             for (const Var &o : f.row_outputs) computed.insert(o.key());
         else
-            computed.insert(v.key());
+            computed.insert(v->key());
         order->push_back(&f);
         stack.pop_back();
     }
