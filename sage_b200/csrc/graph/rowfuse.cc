@@ -211,6 +211,8 @@ bool screen(const std::vector<Var> &targets, const std::unordered_set<Origin *> 
     return largest > 0 && *R > 1 && *C > 1 && (reduces || maps_suffice);
 }
 
+const char *kernel_name(const RowProgram &p) { return p.cols < 32 ? "sage_narrow_rows" : "sage_row_program"; }
+
 // Whole-row values that a thread holds across an exchange at once: each is a register per element.
 int rows_alive(const RowProgram &p) {
     std::vector<int> last(p.vals.size(), -1);  // where a value is read last (outputs are stored where they are computed)
@@ -295,7 +297,7 @@ SG void rp_prefetch(const RowP &p, long long row, uint4 *stage);
     s << "#define RP_STAGE " << (size_t)n_stage * p.nv * p.threads << "\n";
     // at least as many blocks per SM as p.regs registers per thread allow: more warps to hide the latency of
     // exp, shared memory and shuffles (the kernels run at low occupancy by construction)
-    s << "extern \"C\" __global__ void __launch_bounds__(RP_T, " << std::max(1, 65536 / (p.threads * p.regs)) << ") sage_row_program(const RowP p) {\n"
+    s << "extern \"C\" __global__ void __launch_bounds__(RP_T, " << std::max(1, 65536 / (p.threads * p.regs)) << ") " << kernel_name(p) << "(const RowP p) {\n"
       << "  asm volatile(\"griddepcontrol.launch_dependents;\" ::: \"memory\");\n"
       << "  asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");\n"
       << "  __shared__ float sh[2][" << std::max(1, n_red) << "][32];\n  __shared__ uint sh_pick[2][" << std::max(1, n_pick) << "];\n";
@@ -423,12 +425,20 @@ SG void rp_prefetch(const RowP &p, long long row, uint4 *stage);
 
 }  // namespace
 
+// Rows of fewer than 32 columns: a warp each, most of its lanes idle, but the many small launches of a loss over few classes become one
+// (about 3 us each in a training step, ResNet-18's 983 -> 951 us).  Any program up to 4096 rows, losses up to 2^18.  us, kernel by kernel |
+// this; loss and gradient of a cross entropy (18 launches), 10 classes: 128 rows 50.9 | 6.2, 4096 51.0 | 8.9, 65536 127 | 16.0, 2^18 416 |
+// 52.9; 2 classes 49.5 | 6.0, 50.7 | 6.3, 118 | 15.9, 375 | 52.9; 28: 46.7 | 6.1, 46.4 | 6.3, 64.6 | 21.4, 166 | 81.4.  With two exchanges
+// (four launches): 4096 x 2 18.8 | 5.6, x 28 12.0 | 4.7; 65536 x 28 15.1 | 14.5; 2^18 x 2 [12.3] | 28.1, x 28 [40.4] | 52.2.  One (two
+// launches): 4096 x 10 8.7 | 5.5, x 31 6.9 | 5.5; 16384 x 28 [6.8] | 8.5, 65536 x 10 [6.9] | 11.7.
+bool row_space_narrow(long long rows, long long cols, bool loss) { return cols > 1 && cols < 32 && rows <= (loss ? 1 << 18 : 4096); }
+
 std::shared_ptr<RowProgram> row_program_build(const std::vector<Var> &evaluated, const std::vector<Var> &targets, bool whole_program, bool emit_source) {
     std::unordered_set<Origin *> ev;
     for (const Var &v : evaluated) ev.insert(v.key());
     long long R = 0, C = 0;
     if (!screen(targets, ev, !whole_program, &R, &C)) return nullptr;
-    if (C < 32 || C > 16384) return nullptr;
+    if (C > 16384 || (C < 32 && !row_space_narrow(R, C, true))) return nullptr;
     auto p = std::make_shared<RowProgram>();
     p->rows = R;
     p->cols = C;
@@ -452,6 +462,7 @@ std::shared_ptr<RowProgram> row_program_build(const std::vector<Var> &evaluated,
         p->out_val.push_back(id);
         p->out_var.push_back(t);
     }
+    if (C < 32 && !row_space_narrow(R, C, p->n_index > 0 && p->n_reduce + p->n_index >= 4)) return nullptr;
     if (reshaped && p->n_reduce + p->n_index == 0) return nullptr;
     bool full_leaf = false;
     for (int id : p->in_val) full_leaf = full_leaf || p->vals[id].cls == Full;
@@ -462,7 +473,7 @@ std::shared_ptr<RowProgram> row_program_build(const std::vector<Var> &evaluated,
     // issue limit as to the HBM one); 16 per thread from 2048 columns, 8 from 1024, else 4.
     p->vec = C % 4 == 0 ? 4 : 1;
     const long long units = (C + p->vec - 1) / p->vec;  // vectors per row
-    int elems = C >= 2048 ? 16 : C >= 1024 ? 8 : 4;
+    int elems = C >= 2048 ? 16 : C >= 1024 ? 8 : C < 32 ? p->vec : 4;
     if (const char *e = getenv("SAGE_ROW_PROGRAM_ELEMS")) elems = std::max(4, atoi(e));  // tuning aid
     p->nv = std::max(1, elems / p->vec);
     long long t = (units + p->nv - 1) / p->nv;
@@ -552,7 +563,7 @@ sage_status row_program_run(RowProgram &p, Context &ctx, const std::function<boo
         sage_status st = ctx.module_get(p.source, &p.module);
         if (st) return st;
         p.owner = &ctx;
-        p.resident = ctx.blocks_per_sm(p.module, "sage_row_program", p.threads, p.stage_bytes);
+        p.resident = ctx.blocks_per_sm(p.module, kernel_name(p), p.threads, p.stage_bytes);
     }
     std::vector<Tensor> keep;
     const size_t nin = std::max<size_t>(1, p.in_val.size()), nout = std::max<size_t>(1, p.out_val.size());
@@ -608,7 +619,7 @@ sage_status row_program_run(RowProgram &p, Context &ctx, const std::function<boo
     const uint32_t grid[3] = {(uint32_t)std::min<long long>(p.rows, resident), 1, 1};
     const uint32_t block[3] = {(uint32_t)p.threads, 1, 1};
     void *params[1] = {pb.data()};
-    return ctx.launch(p.module, "sage_row_program", grid, block, p.stage_bytes, params, nullptr, true);
+    return ctx.launch(p.module, kernel_name(p), grid, block, p.stage_bytes, params, nullptr, true);
 }
 
 }  // namespace sage

@@ -33,6 +33,8 @@ sage_status row_program_exec(RowProgram &p, Context &ctx, Session &s);
 sage_status row_program_run(RowProgram &p, Context &ctx, const std::function<bool(const Var &, Tensor *)> &fetch, std::vector<Tensor> *outs,
                             const std::vector<char> *planes = nullptr);
 void row_program_space(const RowProgram &p, long long *rows, long long *cols);
+// Rows of fewer than 32 columns that may be a program (rowfuse.cc has the figures); `loss`: one that picks elements and has four exchanges.
+bool row_space_narrow(long long rows, long long cols, bool loss);
 std::vector<Var> row_program_inputs(const RowProgram &p);
 int row_program_exchanges(const RowProgram &p);  // reductions + gathers + scatters in the program
 // Are the evaluated values the program was cut at still held by the session?

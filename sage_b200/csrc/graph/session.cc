@@ -39,6 +39,7 @@ struct Node {
 
 // ops_map.cc / ops_core.cc / ops_gemm.cc / ops_nn.cc
 bool is_copy_map(const Operator &op);
+int index_op_axis(const Operator &op, bool scatter);
 std::shared_ptr<Operator> map_over_expanded(const Operator &op, const Array &extents);
 std::shared_ptr<Operator> make_expand_op(const TensorDesc &in, const Array &extents);
 bool is_expand_op(const Operator &op);
@@ -782,6 +783,19 @@ static std::unique_ptr<Program> compile(const std::vector<Var> &x, std::vector<V
         if (kv.second >= 2 && v.is_op() && !xset.count(kv.first) && !yset.count(kv.first)) candidates.push_back(v);
     }
     for (const Var &v : y) candidates.push_back(v);
+    // A sum over rows that pick an element each (a loss over labels): what is below it stays in a row space and can be one kernel.
+    if (pattern && row_groups)
+        for (auto &kv : nodes) {
+            auto first_input = [&](const Var &v) -> const Var * {
+                return v.is_op() && !v.origin->composite && !xset.count(v.key()) && !v.origin->inputs.empty() ? &v.origin->inputs[0] : nullptr;
+            };
+            const Var *at = kv.second.size() == 1 ? first_input(kv.second) : nullptr;
+            if (!at || kv.second.origin->op->cat() != Cat::Reduce || !first_input(*at) || at->size() < 2 || yset.count(at->key()) || edges[at->key()] != 1) continue;
+            const Var &rows = *at;
+            while (at && first_input(*at) && index_op_axis(*at->origin->op, false) < 0)
+                at = at->origin->op->cat() == Cat::Reduce || map_expr_of(*at->origin->op) || is_view_op(*at->origin->op) ? first_input(*at) : nullptr;
+            if (at && first_input(*at) && first_input(*at)->rank() > 1 && row_space_narrow((long long)rows.size(), (long long)first_input(*at)->extents().back(), true)) candidates.push_back(rows);
+        }
     // A value that is a permuted copy of another one and that only products read (the heads of an attention block in a training
     // step) is not kept: the products read the other one through the view, as they do where the copy has one reader.
     std::unordered_set<Origin *> kept_instead;
