@@ -1252,7 +1252,9 @@ static sage_status exec_scheduled(Program &p, Context &ctx, Session &s) {
                     for (size_t i = 0; i < outs.size(); ++i) p.slots[step.outputs[i]] = std::move(outs[i]);
             } else {
                 SharedMemo memo;
-                st = run_node(f.root, ctx, s, values, memo, &p.slots[step.outputs[0]], step.leaf ? &batch : nullptr);
+                Tensor out;  // (an operator allocates its result first: what a step that failed leaves is no value)
+                st = run_node(f.root, ctx, s, values, memo, &out, step.leaf ? &batch : nullptr);
+                if (!st) p.slots[step.outputs[0]] = std::move(out);
             }
             first.done(st);
             if (st) break;
