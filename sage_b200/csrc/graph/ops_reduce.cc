@@ -60,11 +60,10 @@ struct ReduceOp : Operator {
         x[0].desc.shape.extract(axes, &inner, &outer);
         k::ColumnSum sum;
         if (batch && k::column_sum_of(x[0].desc.dtype, (int)kind, (const char *)x[0].data->dev + outer.offset * 4, to_dims(outer), to_dims(inner), y->ptr(), &sum)) {
-            if (x[0].data.use_count() == 1) batch->own_bytes += x[0].data->bytes;  // worked out for this sum alone
             batch->column_sums.push_back(sum);
             batch->held_by_sums.push_back(x[0].data);
             batch->held_by_sums.push_back(y->data);
-            return batch->own_bytes > k::LeafBatch::kMaxOwnBytes ? batch->run_sums(ctx) : SAGE_OK;
+            return SAGE_OK;
         }
         return k::reduce(ctx, x[0].desc.dtype, (int)kind, (const char *)x[0].data->dev + outer.offset * 4, to_dims(outer),
                          to_dims(inner), y->ptr());

@@ -1031,6 +1031,12 @@ struct Values {
     const Tensor *slots = nullptr;
 };
 
+static size_t planes_bytes(const Storage &st) {
+    size_t n = 0;
+    for (const std::shared_ptr<SplitCache> &c : {st.split, st.split_view}) n += c && c->planes.block ? c->planes.block->size : 0;
+    return n;
+}
+
 // `batch`: where the launches of leaf nodes are collected, or null.
 static sage_status run_node(const Node &n, Context &ctx, Session &s, const Values &values, SharedMemo &memo, Tensor *out, k::LeafBatch *batch = nullptr) {
     if (n.is_data) {
@@ -1079,11 +1085,28 @@ static sage_status run_node(const Node &n, Context &ctx, Session &s, const Value
     ctx.hint_emit_h2 = n.emit_h2;
     ctx.hint_planes_only = (n.emit_planes || n.emit_h2) && n.planes_only;
     ctx.hint_mark_wide = n.mark_wide;
-    ctx.hint_batch = n.leaf ? batch : nullptr;
+    if (!n.leaf) batch = nullptr;
+    ctx.hint_batch = batch;
+    // What a launch that is put off keeps alive: operands worked out for it alone, and planes of a state's that were made for it.
+    // (The states themselves were all alive at the first of the leaves; a program's data keep their planes in any case.)
+    auto kept = [&](bool computed) {
+        size_t bytes = 0;
+        for (size_t i = 0; i < args.size(); ++i) {
+            const Node *from = &n.args[i];
+            while (!from->is_data && !from->shared && is_view_op(*from->op) && from->args.size() == 1) from = &from->args[0];
+            if (from->is_data ? from->var.is_op() : computed) bytes += planes_bytes(*args[i].data) + (from->is_data ? 0 : args[i].data->bytes);
+        }
+        return bytes;
+    };
+    const size_t products = batch ? batch->products.size() : 0, sums = batch ? batch->column_sums.size() : 0, before = batch ? kept(false) : 0;
     sage_status st = n.op->compute(args, ctx, out);
     ctx.hint_emit_planes = ctx.hint_emit_h2 = ctx.hint_planes_only = ctx.hint_mark_wide = false;
     ctx.hint_batch = nullptr;
-    return st;
+    if (!batch || st) return st;
+    const size_t after = kept(true), own = after > before ? after - before : 0;
+    if (batch->products.size() > products && (batch->own_bytes += own) > k::LeafBatch::kMaxOwnBytes) return batch->run_products(ctx);
+    if (batch->column_sums.size() > sums && (batch->own_bytes_of_sums += own) > k::LeafBatch::kMaxOwnBytes) return batch->run_sums(ctx);
+    return SAGE_OK;
 }
 
 static void assign_slots(Node &n, const std::unordered_map<Origin *, int> &slot_of) {
@@ -1201,8 +1224,8 @@ struct FirstRun {
 // A run along the schedule.  Out of memory, it hands what it has computed to the general run, which evicts and recomputes.
 //
 // Steps that follow one another and whose results no step reads (a training step ends with the gradients of all parameters) leave
-// products and column sums to a batch: one launch for all of a kind.  What they read lives until the batch has run, as it
-// did at the first of them.
+// products and column sums to a batch: one launch for all of a kind.  The states they read live until the batch has run, as they
+// did at the first of them; of what a step works out for its own product or sum, or splits for it, 128 MiB of each kind.
 static sage_status exec_scheduled(Program &p, Context &ctx, Session &s) {
     if (!p.times_read) {  // timers of the first run
         p.times_read = true;
@@ -1230,7 +1253,7 @@ static sage_status exec_scheduled(Program &p, Context &ctx, Session &s) {
         std::vector<std::pair<Var, Tensor>> batched;  // results that the batch computes
         auto flush = [&]() {
             const sage_status ran = batch.empty() ? SAGE_OK : batch.run(ctx);
-            if (ran == SAGE_OK && st == SAGE_OK)
+            if (batch.status == SAGE_OK)  // (whatever became of the step at hand)
                 for (auto &v : batched) s.data[v.first.key()] = v;
             batched.clear();
             return ran;
@@ -1266,7 +1289,7 @@ static sage_status exec_scheduled(Program &p, Context &ctx, Session &s) {
                 }
             for (int n : step.release) p.slots[n] = Tensor();
         }
-        const sage_status ran = flush();  // (out of memory or not: what is collected needs no more of it)
+        const sage_status ran = flush();  // (out of memory or not: what is collected needs no more of it, and its results are kept)
         if (!st) st = ran;
         if (st != SAGE_ERR_OOM) return st;
         for (Program::Step &step : p.schedule)

@@ -309,15 +309,22 @@ sage_status LeafBatch::run_sums(Context &ctx) {
     const sage_status st = column_sums.empty() ? SAGE_OK : column_sums_run(ctx, column_sums);
     column_sums.clear();
     held_by_sums.clear();
+    own_bytes_of_sums = 0;
+    if (!status) status = st;
+    return st;
+}
+
+sage_status LeafBatch::run_products(Context &ctx) {
+    const sage_status st = products.empty() ? SAGE_OK : gemm_tc_group_run(ctx, products);
+    products.clear();
+    held.clear();
     own_bytes = 0;
+    if (!status) status = st;
     return st;
 }
 
 sage_status LeafBatch::run(Context &ctx) {
-    sage_status st = products.empty() ? SAGE_OK : gemm_tc_group_run(ctx, products);
-    products.clear();
-    held.clear();
-    const sage_status sums = run_sums(ctx);
+    const sage_status st = run_products(ctx), sums = run_sums(ctx);
     return st ? st : sums;
 }
 

@@ -194,11 +194,14 @@ struct LeafBatch {
     std::vector<ColumnSum> column_sums;
     std::vector<TcGemm> products;
     std::vector<std::shared_ptr<void>> held, held_by_sums;
-    size_t own_bytes = 0;  // of the sums' operands that nothing but the batch keeps alive
+    // Of the operands, what would be gone by now had each launch been made at once: the products' and the sums' kinds run when it passes the limit.
+    size_t own_bytes = 0, own_bytes_of_sums = 0;
     static constexpr size_t kMaxOwnBytes = (size_t)128 << 20;
+    sage_status status = 0;  // of the launches so far
     bool empty() const { return column_sums.empty() && products.empty(); }
     sage_status run(Context &ctx);  // ... and empties it
-    sage_status run_sums(Context &ctx);  // the sums alone
+    sage_status run_products(Context &ctx);
+    sage_status run_sums(Context &ctx);
 };
 // hi/lo split of `n` consecutive floats into planes laid out like the source (dst_hi[i], dst_hi[plane + i]).
 sage_status split_tf32_flat(Context &ctx, const float *src, long long n, float *dst_hi, long long plane);

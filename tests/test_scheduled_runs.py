@@ -126,3 +126,52 @@ def test_first_runs_under_a_limit_give_the_unrestricted_values():
             # (the sum over a product's K slices has no room at some limits: one pass over K instead, 2^-20 of the terms' magnitudes)
             assert np.allclose(run[1], want, rtol=0, atol=2.0 ** -14 * np.abs(want).max()), d
     assert evicted >= 8
+
+
+def independent_products(c, k, x, y):
+    """(x a)^T (y b): products that nothing reads, each with operands of its own, which are put off to run together."""
+    x, y = c.var(x), c.var(y)
+    return [S.transpose(x * float(i + 2), 1, 0).matmul(y * (float(i) - 2.5)) for i in range(k)]
+
+
+def test_products_put_off_keep_little_alive_and_run_once():
+    """Operands of 16 MiB, 32 of planes each: 96 MiB a product, of which 128 and the product's at hand are kept."""
+    x = np.zeros((4096, 1024), np.float32)
+    peaks = {}
+    for k, limits in ((24, (0,)), (8, (0, 168, 184, 232, 264, 312, 328))):
+        for limit in limits:
+            c = S.Context(-1, **({"mem_capacity_bytes": limit * MIB} if limit else {}))
+            out = independent_products(c, k, x, x)
+            for _ in range(2):
+                c.clear()
+                c.trace_begin()
+                c.eval(*out)
+                assert sum("gemm" in t for t in c.trace()) == k, (k, limit)  # out of memory or not, none is worked out again
+            if not limit:
+                peaks[k] = c.mem_stats()["mem_peak"]
+            c.close()
+    assert peaks[24] - peaks[8] == 16 * 4 * MIB  # the results
+    assert peaks[8] <= (32 + 2 * 96 + 32 + 8 * 4 + 3 * 20) * MIB  # x and y, two products' operands, values before their planes, results, segments
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("limit", [0, 168, 200, 264, 328])
+def test_products_put_off_under_a_limit(limit):
+    """Against float64, within (2^-22 + 48 x 2^-23 + (rows / 128 + 1) 2^-24) |x|^T |y|, as grouped products by themselves."""
+    rng = np.random.default_rng(79)
+    x, y = rng.standard_normal((4096, 1024)).astype(np.float32), rng.standard_normal((4096, 1024)).astype(np.float32)
+    c = S.Context(0, **({"mem_capacity_bytes": limit * MIB} if limit else {}))
+    try:
+        out = independent_products(c, 8, x, y)
+        for _ in range(2):
+            c.clear()
+            c.eval(*out)
+        got = [c.read(t).copy() for t in out]
+        assert c.status_word() == 0
+    finally:
+        c.close()
+    xy, size = x.astype(np.float64).T @ y, np.abs(x).astype(np.float64).T @ np.abs(y)
+    bound = (2.0 ** -22 + 48 * 2.0 ** -23 + (4096 / 128 + 1) * 2.0 ** -24 + 2.0 ** -23) * size  # (and the two maps' roundings)
+    for i, g in enumerate(got):
+        a = (i + 2) * (i - 2.5)
+        assert (np.abs(g - a * xy) <= abs(a) * bound).all(), i
