@@ -270,9 +270,10 @@ sage_status sage_peer_write_ptr(sage_ctx *ctx, void *peer_ptr, size_t peer_offse
 /* ------------------------------------------------------------------ introspection (planning + tests) */
 /* Number of kernels / memsets this context has launched (or recorded, on a planning context). */
 sage_status sage_launch_count(sage_ctx *ctx, uint64_t *kernels, uint64_t *memsets);
-/* Start/stop recording kernel names; sage_trace_get copies a '\n'-separated list, a line per launch.  One launch has two
- * lines: the one that brings both operands of a plain product into pieces is listed once for each, so the list can be longer than
- * sage_launch_count's count, which is of launches. */
+/* Start/stop recording kernel names; sage_trace_get copies a '\n'-separated list, a line per launch, except that a launch which
+ * does the work of several has a line for each of them: the one that brings both operands of a plain product into pieces (two lines),
+ * and those that run results together which nothing else of a program reads: products and the sums over their K slices (up to 100
+ * lines), sums over columns and over whole tensors (up to 96).  So the list can be longer than sage_launch_count's count, which is of launches. */
 sage_status sage_trace_begin(sage_ctx *ctx);
 sage_status sage_trace_get(sage_ctx *ctx, char *out, size_t out_len, size_t *needed);
 /* Device time per kernel name.  Between begin and end a CUDA event is recorded on the context's
