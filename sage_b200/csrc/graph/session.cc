@@ -1227,10 +1227,10 @@ struct FirstRun {
 // products and column sums to a batch: one launch for all of a kind.  The states they read live until the batch has run, as they
 // did at the first of them; of what a step works out for its own product or sum, or splits for it, 128 MiB of each kind.
 static sage_status exec_scheduled(Program &p, Context &ctx, Session &s) {
-    if (!p.times_read) {  // timers of the first run
+    if (!p.times_read) {  // the first run's timers, as soon as every step has had one; their events go with them
         p.times_read = true;
-        for (auto &kv : p.routines)
-            if (!kv.second.resolve_time()) p.times_read = false;
+        for (const Program::Step &step : p.schedule)
+            if (!step.routine->timed || !step.routine->resolve_time()) p.times_read = false;
     }
     for (auto &g : p.given) {
         auto it = s.data.find(g.first);
