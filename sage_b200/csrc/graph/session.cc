@@ -619,15 +619,30 @@ static void group_gemms(Node &root) {
     }
 }
 
-// `direct`: how many operands read a state's planes.
-static void mark_plane_readers(Node &n, bool tc, std::unordered_set<Origin *> *states, std::unordered_set<Origin *> *h2_states, std::unordered_set<Origin *> *wide_states,
+// Where a state starts in the storage it lies in: it may be a view of its routine's result, or of another state.
+static long long state_offset(Program &p, Origin *key) {
+    long long at = 0;
+    for (int hops = 0; hops < 8; ++hops) {
+        auto it = p.routines.find(key);
+        if (it == p.routines.end() || it->second.row) break;
+        long long views = 0;
+        const Node *root = skip_views(&it->second.root, &views);
+        at += views;
+        if (!root->is_data || !root->var.is_op()) break;
+        key = root->var.key();
+    }
+    return at;
+}
+
+// `direct_reads`: how many operands read a state's planes.
+static void mark_plane_readers(Node &n, bool tc, Program &program, std::unordered_set<Origin *> *states, std::unordered_set<Origin *> *h2_states, std::unordered_set<Origin *> *wide_states,
                                std::unordered_map<Origin *, int> *direct_reads) {
     if (n.is_data) return;
     if (n.shared && !n.shared->visited) {
         n.shared->visited = true;
-        mark_plane_readers(*n.shared, tc, states, h2_states, wide_states, direct_reads);
+        mark_plane_readers(*n.shared, tc, program, states, h2_states, wide_states, direct_reads);
     }
-    for (Node &a : n.args) mark_plane_readers(a, tc, states, h2_states, wide_states, direct_reads);
+    for (Node &a : n.args) mark_plane_readers(a, tc, program, states, h2_states, wide_states, direct_reads);
     const bool grouped = is_grouped_gemm_op(*n.op);
     if (!grouped && (!is_gemm_op(*n.op) || !gemm_runs_on_tc(*n.op, tc))) return;
     const bool h2 = gemm_is_h2(*n.op), wide = gemm_reads_wide(*n.op);
@@ -635,7 +650,7 @@ static void mark_plane_readers(Node &n, bool tc, std::unordered_set<Origin *> *s
         long long offset = 0;
         Node *p = skip_views(&n.args[idx], &offset);
         if (p->is_data) {
-            if (p->var.is_op() && gemm_operand_static_direct(*n.op, idx, offset)) {
+            if (p->var.is_op() && gemm_operand_static_direct(*n.op, idx, offset + state_offset(program, p->var.key()))) {
                 (wide ? wide_states : h2 ? h2_states : states)->insert(p->var.key());
                 if (!wide && !h2) ++(*direct_reads)[p->var.key()];
             }
@@ -962,7 +977,7 @@ static std::unique_ptr<Program> compile(const std::vector<Var> &x, std::vector<V
         }
         std::unordered_map<Origin *, int> direct_reads;
         for (auto &kv : p->routines)
-            if (!kv.second.row) mark_plane_readers(kv.second.root, tc, &plane_states, &h2_states, &wide_states, &direct_reads);
+            if (!kv.second.row) mark_plane_readers(kv.second.root, tc, *p, &plane_states, &h2_states, &wide_states, &direct_reads);
         for (int form = 0; form < 3; ++form) {
             for (Origin *key : form == 2 ? wide_states : form ? h2_states : plane_states) {
                 // A state that is only a view of another state (reshape(state)) shares its storage, and planes

@@ -55,3 +55,48 @@ def test_gradients_are_those_of_the_plain_evaluation(heads, d, length, batch):
     scale = max(np.abs(g).max() for g in got[1][1:])
     for a, b in zip(got[0][1:], got[1][1:]):
         assert np.abs(a - b).max() <= 2.0 ** (-14 if a.size > 1 else -14 + 7) * max(np.abs(b).max(), 2.0 ** -10 * scale)
+
+
+def views(c, kind, shift, seed=0):
+    """A value, read by products alone, that starts `shift` elements into the storage it lies in."""
+    rng = np.random.default_rng(seed)
+    m, k = 256, 128
+    x = rng.standard_normal({"flat": (m * k + 8,), "columns": (m, k + 8), "rows": (m + 8, k)}[kind]).astype(np.float32)
+    a = c.var(x) * 2.0 + 1.0
+    v = S.view(a.slice(0, shift, shift + m * k), [m, k]) if kind == "flat" else a.slice(1, shift, shift + k) if kind == "columns" else a.slice(0, shift, shift + m)
+    w, u, g = (rng.standard_normal(s).astype(np.float32) for s in ((k, 96), (k, 64), (m, 96)))
+    x = x * 2.0 + 1.0
+    x = x[shift:shift + m * k].reshape(m, k) if kind == "flat" else x[:, shift:shift + k] if kind == "columns" else x[shift:shift + m]
+    return v, [v.matmul(c.var(w)), v.matmul(c.var(u)), S.transpose(v, 1, 0).matmul(c.var(g))], [x @ w, x @ u, x.T @ g], [np.abs(x) @ np.abs(w), np.abs(x) @ np.abs(u), np.abs(x).T @ np.abs(g)]
+
+
+@pytest.mark.parametrize("kind", ["flat", "columns", "rows"])
+@pytest.mark.parametrize("shift", [0, 1, 2, 4])
+def test_what_products_alone_read_keeps_values_only_where_they_need_them(kind, shift):
+    """Products read planes where a view's rows lie on 16 bytes, whatever state the view is; else they gather its values."""
+    for more in (None, "value", "sum"):
+        c = S.Context(-1)
+        v, products, _, _ = views(c, kind, shift)
+        c.eval(*products, *([v] if more == "value" else [v.exp().sum([0], False)] if more == "sum" else []))
+        first = c.describe().splitlines()[0]
+        direct = shift % 4 == 0 or kind == "rows"
+        assert ("=planes" in first) == (direct and more is None) and ("+planes" in first) == (direct and more is not None), first
+        c.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["flat", "columns", "rows"])
+@pytest.mark.parametrize("shift", [0, 1, 2, 4])
+def test_products_of_views_that_start_anywhere(kind, shift):
+    """Within 2^-19 of |a| |b|, the bound of the products."""
+    c = S.Context(0)
+    try:
+        _, products, want, size = views(c, kind, shift)
+        for _ in range(2):
+            c.clear()
+            c.eval(*products)
+        for p, w, s in zip(products, want, size):
+            assert (np.abs(c.read(p) - w) <= 2.0 ** -19 * s).all()
+        assert c.status_word() == 0
+    finally:
+        c.close()
