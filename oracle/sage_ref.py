@@ -492,7 +492,7 @@ class ViewOp:
 
     def grad(self, x, y, gy):
         k, kw, x0 = self.kind, self.kw, x[0]
-        if k == "reshape": return [reshape(gy, Shape(x0.shape.extents, x0.shape.strides, x0.shape.offset))]
+        if k == "reshape": return [reshape(gy, Shape(x0.shape.extents, x0.shape.strides))]  # core.rs:242-244 keeps x0's offset and reads past gy's end
         if k == "expand":  # core.rs:292-313
             surplus = gy.rank() - x0.rank()
             axes = list(range(surplus)) + [i + surplus for i in range(x0.rank()) if gy.extent(i + surplus) != x0.extent(i)]

@@ -43,7 +43,7 @@ struct ViewOp : Operator {
     std::vector<Var> grad(const std::vector<Var> &x, const Var &, const Var &gy) override {
         const Var &x0 = x[0];
         switch (kind) {
-        case VReshape: return {reshape(gy, in[0].shape)};  // core.rs:242-244
+        case VReshape: return {view(gy, in[0].shape.extents)};  // core.rs:242-244, but for the offset there: gy starts where it starts
         case VExpand: {                                     // core.rs:292-313
             const int surplus = gy.rank() - x0.rank();
             std::vector<long long> axes;
