@@ -129,7 +129,8 @@ struct Col2imOp : Operator {
 };
 
 // A map of one operand before a column matrix, as part of it: null where the operand is not laid out like the image or the kernel does not
-// take four channels at a time.  (Storages start on 512 bytes: the offset says where a tensor lies.)
+// take four channels at a time.  (An operand's description does not show every start: a reshaped slice may lie off the 16-byte grid all
+// the same, and the map is then worked out by itself.)
 std::shared_ptr<Operator> im2col_with_map(const Operator &op, const Operator &map, const std::string &expr) {
     const Im2colOp *o = dynamic_cast<const Im2colOp *>(&op);
     if (!o || !o->pre.empty() || map.in.size() != 1 || k::long_expression(expr)) return nullptr;  // (it is worked out for every tap)

@@ -642,17 +642,18 @@ sage_status pool2d(Context &ctx, bool is_max, const float *img, float *out, long
                    long long img_w, long long chan, long long out_h, long long out_w, const Window &w, const PlaneOut &forms) {
     ConvP p{n, img_h, img_w, chan, out_h, out_w, w};
     long long total = n * out_h * out_w * chan;
-    ctx.note_launch(is_max ? "max_pool2d" : "avg_pool2d");
-    if (ctx.dry() || total == 0) return SAGE_OK;
     const bool vec = chan % 4 == 0 && reinterpret_cast<uintptr_t>(img) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0 &&
                      out_h * out_w <= 0x7fffffffLL;
+    const long long chan_blocks = (chan + 63) / 64;
+    // A window's taps shared between threads: from two rounds of taps on, while the blocks are few enough to run at once.
+    const bool window = vec && out && !forms.h2 && w.ker_w * w.ker_h >= 16 && n * out_h * out_w * chan_blocks <= 4LL * ctx.sm_count && img_h <= 0x7fffffffLL && img_w <= 0x7fffffffLL;
+    ctx.note_launch(ctx.verbose_names && window ? (is_max ? "max_pool2d[window]" : "avg_pool2d[window]") : is_max ? "max_pool2d" : "avg_pool2d");
+    if (ctx.dry() || total == 0) return SAGE_OK;
     if (forms.h2 && !(vec && pool2d_writes_pieces(img, chan, out_h, out_w))) return ctx.fail(SAGE_ERR_INVALID, "pool2d: half-precision pieces need whole groups of channels");
     // 32-bit indices where they reach: two 64-bit divisions were a third of a thread's instructions
     const bool narrow = total < (1LL << 31) && img_h * img_w * chan < (1LL << 31);
     const bool mark = forms.h2 && forms.h2_marked;
-    const long long chan_blocks = (chan + 63) / 64;
-    // (from two rounds of taps on, while its blocks are few enough to run at once)
-    if (vec && out && !forms.h2 && w.ker_w * w.ker_h >= 16 && n * out_h * out_w * chan_blocks <= 4LL * ctx.sm_count && img_h <= 0x7fffffffLL && img_w <= 0x7fffffffLL) {
+    if (window) {
         launch_dependent(ctx.pdl, ctx.stream(), pool2d_window_kernel, dim3((unsigned)(n * out_h * out_w * chan_blocks)), dim3(256), 0, img, out, p, (int)chan_blocks, is_max ? 1 : 0, (int)ctx.opts().ref_compat);
         return ctx.check_cuda(cudaGetLastError(), "pool2d launch");
     }

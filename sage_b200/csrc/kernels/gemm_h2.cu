@@ -1167,7 +1167,7 @@ sage_status gemm_h2_run(Context &ctx, const H2Gemm &g) {
     if (ctx.verbose_names)
         label = "gemm_tc_h2[" + std::to_string(g.m) + "x" + std::to_string(g.n) + "x" + std::to_string(g.k) + (g.batch > 1 ? "x" + std::to_string(g.batch) : "") + (sliced ? (fetch ? ",fetched" : over ? ",over" : "") + std::string(",slices") + std::to_string(cut.slices) : "") +
                 (g.conv ? (halo ? ",conv,taps" : boxed ? ",conv,boxes" : ",conv") : "") + ",bn" + std::to_string(bn) + (cols.narrow ? "/" + std::to_string(cols.wide) + "+" + std::to_string(cols.narrow) + "x192" : "") +
-                (ctas == 2 ? ",pair" : "") + "]o" + std::to_string(out_mask);
+                (ctas == 2 ? ",pair" : "") + (roll && !plain ? ",rolled" : "") + (res ? ",residual" + std::to_string(res - 1) : "") + "]o" + std::to_string(out_mask);
     if (plain) {
         ctx.note_launch(ctx.verbose_names ? label.c_str() : "gemm_tc_3xtf32");
         if (ctx.dry()) return SAGE_OK;

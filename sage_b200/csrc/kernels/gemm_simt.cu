@@ -189,12 +189,14 @@ __global__ void __launch_bounds__(512) gemm_skinny_columns_kernel(GemmP p, long 
 }  // namespace
 
 sage_status gemm_simt(Context &ctx, const GemmArgs &g) {
-    ctx.note_launch("gemm_simt");
+    const long long grid_limit = 0x7fffffffLL;
+    const bool skinny = g.m * g.n <= 8192 && g.k >= 128 && (g.m * g.n * g.batch + 7) / 8 <= grid_limit, columns = skinny && !g.tb && g.n >= 32;
+    // launch lists have one name for these products; verbose ones tell the kernels apart
+    ctx.note_launch(!ctx.verbose_names || !skinny ? "gemm_simt" : columns ? "gemm_simt[columns]" : "gemm_simt[skinny]");
     if (ctx.dry() || g.m == 0 || g.n == 0 || g.batch == 0) return SAGE_OK;
     GemmP p{g.m, g.n, g.k, g.a, g.lda, g.stride_a, g.b, g.ldb, g.stride_b, g.c, g.ldc, g.stride_c, (g.n + BN - 1) / BN, (g.m + BM - 1) / BM, g.batch};
-    const long long grid_limit = 0x7fffffffLL;
-    if (g.m * g.n <= 8192 && g.k >= 128 && (g.m * g.n * g.batch + 7) / 8 <= grid_limit) {
-        if (!g.tb && g.n >= 32) {
+    if (skinny) {
+        if (columns) {
             p.tiles_n = (g.n + 31) / 32;
             launch_dependent(ctx.pdl, ctx.stream(), gemm_skinny_columns_kernel, dim3((unsigned)(p.tiles_n * g.m * g.batch)), dim3(512), 0, p, g.ta ? 1 : g.lda, g.ta ? g.lda : 1);
             return ctx.check_cuda(cudaGetLastError(), "gemm_skinny launch");

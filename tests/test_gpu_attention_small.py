@@ -43,8 +43,7 @@ def test_attention(ctx, n, heads, lq, lk, d, small, per_row):
     ctx.eval(y)
     got = ctx.read(y)
     names = [t for t in ctx.trace() if t.startswith("attention")]
-    if names:  # (the smallest products stay by themselves)
-        assert all(t.startswith("attention_tc_h2[") and t.endswith(",small]") == small for t in names), names
+    assert names == ["attention_tc_h2[%dx%dx%dx%d%s]" % (lq, lk, d, n * heads, ",small" if small else "")]
     got_z = z.eval(ctx)
     ctx.clear()
     ctx.eval(z)  # the pieces alone
@@ -60,4 +59,41 @@ def test_attention(ctx, n, heads, lq, lk, d, small, per_row):
     rows = ok.all(1)
     for a in (got_z, again):
         assert np.abs(a[rows] - ref[rows] @ wo.astype(np.float64)).max() <= 2.0 ** -18 * (np.abs(ref[rows]) @ np.abs(wo.astype(np.float64))).max() + 2.0 ** -18 * np.abs(v).max()
+    assert ctx.status_word() == 0
+
+
+@pytest.mark.parametrize("lq,lk", [(24, 24), (33, 47)])
+def test_what_is_not_finite(ctx, lq, lk):
+    """Infinities and nan in queries, keys, values and the expression's operand: in the places where e / sum(e) of exp(s - max(s, 0)) has them, and
+    every other value as close as ever."""
+    n, heads, d = 1, 2, 64
+    rng = np.random.default_rng(lq)
+    w = heads * d
+    q, k, v = (rng.standard_normal((n, l, w)).astype(np.float32) for l in (lq, lk, lk))
+    mask = np.zeros((n, 1, lq, lk), np.float32)
+    mask[0, 0, :, 3] = -np.inf       # a key nobody looks at
+    mask[0, 0, 5, 7] = np.nan
+    mask[0, 0, 6, :] = -np.inf       # a row of nothing
+    mask[0, 0, 8, 2] = np.inf
+    q[0, 10, 4], q[0, 11, 70] = np.nan, np.inf  # a row of one head each
+    k[0, 9, 20] = -np.inf            # a key of the first head: rows of either sign
+    v[0, 3, 100], v[0, 12, 101], v[0, 13, 102] = np.inf, np.inf, np.nan  # one under weights of 0, two that count, in the second head
+
+    def split(t, l):
+        return S.transpose(S.view(t, [n, l, heads, d]), 2, 1)
+    scores = S.matmul_batched(split(ctx.var(q), lq), S.transpose(split(ctx.var(k), lk), -1, -2)) / float(np.sqrt(np.float32(d)))
+    y = S.view(S.transpose(S.matmul_batched(S.softmax(scores + ctx.var(mask), [3]), split(ctx.var(v), lk)), 2, 1), [n * lq, w])
+    ctx.clear()
+    ctx.trace_begin()
+    ctx.eval(y)
+    got = ctx.read(y)
+    assert [t for t in ctx.trace() if t.startswith("attention")] == ["attention_tc_h2[%dx%dx%dx%d,small]" % (lq, lk, d, heads)]
+    with np.errstate(invalid="ignore", over="ignore"):
+        q64, k64, v64 = (t.astype(np.float64).reshape(n, -1, heads, d).transpose(0, 2, 1, 3) for t in (q, k, v))
+        s = np.einsum("bhqd,bhkd->bhqk", q64, k64) / np.sqrt(d) + mask
+        e = np.exp(s - np.maximum(s.max(-1, keepdims=True), 0.0))
+        ref = np.einsum("bhqk,bhkd->bhqd", e / e.sum(-1, keepdims=True), v64).transpose(0, 2, 1, 3).reshape(n * lq, w)
+    assert np.array_equal(np.isnan(got), np.isnan(ref)) and np.array_equal(got[np.isinf(ref)], ref[np.isinf(ref)])
+    ok = np.isfinite(ref)
+    assert 0.3 < ok.mean() < 0.97 and np.abs(got[ok] - ref[ok]).max() <= 2.0 ** -20 * np.abs(v[np.isfinite(v)]).max() * 4
     assert ctx.status_word() == 0

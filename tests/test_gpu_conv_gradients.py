@@ -9,6 +9,11 @@ import sage_b200 as S
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(autouse=True)
+def verbose(monkeypatch):
+    monkeypatch.setenv("SAGE_VERBOSE_NAMES", "1")  # the launch list tells the kernels apart
+
+
 # (batch, size, channels, kernel, stride, padding): whole rows and ragged ones, channels off the fours (which keep their own map), windows
 # larger than the image's rows, a residual, K long enough for slices
 @pytest.mark.parametrize("b,hw,c,ker,stride,pad,residual", [(4, 9, 32, 3, 1, 1, True), (3, 12, 64, 3, 2, 1, False), (2, 7, 34, 3, 1, 1, True), (8, 4, 256, 3, 1, 1, True), (16, 5, 36, 5, 1, 2, False)])
@@ -31,7 +36,14 @@ def test_gradients(b, hw, c, ker, stride, pad, residual, smooth):
         targets = [loss] + [v.grad(loss) for v in [xv] + wv + bv]
         for _ in range(2):
             ctx.clear()
+            ctx.trace_begin()
             ctx.eval(*targets)
+        names = [t.split("{")[0] + "{map}" if "{map}" in t else t for t in ctx.trace()]
+        # three column matrices (a rectifier is part of its own, a tanh too long to be worked out for every tap), and the maps behind every gradient of
+        # an image; channels off the fours keep their own maps
+        assert [names.count(t) for t in ("im2col{map}", "col2im")] == ([0, names.count("col2im")] if c % 4 else [1 if smooth else 3, 0]), names
+        assert ("col2im{map}" in names) == (c % 4 == 0), names
+        assert any(t.startswith("map{") and ",ZG" in t for t in names) == (c == 256), names
         got = [ctx.read(t).copy() for t in targets]
         assert ctx.status_word() == 0
     finally:
@@ -50,3 +62,64 @@ def test_gradients(b, hw, c, ker, stride, pad, residual, smooth):
     for g, ref in zip(got, [tl.detach()] + [v.grad for v in [tx] + tw + tb]):
         ref = ref.numpy()
         assert np.abs(g.reshape(ref.shape) - ref).max() <= 2.0 ** -15 * np.abs(ref).max()
+
+
+# (rows, K, columns) of products in K slices whose sum is part of the map behind them: whole 16-byte loads, and rows that are not
+@pytest.mark.parametrize("m,k,n,vec", [(128, 4096, 64, 4), (129, 4096, 36, 4), (100, 4096, 34, 1), (64, 8192, 65, 1), (128, 4160, 33, 1)])
+def test_slices_in_the_map(m, k, n, vec):
+    """The product within (2^-22 + 128 x 2^-23 + (K / 128 + 1) 2^-24) |x| |w|: the dropped low x low products, a chain's truncating additions, a
+    rounding for every chain and slice; its bias and rectifier add 2^-23 of what they read."""
+    rng = np.random.default_rng(m + n)
+    x, w, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((k, n)).astype(np.float32), rng.standard_normal(n).astype(np.float32)
+    ctx = S.Context(0)
+    try:
+        xv, wv, bv = ctx.var(x), ctx.var(w), ctx.var(b)
+        y = S.relu(xv.matmul(wv) + bv)
+        loss = (y * y).sum([0, 1], False)
+        targets = [y, loss, wv.grad(loss), xv.grad(loss)]
+        for _ in range(2):
+            ctx.clear()
+            ctx.trace_begin()
+            ctx.eval(*targets)
+        assert any(t.startswith("map{") and ",v%d,ZG" % vec in t for t in ctx.trace()), ctx.trace()
+        got = ctx.read(y).copy()
+        assert ctx.status_word() == 0
+    finally:
+        ctx.close()
+    x64, w64 = x.astype(np.float64), w.astype(np.float64)
+    size = np.abs(x64) @ np.abs(w64) + np.abs(b)
+    assert (np.abs(got - np.maximum(x64 @ w64 + b, 0)) <= (2.0 ** -22 + 128 * 2.0 ** -23 + (k / 128 + 1) * 2.0 ** -24 + 2.0 ** -22) * size).all()
+
+
+@pytest.mark.parametrize("shift", [1, 4])
+def test_images_that_start_anywhere(shift):
+    """An image that starts off the 16-byte grid has its map worked out by itself, before the column matrix and behind the gradient of the image:
+    the same values, the same sums in the same order."""
+    b, hw, c = 2, 6, 8
+    n = b * hw * hw * c
+    rng = np.random.default_rng(shift)
+    x, w, bias = rng.standard_normal(n).astype(np.float32), rng.standard_normal((3, 3, c, 32)).astype(np.float32), rng.standard_normal(32).astype(np.float32)
+    got = []
+    for start in (0, shift):
+        ctx = S.Context(0)
+        try:
+            flat = np.zeros(n + 8, np.float32)
+            flat[start:start + n] = x
+            image = S.view(ctx.var(flat).slice(0, start, start + n), [b, hw, hw, c])
+            wv = ctx.var(w)
+            y = S.conv_2d(S.relu(image), wv, 1, 1, 1) + ctx.var(bias)
+            loss = (y * y).sum([0, 1, 2, 3], False)
+            targets = [loss, wv.grad(loss), image.grad(loss)]
+            for _ in range(2):
+                ctx.clear()
+                ctx.trace_begin()
+                ctx.eval(*targets)
+            names = ctx.trace()
+            on_grid = start % 4 == 0
+            assert (("im2col{map}=planes" in names), ("im2col=planes" in names), ("col2im{map}" in names), ("col2im" in names)) == (on_grid, not on_grid, on_grid, not on_grid), names
+            got.append([ctx.read(t).copy() for t in targets])
+            assert ctx.status_word() == 0
+        finally:
+            ctx.close()
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)

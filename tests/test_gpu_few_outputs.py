@@ -8,7 +8,13 @@ import sage_b200 as S
 pytestmark = pytest.mark.gpu
 
 
-# fewer k than a round of loads and one more than two; columns of one block, cut, and of several; both orders of each operand
+@pytest.fixture(autouse=True)
+def verbose(monkeypatch):
+    monkeypatch.setenv("SAGE_VERBOSE_NAMES", "1")  # the launch list tells the kernels apart
+
+
+# fewer k than a round of loads and one more than two; columns of one block, cut, and of several; both orders of each operand (the last
+# is a tensor-core product)
 @pytest.mark.parametrize("m,n,k", [(1, 1000, 512), (32, 2, 768), (1, 2, 1024), (3, 33, 129), (7, 32, 255), (128, 10, 512), (16, 100, 257), (1, 8192, 128)])
 @pytest.mark.parametrize("ta,tb", [(False, False), (False, True), (True, False), (True, True)])
 def test_products_of_few_outputs(m, n, k, ta, tb):
@@ -18,7 +24,9 @@ def test_products_of_few_outputs(m, n, k, ta, tb):
     ctx = S.Context(0)
     try:
         x, y = ctx.var(np.ascontiguousarray(a.T) if ta else a), ctx.var(np.ascontiguousarray(b.T) if tb else b)
-        got = S.gemm(x, y, ta, tb).eval(ctx) if hasattr(S, "gemm") else (S.transpose(x, 1, 0) if ta else x).matmul(S.transpose(y, 1, 0) if tb else y).eval(ctx)
+        ctx.trace_begin()
+        got = S.gemm(x, y, ta, tb).eval(ctx)
+        assert [t.split("x")[0] for t in ctx.trace()][-1] == ("gemm_tc_h2[1" if n == 8192 else "gemm_simt[skinny]" if tb or n < 32 else "gemm_simt[columns]")
         assert ctx.status_word() == 0
     finally:
         ctx.close()
@@ -35,7 +43,9 @@ def test_pooling_of_large_windows(shape, ker, stride, pad, is_max):
     ctx = S.Context(0)
     try:
         v = (S.max_pool_2d if is_max else S.avg_pool_2d)(ctx.var(x), ker, stride, pad, 1)
+        ctx.trace_begin()
         got = v.eval(ctx)
+        assert ctx.trace() == ["max_pool2d[window]" if is_max else "avg_pool2d[window]"]
     finally:
         ctx.close()
     big = np.zeros((shape[0], shape[1] + 2 * pad, shape[2] + 2 * pad, shape[3]))
@@ -47,3 +57,31 @@ def test_pooling_of_large_windows(shape, ker, stride, pad, is_max):
         assert np.array_equal(got, np.maximum(taps.max(0), 0).astype(np.float32))  # (the reference's accumulator starts at 0)
     else:
         assert (np.abs(got - taps.mean(0)) <= ker * ker * 2.0 ** -24 * np.abs(taps).mean(0) + 1e-30).all()
+
+
+@pytest.mark.parametrize("is_max", [False, True])
+def test_pooling_of_what_is_not_finite(is_max):
+    """Infinities and nan in one tap each, of their own windows and channels: a sum passes them on, a maximum takes +infinity and passes
+    over -infinity and nan (fmaxf), as the ordinary kernel does, which the same windows over more pictures take."""
+    rng = np.random.default_rng(8)
+    x = rng.standard_normal((1, 7, 7, 128)).astype(np.float32)
+    x[0, 1, 2, 3], x[0, 6, 6, 64], x[0, 0, 5, 127], x[0, 3, 3, 9], x[0, 4, 3, 9] = np.inf, -np.inf, np.nan, np.inf, -np.inf
+    ctx = S.Context(0)
+    try:
+        got = []
+        for n in (1, 400):
+            ctx.trace_begin()
+            got.append((S.max_pool_2d if is_max else S.avg_pool_2d)(ctx.var(np.repeat(x, n, 0)), 7, 1, 0, 1).eval(ctx)[0].reshape(128).copy())
+            assert ctx.trace()[-1].endswith("[window]") == (n == 1)
+            ctx.clear()
+    finally:
+        ctx.close()
+    with np.errstate(invalid="ignore"):
+        want = np.fmax(np.fmax.reduce(x.reshape(49, 128), 0), 0) if is_max else x.reshape(49, 128).astype(np.float64).mean(0)
+    for g in got:
+        if is_max:
+            assert np.array_equal(g, want)
+        else:
+            odd = ~np.isfinite(want)
+            assert odd.sum() == 4 and np.array_equal(g[odd], want[odd], equal_nan=True)
+            assert (np.abs(g[~odd] - want[~odd]) <= 49 * 2.0 ** -24 * np.abs(x.reshape(49, 128)).mean(0)[~odd]).all()
