@@ -177,9 +177,8 @@ __global__ void __launch_bounds__(256) col2im_quads_kernel(const float *__restri
 
 // One thread per output pixel and group of 4 channels when C % 4 == 0 (16-byte loads, one 64-bit division per thread), else
 // one thread per element.  Nine taps are asked for at a time, then taken in the window's order: tap after tap a thread waited
-// for the cache each time (3 x 3 over 256 x 112 x 112 x 64: 358 us and a split pass of 62 -> 264 with pieces; 7 x 7
-// over 7 x 7 x 512 of one image, between events: 20.5 -> 12.7).  With pieces
-// asked for, 16 threads hold the 64 channels of a group: no split pass reads the result again.
+// for the cache each time (3 x 3 over 256 x 112 x 112 x 64: 358 us and a split pass of 62 -> 264 with pieces).  Large windows
+// with few results are pool2d_window_kernel's.  With pieces asked for, 16 threads hold the 64 channels of a group: no split pass reads the result again.
 template <int VEC, class I, bool MARK>
 __global__ void __launch_bounds__(256) pool2d_kernel(const float *__restrict__ img, float *__restrict__ out, ConvP p,
                                                      long long total, int is_max, int ref_compat, PlaneOut forms) {

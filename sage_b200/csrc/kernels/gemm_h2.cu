@@ -1338,7 +1338,7 @@ sage_status attention_tc_run(Context &ctx, const TcAttn &a) {
     if (a.out.h2 && (!vec || a.d != 64 || a.ldo % 64 || a.so0 % 64 || a.so1 % 64 || !aligned16(a.out.h2) || a.out.h2_plane % 8))
         return ctx.fail(SAGE_ERR_INVALID, "attention_tc: a result in half-precision pieces needs whole groups of 64 columns");
     // Few short sequences: attn_small_device.inc.  Up to 16 keys always; up to 32 where its blocks are few, or so many that the other
-    // form's tiles, a quarter or less filled, come in rounds; up to 48 where there is hardly anything to do.  In between its many small blocks
+    // form's tiles, a quarter or less filled, come in rounds; up to 48 where there is hardly anything to do (36 and 24 blocks on 148 SMs).  In between its many small blocks
     // leave the next product's less room to start early.  us a layer of BERT (other form | this one; 12 heads unless said otherwise):
     // 8 tokens x 1 51.98 | 45.76, x 16 55.92 | 51.61, x 64 79.33 | 62.33; 16 x 1 60.64 | 53.92, x 4 44.38 | 43.05, x 64 92.44 | 78.04;
     // 24 x 1 44.38 | 40.79, x 4 50.22 | 49.04, x 8 (96 blocks) [55.67] | 58.69, x 32 74.76 | 70.80; 32 x 1 44.15 | 41.70, x 2 46.12 | 43.79,

@@ -38,7 +38,8 @@ def test_no_copies_of_heads_are_left(heads, d, length):
 def test_gradients_are_those_of_the_plain_evaluation(heads, d, length, batch):
     """Against the same graph evaluated operator by operator.  Gradients are sums of a few thousand products through two row
     normalisations: the largest difference stays below 2^-14 of the gradient's largest element (rounding 2^-24 x sqrt(terms) ~ 2^-18,
-    times the amplification of two LayerNorms); of LayerNorm's scalars, sums over all n ~ 10^4 elements that cancel, sqrt(n) ~ 2^7 less."""
+    times the amplification of two LayerNorms); of LayerNorm's scalars, sums over all n ~ 10^4 elements that may cancel, below 2^-14 of the
+    largest element of all gradients (2^-14.9 ... 2^-21.7 seen)."""
     got = []
     for fusion in (1, 0):
         c = S.Context(0, pattern_fusion=fusion)
@@ -54,7 +55,7 @@ def test_gradients_are_those_of_the_plain_evaluation(heads, d, length, batch):
     assert np.abs(got[0][0] - got[1][0]).max() <= 1e-5 * max(1.0, np.abs(got[1][0]).max())
     scale = max(np.abs(g).max() for g in got[1][1:])
     for a, b in zip(got[0][1:], got[1][1:]):
-        assert np.abs(a - b).max() <= 2.0 ** (-14 if a.size > 1 else -14 + 7) * max(np.abs(b).max(), 2.0 ** -10 * scale)
+        assert np.abs(a - b).max() <= 2.0 ** -14 * (max(np.abs(b).max(), 2.0 ** -10 * scale) if a.size > 1 else scale)
 
 
 def views(c, kind, shift, seed=0):
