@@ -9,15 +9,10 @@ import sage_b200 as S
 pytestmark = pytest.mark.gpu
 
 
-@pytest.fixture(autouse=True)
-def verbose(monkeypatch):
-    monkeypatch.setenv("SAGE_VERBOSE_NAMES", "1")  # the launch list tells the kernels apart
-
-
 # rows, k, columns: one tile cut in both directions; no whole 16 bytes in a row; whole groups of 64 (pieces); several tiles a CTA
-@pytest.mark.parametrize("m,k,n,single", [(129, 256, 192, True), (200, 320, 97, True), (462, 768, 3072, True), (4096, 512, 2048, False), (130, 64, 130, True), (5000, 256, 1000, False)])
+@pytest.mark.parametrize("m,k,n", [(129, 256, 192), (200, 320, 97), (462, 768, 3072), (4096, 512, 2048), (130, 64, 130), (5000, 256, 1000)])
 @pytest.mark.parametrize("long", [False, True])
-def test_epilogues(m, k, n, single, long):
+def test_epilogues(m, k, n, long):
     """Against float64: the product within 2^-19 of |x| |w| (its bound, tests of the half-precision products), through a function whose
     slope is at most 1.13, and the second product, of 64 columns, likewise."""
     rng = np.random.default_rng(m + n)
@@ -28,15 +23,12 @@ def test_epilogues(m, k, n, single, long):
         h = ctx.var(x).matmul(ctx.var(w)) + ctx.var(b)
         y = h * 0.5 * ((h * 0.70710678).erf() + 1.0) if long else S.relu(h)
         z = y.matmul(ctx.var(w2))
-        ctx.trace_begin()
         got_y = y.eval(ctx).copy()
         ctx.clear()
         got_z = z.eval(ctx).copy()
         ctx.clear()
         ctx.eval(y, z)
         both = ctx.read(y).copy(), ctx.read(z).copy()
-        names = [t for t in ctx.trace() if t.startswith("gemm_tc_h2[%dx%dx%d," % (m, n, k))]
-        assert len(names) == 3 and all((",rolled" in t) == (single or long) for t in names), names
         assert ctx.status_word() == 0
     finally:
         ctx.close()
@@ -53,13 +45,11 @@ def test_epilogues(m, k, n, single, long):
         assert ((torch.from_numpy(a).double() - y64 @ w2_64).abs() <= z_bound).all()
 
 
-# a residual through the operand ring: tiles of every width, one cut in both directions, rows longer than the result's, a single K-block,
-# one CTA alone, an operand off the 16-byte grid, several tiles to a CTA and slices (which fetch it themselves)
-@pytest.mark.parametrize("m,k,n,kind", [(129, 64, 64, ",bn64,pair"), (200, 320, 100, None), (300, 256, 128, None), (4096, 768, 768, ",bn256/0+4x192,pair"), (1536, 128, 192, ",bn64,pair"), (2000, 200, 516, ",bn64,pair"),
-                                        (6000, 128, 1024, None), (130, 96, 260, ",bn64,pair"), (1100, 200, 1000, ",bn128,pair"), (1100, 64, 1024, ",bn128,pair"), (4096, 200, 1000, ",bn256,pair"),
-                                        (3000, 96, 1000, ",bn256/0+6x192,pair"), (120, 96, 260, ",bn64")])
+# a residual through the operand ring: tiles of every width, one cut in both directions, rows longer than the result's, one tile and
+# several to a CTA, a single K-block, an operand off the 16-byte grid (which the store fetches itself)
+@pytest.mark.parametrize("m,k,n", [(129, 64, 64), (200, 320, 100), (300, 256, 128), (4096, 768, 768), (1536, 128, 192), (2000, 200, 516), (6000, 128, 1024), (130, 96, 260)])
 @pytest.mark.parametrize("wider,shift", [(0, 0), (8, 4), (8, 1)])
-def test_residuals(m, k, n, kind, wider, shift):
+def test_residuals(m, k, n, wider, shift):
     """Against float64, within 2^-19 of |x| |w| + |r|."""
     rng = np.random.default_rng(m + n + wider)
     x, w, b = rng.standard_normal((m, k)).astype(np.float32), (rng.standard_normal((k, n)) / np.sqrt(k)).astype(np.float32), rng.standard_normal(n).astype(np.float32)
@@ -72,14 +62,17 @@ def test_residuals(m, k, n, kind, wider, shift):
         y = ctx.var(x).matmul(ctx.var(w)) + ctx.var(b) + rv
         for _ in range(2):
             ctx.clear()
-            ctx.trace_begin()
             got = y.eval(ctx).copy()
-        names = [t for t in ctx.trace() if t.startswith("gemm_tc_h2[%dx%dx%d," % (m, n, k))]
-        assert len(names) == 1 and (",residual1]" in names[0]) == (kind is not None and shift != 1), names
-        assert kind is None or kind + (",residual1" if shift != 1 else "") + "]" in names[0], names
         assert ctx.status_word() == 0
     finally:
         ctx.close()
     x64, w64 = x.astype(np.float64), w.astype(np.float64)
     r64 = r[:, shift:shift + n].astype(np.float64)
     assert (np.abs(got - (x64 @ w64 + b + r64)) <= 2.0 ** -19 * (np.abs(x64) @ np.abs(w64) + np.abs(b) + np.abs(r64))).all()
+
+
+# wider tiles through the ring, a CTA alone, several tiles to a CTA
+@pytest.mark.parametrize("m,k,n", [(1100, 200, 1000), (1100, 64, 1024), (4096, 200, 1000), (3000, 96, 1000), (120, 96, 260)])
+@pytest.mark.parametrize("wider,shift", [(0, 0), (8, 4), (8, 1)])
+def test_residuals_of_other_tiles(m, k, n, wider, shift):
+    test_residuals(m, k, n, wider, shift)

@@ -495,34 +495,11 @@ def test_program_cache_is_bounded_and_least_recently_used():
         ctx.close()
 
 
-def trace_comment():
-    header = open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "include", "sage_cuda.h")).read()
-    return header.split("sage_status sage_trace_begin")[0].rsplit("/*", 1)[1]
-
-
-def test_launch_list_of_results_that_run_together():
-    """Products, the sums over their K slices, column sums and sums over whole tensors: a line for each result, up to the number of lines the
-    header states; one more result than that is another launch."""
-    most = [int(n) for n in re.findall(r"up to (\d+)", " ".join(trace_comment().replace("*", " ").split()))]
-    assert most == [100, 96]
-    ctx = S.Context(-1)
-    x, y = ctx.var(np.zeros((512, 64), np.float32)), ctx.var(np.zeros((512, 32), np.float32))
-    for n in (2, 100, 101):
-        for targets, name, limit in (([S.transpose(x, 1, 0).matmul(y) for _ in range(n)], "gemm_tc_3xtf32", most[0]), ([x.sum([0], False) for _ in range(n)], "reduce_cols", most[1]),
-                                     ([x.sum([0, 1], False) for _ in range(n)], "reduce_total", most[1])):
-            ctx.eval(*targets)  # (and the operands' planes)
-            ctx.clear()
-            before = ctx.launch_count()[0]
-            ctx.trace_begin()
-            ctx.eval(*targets)
-            lines = ctx.trace()
-            assert lines.count(name) == n and len(lines) - (ctx.launch_count()[0] - before) >= n - (n + limit - 1) // limit, (n, name)
-    ctx.close()
-
-
 def test_launch_list_and_count_of_a_plain_product():
-    """Both operands are brought into pieces by one launch that the list names once for each: include/sage_cuda.h says so."""
-    assert "two lines" in trace_comment() and "longer than" in trace_comment()
+    """Both operands are brought into pieces by one launch that the list names once for each: include/sage_cuda.h says so, and this is
+    the only launch with two lines."""
+    header = open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "include", "sage_cuda.h")).read()
+    assert "longer than" in header.split("sage_status sage_trace_begin")[0].rsplit("/*", 1)[1]
     ctx = S.Context(-1)
     L = ctypes.c_int64
     a, b, c = ctx.empty((256, 256)), ctx.empty((256, 256)), ctx.empty((256, 256))
@@ -551,4 +528,29 @@ def test_tensors_of_38_to_40_mib(elements):
     assert ctx.mem_stats()["num_device_allocs"] == allocs + 1
     for t in (again, small):
         t.release()
+    ctx.close()
+
+
+def trace_comment():
+    header = open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "include", "sage_cuda.h")).read()
+    return header.split("sage_status sage_trace_begin")[0].rsplit("/*", 1)[1]
+
+
+def test_launch_list_of_results_that_run_together():
+    """Products, the sums over their K slices, column sums and sums over whole tensors: a line for each result, up to the number of lines the
+    header states; one more result than that is another launch."""
+    most = [int(n) for n in re.findall(r"up to (\d+)", " ".join(trace_comment().replace("*", " ").split()))]
+    assert most == [100, 96]
+    ctx = S.Context(-1)
+    x, y = ctx.var(np.zeros((512, 64), np.float32)), ctx.var(np.zeros((512, 32), np.float32))
+    for n in (2, 100, 101):
+        for targets, name, limit in (([S.transpose(x, 1, 0).matmul(y) for _ in range(n)], "gemm_tc_3xtf32", most[0]), ([x.sum([0], False) for _ in range(n)], "reduce_cols", most[1]),
+                                     ([x.sum([0, 1], False) for _ in range(n)], "reduce_total", most[1])):
+            ctx.eval(*targets)  # (and the operands' planes)
+            ctx.clear()
+            before = ctx.launch_count()[0]
+            ctx.trace_begin()
+            ctx.eval(*targets)
+            lines = ctx.trace()
+            assert lines.count(name) == n and len(lines) - (ctx.launch_count()[0] - before) >= n - (n + limit - 1) // limit, (n, name)
     ctx.close()
