@@ -619,10 +619,11 @@ static void group_gemms(Node &root) {
     }
 }
 
-// Where a state starts in the storage it lies in: it may be a view of its routine's result, or of another state.
+// Where a state starts in the storage it lies in: it may be a view of its routine's result, or of another state, through
+// any number of them.
 static long long state_offset(Program &p, Origin *key) {
     long long at = 0;
-    for (int hops = 0; hops < 8; ++hops) {
+    for (;;) {
         auto it = p.routines.find(key);
         if (it == p.routines.end() || it->second.row) break;
         long long views = 0;

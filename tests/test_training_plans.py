@@ -120,3 +120,24 @@ def test_gradients_of_scalars(heads, d, length, batch):
     scale = max(np.abs(g).max() for g in got[1])
     scalars = [(a, b) for a, b in zip(*got) if a.size == 1]
     assert len(scalars) == 10 and all(np.abs(a - b).max() <= 2.0 ** -14 * scale for a, b in scalars), len(scalars)
+
+
+@pytest.mark.parametrize("levels", [1, 7, 8, 9, 12])
+def test_products_at_the_end_of_a_chain_of_views(levels):
+    """Views of views, each a state: a product on the 16-byte grid reads every one of them, and two off it the last, which gather values."""
+    c = S.Context(-1)
+    m, k = 256, 64
+
+    def matrix(v, at):
+        return S.view(v.slice(0, at, at + m * k), [m, k])
+    size = m * k + 4 * levels + 8
+    v = (c.var(np.zeros(size + 1, np.float32)) * 2.0 + 1.0).slice(0, 1, size + 1)
+    w, g = c.var(np.zeros((k, 96), np.float32)), c.var(np.zeros((m, 96), np.float32))
+    targets = []
+    for _ in range(levels):
+        targets.append(matrix(v, 3).matmul(w))
+        v = v.slice(0, 4, v.extents[0])
+    c.eval(*targets, matrix(v, 0).matmul(w), S.transpose(matrix(v, 0), 1, 0).matmul(g))
+    first = c.describe().splitlines()[0]
+    assert "+planes" in first and "=planes" not in first, first
+    c.close()
