@@ -695,8 +695,6 @@ static std::vector<RowGroupPlan> plan_row_groups(const std::vector<Var> &order, 
     if (n < 1 || n > 4096) return plans;  // the legality test is quadratic in the number of states
     std::unordered_map<Origin *, int> index;
     for (int i = 0; i < n; ++i) index[order[i].key()] = i;
-    const int words = (n + 63) / 64;
-    std::vector<std::vector<uint64_t>> anc(n, std::vector<uint64_t>(words, 0));  // states that state i depends on
     std::vector<std::vector<int>> reads(n);
     std::vector<long long> R(n, 0), C(n, 0);
     std::vector<char> ok(n, 0), exchanges(n, 0);
@@ -706,8 +704,6 @@ static std::vector<RowGroupPlan> plan_row_groups(const std::vector<Var> &order, 
             auto it = index.find(v.key());
             if (it == index.end()) continue;
             reads[i].push_back(it->second);
-            anc[i][it->second / 64] |= 1ull << (it->second % 64);
-            for (int w = 0; w < words; ++w) anc[i][w] |= anc[it->second][w];
         }
         if (auto probe = row_program_build(in, {order[i]}, false, false)) {
             ok[i] = 1;
@@ -721,23 +717,34 @@ static std::vector<RowGroupPlan> plan_row_groups(const std::vector<Var> &order, 
         group[i] = i;
         members[i] = {i};
     }
-    auto in_set = [&](const std::vector<uint64_t> &set, int i) { return (set[i / 64] >> (i % 64)) & 1; };
-    // May groups P and Q become one routine?  Not if some state outside them lies between them (it would
-    // have to run both after and before the merged routine).
+    // May groups P and Q become one routine?  Not if something outside them lies between them (it would have to run both after and
+    // before the merged routine).  A group that something between belongs to counts whole: it is one routine too.
+    std::vector<int> seen(n, -1), pending;
+    int round = 0;
     auto legal = [&](int P, int Q) {
-        std::vector<uint64_t> u(words, 0), au(words, 0);
-        for (int g : {P, Q})
-            for (int m : members[g]) {
-                u[m / 64] |= 1ull << (m % 64);
-                for (int w = 0; w < words; ++w) au[w] |= anc[m][w];
-            }
         if (members[P].size() + members[Q].size() > 24) return false;  // keeps the register arrays of one kernel in hand
-        for (int x = 0; x < n; ++x) {
-            if (!in_set(au, x) || in_set(u, x)) continue;
-            for (int w = 0; w < words; ++w)
-                if (anc[x][w] & u[w]) return false;
+        ++round;
+        for (int g : {P, Q})
+            for (int m : members[g])
+                for (int r : reads[m])
+                    if (group[r] != P && group[r] != Q && seen[group[r]] != round) {
+                        seen[group[r]] = round;
+                        pending.push_back(group[r]);
+                    }
+        bool between = false;
+        while (!pending.empty()) {
+            const int g = pending.back();
+            pending.pop_back();
+            for (int m : members[g])
+                for (int r : reads[m]) {
+                    between = between || group[r] == P || group[r] == Q;
+                    if (!between && seen[group[r]] != round) {
+                        seen[group[r]] = round;
+                        pending.push_back(group[r]);
+                    }
+                }
         }
-        return true;
+        return !between;
     };
     for (int i = 0; i < n; ++i) {
         if (!ok[i]) continue;
